@@ -8,6 +8,8 @@ GPU code path never falls back to eager PyTorch when its library is missing.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import threading
 from pathlib import Path
@@ -49,6 +51,39 @@ def load(name: str, *, build_if_missing: bool = True) -> C.CDLL:
         lib = C.CDLL(str(path), mode=C.RTLD_GLOBAL if name == "libbshmem_cuda.so" else C.RTLD_LOCAL)
         _libs[name] = lib
         return lib
+
+
+_pycall_mod = None
+
+
+def _pycall():
+    """The extension module of csrc/host/pycall.cc (built on first use like the other libraries)."""
+    global _pycall_mod
+    if _pycall_mod is None:
+        with _lock:
+            if _pycall_mod is None:
+                path = _LIB_DIR / "bshmem_pycall.so"
+                if not path.exists():
+                    with _build_lock():
+                        _build.build_pycall()
+                loader = importlib.machinery.ExtensionFileLoader("bshmem_pycall", str(path))
+                spec = importlib.util.spec_from_file_location("bshmem_pycall", str(path), loader=loader)
+                mod = importlib.util.module_from_spec(spec)
+                loader.exec_module(mod)
+                _pycall_mod = mod
+    return _pycall_mod
+
+
+def fast(lib: C.CDLL, name: str):
+    """The declared entry point `name` of `lib` as a callable that takes plain integers (addresses included) and None.
+
+    For entry points on a path that runs once per message or per layer: a ctypes call of the same function costs 1.5 to
+    3 us, this one 0.15 us.  A result declared as a pointer comes back as an integer (0 = null)."""
+    fn = getattr(lib, name)
+    if fn.argtypes is None:
+        raise TypeError(f"{name}: declare argtypes first")
+    kind = 0 if fn.restype is C.c_int else (2 if fn.restype is None else 1)
+    return _pycall().Native(C.cast(fn, C.c_void_p).value, len(fn.argtypes), kind)
 
 
 class _build_lock:
@@ -131,6 +166,8 @@ def declare_runtime_api(lib: C.CDLL) -> None:
     f("bshmem_team_translate_pe", _I, _VP, C.c_int32, _I, C.c_int32)
     for nm in ("putmem", "getmem", "putmem_nbi", "getmem_nbi"):
         f("bshmem_ctx_" + nm, _I, _VP, C.c_int32, _VP, _VP, _SZ, _I)
+    f("bshmem_ctx_p_word", _I, _VP, C.c_int32, _VP, _U64, _SZ, _I)
+    f("bshmem_ctx_g_word", _I, _VP, C.c_int32, _VP, _SZ, _I, C.POINTER(_U64))
     for nm in ("putmem_signal", "putmem_signal_nbi"):
         f("bshmem_ctx_" + nm, _I, _VP, C.c_int32, _VP, _VP, _SZ, _VP, _U64, _I, _I)
     f("bshmem_signal_fetch", _U64, _VP, _VP)

@@ -18,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -101,6 +102,18 @@ def build_host(force: bool = False) -> Path:
     return out
 
 
+def build_pycall(force: bool = False) -> Path:
+    """The CPython callables over the native libraries (csrc/host/pycall.cc); needs the interpreter's own headers."""
+    LIB.mkdir(exist_ok=True)
+    out = LIB / "bshmem_pycall.so"
+    src = CSRC / "host/pycall.cc"
+    if force or _stale(out, [src]):
+        cmd = ["g++", "-std=c++17", "-O2", "-g", "-fPIC", "-shared", "-Wall", "-Wextra", "-Wno-missing-field-initializers",
+               "-I", sysconfig.get_paths()["include"], "-o", str(out), str(src)]
+        _run(cmd, LIB / "bshmem_pycall.build.log")
+    return out
+
+
 def build_sanitizer_driver(kind: str, force: bool = False) -> Path:
     """The host runtime and its native stress driver (csrc/host/sanitize_main.cc) as one executable built with
     -fsanitize=<kind> ("thread" or "address"): data races and memory errors in the allocator, the team table, the
@@ -152,6 +165,7 @@ def build_cuda_target(name: str, force: bool = False) -> Path | None:
 def build_all(force: bool = False, cuda: bool = True) -> dict[str, str]:
     """Build everything that has sources; returns {artefact: path}."""
     built = {"libbshmem_host.so": str(build_host(force))}
+    build_pycall(force)
     if cuda and _nvcc() is not None:
         with ThreadPoolExecutor(max_workers=min(6, os.cpu_count() or 2)) as ex:
             futs = {n: ex.submit(build_cuda_target, n, force) for n in CUDA_TARGETS}

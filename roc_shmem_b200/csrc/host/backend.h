@@ -72,6 +72,9 @@ class Backend {
   virtual int get(int pe, void* local, uint64_t src_off, uint64_t n, bool nbi) = 0;
   virtual int put_signal(int pe, uint64_t dst_off, const void* local, uint64_t n, uint64_t sig_off,
                          uint64_t sig_val, int sig_op, bool nbi) = 0;
+  // One element of 1 to 8 bytes, its value in the low bytes of a word: single-element get (blocking) and put (not).
+  virtual int read_word(int pe, uint64_t off, uint64_t size, uint64_t* out) { *out = 0; return get(pe, out, off, size, false); }
+  virtual int write_word(int pe, uint64_t off, uint64_t bits, uint64_t size) { return put(pe, off, &bits, size, true); }
   virtual int amo(int pe, uint64_t off, int dtype, int op, uint64_t value, uint64_t cond,
                   uint64_t* fetched) = 0;
   virtual int fence() = 0;

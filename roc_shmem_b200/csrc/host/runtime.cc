@@ -433,6 +433,36 @@ int bshmem_ctx_putmem_nbi(bshmem_handle_t h, bshmem_ctx_t c, void* d, const void
 int bshmem_ctx_getmem(bshmem_handle_t h, bshmem_ctx_t c, void* d, const void* s, size_t n, int pe) { return do_get(h, c, d, s, n, pe, false); }
 int bshmem_ctx_getmem_nbi(bshmem_handle_t h, bshmem_ctx_t c, void* d, const void* s, size_t n, int pe) { return do_get(h, c, d, s, n, pe, true); }
 
+int bshmem_ctx_p_word(bshmem_handle_t h, bshmem_ctx_t c, void* dest, uint64_t bits, size_t size, int pe) {
+  CHECK_H(h);
+  HostContext* x = h->ctx(c);
+  if (!x) return h->fail(BSHMEM_ERR_INVALID, "p: invalid context");
+  if (size != 1 && size != 2 && size != 4 && size != 8) return h->fail(BSHMEM_ERR_INVALID, "p: bad element size");
+  int wpe = h->resolve_pe(c, pe);
+  uint64_t off;
+  if (wpe < 0) return h->fail(BSHMEM_ERR_INVALID, "p: PE out of range");
+  if (!h->to_offset(dest, size, &off)) return h->fail(BSHMEM_ERR_RANGE, "p: dest is not symmetric");
+  STAT(h, x, ST_PUT_NBI);
+  STAT(h, x, ST_BYTES_PUT, size);
+  CtxScope sel(h, c);
+  return h->backend->write_word(wpe, off, bits, size);
+}
+
+int bshmem_ctx_g_word(bshmem_handle_t h, bshmem_ctx_t c, const void* src, size_t size, int pe, uint64_t* bits) {
+  CHECK_H(h);
+  HostContext* x = h->ctx(c);
+  if (!x || !bits) return h->fail(BSHMEM_ERR_INVALID, "g: invalid context or result");
+  if (size != 1 && size != 2 && size != 4 && size != 8) return h->fail(BSHMEM_ERR_INVALID, "g: bad element size");
+  int wpe = h->resolve_pe(c, pe);
+  uint64_t off;
+  if (wpe < 0) return h->fail(BSHMEM_ERR_INVALID, "g: PE out of range");
+  if (!h->to_offset(src, size, &off)) return h->fail(BSHMEM_ERR_RANGE, "g: source is not symmetric");
+  STAT(h, x, ST_GET);
+  STAT(h, x, ST_BYTES_GET, size);
+  CtxScope sel(h, c);
+  return h->backend->read_word(wpe, off, size, bits);
+}
+
 static int do_put_signal(bshmem_handle_t h, int c, void* dest, const void* src, size_t n, uint64_t* sig,
                          uint64_t val, int sig_op, int pe, bool nbi) {
   CHECK_H(h);

@@ -96,6 +96,9 @@ int bshmem_ctx_putmem(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void*
 int bshmem_ctx_getmem(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, int pe);
 int bshmem_ctx_putmem_nbi(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, int pe);
 int bshmem_ctx_getmem_nbi(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, int pe);
+/* single element of `size` (1, 2, 4 or 8) bytes, bit pattern in the low bytes of a word */
+int bshmem_ctx_p_word(bshmem_handle_t h, bshmem_ctx_t c, void* dest, uint64_t bits, size_t size, int pe);
+int bshmem_ctx_g_word(bshmem_handle_t h, bshmem_ctx_t c, const void* src, size_t size, int pe, uint64_t* bits);
 int bshmem_ctx_putmem_signal(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n,
                              uint64_t* sig_addr, uint64_t signal, int sig_op, int pe);
 int bshmem_ctx_putmem_signal_nbi(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n,

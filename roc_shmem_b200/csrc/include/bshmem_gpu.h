@@ -81,6 +81,11 @@ int bshmem_gpu_trace_enable(bshmem_handle_t h, int capacity);
 int bshmem_gpu_trace_read(bshmem_handle_t h, uint64_t* out, int max_events, int* n_out, uint64_t* total);
 int bshmem_gpu_rma_kernel(bshmem_handle_t h, void* sym, void* local, uint64_t n, int pe, int is_put, int scope,
                           int ctas, int threads);
+/* context RMA whose local buffer is known to be memory of this PE's GPU */
+int bshmem_gpu_ctx_put_dev(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, int pe, int nbi);
+int bshmem_gpu_ctx_get_dev(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, int pe, int nbi);
+int bshmem_gpu_ctx_put_signal_dev(bshmem_handle_t h, bshmem_ctx_t c, void* dest, const void* src, size_t n, uint64_t* sig, uint64_t value,
+                                  int sig_op, int pe, int nbi);
 int bshmem_gpu_group_collective(bshmem_handle_t* handles, int n, int team_slot, int kind, int dtype, int op, int root,
                                 uint64_t dst_off, uint64_t src_off, uint64_t count, int ctas);
 int bshmem_gpu_group_team_split(bshmem_handle_t* handles, int n, int parent_slot, int start, int stride, int size,

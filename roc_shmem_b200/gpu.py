@@ -24,12 +24,14 @@ from . import _native
 from .bootstrap import Bootstrap
 from .config import Config
 from .cpu import native_config
-from .runtime import Runtime
+from .runtime import Runtime, _ptr_of
 from .utils import dtypes as D
 from .utils.errors import ShmemError, raise_for_status
 
 _VP, _I, _U64 = C.c_void_p, C.c_int, C.c_uint64
 _declared = False
+Tensor = torch.Tensor
+_SCOPES = {"thread": 0, "warp": 1, "block": 2, "bulk": 3}
 
 
 class DevState(C.Structure):
@@ -84,6 +86,10 @@ def cuda_lib() -> C.CDLL:
         f("bshmem_gpu_trace_enable", _I, _VP, _I)
         f("bshmem_gpu_trace_read", _I, _VP, C.POINTER(_U64), _I, C.POINTER(_I), C.POINTER(_U64))
         f("bshmem_gpu_rma_kernel", _I, _VP, _VP, _VP, _U64, _I, _I, _I, _I, _I)
+        CI, SZ = C.c_int32, C.c_size_t
+        f("bshmem_gpu_ctx_put_dev", _I, _VP, CI, _VP, _VP, SZ, _I, _I)
+        f("bshmem_gpu_ctx_get_dev", _I, _VP, CI, _VP, _VP, SZ, _I, _I)
+        f("bshmem_gpu_ctx_put_signal_dev", _I, _VP, CI, _VP, _VP, SZ, _VP, _U64, _I, _I, _I)
         f("bshmem_gpu_group_collective", _I, C.POINTER(_VP), _I, _I, _I, _I, _I, _I, _U64, _U64, _U64, _I)
         f("bshmem_gpu_group_team_split", _I, C.POINTER(_VP), _I, _I, _I, _I, _I, C.POINTER(_I))
         f("bshmem_gpu_get_stream", _I, _VP, C.POINTER(_VP))
@@ -142,6 +148,44 @@ class DeviceRuntime(Runtime):
                          tensor_from_ptr=lambda p, shape, dtype: cuda_tensor_from_ptr(p, shape, dtype, device),
                          device=device)
         self.heap = heap
+        self._dev_index = device.index
+        self._c_put_dev = _native.fast(lib, "bshmem_gpu_ctx_put_dev")
+        self._c_get_dev = _native.fast(lib, "bshmem_gpu_ctx_get_dev")
+        self._c_put_signal_dev = _native.fast(lib, "bshmem_gpu_ctx_put_signal_dev")
+        self._c_rma_kernel = _native.fast(lib, "bshmem_gpu_rma_kernel")
+
+    # RMA between tensors: a local tensor on this PE's GPU is announced as such (csrc/cuda/gpu_backend.cu then moves
+    # small messages without a copy-engine request); anything else takes the general path
+    def put(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
+        """Copy `src` (any local buffer) into `dest`'s location on PE `pe`."""
+        if isinstance(src, Tensor) and src.is_cuda and src.get_device() == self._dev_index and isinstance(dest, Tensor):
+            st = self._c_put_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
+                                 src.nbytes if nbytes is None else nbytes, pe, nbi)
+            if st:
+                self._check(st)
+            return
+        super().put(dest, src, pe, ctx=ctx, nbi=nbi, nbytes=nbytes)
+
+    def get(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
+        """Copy `src`'s location on PE `pe` into the local buffer `dest`."""
+        if isinstance(dest, Tensor) and dest.is_cuda and dest.get_device() == self._dev_index and isinstance(src, Tensor):
+            st = self._c_get_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
+                                 dest.nbytes if nbytes is None else nbytes, pe, nbi)
+            if st:
+                self._check(st)
+            return
+        super().get(dest, src, pe, ctx=ctx, nbi=nbi, nbytes=nbytes)
+
+    def put_signal(self, dest, src, sig, value: int, pe: int, *, op: int = D.SIGNAL_SET, ctx=None, nbi: bool = False) -> None:
+        """Put, then update the 64-bit signal word `sig` on PE `pe` (SET or ADD);
+        the payload is visible to a reader that observed the signal."""
+        if isinstance(src, Tensor) and src.is_cuda and src.get_device() == self._dev_index and isinstance(dest, Tensor):
+            st = self._c_put_signal_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(), src.nbytes,
+                                        _ptr_of(sig), value, op, pe, nbi)
+            if st:
+                self._check(st)
+            return
+        super().put_signal(dest, src, sig, value, pe, op=op, ctx=ctx, nbi=nbi)
 
     # stream-ordered mode: calls enqueue on `stream` and return; errors surface at quiet()
     def set_stream(self, stream: Optional[torch.cuda.Stream]) -> None:
@@ -200,10 +244,10 @@ class DeviceRuntime(Runtime):
                    ctas: int = 32, threads: int = 512, nbytes: Optional[int] = None) -> None:
         """Device-initiated put/get striped over `ctas` CTAs (enqueued, not synchronised).  Scope "bulk" moves the
         data with bulk async copies through shared memory (16-byte aligned addresses and size)."""
-        sc = {"thread": 0, "warp": 1, "block": 2, "bulk": 3}[scope]
-        n = nbytes if nbytes is not None else local.numel() * local.element_size()
-        self._check(self.lib.bshmem_gpu_rma_kernel(self.h, sym.data_ptr(), local.data_ptr(), n, pe, int(put), sc, ctas,
-                                                   threads))
+        st = self._c_rma_kernel(self._hv, sym.data_ptr(), local.data_ptr(), local.nbytes if nbytes is None else nbytes, pe, put,
+                                _SCOPES[scope], ctas, threads)
+        if st:
+            self._check(st)
 
     def offset_of(self, t: torch.Tensor) -> int:
         return t.data_ptr() - int(self.lib.bshmem_heap_base(self.h))
@@ -326,6 +370,12 @@ class DeviceRuntime(Runtime):
         st = C.c_int(-1)
         self._check(self.lib.bshmem_gpu_wg_collectives(self.h, dst.data_ptr(), src.data_ptr(), src.numel(), C.byref(st)))
         return st.value
+
+
+# NVTX ranges around the methods overridden here (the inherited ones are instrumented in runtime.py)
+from .utils.trace import instrument as _instrument  # noqa: E402
+
+_instrument(DeviceRuntime, ("put", "get", "put_signal"))
 
 
 def init_device_runtime(boot: Bootstrap, cfg: Config, device: Optional[int] = None, proxy: bool = False) -> DeviceRuntime:

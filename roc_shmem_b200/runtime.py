@@ -15,6 +15,7 @@ tensors carry their dtype.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Callable, Optional, Sequence
 
 import torch
@@ -30,9 +31,9 @@ CTX_DEFAULT = 0
 CTX_NOSTORE, CTX_SERIALIZED, CTX_WG_PRIVATE, CTX_SHARED = 1, 2, 4, 8
 
 
-def _ptr_of(x) -> int:
+def _ptr_of(x, Tensor=torch.Tensor) -> int:
     """Raw address of a tensor / numpy array / int."""
-    if isinstance(x, torch.Tensor):
+    if isinstance(x, Tensor):
         return x.data_ptr()
     if isinstance(x, int):
         return x
@@ -42,8 +43,6 @@ def _ptr_of(x) -> int:
 
 
 def _nbytes(x) -> int:
-    if isinstance(x, torch.Tensor):
-        return x.numel() * x.element_size()
     return x.nbytes
 
 
@@ -105,11 +104,11 @@ class Context:
         self.destroy()
 
     # convenience forwards
-    def put(self, dest, src, pe, **kw):
-        return self.rt.put(dest, src, pe, ctx=self, **kw)
+    def put(self, dest, src, pe, *, nbi=False, nbytes=None):
+        return self.rt.put(dest, src, pe, ctx=self, nbi=nbi, nbytes=nbytes)
 
-    def get(self, dest, src, pe, **kw):
-        return self.rt.get(dest, src, pe, ctx=self, **kw)
+    def get(self, dest, src, pe, *, nbi=False, nbytes=None):
+        return self.rt.get(dest, src, pe, ctx=self, nbi=nbi, nbytes=nbytes)
 
     def fence(self):
         self.rt.fence(self)
@@ -133,6 +132,16 @@ class Runtime:
                  on_finalize: Optional[Callable] = None):
         self.lib = lib
         self.h = C.c_void_p(handle)
+        # entry points that run once per message: called with plain integers (see _native.fast), handle included
+        self._hv = int(handle)
+        f = lambda name: _native.fast(lib, name)  # noqa: E731
+        self._c_put, self._c_put_nbi = f("bshmem_ctx_putmem"), f("bshmem_ctx_putmem_nbi")
+        self._c_get, self._c_get_nbi = f("bshmem_ctx_getmem"), f("bshmem_ctx_getmem_nbi")
+        self._c_put_signal, self._c_put_signal_nbi = f("bshmem_ctx_putmem_signal"), f("bshmem_ctx_putmem_signal_nbi")
+        self._c_p, self._c_g, self._c_amo = f("bshmem_ctx_p_word"), f("bshmem_ctx_g_word"), f("bshmem_ctx_amo")
+        self._c_fence, self._c_quiet = f("bshmem_ctx_fence"), f("bshmem_ctx_quiet")
+        self._c_wait_until = f("bshmem_wait_until")
+        self._tls = threading.local()                 # a result word per thread
         self._tensor_from_ptr = tensor_from_ptr
         self.device = device
         self._on_finalize = on_finalize
@@ -154,6 +163,15 @@ class Runtime:
 
     def _team(self, team) -> int:
         return TEAM_WORLD if team is None else (team.slot if isinstance(team, Team) else int(team))
+
+    def _word(self):
+        """This thread's 64-bit result word and its address."""
+        try:
+            return self._tls.word
+        except AttributeError:
+            w = C.c_uint64(0)
+            self._tls.word = (w, C.addressof(w))
+            return self._tls.word
 
     def make_current(self) -> None:
         """Bind this PE to the calling thread for the handle-free typed C API."""
@@ -265,22 +283,26 @@ class Runtime:
     # ---- RMA -----------------------------------------------------------------------
     def put(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
         """Copy `src` (any local buffer) into `dest`'s location on PE `pe`."""
-        n = _nbytes(src) if nbytes is None else nbytes
-        fn = self.lib.bshmem_ctx_putmem_nbi if nbi else self.lib.bshmem_ctx_putmem
-        self._check(fn(self.h, self._ctx(ctx), _ptr_of(dest), _ptr_of(src), n, pe))
+        n = src.nbytes if nbytes is None else nbytes
+        st = (self._c_put_nbi if nbi else self._c_put)(self._hv, self._ctx(ctx), _ptr_of(dest), _ptr_of(src), n, pe)
+        if st:
+            self._check(st)
 
     def get(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
         """Copy `src`'s location on PE `pe` into the local buffer `dest`."""
-        n = _nbytes(dest) if nbytes is None else nbytes
-        fn = self.lib.bshmem_ctx_getmem_nbi if nbi else self.lib.bshmem_ctx_getmem
-        self._check(fn(self.h, self._ctx(ctx), _ptr_of(dest), _ptr_of(src), n, pe))
+        n = dest.nbytes if nbytes is None else nbytes
+        st = (self._c_get_nbi if nbi else self._c_get)(self._hv, self._ctx(ctx), _ptr_of(dest), _ptr_of(src), n, pe)
+        if st:
+            self._check(st)
 
     def put_signal(self, dest, src, sig, value: int, pe: int, *, op: int = D.SIGNAL_SET, ctx=None,
                    nbi: bool = False) -> None:
         """Put, then update the 64-bit signal word `sig` on PE `pe` (SET or ADD);
         the payload is visible to a reader that observed the signal."""
-        fn = self.lib.bshmem_ctx_putmem_signal_nbi if nbi else self.lib.bshmem_ctx_putmem_signal
-        self._check(fn(self.h, self._ctx(ctx), _ptr_of(dest), _ptr_of(src), _nbytes(src), _ptr_of(sig), value, op, pe))
+        st = (self._c_put_signal_nbi if nbi else self._c_put_signal)(self._hv, self._ctx(ctx), _ptr_of(dest), _ptr_of(src),
+                                                                     src.nbytes, _ptr_of(sig), value, op, pe)
+        if st:
+            self._check(st)
 
     def signal_fetch(self, sig) -> int:
         return int(self.lib.bshmem_signal_fetch(self.h, _ptr_of(sig)))
@@ -288,25 +310,27 @@ class Runtime:
     def p(self, dest: torch.Tensor, value, pe: int, *, ctx=None) -> None:
         """Single-element put of a scalar into dest[0] on PE `pe`."""
         code = D.code_of(dest.dtype)
-        buf = (C.c_uint64 * 1)(D.to_bits(code, value))
-        self._check(self.lib.bshmem_ctx_putmem_nbi(self.h, self._ctx(ctx), _ptr_of(dest), C.addressof(buf),
-                                                   D.size_of(code), pe))
+        st = self._c_p(self._hv, self._ctx(ctx), _ptr_of(dest), D.to_bits(code, value), D.size_of(code), pe)
+        if st:
+            self._check(st)
 
     def g(self, src: torch.Tensor, pe: int, *, ctx=None):
         """Single-element get of src[0] from PE `pe`."""
         code = D.code_of(src.dtype)
-        buf = (C.c_uint64 * 1)(0)
-        self._check(self.lib.bshmem_ctx_getmem(self.h, self._ctx(ctx), C.addressof(buf), _ptr_of(src),
-                                               D.size_of(code), pe))
-        return D.from_bits(code, buf[0])
+        word, addr = self._word()
+        st = self._c_g(self._hv, self._ctx(ctx), _ptr_of(src), D.size_of(code), pe, addr)
+        if st:
+            self._check(st)
+        return D.from_bits(code, word.value)
 
     # ---- atomics ---------------------------------------------------------------------
     def _amo(self, op: int, dest: torch.Tensor, value, cond, pe: int, ctx) -> object:
         code = D.code_of(dest.dtype)
-        fetched = C.c_uint64(0)
-        self._check(self.lib.bshmem_ctx_amo(self.h, self._ctx(ctx), code, op, _ptr_of(dest), D.to_bits(code, value),
-                                            D.to_bits(code, cond), pe, C.byref(fetched)))
-        return D.from_bits(code, fetched.value)
+        word, addr = self._word()
+        st = self._c_amo(self._hv, self._ctx(ctx), code, op, _ptr_of(dest), D.to_bits(code, value), D.to_bits(code, cond), pe, addr)
+        if st:
+            self._check(st)
+        return D.from_bits(code, word.value)
 
     def atomic_fetch_add(self, dest, value, pe, ctx=None): return self._amo(D.AMO_FETCH_ADD, dest, value, 0, pe, ctx)
     def atomic_fetch_inc(self, dest, pe, ctx=None): return self._amo(D.AMO_FETCH_INC, dest, 0, 0, pe, ctx)
@@ -326,15 +350,15 @@ class Runtime:
 
     # ---- ordering / sync ------------------------------------------------------------------
     def fence(self, ctx=None) -> None:
-        self._check(self.lib.bshmem_ctx_fence(self.h, self._ctx(ctx)))
+        self._check(self._c_fence(self._hv, self._ctx(ctx)))
 
     def quiet(self, ctx=None) -> None:
-        self._check(self.lib.bshmem_ctx_quiet(self.h, self._ctx(ctx)))
+        self._check(self._c_quiet(self._hv, self._ctx(ctx)))
 
     def wait_until(self, ivar: torch.Tensor, cmp, value) -> None:
         code = D.code_of(ivar.dtype)
         c = D.CMPS[cmp] if isinstance(cmp, str) else int(cmp)
-        self._check(self.lib.bshmem_wait_until(self.h, code, _ptr_of(ivar), c, D.to_bits(code, value)))
+        self._check(self._c_wait_until(self._hv, code, _ptr_of(ivar), c, D.to_bits(code, value)))
 
     def test(self, ivar: torch.Tensor, cmp, value) -> bool:
         code = D.code_of(ivar.dtype)

@@ -21,6 +21,8 @@ _SIZES = {INT8: 1, UINT8: 1, INT16: 2, UINT16: 2, INT32: 4, UINT32: 4, INT64: 8,
 _PACK = {INT8: "b", UINT8: "B", INT16: "h", UINT16: "H", INT32: "i", UINT32: "I", INT64: "q", UINT64: "Q",
          FLOAT: "f", DOUBLE: "d"}
 
+_MASKS = {c: (1 << (8 * n)) - 1 for c, n in _SIZES.items()}
+
 # typestr for __cuda_array_interface__ (bf16 has no numpy code: exported as u2 and re-viewed)
 TYPESTR = {INT8: "|i1", UINT8: "|u1", INT16: "<i2", UINT16: "<u2", INT32: "<i4", UINT32: "<u4", INT64: "<i8",
            UINT64: "<u8", FLOAT: "<f4", DOUBLE: "<f8", BF16: "<u2", FP16: "<f2"}
@@ -39,6 +41,9 @@ SIGNAL_SET, SIGNAL_ADD = 0, 1
 
 
 def code_of(dtype) -> int:
+    code = _TORCH.get(dtype)            # the usual case: a tensor's dtype
+    if code is not None:
+        return code
     if isinstance(dtype, int):
         return dtype
     if isinstance(dtype, torch.dtype):
@@ -52,22 +57,21 @@ def size_of(code: int) -> int:
 
 def to_bits(code: int, value) -> int:
     """Bit pattern of `value` as element type `code`, zero-extended to 64 bits."""
+    if code <= UINT64:
+        return int(value) & _MASKS[code]
     if code == BF16:
         return int(torch.tensor(float(value), dtype=torch.bfloat16).view(torch.int16).item()) & 0xFFFF
     if code == FP16:
         return int(torch.tensor(float(value), dtype=torch.float16).view(torch.int16).item()) & 0xFFFF
-    fmt = _PACK[code]
-    if fmt in "fd":
-        raw = struct.pack("<" + fmt, float(value))
-    else:
-        v = int(value)
-        bits = 8 * _SIZES[code]
-        raw = (v & ((1 << bits) - 1)).to_bytes(_SIZES[code], "little")
-    return int.from_bytes(raw, "little")
+    return int.from_bytes(struct.pack("<" + _PACK[code], float(value)), "little")
 
 
 def from_bits(code: int, bits: int):
     n = _SIZES[code]
+    if code <= UINT64:
+        bits &= _MASKS[code]
+        # codes alternate signed, unsigned; a signed value above the sign bit is negative
+        return bits - (1 << (8 * n)) if not code & 1 and bits >> (8 * n - 1) else bits
     raw = (bits & ((1 << (8 * n)) - 1)).to_bytes(n, "little")
     if code == BF16:
         return float(torch.tensor(int.from_bytes(raw, "little", signed=False), dtype=torch.int32).to(torch.int16)

@@ -31,6 +31,8 @@ def tracing() -> bool:
 def set_tracing(on: bool) -> None:
     global _TRACE
     _TRACE = bool(on)
+    for cls, n, plain, with_range in _instrumented:
+        setattr(cls, n, with_range if _TRACE else plain)
 
 
 @contextlib.contextmanager
@@ -55,7 +57,7 @@ def log(pe: int, msg: str, *args, level: int = logging.DEBUG) -> None:
 
 
 def traced(name: str):
-    """Decorator: wrap a host API method in an NVTX range when tracing is on (a flag test otherwise)."""
+    """Decorator: an NVTX range around a function (a flag test while tracing is off)."""
     def deco(fn):
         def wrapper(*a, **k):
             if not _TRACE:
@@ -67,7 +69,14 @@ def traced(name: str):
     return deco
 
 
+_instrumented: list = []        # (class, method name, plain method, traced method)
+
+
 def instrument(cls, names) -> None:
+    """NVTX ranges around the named methods of `cls` while tracing is on.  The methods are swapped when tracing is
+    switched, so that a call pays nothing while it is off (a wrapper costs 0.2 us, a tenth of a message)."""
     for n in names:
-        if hasattr(cls, n):
-            setattr(cls, n, traced(f"bshmem.{n}")(getattr(cls, n)))
+        fn = cls.__dict__.get(n)
+        if fn is not None:
+            _instrumented.append((cls, n, fn, traced(f"bshmem.{n}")(fn)))
+            setattr(cls, n, _instrumented[-1][3 if _TRACE else 2])
