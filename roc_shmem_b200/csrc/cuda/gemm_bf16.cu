@@ -3,8 +3,12 @@
 // accumulation in TMEM, bf16 output through TMA stores; CTA pairs (cta_group::2) with
 // two accumulator stages, see gemm_pair.cuh.  This is the compute core
 // that the fused all-gather→GEMM and GEMM→reduce-scatter kernels build on; it has
-// no counterpart in the reference, which contains no GEMM.
+// no counterpart in the reference, which contains no GEMM.  Problems with few rows of A
+// take the weight-streaming kernel of gemm_skinny.cuh instead (plan_skinny says when).
+#include <atomic>
+
 #include "gemm_pair.cuh"
+#include "gemm_skinny.cuh"
 #include "tma_host.h"
 
 using namespace bshmem;
@@ -37,8 +41,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) gemm
   gemm_mainloop<PlainBf16>(prm, smem_raw);
 }
 
+__global__ void __launch_bounds__(skinny::NUM_THREADS) gemm_skinny_kernel(const __grid_constant__ skinny::Params prm) {
+  extern __shared__ uint8_t smem_raw[];
+  skinny::body(prm, smem_raw);
+}
+
 int* g_err_dev[64] = {};
 int g_pairs[64] = {};
+int g_sms[64] = {};
 
 int ensure_device_state(int dev) {
   if (g_err_dev[dev]) return 0;
@@ -48,6 +58,98 @@ int ensure_device_state(int dev) {
   BSHMEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
   g_pairs[dev] = max_resident_pairs(gemm_bf16_kernel, sms);
+  g_sms[dev] = sms;
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
+  return 0;
+}
+
+// How many clusters of `split` one-per-SM skinny CTAs the device holds at once (clusters do not span GPCs, so eight CTAs
+// per cluster fill fewer SMs than two).
+int skinny_clusters(int dev, int split) {
+  static std::atomic<int> cache[64][4] = {};
+  std::atomic<int>& slot = cache[dev][split == 1 ? 0 : split == 2 ? 1 : split == 4 ? 2 : 3];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(8 * g_sms[dev]));
+  cfg.blockDim = dim3(skinny::NUM_THREADS);
+  cfg.dynamicSmemBytes = skinny::SMEM_FULL;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_skinny_kernel, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = g_sms[dev] / split; }
+  slot.store(n, std::memory_order_relaxed);
+  return n;
+}
+
+struct SkinnyPlan {
+  int split;       // 0: leave the problem to the 256x256 tiles
+  bool half;
+};
+// Split the reduction as far as all clusters still run at once and every CTA keeps four k-blocks.  Times in us, K x N:
+//  - up to 64 tokens two CTAs per SM: 3584x8192, 16 tokens: split 1 / 2 / 4 / 8 = 17.8 / 14.3 / 13.7 / 18.0 (64 tiles:
+//    256 CTAs at split 4, two waves at 8); 14336x4096: 60.6 / 34.1 / 23.7 / 22.5
+//  - 65 to 128 tokens one CTA per SM with six stages, because a stage grows to 32 KiB (3584x8192, 128 tokens: 15.8
+//    against 17.2 for two CTAs of three stages), unless the tiles alone nearly fill the chip and only half-size CTAs
+//    can split (4096x14336: 25.8 against 27.9)
+//  - above, only while the reduction can be split (3584x8192, 256 tokens: 19.8 against 24.7 for 256x256 tiles; 4096x14336
+//    unsplit: 38.0 against 31.6)
+SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
+  if (M > skinny::MAX_TOKENS) return {0, false};
+  const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS, kb = (K + skinny::BK - 1) / skinny::BK;
+  auto best = [&](bool half) {
+    int s = 1;
+    while (s < 8 && kb >= 8 * s && (half ? tiles * s <= g_sms[dev] : tiles <= skinny_clusters(dev, 2 * s))) s *= 2;
+    return s;
+  };
+  if (M <= 64) return {best(true), true};
+  const int full = best(false);
+  if (full > 1) return {full, false};
+  if (M <= 128) return {best(true), true};
+  return {0, false};
+}
+
+// Few tokens: weight-streaming kernel (gemm_skinny.cuh).
+int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, cudaStream_t st, int dev,
+                  unsigned long long timeout_ns, const SkinnyPlan& plan) {
+  if (reinterpret_cast<uintptr_t>(C) & 15) { host::last_error() = "gemm: the output must be 16-byte aligned"; return 1; }
+  skinny::Params p;
+  p.out = static_cast<__nv_bfloat16*>(C);
+  p.ldo = ldc;
+  p.M = M; p.N = N; p.K = K;
+  p.nt = (M + 15) / 16 * 16;
+  p.timeout_ns = timeout_ns;
+  p.err = g_err_dev[dev];
+  const uint32_t budget = (plan.half ? skinny::SMEM_HALF : skinny::SMEM_FULL) - skinny::CTRL_BYTES - 1024;
+  p.stages = (int)(budget / skinny::stage_bytes(p.nt));
+  if (p.stages > skinny::MAX_STAGES) p.stages = skinny::MAX_STAGES;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < (uint32_t)p.nt) p.tmem_cols *= 2;
+  p.split = plan.split;
+  const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS;
+  int rc = host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, N, K, ldb, skinny::ROWS, skinny::BK);
+  if (rc) return rc;
+  rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, p.nt, skinny::BK);
+  if (rc) return rc;
+  // a split tile is parked over the stages as nt x 512 bytes: at most 128 KiB, over four stages of 48 KiB
+  if (p.stages < 2 || (p.split > 1 && (uint32_t)p.stages * skinny::stage_bytes(p.nt) < (uint32_t)p.nt * skinny::ROWS * 4)) {
+    host::last_error() = "gemm: internal error, the split tile does not fit the stages";
+    return 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * p.split));
+  cfg.blockDim = dim3(skinny::NUM_THREADS);
+  cfg.dynamicSmemBytes = skinny::smem_bytes(p.nt, p.stages);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel, p));
   return 0;
 }
 
@@ -68,12 +170,17 @@ int bshmem_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   BSHMEM_CUDA_TRY(cudaGetDevice(&dev));
   int rc = ensure_device_state(dev);
   if (rc) return rc;
+  const unsigned long long timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
+  if (max_ctas <= 1) {                          // an explicit limit on the CTAs keeps the persistent kernel
+    const SkinnyPlan plan = plan_skinny(M, N, K, dev);
+    if (plan.split) return launch_skinny(A, B, C, M, N, K, lda, ldb, ldc, static_cast<cudaStream_t>(stream), dev, timeout_ns, plan);
+  }
   PlainParams p;
   p.core.M = M; p.core.N = N; p.core.K = K;
   p.core.num_m_blocks = (M + BM - 1) / BM;
   p.core.num_n_blocks = (N + BN - 1) / BN;
   p.core.group_m = 8;
-  p.core.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
+  p.core.timeout_ns = timeout_ns;
   p.core.err = g_err_dev[dev];
   rc = host::make_tmap_2d(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, CTA_M, 64);
   if (rc) return rc;

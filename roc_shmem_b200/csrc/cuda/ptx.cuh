@@ -100,6 +100,13 @@ template <int N> __device__ __forceinline__ void tma_wait_group() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// ---- programmatic dependent launch --------------------------------------------------
+// A kernel launched with the programmatic-serialization attribute may start while its predecessor on the stream is
+// still running; it waits here before it touches anything the predecessor may have written (or may still read).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// From here on (once every block has said so, or left) the successor's blocks may be scheduled.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- tcgen05: tensor memory + 5th-gen tensor core MMA ------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t ncols) {   // whole warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(ncols) : "memory");

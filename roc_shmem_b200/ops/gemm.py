@@ -14,10 +14,18 @@ import torch
 from .. import _native
 
 _declared = False
+_run = None                                            # bshmem_gemm_bf16 without ctypes (see _native.fast)
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_BF16 = torch.bfloat16
+
+
+def current_stream() -> int:
+    """Handle of the current CUDA stream of the current device (torch.cuda.current_stream() builds an object)."""
+    return _raw_stream(torch._C._cuda_getDevice())
 
 
 def gemm_lib() -> C.CDLL:
-    global _declared
+    global _declared, _run
     lib = _native.load("libbshmem_gemm.so")
     if not _declared:
         lib.bshmem_gemm_last_error.restype = C.c_char_p
@@ -26,6 +34,7 @@ def gemm_lib() -> C.CDLL:
                                          C.c_int, C.c_void_p, C.c_int, C.c_int]
         lib.bshmem_gemm_error_site.restype = C.c_int
         lib.bshmem_gemm_error_site.argtypes = [C.c_int]
+        _run = _native.fast(lib, "bshmem_gemm_bf16")
         _declared = True
     return lib
 
@@ -38,23 +47,30 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     missing — there is no eager fallback."""
     if not (a.is_cuda and b.is_cuda):
         raise ValueError("gemm_bf16 needs CUDA tensors")
-    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
+    if a.dtype is not _BF16 or b.dtype is not _BF16:
         raise ValueError("gemm_bf16 needs bf16 operands")
-    if a.dim() != 2 or b.dim() != 2 or a.shape[1] != b.shape[1]:
-        raise ValueError(f"shape mismatch: a {tuple(a.shape)} b {tuple(b.shape)}")
-    if a.stride(1) != 1 or b.stride(1) != 1:
+    sa, sb = a.shape, b.shape
+    if len(sa) != 2 or len(sb) != 2 or sa[1] != sb[1]:
+        raise ValueError(f"shape mismatch: a {tuple(sa)} b {tuple(sb)}")
+    lda, ka = a.stride()
+    ldb, kb = b.stride()
+    if ka != 1 or kb != 1:
         raise ValueError("operands must be K-major (last dimension contiguous)")
-    M, K = a.shape
-    N = b.shape[0]
+    M, K = sa
+    N = sb[0]
     if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    elif out.shape != (M, N) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
-        raise ValueError("bad output tensor")
-    lib = gemm_lib()
-    st = lib.bshmem_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-                              out.stride(0), torch.cuda.current_stream().cuda_stream, max_ctas, timeout_ms)
+        out = torch.empty((M, N), dtype=_BF16, device=a.device)
+        ldc = N
+    else:
+        if out.shape != (M, N) or out.dtype is not _BF16 or out.stride(1) != 1:
+            raise ValueError("bad output tensor")
+        ldc = out.stride(0)
+    if _run is None:
+        gemm_lib()
+    st = _run(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, _raw_stream(torch._C._cuda_getDevice()), max_ctas,
+              timeout_ms)
     if st != 0:
-        raise RuntimeError(f"bshmem_gemm_bf16 failed ({st}): {lib.bshmem_gemm_last_error().decode()}")
+        raise RuntimeError(f"bshmem_gemm_bf16 failed ({st}): {gemm_lib().bshmem_gemm_last_error().decode()}")
     return out
 
 
