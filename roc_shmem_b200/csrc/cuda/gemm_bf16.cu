@@ -19,10 +19,38 @@ namespace {
 struct PlainParams {
   CoreParams core;
   CUtensorMap map_a, map_b, map_c;
+  __nv_bfloat16* out;          // split form: the result, written directly
+  long long ldc;
 };
 
+// One policy per operand layout.  K-major (kAmn / kBmn false): A is stored [M][K], one 128-row x 64 box per CTA and stage.
+// MN-major (true): A is stored [K][M], as a gradient GEMM finds it; a stage holds two 64-wide column blocks of 64 reduction
+// rows (8 KiB each, 128-byte swizzle), which the tensor core reads through MN-major descriptors — no transposed copy.
+// Rows and columns beyond the matrix, the reduction included, are zero-filled by TMA.
+template <bool kAmn, bool kBmn, bool kSplitK>
 struct PlainBf16 : PolicyDefaults {
   using Params = PlainParams;
+  static constexpr bool kSplit = kSplitK;
+  static constexpr uint32_t kIdesc = kIdescBf16 | (kAmn ? 1u << 15 : 0u) | (kBmn ? 1u << 16 : 0u);
+  static constexpr uint32_t kBlock = 64 * BK_BYTES;           // one 64 (MN) x 64 (K) block
+  static constexpr uint32_t kKStepA = kAmn ? 2048 : UMMA_K_BYTES, kKStepB = kBmn ? 2048 : UMMA_K_BYTES;
+  __device__ static __forceinline__ uint64_t desc_a0(uint32_t a0) { return kAmn ? ptx::umma_desc_sw128_ex(a0, kBlock, 1024) : ptx::umma_desc_sw128(a0); }
+  __device__ static __forceinline__ uint64_t desc_b0(uint32_t b0) { return kBmn ? ptx::umma_desc_sw128_ex(b0, kBlock, 1024) : ptx::umma_desc_sw128(b0); }
+  __device__ static __forceinline__ void load_stage(const Params&, const CUtensorMap* ma, const CUtensorMap* mb, uint32_t a_smem,
+                                                    uint32_t b_smem, uint32_t bar, int kb, int a_row, int b_row, int, int, int) {
+    if constexpr (kAmn) {
+      ptx::tma_load_2d(a_smem, ma, bar, a_row, kb * BK);
+      ptx::tma_load_2d(a_smem + kBlock, ma, bar, a_row + 64, kb * BK);
+    } else {
+      ptx::tma_load_2d(a_smem, ma, bar, kb * BK, a_row);
+    }
+    if constexpr (kBmn) {
+      ptx::tma_load_2d(b_smem, mb, bar, b_row, kb * BK);
+      ptx::tma_load_2d(b_smem + kBlock, mb, bar, b_row + 64, kb * BK);
+    } else {
+      ptx::tma_load_2d(b_smem, mb, bar, kb * BK, b_row);
+    }
+  }
   __device__ static __forceinline__ const CoreParams& core(const Params& p) { return p.core; }
   __device__ static __forceinline__ const CUtensorMap* map_a(const Params& p) { return &p.map_a; }
   __device__ static __forceinline__ const CUtensorMap* map_b(const Params& p) { return &p.map_b; }
@@ -34,21 +62,44 @@ struct PlainBf16 : PolicyDefaults {
     *x = col;
     *y = row;
   }
+  // 16 columns of a row: one 32-byte sector (N is a multiple of 8)
+  __device__ static __forceinline__ void store_row16(const Params& p, int row, int col, const float4 (&v)[4]) {
+    if (row >= p.core.M) return;
+    uint4* dst = reinterpret_cast<uint4*>(p.out + row * p.ldc + col);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (col + 8 * h < p.core.N)
+        dst[h] = make_uint4(pack_bf16(v[2 * h].x, v[2 * h].y), pack_bf16(v[2 * h].z, v[2 * h].w), pack_bf16(v[2 * h + 1].x, v[2 * h + 1].y),
+                            pack_bf16(v[2 * h + 1].z, v[2 * h + 1].w));
+  }
 };
 
+template <bool kAmn, bool kBmn>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) gemm_bf16_kernel(const __grid_constant__ PlainParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_mainloop<PlainBf16>(prm, smem_raw);
+  gemm_mainloop<PlainBf16<kAmn, kBmn, false>>(prm, smem_raw);
 }
+template <bool kAmn, bool kBmn>                       // cluster size at launch: 2 * split
+__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_bf16_split_kernel(const __grid_constant__ PlainParams prm) {
+  extern __shared__ uint8_t smem_raw[];
+  gemm_mainloop<PlainBf16<kAmn, kBmn, true>>(prm, smem_raw);
+}
+using PlainKernel = void (*)(PlainParams);
+constexpr PlainKernel kPlainKernels[2][2] = {{gemm_bf16_kernel<false, false>, gemm_bf16_kernel<false, true>},
+                                             {gemm_bf16_kernel<true, false>, gemm_bf16_kernel<true, true>}};
+constexpr PlainKernel kSplitKernels[2][2] = {{gemm_bf16_split_kernel<false, false>, gemm_bf16_split_kernel<false, true>},
+                                             {gemm_bf16_split_kernel<true, false>, gemm_bf16_split_kernel<true, true>}};
 
+template <bool kWmn>
 __global__ void __launch_bounds__(skinny::NUM_THREADS) gemm_skinny_kernel(const __grid_constant__ skinny::Params prm) {
   extern __shared__ uint8_t smem_raw[];
-  skinny::body(prm, smem_raw);
+  skinny::body<kWmn>(prm, smem_raw);
 }
 
 int* g_err_dev[64] = {};
 int g_pairs[64] = {};
 int g_sms[64] = {};
+int g_quads[64] = {}, g_octs[64] = {};       // clusters of two / four CTA pairs the device holds at once
 
 int ensure_device_state(int dev) {
   if (g_err_dev[dev]) return 0;
@@ -56,10 +107,16 @@ int ensure_device_state(int dev) {
   BSHMEM_CUDA_TRY(cudaMalloc(&g_err_dev[dev], sizeof(int)));
   BSHMEM_CUDA_TRY(cudaMemset(g_err_dev[dev], 0, sizeof(int)));
   BSHMEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-  g_pairs[dev] = max_resident_pairs(gemm_bf16_kernel, sms);
+  for (auto& row : kPlainKernels)
+    for (PlainKernel k : row) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+  for (auto& row : kSplitKernels)
+    for (PlainKernel k : row) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+  g_pairs[dev] = max_resident_pairs(kPlainKernels[0][0], sms);
+  g_quads[dev] = max_resident_clusters(kSplitKernels[0][0], sms, 4);
+  g_octs[dev] = max_resident_clusters(kSplitKernels[0][0], sms, 8);
   g_sms[dev] = sms;
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_skinny_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_skinny_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
   return 0;
 }
 
@@ -78,7 +135,7 @@ int skinny_clusters(int dev, int split) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_skinny_kernel, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = g_sms[dev] / split; }
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_skinny_kernel<false>, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = g_sms[dev] / split; }
   slot.store(n, std::memory_order_relaxed);
   return n;
 }
@@ -111,8 +168,8 @@ SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
 }
 
 // Few tokens: weight-streaming kernel (gemm_skinny.cuh).
-int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, cudaStream_t st, int dev,
-                  unsigned long long timeout_ns, const SkinnyPlan& plan) {
+int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, bool w_mn, cudaStream_t st,
+                  int dev, unsigned long long timeout_ns, const SkinnyPlan& plan) {
   if (reinterpret_cast<uintptr_t>(C) & 15) { host::last_error() = "gemm: the output must be 16-byte aligned"; return 1; }
   skinny::Params p;
   p.out = static_cast<__nv_bfloat16*>(C);
@@ -128,7 +185,8 @@ int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, in
   while (p.tmem_cols < (uint32_t)p.nt) p.tmem_cols *= 2;
   p.split = plan.split;
   const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS;
-  int rc = host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, N, K, ldb, skinny::ROWS, skinny::BK);
+  int rc = w_mn ? host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, K, N, ldb, skinny::BK, 64)
+                : host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, N, K, ldb, skinny::ROWS, skinny::BK);
   if (rc) return rc;
   rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, p.nt, skinny::BK);
   if (rc) return rc;
@@ -149,7 +207,7 @@ int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, in
   attr[1].val.clusterDim.x = (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.split > 1 ? 2 : 1;
-  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel, p));
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, w_mn ? gemm_skinny_kernel<true> : gemm_skinny_kernel<false>, p));
   return 0;
 }
 
@@ -159,21 +217,27 @@ extern "C" {
 
 const char* bshmem_gemm_last_error() { return host::last_error().c_str(); }
 
-// C = A · B^T.  A: [M, K] row-major (lda elements), B: [N, K] row-major (ldb), C: [M, N] (ldc), all bf16.
-// K, lda, ldb, ldc must be multiples of 8 and the bases 16-byte aligned (TMA).
-// The kernel runs as CTA pairs (clusters of two); max_ctas <= 1 uses every pair the device can hold.  timeout_ms bounds every in-kernel wait.
-int bshmem_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                     void* stream, int max_ctas, int timeout_ms) {
+// C = op(A) · op(B)^T with a reduction of K.  a_mn = 0: A is [M, K] row-major (lda elements); a_mn = 1: A is [K, M] (the
+// reduction runs over its rows).  Likewise B: [N, K] or, with b_mn, [K, N].  C: [M, N] (ldc).  All bf16.
+// lda, ldb, ldc, and K (M, N) where it is the contiguous extent of an operand, must be multiples of 8 and the bases
+// 16-byte aligned (TMA).  The kernel runs as CTA pairs (clusters of two); max_ctas <= 1 uses every pair the device can
+// hold.  timeout_ms bounds every in-kernel wait.
+int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
+                        void* stream, int max_ctas, int timeout_ms) {
   if (M <= 0 || N <= 0 || K <= 0) { host::last_error() = "gemm: empty problem"; return 1; }
-  if ((K % 8) || (lda % 8) || (ldb % 8) || (ldc % 8)) { host::last_error() = "gemm: K and leading dimensions must be multiples of 8"; return 1; }
+  if ((!(a_mn && b_mn) && K % 8) || (a_mn && M % 8) || (b_mn && N % 8) || (lda % 8) || (ldb % 8) || (ldc % 8)) {
+    host::last_error() = "gemm: K and leading dimensions must be multiples of 8";
+    return 1;
+  }
   int dev = 0;
   BSHMEM_CUDA_TRY(cudaGetDevice(&dev));
   int rc = ensure_device_state(dev);
   if (rc) return rc;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned long long timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
-  if (max_ctas <= 1) {                          // an explicit limit on the CTAs keeps the persistent kernel
+  if (max_ctas <= 1 && !a_mn) {        // an explicit limit on the CTAs keeps the persistent kernel
     const SkinnyPlan plan = plan_skinny(M, N, K, dev);
-    if (plan.split) return launch_skinny(A, B, C, M, N, K, lda, ldb, ldc, static_cast<cudaStream_t>(stream), dev, timeout_ns, plan);
+    if (plan.split) return launch_skinny(A, B, C, M, N, K, lda, ldb, ldc, b_mn != 0, st, dev, timeout_ns, plan);
   }
   PlainParams p;
   p.core.M = M; p.core.N = N; p.core.K = K;
@@ -182,20 +246,47 @@ int bshmem_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
   p.core.group_m = 8;
   p.core.timeout_ns = timeout_ns;
   p.core.err = g_err_dev[dev];
-  rc = host::make_tmap_2d(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, CTA_M, 64);
+  const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  rc = a_mn ? host::make_tmap_2d(&p.map_a, bf, 2, A, K, M, lda, 64, 64) : host::make_tmap_2d(&p.map_a, bf, 2, A, M, K, lda, CTA_M, 64);
   if (rc) return rc;
-  rc = host::make_tmap_2d(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, N, K, ldb, CTA_NLOAD, 64);
+  rc = b_mn ? host::make_tmap_2d(&p.map_b, bf, 2, B, K, N, ldb, 64, 64) : host::make_tmap_2d(&p.map_b, bf, 2, B, N, K, ldb, CTA_NLOAD, 64);
   if (rc) return rc;
-  rc = host::make_tmap_2d(&p.map_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, C, M, N, ldc, 32, EPI_COLS);
+  rc = host::make_tmap_2d(&p.map_c, bf, 2, C, M, N, ldc, 32, EPI_COLS);
   if (rc) return rc;
-  int tiles = p.core.num_m_blocks * p.core.num_n_blocks;
+  const int tiles = p.core.num_m_blocks * p.core.num_n_blocks;
   int pairs = g_pairs[dev];
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  p.out = static_cast<__nv_bfloat16*>(C);
+  p.ldc = ldc;
+  // Few tiles: split each over the two or four pairs of a cluster while all clusters run at once.  Parking and adding the
+  // parts costs about 4 us, what a pair needs for 14 k-blocks.
+  const int kb = (K + BK - 1) / BK;
+  p.core.split = 1;
+  if (max_ctas <= 1) {
+    if (tiles <= g_octs[dev] && kb >= 24) p.core.split = 4;
+    else if (tiles <= g_quads[dev] && kb >= 32) p.core.split = 2;
+  }
   if (tiles < pairs) pairs = tiles;
-  const int ctas = 2 * pairs;
-  gemm_bf16_kernel<<<ctas, NUM_THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
-  BSHMEM_CUDA_TRY(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pairs * p.core.split));
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)(2 * p.core.split); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.core.split > 1 ? 2 : 1;
+  const auto& kernels = p.core.split > 1 ? kSplitKernels : kPlainKernels;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernels[a_mn ? 1 : 0][b_mn ? 1 : 0], p));
   return 0;
+}
+
+int bshmem_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                     void* stream, int max_ctas, int timeout_ms) {
+  return bshmem_gemm_bf16_ex(A, B, C, M, N, K, lda, ldb, ldc, 0, 0, stream, max_ctas, timeout_ms);
 }
 
 // Reads (and clears) the device error word of the current device: 0 = no bounded wait ran out.

@@ -56,6 +56,7 @@ struct CoreParams {
   int group_m;             // m-blocks per raster group (L2 reuse)
   unsigned long long timeout_ns;
   int* err;                // device word: first error site, 0 = none
+  int split;               // CTA-pair core, split form: pairs per tile
 };
 
 struct Guard {

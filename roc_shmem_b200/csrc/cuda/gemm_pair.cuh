@@ -23,6 +23,12 @@
 //
 // tcgen05.commit (with its cluster-multicast form, a barrier arrival, not a load) hands
 // stages and accumulators back to BOTH CTAs.
+// Split form (policy with kSplit, for problems with fewer than about half as many tiles as the chip has pairs): the
+// cluster is S = 2 or 4 pairs that share one tile.  Each pair sums its share of K; then every CTA parks its fp32
+// accumulator (128 x 256, 128 KiB) over its drained ring, and after one cluster barrier CTA (pair j, half r) adds the S
+// parked halves r over columns [256 j / S, 256 (j + 1) / S) in pair order and writes them: a reduce-scatter through
+// distributed shared memory, without workspace or atomics.
+//
 // Every wait is bounded by a %globaltimer deadline; on expiry the CTA records a site
 // code in the error word and all roles leave their loops; both CTAs always reach the
 // closing cluster barrier before TMEM is released.  Every load is a plain tiled TMA
@@ -86,6 +92,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // announces is shared-memory or tensor-memory traffic of the async proxies (TMA, tcgen05), not generic-proxy
 // stores, and a cluster-scope acquire on every poll made the MMA issuer the bottleneck (2.5x slower).
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) { return ptx::mbar_try_wait(bar, parity); }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  // volatile keeps it behind the cluster barrier; without a memory clobber a run of them stays together
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -108,26 +120,27 @@ __device__ __forceinline__ void umma2_f16(uint32_t d_tmem, uint64_t a_desc, uint
 }
 // One commit that arrives on the barrier at this offset in BOTH CTAs of the pair (two single-destination commits
 // per k-block cost the issuing thread 6 % of the GEMM's throughput).
-__device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
+__device__ __forceinline__ void umma2_commit_both(uint32_t bar, uint32_t lead) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((uint16_t)3) : "memory");
+               ::"r"(bar), "h"((uint16_t)(3u << lead)) : "memory");
 }
 
-// Host side: how many CTA pairs of `kernel` the device can hold at once (at most one per two SMs).
+// Host side: how many clusters of `size` CTAs of `kernel` the device can hold at once (one CTA per SM).
 template <class Kernel>
-inline int max_resident_pairs(Kernel kernel, int sms) {
+inline int max_resident_clusters(Kernel kernel, int sms, int size) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(sms & ~1), 1, 1);
+  cfg.gridDim = dim3((unsigned)(sms / size * size), 1, 1);
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.x = (unsigned)size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = sms / 2; }
-  return n < sms / 2 ? n : sms / 2;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = sms / size; }
+  return n < sms / size ? n : sms / size;
 }
+template <class Kernel> inline int max_resident_pairs(Kernel kernel, int sms) { return max_resident_clusters(kernel, sms, 2); }
 
 __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, Guard& g, int site) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
@@ -188,6 +201,8 @@ struct Chunk {
 
 struct PolicyDefaults {
   struct EpiState {};
+  // Split form: clusters of 2 * CoreParams::split CTAs, one tile each, output written by store_rows instead of TMA.
+  static constexpr bool kSplit = false;
   // Gated epilogue: inside every 64-column chunk of the accumulator, columns 0-31 are gate pre-activations and 32-63
   // the matching up-projections; the epilogue writes silu(gate) * up, i.e. half as many output columns (the two
   // chunks of a warp make one 32 x 64 output box; out_target gets the OUTPUT column).
@@ -196,7 +211,7 @@ struct PolicyDefaults {
   // shared-memory descriptors that step 32 bytes along K inside the swizzle atom.  A policy with MN-major operands
   // overrides the instruction descriptor, the stage-0 descriptors, the step per MMA and the loads.
   static constexpr uint32_t kIdesc = kIdescBf16;
-  static constexpr uint32_t kKStepBytes = UMMA_K_BYTES;
+  static constexpr uint32_t kKStepA = UMMA_K_BYTES, kKStepB = UMMA_K_BYTES;
   __device__ static __forceinline__ uint64_t desc_a0(uint32_t a0) { return ptx::umma_desc_sw128(a0); }
   __device__ static __forceinline__ uint64_t desc_b0(uint32_t b0) { return ptx::umma_desc_sw128(b0); }
   // a_row / b_row: first row this CTA loads (its rank's half included); kb: k-block of the tile
@@ -229,6 +244,39 @@ struct PolicyDefaults {
   template <class Params> __device__ static __forceinline__ void prologue(const Params&, Guard&) {}
 };
 
+// 64 accumulator columns of this warp's 32 rows (row = lane).
+__device__ __forceinline__ void load_acc_chunk(uint32_t taddr, float (&f)[64]) {
+  uint32_t v[2][32];
+  ptx::tmem_ld_32x32b_x32(taddr, v[0]);
+  ptx::tmem_ld_32x32b_x32(taddr + 32, v[1]);
+  ptx::tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < 64; ++i) f[i] = __uint_as_float(v[i >> 5][i & 31]);
+}
+
+// Split form, behind the cluster barrier: this CTA's share of the sum, 16 columns of a row per thread and step.
+template <class P, int S>
+__device__ __forceinline__ void split_reduce(const typename P::Params& prm, const Smem& L, uint32_t crank, int m_blk, int n_blk) {
+  constexpr int kGroups = BN / S / 16;                       // 16-column groups of the share
+  const int half = crank & 1, j0 = crank >> 1;
+  uint32_t src[S];
+#pragma unroll
+  for (int q = 0; q < S; ++q) src[q] = mapa(L.base, 2 * q + half);
+  for (int i = threadIdx.x; i < kGroups * CTA_M; i += NUM_THREADS) {
+    const int row = i & (CTA_M - 1), col = j0 * (BN / S) + (i / CTA_M) * 16;
+    float4 v[S][4];
+#pragma unroll
+    for (int q = 0; q < S; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[q][e] = ld_cluster_f4(src[q] + ((col / 4 + e) * CTA_M + row) * 16);
+#pragma unroll
+    for (int q = 1; q < S; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { v[0][e].x += v[q][e].x; v[0][e].y += v[q][e].y; v[0][e].z += v[q][e].z; v[0][e].w += v[q][e].w; }
+    P::store_row16(prm, m_blk * BM + half * CTA_M + row, n_blk * BN + col, v[0]);
+  }
+}
+
 // Policy contract (static __device__ members; P::Params is the kernel's by-value parameter):
 //   core(prm) -> const CoreParams&        map_a(prm), map_b(prm) -> const CUtensorMap*
 //   tile_coords(prm, tile, &m_blk, &n_blk)     tile = index in the pair's schedule (pair id + k * pairs)
@@ -242,9 +290,17 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   const Smem L = carve_smem(smem_raw);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();            // 0 issues the MMAs
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_ctarank();
+  const uint32_t rank = crank & 1, lead = crank & ~1u;   // the pair's first CTA issues the MMAs
+  const int S = P::kSplit ? cp.split : 1;
+  const int pair = blockIdx.x / (2 * S), num_pairs = gridDim.x / (2 * S);    // split form: index and number of tiles
   const int num_tiles = P::num_tiles(prm);
+  // k-blocks of a tile that this pair multiplies
+  auto kb_range = [&](int m_blk, int* kb0, int* kb1) {
+    const int n = P::num_kb(prm, m_blk), j = P::kSplit ? (int)(crank >> 1) : 0;
+    *kb0 = P::kSplit ? n * j / S : 0;
+    *kb1 = P::kSplit ? n * (j + 1) / S : n;
+  };
   Guard g{cp.err, L.abort_flag(), cp.timeout_ns};
 
   if (threadIdx.x == 0) {
@@ -274,6 +330,9 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   ptx::tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(L.tmem_slot()));
+  // launched with programmatic serialization, the set-up above overlaps the previous kernel; without, this is a no-op
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   if (threadIdx.x == 64) P::prologue(prm, g);
 
   if (warp == 0) {
@@ -282,13 +341,13 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       int s = 0; uint32_t ph = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int m_blk, n_blk;
+        int m_blk, n_blk, kb0, kb1;
         P::tile_coords(prm, tile, &m_blk, &n_blk);
         if (!P::a_ready(prm, m_blk, g)) break;
-        const int num_kb = P::num_kb(prm, m_blk);
+        kb_range(m_blk, &kb0, &kb1);
         const int a_row = P::a_row(prm, m_blk) + (int)rank * CTA_M;
         const int b_row = P::b_row(prm, m_blk, n_blk) + (int)rank * CTA_NLOAD;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!pair_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(L.full(s), STAGE_BYTES);
           P::load_stage(prm, P::map_a(prm), P::map_b(prm), L.a(s), L.b(s), L.full(s), kb, a_row, b_row, m_blk, n_blk, (int)rank);
@@ -301,20 +360,20 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       // ------------------------------ MMA issuer (first CTA) ---------------------------------
       int s = 0; uint32_t ph = 0;
       uint32_t acc_ph = 0;          // bit a = phase of accumulator a
-      int ord = 0;
       bool ok = true;
       const uint64_t desc_a0 = P::desc_a0(L.a(0)), desc_b0 = P::desc_b0(L.b(0));
+      int ord = 0;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++ord) {
         const int acc = ord & 1;
-        int m_blk, n_blk;
+        int m_blk, n_blk, kb0, kb1;
         P::tile_coords(prm, tile, &m_blk, &n_blk);
-        const int num_kb = P::num_kb(prm, m_blk);
+        kb_range(m_blk, &kb0, &kb1);
         // the epilogue warps of both CTAs must have drained this accumulator (two tiles ago)
         if (!pair_wait(L.tmem_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_MMA_TMEM_EMPTY)) break;
         acc_ph ^= 1u << acc;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!pair_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
           ptx::tc_fence_after();
           // descriptors differ only in the 16-byte-unit start address (low 14 bits; shared memory is < 256 KiB)
@@ -322,13 +381,13 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           const uint64_t db = desc_b0 + (uint64_t)((s * STAGE_BYTES) >> 4);
 #pragma unroll
           for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k)
-            umma2_f16(d_tmem, da + (uint64_t)((k * P::kKStepBytes) >> 4), db + (uint64_t)((k * P::kKStepBytes) >> 4), P::kIdesc,
-                      (kb | k) != 0 ? 1u : 0u);
-          umma2_commit_both(L.empty(s));       // stage reusable in both CTAs once these MMAs retire
+            umma2_f16(d_tmem, da + (uint64_t)((k * P::kKStepA) >> 4), db + (uint64_t)((k * P::kKStepB) >> 4), P::kIdesc,
+                      (kb > kb0 || k != 0) ? 1u : 0u);
+          umma2_commit_both(L.empty(s), lead);       // stage reusable in both CTAs once these MMAs retire
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        umma2_commit_both(L.tmem_full(acc));
+        umma2_commit_both(L.tmem_full(acc), lead);
       }
     }
     else if (lane == 0) {
@@ -336,12 +395,12 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       int s = 0; uint32_t ph = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int m_blk, n_blk;
+        int m_blk, n_blk, kb0, kb1;
         P::tile_coords(prm, tile, &m_blk, &n_blk);
-        const int num_kb = P::num_kb(prm, m_blk);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        kb_range(m_blk, &kb0, &kb1);
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!pair_wait(L.full(s), ph, g, ERR_RELAY_FULL)) { ok = false; break; }
-          mbar_arrive_cluster(mapa(L.full(s), 0));
+          mbar_arrive_cluster(mapa(L.full(s), lead));
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
@@ -373,24 +432,35 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       if (!ok) break;
       full_ph ^= 1u << acc;
       ptx::tc_fence_after();
+      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * ACC_COLS + colhalf * 128;
+      auto acc_done = [&]() {
+        // all TMEM reads of this warp are done: hand the accumulator back to the MMA issuer
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa(L.tmem_empty(acc), lead));
+      };
+      if constexpr (P::kSplit) {
+        // [float4 of the row][row]: the lanes' stores and the reading side's loads are consecutive
+        const uint32_t dst = L.base + (colhalf * 32 * CTA_M + quarter * 32 + lane) * 16;
+#pragma unroll 1
+        for (int c = 0; c < 128; c += 32) {
+          uint32_t v[32];
+          ptx::tmem_ld_32x32b_x32(tacc + c, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (c / 4 + j) * CTA_M * 16), "r"(v[4 * j]), "r"(v[4 * j + 1]),
+                         "r"(v[4 * j + 2]), "r"(v[4 * j + 3]) : "memory");
+        }
+        break;                             // one tile per cluster; the rest happens behind the cluster barrier
+      }
       if (!P::tile_begin(prm, L, st, ck, ew, lane, g)) { ok = false; break; }
       if constexpr (!P::kGated) {
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
-          uint32_t v[2][32];
-          uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * ACC_COLS + colhalf * 128 + c * EPI_COLS;
-          ptx::tmem_ld_32x32b_x32(taddr, v[0]);
-          ptx::tmem_ld_32x32b_x32(taddr + 32, v[1]);
-          ptx::tmem_ld_wait();
-          if (c == 1) {
-            // all TMEM reads of this warp are done: hand the accumulator back to the MMA issuer
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa(L.tmem_empty(acc), 0));
-          }
           float f[64];
-#pragma unroll
-          for (int i = 0; i < 64; ++i) f[i] = __uint_as_float(v[i >> 5][i & 31]);
+          load_acc_chunk(tacc + c * EPI_COLS, f);
+          if (c == 1) acc_done();
           // the previous chunk's TMA store must have finished reading the staging buffer
           if (lane == 0) ptx::tma_wait_group_read<0>();
           __syncwarp();
@@ -424,23 +494,16 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
         const uint32_t rowbase = L.epi(ew) + lane * 128;
 #pragma unroll
         for (int hc = 0; hc < 2; ++hc) {
-          uint32_t v[2][32];
-          uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * ACC_COLS + colhalf * 128 + hc * EPI_COLS;
-          ptx::tmem_ld_32x32b_x32(taddr, v[0]);        // gate
-          ptx::tmem_ld_32x32b_x32(taddr + 32, v[1]);   // up
-          ptx::tmem_ld_wait();
-          if (hc == 1) {
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa(L.tmem_empty(acc), 0));
-          }
+          float f[64];                     // 32 gate pre-activations, then the 32 matching up-projections
+          load_acc_chunk(tacc + hc * EPI_COLS, f);
+          if (hc == 1) acc_done();
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             uint32_t w[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              float g0 = __uint_as_float(v[0][j * 8 + 2 * q]), g1 = __uint_as_float(v[0][j * 8 + 2 * q + 1]);
-              float u0 = __uint_as_float(v[1][j * 8 + 2 * q]), u1 = __uint_as_float(v[1][j * 8 + 2 * q + 1]);
+              float g0 = f[j * 8 + 2 * q], g1 = f[j * 8 + 2 * q + 1];
+              float u0 = f[32 + j * 8 + 2 * q], u1 = f[32 + j * 8 + 2 * q + 1];
               float h0 = g0 / (1.f + __expf(-g0)) * u0, h1 = g1 / (1.f + __expf(-g1)) * u1;
               w[q] = pack_bf16(h0, h1);
             }
@@ -467,6 +530,15 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   // ------------------------------ tail + teardown ---------------------------------------
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (P::kSplit) {
+    cluster_sync_all();                               // every part of the tile is parked
+    int m_blk, n_blk;
+    P::tile_coords(prm, pair, &m_blk, &n_blk);
+    if (!*L.abort_flag()) {
+      if (S == 2) split_reduce<P, 2>(prm, L, crank, m_blk, n_blk);
+      else split_reduce<P, 4>(prm, L, crank, m_blk, n_blk);
+    }
+  }
   if (!*L.abort_flag()) P::tail(prm, L, g);
   __syncthreads();
   if (*L.abort_flag()) {

@@ -41,7 +41,7 @@ constexpr uint32_t SMEM_HALF = 112u << 10, SMEM_FULL = 227u << 10;
 enum ErrSite : int { ERR_PRODUCER_EMPTY = 301, ERR_MMA_FULL = 302, ERR_EPI_FULL = 303 };
 
 struct Params {
-  CUtensorMap map_w, map_x;      // weights [N, K], tokens [M, K]: boxes {64, 128} and {64, nt}
+  CUtensorMap map_w, map_x;      // weights [N, K] or [K, N], tokens [M, K]: boxes {64, 128} or {64, 64}, and {64, nt}
   __nv_bfloat16* out;            // [M, N]
   long long ldo;
   int M, N, K;
@@ -66,6 +66,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
+  // volatile keeps it behind the cluster barrier; without a memory clobber a run of them stays together
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
@@ -122,6 +123,9 @@ __device__ __forceinline__ void add_partials(const Params& p, uint32_t base, int
 }
 
 // One tile per cluster of p.split CTAs: grid = tiles * split.
+// kWmn: the weights are stored [K][N] (the data gradient's operand): a stage is two 64-wide column blocks of 64 reduction
+// rows, read through an MN-major descriptor.
+template <bool kWmn>
 __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
   Smem L;
   {
@@ -167,7 +171,12 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) break;
         ptx::mbar_arrive_expect_tx(L.full(s), L.stage);
-        ptx::tma_load_2d(L.w(s), &p.map_w, L.full(s), kb * BK, n0);
+        if constexpr (kWmn) {
+          ptx::tma_load_2d(L.w(s), &p.map_w, L.full(s), n0, kb * BK);
+          ptx::tma_load_2d(L.w(s) + W_STAGE_BYTES / 2, &p.map_w, L.full(s), n0 + 64, kb * BK);
+        } else {
+          ptx::tma_load_2d(L.w(s), &p.map_w, L.full(s), kb * BK, n0);
+        }
         ptx::tma_load_2d(L.x(s), &p.map_x, L.full(s), kb * BK, 0);
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
@@ -175,13 +184,14 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
   } else if (warp == 1) {
     if (lane == 0) {
       int s = 0; uint32_t ph = 0;
-      const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)p.nt);
+      const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)p.nt) | (kWmn ? 1u << 15 : 0u);
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
         ptx::tc_fence_after();
-        const uint64_t dw = ptx::umma_desc_sw128(L.w(s)), dx = ptx::umma_desc_sw128(L.x(s));
+        const uint64_t dw = kWmn ? ptx::umma_desc_sw128_ex(L.w(s), W_STAGE_BYTES / 2, 1024) : ptx::umma_desc_sw128(L.w(s));
+        const uint64_t dx = ptx::umma_desc_sw128(L.x(s));
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(tmem, dw + 2 * k, dx + 2 * k, idesc, (kb > kb0 || k) ? 1u : 0u);
+        for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(tmem, dw + (kWmn ? 128 : 2) * k, dx + 2 * k, idesc, (kb > kb0 || k) ? 1u : 0u);
         ptx::umma_commit(L.empty(s));
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }

@@ -188,7 +188,7 @@ struct GroupedPair : g2::PolicyDefaults {
 struct GroupedPairTN : GroupedPair<false> {
   static constexpr uint32_t kIdesc = ptx::umma_idesc_mn_major(1, 1, g2::BM, g2::BN);
   static constexpr uint32_t kBlock = 64 * g2::BK_BYTES;         // one 64 (MN) x 64 (tokens) block: 8 KiB
-  static constexpr uint32_t kKStepBytes = 2048;                 // one MMA consumes 16 tokens = two swizzle atoms
+  static constexpr uint32_t kKStepA = 2048, kKStepB = 2048;     // one MMA consumes 16 tokens = two swizzle atoms
   __device__ static __forceinline__ uint64_t desc_a0(uint32_t a0) { return ptx::umma_desc_sw128_ex(a0, kBlock, 1024); }
   __device__ static __forceinline__ uint64_t desc_b0(uint32_t b0) { return ptx::umma_desc_sw128_ex(b0, kBlock, 1024); }
   __device__ static __forceinline__ int num_kb(const Params& p, int m_blk) {

@@ -41,6 +41,15 @@ inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
+// Runs an encode; a thread that has not used CUDA yet (an autograd worker) has no current context, and the encoder is a
+// driver call that does not create one.
+template <class F> inline CUresult encode_in_context(F&& f) {
+  CUresult r = f();
+  int dev = 0;
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = f();
+  return r;
+}
+
 // 2-D row-major tensor [rows, cols] with row pitch `ld` elements; box = [box_rows, box_cols],
 // 128-byte swizzle (box_cols * elem_bytes must be 128).
 inline int make_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t rows,
@@ -57,8 +66,10 @@ inline int make_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes
   cuuint64_t strides[1] = {ld * (uint64_t)elem_bytes};
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                  l2, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_in_context([&] {
+    return fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, l2,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) {
     last_error() = "cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r);
     return 7;
@@ -82,8 +93,10 @@ inline int make_tmap_colblocks_3d(CUtensorMap* out, CUtensorMapDataType dt, cons
   cuuint64_t strides[2] = {ld * 2, 128};
   cuuint32_t box[3] = {64, box_rows, box_blocks};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_in_context([&] {
+    return fn(out, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) {
     last_error() = "cuTensorMapEncodeTiled (3-D column blocks) failed with CUresult " + std::to_string((int)r);
     return 7;

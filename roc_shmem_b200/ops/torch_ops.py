@@ -2,9 +2,9 @@
 
 ``torch.ops.bshmem.linear(x, w)`` is ``x @ w.T`` on the tcgen05 GEMM with a registered fake (meta)
 implementation and an autograd formula whose two gradients also run on the tcgen05 kernels
-(data gradient: K-major GEMM on a transposed weight copy; weight gradient: the transposed-operand
-MN-major GEMM, no activation transpose).  ``torch.ops.bshmem.linear_fp8`` quantises both operands
-to block-scaled e4m3 and runs the fp8 kernel (forward only).  The reference has no PyTorch layer.
+(data gradient: MN-major weight operand; weight gradient: both operands MN-major; nothing is
+transposed).  ``torch.ops.bshmem.linear_fp8`` quantises both operands to block-scaled e4m3 and runs
+the fp8 kernel (forward only).  The reference has no PyTorch layer.
 """
 from __future__ import annotations
 
@@ -34,24 +34,24 @@ def _(x, w):
 
 @torch.library.custom_op("bshmem::linear_wgrad", mutates_args=())
 def linear_wgrad(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
-    """dW[N, K] = dy[M, N].T @ x[M, K] on token-major operands (needs M % 64 == 0, N % 256 == 0, K % 256 == 0;
-    other shapes fall back to transposing dy and x once and using the K-major kernel)."""
-    from .moe import grouped_gemm_tn
-    M, N = dy.shape
-    K = x.shape[1]
-    out = torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
-    if M % 64 == 0 and N % 256 == 0 and K % 256 == 0:
-        rows = torch.full((1,), M, dtype=torch.int32, device=x.device)
-        grouped_gemm_tn(dy.contiguous(), x.contiguous(), out, 1, rows)
-        return out
-    if M % 8:
-        raise ValueError("linear_wgrad: the token count must be a multiple of 8")
-    return gemm_bf16(dy.t().contiguous(), x.t().contiguous(), out)
+    """dW[N, K] = dy[M, N].T @ x[M, K] on token-major operands, for any number of tokens."""
+    return gemm_bf16(dy.contiguous(), x.contiguous(), a_mn=True, b_mn=True)
 
 
 @linear_wgrad.register_fake
 def _(dy, x):
     return x.new_empty((dy.shape[1], x.shape[1]))
+
+
+@torch.library.custom_op("bshmem::linear_dgrad", mutates_args=())
+def linear_dgrad(dy: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """dX[M, K] = dy[M, N] @ w[N, K]; the weight is read as it is stored."""
+    return gemm_bf16(dy.contiguous(), w.contiguous(), b_mn=True)
+
+
+@linear_dgrad.register_fake
+def _(dy, w):
+    return dy.new_empty((dy.shape[0], w.shape[1]))
 
 
 def _linear_setup(ctx, inputs, output):
@@ -61,7 +61,7 @@ def _linear_setup(ctx, inputs, output):
 def _linear_backward(ctx, dy):
     x, w = ctx.saved_tensors
     dy = dy.contiguous()
-    dx = torch.ops.bshmem.linear(dy, w.t().contiguous()) if ctx.needs_input_grad[0] else None
+    dx = torch.ops.bshmem.linear_dgrad(dy, w) if ctx.needs_input_grad[0] else None
     dw = torch.ops.bshmem.linear_wgrad(dy, x) if ctx.needs_input_grad[1] else None
     return dx, dw
 
@@ -81,6 +81,25 @@ def _(x, w):
     return x.new_empty((x.shape[0], w.shape[0]))
 
 
+class _LinearFn(torch.autograd.Function):
+    """The same layer without the dispatcher: a custom operator costs 60 to 100 us of host time per call (fake-tensor
+    and schema machinery), a training step of the layer makes three of them."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        _check_linear(x, w)
+        x, w = x.contiguous(), w.contiguous()
+        ctx.save_for_backward(x, w)
+        return gemm_bf16(x, w)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        dy = dy.contiguous()
+        need_x, need_w = ctx.needs_input_grad
+        return (gemm_bf16(dy, w, b_mn=True) if need_x else None, gemm_bf16(dy, x, a_mn=True, b_mn=True) if need_w else None)
+
+
 class Linear(torch.nn.Module):
     """Drop-in bf16 ``nn.Linear`` (no bias) whose forward and both gradients run on the tcgen05 kernels."""
 
@@ -90,9 +109,12 @@ class Linear(torch.nn.Module):
         torch.nn.init.normal_(self.weight, std=0.02)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
-        y = torch.ops.bshmem.linear(x.reshape(-1, x.shape[-1]), self.weight)
-        return y.reshape(*lead, -1)
+        if torch.compiler.is_compiling():               # a traced program needs the registered operator
+            lead = x.shape[:-1]
+            return torch.ops.bshmem.linear(x.reshape(-1, x.shape[-1]), self.weight).reshape(*lead, -1)
+        if x.dim() == 2:
+            return _LinearFn.apply(x, self.weight)
+        return _LinearFn.apply(x.reshape(-1, x.shape[-1]), self.weight).reshape(*x.shape[:-1], -1)
 
 
 # ---- collectives on the calling PE's runtime (roc_shmem_b200.current()) --------------------------------
