@@ -332,7 +332,6 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(L.tmem_slot()));
   // launched with programmatic serialization, the set-up above overlaps the previous kernel; without, this is a no-op
   ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
   if (threadIdx.x == 64) P::prologue(prm, g);
 
   if (warp == 0) {
@@ -354,6 +353,7 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
+      ptx::grid_launch_dependents();       // all loads are on their way: the next kernel's blocks may take their places
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {

@@ -17,6 +17,7 @@ import torch
 
 from .. import _native
 from ..gpu import DevState
+from .gemm import current_stream
 
 _declared = False
 SIG_FWD_DISPATCH, SIG_FWD_COMBINE, SIG_BWD_DISPATCH, SIG_BWD_COMBINE = range(4)
@@ -44,6 +45,10 @@ def moe_lib() -> C.CDLL:
         f("bshmem_moe_router_topk", VP, VP, I, I, I, I, VP, VP, VP, VP)
         f("bshmem_moe_plan", VP, I, I, VP, VP, VP)
         f("bshmem_moe_offsets", PP, VP, I, VP)
+        f("bshmem_moe_plan_local", PP, VP, I, VP, VP, VP, VP, I, VP)
+        f("bshmem_moe_dispatch_local", PP, VP, VP, VP, I, I, I, VP, VP)
+        f("bshmem_moe_dispatch_grad_local", PP, VP, VP, VP, VP, I, I, I, VP, VP, VP, VP, VP)
+        f("bshmem_moe_combine_local", PP, VP, VP, VP, VP, I, I, I, VP, VP, VP)
         f("bshmem_moe_dispatch", PS, PP, VP, VP, VP, VP, I, I, I, VP, VP, I, I, I, VP)
         f("bshmem_moe_wait_arrivals", PP, I, I, VP, I, VP, VP)
         f("bshmem_moe_combine_send", PS, PP, VP, VP, I, VP, I, I, I, VP)
@@ -63,8 +68,17 @@ def moe_lib() -> C.CDLL:
     return lib
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+class _Fast:
+    """The library's entry points as plain callables of integers (see _native.fast), bound on first use."""
+
+    def __getattr__(self, name):
+        fn = _native.fast(moe_lib(), "bshmem_moe_" + name)
+        setattr(self, name, fn)
+        return fn
+
+
+_fast = _Fast()
+_stream = current_stream
 
 
 def _p(t: Optional[torch.Tensor]) -> int:
@@ -83,16 +97,12 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
                  fixed_rows: int = 0, klen: Optional[torch.Tensor] = None, gated: bool = False, arrive=None, expected=None,
                  n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0) -> None:
     """out_g = a_g @ b_g.T per group on the tcgen05 grouped kernel.  a: [G*Ra, K], b: [G*Rb, K], out: [G*Ra, N or N/2]."""
-    lib = moe_lib()
     G = groups
     ra, rb = a.shape[0] // G, b.shape[0] // G
-    K = a.shape[1]
-    N = rb
-    st = lib.bshmem_moe_grouped_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, N, K, a.stride(0), b.stride(0),
-                                     out.stride(0), _p(rows), fixed_rows, _p(klen), int(gated), arrive or 0, _p(expected),
-                                     n_arrive, _stream(), timeout_ms, max_ctas)
+    st = _fast.grouped_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, rb, a.shape[1], a.stride(0), b.stride(0), out.stride(0),
+                            _p(rows), fixed_rows, _p(klen), gated, arrive, _p(expected), n_arrive, _stream(), timeout_ms, max_ctas)
     if st != 0:
-        raise RuntimeError(f"grouped gemm failed ({st}): {lib.bshmem_moe_gemm_last_error().decode()}")
+        raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 def grouped_gemm_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: int, counts: torch.Tensor, *,
@@ -100,22 +110,20 @@ def grouped_gemm_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups:
     """out_g[M, N] = a_g.T @ b_g per group with token-major operands a: [G*cap, M], b: [G*cap, N] and
     `counts[g]` tokens per group; both operands go to the tensor core MN-major, no transpose is materialised.
     Token rows [counts[g], next multiple of 64) of a and b must be zero (see zero_pad_rows)."""
-    lib = moe_lib()
     G = groups
     cap = a.shape[0] // G
-    st = lib.bshmem_moe_grouped_gemm_tn(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, cap, a.shape[1], b.shape[1], a.stride(0),
-                                        b.stride(0), out.stride(0), counts.data_ptr(), _stream(), timeout_ms, max_ctas)
+    st = _fast.grouped_gemm_tn(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, cap, a.shape[1], b.shape[1], a.stride(0), b.stride(0),
+                               out.stride(0), counts.data_ptr(), _stream(), timeout_ms, max_ctas)
     if st != 0:
-        raise RuntimeError(f"grouped gemm (tn) failed ({st}): {lib.bshmem_moe_gemm_last_error().decode()}")
+        raise RuntimeError(f"grouped gemm (tn) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 def zero_pad_rows(buf: torch.Tensor, groups: int, counts: torch.Tensor) -> None:
     """Zero rows [counts[g], next multiple of 64) of every group of a contiguous [G*cap, cols] bf16 buffer."""
-    lib = moe_lib()
     assert buf.is_contiguous()
-    st = lib.bshmem_moe_zero_pad_rows(buf.data_ptr(), counts.data_ptr(), groups, buf.shape[0] // groups, buf.shape[1], _stream())
+    st = _fast.zero_pad_rows(buf.data_ptr(), counts.data_ptr(), groups, buf.shape[0] // groups, buf.shape[1], _stream())
     if st != 0:
-        raise RuntimeError(f"zero_pad_rows failed ({st}): {lib.bshmem_moe_gemm_last_error().decode()}")
+        raise RuntimeError(f"zero_pad_rows failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 class MoELayer:
@@ -192,6 +200,10 @@ class MoELayer:
                             expect_from=self.expect_from.data_ptr(), send_to=self.send_to.data_ptr(),
                             dropped=self.dropped.data_ptr(), arrive_sig=self.arrive.data_ptr())
         self.state = rt.device_state()
+        self.ticket = torch.zeros((1,), dtype=torch.int32, device=dev)        # of the one-PE plan kernel
+        # addresses of the buffers above, which live as long as the layer
+        self._plan_a, self._state_a = C.addressof(self.plan), C.addressof(self.state)
+        self._a = {k: v.data_ptr() for k, v in vars(self).items() if isinstance(v, torch.Tensor)}
         self.err_word = self.lib.bshmem_moe_gemm_error_word()
         self.calls = 0
         self.launches = 0
@@ -215,51 +227,53 @@ class MoELayer:
 
     def route(self, x: torch.Tensor) -> None:
         """Router, plan, count exchange and offsets for this call's tokens."""
-        lib, T, s = self.lib, x.shape[0], _stream()
+        T, s, a = x.shape[0], _stream(), self._a
         n_entries = T * self.topk
         self.calls += 1
         self.parity = self.calls & 1
-        self._chk(lib.bshmem_moe_router_topk(x.data_ptr(), self.wr.data_ptr(), T, self.H, self.E, self.topk,
-                                             self.topk_idx.data_ptr(), self.topk_w.data_ptr(), 0, s), "router")
-        self._chk(lib.bshmem_moe_plan(self.topk_idx.data_ptr(), n_entries, self.E, self.pos.data_ptr(),
-                                      self.counts.data_ptr(), s), "plan")
-        if self.P > 1:
-            self.rt.fcollect(self.counts_all, self.counts)        # all-gather of the per-expert counts (device collective)
-            self.launches += 1
-        else:
-            self.counts_all.copy_(self.counts)
-        self._chk(lib.bshmem_moe_offsets(C.byref(self.plan), self.counts_all.data_ptr(), self.parity, s), "offsets")
+        self._chk(_fast.router_topk(x.data_ptr(), self.wr.data_ptr(), T, self.H, self.E, self.topk, a["topk_idx"], a["topk_w"], 0, s), "router")
+        if self.P == 1:
+            self._chk(_fast.plan_local(self._plan_a, a["topk_idx"], n_entries, a["pos"], a["counts"], a["counts_all"], a["ticket"],
+                                       self.parity, s), "plan")
+            return
+        self._chk(_fast.plan(a["topk_idx"], n_entries, self.E, a["pos"], a["counts"], s), "plan")
+        self.rt.fcollect(self.counts_all, self.counts)            # all-gather of the per-expert counts (device collective)
+        self.launches += 1
+        self._chk(_fast.offsets(self._plan_a, a["counts_all"], self.parity, s), "offsets")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lib, T, s = self.lib, x.shape[0], _stream()
+        T, s, a = x.shape[0], _stream(), self._a
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
+        local = P == 1                                             # no row leaves this GPU: no signals, no return buffer
         self.route(x)
         par = self.parity
-        self._chk(lib.bshmem_moe_dispatch(C.byref(self.state), C.byref(self.plan), x.data_ptr(), 0, self.topk_idx.data_ptr(),
-                                          self.pos.data_ptr(), n_entries, self.topk, H, self.recv.data_ptr(), self.meta.data_ptr(),
-                                          par, SIG_FWD_DISPATCH, self.ctas, s), "dispatch")
-        # gate/up projection waits on the arrival words inside the kernel, then SwiGLU, then down projection
+        if local:
+            self._chk(_fast.dispatch_local(self._plan_a, x.data_ptr(), a["topk_idx"], a["pos"], T, self.topk, H, a["recv"], s), "dispatch")
+            wait = {}
+        else:
+            self._chk(_fast.dispatch(self._state_a, self._plan_a, x.data_ptr(), 0, a["topk_idx"], a["pos"], n_entries, self.topk, H,
+                                     a["recv"], a["meta"], par, SIG_FWD_DISPATCH, self.ctas, s), "dispatch")
+            wait = dict(arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P)
+        # gate/up projection (waits on the arrival words inside the kernel), then SwiGLU, then down projection
         if self.training:
-            grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count,
-                         arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P,
-                         timeout_ms=self.timeout_ms)
-            self._chk(lib.bshmem_moe_swiglu_fwd(self.gu.data_ptr(), self.recv_count.data_ptr(), G, cap, F, self.hact.data_ptr(), s),
-                      "swiglu")
+            grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms, **wait)
+            self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
             self._x_in = x                                         # the router's backward needs the layer input
         else:
             grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.hact, G, rows=self.recv_count, gated=True,
-                         arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P,
-                         timeout_ms=self.timeout_ms)
+                         timeout_ms=self.timeout_ms, **wait)
         self.launches += 1
         grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms)
         self.launches += 1
-        self._chk(lib.bshmem_moe_combine_send(C.byref(self.state), C.byref(self.plan), self.yexp.data_ptr(), self.meta.data_ptr(), H,
-                                              self.ybuf.data_ptr(), par, SIG_FWD_COMBINE, self.ctas, s), "combine_send")
-        self._chk(lib.bshmem_moe_wait_arrivals(C.byref(self.plan), par, SIG_FWD_COMBINE, self.send_to.data_ptr(), self.timeout_ms,
-                                               self.err_word, s), "wait")
-        self._chk(lib.bshmem_moe_combine_reduce(C.byref(self.plan), self.ybuf.data_ptr(), self.topk_w.data_ptr(),
-                                                self.topk_idx.data_ptr(), self.pos.data_ptr(), T, self.topk, H, self.out.data_ptr(), s),
+        if local:
+            self._chk(_fast.combine_local(self._plan_a, a["yexp"], a["topk_w"], a["topk_idx"], a["pos"], T, self.topk, H, a["out"], 0, s),
+                      "combine")
+            return self.out[:T]
+        self._chk(_fast.combine_send(self._state_a, self._plan_a, a["yexp"], a["meta"], H, a["ybuf"], par, SIG_FWD_COMBINE, self.ctas, s),
+                  "combine_send")
+        self._chk(_fast.wait_arrivals(self._plan_a, par, SIG_FWD_COMBINE, a["send_to"], self.timeout_ms, self.err_word, s), "wait")
+        self._chk(_fast.combine_reduce(self._plan_a, a["ybuf"], a["topk_w"], a["topk_idx"], a["pos"], T, self.topk, H, a["out"], s),
                   "combine_reduce")
         return self.out[:T]
 
@@ -268,27 +282,35 @@ class MoELayer:
         self.dw2), the routing weights (self.dtopk_w) and, through the softmax over the chosen experts, the router
         weights (self.dwr).  Must follow forward() of the same tokens; the forward's input must still be intact."""
         assert self.training
-        lib, T, s = self.lib, dout.shape[0], _stream()
+        T, s, a = dout.shape[0], _stream(), self._a
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
+        local = P == 1
         par = self.parity
         rc = self.recv_count
-        self._chk(lib.bshmem_moe_router_weight_grad(C.byref(self.plan), self.ybuf.data_ptr(), dout.data_ptr(),
-                                                    self.topk_idx.data_ptr(), self.pos.data_ptr(), n_entries, self.topk, H,
-                                                    self.dtopk_w.data_ptr(), s), "router weight grad")
-        # router backward: d_logits of the chosen experts and d_Wr = d_logits^T · x
-        self._chk(lib.bshmem_moe_router_backward(self._x_in.data_ptr(), self.topk_idx.data_ptr(), self.topk_w.data_ptr(),
-                                                 self.dtopk_w.data_ptr(), T, H, self.E, self.topk, self.dlogit.data_ptr(),
-                                                 self.dwr_f32.data_ptr(), self.dwr.data_ptr(), s), "router backward")
-        self.launches += 2
-        # combine-backward = dispatch of w * d_out into the experts' gradient receive buffers (same slots as forward)
         dy = self.recv_bwd
-        self._chk(lib.bshmem_moe_dispatch(C.byref(self.state), C.byref(self.plan), dout.data_ptr(), self.topk_w.data_ptr(),
-                                          self.topk_idx.data_ptr(), self.pos.data_ptr(), n_entries, self.topk, H, dy.data_ptr(),
-                                          0, par, SIG_BWD_DISPATCH, self.ctas, s), "dispatch(bwd)")
+        if local:
+            # w * d_out into the experts' gradient buffers, and in the same pass the gradients of the routing weights and of
+            # the chosen experts' logits
+            self._chk(_fast.dispatch_grad_local(self._plan_a, dout.data_ptr(), a["topk_idx"], a["pos"], a["topk_w"], T, self.topk, H,
+                                                a["recv_bwd"], a["yexp"], a["dtopk_w"], a["dlogit"], s), "dispatch(bwd)")
+            self._chk(_fast.router_backward(self._x_in.data_ptr(), a["topk_idx"], 0, 0, T, H, self.E, self.topk, a["dlogit"], a["dwr_f32"],
+                                            a["dwr"], s), "router backward")
+            self.launches += 1
+            wait = {}
+        else:
+            self._chk(_fast.router_weight_grad(self._plan_a, a["ybuf"], dout.data_ptr(), a["topk_idx"], a["pos"], n_entries, self.topk, H,
+                                               a["dtopk_w"], s), "router weight grad")
+            # router backward: d_logits of the chosen experts and d_Wr = d_logits^T · x
+            self._chk(_fast.router_backward(self._x_in.data_ptr(), a["topk_idx"], a["topk_w"], a["dtopk_w"], T, H, self.E, self.topk,
+                                            a["dlogit"], a["dwr_f32"], a["dwr"], s), "router backward")
+            self.launches += 2
+            # combine-backward = dispatch of w * d_out into the experts' gradient receive buffers (same slots as forward)
+            self._chk(_fast.dispatch(self._state_a, self._plan_a, dout.data_ptr(), a["topk_w"], a["topk_idx"], a["pos"], n_entries, self.topk,
+                                     H, a["recv_bwd"], 0, par, SIG_BWD_DISPATCH, self.ctas, s), "dispatch(bwd)")
+            wait = dict(arrive=self._sig_ptr(par, SIG_BWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # d_hact = d_y · W2            (B operand = W2^T [F, H], K = H)
-        grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, arrive=self._sig_ptr(par, SIG_BWD_DISPATCH),
-                     expected=self.expect_from, n_arrive=P, timeout_ms=self.timeout_ms)
+        grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, **wait)
         # dW2 = d_y^T · hact: token-major operands straight into the MN-major tensor-core path
         if self.tn_gemm:
             zero_pad_rows(dy, G, rc)
@@ -297,12 +319,11 @@ class MoELayer:
         else:                          # explicit transposes + ragged-K K-major GEMM
             ta = self.t_a[: G * H * cap].view(G * H, cap)
             tb = self.t_b[: G * F * cap].view(G * F, cap)
-            self._chk(lib.bshmem_moe_transpose_pad(dy.data_ptr(), rc.data_ptr(), G, cap, H, ta.data_ptr(), s), "transpose")
-            self._chk(lib.bshmem_moe_transpose_pad(self.hact.data_ptr(), rc.data_ptr(), G, cap, F, tb.data_ptr(), s), "transpose")
+            self._chk(_fast.transpose_pad(dy.data_ptr(), rc.data_ptr(), G, cap, H, ta.data_ptr(), s), "transpose")
+            self._chk(_fast.transpose_pad(a["hact"], rc.data_ptr(), G, cap, F, tb.data_ptr(), s), "transpose")
             grouped_gemm(ta, tb, self.dw2.view(G * H, F), G, fixed_rows=H, klen=rc, timeout_ms=self.timeout_ms)
         # SwiGLU backward, then dW13 = d_gu^T · x and d_x = d_gu · W13
-        self._chk(lib.bshmem_moe_swiglu_bwd(self.gu.data_ptr(), self.dh.data_ptr(), rc.data_ptr(), G, cap, F, self.dgu.data_ptr(), s),
-                  "swiglu bwd")
+        self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
         if self.tn_gemm:
             zero_pad_rows(self.dgu, G, rc)
             zero_pad_rows(self.xsave, G, rc)
@@ -310,20 +331,23 @@ class MoELayer:
         else:
             ta2 = self.t_a[: G * 2 * F * cap].view(G * 2 * F, cap)
             tb2 = self.t_b[: G * H * cap].view(G * H, cap)
-            self._chk(lib.bshmem_moe_transpose_pad(self.dgu.data_ptr(), rc.data_ptr(), G, cap, 2 * F, ta2.data_ptr(), s), "transpose")
-            self._chk(lib.bshmem_moe_transpose_pad(self.xsave.data_ptr(), rc.data_ptr(), G, cap, H, tb2.data_ptr(), s), "transpose")
+            self._chk(_fast.transpose_pad(a["dgu"], rc.data_ptr(), G, cap, 2 * F, ta2.data_ptr(), s), "transpose")
+            self._chk(_fast.transpose_pad(self.xsave.data_ptr(), rc.data_ptr(), G, cap, H, tb2.data_ptr(), s), "transpose")
             grouped_gemm(ta2, tb2, self.dw13.view(G * 2 * F, H), G, fixed_rows=2 * F, klen=rc, timeout_ms=self.timeout_ms)
         grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms)
         self.launches += 4
+        if local:
+            # d_x = sum over k of the experts' rows + the router path (d_logits · Wr), written once
+            self._chk(_fast.combine_local(self._plan_a, a["dxe"], a["dlogit"], a["topk_idx"], a["pos"], T, self.topk, H, a["dx"], self.wr.data_ptr(), s),
+                      "combine(bwd)")
+            return self.dx[:T]
         # dispatch-backward = combine of the d_x rows back to their source entries, summed over k
-        self._chk(lib.bshmem_moe_combine_send(C.byref(self.state), C.byref(self.plan), self.dxe.data_ptr(), self.meta.data_ptr(), H,
-                                              self.dxbuf.data_ptr(), par, SIG_BWD_COMBINE, self.ctas, s), "combine_send(bwd)")
-        self._chk(lib.bshmem_moe_wait_arrivals(C.byref(self.plan), par, SIG_BWD_COMBINE, self.send_to.data_ptr(), self.timeout_ms,
-                                               self.err_word, s), "wait")
+        self._chk(_fast.combine_send(self._state_a, self._plan_a, a["dxe"], a["meta"], H, a["dxbuf"], par, SIG_BWD_COMBINE, self.ctas, s),
+                  "combine_send(bwd)")
+        self._chk(_fast.wait_arrivals(self._plan_a, par, SIG_BWD_COMBINE, a["send_to"], self.timeout_ms, self.err_word, s), "wait")
         # d_x = sum over k of the returned rows + the router path (d_logits · Wr), written once
-        self._chk(lib.bshmem_moe_combine_reduce_router(C.byref(self.plan), self.dxbuf.data_ptr(), self.topk_idx.data_ptr(),
-                                                       self.pos.data_ptr(), T, self.topk, H, self.dx.data_ptr(),
-                                                       self.dlogit.data_ptr(), self.wr.data_ptr(), s), "combine_reduce(bwd)")
+        self._chk(_fast.combine_reduce_router(self._plan_a, a["dxbuf"], a["topk_idx"], a["pos"], T, self.topk, H, a["dx"], a["dlogit"],
+                                              self.wr.data_ptr(), s), "combine_reduce(bwd)")
         return self.dx[:T]
 
     def check(self) -> None:
