@@ -30,7 +30,7 @@ using gemm::pack_bf16;
 constexpr int ROWS = 128;                          // weight rows of a tile
 constexpr int BK = 64;                             // bf16 elements per k-block: one 128-byte swizzle atom
 constexpr int MAX_TOKENS = 256;
-constexpr int MAX_STAGES = 8;
+constexpr int MAX_STAGES = 8;                     // of the dense form; the grouped form: MAX_GROUP_STAGES
 constexpr int NUM_EPI_WARPS = 4;
 constexpr int NUM_THREADS = 32 * (2 + NUM_EPI_WARPS);
 constexpr uint32_t W_STAGE_BYTES = ROWS * BK * 2;  // 16 KiB
@@ -243,6 +243,226 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
   }
   if (*L.abort_flag()) {
     // let copies and MMAs that are still in flight land before shared and tensor memory go away
+    const unsigned long long t0 = ptx::globaltimer();
+    while (ptx::globaltimer() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, p.tmem_cols);
+  }
+}
+
+}  // namespace skinny
+}  // namespace bshmem
+
+// ---- grouped form: few tokens per group (the experts of a decode step) -----------------------------------------------
+//   C_g[rows_g, N] = X_g[rows_g, K] · W_g[N, K]^T  for every group g, the row counts read on the device.
+// Persistent CTAs over (group, chunk of up to 256 tokens, 128 weight rows); groups without rows cost nothing.  Two
+// accumulators, so that the epilogue of a tile overlaps the loads and MMAs of the next.  The stage size follows the
+// largest group of the call: 16 KiB of weights plus 128 bytes per token, as many stages as fit.
+// Gated: the weight rows are 32 gate rows followed by the matching 32 up rows, i.e. alternating quarters of the tensor
+// memory; the up warps hand their values to the gate warps through shared memory, 16 tokens at a time, and the gate warps
+// write silu(gate) * up.
+namespace bshmem {
+namespace skinny {
+
+constexpr int MAX_GROUPS = 64, MAX_GROUP_STAGES = 12;
+constexpr int XBOX = 16;                           // token rows per TMA box
+constexpr uint32_t GROUP_XCHG_BYTES = 2 * 2 * 16 * 32 * 4;             // two warp pairs x two buffers x 16 tokens x 32 columns
+constexpr uint32_t GROUP_CTRL_BYTES = 8 * (2 * MAX_GROUP_STAGES + 6) + 16 + 4 * MAX_GROUPS;
+
+struct GroupedParams {
+  CUtensorMap map_w, map_x;      // weights [G * N, K] box {64, 128}; tokens [G * cap, K] box {64, 16}
+  __nv_bfloat16* out;            // [G * cap, N] or gated [G * cap, N / 2]
+  long long ldo;
+  const int* rows;
+  int G, cap, N, K;
+  uint32_t ring_bytes;           // shared memory of the stages
+  uint32_t tmem_cols;            // two accumulators
+  int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 256)
+  int P;                         // arrival words to wait for before the first token load (0: none)
+  const unsigned long long* arrive;
+  const int* expected;
+  unsigned long long timeout_ns;
+  int* err;
+};
+
+enum GroupErrSite : int { ERR_G_PRODUCER_EMPTY = 311, ERR_G_MMA_FULL = 312, ERR_G_MMA_ACC = 313, ERR_G_EPI_FULL = 314, ERR_G_ARRIVE = 315 };
+
+struct GroupedSmem {
+  uint32_t base, ctrl;
+  uint8_t* gen;
+  __device__ __forceinline__ uint32_t full(int s) const { return ctrl + 8 * s; }
+  __device__ __forceinline__ uint32_t empty(int s) const { return ctrl + 8 * (MAX_GROUP_STAGES + s); }
+  __device__ __forceinline__ uint32_t acc_full(int a) const { return ctrl + 8 * (2 * MAX_GROUP_STAGES + a); }
+  __device__ __forceinline__ uint32_t acc_empty(int a) const { return ctrl + 8 * (2 * MAX_GROUP_STAGES + 2 + a); }
+  __device__ __forceinline__ uint32_t tmem_slot() const { return ctrl + 8 * (2 * MAX_GROUP_STAGES + 4); }
+  __device__ __forceinline__ volatile int* abort_flag() const { return reinterpret_cast<volatile int*>(gen + 8 * (2 * MAX_GROUP_STAGES + 5)); }
+  __device__ __forceinline__ int* rows() const { return reinterpret_cast<int*>(gen + 8 * (2 * MAX_GROUP_STAGES + 6)); }
+};
+
+// Walks the tiles first, first + step, ...: weight blocks fastest, then chunks, then groups.
+struct GroupedTiles {
+  const int* rows;
+  int G, nb, chunk;              // groups, weight blocks per group, tokens per chunk
+  int tile, step, g, base;       // base: index of the first tile of group g
+  __device__ __forceinline__ bool next(int* group, int* n_blk, int* tok0, int* ntok) {
+    for (; g < G; ++g) {
+      const int r = rows[g], n = (r + chunk - 1) / chunk * nb;
+      if (tile < base + n) {
+        const int in = tile - base, c = in / nb;
+        *group = g; *n_blk = in - c * nb; *tok0 = c * chunk; *ntok = min(chunk, r - c * chunk);
+        tile += step;
+        return true;
+      }
+      base += n;
+    }
+    return false;
+  }
+};
+
+template <bool kGated>
+__device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* smem_raw) {
+  GroupedSmem L;
+  uint32_t xchg;
+  {
+    const uint32_t r = ptx::smem_u32(smem_raw);
+    L.base = (r + 1023u) & ~1023u;
+    xchg = L.base + p.ring_bytes;
+    L.ctrl = xchg + (kGated ? GROUP_XCHG_BYTES : 0);
+    L.gen = smem_raw + (L.ctrl - r);
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Guard g{p.err, L.abort_flag(), p.timeout_ns};
+  if (threadIdx.x == 0) {
+    *L.abort_flag() = 0;
+    for (int s = 0; s < MAX_GROUP_STAGES; ++s) { ptx::mbar_init(L.full(s), 1); ptx::mbar_init(L.empty(s), 1); }
+    for (int a = 0; a < 2; ++a) { ptx::mbar_init(L.acc_full(a), 1); ptx::mbar_init(L.acc_empty(a), NUM_EPI_WARPS); }
+    ptx::fence_mbar_init();
+    ptx::prefetch_tensormap(&p.map_w);
+    ptx::prefetch_tensormap(&p.map_x);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(L.tmem_slot(), p.tmem_cols);
+    ptx::tmem_relinquish();
+  }
+  ptx::grid_dependency_wait();
+  for (int i = threadIdx.x; i < p.G; i += NUM_THREADS) L.rows()[i] = __ldcg(p.rows + i);
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(L.tmem_slot()));
+  int most = 1;
+  for (int i = 0; i < p.G; ++i) most = max(most, L.rows()[i]);
+  const int nt_max = min((most + 15) / 16 * 16, p.nt_cap);
+  const uint32_t stage = W_STAGE_BYTES + (uint32_t)nt_max * BK * 2;
+  const int stages = min((int)(p.ring_bytes / stage), MAX_GROUP_STAGES);
+  const int num_kb = (p.K + BK - 1) / BK;
+  GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x, (int)gridDim.x, 0, 0};
+  int grp, n_blk, tok0, ntok;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0; uint32_t ph = 0;
+      bool ok = true;
+      for (int q = 0; q < p.P && ok; ++q) ok = gemm::wait_ge<true>(p.arrive + q, (unsigned long long)p.expected[q], g, ERR_G_ARRIVE);
+      if (p.P) ptx::fence_proxy_async_all();         // peer stores (generic proxy) before the TMA reads
+      while (ok && it.next(&grp, &n_blk, &tok0, &ntok)) {
+        const int boxes = (ntok + XBOX - 1) / XBOX;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_G_PRODUCER_EMPTY)) { ok = false; break; }
+          const uint32_t w = L.base + s * stage, x = w + W_STAGE_BYTES;
+          ptx::mbar_arrive_expect_tx(L.full(s), W_STAGE_BYTES + boxes * (XBOX * BK * 2));
+          ptx::tma_load_2d(w, &p.map_w, L.full(s), kb * BK, grp * p.N + n_blk * ROWS);
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d(x + b * (XBOX * BK * 2), &p.map_x, L.full(s), kb * BK, grp * p.cap + tok0 + b * XBOX);
+          if (++s == stages) { s = 0; ph ^= 1; }
+        }
+      }
+      ptx::grid_launch_dependents();
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0; uint32_t ph = 0, acc_ph = 0;
+      bool ok = true;
+      for (int ord = 0; ok && it.next(&grp, &n_blk, &tok0, &ntok); ++ord) {
+        const int acc = ord & 1;
+        if (!mbar_wait(L.acc_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_G_MMA_ACC)) break;
+        acc_ph ^= 1u << acc;
+        ptx::tc_fence_after();
+        const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)((ntok + 15) / 16 * 16));
+        const uint32_t d = tmem + acc * p.nt_cap;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(L.full(s), ph, g, ERR_G_MMA_FULL)) { ok = false; break; }
+          ptx::tc_fence_after();
+          const uint64_t dw = ptx::umma_desc_sw128(L.base + s * stage), dx = ptx::umma_desc_sw128(L.base + s * stage + W_STAGE_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(d, dw + 2 * k, dx + 2 * k, idesc, (kb || k) ? 1u : 0u);
+          ptx::umma_commit(L.empty(s));
+          if (++s == stages) { s = 0; ph ^= 1; }
+        }
+        if (ok) ptx::umma_commit(L.acc_full(acc));
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+    uint32_t acc_ph = 0;
+    uint32_t vote = 1;
+    uint32_t turn = 0;                               // exchange buffer of the next 16 tokens
+    for (int ord = 0; it.next(&grp, &n_blk, &tok0, &ntok); ++ord) {
+      const int acc = ord & 1;
+      bool ok = mbar_wait(L.acc_full(acc), (acc_ph >> acc) & 1, g, ERR_G_EPI_FULL);
+      if constexpr (kGated) {
+        // a gate and an up warp meet at barriers below: both go on or both leave
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(vote) : "r"((uint32_t)ok), "r"(1 + (quarter >> 1)) : "memory");
+        ok = vote != 0;
+      }
+      if (!ok) break;
+      acc_ph ^= 1u << acc;
+      ptx::tc_fence_after();
+      const uint32_t taddr = lanes + acc * p.nt_cap;
+      __nv_bfloat16* out = p.out + ((long long)grp * p.cap + tok0) * p.ldo + (kGated ? n_blk * (ROWS / 2) + (quarter >> 1) * 32 : n_blk * ROWS + quarter * 32) + lane;
+      for (int c = 0; c < ntok; c += 16) {
+        uint32_t v[16];
+        ptx::tmem_ld_32x32b_x16(taddr + c, v);
+        ptx::tmem_ld_wait();
+        if constexpr (!kGated) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < ntok) out[(long long)(c + j) * p.ldo] = __float2bfloat16_rn(__uint_as_float(v[j]));
+        } else {
+          // buffer `turn` is free: the gate warp read it before it came to the barrier of the previous 16 tokens
+          const uint32_t buf = xchg + (((quarter >> 1) * 2 + turn) * 16 * 32 + lane) * 4;
+          if (quarter & 1) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(buf + j * 128), "r"(v[j]) : "memory");
+          }
+          asm volatile("bar.sync %0, 64;" ::"r"(1 + (quarter >> 1)) : "memory");
+          if (!(quarter & 1)) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              float u;
+              asm volatile("ld.shared.f32 %0, [%1];" : "=f"(u) : "r"(buf + j * 128) : "memory");
+              const float gate = __uint_as_float(v[j]);
+              if (c + j < ntok) out[(long long)(c + j) * p.ldo] = __float2bfloat16_rn(gate / (1.f + __expf(-gate)) * u);
+            }
+          }
+          turn ^= 1;
+        }
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(L.acc_empty(acc));
+    }
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (*L.abort_flag()) {
     const unsigned long long t0 = ptx::globaltimer();
     while (ptx::globaltimer() - t0 < 2000000ull) __nanosleep(1000);
     __syncthreads();

@@ -17,6 +17,7 @@
 #include <cstdlib>
 
 #include "gemm_pair.cuh"
+#include "gemm_skinny.cuh"
 #include "moe_common.h"
 #include "tma_host.h"
 
@@ -230,6 +231,13 @@ grouped_gemm_pair_tn_kernel(const __grid_constant__ GroupedParams prm) {
   g2::gemm_mainloop<GroupedPairTN>(prm, smem_raw);
 }
 
+// Few rows per group (decode): weight-streaming tiles, see gemm_skinny.cuh.
+template <bool kGated>
+__global__ void __launch_bounds__(skinny::NUM_THREADS) grouped_gemm_few_kernel(const __grid_constant__ skinny::GroupedParams prm) {
+  extern __shared__ uint8_t smem_raw[];
+  skinny::grouped_body<kGated>(prm, smem_raw);
+}
+
 // Zero the token rows [count_g, next multiple of 64) — rows [0, 64) of an empty group — of every group of a
 // [G][cap][cols] bf16 buffer.
 __global__ void zero_pad_rows_kernel(__nv_bfloat16* buf, const int* counts, int cap, int cols) {
@@ -259,6 +267,8 @@ int ensure(int dev) {
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
   g_pairs[dev] = g2::max_resident_pairs(grouped_gemm_pair_kernel, g_sms[dev]);
   return 0;
 }
@@ -320,6 +330,59 @@ int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_
     else grouped_gemm_kernel<<<ctas, NUM_THREADS, SMEM_BYTES, st>>>(p);
   }
   BSHMEM_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
+// The same product for few rows per group (up to about 128; more are taken in chunks of 128, reading the weights again).
+// max_rows and max_active bound the largest group and the number of groups with rows as far as the host knows them (the
+// tokens and the token-expert entries of a decode step).  Up to 64 groups, a_rows_per_group and N multiples of 256; rows of
+// C beyond a group's count are not written.
+// us, 8 groups, N x K = 28672 x 4096 gated: 8 rows each 285 against 406 for the 256-row tiles (weights at the measured copy
+// rate: 288), 64 rows 316 / 388, 128 rows 416 / 439, 200 rows 1062 / 384.
+int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, int a_rows_per_group, int N, int K, int lda, int ldb, int ldc,
+                                const int* rows_dev, int max_rows, int max_active, int gated, const void* arrive, const int* expected, int P,
+                                void* stream, int timeout_ms) {
+  if (G < 1 || G > skinny::MAX_GROUPS || a_rows_per_group % BM || N % BN || K % 8 || lda % 8 || ldb % 8 || ldc % 8 || !rows_dev || max_rows < 1) {
+    host::last_error() = "grouped gemm (few rows): needs 1 to 64 groups, rows-per-group % 256 == 0, N % 256 == 0, K and leading dimensions % 8 == 0";
+    return 1;
+  }
+  int dev = 0;
+  BSHMEM_CUDA_TRY(cudaGetDevice(&dev));
+  int rc = ensure(dev);
+  if (rc) return rc;
+  skinny::GroupedParams p;
+  p.out = static_cast<__nv_bfloat16*>(C);
+  p.ldo = ldc;
+  p.rows = rows_dev;
+  p.G = G; p.cap = a_rows_per_group; p.N = N; p.K = K;
+  if (max_rows > a_rows_per_group) max_rows = a_rows_per_group;
+  p.nt_cap = max_rows >= 128 ? 128 : (max_rows + 15) / 16 * 16;
+  // Two CTAs per SM, except where the tiles cannot occupy more than one: then that one gets all the stages (two groups with
+  // one row, N x K = 4096 x 14336: 64 CTAs with half the shared memory stream at 45 GB/s each).
+  if (max_active < 1 || max_active > G) max_active = G;
+  const bool half = (long long)max_active * (N / skinny::ROWS) * ((max_rows + p.nt_cap - 1) / p.nt_cap) > g_sms[dev];
+  const uint32_t fixed = 1024 + skinny::GROUP_CTRL_BYTES + (gated ? skinny::GROUP_XCHG_BYTES : 0);
+  p.ring_bytes = ((half ? skinny::SMEM_HALF : skinny::SMEM_FULL) - fixed) & ~1023u;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < 2u * p.nt_cap) p.tmem_cols *= 2;
+  p.P = P; p.arrive = static_cast<const unsigned long long*>(arrive); p.expected = expected;
+  p.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 4000) * 1000000ull;
+  p.err = g_err_dev[dev];
+  rc = host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, (uint64_t)G * N, K, ldb, skinny::ROWS, skinny::BK);
+  if (rc) return rc;
+  rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, skinny::XBOX, skinny::BK);
+  if (rc) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(g_sms[dev] * (half ? 2 : 1)));
+  cfg.blockDim = dim3(skinny::NUM_THREADS);
+  cfg.dynamicSmemBytes = p.ring_bytes + fixed;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, gated ? grouped_gemm_few_kernel<true> : grouped_gemm_few_kernel<false>, p));
   return 0;
 }
 

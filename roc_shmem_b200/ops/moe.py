@@ -21,6 +21,9 @@ from .gemm import current_stream
 
 _declared = False
 SIG_FWD_DISPATCH, SIG_FWD_COMBINE, SIG_BWD_DISPATCH, SIG_BWD_COMBINE = range(4)
+# Average rows per expert up to which the weight-streaming GEMM is the faster one (it is up to 128 rows in a group; a router
+# spreads the tokens of a batch unevenly, and a group beyond 128 reads its weights twice)
+FEW_ROWS = 64
 
 
 class PlanDev(C.Structure):
@@ -60,6 +63,7 @@ def moe_lib() -> C.CDLL:
         f("bshmem_moe_swiglu_bwd", VP, VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_transpose_pad", VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_grouped_gemm", VP, VP, VP, I, I, I, I, I, I, I, I, VP, I, VP, I, VP, VP, I, VP, I, I)
+        f("bshmem_moe_grouped_gemm_few", VP, VP, VP, I, I, I, I, I, I, I, VP, I, I, I, VP, VP, I, VP, I)
         f("bshmem_moe_grouped_gemm_tn", VP, VP, VP, I, I, I, I, I, I, I, VP, VP, I, I)
         f("bshmem_moe_zero_pad_rows", VP, VP, I, I, I, VP)
         f("bshmem_moe_gemm_error_site", I)
@@ -95,10 +99,19 @@ def interleave_gate_up(w1: torch.Tensor, w3: torch.Tensor) -> torch.Tensor:
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: int, *, rows: Optional[torch.Tensor] = None,
                  fixed_rows: int = 0, klen: Optional[torch.Tensor] = None, gated: bool = False, arrive=None, expected=None,
-                 n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0) -> None:
-    """out_g = a_g @ b_g.T per group on the tcgen05 grouped kernel.  a: [G*Ra, K], b: [G*Rb, K], out: [G*Ra, N or N/2]."""
+                 n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0, few: Optional[tuple] = None) -> None:
+    """out_g = a_g @ b_g.T per group on the tcgen05 grouped kernel.  a: [G*Ra, K], b: [G*Rb, K], out: [G*Ra, N or N/2].
+    `few` = (most rows of a group, most groups with rows): the caller expects about 100 rows per group or less; the
+    weight-streaming form takes such problems."""
     G = groups
     ra, rb = a.shape[0] // G, b.shape[0] // G
+    if few is not None and rows is not None and G <= 64:
+        st = _fast.grouped_gemm_few(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, a.shape[1], a.stride(0), b.stride(0),
+                                    out.stride(0), rows.data_ptr(), few[0], few[1], gated, arrive, _p(expected), n_arrive, _stream(),
+                                    timeout_ms)
+        if st != 0:
+            raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
+        return
     st = _fast.grouped_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, rb, a.shape[1], a.stride(0), b.stride(0), out.stride(0),
                             _p(rows), fixed_rows, _p(klen), gated, arrive, _p(expected), n_arrive, _stream(), timeout_ms, max_ctas)
     if st != 0:
@@ -246,6 +259,8 @@ class MoELayer:
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
         local = P == 1                                             # no row leaves this GPU: no signals, no return buffer
+        # (every PE brings about as many tokens; a group has at most one row per token of each PE)
+        few = (P * T, P * n_entries) if P * n_entries <= FEW_ROWS * self.E else None
         self.route(x)
         par = self.parity
         if local:
@@ -257,14 +272,15 @@ class MoELayer:
             wait = dict(arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # gate/up projection (waits on the arrival words inside the kernel), then SwiGLU, then down projection
         if self.training:
-            grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms, **wait)
+            grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms,
+                         few=few, **wait)
             self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
             self._x_in = x                                         # the router's backward needs the layer input
         else:
             grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.hact, G, rows=self.recv_count, gated=True,
-                         timeout_ms=self.timeout_ms, **wait)
+                         timeout_ms=self.timeout_ms, few=few, **wait)
         self.launches += 1
-        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms)
+        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms, few=few)
         self.launches += 1
         if local:
             self._chk(_fast.combine_local(self._plan_a, a["yexp"], a["topk_w"], a["topk_idx"], a["pos"], T, self.topk, H, a["out"], 0, s),

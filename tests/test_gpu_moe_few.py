@@ -1,0 +1,63 @@
+"""Grouped GEMM for few rows per group and the one-PE MoE data movement at the sizes where they can go wrong: empty groups,
+counts around the MMA's steps of 16 and the chunk of 128, one group only, both epilogues."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("rows", [[0, 0, 1], [16, 17, 0], [127, 128, 129], [256, 3, 0], [0, 250, 15]])
+@pytest.mark.parametrize("N,K", [(256, 64), (512, 1000), (2048, 2048)])
+def test_grouped_gemm_few_rows(rows, gated, N, K):
+    from roc_shmem_b200.ops.moe import grouped_gemm, moe_lib
+    torch.manual_seed(sum(rows) + N)
+    G, cap = len(rows), 256
+    a = torch.randn(G * cap, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(G * N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    cnt = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    out = torch.full((G * cap, N // 2 if gated else N), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm(a, b, out, G, rows=cnt, gated=gated, few=(max(rows), sum(r > 0 for r in rows)))
+    torch.cuda.synchronize()
+    assert moe_lib().bshmem_moe_gemm_error_site(1) == 0
+    for g, n in enumerate(rows):
+        assert bool((out[g * cap + n:(g + 1) * cap] == 7).all())                     # nothing beyond a group's rows
+        ref = a[g * cap:g * cap + n].double() @ b[g * N:(g + 1) * N].double().t()
+        tol = K * K * 2 ** -24 / K ** 0.5 * 0.1 + 1e-6                               # fp32 sums in another order
+        if gated:                                                                    # 32 gate columns, then the 32 up columns
+            pair = ref.view(n, N // 64, 2, 32)
+            ref = (torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).reshape(n, N // 2)
+            tol = tol * (1 + pair.abs().max().item() if n else 1) * 2 + 1e-4          # times the other factor; __expf
+        err = (out[g * cap:g * cap + n].double() - ref).abs()
+        assert bool((err <= ref.abs() * 2 ** -8 + tol).all()), (g, err.max().item())
+
+
+@pytest.mark.parametrize("T,E,topk", [(1, 8, 2), (5, 64, 8), (129, 16, 1), (4096, 8, 2), (4099, 12, 3)])
+def test_router_and_plan(T, E, topk):
+    """Router forms on both sides of their limit, uneven expert counts, and the plan's positions in entry order."""
+    from roc_shmem_b200.baseline.moe import route
+    from roc_shmem_b200.ops.moe import moe_lib
+    torch.manual_seed(T + E)
+    lib, H = moe_lib(), 264
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    wr = torch.randn(E, H, device="cuda").to(torch.bfloat16)
+    n = T * topk
+    idx = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    w = torch.empty(n, dtype=torch.float32, device="cuda")
+    probs = torch.empty(T, E, dtype=torch.float32, device="cuda")
+    pos, cnt = torch.empty_like(idx), torch.empty(E, dtype=torch.int32, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib.bshmem_moe_router_topk(x.data_ptr(), wr.data_ptr(), T, H, E, topk, idx.data_ptr(), w.data_ptr(), probs.data_ptr(), s) == 0
+    assert lib.bshmem_moe_plan(idx.data_ptr(), n, E, pos.data_ptr(), cnt.data_ptr(), s) == 0
+    torch.cuda.synchronize()
+    ridx, rw = route(x, wr, topk)
+    same = (idx.view(T, topk).long() == ridx).all(-1)
+    assert same.float().mean() > 0.99                                                # fp32 order may flip near-ties
+    assert torch.allclose(w.view(T, topk)[same], rw[same], atol=2e-3)
+    assert torch.allclose(probs.sum(-1), torch.ones(T, device="cuda"), atol=1e-5)
+    flat, p = idx.tolist(), pos.tolist()
+    seen = [0] * E
+    for i, e in enumerate(flat):
+        assert p[i] == seen[e]
+        seen[e] += 1
+    assert cnt.tolist() == seen
