@@ -70,6 +70,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ float ld_cluster_f1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
@@ -264,6 +269,8 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
 // Gated: the weight rows are 32 gate rows followed by the matching 32 up rows, i.e. alternating quarters of the tensor
 // memory; the up warps hand their values to the gate warps through shared memory, 16 tokens at a time, and the gate warps
 // write silu(gate) * up.
+// Split (few active groups with few weight rows): as in the dense form, a cluster shares one tile and adds its parts
+// through distributed shared memory; a CTA has no second tile then.
 namespace bshmem {
 namespace skinny {
 
@@ -281,6 +288,7 @@ struct GroupedParams {
   uint32_t ring_bytes;           // shared memory of the stages
   uint32_t tmem_cols;            // two accumulators
   int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 256)
+  int split;                     // > 1: clusters of that many CTAs share the reduction of a tile, one tile per cluster
   int P;                         // arrival words to wait for before the first token load (0: none)
   const unsigned long long* arrive;
   const int* expected;
@@ -359,8 +367,16 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   const int nt_max = min((most + 15) / 16 * 16, p.nt_cap);
   const uint32_t stage = W_STAGE_BYTES + (uint32_t)nt_max * BK * 2;
   const int stages = min((int)(p.ring_bytes / stage), MAX_GROUP_STAGES);
-  const int num_kb = (p.K + BK - 1) / BK;
-  GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x, (int)gridDim.x, 0, 0};
+  const int kb_all = (p.K + BK - 1) / BK;
+  const int rank = p.split > 1 ? (int)cluster_rank() : 0;
+  const int kb0 = kb_all * rank / p.split, kb1 = kb_all * (rank + 1) / p.split;
+  GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x / p.split, (int)gridDim.x / p.split, 0, 0};
+  struct { int grp, n_blk, tok0, ntok; } split_tile = {0, 0, 0, 0};
+  bool mine = false;                                 // split form: there is a tile for this cluster
+  if (p.split > 1) {
+    GroupedTiles probe = it;
+    mine = probe.next(&split_tile.grp, &split_tile.n_blk, &split_tile.tok0, &split_tile.ntok);
+  }
   int grp, n_blk, tok0, ntok;
 
   if (warp == 0) {
@@ -371,7 +387,7 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
       if (p.P) ptx::fence_proxy_async_all();         // peer stores (generic proxy) before the TMA reads
       while (ok && it.next(&grp, &n_blk, &tok0, &ntok)) {
         const int boxes = (ntok + XBOX - 1) / XBOX;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_G_PRODUCER_EMPTY)) { ok = false; break; }
           const uint32_t w = L.base + s * stage, x = w + W_STAGE_BYTES;
           ptx::mbar_arrive_expect_tx(L.full(s), W_STAGE_BYTES + boxes * (XBOX * BK * 2));
@@ -394,12 +410,12 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
         ptx::tc_fence_after();
         const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)((ntok + 15) / 16 * 16));
         const uint32_t d = tmem + acc * p.nt_cap;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(L.full(s), ph, g, ERR_G_MMA_FULL)) { ok = false; break; }
           ptx::tc_fence_after();
           const uint64_t dw = ptx::umma_desc_sw128(L.base + s * stage), dx = ptx::umma_desc_sw128(L.base + s * stage + W_STAGE_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(d, dw + 2 * k, dx + 2 * k, idesc, (kb || k) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(d, dw + 2 * k, dx + 2 * k, idesc, (kb > kb0 || k) ? 1u : 0u);
           ptx::umma_commit(L.empty(s));
           if (++s == stages) { s = 0; ph ^= 1; }
         }
@@ -426,6 +442,18 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
       acc_ph ^= 1u << acc;
       ptx::tc_fence_after();
       const uint32_t taddr = lanes + acc * p.nt_cap;
+      if (p.split > 1) {
+        // [token][weight row] floats over the drained stages
+        const uint32_t dst = L.base + (quarter * 32 + lane) * 4;
+        for (int c = 0; c < ntok; c += 16) {
+          uint32_t v[16];
+          ptx::tmem_ld_32x32b_x16(taddr + c, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (c + j) * (ROWS * 4)), "r"(v[j]) : "memory");
+        }
+        break;
+      }
       __nv_bfloat16* out = p.out + ((long long)grp * p.cap + tok0) * p.ldo + (kGated ? n_blk * (ROWS / 2) + (quarter >> 1) * 32 : n_blk * ROWS + quarter * 32) + lane;
       for (int c = 0; c < ntok; c += 16) {
         uint32_t v[16];
@@ -462,6 +490,32 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if (p.split > 1) {
+    cluster_sync();
+    if (mine && !*L.abort_flag()) {
+      // one warp per token; a lane's sum over the parts of weight row r of token t
+      auto sum = [&](int t, int r) {
+        float f = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < p.split; ++q) f += ld_cluster_f1(map_rank(L.base + (t * ROWS + r) * 4, q));
+        return f;
+      };
+      for (int t = rank + warp * p.split; t < split_tile.ntok; t += p.split * (NUM_THREADS / 32)) {
+        __nv_bfloat16* out = p.out + ((long long)split_tile.grp * p.cap + split_tile.tok0 + t) * p.ldo;
+        if constexpr (kGated) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float gate = sum(t, h * 64 + lane), u = sum(t, h * 64 + 32 + lane);
+            out[split_tile.n_blk * (ROWS / 2) + h * 32 + lane] = __float2bfloat16_rn(gate / (1.f + __expf(-gate)) * u);
+          }
+        } else {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) out[split_tile.n_blk * ROWS + h * 32 + lane] = __float2bfloat16_rn(sum(t, h * 32 + lane));
+        }
+      }
+    }
+    cluster_sync();                                  // nobody's shared memory goes away while it is being read
+  }
   if (*L.abort_flag()) {
     const unsigned long long t0 = ptx::globaltimer();
     while (ptx::globaltimer() - t0 < 2000000ull) __nanosleep(1000);

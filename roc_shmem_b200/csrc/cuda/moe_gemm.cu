@@ -357,12 +357,16 @@ int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, in
   p.G = G; p.cap = a_rows_per_group; p.N = N; p.K = K;
   if (max_rows > a_rows_per_group) max_rows = a_rows_per_group;
   p.nt_cap = max_rows >= 128 ? 128 : (max_rows + 15) / 16 * 16;
-  // Two CTAs per SM, except where the tiles cannot occupy more than one: then that one gets all the stages (two groups with
-  // one row, N x K = 4096 x 14336: 64 CTAs with half the shared memory stream at 45 GB/s each).
+  // Two CTAs per SM.  An SM does not get more than about 45 GB/s out of HBM however many stages it keeps in flight, so
+  // where the tiles cannot occupy the chip (two groups with one row, N x K = 4096 x 14336: 64 tiles, 2.1 TB/s) each is
+  // split over a cluster while at least eight k-blocks remain per CTA.
   if (max_active < 1 || max_active > G) max_active = G;
-  const bool half = (long long)max_active * (N / skinny::ROWS) * ((max_rows + p.nt_cap - 1) / p.nt_cap) > g_sms[dev];
+  const long long tiles = (long long)max_active * (N / skinny::ROWS) * ((max_rows + p.nt_cap - 1) / p.nt_cap);
+  const int kb = (K + skinny::BK - 1) / skinny::BK;
+  p.split = 1;
+  while (p.split < 8 && tiles * p.split <= g_sms[dev] && kb >= 16 * p.split) p.split *= 2;
   const uint32_t fixed = 1024 + skinny::GROUP_CTRL_BYTES + (gated ? skinny::GROUP_XCHG_BYTES : 0);
-  p.ring_bytes = ((half ? skinny::SMEM_HALF : skinny::SMEM_FULL) - fixed) & ~1023u;
+  p.ring_bytes = (skinny::SMEM_HALF - fixed) & ~1023u;          // also holds a split tile's 512 bytes per token
   p.tmem_cols = 32;
   while (p.tmem_cols < 2u * p.nt_cap) p.tmem_cols *= 2;
   p.P = P; p.arrive = static_cast<const unsigned long long*>(arrive); p.expected = expected;
@@ -373,15 +377,17 @@ int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, in
   rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, skinny::XBOX, skinny::BK);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(g_sms[dev] * (half ? 2 : 1)));
+  cfg.gridDim = dim3((unsigned)(p.split > 1 ? tiles * p.split : 2 * g_sms[dev]));
   cfg.blockDim = dim3(skinny::NUM_THREADS);
   cfg.dynamicSmemBytes = p.ring_bytes + fixed;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
   BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, gated ? grouped_gemm_few_kernel<true> : grouped_gemm_few_kernel<false>, p));
   return 0;
 }

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("gated", [False, True])
 @pytest.mark.parametrize("rows", [[0, 0, 1], [16, 17, 0], [127, 128, 129], [256, 3, 0], [0, 250, 15]])
-@pytest.mark.parametrize("N,K", [(256, 64), (512, 1000), (2048, 2048)])
+@pytest.mark.parametrize("N,K", [(256, 64), (512, 1000), (512, 8192), (2048, 2048), (9472, 1024)])
 def test_grouped_gemm_few_rows(rows, gated, N, K):
     from roc_shmem_b200.ops.moe import grouped_gemm, moe_lib
     torch.manual_seed(sum(rows) + N)
