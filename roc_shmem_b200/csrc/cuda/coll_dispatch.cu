@@ -30,13 +30,13 @@ cudaError_t launch(const State& s, const DTeam& t, const CollArgs& a, int ctas, 
 }
 
 cudaError_t launch_group(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, const GroupDone& done) {
   switch (unit_of(a)) {
-    case U_MOVE: return launch_group_move(states, teams, a, ctas, n, status, stream);
-    case U_F32: return launch_group_f32(states, teams, a, ctas, n, status, stream);
-    case U_F16: return launch_group_f16(states, teams, a, ctas, n, status, stream);
-    case U_I32: return launch_group_i32(states, teams, a, ctas, n, status, stream);
-    case U_I8: return launch_group_i8(states, teams, a, ctas, n, status, stream);
+    case U_MOVE: return launch_group_move(states, teams, a, ctas, n, status, stream, done);
+    case U_F32: return launch_group_f32(states, teams, a, ctas, n, status, stream, done);
+    case U_F16: return launch_group_f16(states, teams, a, ctas, n, status, stream, done);
+    case U_I32: return launch_group_i32(states, teams, a, ctas, n, status, stream, done);
+    case U_I8: return launch_group_i8(states, teams, a, ctas, n, status, stream, done);
     default: return cudaErrorInvalidValue;
   }
 }

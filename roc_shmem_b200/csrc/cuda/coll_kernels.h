@@ -51,16 +51,24 @@ inline void extent(int kind, int dtype, uint64_t count, int team_size, uint64_t*
 
 // One PE: `ctas` blocks on `stream`; a non-zero device status lands in *status (first one wins).
 cudaError_t launch(const State& s, const DTeam& t, const CollArgs& a, int ctas, int* status, cudaStream_t stream);
+// How a group launch tells the host that all of its blocks are done: a pinned word that receives `token`, and a device
+// counter (zero, and zero again afterwards).  word == null: the caller synchronises the stream instead.
+struct GroupDone {
+  unsigned int* count = nullptr;
+  uint64_t* word = nullptr;
+  uint64_t token = 0;
+};
 // All PEs of a local group at once: states / teams are device arrays of n entries (a team with my_idx < 0 sits out).
 cudaError_t launch_group(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status,
-                         cudaStream_t stream);
+                         cudaStream_t stream, const GroupDone& done = GroupDone());
 // Loads every kernel module now (a lazy first load from another thread could need a device-wide quiet point).
 void preload();
 
 // per element class (defined by coll_kernels_impl.cuh in each unit)
 #define BSHMEM_COLL_UNIT(name)                                                                                          \
   cudaError_t launch_##name(const State&, const DTeam&, const CollArgs&, int, int*, cudaStream_t);                       \
-  cudaError_t launch_group_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t);           \
+  cudaError_t launch_group_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t,             \
+                                  const GroupDone&);                                                                     \
   void preload_##name();
 BSHMEM_COLL_UNIT(move)
 BSHMEM_COLL_UNIT(f32)

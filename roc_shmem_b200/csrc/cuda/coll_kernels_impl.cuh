@@ -99,13 +99,30 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_, COLL_UNIT)(State s
 
 // All PEs of a local group in ONE cooperative launch: blockIdx.y is the PE.  Used to exercise the multi-PE
 // algorithms on a single GPU (kernels that wait on one another must not be separate launches on one device).
+// The block works on a copy of its PE's state in shared memory (a private copy is 220 bytes of local memory per thread).
 __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(const State* states, const DTeam* teams,
-                                                                                CollArgs a, int* status) {
-  State s = states[blockIdx.y];
-  DTeam t = teams[blockIdx.y];
-  if (t.my_idx < 0) return;
-  int rc = run_coll(s, t, a, blockIdx.x, gridDim.x);
-  if (rc != BSHMEM_OK && threadIdx.x == 0) atomicCAS(status, 0, rc);
+                                                                                CollArgs a, int* status, GroupDone done) {
+  static_assert(sizeof(State) % 4 == 0, "copied in words");
+  __shared__ State s;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(states + blockIdx.y);
+  for (unsigned i = threadIdx.x; i < sizeof(State) / 4; i += kThreads) reinterpret_cast<uint32_t*>(&s)[i] = src[i];
+  const DTeam t = teams[blockIdx.y];
+  __syncthreads();
+  if (t.my_idx >= 0) {
+    const int rc = run_coll(s, t, a, blockIdx.x, gridDim.x);
+    if (rc != BSHMEM_OK && threadIdx.x == 0) atomicCAS(status, 0, rc);
+  }
+  if (done.word == nullptr) return;
+  // the last block to get here tells the host; the count is back at zero then
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    const unsigned n = gridDim.x * gridDim.y;
+    if (atomicInc(done.count, n - 1) == n - 1) {
+      __threadfence_system();
+      asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(done.word), "l"(done.token) : "memory");
+    }
+  }
 }
 
 }  // namespace
@@ -116,9 +133,10 @@ cudaError_t COLL_CAT(launch_, COLL_UNIT)(const State& s, const DTeam& t, const C
 }
 
 cudaError_t COLL_CAT(launch_group_, COLL_UNIT)(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n,
-                                               int* status, cudaStream_t stream) {
+                                               int* status, cudaStream_t stream, const GroupDone& done) {
   CollArgs args_copy = a;
-  void* args[] = {&states, &teams, &args_copy, &status};
+  GroupDone done_copy = done;
+  void* args[] = {&states, &teams, &args_copy, &status, &done_copy};
   return cudaLaunchCooperativeKernel((void*)COLL_CAT(k_coll_group_, COLL_UNIT), dim3(ctas, n), dim3(kThreads), args, kDynSmem, stream);
 }
 

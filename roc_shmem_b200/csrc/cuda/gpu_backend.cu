@@ -17,6 +17,7 @@
 
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 
 #include "../host/backend.h"
@@ -287,6 +288,7 @@ class GpuBackend final : public Backend {
     cudaDeviceSynchronize();
     for (int i = 1; i < BSHMEM_MAX_CTXS; ++i) ctx_close(i);
     if (own_stream_) cudaStreamDestroy(own_stream_);
+    if (group_dev_) cudaFree(group_dev_);
     if (dstats_) cudaFree(dstats_);
     if (dstatus_) cudaFree(dstatus_);
     if (pinned_) cudaFreeHost(pinned_);
@@ -680,7 +682,46 @@ class GpuBackend final : public Backend {
 
   int* dstatus() const { return dstatus_; }
 
+  // A collective of the local group whose first PE this is.  The PE table stays on the device and is rewritten only when
+  // it differs from the last call's; completion and status come back through pinned words.  (With a table allocated,
+  // copied and freed per call and a synchronous read of the status, the call cost 40 us around a 16 us kernel.)
+  int group_launch(const State* hs, const DTeam* ht, int n, const CollArgs& a, int ctas) {
+    std::lock_guard<std::mutex> lock(group_mu_);
+    if (!group_dev_) {
+      RT_TRY(cudaMalloc(&group_dev_, sizeof(GroupTable) + 16));
+      RT_TRY(cudaMemset(group_dev_, 0, sizeof(GroupTable) + 16));
+      memset(&group_host_, 0, sizeof(group_host_));
+    }
+    GroupTable img;
+    memset(&img, 0, sizeof(img));
+    memcpy(img.states, hs, sizeof(State) * n);
+    memcpy(img.teams, ht, sizeof(DTeam) * n);
+    if (memcmp(&img, &group_host_, sizeof(img)) != 0) {
+      RT_TRY(cudaMemcpyAsync(group_dev_, &img, sizeof(img), cudaMemcpyHostToDevice, stream_));
+      group_host_ = img;
+    }
+    GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
+    const Ticket t = draw(lanes_[0]);
+    int* status = &pinned_->status[t.slot];
+    *status = 0;
+    collk::GroupDone done;
+    done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
+    done.word = t.done.word;
+    done.token = t.done.token;
+    cudaError_t e = collk::launch_group(dev->states, dev->teams, a, ctas, n, status, stream_, done);
+    if (e != cudaSuccess) { tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e); return BSHMEM_ERR_CUDA; }
+    const int rc = wait_done(t, stream_);
+    return rc != BSHMEM_OK ? rc : *status;
+  }
+
  private:
+  struct GroupTable {
+    State states[BSHMEM_MAX_PES];
+    DTeam teams[BSHMEM_MAX_PES];
+  };
+  std::mutex group_mu_;
+  char* group_dev_ = nullptr;           // GroupTable, then the count of finished blocks
+  GroupTable group_host_;               // what group_dev_ holds
   gpu::Heap* heap_;
   bool own_heap_;
   State state_{};
@@ -712,6 +753,7 @@ extern "C" {
 
 const char* bshmem_gpu_last_error(void) {
   if (!g_err.empty()) return g_err.c_str();
+  if (!tl_err.empty()) return tl_err.c_str();
   return gpu::heap_error().c_str();
 }
 
@@ -961,27 +1003,10 @@ int bshmem_gpu_group_collective(bshmem_handle_t* handles, int n, int team_slot, 
     if (src_off > hs[i].heap_bytes || sb > hs[i].heap_bytes - src_off || dst_off > hs[i].heap_bytes || db > hs[i].heap_bytes - dst_off)
       return BSHMEM_ERR_RANGE;
   }
-  State* ds = nullptr;
-  DTeam* dt = nullptr;
-  if (cudaMalloc(&ds, sizeof(State) * n) != cudaSuccess || cudaMalloc(&dt, sizeof(DTeam) * n) != cudaSuccess) return BSHMEM_ERR_CUDA;
-  cudaMemcpy(ds, hs, sizeof(State) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(dt, ht, sizeof(DTeam) * n, cudaMemcpyHostToDevice);
   CollArgs a{};
   a.kind = kind; a.dtype = dtype; a.op = op; a.root = root; a.dst_off = dst_off; a.src_off = src_off; a.n = count;
-  int* status = g0->dstatus();
   if (ctas < 1) ctas = 1;
-  cudaError_t e = collk::launch_group(ds, dt, a, ctas, n, status, g0->stream());
-  int rc = BSHMEM_OK;
-  if (e != cudaSuccess) { g_err = std::string("cooperative launch: ") + cudaGetErrorString(e); rc = BSHMEM_ERR_CUDA; }
-  else if (cudaStreamSynchronize(g0->stream()) != cudaSuccess) rc = BSHMEM_ERR_CUDA;
-  else {
-    int st = 0;
-    cudaMemcpy(&st, status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (st) { cudaMemset(status, 0, sizeof(int)); rc = st; }
-  }
-  cudaFree(ds);
-  cudaFree(dt);
-  return rc;
+  return g0->group_launch(hs, ht, n, a, ctas);
 }
 
 

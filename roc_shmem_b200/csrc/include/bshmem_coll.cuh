@@ -116,9 +116,11 @@ __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta 
   __shared__ int sync_status;
   const int tid = threadIdx.x;
   unsigned long long t0 = s.stats ? dev::timer() : 0;
+  // loads whose answers are needed further down travel while the block gathers and the flags are exchanged
+  const uint64_t epoch = *reinterpret_cast<volatile uint64_t*>(epoch_addr(s, t.slot, cta)) + 1;
+  const unsigned long long cap = tid == 0 ? dev::trace_capacity(s) : 0;
   if (tid == 0) sync_status = BSHMEM_OK;
   __syncthreads();                       // all stores of the block precede the release below
-  uint64_t epoch = *epoch_addr(s, t.slot, cta) + 1;
   if (tid < t.size) {
     // release pattern: one system fence per signalling thread, then the flag.  The block barrier above makes every
     // thread's earlier stores (remote ones included) precede this fence, so they are visible to whoever sees the flag.
@@ -135,7 +137,7 @@ __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta 
     if (s.stats) {
       dev::stat(s, BSHMEM_DSTAT_BARRIER);
       dev::stat(s, BSHMEM_DSTAT_BARRIER_NS, dev::timer() - t0);
-      dev::trace(s, BSHMEM_TRACE_BARRIER, s.my_pe, dev::timer() - t0);
+      dev::trace_with(s, cap, BSHMEM_TRACE_BARRIER, s.my_pe, dev::timer() - t0);
     }
   }
   int rc = sync_status;
@@ -256,16 +258,52 @@ __device__ __forceinline__ void reduce_vec_body(int nsrc, const T* const* srcs, 
 // fetches a chunk of EVERY source with cp.async.bulk (global -> shared, mbarrier completion; sources may be peer
 // memory, nothing is multicast) into a ring of kBulkStages stages, all threads reduce the stage out of shared memory
 // and write the result with ordinary (fire-and-forget) stores to the ndst destinations.
-constexpr int kBulkStages = 3;
-constexpr uint32_t kBulkStageBytes = 48 * 1024;
+// A stage is 32 KiB whatever the number of sources, so that a source's share is a whole number of 16-byte vectors per
+// thread for up to eight sources and 256 threads (with 48 KiB, 1.5 vectors), and four of them leave three on their way
+// while one is reduced.
+constexpr int kBulkStages = 4;
+constexpr uint32_t kBulkStageBytes = 32 * 1024;
 constexpr uint32_t kBulkSmemBytes = kBulkStages * kBulkStageBytes + 64;   // + mbarriers
+// One stage: vectors threadIdx.x, + blockDim.x, ... of every source.  NS > 0: exactly NS sources, all of a vector's
+// shared-memory loads in flight together; NS = 0: nsrc sources, one after the other.
+template <typename T, int OP, int NS>
+__device__ __forceinline__ void reduce_stage(const char* stage, uint32_t chunk, uint32_t nvec, int nsrc, int ndst, T* const* dsts, size_t v_base) {
+  using A = typename Acc<T>::type;
+  constexpr int VE = 16 / sizeof(T);
+  for (uint32_t v = threadIdx.x; v < nvec; v += blockDim.x) {
+    A acc[VE];
+    if constexpr (NS > 0) {
+      Vec16<T> in[NS];
+#pragma unroll
+      for (int k = 0; k < NS; ++k) in[k].raw = *reinterpret_cast<const uint4*>(stage + (size_t)k * chunk + (size_t)v * 16);
+#pragma unroll
+      for (int e = 0; e < VE; ++e) acc[e] = to_acc<T>(in[0].e[e]);
+#pragma unroll
+      for (int k = 1; k < NS; ++k)
+#pragma unroll
+        for (int e = 0; e < VE; ++e) acc[e] = apply<A>(OP, acc[e], to_acc<T>(in[k].e[e]));
+    } else {
+      Vec16<T> in;
+      in.raw = *reinterpret_cast<const uint4*>(stage + (size_t)v * 16);
+#pragma unroll
+      for (int e = 0; e < VE; ++e) acc[e] = to_acc<T>(in.e[e]);
+      for (int k = 1; k < nsrc; ++k) {
+        in.raw = *reinterpret_cast<const uint4*>(stage + (size_t)k * chunk + (size_t)v * 16);
+#pragma unroll
+        for (int e = 0; e < VE; ++e) acc[e] = apply<A>(OP, acc[e], to_acc<T>(in.e[e]));
+      }
+    }
+    Vec16<T> out;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) out.e[e] = from_acc<T>(acc[e]);
+    for (int d = 0; d < ndst; ++d) reinterpret_cast<uint4*>(dsts[d])[v_base + v] = out.raw;
+  }
+}
 // Range [begin, end) in elements, both multiples of 16 / sizeof(T); every pointer 16-byte aligned.  Returns false if
 // a bounded wait ran out (the error record is filled).
 template <typename T, int OP>
 __device__ __forceinline__ bool reduce_bulk(const State& s, int nsrc, const T* const* srcs, int ndst, T* const* dsts, size_t begin,
                                             size_t end, char* smem) {
-  using A = typename Acc<T>::type;
-  constexpr int VE = 16 / sizeof(T);
   __shared__ int bulk_ok;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBulkStages * kBulkStageBytes);
   const uint32_t chunk = (kBulkStageBytes / nsrc) & ~127u;            // bytes per source and stage
@@ -313,20 +351,11 @@ __device__ __forceinline__ bool reduce_bulk(const State& s, int nsrc, const T* c
     const uint32_t nb = (uint32_t)((c + 1) * (size_t)chunk <= bytes ? chunk : bytes - c * (size_t)chunk);
     const char* stage = smem + (size_t)st * kBulkStageBytes;
     const size_t v_base = (begin * sizeof(T) + c * (size_t)chunk) >> 4;          // 16-byte vector index in the tensors
-    for (uint32_t v = threadIdx.x; v < (nb >> 4); v += blockDim.x) {
-      Vec16<T> in, out;
-      in.raw = *reinterpret_cast<const uint4*>(stage + (size_t)v * 16);
-      A acc[VE];
-#pragma unroll
-      for (int e = 0; e < VE; ++e) acc[e] = to_acc<T>(in.e[e]);
-      for (int k = 1; k < nsrc; ++k) {
-        in.raw = *reinterpret_cast<const uint4*>(stage + (size_t)k * chunk + (size_t)v * 16);
-#pragma unroll
-        for (int e = 0; e < VE; ++e) acc[e] = apply<A>(OP, acc[e], to_acc<T>(in.e[e]));
-      }
-#pragma unroll
-      for (int e = 0; e < VE; ++e) out.e[e] = from_acc<T>(acc[e]);
-      for (int d = 0; d < ndst; ++d) reinterpret_cast<uint4*>(dsts[d])[v_base + v] = out.raw;
+    switch (nsrc) {
+      case 2: reduce_stage<T, OP, 2>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
+      case 4: reduce_stage<T, OP, 4>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
+      case 8: reduce_stage<T, OP, 8>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
+      default: reduce_stage<T, OP, 0>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base);
     }
     __syncthreads();                       // the stage has been read by everybody: refill it
     if (threadIdx.x == 0 && c + kBulkStages < nchunks) issue(c + kBulkStages);
@@ -547,6 +576,7 @@ __device__ __forceinline__ int team_reduce(const State& s, const Team& t, int op
     srcs[k] = dev::ptr(s, source, dev::team_pe(t, k));
     dsts[k] = dev::ptr(s, dest, dev::team_pe(t, k));
   }
+  const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);          // every member's source is ready
   if (rc != BSHMEM_OK) return rc;
   constexpr size_t VE = 16 / sizeof(T);
@@ -563,7 +593,7 @@ __device__ __forceinline__ int team_reduce(const State& s, const Team& t, int op
     split_range(se - sb, ncta, cta, VE, &b, &e);
     reduce_range<T>(s, op, t.size, srcs, t.size, dsts, sb + b, sb + e, bulk);
   }
-  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace(s, BSHMEM_TRACE_COLL, s.my_pe, 0); }
+  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);         // results delivered; sources reusable
 }
 
@@ -593,19 +623,21 @@ __device__ __forceinline__ int team_reduce_scatter(const State& s, const Team& t
                                                    size_t n, int cta = 0, int ncta = 1, char* bulk = nullptr) {
   const T* srcs[BSHMEM_MAX_PES];
   for (int k = 0; k < t.size; ++k) srcs[k] = dev::ptr(s, source, dev::team_pe(t, k)) + (size_t)t.my_idx * n;
+  const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);
   if (rc != BSHMEM_OK) return rc;
   size_t b, e;
   split_range(n, ncta, cta, 16 / sizeof(T), &b, &e);
   T* mine[1] = {dest};
   reduce_range<T>(s, op, t.size, srcs, 1, mine, b, e, bulk);
-  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace(s, BSHMEM_TRACE_COLL, s.my_pe, 0); }
+  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);
 }
 
 // broadcast: the root's source lands in every other member's dest (the root's dest is untouched).
 __device__ __forceinline__ int team_broadcast(const State& s, const Team& t, void* dest, const void* source, size_t nbytes,
                                               int root, int cta = 0, int ncta = 1) {
+  const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);
   if (rc != BSHMEM_OK) return rc;
   if (t.my_idx != root) {
@@ -614,13 +646,14 @@ __device__ __forceinline__ int team_broadcast(const State& s, const Team& t, voi
     const char* src = dev::ptr(s, reinterpret_cast<const char*>(source), dev::team_pe(t, root));
     dev::copy_bytes<dev::BLOCK>(reinterpret_cast<char*>(dest) + b, src + b, e - b);
   }
-  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace(s, BSHMEM_TRACE_COLL, s.my_pe, 0); }
+  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);
 }
 
 // fcollect (all-gather): my source lands in block my_idx of every member's dest.
 __device__ __forceinline__ int team_fcollect(const State& s, const Team& t, void* dest, const void* source, size_t nbytes,
                                              int cta = 0, int ncta = 1) {
+  const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);          // every member's dest may be overwritten
   if (rc != BSHMEM_OK) return rc;
   size_t b, e;
@@ -630,13 +663,14 @@ __device__ __forceinline__ int team_fcollect(const State& s, const Team& t, void
     char* d = dev::ptr(s, reinterpret_cast<char*>(dest), dev::team_pe(t, peer_idx)) + (size_t)t.my_idx * nbytes;
     dev::copy_bytes<dev::BLOCK>(d + b, reinterpret_cast<const char*>(source) + b, e - b);
   }
-  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace(s, BSHMEM_TRACE_COLL, s.my_pe, 0); }
+  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);
 }
 
 // alltoall: block j of my source lands in block my_idx of member j's dest.
 __device__ __forceinline__ int team_alltoall(const State& s, const Team& t, void* dest, const void* source, size_t nbytes,
                                              int cta = 0, int ncta = 1) {
+  const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);
   if (rc != BSHMEM_OK) return rc;
   size_t b, e;
@@ -647,7 +681,7 @@ __device__ __forceinline__ int team_alltoall(const State& s, const Team& t, void
     const char* sp = reinterpret_cast<const char*>(source) + (size_t)j * nbytes;
     dev::copy_bytes<dev::BLOCK>(d + b, sp + b, e - b);
   }
-  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace(s, BSHMEM_TRACE_COLL, s.my_pe, 0); }
+  if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);
 }
 

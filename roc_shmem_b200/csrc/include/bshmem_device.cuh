@@ -122,10 +122,13 @@ __device__ __forceinline__ int n_pes(const State& s) { return s.n_pes; }
 __device__ __forceinline__ void stat(const State& s, int idx, unsigned long long by = 1) {
   if (s.stats) atomicAdd(&s.stats[idx], by);
 }
+// Capacity of the event ring, 0 while the host has tracing switched off.  The load takes 0.7 us: whoever traces at the end
+// of something that others wait for issues it at the beginning, so that it returns meanwhile.
+__device__ __forceinline__ unsigned long long trace_capacity(const State& s) {
+  return s.stats ? *reinterpret_cast<volatile unsigned long long*>(&s.stats[BSHMEM_DSTAT_COUNT]) : 0ull;
+}
 // One timeline event (who, what, how much, when); a no-op unless the host switched tracing on.
-__device__ __forceinline__ void trace(const State& s, int op, int pe, unsigned long long bytes) {
-  if (!s.stats) return;
-  const unsigned long long cap = *reinterpret_cast<volatile unsigned long long*>(&s.stats[BSHMEM_DSTAT_COUNT]);
+__device__ __forceinline__ void trace_with(const State& s, unsigned long long cap, int op, int pe, unsigned long long bytes) {
   if (!cap) return;
   const unsigned long long i = atomicAdd(&s.stats[BSHMEM_DSTAT_COUNT + 1], 1ull);
   unsigned long long* e = s.stats + BSHMEM_DSTAT_COUNT + 2 + 4 * (i % cap);
@@ -133,6 +136,9 @@ __device__ __forceinline__ void trace(const State& s, int op, int pe, unsigned l
   e[1] = (unsigned long long)(op & 0xFF) | ((unsigned long long)(pe & 0xFFFFFF) << 8) | ((unsigned long long)blockIdx.x << 32);
   e[2] = bytes;
   e[3] = i;
+}
+__device__ __forceinline__ void trace(const State& s, int op, int pe, unsigned long long bytes) {
+  trace_with(s, trace_capacity(s), op, pe, bytes);
 }
 __device__ __forceinline__ int team_pe(const Team& t, int idx) { return t.pe_start + idx * t.stride; }
 // world PE -> index in team, -1 if not a member
@@ -481,6 +487,7 @@ __device__ __forceinline__ int wait_until(const State& s, const T* ivar, int cmp
   T seen = load_acquire_sys(ivar);
   if (cmp_holds(cmp, seen, value)) return BSHMEM_OK;
   unsigned long long t0 = timer();
+  const unsigned long long cap = trace_capacity(s);
   unsigned it = 0;
   while (true) {
     seen = load_acquire_sys(ivar);
@@ -496,7 +503,7 @@ __device__ __forceinline__ int wait_until(const State& s, const T* ivar, int cmp
       __nanosleep(64);
     }
   }
-  if (s.stats) { stat(s, BSHMEM_DSTAT_WAIT); stat(s, BSHMEM_DSTAT_WAIT_NS, timer() - t0); trace(s, BSHMEM_TRACE_WAIT, s.my_pe, timer() - t0); }
+  if (s.stats) { stat(s, BSHMEM_DSTAT_WAIT); stat(s, BSHMEM_DSTAT_WAIT_NS, timer() - t0); trace_with(s, cap, BSHMEM_TRACE_WAIT, s.my_pe, timer() - t0); }
   return BSHMEM_OK;
 }
 

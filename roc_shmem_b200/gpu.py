@@ -487,6 +487,9 @@ class LocalGroup:
             rt.set_stream(torch.cuda.current_stream())
             self.pes.append(rt)
         self._handles = (C.c_void_p * n_pes)(*[rt.h.value for rt in self.pes])
+        self._handles_a = C.addressof(self._handles)
+        self._base0 = int(self.lib.bshmem_heap_base(self.pes[0].h))
+        self._c_collective = _native.fast(self.lib, "bshmem_gpu_group_collective")
 
     def empty(self, shape, dtype) -> list[torch.Tensor]:
         """The same symmetric allocation on every PE."""
@@ -494,12 +497,12 @@ class LocalGroup:
 
     def collective(self, kind: int, dests, srcs, count: int, *, dtype=None, op: int = 0, root: int = 0,
                    team_slot: int = 0, ctas: int = 2) -> None:
-        d_off = self.pes[0].offset_of(dests[0]) if dests is not None else 0
-        s_off = self.pes[0].offset_of(srcs[0]) if srcs is not None else 0
+        d_off = dests[0].data_ptr() - self._base0 if dests is not None else 0
+        s_off = srcs[0].data_ptr() - self._base0 if srcs is not None else 0
         code = D.code_of(dtype) if dtype is not None else 0
-        st = self.lib.bshmem_gpu_group_collective(self._handles, self.n_pes, team_slot, kind, code, op, root, d_off, s_off,
-                                                  count, ctas)
-        _gpu_error(self.lib, "group_collective", st)
+        st = self._c_collective(self._handles_a, self.n_pes, team_slot, kind, code, op, root, d_off, s_off, count, ctas)
+        if st:
+            _gpu_error(self.lib, "group_collective", st)
 
     def team_split(self, parent_slot: int, start: int, stride: int, size: int) -> list[int]:
         out = (C.c_int * self.n_pes)()
