@@ -127,11 +127,11 @@ __device__ __forceinline__ void umma2_commit_both(uint32_t bar, uint32_t lead) {
 
 // Host side: how many clusters of `size` CTAs of `kernel` the device can hold at once (one CTA per SM).
 template <class Kernel>
-inline int max_resident_clusters(Kernel kernel, int sms, int size) {
+inline int max_resident_clusters(Kernel kernel, int sms, int size, int threads = NUM_THREADS, uint32_t smem = SMEM_BYTES) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(sms / size * size), 1, 1);
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -207,6 +207,11 @@ struct PolicyDefaults {
   // the matching up-projections; the epilogue writes silu(gate) * up, i.e. half as many output columns (the two
   // chunks of a warp make one 32 x 64 output box; out_target gets the OUTPUT column).
   static constexpr bool kGated = false;
+  // Training forms of the gated MLP, on the plain epilogue (the accumulator's columns are stored as they are or replaced):
+  // kStoreAct: store_act() additionally gets every chunk (32 gate, 32 up) before it is stored, to write silu(gate) * up.
+  // kSwigluBwd: the accumulator is the gradient of the activations; each 32 columns of it become 64 columns of output, the
+  // gradients of the matching gate and up pre-activations (swiglu_grad), and out_target gets the output column.
+  static constexpr bool kStoreAct = false, kSwigluBwd = false;
   // Operand layout.  Default: both operands K-major, one 128-row x 128-byte TMA box per operand, CTA and stage, and
   // shared-memory descriptors that step 32 bytes along K inside the swizzle atom.  A policy with MN-major operands
   // overrides the instruction descriptor, the stage-0 descriptors, the step per MMA and the loads.
@@ -243,6 +248,21 @@ struct PolicyDefaults {
   template <class Params> __device__ static __forceinline__ void tail(const Params&, const Smem&, Guard&) {}
   template <class Params> __device__ static __forceinline__ void prologue(const Params&, Guard&) {}
 };
+
+// Parks 64 bf16 columns of the warp's 32 rows (row = lane) in its staging buffer for a TMA store: eight 16-byte pieces per
+// row, piece j at (j ^ (row & 7)) under the 128-byte swizzle.
+__device__ __forceinline__ void stage_chunk(uint32_t buf, int lane, const float (&f)[64]) {
+  const uint32_t rowbase = buf + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t w0 = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]), w1 = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
+    const uint32_t w2 = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]), w3 = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
+    const uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
 
 // 64 accumulator columns of this warp's 32 rows (row = lane).
 __device__ __forceinline__ void load_acc_chunk(uint32_t taddr, float (&f)[64]) {
@@ -466,20 +486,30 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           __syncwarp();
           Chunk cc = ck;
           cc.col0 = ck.col0 + c * EPI_COLS;
-          P::adjust(prm, L, st, cc, f, ew, lane);
-          // row = lane; 8 x 16-byte pieces, piece j lives at (j ^ (row & 7)) under the 128-byte swizzle
-          const uint32_t rowbase = L.epi(ew) + lane * 128;
+          if constexpr (P::kSwigluBwd) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              float d[32], o[64];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            uint32_t w0 = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]);
-            uint32_t w1 = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
-            uint32_t w2 = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]);
-            uint32_t w3 = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
-            uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+              for (int i = 0; i < 32; ++i) d[i] = h == 0 ? f[i] : f[32 + i];
+              P::swiglu_grad(prm, cc.row0 + lane, cc.col0 + 32 * h, d, o);
+              if (h == 1) {                  // the first half's store has read the staging buffer
+                if (lane == 0) ptx::tma_wait_group_read<0>();
+                __syncwarp();
+              }
+              stage_chunk(L.epi(ew), lane, o);
+              if (lane == 0) {
+                const CUtensorMap* map; int x, y;
+                P::out_target(prm, cc.row0, 2 * (cc.col0 + 32 * h), &map, &x, &y);
+                if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
+                ptx::tma_commit_group();
+              }
+            }
+            continue;
           }
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
+          P::adjust(prm, L, st, cc, f, ew, lane);
+          if constexpr (P::kStoreAct) P::store_act(prm, cc.row0 + lane, cc.col0, f);
+          stage_chunk(L.epi(ew), lane, f);
           if (lane == 0) {
             const CUtensorMap* map; int x, y;
             P::out_target(prm, cc.row0, cc.col0, &map, &x, &y);

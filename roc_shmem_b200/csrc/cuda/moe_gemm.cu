@@ -40,6 +40,10 @@ struct GroupedParams {
   int P;                           // arrival wait: number of words, 0 = no wait
   const unsigned long long* arrive;
   const int* expected;
+  __nv_bfloat16* act;              // training forward: activations [G * rows, N / 2] next to the pre-activations C
+  long long ld_act;
+  const __nv_bfloat16* gu;         // SwiGLU backward: saved pre-activations [G * rows, 2 N]
+  long long ld_gu;
 };
 
 template <bool kGatedEpi>
@@ -183,6 +187,60 @@ struct GroupedPair : g2::PolicyDefaults {
   }
 };
 
+// Training forward of the gated MLP: C keeps the interleaved gate / up pre-activations for the backward pass, and the
+// activations silu(gate) * up are written in the same epilogue, from the rounded values that C holds (a pass of its own
+// over C reads 2 and writes 1 of the 3 x 940 MB at 32768 rows x 14336: 440 us).  A lane owns a row: 64 consecutive bytes.
+struct GroupedPairAct : GroupedPair<false> {
+  static constexpr bool kStoreAct = true;
+  __device__ static __forceinline__ void store_act(const Params& p, int row, int col, const float (&f)[64]) {
+    uint4* dst = reinterpret_cast<uint4*>(p.act + row * p.ld_act + col / 2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float h[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float gate = __bfloat162float(__float2bfloat16_rn(f[j * 8 + 2 * q + e])), up = __bfloat162float(__float2bfloat16_rn(f[32 + j * 8 + 2 * q + e]));
+          h[e] = gate / (1.f + __expf(-gate)) * up;
+        }
+        w[q] = pack_bf16(h[0], h[1]);
+      }
+      dst[j] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+};
+
+// Backward through the activations: the accumulator is d_h = d_y · W2; the epilogue reads the saved pre-activations and
+// writes the gradients of the gate / up pre-activations, so that d_h never goes to memory (written and read again it was
+// 1.9 of the 4.7 GB that the separate pass moved in 700 us).
+struct GroupedPairSwigluBwd : GroupedPair<false> {
+  static constexpr bool kSwigluBwd = true;
+  __device__ static __forceinline__ void swiglu_grad(const Params& p, int row, int col, const float (&d)[32], float (&o)[64]) {
+    const uint4* src = reinterpret_cast<const uint4*>(p.gu + row * p.ld_gu + 2 * col);
+    uint4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = src[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
+      const __nv_bfloat162* uh = reinterpret_cast<const __nv_bfloat162*>(&v[4 + j]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 gf = __bfloat1622float2(gh[q]), uf = __bfloat1622float2(uh[q]);
+        const float dx = __bfloat162float(__float2bfloat16_rn(d[j * 8 + 2 * q])), dy = __bfloat162float(__float2bfloat16_rn(d[j * 8 + 2 * q + 1]));
+        const float sx = 1.f / (1.f + __expf(-gf.x)), sy = 1.f / (1.f + __expf(-gf.y));
+        // d silu(g)/dg = s * (1 + g * (1 - s))
+        o[j * 8 + 2 * q] = dx * uf.x * sx * (1.f + gf.x * (1.f - sx));
+        o[j * 8 + 2 * q + 1] = dy * uf.y * sy * (1.f + gf.y * (1.f - sy));
+        o[32 + j * 8 + 2 * q] = dx * (gf.x * sx);
+        o[32 + j * 8 + 2 * q + 1] = dy * (gf.y * sy);
+      }
+    }
+  }
+};
+
 // Weight-gradient flavour on CTA pairs: both operands MN-major (token-major activations as they are), ragged
 // reduction over the group's tokens.  Per CTA and stage, each operand is two 64-wide MN blocks of 64 tokens (8 KiB per
 // block, 128-byte swizzle), i.e. the CTA's 128 of the tile's 256 rows / columns.
@@ -226,6 +284,16 @@ grouped_gemm_pair_gated_kernel(const __grid_constant__ GroupedParams prm) {
   g2::gemm_mainloop<GroupedPair<true>>(prm, smem_raw);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
+grouped_gemm_pair_act_kernel(const __grid_constant__ GroupedParams prm) {
+  extern __shared__ uint8_t smem_raw[];
+  g2::gemm_mainloop<GroupedPairAct>(prm, smem_raw);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
+grouped_gemm_pair_swiglu_bwd_kernel(const __grid_constant__ GroupedParams prm) {
+  extern __shared__ uint8_t smem_raw[];
+  g2::gemm_mainloop<GroupedPairSwigluBwd>(prm, smem_raw);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
 grouped_gemm_pair_tn_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
   g2::gemm_mainloop<GroupedPairTN>(prm, smem_raw);
@@ -266,10 +334,30 @@ int ensure(int dev) {
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_swiglu_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
   g_pairs[dev] = g2::max_resident_pairs(grouped_gemm_pair_kernel, g_sms[dev]);
+  return 0;
+}
+
+enum RowsForm { ROWS_PLAIN, ROWS_GATED, ROWS_ACT, ROWS_SWIGLU_BWD };
+
+// A launch of the CTA-pair kernels that may overlap the tail of the stream's previous kernel.
+int launch_pairs(void (*kernel)(GroupedParams), const GroupedParams& p, int pairs, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pairs));
+  cfg.blockDim = dim3(g2::NUM_THREADS);
+  cfg.dynamicSmemBytes = g2::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
   return 0;
 }
 
@@ -284,9 +372,10 @@ const char* bshmem_moe_gemm_last_error() { return host::last_error().c_str(); }
 //   klen_dev   per-group reduction lengths on the device, or null → K
 //   gated      1: accumulator columns are interleaved gate/up, C gets N/2 columns of silu(gate)*up
 //   arrive/expected/P  optional arrival words to wait for before the first load (P = 0: none)
-int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_rows_per_group, int b_rows_per_group, int N, int K,
-                            int lda, int ldb, int ldc, const int* rows_dev, int fixed_rows, const int* klen_dev, int gated,
-                            const void* arrive, const int* expected, int P, void* stream, int timeout_ms, int max_ctas) {
+static int grouped_gemm_rows(RowsForm form, const void* A, const void* B, void* C, int G, int a_rows_per_group, int b_rows_per_group, int N,
+                             int K, int lda, int ldb, int ldc, const int* rows_dev, int fixed_rows, const int* klen_dev, const void* arrive,
+                             const int* expected, int P, void* stream, int timeout_ms, int max_ctas, void* act, int ld_act, const void* gu,
+                             int ld_gu) {
   if (G < 1 || a_rows_per_group % BM || N % BN || K % 8 || lda % 8 || ldb % 8 || ldc % 8) {
     host::last_error() = "grouped gemm: needs rows-per-group % 256 == 0, N % 256 == 0, K and leading dimensions % 8 == 0";
     return 1;
@@ -309,20 +398,25 @@ int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_
   p.P = P; p.arrive = static_cast<const unsigned long long*>(arrive); p.expected = expected;
   // K-major rows mode with a uniform reduction length: CTA pairs; a ragged reduction length (legacy weight-gradient
   // form on transposed copies) stays on the single-CTA loop
-  const bool pair = klen_dev == nullptr && g_pairs[dev] > 0;
+  const bool pair = klen_dev == nullptr && g_pairs[dev] > 0, gated = form == ROWS_GATED;
+  if (!pair && (form == ROWS_ACT || form == ROWS_SWIGLU_BWD)) { host::last_error() = "grouped gemm: this form needs CTA pairs"; return 1; }
+  p.act = static_cast<__nv_bfloat16*>(act); p.ld_act = ld_act;
+  p.gu = static_cast<const __nv_bfloat16*>(gu); p.ld_gu = ld_gu;
   const int box_rows_a = pair ? g2::CTA_M : BM, box_rows_b = pair ? g2::CTA_NLOAD : BN;
   rc = host::make_tmap_2d(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, box_rows_a, 64);
   if (rc) return rc;
   rc = host::make_tmap_2d(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, (uint64_t)G * b_rows_per_group, K, ldb, box_rows_b, 64);
   if (rc) return rc;
-  rc = host::make_tmap_2d(&p.map_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, C, (uint64_t)G * a_rows_per_group, gated ? N / 2 : N, ldc, 32, EPI_COLS);
+  rc = host::make_tmap_2d(&p.map_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, C, (uint64_t)G * a_rows_per_group,
+                          form == ROWS_GATED ? N / 2 : form == ROWS_SWIGLU_BWD ? 2 * N : N, ldc, 32, EPI_COLS);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (pair) {
     int pairs = g_pairs[dev];
     if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-    if (gated) grouped_gemm_pair_gated_kernel<<<2 * pairs, g2::NUM_THREADS, g2::SMEM_BYTES, st>>>(p);
-    else grouped_gemm_pair_kernel<<<2 * pairs, g2::NUM_THREADS, g2::SMEM_BYTES, st>>>(p);
+    constexpr void (*kernels[])(GroupedParams) = {grouped_gemm_pair_kernel, grouped_gemm_pair_gated_kernel, grouped_gemm_pair_act_kernel,
+                                                  grouped_gemm_pair_swiglu_bwd_kernel};
+    return launch_pairs(kernels[form], p, pairs, st);
   } else {
     int ctas = g_sms[dev];
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
@@ -331,6 +425,33 @@ int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_
   }
   BSHMEM_CUDA_TRY(cudaGetLastError());
   return 0;
+}
+
+int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_rows_per_group, int b_rows_per_group, int N, int K,
+                            int lda, int ldb, int ldc, const int* rows_dev, int fixed_rows, const int* klen_dev, int gated,
+                            const void* arrive, const int* expected, int P, void* stream, int timeout_ms, int max_ctas) {
+  return grouped_gemm_rows(gated ? ROWS_GATED : ROWS_PLAIN, A, B, C, G, a_rows_per_group, b_rows_per_group, N, K, lda, ldb, ldc, rows_dev,
+                           fixed_rows, klen_dev, arrive, expected, P, stream, timeout_ms, max_ctas, nullptr, 0, nullptr, 0);
+}
+
+// Training forward of the gated MLP: C [G * a_rows_per_group, N] keeps the interleaved gate / up pre-activations, act
+// [.., N / 2] (ld_act % 8 == 0) gets silu(gate) * up.
+int bshmem_moe_grouped_gemm_act(const void* A, const void* B, void* C, void* act, int G, int a_rows_per_group, int N, int K, int lda, int ldb,
+                                int ldc, int ld_act, const int* rows_dev, const void* arrive, const int* expected, int P, void* stream,
+                                int timeout_ms) {
+  if (!act || ld_act % 8) { host::last_error() = "grouped gemm (act): needs an activation buffer, leading dimension % 8 == 0"; return 1; }
+  return grouped_gemm_rows(ROWS_ACT, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, 0, nullptr, arrive, expected, P, stream,
+                           timeout_ms, 0, act, ld_act, nullptr, 0);
+}
+
+// Backward of the same: d_h = A · B^T (N columns) goes through SwiGLU's derivative at the saved pre-activations gu
+// [.., 2 N] (ld_gu % 8 == 0); C [.., 2 N] gets their gradients.
+int bshmem_moe_grouped_gemm_swiglu_bwd(const void* A, const void* B, const void* gu, void* C, int G, int a_rows_per_group, int N, int K,
+                                       int lda, int ldb, int ld_gu, int ldc, const int* rows_dev, const void* arrive, const int* expected,
+                                       int P, void* stream, int timeout_ms) {
+  if (!gu || ld_gu % 8) { host::last_error() = "grouped gemm (swiglu): needs the pre-activations, leading dimension % 8 == 0"; return 1; }
+  return grouped_gemm_rows(ROWS_SWIGLU_BWD, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, 0, nullptr, arrive, expected, P,
+                           stream, timeout_ms, 0, nullptr, 0, gu, ld_gu);
 }
 
 // The same product for few rows per group (up to about 128; more are taken in chunks of 128, reading the weights again).
@@ -439,7 +560,7 @@ int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int
   if (pair) {
     int pairs = g_pairs[dev];
     if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-    grouped_gemm_pair_tn_kernel<<<2 * pairs, g2::NUM_THREADS, g2::SMEM_BYTES, st>>>(p);
+    return launch_pairs(grouped_gemm_pair_tn_kernel, p, pairs, st);
   } else {
     int ctas = g_sms[dev];
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;

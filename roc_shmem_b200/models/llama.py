@@ -16,7 +16,9 @@ from typing import Optional
 
 import torch
 
-from ..ops.moe import grouped_gemm_tn, interleave_gate_up, moe_lib
+from ..ops.gemm import current_stream, gemm_bf16
+from ..ops.moe import _fast as moe_fast
+from ..ops.moe import (grouped_gemm, grouped_gemm_act, grouped_gemm_swiglu_bwd, grouped_gemm_tn, interleave_gate_up, moe_lib)
 from ..parallel.tp import ColumnParallelLinear, RowParallelLinear
 
 
@@ -67,28 +69,61 @@ class LlamaMLP:
             raise RuntimeError(f"{what} failed ({st}): {self.lib.bshmem_moe_last_error().decode()}")
 
     # ---- forward / backward ------------------------------------------------------------------
+    def _fills(self, cols: int) -> bool:
+        """Whether 256x256 tiles of [tokens, cols] occupy at least half of the CTA pairs.  With fewer, the plain GEMM (which
+        splits a tile over a cluster) and a separate SwiGLU pass are faster than the one fused kernel."""
+        return self.M * cols >= 37 * 256 * 256
+
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
-        s = torch.cuda.current_stream().cuda_stream
-        self.up(x_shard)
-        self._chk(self.lib.bshmem_moe_swiglu_fwd(self.gu.data_ptr(), self.rows.data_ptr(), 1, self.M, self.Fp, self.h.data_ptr(), s),
-                  "swiglu")
+        s = current_stream()
+        if self.P == 1 and self._fills(2 * self.Fp):
+            # one PE: nothing to gather, SwiGLU happens in the projection's epilogue
+            if self.training:
+                if x_shard.data_ptr() != self.up.x_shard.data_ptr():
+                    self.up.x_shard.copy_(x_shard)               # the weight gradient reads it
+                grouped_gemm_act(self.up.gathered, self.w13, self.gu, self.h, 1)
+            else:
+                grouped_gemm(self._operand(x_shard), self.w13, self.h, 1, fixed_rows=self.M, gated=True)
+            self.launches += 1
+        else:
+            if self.P == 1 and not self.training:
+                gemm_bf16(self._operand(x_shard), self.w13, self.gu)
+            else:
+                self.up(x_shard)
+            self._chk(moe_fast.swiglu_fwd(self.gu.data_ptr(), self.rows.data_ptr(), 1, self.M, self.Fp, self.h.data_ptr(), s), "swiglu")
+            self.launches += 2
         y = self.down(self.h)
-        self.launches += 3
+        self.launches += 1
         return y
 
     __call__ = forward
 
+    @staticmethod
+    def _operand(x: torch.Tensor) -> torch.Tensor:
+        """`x` if the kernels can read it in place (rows contiguous and 16-byte aligned), else a copy."""
+        return x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
+
     def backward(self, dy_shard: torch.Tensor) -> torch.Tensor:
         """Returns dx_shard [M/P, H]; weight gradients land in ``dw13`` / ``dw2``.  Must follow forward()."""
         assert self.training
-        s = torch.cuda.current_stream().cuda_stream
-        dh = self.dgrad_h(dy_shard, weight=self.w2_t)                              # [M, F/P], gathers dy
-        grouped_gemm_tn(self.dgrad_h.gathered, self.h, self.dw2, 1, self.rows)     # dW2 = dy^T h
-        self._chk(self.lib.bshmem_moe_swiglu_bwd(self.gu.data_ptr(), dh.data_ptr(), self.rows.data_ptr(), 1, self.M, self.Fp,
-                                                 self.dgu.data_ptr(), s), "swiglu bwd")
+        s = current_stream()
+        fused = self.P == 1 and self._fills(self.Fp)
+        if self.P == 1:
+            dy = self._operand(dy_shard)                                           # nothing to gather
+            if fused:
+                grouped_gemm_swiglu_bwd(dy, self.w2_t, self.gu, self.dgu, 1)       # dgu = SwiGLU' (dy @ W2)
+            else:
+                dh = gemm_bf16(dy, self.w2_t, self.dgrad_h.out)
+        else:
+            dh = self.dgrad_h(dy_shard, weight=self.w2_t)                          # [M, F/P], gathers dy
+            dy = self.dgrad_h.gathered
+        grouped_gemm_tn(dy, self.h, self.dw2, 1, self.rows)                        # dW2 = dy^T h
+        if not fused:
+            self._chk(moe_fast.swiglu_bwd(self.gu.data_ptr(), dh.data_ptr(), self.rows.data_ptr(), 1, self.M, self.Fp,
+                                          self.dgu.data_ptr(), s), "swiglu bwd")
         grouped_gemm_tn(self.dgu, self.up.gathered, self.dw13, 1, self.rows)       # dW13 = dgu^T x
         dx = self.dgrad_x(self.dgu, weight=self.w13_t)
-        self.launches += 5
+        self.launches += 4 if fused else 5
         return dx
 
     def check(self) -> None:

@@ -63,6 +63,8 @@ def moe_lib() -> C.CDLL:
         f("bshmem_moe_swiglu_bwd", VP, VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_transpose_pad", VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_grouped_gemm", VP, VP, VP, I, I, I, I, I, I, I, I, VP, I, VP, I, VP, VP, I, VP, I, I)
+        f("bshmem_moe_grouped_gemm_act", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I)
+        f("bshmem_moe_grouped_gemm_swiglu_bwd", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I)
         f("bshmem_moe_grouped_gemm_few", VP, VP, VP, I, I, I, I, I, I, I, VP, I, I, I, VP, VP, I, VP, I)
         f("bshmem_moe_grouped_gemm_tn", VP, VP, VP, I, I, I, I, I, I, I, VP, VP, I, I)
         f("bshmem_moe_zero_pad_rows", VP, VP, I, I, I, VP)
@@ -116,6 +118,31 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
                             _p(rows), fixed_rows, _p(klen), gated, arrive, _p(expected), n_arrive, _stream(), timeout_ms, max_ctas)
     if st != 0:
         raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
+
+
+def grouped_gemm_act(a: torch.Tensor, b: torch.Tensor, gu: torch.Tensor, act: torch.Tensor, groups: int, *,
+                     rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0, timeout_ms: int = 4000) -> None:
+    """Training forward of the gated MLP in one kernel: gu_g = a_g @ b_g.T (interleaved gate / up pre-activations, kept for
+    the backward pass) and act_g = silu(gate) * up.  a: [G*R, K], b: [G*N, K], gu: [G*R, N], act: [G*R, N/2]."""
+    G = groups
+    st = _fast.grouped_gemm_act(a.data_ptr(), b.data_ptr(), gu.data_ptr(), act.data_ptr(), G, a.shape[0] // G, b.shape[0] // G, a.shape[1],
+                                a.stride(0), b.stride(0), gu.stride(0), act.stride(0), _p(rows), arrive, _p(expected), n_arrive, _stream(),
+                                timeout_ms)
+    if st != 0:
+        raise RuntimeError(f"grouped gemm (act) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
+
+
+def grouped_gemm_swiglu_bwd(dy: torch.Tensor, w2_t: torch.Tensor, gu: torch.Tensor, dgu: torch.Tensor, groups: int, *,
+                            rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0,
+                            timeout_ms: int = 4000) -> None:
+    """d_gu_g = SwiGLU backward of (dy_g @ w2_t_g.T) at the pre-activations gu_g, in one kernel: the gradient of the
+    activations never goes to memory.  dy: [G*R, K], w2_t: [G*N, K], gu and dgu: [G*R, 2N] (interleaved)."""
+    G = groups
+    st = _fast.grouped_gemm_swiglu_bwd(dy.data_ptr(), w2_t.data_ptr(), gu.data_ptr(), dgu.data_ptr(), G, dy.shape[0] // G,
+                                       w2_t.shape[0] // G, dy.shape[1], dy.stride(0), w2_t.stride(0), gu.stride(0), dgu.stride(0), _p(rows),
+                                       arrive, _p(expected), n_arrive, _stream(), timeout_ms)
+    if st != 0:
+        raise RuntimeError(f"grouped gemm (swiglu) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 def grouped_gemm_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: int, counts: torch.Tensor, *,
@@ -193,7 +220,7 @@ class MoELayer:
             self.xsave = self.recv
             self.w13_t = torch.empty((G, H, 2 * F), dtype=bf, device=dev)
             self.w2_t = torch.empty((G, F, H), dtype=bf, device=dev)
-            self.dh = torch.empty((G * cap, F), dtype=bf, device=dev)
+            self.dh = torch.empty((G * cap, F), dtype=bf, device=dev)             # used where experts have few rows
             self.dgu = torch.empty((G * cap, 2 * F), dtype=bf, device=dev)
             self.dxe = torch.empty((G * cap, H), dtype=bf, device=dev)
             if not tn_gemm:
@@ -272,10 +299,14 @@ class MoELayer:
             wait = dict(arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # gate/up projection (waits on the arrival words inside the kernel), then SwiGLU, then down projection
         if self.training:
-            grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms,
-                         few=few, **wait)
-            self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
-            self._x_in = x                                         # the router's backward needs the layer input
+            if few is None:
+                grouped_gemm_act(self.recv, self.w13.view(G * 2 * F, H), self.gu, self.hact, G, rows=self.recv_count,
+                                 timeout_ms=self.timeout_ms, **wait)
+            else:
+                grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms,
+                             few=few, **wait)
+                self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
+            self._x_in, self._few = x, few                         # the router's backward needs the layer input
         else:
             grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.hact, G, rows=self.recv_count, gated=True,
                          timeout_ms=self.timeout_ms, few=few, **wait)
@@ -325,8 +356,12 @@ class MoELayer:
             self._chk(_fast.dispatch(self._state_a, self._plan_a, dout.data_ptr(), a["topk_w"], a["topk_idx"], a["pos"], n_entries, self.topk,
                                      H, a["recv_bwd"], 0, par, SIG_BWD_DISPATCH, self.ctas, s), "dispatch(bwd)")
             wait = dict(arrive=self._sig_ptr(par, SIG_BWD_DISPATCH), expected=self.expect_from, n_arrive=P)
-        # d_hact = d_y · W2            (B operand = W2^T [F, H], K = H)
-        grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, **wait)
+        # d_hact = d_y · W2 (B operand = W2^T [F, H], K = H) and through SwiGLU to d_gu
+        if self._few is None:
+            grouped_gemm_swiglu_bwd(dy, self.w2_t.view(G * F, H), self.gu, self.dgu, G, rows=rc, timeout_ms=self.timeout_ms, **wait)
+        else:
+            grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few, **wait)
+            self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
         # dW2 = d_y^T · hact: token-major operands straight into the MN-major tensor-core path
         if self.tn_gemm:
             zero_pad_rows(dy, G, rc)
@@ -338,8 +373,7 @@ class MoELayer:
             self._chk(_fast.transpose_pad(dy.data_ptr(), rc.data_ptr(), G, cap, H, ta.data_ptr(), s), "transpose")
             self._chk(_fast.transpose_pad(a["hact"], rc.data_ptr(), G, cap, F, tb.data_ptr(), s), "transpose")
             grouped_gemm(ta, tb, self.dw2.view(G * H, F), G, fixed_rows=H, klen=rc, timeout_ms=self.timeout_ms)
-        # SwiGLU backward, then dW13 = d_gu^T · x and d_x = d_gu · W13
-        self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
+        # dW13 = d_gu^T · x and d_x = d_gu · W13
         if self.tn_gemm:
             zero_pad_rows(self.dgu, G, rc)
             zero_pad_rows(self.xsave, G, rc)
@@ -350,7 +384,7 @@ class MoELayer:
             self._chk(_fast.transpose_pad(a["dgu"], rc.data_ptr(), G, cap, 2 * F, ta2.data_ptr(), s), "transpose")
             self._chk(_fast.transpose_pad(self.xsave.data_ptr(), rc.data_ptr(), G, cap, H, tb2.data_ptr(), s), "transpose")
             grouped_gemm(ta2, tb2, self.dw13.view(G * 2 * F, H), G, fixed_rows=2 * F, klen=rc, timeout_ms=self.timeout_ms)
-        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms)
+        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few)
         self.launches += 4
         if local:
             # d_x = sum over k of the experts' rows + the router path (d_logits · Wr), written once
