@@ -9,19 +9,24 @@
 //
 // The scales differ from k-block to k-block, so the tensor core cannot keep one running
 // accumulator.  Each k-block's product (M128 x N256 x K128, four tcgen05.mma kind::f8f6f4)
-// goes into one of two 256-column TMEM buffers; sixteen epilogue warps read the buffer that
-// just completed, multiply by the row's scale and add into fp32 registers (64 per thread,
-// packed two-wide FMAs) while the tensor core fills the other buffer.  Four warps per SM
-// sub-partition hide the TMEM load latency.  One CTA per SM, persistent over 128x256 tiles:
+// goes into one of two 256-column TMEM buffers; the promotion warps read the buffer that
+// just completed, multiply by the row's scale and add into fp32 registers (packed two-wide
+// FMAs) while the tensor core fills the other buffer.  One CTA per SM, persistent over
+// 128x256 tiles (or, with few tiles, a cluster of CTAs per tile):
 //   warp 0      TMA producer: 3-stage ring of 48 KiB (A 128 rows + B 256 rows of 128 bytes)
 //   warp 1      MMA issuer, commits each k-block to the stage's and the buffer's mbarrier
-//   warps 2-17  promote partial products (32 rows x 64 columns each), then convert, stage in
-//               swizzled smem and TMA-store
+//   warps 2-9   (2-17 in the fused collectives) promote partial products, then convert, stage
+//               in swizzled smem and TMA-store
+// What bounds it is the life of a product (MMAs, commit, barrier, tensor-memory load, release):
+// about 0.5 us per k-block with two of them on their way.  4096 x 7168 x 8192 takes 235 us; with
+// the scales fetched into registers, where every use of the queue waited for an L2 round trip, it
+// took 272.  CTA pairs on 256x256 or 256x128 tiles (half the loads of B) were slower, 245 and 398 us.
 // Every wait is bounded (see gemm_core.cuh); there is no counterpart in the reference.
 #include <cuda_fp8.h>
 
 #include "../include/bshmem_device.cuh"
 #include "gemm_core.cuh"
+#include "gemm_pair.cuh"
 #include "tma_host.h"
 
 using namespace bshmem;
@@ -35,7 +40,9 @@ constexpr int FEPI_WARPS = 16;
 constexpr int FNUM_THREADS = 32 * (2 + FEPI_WARPS);
 constexpr uint32_t FA_BYTES = FBM * FBK, FB_BYTES = FBN * FBK, FSTAGE_BYTES = FA_BYTES + FB_BYTES;
 constexpr uint32_t FEPI_BYTES = 32 * 128;               // one warp: 32 rows x 64 bf16
-constexpr uint32_t FSMEM_TILES = FSTAGES * FSTAGE_BYTES + FEPI_WARPS * FEPI_BYTES;
+constexpr int FSCALES = 8;                              // k-blocks whose activation scales are on their way or in use
+constexpr uint32_t FSCALE_BYTES = FSCALES * 32 * 4;     // one warp
+constexpr uint32_t FSMEM_TILES = FSTAGES * FSTAGE_BYTES + FEPI_WARPS * (FEPI_BYTES + FSCALE_BYTES);
 constexpr uint32_t FSMEM_BYTES = FSMEM_TILES + 256 + 1024;
 constexpr uint32_t kIdescFp8 = ptx::umma_idesc(0, 0, 128, 256);   // e4m3 x e4m3 -> fp32, M128 N256
 
@@ -88,13 +95,16 @@ struct Fp8Params {
   CUtensorMap map_a, map_b, map_c;
   const float* sa;             // [K/128][M]
   const float* sb;             // [K/128][N/128]
+  __nv_bfloat16* c;            // split form: output and its leading dimension, and CTAs per tile
+  long long ldc;
+  int split;
   Fp8Ag ag;                    // used by the all-gather variant only
 };
 struct Fp8RsParams {
   Fp8Params base;
   Fp8Rs rs;
 };
-enum : int { F8_PLAIN = 0, F8_AG = 1, F8_RS = 2 };
+enum : int { F8_PLAIN = 0, F8_AG = 1, F8_RS = 2, F8_SPLIT = 3 };
 
 enum : int { ERR_F8_A_READY = 123, ERR_F8_PEER_READY = 124, ERR_F8_PEER_DONE = 125, ERR_F8_RS_SIGNAL = 126 };
 
@@ -102,7 +112,7 @@ enum : int { ERR_F8_A_READY = 123, ERR_F8_PEER_READY = 124, ERR_F8_PEER_DONE = 1
 // rank me+1, me+2, ... which is also the order in which the pull warps fetch them.
 template <int kMode>
 __device__ __forceinline__ void f8_tile_coords(const Fp8Params& p, const Fp8Rs* rs, int tile, int* m_blk, int* n_blk) {
-  if constexpr (kMode == F8_PLAIN) {
+  if constexpr (kMode == F8_PLAIN || kMode == F8_SPLIT) {
     raster_coords(p.core, tile, m_blk, n_blk);
   } else if constexpr (kMode == F8_RS) {
     // owner-major, owners visited in the order me+1, me+2, ..., me: the P ranks always write to P different owners
@@ -183,12 +193,22 @@ __device__ __forceinline__ bool f8_pull_piece(const Fp8Params& prm, int lane, Gu
   return true;
 }
 
+// Eight promotion warps of 128 columns each have 168 registers per thread to work with; with sixteen of 64 columns (96
+// registers) the accumulators and the products on their way spill, and 4096 x 7168 x 8192 takes 240 us instead of 235.  The
+// reduce-scatter form keeps sixteen for its epilogue, which adds the peers' partials to 64 columns at a time.
+constexpr int f8_epi_warps(int mode) { return mode == F8_PLAIN || mode == F8_SPLIT ? 8 : FEPI_WARPS; }
+constexpr int FPART_PITCH = FBN + 4;                    // floats per row of a parked partial tile (split form): no bank conflicts
+static_assert(FBM * FPART_PITCH * 4 <= FSTAGES * FSTAGE_BYTES, "the partial tile takes the place of the stages");
+
 struct FSmem {
   uint32_t base;
   uint8_t* gen;
   __device__ __forceinline__ uint32_t a(int s) const { return base + s * FSTAGE_BYTES; }
   __device__ __forceinline__ uint32_t b(int s) const { return base + s * FSTAGE_BYTES + FA_BYTES; }
   __device__ __forceinline__ uint32_t epi(int w) const { return base + FSTAGES * FSTAGE_BYTES + w * FEPI_BYTES; }
+  __device__ __forceinline__ uint32_t scale(int w, int slot, int lane) const {
+    return base + FSTAGES * FSTAGE_BYTES + FEPI_WARPS * FEPI_BYTES + w * FSCALE_BYTES + (slot * 32 + lane) * 4;
+  }
   __device__ __forceinline__ uint32_t bars() const { return base + FSMEM_TILES; }
   __device__ __forceinline__ uint32_t full(int s) const { return bars() + 8 * s; }
   __device__ __forceinline__ uint32_t empty(int s) const { return bars() + 8 * (FSTAGES + s); }
@@ -220,10 +240,47 @@ __device__ __forceinline__ void rs_publish(unsigned int* count, uint64_t* sig) {
   }
 }
 
+// Parks 64 accumulator columns of a warp's 32 rows (row = lane) as bf16 under the 128-byte swizzle, ready for a TMA store.
+__device__ __forceinline__ void f8_stage_chunk(uint32_t buf, int lane, const float2* acc) {
+  const uint32_t rowbase = buf + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2* src = acc + j * 4;
+    const uint32_t w0 = pack_bf16(src[0].x, src[0].y), w1 = pack_bf16(src[1].x, src[1].y);
+    const uint32_t w2 = pack_bf16(src[2].x, src[2].y), w3 = pack_bf16(src[3].x, src[3].y);
+    const uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
+
+// Split form: CTA `rank` of the S that share a tile adds up its 128 / S rows, in rank order, and writes them as bf16.
+template <int S>
+__device__ __forceinline__ void f8_split_reduce(const Fp8Params& prm, const FSmem& L, int rank, int m_blk, int n_blk) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kRows = FBM / S;
+  uint32_t src[S];
+#pragma unroll
+  for (int q = 0; q < S; ++q) src[q] = gemm2::mapa(L.base, q);
+  for (int u = warp; u < 2 * kRows; u += f8_epi_warps(F8_SPLIT) + 2) {          // unit: half a row, 4 columns per lane
+    const int row = rank * kRows + (u >> 1), col = (u & 1) * (FBN / 2) + lane * 4;
+    float4 v[S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) v[q] = gemm2::ld_cluster_f4(src[q] + (row * FPART_PITCH + col) * 4);
+#pragma unroll
+    for (int q = 1; q < S; ++q) { v[0].x += v[q].x; v[0].y += v[q].y; v[0].z += v[q].z; v[0].w += v[q].w; }
+    *reinterpret_cast<uint2*>(prm.c + (size_t)(m_blk * FBM + row) * prm.ldc + n_blk * FBN + col) =
+        make_uint2(pack_bf16(v[0].x, v[0].y), pack_bf16(v[0].z, v[0].w));
+  }
+}
+
 template <int kMode>
 __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs* rs, uint8_t* smem_raw) {
   constexpr bool kAG = kMode == F8_AG;
   constexpr bool kRS = kMode == F8_RS;
+  constexpr bool kSplit = kMode == F8_SPLIT;
+  constexpr int kWarps = f8_epi_warps(kMode), kCols = FBN / (kWarps / 4);      // a warp promotes 32 rows x kCols columns
   FSmem L;
   {
     uint32_t r = ptx::smem_u32(smem_raw);
@@ -233,14 +290,18 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
   const CoreParams& cp = prm.core;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = cp.num_m_blocks * cp.num_n_blocks;
-  const int num_kb = cp.K / FBK;
+  const int S = kSplit ? prm.split : 1;
+  const int crank = kSplit ? (int)gemm2::cluster_ctarank() : 0;
+  // this CTA's tiles and k-blocks: in the split form a cluster has one tile, and its CTAs a share of the k-blocks each
+  const int tile0 = (int)blockIdx.x / S, tile_step = (int)gridDim.x / S;
+  const int kb0 = (cp.K / FBK) * crank / S, num_kb = (cp.K / FBK) * (crank + 1) / S - kb0;
   Guard g{cp.err, L.abort_flag(), cp.timeout_ns};
 
   if (threadIdx.x == 0) {
     *L.abort_flag() = 0;
     for (int i = 0; i < 4; ++i) *L.rs_count(i) = 0;
     for (int s = 0; s < FSTAGES; ++s) { ptx::mbar_init(L.full(s), 1); ptx::mbar_init(L.empty(s), 1); }
-    for (int b = 0; b < 2; ++b) { ptx::mbar_init(L.part_full(b), 1); ptx::mbar_init(L.part_empty(b), FEPI_WARPS); }
+    for (int b = 0; b < 2; ++b) { ptx::mbar_init(L.part_full(b), 1); ptx::mbar_init(L.part_empty(b), kWarps); }
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&prm.map_a);
     ptx::prefetch_tensormap(&prm.map_b);
@@ -266,7 +327,9 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
     }
   }
 
-  if (warp >= 2 + FEPI_WARPS) {
+  if constexpr (kMode == F8_PLAIN || kSplit) ptx::grid_dependency_wait();
+
+  if (warp >= 2 + kWarps) {
     // ------------------------------ pull warps (all-gather variant) ------------
     if constexpr (kAG) {
       if (prm.ag.P > 1)
@@ -277,7 +340,7 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
     if (lane == 0) {
       int s = 0; uint32_t ph = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
         int m_blk, n_blk;
         f8_tile_coords<kMode>(prm, rs, tile, &m_blk, &n_blk);
         if constexpr (kAG) {
@@ -289,11 +352,12 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(L.full(s), FSTAGE_BYTES);
-          ptx::tma_load_2d(L.a(s), &prm.map_a, L.full(s), kb * FBK, m_blk * FBM);
-          ptx::tma_load_2d(L.b(s), &prm.map_b, L.full(s), kb * FBK, n_blk * FBN);
+          ptx::tma_load_2d(L.a(s), &prm.map_a, L.full(s), (kb0 + kb) * FBK, m_blk * FBM);
+          ptx::tma_load_2d(L.b(s), &prm.map_b, L.full(s), (kb0 + kb) * FBK, n_blk * FBN);
           if (++s == FSTAGES) { s = 0; ph ^= 1; }
         }
       }
+      if constexpr (kMode == F8_PLAIN || kSplit) ptx::grid_launch_dependents();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
@@ -301,7 +365,7 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
       int s = 0; uint32_t ph = 0;
       uint32_t it = 0;                       // k-blocks issued so far: buffer = it & 1, use count = it >> 1
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int buf = it & 1;
           // the epilogue must have drained this buffer's previous product
@@ -321,14 +385,14 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
     }
   } else {
     // ------------------------------ promotion + epilogue -------------------------
-    const int ew = warp - 2;               // 0..15
+    const int ew = warp - 2;
     const int quarter = warp & 3;          // TMEM lanes 32*quarter.. belong to this warp
-    const int cg = ew >> 2;                // columns [64*cg, 64*cg + 64) of the tile
+    const int cg = ew >> 2;                // columns [kCols*cg, kCols*cg + kCols) of the tile
     uint64_t* pend_sig = nullptr;          // reduce-scatter variant: signal word of the tile whose store is in flight
     int pend_par = 0, tiles_done = 0;      // ... and which of the four arrival counters that tile uses
     uint32_t it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
       int m_blk, n_blk;
       f8_tile_coords<kMode>(prm, rs, tile, &m_blk, &n_blk);
       if constexpr (kAG) {
@@ -342,45 +406,91 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
         }
       }
       const int row = m_blk * FBM + quarter * 32 + lane;
-      const float* sa = prm.sa + row;
-      const float* sb = prm.sb + (n_blk * (FBN / 128) + (cg >> 1));
+      const float* sa = prm.sa + (size_t)kb0 * cp.M + row;
       const int sb_stride = cp.N / 128;
-      float2 acc[32];
+      const float* sb = prm.sb + (size_t)kb0 * sb_stride + (n_blk * (FBN / 128) + cg * kCols / 128);
+      float2 acc[kCols / 2];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) acc[i] = make_float2(0.f, 0.f);
-      // scales are fetched three k-blocks ahead of their use (an L2 round trip is longer than a k-block)
-      auto scale_at = [&](int kb) -> float {
-        if (kb >= num_kb) return 0.f;
-        // pulled scales were written during this kernel: no non-coherent load for them
-        const float a = kAG ? *reinterpret_cast<const volatile float*>(sa + (size_t)kb * cp.M) : __ldg(sa + (size_t)kb * cp.M);
-        return a * __ldg(sb + (size_t)kb * sb_stride);
+      for (int i = 0; i < kCols / 2; ++i) acc[i] = make_float2(0.f, 0.f);
+      // Scales travel ahead of their use, because an L2 round trip takes longer than a k-block.  A register would not do as
+      // the queue: moving or multiplying it waits for the load.  Each lane copies its row's scale into a ring of its own in
+      // shared memory (4 bytes, no alignment rule, nobody else reads it); the weight's scale is one value per k-block, 32 of
+      // them are held across the warp's lanes and the next 32 are on their way.
+      // Scales that were pulled during this kernel (all-gather form) must not come through L1: volatile loads.
+      auto sa_load = [&](int kb) -> float {
+        return kb < num_kb ? *reinterpret_cast<const volatile float*>(sa + (size_t)kb * cp.M) * __ldg(sb + (size_t)kb * sb_stride) : 0.f;
       };
-      float s0 = scale_at(0), s1 = scale_at(1), s2n = scale_at(2);
+      auto sa_copy = [&](int kb) {
+        if (kb < num_kb) ptx::cp_async_4(L.scale(ew, kb % FSCALES, lane), sa + (size_t)kb * cp.M);
+        ptx::cp_async_commit();
+      };
+      auto sb_load = [&](int kb) -> float { return kb + lane < num_kb ? __ldg(sb + (size_t)(kb + lane) * sb_stride) : 0.f; };
+      float s0 = 0.f, s1 = 0.f, s2 = 0.f, sb_now = 0.f, sb_next = 0.f;
+      if constexpr (kAG) {
+        s0 = sa_load(0); s1 = sa_load(1); s2 = sa_load(2);
+      } else {
+        sb_next = sb_load(0);
+#pragma unroll 1
+        for (int kb = 0; kb < FSCALES - 1; ++kb) sa_copy(kb);
+      }
 #pragma unroll 1
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
-        const float s3 = scale_at(kb + 3);
+        float s3 = 0.f;
+        if constexpr (kAG) {
+          s3 = sa_load(kb + 3);
+        } else {
+          sa_copy(kb + FSCALES - 1);
+          if ((kb & 31) == 0) { sb_now = sb_next; sb_next = sb_load(kb + 32); }
+        }
         const int buf = it & 1;
         if (!mbar_wait(L.part_full(buf), (it >> 1) & 1, g, ERR_F8_PART_FULL)) { ok = false; break; }
         ptx::tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * FBN + cg * 64;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * FBN + cg * kCols;
+        if constexpr (!kAG) {
+          ptx::cp_async_wait<FSCALES - 1>();
+          s0 = ptx::ld_shared_f32(L.scale(ew, kb % FSCALES, lane)) * __shfl_sync(0xffffffffu, sb_now, kb & 31);
+        }
         const float2 sc = make_float2(s0, s0);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kCols / 16; ++c) {
           uint32_t v[16];
           ptx::tmem_ld_32x32b_x16(taddr + c * 16, v);
           ptx::tmem_ld_wait();
+          if (c == kCols / 16 - 1) {           // everything is read: the buffer may be overwritten
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(L.part_empty(buf));
+          }
 #pragma unroll
           for (int i = 0; i < 8; ++i)
             acc[c * 8 + i] = __ffma2_rn(sc, make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), acc[c * 8 + i]);
         }
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(L.part_empty(buf));
-        s0 = s1; s1 = s2n; s2n = s3;
+        if constexpr (kAG) { s0 = s1; s1 = s2; s2 = s3; }
       }
+      if constexpr (!kAG) ptx::cp_async_wait<0>();
       if (!ok) break;
-      // ---- tile output: one 64-column chunk per warp through its swizzled staging buffer ----
-      if constexpr (kRS) {
+      if constexpr (kSplit) {
+        // park the partial tile over the stages: every copy into them has landed and every MMA has read them
+        const uint32_t part = L.base + ((quarter * 32 + lane) * FPART_PITCH + cg * kCols) * 4;
+#pragma unroll
+        for (int i = 0; i < kCols / 4; ++i)
+          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(part + i * 16), "f"(acc[2 * i].x), "f"(acc[2 * i].y),
+                       "f"(acc[2 * i + 1].x), "f"(acc[2 * i + 1].y) : "memory");
+        continue;
+      }
+      // ---- tile output: 64-column chunks through the warp's swizzled staging buffer ----
+      if constexpr (!kRS) {
+#pragma unroll
+        for (int h = 0; h < kCols / 64; ++h) {
+          if (lane == 0) ptx::tma_wait_group_read<0>();       // the previous store has read the buffer
+          __syncwarp();
+          f8_stage_chunk(L.epi(ew), lane, acc + 32 * h);
+          if (lane == 0) {
+            ptx::tma_store_2d(&prm.map_c, L.epi(ew), n_blk * FBN + cg * kCols + 64 * h, m_blk * FBM + quarter * 32);
+            ptx::tma_commit_group();
+          }
+        }
+      } else {
         // the previous tile's store has had a whole tile of promotion work to land: complete it and publish it now
         if (lane == 0) {
           ptx::tma_wait_group<0>();
@@ -389,11 +499,7 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
             pend_sig = nullptr;
           }
         }
-      } else {
-        if (lane == 0) ptx::tma_wait_group_read<0>();
-      }
-      __syncwarp();
-      if constexpr (kRS) {
+        __syncwarp();
         const int owner = m_blk / rs->blocks_per_rank;
         if (owner == rs->my_rank && rs->P > 1) {
           // own rows: the P-1 partials of this tile must have landed; add them (source order, fixed) to the accumulators
@@ -409,26 +515,9 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
                                       (long long)n_blk * FBN + cg * 64 + (lane & 7) * 8;
           add_partial_chunks<false>(reinterpret_cast<float(&)[64]>(acc), src0, (long long)(cp.M / rs->P) * N, N, rs->P, rs->my_rank, L.epi(ew), lane);
         }
-      }
-      const uint32_t rowbase = L.epi(ew) + lane * 128;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2* src = &acc[j * 4];
-        uint32_t w0 = pack_bf16(src[0].x, src[0].y), w1 = pack_bf16(src[1].x, src[1].y);
-        uint32_t w2 = pack_bf16(src[2].x, src[2].y), w3 = pack_bf16(src[3].x, src[3].y);
-        uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
-      }
-      ptx::fence_proxy_async_smem();
-      __syncwarp();
-      if constexpr (!kRS) {
+        f8_stage_chunk(L.epi(ew), lane, acc);
         if (lane == 0) {
-          ptx::tma_store_2d(&prm.map_c, L.epi(ew), n_blk * FBN + cg * 64, m_blk * FBM + quarter * 32);
-          ptx::tma_commit_group();
-        }
-      } else {
-        if (lane == 0) {
-          const int owner = m_blk / rs->blocks_per_rank, m_in = m_blk - owner * rs->blocks_per_rank;
+          const int m_in = m_blk - owner * rs->blocks_per_rank;
           if (owner == rs->my_rank) {
             // the reduced chunk of this PE's own rows goes straight to the output
             ptx::tma_store_2d(&rs->map_out, L.epi(ew), n_blk * FBN + cg * 64, m_in * FBM + quarter * 32);
@@ -457,6 +546,18 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
   // ------------------------------ teardown ---------------------------------------
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (kSplit) {
+    gemm2::cluster_sync_all();             // every part of the tile is parked
+    int m_blk, n_blk;
+    f8_tile_coords<kMode>(prm, rs, tile0, &m_blk, &n_blk);
+    if (!*L.abort_flag()) {
+      if (S == 2) f8_split_reduce<2>(prm, L, crank, m_blk, n_blk);
+      else if (S == 4) f8_split_reduce<4>(prm, L, crank, m_blk, n_blk);
+      else f8_split_reduce<8>(prm, L, crank, m_blk, n_blk);
+    }
+    __syncthreads();
+    gemm2::cluster_sync_all();             // nobody leaves while a peer still reads its part
+  }
   if constexpr (kAG) {
     // before the kernel ends, CTA 0 makes sure every peer has finished pulling this PE's rows
     if (!*L.abort_flag() && blockIdx.x == 0 && (int)threadIdx.x < prm.ag.P && (int)threadIdx.x != prm.ag.my_rank)
@@ -475,9 +576,15 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
   }
 }
 
-__global__ void __launch_bounds__(FNUM_THREADS, 1) gemm_fp8_blockscale_kernel(const __grid_constant__ Fp8Params prm) {
+constexpr int FPLAIN_THREADS = 32 * (2 + f8_epi_warps(F8_PLAIN));
+__global__ void __launch_bounds__(FPLAIN_THREADS, 1) gemm_fp8_blockscale_kernel(const __grid_constant__ Fp8Params prm) {
   extern __shared__ uint8_t smem_raw[];
   gemm_fp8_body<F8_PLAIN>(prm, nullptr, smem_raw);
+}
+// Fewer tiles than SMs: a cluster per tile.
+__global__ void __launch_bounds__(FPLAIN_THREADS, 1) gemm_fp8_split_kernel(const __grid_constant__ Fp8Params prm) {
+  extern __shared__ uint8_t smem_raw[];
+  gemm_fp8_body<F8_SPLIT>(prm, nullptr, smem_raw);
 }
 // all-gather -> GEMM: two more warps per CTA pull the peers' rows and scales while the tensor core runs
 __global__ void __launch_bounds__(FNUM_THREADS + 32 * FPULL_WARPS, 1) ag_gemm_fp8_kernel(const __grid_constant__ Fp8Params prm) {
@@ -517,6 +624,65 @@ __global__ void quant_act_1x128_kernel(const __nv_bfloat16* __restrict__ x, int 
     *reinterpret_cast<uint32_t*>(q + (size_t)m * K + kb * 128 + lane * 4) = packed;
     if (lane == 0) scales[(size_t)kb * scale_ld + m] = scale;
   }
+}
+
+// The same for 16-byte aligned rows.  A block takes 32 rows x 512 columns: eight lanes share a 128-column block (16
+// elements each), a warp covers 512 columns of four rows with all of its loads in flight together, and the block's scales
+// leave as 128-byte rows of the [K/128][M] matrix.  The kernel above moves 8 bytes per lane and one 4-byte scale per warp:
+// 36.7 us for 4096 x 8192, where the bytes take 15.4.
+__global__ void __launch_bounds__(256) quant_act_1x128_tile_kernel(const __nv_bfloat16* __restrict__ x, int M, int K, int ldx, uint8_t* __restrict__ q,
+                                                                   float* __restrict__ scales, int scale_ld) {
+  __shared__ float sc[4][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kb0 = blockIdx.x * 4, m0 = blockIdx.y * 32;
+  const int kb = kb0 + (lane >> 3), nkb = K / 128;
+  const int col = kb * 128 + (lane & 7) * 16;
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();           // the GEMM sets itself up meanwhile (it waits for this grid before it reads)
+  uint4 raw[4][2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int m = m0 + warp * 4 + r;
+    if (m < M && kb < nkb) {
+      const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)m * ldx + col);
+      raw[r][0] = __ldcg(src);
+      raw[r][1] = __ldcg(src + 1);
+    } else {
+      raw[r][0] = raw[r][1] = make_uint4(0, 0, 0, 0);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int m = m0 + warp * 4 + r;
+    float v[16];
+    float amax = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw[r][h]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[h * 8 + 2 * j] = __low2float(p[j]);
+        v[h * 8 + 2 * j + 1] = __high2float(p[j]);
+        amax = fmaxf(amax, fmaxf(fabsf(v[h * 8 + 2 * j]), fabsf(v[h * 8 + 2 * j + 1])));
+      }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float scale = amax > 0.f ? amax / 448.f : 1.f;
+    const float inv = 1.f / scale;
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint16_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] * inv, v[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+      const uint16_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j + 2] * inv, v[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+      o[j] = lo | ((uint32_t)hi << 16);
+    }
+    if (m < M && kb < nkb) *reinterpret_cast<uint4*>(q + (size_t)m * K + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    if ((lane & 7) == 0) sc[lane >> 3][warp * 4 + r] = scale;
+  }
+  __syncthreads();
+  const int k = threadIdx.x >> 5, m = m0 + lane;
+  if (k < 4 && kb0 + k < nkb && m < M) scales[(size_t)(kb0 + k) * scale_ld + m] = sc[k][lane];
 }
 
 // Weights: one scale per 128x128 block.  One CTA (256 threads) per block; scales: [K/128][N/128].
@@ -569,6 +735,7 @@ __global__ void quant_w_128x128_kernel(const __nv_bfloat16* __restrict__ w, int 
 
 int* g_err_dev[64] = {};
 int g_sms[64] = {};
+int g_clusters[64][3] = {};    // clusters of 2 / 4 / 8 CTAs of the split form that the device holds at once
 
 struct AgPlan {
   bshmem_dev_state_t st;
@@ -607,6 +774,9 @@ int ensure(int dev) {
   BSHMEM_CUDA_TRY(cudaMemset(g_err_dev[dev], 0, sizeof(int)));
   BSHMEM_CUDA_TRY(cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_fp8_blockscale_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_fp8_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
+  for (int i = 0; i < 3; ++i)
+    g_clusters[dev][i] = gemm2::max_resident_clusters(gemm_fp8_split_kernel, g_sms[dev], 2 << i, FPLAIN_THREADS, FSMEM_BYTES);
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(ag_gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_rs_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
   return 0;
@@ -648,8 +818,29 @@ int bshmem_gemm_fp8_blockscale(const void* A8, const float* scale_a, const void*
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   const int tiles = p.core.num_m_blocks * p.core.num_n_blocks;
   if (ctas > tiles) ctas = tiles;
-  gemm_fp8_blockscale_kernel<<<ctas, FNUM_THREADS, FSMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
-  BSHMEM_CUDA_TRY(cudaGetLastError());
+  p.c = static_cast<__nv_bfloat16*>(C);
+  p.ldc = ldc;
+  p.split = 1;
+  // While every tile can have a cluster of its own, the k-blocks of a tile are shared by its CTAs: the largest cluster for
+  // which all clusters are resident at once and a CTA keeps four k-blocks (below that the reduction through distributed
+  // shared memory, about 3 us, costs as much as the k-blocks it saves).  With one, two and four CTAs per tile 128 x 7168 x
+  // 8192 takes 32.5, 21.7 and 16.9 us, 128 x 2048 x 2048 11.7, 10.9 and 10.2.
+  if (max_ctas <= 0)
+    for (int i = 2; i >= 0; --i)
+      if (tiles <= g_clusters[dev][i] && K / FBK >= 4 * (2 << i)) { p.split = 2 << i; break; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ctas * p.split));
+  cfg.blockDim = dim3(FPLAIN_THREADS);
+  cfg.dynamicSmemBytes = FSMEM_BYTES;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, p.split > 1 ? gemm_fp8_split_kernel : gemm_fp8_blockscale_kernel, p));
   return 0;
 }
 
@@ -657,6 +848,20 @@ int bshmem_gemm_fp8_blockscale(const void* A8, const float* scale_a, const void*
 // k-block kb goes to scales[kb * scale_ld + m] (scale_ld >= M: a shard can write its columns of a wider matrix).
 int bshmem_fp8_quant_act_ld(const void* x, int M, int K, int ldx, void* q, float* scales, int scale_ld, void* stream) {
   if (K % 128 || ldx % 4 || scale_ld < M) { host::last_error() = "fp8 quant: K % 128 != 0, ldx % 4 != 0 or scale_ld < M"; return 1; }
+  if (ldx % 8 == 0 && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q)) & 15)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((K / 128 + 3) / 4), (unsigned)((M + 31) / 32));
+    cfg.blockDim = dim3(256);
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, quant_act_1x128_tile_kernel, static_cast<const __nv_bfloat16*>(x), M, K, ldx,
+                                       static_cast<uint8_t*>(q), scales, scale_ld));
+    return 0;
+  }
   long long nblk = (long long)M * (K / 128);
   int blocks = (int)((nblk + 7) / 8 < 148 * 16 ? (nblk + 7) / 8 : 148 * 16);
   if (blocks < 1) blocks = 1;

@@ -14,12 +14,14 @@ from typing import Optional
 import torch
 
 from .. import _native
+from .gemm import current_stream
 
 _declared = False
+_run = _quant_act = None                 # the entry points that run once per layer, as direct native calls
 
 
 def fp8_lib() -> C.CDLL:
-    global _declared
+    global _declared, _run, _quant_act
     lib = _native.load("libbshmem_fp8.so")
     if not _declared:
         VP, I = C.c_void_p, C.c_int
@@ -56,6 +58,7 @@ def fp8_lib() -> C.CDLL:
         lib.bshmem_fp8_rs_error_site.argtypes = [VP, I]
         lib.bshmem_fp8_rs_destroy.restype = I
         lib.bshmem_fp8_rs_destroy.argtypes = [VP]
+        _run, _quant_act = _native.fast(lib, "bshmem_gemm_fp8_blockscale"), _native.fast(lib, "bshmem_fp8_quant_act")
         _declared = True
     return lib
 
@@ -90,7 +93,7 @@ def quantize_act(x: torch.Tensor) -> Fp8Tensor:
     q = torch.empty((M, K), dtype=torch.uint8, device=x.device)
     s = torch.empty((K // 128, M), dtype=torch.float32, device=x.device)
     lib = fp8_lib()
-    st = lib.bshmem_fp8_quant_act(x.data_ptr(), M, K, x.stride(0), q.data_ptr(), s.data_ptr(), _stream())
+    st = _quant_act(x.data_ptr(), M, K, x.stride(0), q.data_ptr(), s.data_ptr(), current_stream())
     if st != 0:
         raise RuntimeError(f"fp8 quantize_act failed ({st}): {lib.bshmem_fp8_last_error().decode()}")
     return Fp8Tensor(q, s, "act")
@@ -125,8 +128,8 @@ def gemm_fp8(a: Fp8Tensor, b: Fp8Tensor, out: Optional[torch.Tensor] = None, *, 
     elif out.shape != (M, N) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ValueError("bad output tensor")
     lib = fp8_lib()
-    st = lib.bshmem_gemm_fp8_blockscale(a.q.data_ptr(), a.scales.data_ptr(), b.q.data_ptr(), b.scales.data_ptr(), out.data_ptr(),
-                                        M, N, K, out.stride(0), _stream(), max_ctas, timeout_ms)
+    st = _run(a.q.data_ptr(), a.scales.data_ptr(), b.q.data_ptr(), b.scales.data_ptr(), out.data_ptr(), M, N, K, out.stride(0),
+              current_stream(), max_ctas, timeout_ms)
     if st != 0:
         raise RuntimeError(f"fp8 gemm failed ({st}): {lib.bshmem_fp8_last_error().decode()}")
     return out
