@@ -306,16 +306,22 @@ __global__ void __launch_bounds__(skinny::NUM_THREADS) grouped_gemm_few_kernel(c
   skinny::grouped_body<kGated>(prm, smem_raw);
 }
 
-// Zero the token rows [count_g, next multiple of 64) — rows [0, 64) of an empty group — of every group of a
-// [G][cap][cols] bf16 buffer.
-__global__ void zero_pad_rows_kernel(__nv_bfloat16* buf, const int* counts, int cap, int cols) {
+// Zero the token rows [count_g, next multiple of 64) — rows [0, 64) of an empty group — of every group of up to four
+// [G][cap][cols] bf16 buffers.
+struct PadBuffers {
+  __nv_bfloat16* buf[4];
+  int cols[4];
+};
+__global__ void zero_pad_rows_kernel(PadBuffers pb, const int* counts, int cap) {
+  ptx::grid_dependency_wait();
   const int g = blockIdx.y;
-  const int c = counts[g];
+  const int c = __ldcg(counts + g);
   int end = c == 0 ? 64 : (c + 63) / 64 * 64;      // an empty group still feeds one (all-zero) block to the GEMM
   if (end > cap) end = cap;
+  const int cols = pb.cols[blockIdx.z];
   const int vec_per_row = cols / 8;
   const long long n = (long long)(end - c) * vec_per_row;
-  uint4* base = reinterpret_cast<uint4*>(buf + ((size_t)g * cap + c) * cols);
+  uint4* base = reinterpret_cast<uint4*>(pb.buf[blockIdx.z] + ((size_t)g * cap + c) * cols);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     base[i] = make_uint4(0, 0, 0, 0);
 }
@@ -570,11 +576,32 @@ int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int
   return 0;
 }
 
-// buf: [G][cap][cols] bf16, cols % 8 == 0: zero rows [counts[g], next multiple of 64) of every group.
-int bshmem_moe_zero_pad_rows(void* buf, const int* counts_dev, int G, int cap, int cols, void* stream) {
-  if (cols % 8 || G < 1) { host::last_error() = "zero_pad_rows: cols % 8 != 0"; return 1; }
-  zero_pad_rows_kernel<<<dim3(8, G), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<__nv_bfloat16*>(buf), counts_dev, cap, cols);
-  BSHMEM_CUDA_TRY(cudaGetLastError());
+// Up to four [G][cap][cols] bf16 buffers (null: none), cols % 8 == 0: zero rows [counts[g], next multiple of 64) of every
+// group.  One launch for all: four in a row took 12 us of a backward pass.
+int bshmem_moe_zero_pad_rows(void* b0, int cols0, void* b1, int cols1, void* b2, int cols2, void* b3, int cols3, const int* counts_dev, int G,
+                             int cap, void* stream) {
+  PadBuffers pb;
+  memset(&pb, 0, sizeof(pb));
+  void* bufs[4] = {b0, b1, b2, b3};
+  const int cols[4] = {cols0, cols1, cols2, cols3};
+  int n = 0;
+  for (int i = 0; i < 4; ++i) {
+    if (!bufs[i]) continue;
+    if (cols[i] % 8) { host::last_error() = "zero_pad_rows: cols % 8 != 0"; return 1; }
+    pb.buf[n] = static_cast<__nv_bfloat16*>(bufs[i]);
+    pb.cols[n++] = cols[i];
+  }
+  if (G < 1 || n == 0) { host::last_error() = "zero_pad_rows: nothing to do"; return 1; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(8, (unsigned)G, (unsigned)n);
+  cfg.blockDim = dim3(256);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, zero_pad_rows_kernel, pb, counts_dev, cap));
   return 0;
 }
 

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <utility>
 
@@ -158,16 +159,18 @@ __device__ __forceinline__ void router_select(float* lg, int E, int topk, int la
 
 // Few tokens: one block per token, its eight warps share the experts (32 tokens of 4096, 8 experts: 74 us with one warp
 // per token, which walks eight rows of 8 KiB alone).
+template <int kTok>
 __global__ void __launch_bounds__(256) k_router_topk_few(const bf16* __restrict__ x, const bf16* __restrict__ wr, int T, int H, int E, int topk,
                                                          int* __restrict__ topk_idx, float* __restrict__ topk_w, float* __restrict__ probs) {
-  __shared__ float lg[64];
-  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ float lg[kTok * 64];
+  const int t0 = blockIdx.x * kTok, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = (E + 7) / 8, e0 = warp * per;
   ptx::grid_dependency_wait();
-  if (e0 < E) router_logits<1>(x, wr, t, T, H, e0, min(per, E - e0), lane, lg);
+  if (e0 < E) router_logits<kTok>(x, wr, t0, T, H, e0, min(per, E - e0), lane, lg);
   __syncthreads();
-  if (warp == 0)
-    router_select(lg, E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk, probs ? probs + (size_t)t * E : nullptr);
+  const int t = t0 + warp;
+  if (warp < kTok && t < T)
+    router_select(lg + warp * 64, E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk, probs ? probs + (size_t)t * E : nullptr);
 }
 // Many tokens: a warp takes four of them, so that a row of Wr is read once for four tokens (one warp per token reads E
 // rows of Wr from L2 for every row of x: 193 us for 16384 tokens of 4096 and 8 experts, where x itself takes 21 us; here
@@ -271,30 +274,29 @@ __device__ __forceinline__ void offsets_block(const MoePlanDev& pl, const int* c
     if (run > cap) atomicAdd(pl.dropped, run - cap);
   }
   __syncthreads();
-  for (int s = tid; s < P; s += blockDim.x) {
-    // entries of source s that fit into my experts' buffers (what will arrive from s)
-    int exp_in = 0;
-    for (int el = 0; el < Epr; ++el) {
+  // a warp per source, its lanes over the experts (one thread walking 64 experts of the only PE took 12 us)
+  const int lane = tid & 31;
+  for (int s = tid >> 5; s < P; s += blockDim.x >> 5) {
+    // entries of source s that fit into my experts' buffers (what will arrive from s), and my entries that fit into PE s's
+    // experts (what comes back from s in the combine)
+    int exp_in = 0, out = 0;
+    for (int el = lane; el < Epr; el += 32) {
       int a = pl.src_start[el * (P + 1) + s], b = pl.src_start[el * (P + 1) + s + 1];
-      a = a < cap ? a : cap;
-      b = b < cap ? b : cap;
-      exp_in += b - a;
-    }
-    pl.expect_from[s] = exp_in;
-    // my entries that fit into PE s's experts (what comes back from s in the combine)
-    int out = 0;
-    for (int el = 0; el < Epr; ++el) {
-      int e = s * Epr + el;
-      int a = 0;
+      exp_in += min(b, cap) - min(a, cap);
+      const int e = s * Epr + el;
+      a = 0;
       for (int q = 0; q < me; ++q) a += __ldcg(counts_all + q * E + e);
-      int b = a + __ldcg(counts_all + me * E + e);
-      a = a < cap ? a : cap;
-      b = b < cap ? b : cap;
-      out += b - a;
+      b = a + __ldcg(counts_all + me * E + e);
+      out += min(b, cap) - min(a, cap);
     }
-    pl.send_to[s] = out;
+    exp_in = __reduce_add_sync(0xffffffffu, exp_in);
+    out = __reduce_add_sync(0xffffffffu, out);
+    if (lane == 0) {
+      pl.expect_from[s] = exp_in;
+      pl.send_to[s] = out;
+    }
     // recycle the other parity's arrival words for the next call
-    for (int which = 0; which < 4; ++which) pl.arrive_sig[(parity ^ 1) * 4 * P + which * P + s] = 0;
+    if (lane < 4) pl.arrive_sig[(parity ^ 1) * 4 * P + lane * P + s] = 0;
   }
 }
 __global__ void k_offsets(MoePlanDev pl, const int* __restrict__ counts_all, int parity) {
@@ -639,62 +641,80 @@ __global__ void k_router_dlogits(const float* __restrict__ w, const float* __res
 }
 
 // d_Wr[e, :] += sum over the CTA's tokens routed to e of d_logit * x[token, :]   (fp32 accumulation, atomics across CTAs).
-// A CTA takes kTok tokens and 2048 columns; its (token, k) entries are first bucketed by expert in shared memory, so
-// the loads of the hit rows can be issued back to back.
-constexpr int kDwrTok = 128;
+// A CTA stages `tok` rows x 256 columns of x in shared memory and sorts its (token, k) entries by expert meanwhile; its
+// warps then take equal shares of the sorted entries, with eight columns to a lane, and add a sum to global memory whenever
+// the expert changes.  So x is read once, all of a CTA's loads are in flight together, and neither the number of experts
+// nor an uneven routing leaves warps idle (with all warps walking the experts one after the other, every expert cost a
+// round trip: 300 tokens, 64 experts, top-8: 191 us; 16384 tokens of 4096, 8 experts, top-2: 146 us).
+constexpr int kDwrTok = 128, kDwrCols = 256, kDwrPitch = kDwrCols * 2 + 16;       // bytes per staged row
+constexpr uint32_t kDwrSmem = kDwrTok * kDwrPitch;
 __global__ void __launch_bounds__(256) k_router_dwr(const bf16* __restrict__ x, const int* __restrict__ topk_idx, const float* __restrict__ dlog,
-                                                   int T, int H, int E, int topk, float* __restrict__ dwr) {
-  __shared__ int cnt[64], start[65], fill[64];
-  __shared__ int ent[kDwrTok * 8];
-  const int t0 = blockIdx.x * kDwrTok;
-  const int nt = min(kDwrTok, T - t0);
-  const int n_ent = nt * topk;
-  if (threadIdx.x < 64) { cnt[threadIdx.x] = 0; fill[threadIdx.x] = 0; }
+                                                   int T, int H, int E, int topk, int tok, float* __restrict__ dwr) {
+  extern __shared__ __align__(16) char rows[];
+  __shared__ int cnt[64], fill[64];
+  __shared__ unsigned short ent[kDwrTok * 8];            // sorted entries: token << 6 | expert
+  __shared__ float grad[kDwrTok * 8];
+  const int t0 = blockIdx.x * tok, nt = min(tok, T - t0), n_ent = nt * topk;
+  const int c0 = blockIdx.y * kDwrCols, nv = min(kDwrCols, H - c0) / 8;      // 16-byte pieces per staged row
+  const uint32_t rows_a = ptx::smem_u32(rows);
+  if (threadIdx.x < 64) cnt[threadIdx.x] = 0;
+  ptx::grid_dependency_wait();
+  for (int i = threadIdx.x; i < nt * 32; i += 256) {
+    const int r = i >> 5, v = i & 31;
+    if (v < nv) ptx::cp_async_16(rows_a + r * kDwrPitch + v * 16, x + (size_t)(t0 + r) * H + c0 + v * 8);
+  }
+  ptx::cp_async_commit();
   __syncthreads();
-  for (int i = threadIdx.x; i < n_ent; i += blockDim.x) atomicAdd(&cnt[topk_idx[t0 * topk + i]], 1);
+  for (int i = threadIdx.x; i < n_ent; i += 256) atomicAdd(&cnt[topk_idx[(size_t)t0 * topk + i]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int a = 0;
-    for (int e = 0; e < E; ++e) { start[e] = a; a += cnt[e]; }
-    start[E] = a;
+  if (threadIdx.x < 32) {                                // exclusive scan over 64 counts
+    const int c_lo = cnt[2 * threadIdx.x], c_hi = cnt[2 * threadIdx.x + 1];
+    int incl = c_lo + c_hi;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)threadIdx.x >= o) incl += up;
+    }
+    fill[2 * threadIdx.x] = incl - c_lo - c_hi;
+    fill[2 * threadIdx.x + 1] = incl - c_hi;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_ent; i += blockDim.x) {
-    const int e = topk_idx[t0 * topk + i];
-    ent[start[e] + atomicAdd(&fill[e], 1)] = i;
+  for (int i = threadIdx.x; i < n_ent; i += 256) {
+    const int e = topk_idx[(size_t)t0 * topk + i], at = atomicAdd(&fill[e], 1);
+    ent[at] = (unsigned short)(i / topk << 6 | e);
+    grad[at] = dlog[(size_t)t0 * topk + i];
   }
+  ptx::cp_async_wait<0>();
   __syncthreads();
-  const int col = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (col >= H) return;
-  for (int e = 0; e < E; ++e) {
-    const int b = start[e], n = start[e + 1] - b;
-    if (n == 0) continue;
-    float acc[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane >= nv) return;
+  const int i0 = n_ent * warp / 8, i1 = n_ent * (warp + 1) / 8;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  auto flush = [&](int e) {
+    float4* dst = reinterpret_cast<float4*>(dwr + (size_t)e * H + c0 + lane * 8);
+    atomicAdd(dst, make_float4(acc[0], acc[1], acc[2], acc[3]));
+    atomicAdd(dst + 1, make_float4(acc[4], acc[5], acc[6], acc[7]));
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int j0 = 0; j0 < n; j0 += 4) {
-      uint4 xv[4];
-      float g[4];
+  };
+  int e_now = i0 < i1 ? ent[i0] & 63 : 0;
+#pragma unroll 4
+  for (int i = i0; i < i1; ++i) {
+    const int v = ent[i];
+    const float g = grad[i];
+    const uint4 raw = *reinterpret_cast<const uint4*>(rows + (v >> 6) * kDwrPitch + lane * 16);
+    if ((v & 63) != e_now) { flush(e_now); e_now = v & 63; }
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = ent[b + min(j0 + u, n - 1)];
-        g[u] = j0 + u < n ? dlog[t0 * topk + i] : 0.f;
-        xv[u] = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + i / topk) * H + col);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&xv[u]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 f = __bfloat1622float2(h[q]);
-          acc[2 * q] += g[u] * f.x;
-          acc[2 * q + 1] += g[u] * f.y;
-        }
-      }
+    for (int q = 0; q < 4; ++q) {
+      const float2 f = __bfloat1622float2(h[q]);
+      acc[2 * q] += g * f.x;
+      acc[2 * q + 1] += g * f.y;
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(&dwr[(size_t)e * H + col + j], acc[j]);
   }
+  if (i0 < i1) flush(e_now);
 }
 
 __global__ void k_f32_to_bf16(const float* __restrict__ in, bf16* __restrict__ out, size_t n) {
@@ -789,8 +809,9 @@ int plan_threads(int n_entries) {
 
 // Launch that may overlap the tail of the stream's previous kernel; `k` calls ptx::grid_dependency_wait() first thing.
 template <class... P, class... A>
-cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, void* stream, A&&... args) {
+cudaError_t launch_pdl_smem(void (*k)(P...), dim3 grid, dim3 block, uint32_t smem, void* stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
+  cfg.dynamicSmemBytes = smem;
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.stream = static_cast<cudaStream_t>(stream);
@@ -800,6 +821,10 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, void* stream, A&&
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, static_cast<P>(std::forward<A>(args))...);
+}
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, void* stream, A&&... args) {
+  return launch_pdl_smem(k, grid, block, 0, stream, std::forward<A>(args)...);
 }
 
 thread_local std::string g_err;
@@ -817,7 +842,9 @@ int bshmem_moe_router_topk(const void* x, const void* wr, int T, int H, int E, i
   if (T <= 0) return 0;
   // below about two rounds of the chip in warps of four tokens, the block-per-token form has the shorter chain
   if (T < 4096) {
-    RT_TRY(launch_pdl(k_router_topk_few, dim3(T), dim3(256), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
+    // four tokens to a block, which then reads Wr once for the four, as soon as that leaves two blocks per multiprocessor
+    const int tok = T >= 4 * 2 * 148 ? 4 : 1;
+    RT_TRY(launch_pdl(tok == 4 ? k_router_topk_few<4> : k_router_topk_few<1>, dim3((T + tok - 1) / tok), dim3(256), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
   } else {
     RT_TRY(launch_pdl(k_router_topk, dim3((T + 4 * kRouterWarps - 1) / (4 * kRouterWarps)), dim3(32 * kRouterWarps), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
   }
@@ -929,9 +956,16 @@ int bshmem_moe_router_backward(const void* x, const int* topk_idx, const float* 
     RT_TRY(cudaGetLastError());
   }
   RT_TRY(cudaMemsetAsync(dwr_f32, 0, sizeof(float) * (size_t)E * H, st));
-  dim3 grid((T + kDwrTok - 1) / kDwrTok, (H + 2047) / 2048);
-  k_router_dwr<<<grid, 256, 0, st>>>((const bf16*)x, topk_idx, dlog, T, H, E, topk, dwr_f32);
-  RT_TRY(cudaGetLastError());
+  // fewer tokens to a CTA while that leaves multiprocessors idle (each CTA adds up to E x 256 sums at its end)
+  const int col_blocks = (H + kDwrCols - 1) / kDwrCols;
+  int tok = kDwrTok;
+  while (tok > 16 && (long long)((T + tok - 1) / tok) * col_blocks < 148) tok /= 2;
+  static std::once_flag once[64];
+  int dev = 0;
+  RT_TRY(cudaGetDevice(&dev));
+  std::call_once(once[dev & 63], [] { cudaFuncSetAttribute(k_router_dwr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwrSmem); });
+  RT_TRY(launch_pdl_smem(k_router_dwr, dim3((T + tok - 1) / tok, col_blocks), dim3(256), (uint32_t)(tok * kDwrPitch), stream, (const bf16*)x, topk_idx, (const float*)dlog, T, H, E, topk,
+                    tok, dwr_f32));
   k_f32_to_bf16<<<64, 256, 0, st>>>(dwr_f32, (bf16*)dwr, (size_t)E * H);
   RT_TRY(cudaGetLastError());
   return 0;

@@ -67,7 +67,7 @@ def moe_lib() -> C.CDLL:
         f("bshmem_moe_grouped_gemm_swiglu_bwd", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I)
         f("bshmem_moe_grouped_gemm_few", VP, VP, VP, I, I, I, I, I, I, I, VP, I, I, I, VP, VP, I, VP, I)
         f("bshmem_moe_grouped_gemm_tn", VP, VP, VP, I, I, I, I, I, I, I, VP, VP, I, I)
-        f("bshmem_moe_zero_pad_rows", VP, VP, I, I, I, VP)
+        f("bshmem_moe_zero_pad_rows", VP, I, VP, I, VP, I, VP, I, VP, I, I, VP)
         f("bshmem_moe_gemm_error_site", I)
         f("bshmem_moe_gemm_error_word", res=VP)
         _declared = True
@@ -158,10 +158,14 @@ def grouped_gemm_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups:
         raise RuntimeError(f"grouped gemm (tn) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
-def zero_pad_rows(buf: torch.Tensor, groups: int, counts: torch.Tensor) -> None:
-    """Zero rows [counts[g], next multiple of 64) of every group of a contiguous [G*cap, cols] bf16 buffer."""
-    assert buf.is_contiguous()
-    st = _fast.zero_pad_rows(buf.data_ptr(), counts.data_ptr(), groups, buf.shape[0] // groups, buf.shape[1], _stream())
+def zero_pad_rows(buf, groups: int, counts: torch.Tensor) -> None:
+    """Zero rows [counts[g], next multiple of 64) of every group of a contiguous [G*cap, cols] bf16 buffer, or of up to four
+    buffers with the same number of rows in one launch."""
+    bufs = [buf] if isinstance(buf, torch.Tensor) else list(buf)
+    rows = bufs[0].shape[0]
+    assert all(b.is_contiguous() and b.shape[0] == rows for b in bufs)
+    args = [v for b in bufs for v in (b.data_ptr(), b.shape[1])] + [0, 0] * (4 - len(bufs))
+    st = _fast.zero_pad_rows(*args, counts.data_ptr(), groups, rows // groups, _stream())
     if st != 0:
         raise RuntimeError(f"zero_pad_rows failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
@@ -364,8 +368,7 @@ class MoELayer:
             self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
         # dW2 = d_y^T · hact: token-major operands straight into the MN-major tensor-core path
         if self.tn_gemm:
-            zero_pad_rows(dy, G, rc)
-            zero_pad_rows(self.hact, G, rc)
+            zero_pad_rows((dy, self.hact, self.dgu, self.xsave), G, rc)
             grouped_gemm_tn(dy, self.hact, self.dw2.view(G * H, F), G, rc, timeout_ms=self.timeout_ms)
         else:                          # explicit transposes + ragged-K K-major GEMM
             ta = self.t_a[: G * H * cap].view(G * H, cap)
@@ -375,8 +378,6 @@ class MoELayer:
             grouped_gemm(ta, tb, self.dw2.view(G * H, F), G, fixed_rows=H, klen=rc, timeout_ms=self.timeout_ms)
         # dW13 = d_gu^T · x and d_x = d_gu · W13
         if self.tn_gemm:
-            zero_pad_rows(self.dgu, G, rc)
-            zero_pad_rows(self.xsave, G, rc)
             grouped_gemm_tn(self.dgu, self.xsave, self.dw13.view(G * 2 * F, H), G, rc, timeout_ms=self.timeout_ms)
         else:
             ta2 = self.t_a[: G * 2 * F * cap].view(G * 2 * F, cap)

@@ -61,3 +61,28 @@ def test_router_and_plan(T, E, topk):
         assert p[i] == seen[e]
         seen[e] += 1
     assert cnt.tolist() == seen
+
+
+@pytest.mark.parametrize("T,E,topk,H", [(1, 8, 2, 8), (17, 64, 8, 264), (300, 64, 8, 2048), (2400, 3, 1, 520), (8200, 16, 2, 1032)])
+def test_router_backward(T, E, topk, H):
+    """d_Wr on both sides of its token block, columns that do not fill one, more experts than warps and fewer, one expert that
+    takes most tokens and one that takes none."""
+    from roc_shmem_b200.ops.moe import moe_lib
+    torch.manual_seed(T + E)
+    lib = moe_lib()
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    score = torch.rand(T, E, device="cuda")
+    score[: T * 3 // 4, 0] += 1
+    if E > topk:
+        score[:, E - 1] = -1
+    idx = score.topk(topk, dim=1).indices.to(torch.int32).contiguous()
+    dlog = torch.randn(T, topk, device="cuda")
+    scratch = torch.full((E, H), 5.0, device="cuda")
+    dwr = torch.empty(E, H, dtype=torch.bfloat16, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib.bshmem_moe_router_backward(x.data_ptr(), idx.data_ptr(), 0, 0, T, H, E, topk, dlog.data_ptr(), scratch.data_ptr(),
+                                          dwr.data_ptr(), s) == 0
+    torch.cuda.synchronize()
+    d = torch.zeros(T, E, dtype=torch.float64, device="cuda").scatter_(1, idx.long(), dlog.double())
+    ref, mag = d.t() @ x.double(), d.abs().t() @ x.double().abs()
+    assert bool(((dwr.double() - ref).abs() <= ref.abs() * 2 ** -8 + mag * T * 2 ** -24).all())     # bf16; fp32 sums in any order
