@@ -469,7 +469,7 @@ int bshmem_moe_grouped_gemm_swiglu_bwd(const void* A, const void* B, const void*
 int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, int a_rows_per_group, int N, int K, int lda, int ldb, int ldc,
                                 const int* rows_dev, int max_rows, int max_active, int gated, const void* arrive, const int* expected, int P,
                                 void* stream, int timeout_ms) {
-  if (G < 1 || G > skinny::MAX_GROUPS || a_rows_per_group % BM || N % BN || K % 8 || lda % 8 || ldb % 8 || ldc % 8 || !rows_dev || max_rows < 1) {
+  if (G < 1 || G > skinny::MAX_GROUPS || a_rows_per_group < BM || a_rows_per_group % BM || N % BN || K % 8 || lda % 8 || ldb % 8 || ldc % 8 || !rows_dev || max_rows < 1) {
     host::last_error() = "grouped gemm (few rows): needs 1 to 64 groups, rows-per-group % 256 == 0, N % 256 == 0, K and leading dimensions % 8 == 0";
     return 1;
   }

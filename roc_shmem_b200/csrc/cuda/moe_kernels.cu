@@ -48,72 +48,18 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ---------------------------------------------------------------------------------------
 // router; E <= 64 experts, top-k <= 8
 // ---------------------------------------------------------------------------------------
-// Logits of kTok tokens and kExp experts by one warp.  Per (token, expert) a lane adds the products of its 8-element
-// vectors lane, lane + 32, ... in order and the lanes are added as a tree: the sum does not depend on how tokens and
-// experts are dealt to warps.  The loads of kUnroll steps are in flight together (one by one, the latency of L2 is what
-// a warp spends its time on).
-template <int kTok, int kExp>
-__device__ __forceinline__ void router_dots(const bf16* x, const bf16* __restrict__ wr, int t0, int T, int H, int e0, int lane, float* logits) {
-  constexpr int kUnroll = 16 / (kTok + kExp) < 1 ? 1 : 16 / (kTok + kExp);
-  const int nv = H / 8;
-  const uint4* xp[kTok];
-#pragma unroll
-  for (int t = 0; t < kTok; ++t) xp[t] = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + t, T - 1) * H);
-  const uint4* wp = reinterpret_cast<const uint4*>(wr + (size_t)e0 * H);
-  float acc[kTok][kExp];
-#pragma unroll
-  for (int t = 0; t < kTok; ++t)
-#pragma unroll
-    for (int j = 0; j < kExp; ++j) acc[t][j] = 0.f;
-  auto step = [&](const uint4 (&xv)[kTok], const uint4 (&wv)[kExp]) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float2 xf[kTok];
-#pragma unroll
-      for (int t = 0; t < kTok; ++t) xf[t] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&xv[t])[q]);
-#pragma unroll
-      for (int j = 0; j < kExp; ++j) {
-        const float2 wf = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv[j])[q]);
-#pragma unroll
-        for (int t = 0; t < kTok; ++t) acc[t][j] += xf[t].x * wf.x + xf[t].y * wf.y;
-      }
-    }
-  };
-  int v = lane;
-  for (; v + (kUnroll - 1) * 32 < nv; v += kUnroll * 32) {
-    uint4 xv[kUnroll][kTok], wv[kUnroll][kExp];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-#pragma unroll
-      for (int t = 0; t < kTok; ++t) xv[u][t] = __ldcg(xp[t] + v + 32 * u);
-#pragma unroll
-      for (int j = 0; j < kExp; ++j) wv[u][j] = __ldg(wp + (size_t)j * nv + v + 32 * u);
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) step(xv[u], wv[u]);
-  }
-  for (; v < nv; v += 32) {
-    uint4 xv[kTok], wv[kExp];
-#pragma unroll
-    for (int t = 0; t < kTok; ++t) xv[t] = __ldcg(xp[t] + v);
-#pragma unroll
-    for (int j = 0; j < kExp; ++j) wv[j] = __ldg(wp + (size_t)j * nv + v);
-    step(xv, wv);
-  }
-#pragma unroll
-  for (int t = 0; t < kTok; ++t)
-#pragma unroll
-    for (int j = 0; j < kExp; ++j) {
-      const float s = warp_sum(acc[t][j]);
-      if (lane == 0) logits[t * 64 + e0 + j] = s;
-    }
-}
-template <int kTok>
-__device__ __forceinline__ void router_logits(const bf16* x, const bf16* __restrict__ wr, int t0, int T, int H, int e0, int ne, int lane,
-                                              float* logits /* [kTok][64] */) {
-  for (; ne >= 8; ne -= 8, e0 += 8) router_dots<kTok, 8>(x, wr, t0, T, H, e0, lane, logits);
-  for (; ne >= 2; ne -= 2, e0 += 2) router_dots<kTok, 2>(x, wr, t0, T, H, e0, lane, logits);
-  if (ne) router_dots<kTok, 1>(x, wr, t0, T, H, e0, lane, logits);
+// The logits are a skinny product, T x H by H x E: a block takes 16 tokens, its eight warps share the reduction in steps of
+// 32 columns, and the tensor cores multiply (mma.sync: 64 columns at most are no work for a tcgen05 tile, whose launch and
+// epilogue cost more than these kernels take).  The products of bf16 numbers are exact in fp32; a warp's accumulator takes
+// at most H / 128 additions and the warps' sums are added in order, a shorter chain than the H / 32 of a warp that multiplies with
+// FMAs.  Fragments come straight from global memory, 16 bytes per lane: the reduction may run over the columns in any order
+// as long as both operands agree, so a lane's eight consecutive columns stand for two k-steps' worth of its elements.
+// With a warp of FMAs per four tokens, Wr was read from L2 for every four and the FMAs took over for many experts: 16384 x
+// 4096, 8 experts 92 us; 12000 x 2048, 64 experts 245 us.
+constexpr int kRouterTok = 16;
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // Softmax over the experts, top-k, weights renormalised over the chosen ones; one warp per token, `lg` in shared memory.
@@ -123,71 +69,111 @@ __device__ __forceinline__ void router_select(float* lg, int E, int topk, int la
   for (int e = lane; e < E; e += 32) mx = fmaxf(mx, lg[e]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  for (int e = lane; e < E; e += 32) lg[e] = __expf(lg[e] - mx);
-  __syncwarp();
-  float den = 0.f;
-  for (int e = 0; e < E; ++e) den += lg[e];          // every lane, in expert order
-  // probabilities are not negative: their bit patterns order like the numbers; ties go to the lower expert index
-  unsigned long long key[2];
+  float p[2], den = 0.f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    p[h] = lane + 32 * h < E ? __expf(lg[lane + 32 * h] - mx) : 0.f;
+    den += p[h];
+  }
+  den = warp_sum(den);
+  // probabilities are not negative: their bit patterns order like the numbers (+1: 0 stands for taken); ties go to the lower
+  // expert index
+  unsigned key[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int e = lane + 32 * h;
-    key[h] = 0;
-    if (e < E) {
-      const float p = lg[e] / den;
-      if (probs) probs[e] = p;
-      key[h] = ((unsigned long long)__float_as_uint(p) << 32) | (unsigned)(64 - e);
-    }
+    p[h] /= den;
+    if (e < E && probs) probs[e] = p[h];
+    key[h] = e < E ? __float_as_uint(p[h]) + 1u : 0u;
   }
   float wsum = 0.f, mine = 0.f;
   int best_e = 0;
   for (int k = 0; k < topk; ++k) {
-    unsigned long long best = key[0] > key[1] ? key[0] : key[1];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-      if (other > best) best = other;
-    }
-    if (key[0] == best) key[0] = 0;
-    if (key[1] == best) key[1] = 0;
-    const float p = __uint_as_float((unsigned)(best >> 32));
-    wsum += p;
-    if (lane == k) { mine = p; best_e = 64 - (int)(best & 0xffffffffu); }
+    const unsigned best = __reduce_max_sync(0xffffffffu, max(key[0], key[1]));
+    const unsigned low = __ballot_sync(0xffffffffu, key[0] == best), high = __ballot_sync(0xffffffffu, key[1] == best);
+    const int e = min(low ? __ffs(low) - 1 : 31 + __ffs(high), E - 1);
+    if (e == lane) key[0] = 0;
+    if (e == lane + 32) key[1] = 0;
+    const float pe = __uint_as_float(best - 1u);
+    wsum += pe;
+    if (lane == k) { mine = pe; best_e = e; }
   }
   if (lane < topk) { idx[lane] = best_e; w[lane] = mine / wsum; }
 }
 
-// Few tokens: one block per token, its eight warps share the experts (32 tokens of 4096, 8 experts: 74 us with one warp
-// per token, which walks eight rows of 8 KiB alone).
-template <int kTok>
-__global__ void __launch_bounds__(256) k_router_topk_few(const bf16* __restrict__ x, const bf16* __restrict__ wr, int T, int H, int E, int topk,
-                                                         int* __restrict__ topk_idx, float* __restrict__ topk_w, float* __restrict__ probs) {
-  __shared__ float lg[kTok * 64];
-  const int t0 = blockIdx.x * kTok, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per = (E + 7) / 8, e0 = warp * per;
+// kTiles: tiles of eight experts.  kWarps: eight, or sixteen with half the steps each while there are few blocks.
+template <int kTiles, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) k_router_topk(const bf16* __restrict__ x, const bf16* __restrict__ wr, int T, int H, int E,
+                                                                   int topk, int* __restrict__ topk_idx, float* __restrict__ topk_w,
+                                                                   float* __restrict__ probs) {
+  constexpr int kPitch = kTiles * 8 + 2;
+  __shared__ float part[8][kRouterTok * kPitch];
+  __shared__ float lg[kWarps][64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int t0 = blockIdx.x * kRouterTok;
+  constexpr int kUnroll = kTiles >= 8 ? 2 : 4;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
   ptx::grid_dependency_wait();
-  if (e0 < E) router_logits<kTok>(x, wr, t0, T, H, e0, min(per, E - e0), lane, lg);
+  const bf16* xa = x + (size_t)min(t0 + g, T - 1) * H;
+  const bf16* xb = x + (size_t)min(t0 + g + 8, T - 1) * H;
+  float acc[kTiles][4];
+#pragma unroll
+  for (int j = 0; j < kTiles; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
+  const int steps = (H + 31) / 32;
+  for (int s0 = warp; s0 < steps; s0 += kUnroll * kWarps) {
+    uint4 a[kUnroll], b[kUnroll], w[kUnroll][kTiles];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int col = (s0 + u * kWarps) * 32 + c * 8;
+      const bool in = col < H;
+      a[u] = in ? __ldcg(reinterpret_cast<const uint4*>(xa + col)) : zero;
+      b[u] = in ? __ldcg(reinterpret_cast<const uint4*>(xb + col)) : zero;
+#pragma unroll
+      for (int j = 0; j < kTiles; ++j)
+        w[u][j] = in && j * 8 + g < E ? __ldg(reinterpret_cast<const uint4*>(wr + (size_t)(j * 8 + g) * H + col)) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+#pragma unroll
+      for (int j = 0; j < kTiles; ++j) {
+        mma_bf16(acc[j], a[u].x, b[u].x, a[u].y, b[u].y, w[u][j].x, w[u][j].y);
+        mma_bf16(acc[j], a[u].z, b[u].z, a[u].w, b[u].w, w[u][j].z, w[u][j].w);
+      }
+  }
+  auto park = [&](bool add) {
+    float* p0 = part[warp & 7] + g * kPitch + c * 2;
+    float* p1 = p0 + 8 * kPitch;
+#pragma unroll
+    for (int j = 0; j < kTiles; ++j) {
+      float2 lo = make_float2(acc[j][0], acc[j][1]), hi = make_float2(acc[j][2], acc[j][3]);
+      float2* d0 = reinterpret_cast<float2*>(p0 + j * 8);
+      float2* d1 = reinterpret_cast<float2*>(p1 + j * 8);
+      if (add) { lo.x += d0->x; lo.y += d0->y; hi.x += d1->x; hi.y += d1->y; }
+      *d0 = lo;
+      *d1 = hi;
+    }
+  };
+  if (kWarps > 8) {
+    if (warp >= 8) park(false);
+    __syncthreads();
+  }
+  if (warp < 8) park(kWarps > 8);
   __syncthreads();
-  const int t = t0 + warp;
-  if (warp < kTok && t < T)
-    router_select(lg + warp * 64, E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk, probs ? probs + (size_t)t * E : nullptr);
-}
-// Many tokens: a warp takes four of them, so that a row of Wr is read once for four tokens (one warp per token reads E
-// rows of Wr from L2 for every row of x: 193 us for 16384 tokens of 4096 and 8 experts, where x itself takes 21 us; here
-// 70 us, and 83 us with eight warps to a block that walk the experts in step).
-constexpr int kRouterWarps = 4;
-__global__ void __launch_bounds__(32 * kRouterWarps) k_router_topk(const bf16* x, const bf16* __restrict__ wr, int T, int H, int E, int topk,
-                                                                   int* __restrict__ topk_idx, float* __restrict__ topk_w, float* __restrict__ probs) {
-  __shared__ float lg[kRouterWarps][4 * 64];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = (blockIdx.x * kRouterWarps + warp) * 4;
-  ptx::grid_dependency_wait();
-  if (t0 >= T) return;
-  router_logits<4>(x, wr, t0, T, H, 0, E, lane, lg[warp]);
-  __syncwarp();
-  for (int t = t0; t < min(t0 + 4, T); ++t)
-    router_select(lg[warp] + (t - t0) * 64, E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk,
-                  probs ? probs + (size_t)t * E : nullptr);
+  for (int r = warp; r < kRouterTok; r += kWarps) {
+    const int t = t0 + r;
+    if (t >= T) break;
+    __syncwarp();
+    for (int e = lane; e < E; e += 32) {
+      float sum = part[0][r * kPitch + e];
+#pragma unroll
+      for (int q = 1; q < 8; ++q) sum += part[q][r * kPitch + e];
+      lg[warp][e] = sum;
+    }
+    __syncwarp();
+    router_select(lg[warp], E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk, probs ? probs + (size_t)t * E : nullptr);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -253,13 +239,15 @@ __global__ void __launch_bounds__(1024) k_plan(const int* __restrict__ topk_idx,
 // ---------------------------------------------------------------------------------------
 // offsets: from the gathered counts [P][E] derive everything the data movement needs
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void offsets_block(const MoePlanDev& pl, const int* counts_all, int parity) {
+// count(s, e): entries of source s for expert e
+template <class Count>
+__device__ __forceinline__ void offsets_block(const MoePlanDev& pl, Count count, int parity) {
   const int P = pl.P, E = pl.E, Epr = E / P, me = pl.me, cap = pl.cap;
   const int tid = threadIdx.x;
   // start of my entries inside every expert's buffer
   for (int e = tid; e < E; e += blockDim.x) {
     int b = 0;
-    for (int s = 0; s < me; ++s) b += __ldcg(counts_all + s * E + e);
+    for (int s = 0; s < me; ++s) b += count(s, e);
     pl.base_me[e] = b;
   }
   // local experts: rows that will arrive (clamped to the capacity), and each source's share
@@ -267,7 +255,7 @@ __device__ __forceinline__ void offsets_block(const MoePlanDev& pl, const int* c
     int e = me * Epr + el, run = 0;
     for (int s = 0; s < P; ++s) {
       pl.src_start[el * (P + 1) + s] = run;
-      run += __ldcg(counts_all + s * E + e);
+      run += count(s, e);
     }
     pl.src_start[el * (P + 1) + P] = run;
     pl.recv_count[el] = run < cap ? run : cap;
@@ -285,8 +273,8 @@ __device__ __forceinline__ void offsets_block(const MoePlanDev& pl, const int* c
       exp_in += min(b, cap) - min(a, cap);
       const int e = s * Epr + el;
       a = 0;
-      for (int q = 0; q < me; ++q) a += __ldcg(counts_all + q * E + e);
-      b = a + __ldcg(counts_all + me * E + e);
+      for (int q = 0; q < me; ++q) a += count(q, e);
+      b = a + count(me, e);
       out += min(b, cap) - min(a, cap);
     }
     exp_in = __reduce_add_sync(0xffffffffu, exp_in);
@@ -301,7 +289,7 @@ __device__ __forceinline__ void offsets_block(const MoePlanDev& pl, const int* c
 }
 __global__ void k_offsets(MoePlanDev pl, const int* __restrict__ counts_all, int parity) {
   ptx::grid_dependency_wait();
-  offsets_block(pl, counts_all, parity);
+  offsets_block(pl, [&](int s, int e) { return __ldcg(counts_all + s * pl.E + e); }, parity);
 }
 // One PE: its own counts are all there is, so plan and offsets are one launch; the last block to finish (ticket, back
 // to zero afterwards) derives the offsets.
@@ -318,7 +306,36 @@ __global__ void __launch_bounds__(1024) k_plan_local(MoePlanDev pl, const int* _
     __threadfence();
   }
   __syncthreads();
-  if (last) offsets_block(pl, counts_all, parity);
+  if (last) offsets_block(pl, [&](int s, int e) { return __ldcg(counts_all + s * pl.E + e); }, parity);
+}
+// Up to kPlanFew entries: one block, a warp per expert (and 32 further on), everything in shared memory; no ticket and no
+// round trips between blocks (8 entries, 16 experts: 4.8 us with a block per expert, 2.9 so; equal at about 512).
+constexpr int kPlanFew = 256;
+__global__ void __launch_bounds__(1024) k_plan_local_few(MoePlanDev pl, const int* __restrict__ topk_idx, int n_entries, int* __restrict__ pos,
+                                                         int* counts, int* counts_all, int parity) {
+  __shared__ int ent[kPlanFew];
+  __shared__ int cnt[64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ptx::grid_dependency_wait();
+  for (int i = threadIdx.x; i < n_entries; i += 1024) ent[i] = __ldcg(topk_idx + i);
+  __syncthreads();
+  for (int e = warp; e < pl.E; e += 32) {
+    int before = 0;
+#pragma unroll 4
+    for (int i0 = 0; i0 < n_entries; i0 += 32) {
+      const int i = i0 + lane;
+      const unsigned hits = __ballot_sync(0xffffffffu, i < n_entries && ent[i < n_entries ? i : 0] == e);
+      if (hits >> lane & 1) pos[i] = before + __popc(hits & ((1u << lane) - 1));
+      before += __popc(hits);
+    }
+    if (lane == 0) {
+      cnt[e] = before;
+      counts[e] = before;
+      counts_all[e] = before;
+    }
+  }
+  __syncthreads();
+  offsets_block(pl, [&](int, int e) { return cnt[e]; }, parity);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -475,43 +492,49 @@ __global__ void k_combine_reduce(MoePlanDev pl, const bf16* __restrict__ ybuf, c
 // of their predecessor (programmatic serialization), so what that may have written is read past the first-level cache.
 constexpr int kRowThreads = 128;
 
-template <bool kGrad>
+// kTop: top-k rounded up to a power of two, so that the loads of a token's rows are issued together.
+template <int kTop, bool kGrad>
 __global__ void __launch_bounds__(kRowThreads) k_dispatch_local(MoePlanDev pl, const bf16* __restrict__ rows, const int* __restrict__ topk_idx,
                                                                 const int* __restrict__ pos, const float* __restrict__ w, int topk, int H,
                                                                 bf16* __restrict__ recv, const bf16* __restrict__ y, float* __restrict__ dw,
                                                                 float* __restrict__ dlog) {
   // kGrad (backward): the rows go out scaled by their routing weight, and with the experts' outputs y the block also has
   // everything for the routing gradient: dw_k = <y_k, row>, dlog_k = w_k (dw_k - sum_j w_j dw_j)
-  __shared__ float part[8][kRowThreads / 32];
+  __shared__ float part[kTop][kRowThreads / 32];
   const int t = blockIdx.x;
   ptx::grid_dependency_wait();
-  size_t slot[8];
-  float wk[8], acc[8];
+  size_t slot[kTop];
+  float wk[kTop], acc[kTop];
   unsigned live = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
+  for (int k = 0; k < kTop; ++k) {
     acc[k] = 0.f;
     wk[k] = 0.f;
     slot[k] = 0;
     if (k < topk) {
       const int e = __ldcg(topk_idx + t * topk + k), p = __ldcg(pos + t * topk + k);
-      if (p < pl.cap) live |= 1u << k;               // over capacity: dropped (counted with the offsets)
-      slot[k] = ((size_t)e * pl.cap + p) * (H / 8);
+      if (p < pl.cap) {                              // over capacity: dropped (counted with the offsets)
+        live |= 1u << k;
+        slot[k] = ((size_t)e * pl.cap + p) * (H / 8);
+      }
       if (kGrad) wk[k] = __ldcg(w + t * topk + k);
     }
   }
   const uint4* src = reinterpret_cast<const uint4*>(rows + (size_t)t * H);
   for (int v = threadIdx.x; v < H / 8; v += kRowThreads) {
+    uint4 yv[kTop];
+    if (kGrad) {                                     // a dead entry reads row 0 and does not count
+#pragma unroll
+      for (int k = 0; k < kTop; ++k) yv[k] = __ldcg(reinterpret_cast<const uint4*>(y) + slot[k] + v);
+    }
     const uint4 xv = __ldcg(src + v);
     const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (k >= topk) break;
+    for (int k = 0; k < kTop; ++k) {
       if (!(live >> k & 1)) continue;
       uint4 o = xv;
       if (kGrad) {
-        const uint4 yv = __ldcg(reinterpret_cast<const uint4*>(y) + slot[k] + v);
-        const __nv_bfloat162* yh = reinterpret_cast<const __nv_bfloat162*>(&yv);
+        const __nv_bfloat162* yh = reinterpret_cast<const __nv_bfloat162*>(&yv[k]);
         __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -526,23 +549,23 @@ __global__ void __launch_bounds__(kRowThreads) k_dispatch_local(MoePlanDev pl, c
   if (kGrad) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < kTop; ++k) {
       if (k >= topk) break;
       const float s = warp_sum(acc[k]);
       if (lane == 0) part[k][warp] = s;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      float d[8], sum = 0.f;
+      float d[kTop], sum = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < kTop; ++k) {
         if (k >= topk) break;
         d[k] = part[k][0] + part[k][1] + part[k][2] + part[k][3];
         dw[t * topk + k] = d[k];
         sum += wk[k] * d[k];
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < kTop; ++k) {
         if (k >= topk) break;
         dlog[t * topk + k] = wk[k] * (d[k] - sum);
       }
@@ -551,33 +574,53 @@ __global__ void __launch_bounds__(kRowThreads) k_dispatch_local(MoePlanDev pl, c
 }
 
 // out[token] = sum_k w_k * y[row of entry k], in k order; backward (kRouter): unweighted, plus sum_k dlog_k * wr[expert k].
-template <bool kRouter>
-__global__ void __launch_bounds__(kRowThreads) k_combine_local(MoePlanDev pl, const bf16* __restrict__ y, const float* __restrict__ w,
-                                                               const int* __restrict__ topk_idx, const int* __restrict__ pos, int topk, int H,
-                                                               bf16* __restrict__ out, const bf16* __restrict__ wr) {
-  const int t = blockIdx.x;
+// A warp takes a token's 256 columns (16 bytes per lane) at a time, `per` tokens one after the other, with all rows of a
+// token in flight together; the lanes hold the token's entries, and the next token's are on their way.  The block's slice of
+// wr waits in shared memory: read per token it was as many bytes as y itself.
+constexpr int kCombineCols = 256, kCombineWarps = 8;
+template <int kTop, bool kRouter>
+__global__ void __launch_bounds__(32 * kCombineWarps) k_combine_local(MoePlanDev pl, const bf16* __restrict__ y, const float* __restrict__ w,
+                                                                      const int* __restrict__ topk_idx, const int* __restrict__ pos, int T,
+                                                                      int topk, int H, int per, bf16* __restrict__ out,
+                                                                      const bf16* __restrict__ wr) {
+  extern __shared__ __align__(16) char wr_s[];       // kRouter: [E][256 columns]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = blockIdx.y * kCombineCols, nv = min(kCombineCols, H - c0) / 8;
   ptx::grid_dependency_wait();
-  size_t slot[8], row[8];
-  float wk[8];
-  unsigned live = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    slot[k] = row[k] = 0;
-    wk[k] = 0.f;
-    if (k < topk) {
-      const int e = __ldcg(topk_idx + t * topk + k), p = __ldcg(pos + t * topk + k);
-      if (p < pl.cap) live |= 1u << k;               // over capacity: contributes nothing
-      slot[k] = ((size_t)e * pl.cap + p) * (H / 8);
-      row[k] = (size_t)e * (H / 8);
-      wk[k] = __ldcg(w + t * topk + k);              // routing weight, or dlog
-    }
+  if (kRouter) {
+    for (int i = threadIdx.x; i < pl.E * 32; i += 32 * kCombineWarps)
+      if ((i & 31) < nv) ptx::cp_async_16(ptx::smem_u32(wr_s) + i * 16, wr + (size_t)(i >> 5) * H + c0 + (i & 31) * 8);
+    ptx::cp_async_commit();
+    ptx::cp_async_wait<0>();
+    __syncthreads();
   }
-  for (int v = threadIdx.x; v < H / 8; v += kRowThreads) {
+  const int t_first = (blockIdx.x * kCombineWarps + warp) * per, t_end = min(t_first + per, T);
+  int e_next = 0, p_next = 0;
+  float w_next = 0.f;
+  auto fetch = [&](int t) {                          // lane k: entry k of token t (w: routing weight, or dlog)
+    if (lane < topk && t < t_end) {
+      e_next = __ldcg(topk_idx + (size_t)t * topk + lane);
+      p_next = __ldcg(pos + (size_t)t * topk + lane);
+      w_next = __ldcg(w + (size_t)t * topk + lane);
+    }
+  };
+  fetch(t_first);
+  const uint4* yl = reinterpret_cast<const uint4*>(y + c0) + min(lane, nv - 1);
+  for (int t = t_first; t < t_end; ++t) {
+    const int e = e_next;
+    const float wl = w_next;
+    const bool fits = p_next < pl.cap;               // over capacity: contributes nothing
+    const unsigned live = __ballot_sync(0xffffffffu, fits && lane < topk);
+    const unsigned row = fits ? (unsigned)e * (unsigned)pl.cap + (unsigned)p_next : 0u;
+    fetch(t + 1);
+    uint4 yv[kTop];
+#pragma unroll
+    for (int k = 0; k < kTop; ++k) yv[k] = __ldcg(yl + (size_t)__shfl_sync(0xffffffffu, row, k) * (H / 8));
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    auto add = [&](const uint4& yv, float f) {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&yv);
+    auto add = [&](const uint4& v, float f) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float2 u = __bfloat1622float2(h[q]);
@@ -586,22 +629,23 @@ __global__ void __launch_bounds__(kRowThreads) k_combine_local(MoePlanDev pl, co
       }
     };
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (k >= topk) break;
-      if (live >> k & 1) add(__ldcg(reinterpret_cast<const uint4*>(y) + slot[k] + v), kRouter ? 1.f : wk[k]);
+    for (int k = 0; k < kTop; ++k) {
+      const float wk = __shfl_sync(0xffffffffu, wl, k);
+      if (live >> k & 1) add(yv[k], kRouter ? 1.f : wk);
     }
     if (kRouter) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k >= topk) break;
-        add(__ldcg(reinterpret_cast<const uint4*>(wr) + row[k] + v), wk[k]);
+      for (int k = 0; k < kTop; ++k) {
+        const float wk = __shfl_sync(0xffffffffu, wl, k);
+        const int ek = __shfl_sync(0xffffffffu, e, k);
+        if (k < topk) add(*reinterpret_cast<const uint4*>(wr_s + (ek * 32 + lane) * 16), wk);
       }
     }
     uint4 o;
     __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
     for (int q = 0; q < 4; ++q) oh[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-    reinterpret_cast<uint4*>(out + (size_t)t * H)[v] = o;
+    if (lane < nv) reinterpret_cast<uint4*>(out + (size_t)t * H + c0)[lane] = o;
   }
 }
 
@@ -827,6 +871,10 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, void* stream, A&&
   return launch_pdl_smem(k, grid, block, 0, stream, std::forward<A>(args)...);
 }
 
+// The instance of a kernel for top-k rounded up to a power of two.
+template <class K>
+K by_top(int topk, K k1, K k2, K k4, K k8) { return topk <= 1 ? k1 : topk <= 2 ? k2 : topk <= 4 ? k4 : k8; }
+
 thread_local std::string g_err;
 #define RT_TRY(call) do { cudaError_t _e = (call); if (_e != cudaSuccess) { g_err = std::string(#call) + ": " + cudaGetErrorString(_e); return 7; } } while (0)
 
@@ -840,14 +888,11 @@ int bshmem_moe_router_topk(const void* x, const void* wr, int T, int H, int E, i
                            void* stream) {
   if (E > 64 || topk > 8 || topk > E || H % 8) { g_err = "router: E <= 64, topk <= min(8, E), H % 8 == 0"; return 1; }
   if (T <= 0) return 0;
-  // below about two rounds of the chip in warps of four tokens, the block-per-token form has the shorter chain
-  if (T < 4096) {
-    // four tokens to a block, which then reads Wr once for the four, as soon as that leaves two blocks per multiprocessor
-    const int tok = T >= 4 * 2 * 148 ? 4 : 1;
-    RT_TRY(launch_pdl(tok == 4 ? k_router_topk_few<4> : k_router_topk_few<1>, dim3((T + tok - 1) / tok), dim3(256), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
-  } else {
-    RT_TRY(launch_pdl(k_router_topk, dim3((T + 4 * kRouterWarps - 1) / (4 * kRouterWarps)), dim3(32 * kRouterWarps), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
-  }
+  const int blocks = (T + kRouterTok - 1) / kRouterTok;
+  const bool few = blocks <= 148;
+  auto k = E <= 8 ? (few ? k_router_topk<1, 16> : k_router_topk<1, 8>) : E <= 16 ? (few ? k_router_topk<2, 16> : k_router_topk<2, 8>)
+           : E <= 32 ? (few ? k_router_topk<4, 16> : k_router_topk<4, 8>) : (few ? k_router_topk<8, 16> : k_router_topk<8, 8>);
+  RT_TRY(launch_pdl(k, dim3(blocks), dim3(few ? 512 : 256), stream, (const bf16*)x, (const bf16*)wr, T, H, E, topk, topk_idx, topk_w, probs));
   return 0;
 }
 
@@ -866,6 +911,10 @@ int bshmem_moe_offsets(const MoePlanDev* pl, const int* counts_all, int parity, 
 int bshmem_moe_plan_local(const MoePlanDev* pl, const int* topk_idx, int n_entries, int* pos, int* counts, int* counts_all,
                           unsigned int* ticket, int parity, void* stream) {
   if (pl->P != 1) { g_err = "plan_local: more than one PE"; return 1; }
+  if (n_entries <= kPlanFew && pl->E <= 64) {
+    RT_TRY(launch_pdl(k_plan_local_few, dim3(1), dim3(1024), stream, *pl, topk_idx, n_entries, pos, counts, counts_all, parity));
+    return 0;
+  }
   RT_TRY(launch_pdl(k_plan_local, dim3(pl->E), dim3(plan_threads(n_entries)), stream, *pl, topk_idx, n_entries, pos, counts, counts_all, ticket,
                     parity));
   return 0;
@@ -875,8 +924,9 @@ int bshmem_moe_plan_local(const MoePlanDev* pl, const int* topk_idx, int n_entri
 int bshmem_moe_dispatch_local(const MoePlanDev* pl, const void* rows, const int* topk_idx, const int* pos, int T, int topk, int H, void* recv,
                               void* stream) {
   if (pl->P != 1 || H % 8 || topk > 8) { g_err = "dispatch_local: one PE, H % 8 == 0, at most top-8"; return 1; }
-  RT_TRY(launch_pdl(k_dispatch_local<false>, dim3(T), dim3(kRowThreads), stream, *pl, (const bf16*)rows, topk_idx, pos, nullptr, topk, H,
-                    (bf16*)recv, nullptr, nullptr, nullptr));
+  RT_TRY(launch_pdl(by_top(topk, k_dispatch_local<1, false>, k_dispatch_local<2, false>, k_dispatch_local<4, false>, k_dispatch_local<8, false>),
+                    dim3(T), dim3(kRowThreads), stream, *pl, (const bf16*)rows, topk_idx, pos, nullptr, topk, H, (bf16*)recv, nullptr, nullptr,
+                    nullptr));
   return 0;
 }
 // One PE, backward: w * d_out to the experts' gradient buffers, and the gradients of the routing weights (dw) and of the
@@ -884,7 +934,8 @@ int bshmem_moe_dispatch_local(const MoePlanDev* pl, const void* rows, const int*
 int bshmem_moe_dispatch_grad_local(const MoePlanDev* pl, const void* dout, const int* topk_idx, const int* pos, const float* w, int T, int topk,
                                    int H, void* recv, const void* y, float* dw, float* dlog, void* stream) {
   if (pl->P != 1 || H % 8 || topk > 8) { g_err = "dispatch_local: one PE, H % 8 == 0, at most top-8"; return 1; }
-  RT_TRY(launch_pdl(k_dispatch_local<true>, dim3(T), dim3(kRowThreads), stream, *pl, (const bf16*)dout, topk_idx, pos, w, topk, H, (bf16*)recv,
+  RT_TRY(launch_pdl(by_top(topk, k_dispatch_local<1, true>, k_dispatch_local<2, true>, k_dispatch_local<4, true>, k_dispatch_local<8, true>),
+                    dim3(T), dim3(kRowThreads), stream, *pl, (const bf16*)dout, topk_idx, pos, w, topk, H, (bf16*)recv,
                     (const bf16*)y, dw, dlog));
   return 0;
 }
@@ -893,8 +944,14 @@ int bshmem_moe_dispatch_grad_local(const MoePlanDev* pl, const void* dout, const
 int bshmem_moe_combine_local(const MoePlanDev* pl, const void* y, const float* w, const int* topk_idx, const int* pos, int T, int topk, int H,
                              void* out, const void* wr, void* stream) {
   if (pl->P != 1 || H % 8 || topk > 8) { g_err = "combine_local: one PE, H % 8 == 0, at most top-8"; return 1; }
-  auto k = wr ? k_combine_local<true> : k_combine_local<false>;
-  RT_TRY(launch_pdl(k, dim3(T), dim3(kRowThreads), stream, *pl, (const bf16*)y, w, topk_idx, pos, topk, H, (bf16*)out, (const bf16*)wr));
+  auto k = wr ? by_top(topk, k_combine_local<1, true>, k_combine_local<2, true>, k_combine_local<4, true>, k_combine_local<8, true>)
+              : by_top(topk, k_combine_local<1, false>, k_combine_local<2, false>, k_combine_local<4, false>, k_combine_local<8, false>);
+  // four tokens per warp share the block's slice of wr and hide the entries' round trip; one while that fills the chip better
+  const int col_blocks = (H + kCombineCols - 1) / kCombineCols;
+  const int per = (long long)T * col_blocks >= 4ll * kCombineWarps * 4 * 148 ? 4 : 1;
+  RT_TRY(launch_pdl_smem(k, dim3((T + kCombineWarps * per - 1) / (kCombineWarps * per), col_blocks), dim3(32 * kCombineWarps),
+                         wr ? (uint32_t)pl->E * 512u : 0u, stream, *pl, (const bf16*)y, w, topk_idx, pos, T, topk, H, per, (bf16*)out,
+                         (const bf16*)wr));
   return 0;
 }
 

@@ -86,3 +86,59 @@ def test_router_backward(T, E, topk, H):
     d = torch.zeros(T, E, dtype=torch.float64, device="cuda").scatter_(1, idx.long(), dlog.double())
     ref, mag = d.t() @ x.double(), d.abs().t() @ x.double().abs()
     assert bool(((dwr.double() - ref).abs() <= ref.abs() * 2 ** -8 + mag * T * 2 ** -24).all())     # bf16; fp32 sums in any order
+
+
+@pytest.mark.parametrize("T,E,topk", [(17, 24, 4), (2369, 64, 8), (2400, 32, 1)])
+def test_router_and_plan_more_forms(T, E, topk):
+    """Expert counts that leave a tile partly empty and the largest, with eight and with sixteen warps to a block."""
+    test_router_and_plan(T, E, topk)
+
+
+@pytest.mark.parametrize("T,H,E,topk", [(1, 256, 8, 1), (37, 768, 8, 3), (100, 256, 64, 8), (2500, 2048, 8, 2), (4800, 1024, 12, 5)])
+def test_local_rows(T, H, E, topk):
+    """Dispatch, combine and their backward forms on one PE for every rounding of top-k, one token and four per warp, a
+    capacity that some entries exceed."""
+    import roc_shmem_b200 as shmem
+    from roc_shmem_b200.ops.moe import MoELayer, _fast
+    rt = shmem.init("device", rank=0, world_size=1, heap_bytes=512 << 20, timeout_ms=5000)
+    try:
+        torch.manual_seed(T + H)
+        layer = MoELayer(rt, H, 256, E, topk, T, capacity_factor=8.0 if T == 1 else 1.0, training=True)
+        for t in (layer.wr, layer.w13, layer.w2):
+            t.normal_(std=0.05)
+        layer.sync_transposes()
+        x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+        layer.forward(x)
+        torch.cuda.synchronize()
+        cap, s = layer.cap, torch.cuda.current_stream().cuda_stream
+        idx, pos = layer.topk_idx[:T * topk].view(T, topk).long(), layer.pos[:T * topk].view(T, topk).long()
+        live = pos < cap
+        row = (idx * cap + pos.clamp(max=cap - 1))
+        assert torch.equal(layer.recv[row[live]], x.view(T, 1, H).expand(T, topk, H)[live])
+        y = torch.randn(E * cap, H, device="cuda").to(torch.bfloat16)
+        w = torch.randn(T, topk, device="cuda")
+        wr = torch.randn(E, H, device="cuda").to(torch.bfloat16)
+        picked = y[row].double() * live.unsqueeze(-1)
+        out = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+        p = (layer._plan_a, y.data_ptr(), w.data_ptr(), layer.topk_idx.data_ptr(), layer.pos.data_ptr(), T, topk, H, out.data_ptr())
+        for with_wr in (0, wr.data_ptr()):
+            assert _fast.combine_local(*p, with_wr, s) == 0
+            torch.cuda.synchronize()
+            parts = torch.cat([picked, w.double().unsqueeze(-1) * wr[idx].double()], 1) if with_wr else picked * w.double().unsqueeze(-1)
+            ref, mag = parts.sum(1), parts.abs().sum(1)
+            assert bool(((out.double() - ref).abs() <= ref.abs() * 2 ** -8 + mag * 2 * topk * 2 ** -24).all())
+        dout = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+        g, dw, dlog = torch.zeros_like(y), torch.empty_like(w), torch.empty_like(w)
+        assert _fast.dispatch_grad_local(layer._plan_a, dout.data_ptr(), layer.topk_idx.data_ptr(), layer.pos.data_ptr(), w.data_ptr(), T, topk, H,
+                                         g.data_ptr(), y.data_ptr(), dw.data_ptr(), dlog.data_ptr(), s) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(g[row[live]], (dout.float().view(T, 1, H) * w.unsqueeze(-1)).to(torch.bfloat16)[live])
+        dref = (picked * dout.double().view(T, 1, H)).sum(-1)
+        tol = (picked * dout.double().view(T, 1, H)).abs().sum(-1) * H * 2 ** -24 + 1e-12
+        assert bool(((dw.double() - dref).abs() <= tol).all())
+        wd = w.double()
+        lref = wd * (dref - (wd * dref).sum(1, keepdim=True))
+        ltol = wd.abs() * (tol + (wd.abs() * (tol + dref.abs() * topk * 2 ** -23)).sum(1, keepdim=True) + dref.abs() * 2 ** -22)
+        assert bool(((dlog.double() - lref).abs() <= ltol + lref.abs() * 2 ** -22).all())
+    finally:
+        shmem.finalize()
