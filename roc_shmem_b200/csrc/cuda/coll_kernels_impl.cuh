@@ -19,11 +19,26 @@ constexpr int kThreads = kReduceThreads;
 #define COLL_CAT2(a, b) a##b
 #define COLL_CAT(a, b) COLL_CAT2(a, b)
 
-// dynamic shared memory of the reduction kernels: the staging ring of coll::reduce_bulk
+// dynamic shared memory: the staging rings of coll::reduce_bulk and of the bulk moves.  A move gets its ring only where it
+// is used and all blocks are resident with it (one to a multiprocessor).
 #ifndef COLL_UNIT_MOVE
 constexpr uint32_t kDynSmem = coll::kBulkSmemBytes;
+uint32_t dyn_smem(const CollArgs&, int, int) { return kDynSmem; }
 #else
-constexpr uint32_t kDynSmem = 0;
+constexpr uint32_t kDynSmem = coll::kMoveSmemBytes;
+uint32_t dyn_smem(const CollArgs& a, int ctas, int blocks) {
+  int dev = 0, sms = 0;
+  if (a.n / ctas < coll::kMoveMinBytes || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || blocks > sms)
+    return 0;
+  return kDynSmem;
+}
+__device__ __forceinline__ char* move_smem() {
+  extern __shared__ __align__(128) char coll_dyn_smem[];
+  uint32_t bytes;
+  asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+  return bytes >= kDynSmem ? coll_dyn_smem : nullptr;
+}
 #endif
 
 template <typename T>
@@ -65,10 +80,10 @@ __device__ __noinline__ int run_coll(const State& s, DTeam t, const CollArgs& a,
     case BSHMEM_COLL_BROADCAST: return coll::team_broadcast(s, t, base + a.dst_off, base + a.src_off, a.n, a.root, cta, ncta);
     case BSHMEM_COLL_FCOLLECT:
       if (a.stage_seq) return coll::team_fcollect_staged(s, t, base + a.dst_off, base + a.src_off, a.n, a.stage_seq, a.use_nvls, cta, ncta);
-      return coll::team_fcollect(s, t, base + a.dst_off, base + a.src_off, a.n, cta, ncta);
+      return coll::team_fcollect(s, t, base + a.dst_off, base + a.src_off, a.n, cta, ncta, move_smem());
     case BSHMEM_COLL_ALLTOALL:
       if (a.stage_seq) return coll::team_alltoall_staged(s, t, base + a.dst_off, base + a.src_off, a.n, a.stage_seq, cta, ncta);
-      return coll::team_alltoall(s, t, base + a.dst_off, base + a.src_off, a.n, cta, ncta);
+      return coll::team_alltoall(s, t, base + a.dst_off, base + a.src_off, a.n, cta, ncta, move_smem());
     case BSHMEM_COLL_EXCHANGE: {
       // publish one u64 (held in a.n) in every member's exchange row, sync, leave the row for the host
       if (threadIdx.x < t.size) {
@@ -116,19 +131,17 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(c
   // the last block to get here tells the host; the count is back at zero then
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();
+    __threadfence();                       // a system fence per block took 4 us; the blocks of a group share the GPU
     const unsigned n = gridDim.x * gridDim.y;
-    if (atomicInc(done.count, n - 1) == n - 1) {
-      __threadfence_system();
+    if (atomicInc(done.count, n - 1) == n - 1)
       asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(done.word), "l"(done.token) : "memory");
-    }
   }
 }
 
 }  // namespace
 
 cudaError_t COLL_CAT(launch_, COLL_UNIT)(const State& s, const DTeam& t, const CollArgs& a, int ctas, int* status, cudaStream_t stream) {
-  COLL_CAT(k_coll_, COLL_UNIT)<<<ctas, kThreads, kDynSmem, stream>>>(s, t, a, status);
+  COLL_CAT(k_coll_, COLL_UNIT)<<<ctas, kThreads, dyn_smem(a, ctas, ctas), stream>>>(s, t, a, status);
   return cudaGetLastError();
 }
 
@@ -137,7 +150,8 @@ cudaError_t COLL_CAT(launch_group_, COLL_UNIT)(const State* states, const DTeam*
   CollArgs args_copy = a;
   GroupDone done_copy = done;
   void* args[] = {&states, &teams, &args_copy, &status, &done_copy};
-  return cudaLaunchCooperativeKernel((void*)COLL_CAT(k_coll_group_, COLL_UNIT), dim3(ctas, n), dim3(kThreads), args, kDynSmem, stream);
+  return cudaLaunchCooperativeKernel((void*)COLL_CAT(k_coll_group_, COLL_UNIT), dim3(ctas, n), dim3(kThreads), args,
+                                     dyn_smem(a, ctas, ctas * n), stream);
 }
 
 void COLL_CAT(preload_, COLL_UNIT)() {

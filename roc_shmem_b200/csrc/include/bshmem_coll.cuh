@@ -48,7 +48,7 @@ __device__ __forceinline__ int active_set_sync(const State& s, const Team& t) {
   if (threadIdx.x == 0) as_status = BSHMEM_OK;
   __syncthreads();
   if (threadIdx.x == 0) {
-    asm volatile("fence.acq_rel.sys;" ::: "memory");
+    dev::fence_peers(s);
     int root = dev::team_pe(t, 0);
     unsigned long long* root_count = reinterpret_cast<unsigned long long*>(dev::ptr(s, t.psync, root));
     atomicAdd_system(root_count, 1ull);
@@ -122,9 +122,9 @@ __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta 
   if (tid == 0) sync_status = BSHMEM_OK;
   __syncthreads();                       // all stores of the block precede the release below
   if (tid < t.size) {
-    // release pattern: one system fence per signalling thread, then the flag.  The block barrier above makes every
+    // release pattern: one fence per signalling thread, then the flag.  The block barrier above makes every
     // thread's earlier stores (remote ones included) precede this fence, so they are visible to whoever sees the flag.
-    asm volatile("fence.acq_rel.sys;" ::: "memory");
+    dev::fence_peers(s);
     uint64_t* remote = flag_addr(s, dev::team_pe(t, tid), t.slot, cta, t.my_idx);
     asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(remote), "l"(epoch) : "memory");
     const uint64_t* mine = flag_addr(s, s.my_pe, t.slot, cta, tid);
@@ -144,9 +144,9 @@ __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta 
   __syncthreads();
   return rc;
 }
-// barrier = quiet + sync.  The sync's own release (block barrier, then a system fence by each signalling thread before
+// barrier = quiet + sync.  The sync's own release (block barrier, then a fence by each signalling thread before
 // its flag store) already orders every earlier store of the calling block, puts to peers included, before the flags;
-// a second fence by all threads of the block would only add system-scope fences that contend across blocks.
+// a second fence by all threads of the block would only add fences that contend across blocks.
 __device__ __forceinline__ int team_barrier(const State& s, const Team& t, int cta = 0) {
   return team_sync(s, t, cta);
 }
@@ -254,20 +254,23 @@ __device__ __forceinline__ void reduce_vec_body(int nsrc, const T* const* srcs, 
 
 // ---- large reductions through shared memory with bulk async copies ------------------------------------------------
 // Plain loads are bounded by the outstanding-miss capacity of an SM's load/store unit: about 1.3 TB/s of local HBM
-// and a few hundred GB/s over NVLink (3 us latency) however many loads a thread keeps in flight.  Here one thread
-// fetches a chunk of EVERY source with cp.async.bulk (global -> shared, mbarrier completion; sources may be peer
-// memory, nothing is multicast) into a ring of kBulkStages stages, all threads reduce the stage out of shared memory
-// and write the result with ordinary (fire-and-forget) stores to the ndst destinations.
+// and a few hundred GB/s over NVLink (3 us latency) however many loads a thread keeps in flight.  Here the first
+// warp fetches a chunk of EVERY source with cp.async.bulk (global -> shared, mbarrier completion; sources may be peer
+// memory, nothing is multicast) into a ring of kBulkStages stages and all threads reduce the stage out of shared memory.
 // A stage is 32 KiB whatever the number of sources, so that a source's share is a whole number of 16-byte vectors per
 // thread for up to eight sources and 256 threads (with 48 KiB, 1.5 vectors), and four of them leave three on their way
 // while one is reduced.
 constexpr int kBulkStages = 4;
 constexpr uint32_t kBulkStageBytes = 32 * 1024;
-constexpr uint32_t kBulkSmemBytes = kBulkStages * kBulkStageBytes + 64;   // + mbarriers
+// Results leave the same way: parked in one of two buffers of a source's share of a stage, copied to all destinations
+// while the block reduces the next stage.  (With ordinary stores an allreduce of 32 MiB over eight PEs spent
+// 192 us of its 223 here; its bytes take 82.)
+constexpr uint32_t kBulkOutBytes = 16 * 1024;
+constexpr uint32_t kBulkSmemBytes = kBulkStages * kBulkStageBytes + 2 * kBulkOutBytes + 64;   // + mbarriers
 // One stage: vectors threadIdx.x, + blockDim.x, ... of every source.  NS > 0: exactly NS sources, all of a vector's
 // shared-memory loads in flight together; NS = 0: nsrc sources, one after the other.
 template <typename T, int OP, int NS>
-__device__ __forceinline__ void reduce_stage(const char* stage, uint32_t chunk, uint32_t nvec, int nsrc, int ndst, T* const* dsts, size_t v_base) {
+__device__ __forceinline__ void reduce_stage(const char* stage, uint32_t chunk, uint32_t nvec, int nsrc, char* result) {
   using A = typename Acc<T>::type;
   constexpr int VE = 16 / sizeof(T);
   for (uint32_t v = threadIdx.x; v < nvec; v += blockDim.x) {
@@ -296,7 +299,7 @@ __device__ __forceinline__ void reduce_stage(const char* stage, uint32_t chunk, 
     Vec16<T> out;
 #pragma unroll
     for (int e = 0; e < VE; ++e) out.e[e] = from_acc<T>(acc[e]);
-    for (int d = 0; d < ndst; ++d) reinterpret_cast<uint4*>(dsts[d])[v_base + v] = out.raw;
+    reinterpret_cast<uint4*>(result)[v] = out.raw;
   }
 }
 // Range [begin, end) in elements, both multiples of 16 / sizeof(T); every pointer 16-byte aligned.  Returns false if
@@ -305,8 +308,9 @@ template <typename T, int OP>
 __device__ __forceinline__ bool reduce_bulk(const State& s, int nsrc, const T* const* srcs, int ndst, T* const* dsts, size_t begin,
                                             size_t end, char* smem) {
   __shared__ int bulk_ok;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBulkStages * kBulkStageBytes);
-  const uint32_t chunk = (kBulkStageBytes / nsrc) & ~127u;            // bytes per source and stage
+  char* results = smem + kBulkStages * kBulkStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(results + 2 * kBulkOutBytes);
+  const uint32_t chunk = min((kBulkStageBytes / nsrc) & ~127u, kBulkOutBytes);   // bytes per source and stage
   const size_t bytes = (end - begin) * sizeof(T);
   const size_t nchunks = (bytes + chunk - 1) / chunk;
   if (threadIdx.x == 0) {
@@ -316,19 +320,26 @@ __device__ __forceinline__ bool reduce_bulk(const State& s, int nsrc, const T* c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  auto issue = [&](size_t c) {           // thread 0: chunk c of every source into stage c % kBulkStages
+  // The first warp moves the data, a lane per source and per destination with the address in a register: one thread that
+  // issues eight copies from a table of pointers holds up the block for longer than the reduction of a stage takes.
+  const int lane = threadIdx.x;
+  const bool mover = threadIdx.x < 32;
+  const char* my_src = mover && lane < nsrc ? reinterpret_cast<const char*>(srcs[lane] + begin) : nullptr;
+  char* my_dst = mover && lane < ndst ? reinterpret_cast<char*>(dsts[lane] + begin) : nullptr;
+  auto issue = [&](size_t c) {           // first warp: chunk c of every source into stage c % kBulkStages
     const int st = (int)(c % kBulkStages);
     const uint32_t nb = (uint32_t)((c + 1) * (size_t)chunk <= bytes ? chunk : bytes - c * (size_t)chunk);
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bars[st]);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb * (uint32_t)nsrc) : "memory");
-    for (int k = 0; k < nsrc; ++k) {
-      const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem + (size_t)st * kBulkStageBytes + (size_t)k * chunk);
-      const char* g = reinterpret_cast<const char*>(srcs[k] + begin) + c * (size_t)chunk;
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb * (uint32_t)nsrc) : "memory");
+    __syncwarp();
+    if (my_src) {
+      const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem + (size_t)st * kBulkStageBytes + (size_t)lane * chunk);
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                   ::"r"(sm), "l"(g), "r"(nb), "r"(bar) : "memory");
+                   ::"r"(sm), "l"(my_src + c * (size_t)chunk), "r"(nb), "r"(bar) : "memory");
     }
   };
-  if (threadIdx.x == 0)
+  if (mover)
     for (size_t c = 0; c < nchunks && c < (size_t)kBulkStages; ++c) issue(c);
   const unsigned long long t0 = dev::timer();
   for (size_t c = 0; c < nchunks; ++c) {
@@ -350,16 +361,26 @@ __device__ __forceinline__ bool reduce_bulk(const State& s, int nsrc, const T* c
     if (!bulk_ok) break;
     const uint32_t nb = (uint32_t)((c + 1) * (size_t)chunk <= bytes ? chunk : bytes - c * (size_t)chunk);
     const char* stage = smem + (size_t)st * kBulkStageBytes;
-    const size_t v_base = (begin * sizeof(T) + c * (size_t)chunk) >> 4;          // 16-byte vector index in the tensors
+    char* result = results + (c & 1) * kBulkOutBytes;
     switch (nsrc) {
-      case 2: reduce_stage<T, OP, 2>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
-      case 4: reduce_stage<T, OP, 4>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
-      case 8: reduce_stage<T, OP, 8>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base); break;
-      default: reduce_stage<T, OP, 0>(stage, chunk, nb >> 4, nsrc, ndst, dsts, v_base);
+      case 2: reduce_stage<T, OP, 2>(stage, chunk, nb >> 4, nsrc, result); break;
+      case 4: reduce_stage<T, OP, 4>(stage, chunk, nb >> 4, nsrc, result); break;
+      case 8: reduce_stage<T, OP, 8>(stage, chunk, nb >> 4, nsrc, result); break;
+      default: reduce_stage<T, OP, 0>(stage, chunk, nb >> 4, nsrc, result);
     }
-    __syncthreads();                       // the stage has been read by everybody: refill it
-    if (threadIdx.x == 0 && c + kBulkStages < nchunks) issue(c + kBulkStages);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copies below read what this thread has parked
+    __syncthreads();                       // the stage has been read by everybody and the result is complete
+    if (mover) {
+      if (c + kBulkStages < nchunks) issue(c + kBulkStages);
+      if (my_dst)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                     ::"l"(my_dst + c * (size_t)chunk), "r"((uint32_t)__cvta_generic_to_shared(result)), "r"(nb) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      // the other buffer is parked into next (behind the barrier at the top): its copies must have read it
+      asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    }
   }
+  if (mover) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // every result has been written
   __syncthreads();
   return bulk_ok != 0;
 }
@@ -651,17 +672,33 @@ __device__ __forceinline__ int team_broadcast(const State& s, const Team& t, voi
 }
 
 // fcollect (all-gather): my source lands in block my_idx of every member's dest.
+// With `bulk` (kMoveSmemBytes of 128-byte aligned dynamic shared memory) a block's share of at least kMoveMinBytes goes
+// through shared memory with bulk copies: the source is read once for all destinations, and a block is not limited by the
+// loads that its threads keep in flight.
+constexpr int kMoveStages = 4, kMoveChunk = 32 * 1024;
+constexpr uint32_t kMoveSmemBytes = kMoveStages * kMoveChunk + 64;
+constexpr size_t kMoveMinBytes = 32 * 1024;
+__device__ __forceinline__ bool moves_in_bulk(const char* bulk, const void* dest, const void* source, size_t nbytes, size_t share) {
+  return bulk != nullptr && share >= kMoveMinBytes && ((reinterpret_cast<uintptr_t>(dest) | reinterpret_cast<uintptr_t>(source) | nbytes) & 15) == 0;
+}
 __device__ __forceinline__ int team_fcollect(const State& s, const Team& t, void* dest, const void* source, size_t nbytes,
-                                             int cta = 0, int ncta = 1) {
+                                             int cta = 0, int ncta = 1, char* bulk = nullptr) {
   const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);          // every member's dest may be overwritten
   if (rc != BSHMEM_OK) return rc;
   size_t b, e;
   split_range(nbytes, ncta, cta, 16, &b, &e);
-  for (int k = 0; k < t.size; ++k) {
-    int peer_idx = (t.my_idx + k) % t.size;   // stagger the targets so the PEs do not gang up on one peer
-    char* d = dev::ptr(s, reinterpret_cast<char*>(dest), dev::team_pe(t, peer_idx)) + (size_t)t.my_idx * nbytes;
-    dev::copy_bytes<dev::BLOCK>(d + b, reinterpret_cast<const char*>(source) + b, e - b);
+  // stagger the targets so the PEs do not gang up on one peer
+  auto target = [&](int k) {
+    return dev::ptr(s, reinterpret_cast<char*>(dest), dev::team_pe(t, (t.my_idx + k) % t.size)) + (size_t)t.my_idx * nbytes + b;
+  };
+  const char* mine = reinterpret_cast<const char*>(source) + b;
+  if (moves_in_bulk(bulk, dest, source, nbytes, e - b)) {
+    rc = dev::bulk_segments<kMoveStages, kMoveChunk>(s, 1, e - b, t.size, [&](int) { return mine; }, [&](int, int k) { return target(k); }, bulk,
+                                                     reinterpret_cast<uint64_t*>(bulk + kMoveStages * kMoveChunk));
+    if (rc != BSHMEM_OK) return rc;
+  } else {
+    for (int k = 0; k < t.size; ++k) dev::copy_bytes<dev::BLOCK>(target(k), mine, e - b);
   }
   if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);
@@ -669,17 +706,22 @@ __device__ __forceinline__ int team_fcollect(const State& s, const Team& t, void
 
 // alltoall: block j of my source lands in block my_idx of member j's dest.
 __device__ __forceinline__ int team_alltoall(const State& s, const Team& t, void* dest, const void* source, size_t nbytes,
-                                             int cta = 0, int ncta = 1) {
+                                             int cta = 0, int ncta = 1, char* bulk = nullptr) {
   const unsigned long long cap = dev::trace_capacity(s);
   int rc = team_sync(s, t, cta);
   if (rc != BSHMEM_OK) return rc;
   size_t b, e;
   split_range(nbytes, ncta, cta, 16, &b, &e);
-  for (int k = 0; k < t.size; ++k) {
-    int j = (t.my_idx + k) % t.size;
-    char* d = dev::ptr(s, reinterpret_cast<char*>(dest), dev::team_pe(t, j)) + (size_t)t.my_idx * nbytes;
-    const char* sp = reinterpret_cast<const char*>(source) + (size_t)j * nbytes;
-    dev::copy_bytes<dev::BLOCK>(d + b, sp + b, e - b);
+  auto from = [&](int k) { return reinterpret_cast<const char*>(source) + (size_t)((t.my_idx + k) % t.size) * nbytes + b; };
+  auto to = [&](int k) {
+    return dev::ptr(s, reinterpret_cast<char*>(dest), dev::team_pe(t, (t.my_idx + k) % t.size)) + (size_t)t.my_idx * nbytes + b;
+  };
+  if (moves_in_bulk(bulk, dest, source, nbytes, e - b)) {
+    rc = dev::bulk_segments<kMoveStages, kMoveChunk>(s, t.size, e - b, 1, from, [&](int k, int) { return to(k); }, bulk,
+                                                     reinterpret_cast<uint64_t*>(bulk + kMoveStages * kMoveChunk));
+    if (rc != BSHMEM_OK) return rc;
+  } else {
+    for (int k = 0; k < t.size; ++k) dev::copy_bytes<dev::BLOCK>(to(k), from(k), e - b);
   }
   if (cta == 0 && threadIdx.x == 0) { dev::stat(s, BSHMEM_DSTAT_COLL); dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, 0); }
   return team_barrier(s, t, cta);

@@ -82,7 +82,7 @@ typedef struct {
   unsigned long long* stats;           /* device counters (BSHMEM_DSTAT_*), or null              */
   void* proxy;                         /* reverse-offload ring descriptor, or null               */
   uint32_t debug;
-  uint32_t reserved;
+  uint32_t one_gpu;                    /* every PE lives on this GPU: GPU scope orders accesses for all of them */
 } bshmem_dev_state_t;
 
 enum {
@@ -191,9 +191,15 @@ __device__ __forceinline__ bool check_target(const State& s, const void* sym, si
 // fence: puts issued before it are delivered to each PE before puts issued after it.
 // quiet: every outstanding put/get/atomic of this thread is complete and visible.
 // With a load/store transport both are a system-scope fence.
-__device__ __forceinline__ void fence(const State& s) { asm volatile("fence.acq_rel.sys;" ::: "memory"); stat(s, BSHMEM_DSTAT_FENCE); }
+// Orders the thread's earlier accesses before its later ones as every PE sees them.  A system-scope fence takes 3 to 4 us on
+// a busy GPU, a GPU-scope one less than 1; the latter does when all PEs share the GPU.
+__device__ __forceinline__ void fence_peers(const State& s) {
+  if (s.one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  else asm volatile("fence.acq_rel.sys;" ::: "memory");
+}
+__device__ __forceinline__ void fence(const State& s) { fence_peers(s); stat(s, BSHMEM_DSTAT_FENCE); }
 __device__ __forceinline__ void fence_pe(const State& s, int) { fence(s); }
-__device__ __forceinline__ void quiet(const State& s) { asm volatile("fence.acq_rel.sys;" ::: "memory"); stat(s, BSHMEM_DSTAT_QUIET); }
+__device__ __forceinline__ void quiet(const State& s) { fence_peers(s); stat(s, BSHMEM_DSTAT_QUIET); }
 __device__ __forceinline__ void threadfence_system() { __threadfence_system(); }
 
 // ---- the copy engine: 16-byte vectors when both sides allow it ---------------------------
@@ -253,10 +259,12 @@ __device__ __forceinline__ void copy_bytes(char* __restrict__ dst, const char* _
 // One thread drives a ring of kStages chunks: cp.async.bulk global -> shared (completion on an mbarrier), then
 // cp.async.bulk shared -> global (bulk-group completion).  Either side may be a peer's memory; nothing here is a
 // multicast copy.  No registers carry payload, so one CTA keeps (kStages - 1) * kChunk bytes of loads in flight.
-// Needs 16-byte aligned src, dst and n, `smem` of kStages * kChunk bytes (16-byte aligned) plus kStages mbarriers.
+// nseg segments of n bytes, segment i from src(i) to each of dst(i, 0) .. dst(i, ndst - 1): a segment that goes to several
+// places is read once, and there is no pause between segments.
+// Needs 16-byte aligned addresses and n, `smem` of kStages * kChunk bytes (16-byte aligned) plus kStages mbarriers.
 // Block scope: every thread calls; returns BSHMEM_OK or BSHMEM_ERR_TIMEOUT (a bounded mbarrier wait ran out).
-template <int kStages, int kChunk>
-__device__ __forceinline__ int bulk_copy_block(const State& s, char* dst, const char* src, size_t n, char* smem, uint64_t* bars) {
+template <int kStages, int kChunk, class Src, class Dst>
+__device__ __forceinline__ int bulk_segments(const State& s, int nseg, size_t n, int ndst, Src src, Dst dst, char* smem, uint64_t* bars) {
   __shared__ int bulk_status;
   if (threadIdx.x == 0) {
     bulk_status = BSHMEM_OK;
@@ -266,15 +274,20 @@ __device__ __forceinline__ int bulk_copy_block(const State& s, char* dst, const 
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    const size_t nchunks = (n + kChunk - 1) / kChunk;
-    auto issue_load = [&](size_t k) {
+    const size_t per_seg = (n + kChunk - 1) / kChunk, nchunks = per_seg * nseg;
+    struct Cursor { int seg; size_t at; };             // segment and chunk within it
+    Cursor ld{0, 0}, st_c{0, 0};
+    auto advance = [&](Cursor& c) { if (++c.at == per_seg) { c.at = 0; ++c.seg; } };
+    auto chunk_bytes = [&](const Cursor& c) { return (uint32_t)((c.at + 1) * (size_t)kChunk <= n ? kChunk : n - c.at * (size_t)kChunk); };
+    auto issue_load = [&](size_t k) {                  // chunks are loaded in order: `ld` is chunk k
       const int st = (int)(k % kStages);
-      const uint32_t bytes = (uint32_t)((k + 1) * (size_t)kChunk <= n ? kChunk : n - k * (size_t)kChunk);
+      const uint32_t bytes = chunk_bytes(ld);
       const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bars[st]);
       const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem + (size_t)st * kChunk);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                   ::"r"(sm), "l"(src + k * (size_t)kChunk), "r"(bytes), "r"(bar) : "memory");
+                   ::"r"(sm), "l"(src(ld.seg) + ld.at * (size_t)kChunk), "r"(bytes), "r"(bar) : "memory");
+      advance(ld);
     };
     for (size_t k = 0; k < nchunks && k < (size_t)(kStages - 1); ++k) issue_load(k);
     const unsigned long long t0 = timer();
@@ -288,16 +301,19 @@ __device__ __forceinline__ int bulk_copy_block(const State& s, char* dst, const 
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         if (ok) break;
         if ((++it & 63) == 0 && timer() - t0 > s.timeout_ns) {
-          record_error(s, BSHMEM_ERR_TIMEOUT, -1, BSHMEM_WHERE_MBARRIER, (uint64_t)(src + i * (size_t)kChunk), i, 0);
+          record_error(s, BSHMEM_ERR_TIMEOUT, -1, BSHMEM_WHERE_MBARRIER, (uint64_t)(src(st_c.seg) + st_c.at * (size_t)kChunk), i, 0);
           bulk_status = BSHMEM_ERR_TIMEOUT;
           break;
         }
       }
       if (!ok) break;
-      const uint32_t bytes = (uint32_t)((i + 1) * (size_t)kChunk <= n ? kChunk : n - i * (size_t)kChunk);
+      const uint32_t bytes = chunk_bytes(st_c);
       const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem + (size_t)st * kChunk);
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + i * (size_t)kChunk), "r"(sm), "r"(bytes) : "memory");
+      for (int d = 0; d < ndst; ++d)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                     ::"l"(dst(st_c.seg, d) + st_c.at * (size_t)kChunk), "r"(sm), "r"(bytes) : "memory");
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      advance(st_c);
       // chunk i + kStages - 1 goes into the stage chunk i - 1 was stored from: that store must have read its data
       const size_t nxt = i + kStages - 1;
       if (nxt < nchunks) {
@@ -311,6 +327,10 @@ __device__ __forceinline__ int bulk_copy_block(const State& s, char* dst, const 
   const int rc = bulk_status;
   __syncthreads();
   return rc;
+}
+template <int kStages, int kChunk>
+__device__ __forceinline__ int bulk_copy_block(const State& s, char* dst, const char* src, size_t n, char* smem, uint64_t* bars) {
+  return bulk_segments<kStages, kChunk>(s, 1, n, 1, [&](int) { return src; }, [&](int, int) { return dst; }, smem, bars);
 }
 
 // ---- RMA ------------------------------------------------------------------------------------
@@ -358,6 +378,10 @@ __device__ __forceinline__ T g(const State& s, const T* src, int pe) {
   return *reinterpret_cast<const volatile T*>(ptr(s, src, pe));
 }
 
+__device__ __forceinline__ void signal_update(uint64_t* sig, uint64_t value, int sig_op) {
+  if (sig_op == BSHMEM_SIGNAL_ADD) asm volatile("red.relaxed.sys.global.add.u64 [%0], %1;" ::"l"(sig), "l"(value) : "memory");
+  else asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(sig), "l"(value) : "memory");
+}
 // put-with-signal (OpenSHMEM 1.5): the payload is visible to whoever observes the signal update.
 template <Scope S = THREAD>
 __device__ __forceinline__ void putmem_signal(const State& s, void* dest, const void* src, size_t n, uint64_t* sig_addr,
@@ -367,9 +391,8 @@ __device__ __forceinline__ void putmem_signal(const State& s, void* dest, const 
   scope_sync<S>();   // every participant's stores are ordered before the leader's release
   if (scope_rank<S>() == 0) {
     uint64_t* rs = ptr(s, sig_addr, pe);
-    asm volatile("fence.acq_rel.sys;" ::: "memory");
-    if (sig_op == BSHMEM_SIGNAL_ADD) asm volatile("red.release.sys.global.add.u64 [%0], %1;" ::"l"(rs), "l"(signal) : "memory");
-    else asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(rs), "l"(signal) : "memory");
+    fence_peers(s);    // with the barrier above, the release; the signal itself can be relaxed
+    signal_update(rs, signal, sig_op);
     stat(s, BSHMEM_DSTAT_PUT_SIGNAL);
     trace(s, BSHMEM_TRACE_PUT_SIGNAL, pe, n);
     stat(s, BSHMEM_DSTAT_BYTES_PUT, n);
@@ -476,21 +499,32 @@ template <typename T> __device__ __forceinline__ T load_acquire_sys(const T* p) 
   else { uint32_t w; asm volatile("ld.acquire.sys.global.u8 %0, [%1];" : "=r"(w) : "l"(p) : "memory"); uint8_t b = (uint8_t)w; memcpy(&v, &b, 1); }
   return v;
 }
+template <typename T> __device__ __forceinline__ T load_acquire_gpu(const T* p) {
+  T v;
+  if constexpr (sizeof(T) == 8) { uint64_t w; asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory"); memcpy(&v, &w, 8); }
+  else if constexpr (sizeof(T) == 4) { uint32_t w; asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(w) : "l"(p) : "memory"); memcpy(&v, &w, 4); }
+  else if constexpr (sizeof(T) == 2) { uint16_t w; asm volatile("ld.acquire.gpu.global.u16 %0, [%1];" : "=h"(w) : "l"(p) : "memory"); memcpy(&v, &w, 2); }
+  else { uint32_t w; asm volatile("ld.acquire.gpu.global.u8 %0, [%1];" : "=r"(w) : "l"(p) : "memory"); uint8_t b = (uint8_t)w; memcpy(&v, &b, 1); }
+  return v;
+}
+template <typename T> __device__ __forceinline__ T load_acquire(const State& s, const T* p) {
+  return s.one_gpu ? load_acquire_gpu(p) : load_acquire_sys(p);
+}
 template <typename T>
-__device__ __forceinline__ int test(const State&, const T* ivar, int cmp, T value) {
-  return cmp_holds(cmp, load_acquire_sys(ivar), value) ? 1 : 0;
+__device__ __forceinline__ int test(const State& s, const T* ivar, int cmp, T value) {
+  return cmp_holds(cmp, load_acquire(s, ivar), value) ? 1 : 0;
 }
 // Spins on local symmetric memory until `*ivar cmp value`, at most state.timeout_ns.
 // Returns BSHMEM_OK or BSHMEM_ERR_TIMEOUT (and fills the error record).
 template <typename T>
 __device__ __forceinline__ int wait_until(const State& s, const T* ivar, int cmp, T value, uint32_t where = BSHMEM_WHERE_WAIT_UNTIL, int pe = -1) {
-  T seen = load_acquire_sys(ivar);
+  T seen = load_acquire(s, ivar);
   if (cmp_holds(cmp, seen, value)) return BSHMEM_OK;
   unsigned long long t0 = timer();
   const unsigned long long cap = trace_capacity(s);
   unsigned it = 0;
   while (true) {
-    seen = load_acquire_sys(ivar);
+    seen = load_acquire(s, ivar);
     if (cmp_holds(cmp, seen, value)) break;
     if ((++it & 31) == 0) {
       if (timer() - t0 > s.timeout_ns) {

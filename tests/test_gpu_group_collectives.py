@@ -41,3 +41,26 @@ def test_group_reductions(pes, dtype):
                     assert torch.equal(t[:share].double(), total[pe * share:(pe + 1) * share]) and bool((t[share:] == 99).all())
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("pes,ctas", [(2, 1), (3, 5), (8, 16), (8, 18)])
+@pytest.mark.parametrize("nbytes", [16, 32 * KIB - 16, 32 * KIB, 96 * KIB + 16, 160 * KIB + 8, 700 * KIB + 48])
+def test_group_moves(pes, ctas, nbytes):
+    """fcollect and alltoall on both sides of the size and the alignment from which blocks move their share with bulk copies,
+    and shares that do not fill the last chunk."""
+    from roc_shmem_b200.gpu import COLL_ALLTOALL, COLL_FCOLLECT, LocalGroup
+    g = LocalGroup(pes, heap_bytes=64 << 20)
+    try:
+        torch.manual_seed(nbytes)
+        src, dst = g.empty((pes * nbytes,), torch.uint8), g.empty((pes * nbytes + 64,), torch.uint8)
+        for kind in (COLL_FCOLLECT, COLL_ALLTOALL):
+            for s, d in zip(src, dst):
+                s.copy_(torch.randint(0, 256, s.shape, device="cuda", dtype=torch.uint8))
+                d.fill_(7)
+            torch.cuda.synchronize()
+            g.collective(kind, dst, src, nbytes, ctas=ctas)
+            for me, d in enumerate(dst):
+                part = slice(0, nbytes) if kind == COLL_FCOLLECT else slice(me * nbytes, (me + 1) * nbytes)
+                assert torch.equal(d[:pes * nbytes], torch.cat([s[part] for s in src])) and bool((d[pes * nbytes:] == 7).all())
+    finally:
+        g.close()
