@@ -24,7 +24,7 @@ from . import _native
 from .bootstrap import Bootstrap
 from .config import Config
 from .cpu import native_config
-from .runtime import Runtime, _ptr_of
+from .runtime import Context, Runtime, _ptr_of
 from .utils import dtypes as D
 from .utils.errors import ShmemError, raise_for_status
 
@@ -39,7 +39,7 @@ class DevState(C.Structure):
     _fields_ = [("my_pe", C.c_int32), ("n_pes", C.c_int32), ("heap_bytes", C.c_uint64),
                 ("heap_base", C.c_void_p * 16), ("mc_base", C.c_void_p), ("err", C.c_void_p),
                 ("timeout_ns", C.c_ulonglong), ("stats", C.c_void_p), ("proxy", C.c_void_p),
-                ("debug", C.c_uint32), ("reserved", C.c_uint32)]
+                ("debug", C.c_uint32), ("one_gpu", C.c_uint32)]
 
 
 DSTAT_NAMES = ("put", "get", "put_signal", "p", "g", "amo", "fence", "quiet", "wait", "wait_ns", "barrier",
@@ -138,10 +138,33 @@ def _gpu_error(lib, what: str, status: int) -> None:
         raise_for_status(status, f"{what}: {msg.decode() if msg else ''}")
 
 
+class DeviceContext(Context):
+    """Context of a DeviceRuntime: messages between device buffers go straight to the native call."""
+
+    def put(self, dest, src, pe, *, nbi=False, nbytes=None):
+        rt = self.rt
+        if isinstance(src, Tensor) and src.get_device() == rt._dev_index and isinstance(dest, Tensor):
+            st = rt._c_put_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), src.nbytes if nbytes is None else nbytes, pe, nbi)
+            if st:
+                rt._check(st)
+            return
+        rt.put(dest, src, pe, ctx=self, nbi=nbi, nbytes=nbytes)
+
+    def get(self, dest, src, pe, *, nbi=False, nbytes=None):
+        rt = self.rt
+        if isinstance(dest, Tensor) and dest.get_device() == rt._dev_index and isinstance(src, Tensor):
+            st = rt._c_get_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), dest.nbytes if nbytes is None else nbytes, pe, nbi)
+            if st:
+                rt._check(st)
+            return
+        rt.get(dest, src, pe, ctx=self, nbi=nbi, nbytes=nbytes)
+
+
 class DeviceRuntime(Runtime):
     """Runtime over the NVLink backend, plus the GPU-only knobs."""
 
     backend = "device"
+    _context_type = DeviceContext
 
     def __init__(self, lib, handle, device: torch.device, heap, own_heap: bool = True):
         super().__init__(lib, handle,
@@ -158,7 +181,7 @@ class DeviceRuntime(Runtime):
     # small messages without a copy-engine request); anything else takes the general path
     def put(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
         """Copy `src` (any local buffer) into `dest`'s location on PE `pe`."""
-        if isinstance(src, Tensor) and src.is_cuda and src.get_device() == self._dev_index and isinstance(dest, Tensor):
+        if isinstance(src, Tensor) and src.get_device() == self._dev_index and isinstance(dest, Tensor):
             st = self._c_put_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
                                  src.nbytes if nbytes is None else nbytes, pe, nbi)
             if st:
@@ -168,7 +191,7 @@ class DeviceRuntime(Runtime):
 
     def get(self, dest, src, pe: int, *, ctx=None, nbi: bool = False, nbytes: Optional[int] = None) -> None:
         """Copy `src`'s location on PE `pe` into the local buffer `dest`."""
-        if isinstance(dest, Tensor) and dest.is_cuda and dest.get_device() == self._dev_index and isinstance(src, Tensor):
+        if isinstance(dest, Tensor) and dest.get_device() == self._dev_index and isinstance(src, Tensor):
             st = self._c_get_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
                                  dest.nbytes if nbytes is None else nbytes, pe, nbi)
             if st:
@@ -179,7 +202,7 @@ class DeviceRuntime(Runtime):
     def put_signal(self, dest, src, sig, value: int, pe: int, *, op: int = D.SIGNAL_SET, ctx=None, nbi: bool = False) -> None:
         """Put, then update the 64-bit signal word `sig` on PE `pe` (SET or ADD);
         the payload is visible to a reader that observed the signal."""
-        if isinstance(src, Tensor) and src.is_cuda and src.get_device() == self._dev_index and isinstance(dest, Tensor):
+        if isinstance(src, Tensor) and src.get_device() == self._dev_index and isinstance(dest, Tensor):
             st = self._c_put_signal_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(), src.nbytes,
                                         _ptr_of(sig), value, op, pe, nbi)
             if st:

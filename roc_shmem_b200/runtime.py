@@ -128,6 +128,8 @@ class Context:
 
 
 class Runtime:
+    _context_type = Context
+
     def __init__(self, lib: C.CDLL, handle: int, *, tensor_from_ptr: Callable, device: torch.device,
                  on_finalize: Optional[Callable] = None):
         self.lib = lib
@@ -273,7 +275,7 @@ class Runtime:
         out = C.c_int32(-1)
         tm = team or self.team_world
         self._check(self.lib.bshmem_team_create_ctx(self.h, tm.slot, options, C.byref(out)))
-        return Context(self, out.value, options, tm)
+        return self._context_type(self, out.value, options, tm)
 
     def team_split_strided(self, parent: Optional[Team], start: int, stride: int, size: int) -> Team:
         out = C.c_int32(-1)
