@@ -247,6 +247,9 @@ struct PolicyDefaults {
   template <class Params, class St> __device__ static __forceinline__ void epilogue_drain(const Params&, const Smem&, St&, int, int, Guard&) {}
   template <class Params> __device__ static __forceinline__ void tail(const Params&, const Smem&, Guard&) {}
   template <class Params> __device__ static __forceinline__ void prologue(const Params&, Guard&) {}
+  // kTileTable: fill_tile_table(prm) runs in every thread before the first tile_coords().
+  static constexpr bool kTileTable = false;
+  template <class Params> __device__ static __forceinline__ void fill_tile_table(const Params&) {}
 };
 
 // Parks 64 bf16 columns of the warp's 32 rows (row = lane) in its staging buffer for a TMA store: eight 16-byte pieces per
@@ -314,7 +317,6 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   const uint32_t rank = crank & 1, lead = crank & ~1u;   // the pair's first CTA issues the MMAs
   const int S = P::kSplit ? cp.split : 1;
   const int pair = blockIdx.x / (2 * S), num_pairs = gridDim.x / (2 * S);    // split form: index and number of tiles
-  const int num_tiles = P::num_tiles(prm);
   // k-blocks of a tile that this pair multiplies
   auto kb_range = [&](int m_blk, int* kb0, int* kb1) {
     const int n = P::num_kb(prm, m_blk), j = P::kSplit ? (int)(crank >> 1) : 0;
@@ -353,6 +355,11 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   // launched with programmatic serialization, the set-up above overlaps the previous kernel; without, this is a no-op
   ptx::grid_dependency_wait();
   if (threadIdx.x == 64) P::prologue(prm, g);
+  if constexpr (P::kTileTable) {
+    P::fill_tile_table(prm);
+    __syncthreads();
+  }
+  const int num_tiles = P::num_tiles(prm);            // may come from device memory: behind the wait
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------

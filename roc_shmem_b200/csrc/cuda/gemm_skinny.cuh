@@ -275,7 +275,6 @@ namespace bshmem {
 namespace skinny {
 
 constexpr int MAX_GROUPS = 64, MAX_GROUP_STAGES = 12;
-constexpr int XBOX = 16;                           // token rows per TMA box
 constexpr uint32_t GROUP_XCHG_BYTES = 2 * 2 * 16 * 32 * 4;             // two warp pairs x two buffers x 16 tokens x 32 columns
 constexpr uint32_t GROUP_CTRL_BYTES = 8 * (2 * MAX_GROUP_STAGES + 6) + 16 + 4 * MAX_GROUPS;
 
@@ -285,6 +284,7 @@ struct GroupedParams {
   long long ldo;
   const int* rows;
   int G, cap, N, K;
+  int xbox;                      // token rows per TMA box: 16, 32, 64 or 128
   uint32_t ring_bytes;           // shared memory of the stages
   uint32_t tmem_cols;            // two accumulators
   int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 256)
@@ -365,7 +365,7 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   int most = 1;
   for (int i = 0; i < p.G; ++i) most = max(most, L.rows()[i]);
   const int nt_max = min((most + 15) / 16 * 16, p.nt_cap);
-  const uint32_t stage = W_STAGE_BYTES + (uint32_t)nt_max * BK * 2;
+  const uint32_t stage = W_STAGE_BYTES + (uint32_t)((nt_max + p.xbox - 1) / p.xbox * p.xbox) * BK * 2;
   const int stages = min((int)(p.ring_bytes / stage), MAX_GROUP_STAGES);
   const int kb_all = (p.K + BK - 1) / BK;
   const int rank = p.split > 1 ? (int)cluster_rank() : 0;
@@ -386,14 +386,15 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
       for (int q = 0; q < p.P && ok; ++q) ok = gemm::wait_ge<true>(p.arrive + q, (unsigned long long)p.expected[q], g, ERR_G_ARRIVE);
       if (p.P) ptx::fence_proxy_async_all();         // peer stores (generic proxy) before the TMA reads
       while (ok && it.next(&grp, &n_blk, &tok0, &ntok)) {
-        const int boxes = (ntok + XBOX - 1) / XBOX;
+        const int boxes = (ntok + p.xbox - 1) / p.xbox;
+        const uint32_t box_bytes = (uint32_t)p.xbox * BK * 2;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_G_PRODUCER_EMPTY)) { ok = false; break; }
           const uint32_t w = L.base + s * stage, x = w + W_STAGE_BYTES;
-          ptx::mbar_arrive_expect_tx(L.full(s), W_STAGE_BYTES + boxes * (XBOX * BK * 2));
+          ptx::mbar_arrive_expect_tx(L.full(s), W_STAGE_BYTES + boxes * box_bytes);
           ptx::tma_load_2d(w, &p.map_w, L.full(s), kb * BK, grp * p.N + n_blk * ROWS);
           for (int b = 0; b < boxes; ++b)
-            ptx::tma_load_2d(x + b * (XBOX * BK * 2), &p.map_x, L.full(s), kb * BK, grp * p.cap + tok0 + b * XBOX);
+            ptx::tma_load_2d(x + b * box_bytes, &p.map_x, L.full(s), kb * BK, grp * p.cap + tok0 + b * p.xbox);
           if (++s == stages) { s = 0; ph ^= 1; }
         }
       }

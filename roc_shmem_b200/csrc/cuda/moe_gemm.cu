@@ -70,10 +70,14 @@ struct Grouped : PolicyDefaults {
       if (tile < tg) break;
       tile -= tg;
     }
-    int per = p.group_m * p.core.num_n_blocks;
-    int sg = tile / per, first = sg * p.group_m;
-    int rows = min(p.group_m, mb_g - first);
-    int in = tile - sg * per;
+    coords_in_group(p, g, mb_g, tile, m_blk, n_blk);
+  }
+  // tile number `tile` of group g, which has `blocks` row blocks
+  __device__ static __forceinline__ void coords_in_group(const Params& p, int g, int blocks, int tile, int* m_blk, int* n_blk) {
+    const int per = p.group_m * p.core.num_n_blocks;
+    const int sg = tile / per, first = sg * p.group_m;
+    const int rows = min(p.group_m, blocks - first);
+    const int in = tile - sg * per;
     *m_blk = g * p.a_blocks_per_group + first + in % rows;
     *n_blk = in / rows;
   }
@@ -157,6 +161,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) grouped_gemm_tn_kernel(const _
 // the pair loads 128 rows of the A block and 128 rows of the B block, so the tensor maps have 128-row boxes.
 namespace g2 = bshmem::gemm2;
 
+constexpr int kTableGroups = 64;
+
 template <bool kGatedEpi>
 struct GroupedPair : g2::PolicyDefaults {
   using Params = GroupedParams;
@@ -165,9 +171,41 @@ struct GroupedPair : g2::PolicyDefaults {
   __device__ static __forceinline__ const CoreParams& core(const Params& p) { return p.core; }
   __device__ static __forceinline__ const CUtensorMap* map_a(const Params& p) { return &p.map_a; }
   __device__ static __forceinline__ const CUtensorMap* map_b(const Params& p) { return &p.map_b; }
-  __device__ static __forceinline__ int num_tiles(const Params& p) { return Base::num_tiles(p); }
+  // First tile of every group, in shared memory: walking the groups' counts in global memory took every role of the CTA
+  // 1.5 us per tile with 64 groups.
+  static constexpr bool kTileTable = true;
+  __device__ static __forceinline__ int* tile_starts() {
+    __shared__ int starts[kTableGroups + 1];
+    return starts;
+  }
+  __device__ static __forceinline__ int group_blocks(const Params& p, int g) { return (Base::group_rows(p, g) + g2::BM - 1) / g2::BM; }
+  __device__ static __forceinline__ void fill_tile_table(const Params& p) {
+    if (p.G > kTableGroups || threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    int before = 0;
+    for (int g0 = 0; g0 < p.G; g0 += 32) {
+      const int mine = g0 + lane < p.G ? group_blocks(p, g0 + lane) * p.core.num_n_blocks : 0;
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      if (g0 + lane < p.G) tile_starts()[g0 + lane] = before + incl - mine;
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tile_starts()[p.G] = before;
+  }
+  __device__ static __forceinline__ int num_tiles(const Params& p) { return p.G > kTableGroups ? Base::num_tiles(p) : tile_starts()[p.G]; }
   __device__ static __forceinline__ void tile_coords(const Params& p, int tile, int* m_blk, int* n_blk) {
-    Base::tile_coords(p, tile, m_blk, n_blk);
+    if (p.G > kTableGroups) return Base::tile_coords(p, tile, m_blk, n_blk);
+    const int* starts = tile_starts();
+    int g = 0, end = p.G;                 // starts[g] <= tile < starts[end]; an empty group starts where the next one does
+    while (end - g > 1) {
+      const int mid = (g + end) >> 1;
+      if (starts[mid] <= tile) g = mid; else end = mid;
+    }
+    Base::coords_in_group(p, g, (starts[g + 1] - starts[g]) / p.core.num_n_blocks, tile - starts[g], m_blk, n_blk);
   }
   __device__ static __forceinline__ int a_row(const Params&, int m_blk) { return m_blk * g2::BM; }
   __device__ static __forceinline__ int b_row(const Params& p, int m_blk, int n_blk) {
@@ -180,8 +218,13 @@ struct GroupedPair : g2::PolicyDefaults {
     if (p.P) ptx::fence_proxy_async_all();   // peer stores (generic proxy) before the TMA reads
     return true;
   }
+  // whether row `row` of C belongs to its group's rows (those behind them are scratch inside the group's own region)
+  __device__ static __forceinline__ bool live(const Params& p, int row) {
+    const int per = p.a_blocks_per_group * g2::BM, g = row / per;
+    return row - g * per < Base::group_rows(p, g);
+  }
   __device__ static __forceinline__ void out_target(const Params& p, int row, int col, const CUtensorMap** map, int* x, int* y) {
-    *map = &p.map_c;       // rows beyond a group's count are scratch inside the group's own region
+    *map = live(p, row) ? &p.map_c : nullptr;        // 32 rows: none of them is the group's, nothing to write
     *x = col;
     *y = row;
   }
@@ -193,6 +236,7 @@ struct GroupedPair : g2::PolicyDefaults {
 struct GroupedPairAct : GroupedPair<false> {
   static constexpr bool kStoreAct = true;
   __device__ static __forceinline__ void store_act(const Params& p, int row, int col, const float (&f)[64]) {
+    if (!live(p, row)) return;
     uint4* dst = reinterpret_cast<uint4*>(p.act + row * p.ld_act + col / 2);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -219,9 +263,10 @@ struct GroupedPairSwigluBwd : GroupedPair<false> {
   static constexpr bool kSwigluBwd = true;
   __device__ static __forceinline__ void swiglu_grad(const Params& p, int row, int col, const float (&d)[32], float (&o)[64]) {
     const uint4* src = reinterpret_cast<const uint4*>(p.gu + row * p.ld_gu + 2 * col);
+    const bool used = live(p, row);
     uint4 v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = src[j];
+    for (int j = 0; j < 8; ++j) v[j] = used ? src[j] : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
@@ -464,8 +509,9 @@ int bshmem_moe_grouped_gemm_swiglu_bwd(const void* A, const void* B, const void*
 // max_rows and max_active bound the largest group and the number of groups with rows as far as the host knows them (the
 // tokens and the token-expert entries of a decode step).  Up to 64 groups, a_rows_per_group and N multiples of 256; rows of
 // C beyond a group's count are not written.
-// us, 8 groups, N x K = 28672 x 4096 gated: 8 rows each 285 against 406 for the 256-row tiles (weights at the measured copy
-// rate: 288), 64 rows 316 / 388, 128 rows 416 / 439, 200 rows 1062 / 384.
+// us, 8 groups, N x K = 28672 x 4096 gated: 8 rows each 285 against 380 for the 256-row tiles (weights at the measured copy
+// rate: 288), 64 rows 315 / 375, 100 rows 325 / 373, 128 rows 410 / 380 (some groups have more than the chunk of 128 rows
+// then and read their weights twice).
 int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, int a_rows_per_group, int N, int K, int lda, int ldb, int ldc,
                                 const int* rows_dev, int max_rows, int max_active, int gated, const void* arrive, const int* expected, int P,
                                 void* stream, int timeout_ms) {
@@ -494,6 +540,7 @@ int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, in
   while (p.split < 8 && tiles * p.split <= g_sms[dev] && kb >= 16 * p.split) p.split *= 2;
   const uint32_t fixed = 1024 + skinny::GROUP_CTRL_BYTES + (gated ? skinny::GROUP_XCHG_BYTES : 0);
   p.ring_bytes = (skinny::SMEM_HALF - fixed) & ~1023u;          // also holds a split tile's 512 bytes per token
+  p.xbox = max_rows <= 16 ? 16 : 32;     // a copy of 16 rows takes the copy unit as long as one of 32
   p.tmem_cols = 32;
   while (p.tmem_cols < 2u * p.nt_cap) p.tmem_cols *= 2;
   p.P = P; p.arrive = static_cast<const unsigned long long*>(arrive); p.expected = expected;
@@ -501,7 +548,7 @@ int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, in
   p.err = g_err_dev[dev];
   rc = host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, (uint64_t)G * N, K, ldb, skinny::ROWS, skinny::BK);
   if (rc) return rc;
-  rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, skinny::XBOX, skinny::BK);
+  rc = host::make_tmap_2d(&p.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, p.xbox, skinny::BK);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.split > 1 ? tiles * p.split : 2 * g_sms[dev]));

@@ -21,9 +21,11 @@ from .gemm import current_stream
 
 _declared = False
 SIG_FWD_DISPATCH, SIG_FWD_COMBINE, SIG_BWD_DISPATCH, SIG_BWD_COMBINE = range(4)
-# Average rows per expert up to which the weight-streaming GEMM is the faster one (it is up to 128 rows in a group; a router
-# spreads the tokens of a batch unevenly, and a group beyond 128 reads its weights twice)
-FEW_ROWS = 64
+# Average rows per expert up to which the weight-streaming GEMM is the faster one.  It is up to about 110 rows in a group (8
+# groups, N x K = 28672 x 4096, 100 rows: 325 us against 373), but a router spreads the tokens of a batch unevenly and a group
+# beyond 128 reads its weights twice.  Where its tiles of 128 columns do not occupy the chip and each is split over a cluster,
+# the reduction grows with the rows (16 groups, 1024 x 2048: 24 us against 23 with 24 rows, 30 against 24 with 64).
+FEW_ROWS, FEW_ROWS_SPLIT, FEW_TILES = 80, 32, 148
 
 
 class PlanDev(C.Structure):
@@ -291,7 +293,14 @@ class MoELayer:
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
         local = P == 1                                             # no row leaves this GPU: no signals, no return buffer
         # (every PE brings about as many tokens; a group has at most one row per token of each PE)
-        few = (P * T, P * n_entries) if P * n_entries <= FEW_ROWS * self.E else None
+        hint = (P * T, P * n_entries)
+
+        def few(cols):
+            """The hint if the product with `cols` columns is one for the weight-streaming GEMM, else None."""
+            limit = FEW_ROWS if G * cols // 128 > FEW_TILES else FEW_ROWS_SPLIT
+            return hint if hint[1] <= limit * self.E else None
+
+        few_up, few_down = few(2 * F), few(H)
         self.route(x)
         par = self.parity
         if local:
@@ -303,19 +312,20 @@ class MoELayer:
             wait = dict(arrive=self._sig_ptr(par, SIG_FWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # gate/up projection (waits on the arrival words inside the kernel), then SwiGLU, then down projection
         if self.training:
-            if few is None:
+            if few_up is None:
                 grouped_gemm_act(self.recv, self.w13.view(G * 2 * F, H), self.gu, self.hact, G, rows=self.recv_count,
                                  timeout_ms=self.timeout_ms, **wait)
             else:
                 grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms,
-                             few=few, **wait)
+                             few=few_up, **wait)
                 self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
-            self._x_in, self._few = x, few                         # the router's backward needs the layer input
+            self._x_in = x                                         # the router's backward needs the layer input
+            self._few_h, self._few_x = few(F), few_down
         else:
             grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.hact, G, rows=self.recv_count, gated=True,
-                         timeout_ms=self.timeout_ms, few=few, **wait)
+                         timeout_ms=self.timeout_ms, few=few_up, **wait)
         self.launches += 1
-        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms, few=few)
+        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms, few=few_down)
         self.launches += 1
         if local:
             self._chk(_fast.combine_local(self._plan_a, a["yexp"], a["topk_w"], a["topk_idx"], a["pos"], T, self.topk, H, a["out"], 0, s),
@@ -361,10 +371,10 @@ class MoELayer:
                                      H, a["recv_bwd"], 0, par, SIG_BWD_DISPATCH, self.ctas, s), "dispatch(bwd)")
             wait = dict(arrive=self._sig_ptr(par, SIG_BWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # d_hact = d_y · W2 (B operand = W2^T [F, H], K = H) and through SwiGLU to d_gu
-        if self._few is None:
+        if self._few_h is None:
             grouped_gemm_swiglu_bwd(dy, self.w2_t.view(G * F, H), self.gu, self.dgu, G, rows=rc, timeout_ms=self.timeout_ms, **wait)
         else:
-            grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few, **wait)
+            grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_h, **wait)
             self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
         # dW2 = d_y^T · hact: token-major operands straight into the MN-major tensor-core path
         if self.tn_gemm:
@@ -385,7 +395,7 @@ class MoELayer:
             self._chk(_fast.transpose_pad(a["dgu"], rc.data_ptr(), G, cap, 2 * F, ta2.data_ptr(), s), "transpose")
             self._chk(_fast.transpose_pad(self.xsave.data_ptr(), rc.data_ptr(), G, cap, H, tb2.data_ptr(), s), "transpose")
             grouped_gemm(ta2, tb2, self.dw13.view(G * 2 * F, H), G, fixed_rows=2 * F, klen=rc, timeout_ms=self.timeout_ms)
-        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few)
+        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_x)
         self.launches += 4
         if local:
             # d_x = sum over k of the experts' rows + the router path (d_logits · Wr), written once

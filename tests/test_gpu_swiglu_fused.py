@@ -29,7 +29,7 @@ def test_fused_swiglu_forward_and_backward(rows, F, K):
     torch.cuda.synchronize()
     assert moe_lib().bshmem_moe_gemm_error_site(1) == 0
     for g, n in enumerate(rows):
-        used, rest = slice(g * cap, g * cap + n), slice(g * cap + -(-n // 256) * 256, (g + 1) * cap)     # whole tiles
+        used, rest = slice(g * cap, g * cap + n), slice(g * cap + -(-n // 32) * 32, (g + 1) * cap)     # stored by 32 rows
         assert bool((gu[rest] == 7).all()) and bool((act[rest] == 7).all()) and bool((dgu[rest] == 7).all())
         if not n:
             continue
