@@ -300,6 +300,12 @@ struct GroupedPairTN : GroupedPair<false> {
     return n < 1 ? 1 : n;     // an empty group still runs one (all-zero) k-block so that C becomes 0
   }
   __device__ static __forceinline__ bool a_ready(const Params&, int, Guard&) { return true; }
+  // every row of a gradient is live (asking costs 8 % where a tile has one or two k-blocks)
+  __device__ static __forceinline__ void out_target(const Params& p, int row, int col, const CUtensorMap** map, int* x, int* y) {
+    *map = &p.map_c;
+    *x = col;
+    *y = row;
+  }
   __device__ static __forceinline__ void load_stage(const Params& p, const CUtensorMap* ma, const CUtensorMap* mb, uint32_t a_smem,
                                                     uint32_t b_smem, uint32_t bar, int kb, int, int, int m_blk, int n_blk, int rank) {
     const int g = m_blk / p.a_blocks_per_group;

@@ -94,10 +94,10 @@ def test_router_and_plan_more_forms(T, E, topk):
     test_router_and_plan(T, E, topk)
 
 
-@pytest.mark.parametrize("T,H,E,topk", [(1, 256, 8, 1), (37, 768, 8, 3), (100, 256, 64, 8), (2500, 2048, 8, 2), (4800, 1024, 12, 5)])
+@pytest.mark.parametrize("T,H,E,topk", [(1, 256, 8, 1), (32, 512, 64, 8), (33, 512, 24, 8), (37, 768, 8, 3), (100, 256, 64, 8), (2500, 2048, 8, 2), (4800, 1024, 12, 5)])
 def test_local_rows(T, H, E, topk):
-    """Dispatch, combine and their backward forms on one PE for every rounding of top-k, one token and four per warp, a
-    capacity that some entries exceed."""
+    """Plans of few entries and of more, dispatch, combine and their backward forms on one PE for every rounding of top-k, one
+    token and four per warp, a capacity that some entries exceed."""
     import roc_shmem_b200 as shmem
     from roc_shmem_b200.ops.moe import MoELayer, _fast
     rt = shmem.init("device", rank=0, world_size=1, heap_bytes=512 << 20, timeout_ms=5000)
@@ -113,6 +113,11 @@ def test_local_rows(T, H, E, topk):
         cap, s = layer.cap, torch.cuda.current_stream().cuda_stream
         idx, pos = layer.topk_idx[:T * topk].view(T, topk).long(), layer.pos[:T * topk].view(T, topk).long()
         live = pos < cap
+        seen = [0] * E
+        for e, q in zip(idx.view(-1).tolist(), pos.view(-1).tolist()):               # positions in entry order
+            assert q == seen[e]
+            seen[e] += 1
+        assert layer.recv_count.tolist() == [min(c, cap) for c in seen]
         row = (idx * cap + pos.clamp(max=cap - 1))
         assert torch.equal(layer.recv[row[live]], x.view(T, 1, H).expand(T, topk, H)[live])
         y = torch.randn(E * cap, H, device="cuda").to(torch.bfloat16)
