@@ -63,7 +63,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     K, M = sa if a_mn else sa[::-1]
     N = sb[b_mn]
     if out is None:
-        out = torch.empty((M, N), dtype=_BF16, device=a.device)
+        out = a.new_empty((M, N))
         ldc = N
     else:
         if out.shape != (M, N) or out.dtype is not _BF16 or out.stride(1) != 1:
