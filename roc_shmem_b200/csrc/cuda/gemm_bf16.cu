@@ -151,7 +151,9 @@ struct SkinnyPlan {
 //    against 17.2 for two CTAs of three stages), unless the tiles alone nearly fill the chip and only half-size CTAs
 //    can split (4096x14336: 25.8 against 27.9)
 //  - above, only while the reduction can be split (3584x8192, 256 tokens: 19.8 against 24.7 for 256x256 tiles; 4096x14336
-//    unsplit: 38.0 against 31.6)
+//    unsplit: 38.0 against 31.6), and beyond 208 tokens only by four or more: split in two, a CTA loads all tokens for half of
+//    the reduction, a CTA pair on 256x256 tiles half of them (256 tokens: 8192x7168 34.6 against 31.6, 6168x4784 35.9 against
+//    27.5; 192 tokens: 29.1 against 31.1, 30.1 against 27.6; split in four, 14336x4096, 256 tokens: 33.6 against 42.9)
 SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   if (M > skinny::MAX_TOKENS) return {0, false};
   const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS, kb = (K + skinny::BK - 1) / skinny::BK;
@@ -162,6 +164,7 @@ SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   };
   if (M <= 64) return {best(true), true};
   const int full = best(false);
+  if (full == 2 && M > 208 && kb >= 32 && (N + BN - 1) / BN <= g_quads[dev]) return {0, false};
   if (full > 1) return {full, false};
   if (M <= 128) return {best(true), true};
   return {0, false};
