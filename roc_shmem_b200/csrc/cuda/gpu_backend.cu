@@ -166,10 +166,14 @@ __global__ void k_write_word(char* dst, uint64_t v, int size) {
   for (int i = 0; i < size; ++i) reinterpret_cast<uint8_t*>(dst)[i] = (uint8_t)(v >> (8 * i));
 }
 
-// Small device-to-device messages.  A copy-engine request costs the host 3.1 us, a kernel launch 2.6 us (both measured
+// Small device-to-device messages.  A copy-engine request costs the host 3.4 us, a kernel launch 2.4 us (both measured
 // back to back), and that is the message rate; the copy itself is shorter than either.  A block moves kSmallPiece
 // bytes: one 16-byte access per thread, so a message of up to kSmallCopyMax takes one round trip to memory.
-constexpr uint64_t kSmallPiece = 4096, kSmallCopyMax = 128u << 10;
+// The line: 64 puts of 256 KiB to 1 MiB take 157 to 162 us through the kernel and 245 to 259 us through the copy engine.
+// At 2 MiB (230 and 262 us) the kernel's own time shows, and that size stays with the copy engine, which takes no SM.
+// Where the two sides are misaligned against each other the kernel moves words or bytes and falls behind beyond 128 KiB
+// (64 puts of 256 KiB - 1, one byte apart: 248 us against 227; of 1 MiB - 1: 656 against 400).
+constexpr uint64_t kSmallPiece = 4096, kSmallCopyMax = 1u << 20, kSmallCopyMaxSkewed = 128u << 10;
 __global__ void __launch_bounds__(256) k_copy_small(char* dst, const char* src, uint64_t n) {
   after_predecessor();
   const uint64_t b = blockIdx.x * kSmallPiece, e = b + kSmallPiece < n ? b + kSmallPiece : n;
@@ -466,7 +470,8 @@ class GpuBackend final : public Backend {
   // Small messages between device buffers go through a kernel (k_copy_small); everything else — host buffers, whose
   // lifetime and staging the copy engine handles, and messages it moves faster — through cudaMemcpyAsync.
   int move(char* dst, const char* src, uint64_t n, cudaStream_t st) {
-    if (tl_local_is_device && n <= kSmallCopyMax) {
+    const bool skewed = ((reinterpret_cast<uintptr_t>(dst) ^ reinterpret_cast<uintptr_t>(src)) & 15) != 0;
+    if (tl_local_is_device && n <= (skewed ? kSmallCopyMaxSkewed : kSmallCopyMax)) {
       RT_TRY(launch_small(k_copy_small, (unsigned)((n + kSmallPiece - 1) / kSmallPiece), n >= kSmallPiece ? 256 : 64, st, dst, src, n));
     } else {
       RT_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyDefault, st));

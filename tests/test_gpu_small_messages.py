@@ -43,6 +43,20 @@ def test_put_get_signal_sizes(rt, n, shift):
     rt.free(sig)
 
 
+@pytest.mark.parametrize("n", [131073, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("to,frm", [(0, 0), (5, 5), (5, 0)])
+def test_put_get_up_to_the_copy_engine(rt, n, to, frm):
+    sym = rt.zeros((n + 64,), torch.uint8)
+    src = torch.randint(0, 256, (n + 16,), dtype=torch.uint8, device="cuda")
+    back = torch.zeros(n + 64, dtype=torch.uint8, device="cuda")
+    rt.put(sym[to:to + n], src[frm:frm + n], 0)
+    rt.get(back[frm:frm + n], sym[to:to + n], 0)
+    for got, at in ((sym, to), (back, frm)):
+        assert torch.equal(got[at:at + n], src[frm:frm + n])
+        assert int(got[:at].sum()) == 0 and int(got[at + n:].sum()) == 0
+    rt.free(sym)
+
+
 @pytest.mark.parametrize("dtype,values", [(torch.uint8, (0, 255)), (torch.int8, (-128, 127)), (torch.int16, (-32768, 5)),
                                           (torch.int32, (-1, 2**31 - 1)), (torch.int64, (-2**63, 2**63 - 1)),
                                           (torch.float32, (-0.5, 3.25)), (torch.float64, (1e-300, -2.0)), (torch.bfloat16, (1.5, -3.0))])
