@@ -190,8 +190,7 @@ __device__ __forceinline__ bool check_target(const State& s, const void* sym, si
 // ---- ordering ---------------------------------------------------------------------------
 // fence: puts issued before it are delivered to each PE before puts issued after it.
 // quiet: every outstanding put/get/atomic of this thread is complete and visible.
-// With a load/store transport both are a system-scope fence.
-// Orders the thread's earlier accesses before its later ones as every PE sees them.  A system-scope fence takes 3 to 4 us on
+// With a load/store transport both are one fence, fence_peers.  It orders the thread's earlier accesses before its later ones as every PE sees them.  A system-scope fence takes 3 to 4 us on
 // a busy GPU, a GPU-scope one less than 1; the latter does when all PEs share the GPU.
 __device__ __forceinline__ void fence_peers(const State& s) {
   if (s.one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
