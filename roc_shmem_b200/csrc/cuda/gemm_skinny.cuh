@@ -270,7 +270,8 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
 // memory; the up warps hand their values to the gate warps through shared memory, 16 tokens at a time, and the gate warps
 // write silu(gate) * up.
 // Split (few active groups with few weight rows): as in the dense form, a cluster shares one tile and adds its parts
-// through distributed shared memory; a CTA has no second tile then.
+// through distributed shared memory; a CTA has no second tile then.  The counts on the device decide whether that holds: with
+// more tiles than clusters the CTAs take whole tiles, each on its own.
 namespace bshmem {
 namespace skinny {
 
@@ -288,7 +289,7 @@ struct GroupedParams {
   uint32_t ring_bytes;           // shared memory of the stages
   uint32_t tmem_cols;            // two accumulators
   int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 256)
-  int split;                     // > 1: clusters of that many CTAs share the reduction of a tile, one tile per cluster
+  int split;                     // > 1: clusters of that many CTAs share the reduction of a tile while each has one at most
   int P;                         // arrival words to wait for before the first token load (0: none)
   const unsigned long long* arrive;
   const int* expected;
@@ -362,18 +363,26 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   ptx::tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(L.tmem_slot()));
-  int most = 1;
-  for (int i = 0; i < p.G; ++i) most = max(most, L.rows()[i]);
+  int most = 1, tiles = 0;
+  for (int i = lane; i < p.G; i += 32) {
+    most = max(most, L.rows()[i]);
+    tiles += (L.rows()[i] + p.nt_cap - 1) / p.nt_cap * (p.N / ROWS);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  tiles = __reduce_add_sync(0xffffffffu, tiles);
+  // A cluster has room for the parts of one tile.  The host chose the split from the counts it expected; where the real ones
+  // make more tiles than there are clusters, every CTA of the grid (all read the same counts) walks whole tiles on its own.
+  const int split = p.split > 1 && tiles <= (int)gridDim.x / p.split ? p.split : 1;
   const int nt_max = min((most + 15) / 16 * 16, p.nt_cap);
   const uint32_t stage = W_STAGE_BYTES + (uint32_t)((nt_max + p.xbox - 1) / p.xbox * p.xbox) * BK * 2;
   const int stages = min((int)(p.ring_bytes / stage), MAX_GROUP_STAGES);
   const int kb_all = (p.K + BK - 1) / BK;
-  const int rank = p.split > 1 ? (int)cluster_rank() : 0;
-  const int kb0 = kb_all * rank / p.split, kb1 = kb_all * (rank + 1) / p.split;
-  GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x / p.split, (int)gridDim.x / p.split, 0, 0};
+  const int rank = split > 1 ? (int)cluster_rank() : 0;
+  const int kb0 = kb_all * rank / split, kb1 = kb_all * (rank + 1) / split;
+  GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x / split, (int)gridDim.x / split, 0, 0};
   struct { int grp, n_blk, tok0, ntok; } split_tile = {0, 0, 0, 0};
   bool mine = false;                                 // split form: there is a tile for this cluster
-  if (p.split > 1) {
+  if (split > 1) {
     GroupedTiles probe = it;
     mine = probe.next(&split_tile.grp, &split_tile.n_blk, &split_tile.tok0, &split_tile.ntok);
   }
@@ -443,7 +452,7 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
       acc_ph ^= 1u << acc;
       ptx::tc_fence_after();
       const uint32_t taddr = lanes + acc * p.nt_cap;
-      if (p.split > 1) {
+      if (split > 1) {
         // [token][weight row] floats over the drained stages
         const uint32_t dst = L.base + (quarter * 32 + lane) * 4;
         for (int c = 0; c < ntok; c += 16) {
@@ -491,17 +500,17 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (p.split > 1) {
+  if (split > 1) {
     cluster_sync();
     if (mine && !*L.abort_flag()) {
       // one warp per token; a lane's sum over the parts of weight row r of token t
       auto sum = [&](int t, int r) {
         float f = 0.f;
 #pragma unroll 4
-        for (int q = 0; q < p.split; ++q) f += ld_cluster_f1(map_rank(L.base + (t * ROWS + r) * 4, q));
+        for (int q = 0; q < split; ++q) f += ld_cluster_f1(map_rank(L.base + (t * ROWS + r) * 4, q));
         return f;
       };
-      for (int t = rank + warp * p.split; t < split_tile.ntok; t += p.split * (NUM_THREADS / 32)) {
+      for (int t = rank + warp * split; t < split_tile.ntok; t += split * (NUM_THREADS / 32)) {
         __nv_bfloat16* out = p.out + ((long long)split_tile.grp * p.cap + split_tile.tok0 + t) * p.ldo;
         if constexpr (kGated) {
 #pragma unroll

@@ -511,9 +511,10 @@ int bshmem_moe_grouped_gemm_swiglu_bwd(const void* A, const void* B, const void*
                            stream, timeout_ms, 0, nullptr, 0, gu, ld_gu);
 }
 
-// The same product for few rows per group (up to about 128; more are taken in chunks of 128, reading the weights again).
-// max_rows and max_active bound the largest group and the number of groups with rows as far as the host knows them (the
-// tokens and the token-expert entries of a decode step).  Up to 64 groups, a_rows_per_group and N multiples of 256; rows of
+// The same product for few rows per group (up to about 128; more are taken in chunks, reading the weights again).
+// max_rows and max_active are the largest group and the number of groups with rows as far as the host knows them (the tokens
+// and the token-expert entries of a decode step); they choose chunk, split and grid, and the product is right for any counts
+// on the device: larger groups are taken in more chunks, and more tiles than clusters are not split.  Up to 64 groups, a_rows_per_group and N multiples of 256; rows of
 // C beyond a group's count are not written.
 // us, 8 groups, N x K = 28672 x 4096 gated: 8 rows each 285 against 380 for the 256-row tiles (weights at the measured copy
 // rate: 288), 64 rows 315 / 375, 100 rows 325 / 373, 128 rows 410 / 380 (some groups have more than the chunk of 128 rows

@@ -106,7 +106,8 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
                  n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0, few: Optional[tuple] = None) -> None:
     """out_g = a_g @ b_g.T per group on the tcgen05 grouped kernel.  a: [G*Ra, K], b: [G*Rb, K], out: [G*Ra, N or N/2].
     `few` = (most rows of a group, most groups with rows): the caller expects about 100 rows per group or less; the
-    weight-streaming form takes such problems."""
+    weight-streaming form takes such problems.  The two numbers set its launch shape; a call whose counts exceed them is
+    slower and as right."""
     G = groups
     ra, rb = a.shape[0] // G, b.shape[0] // G
     if few is not None and rows is not None and G <= 64:
@@ -170,6 +171,14 @@ def zero_pad_rows(buf, groups: int, counts: torch.Tensor) -> None:
     st = _fast.zero_pad_rows(*args, counts.data_ptr(), groups, rows // groups, _stream())
     if st != 0:
         raise RuntimeError(f"zero_pad_rows failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
+
+
+def few_bounds(P: int, G: int, cap: int, tokens: int, topk: int, max_tokens: int) -> tuple:
+    """(most rows a group of this PE can get, most of its G groups that can get any).  A token sends at most one row to a
+    group.  One PE knows the call's tokens; with several, the others may bring up to the layer's limit, whatever this one brings."""
+    if P == 1:
+        return min(cap, tokens), min(G, tokens * topk)
+    return min(cap, P * max_tokens), G
 
 
 class MoELayer:
@@ -292,13 +301,13 @@ class MoELayer:
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
         local = P == 1                                             # no row leaves this GPU: no signals, no return buffer
-        # (every PE brings about as many tokens; a group has at most one row per token of each PE)
-        hint = (P * T, P * n_entries)
+        bounds = few_bounds(P, G, cap, T, self.topk, self.T)
 
         def few(cols):
-            """The hint if the product with `cols` columns is one for the weight-streaming GEMM, else None."""
+            """The bounds if the product with `cols` columns is one for the weight-streaming GEMM, else None.  The choice goes by
+            the expected rows (every PE brings about as many tokens)."""
             limit = FEW_ROWS if G * cols // 128 > FEW_TILES else FEW_ROWS_SPLIT
-            return hint if hint[1] <= limit * self.E else None
+            return bounds if P * n_entries <= limit * self.E else None
 
         few_up, few_down = few(2 * F), few(H)
         self.route(x)

@@ -147,3 +147,32 @@ def test_local_rows(T, H, E, topk):
         assert bool(((dlog.double() - lref).abs() <= ltol + lref.abs() * 2 ** -22).all())
     finally:
         shmem.finalize()
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("rows,few", [([65, 0, 130], (1, 1)), ([17, 16, 1], (16, 1)), ([0, 0, 33], (2, 3)), ([5, 9, 2], (9, 3))])
+@pytest.mark.parametrize("N,K", [(256, 8192), (1280, 2048)])
+def test_more_rows_and_groups_than_expected(rows, few, gated, N, K):
+    """Counts beyond the bounds that chose the launch: more tiles than clusters where the reduction is split, more chunks."""
+    from roc_shmem_b200.ops.moe import grouped_gemm, moe_lib
+    torch.manual_seed(sum(rows) + N)
+    G, cap = len(rows), 256
+    a = torch.randn(G * cap, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(G * N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    cnt = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    out = torch.full((G * cap, N // 2 if gated else N), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm(a, b, out, G, rows=cnt, gated=gated, few=few)
+    torch.cuda.synchronize()
+    assert moe_lib().bshmem_moe_gemm_error_site(1) == 0
+    for g, n in enumerate(rows):
+        assert bool((out[g * cap + n:(g + 1) * cap] == 7).all())
+        x, w = a[g * cap:g * cap + n].double(), b[g * N:(g + 1) * N].double()
+        ref, tol = x @ w.t(), K * 2 ** -24 * (x.abs() @ w.abs().t())                 # fp32 sums in any order
+        if gated:
+            (gate, up), (tg, tu) = ref.view(n, N // 64, 2, 32).unbind(2), tol.view(n, N // 64, 2, 32).unbind(2)
+            s = torch.sigmoid(gate)
+            # slope of silu at most 1.1; 2^-18 for __expf; the factors' own errors
+            ref, tol = gate * s * up, (1.1 * tg * (up.abs() + tu) + tu * gate.abs() + (gate * up).abs() * 2 ** -18)
+            ref, tol = ref.reshape(n, N // 2), tol.reshape(n, N // 2)
+        err = (out[g * cap:g * cap + n].double() - ref).abs()
+        assert bool((err <= ref.abs() * 2 ** -8 + tol + 1e-30).all()), (g, (err - tol).max().item())
