@@ -62,15 +62,23 @@ struct PlainBf16 : PolicyDefaults {
     *x = col;
     *y = row;
   }
-  // 16 columns of a row: one 32-byte sector (N is a multiple of 8)
+  // 16 columns of a row: one 32-byte sector, as far as the matrix goes (N need not be a multiple of 8 when B is K-major)
   __device__ static __forceinline__ void store_row16(const Params& p, int row, int col, const float4 (&v)[4]) {
     if (row >= p.core.M) return;
-    uint4* dst = reinterpret_cast<uint4*>(p.out + row * p.ldc + col);
+    __nv_bfloat16* dst = p.out + row * p.ldc + col;
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (col + 8 * h < p.core.N)
-        dst[h] = make_uint4(pack_bf16(v[2 * h].x, v[2 * h].y), pack_bf16(v[2 * h].z, v[2 * h].w), pack_bf16(v[2 * h + 1].x, v[2 * h + 1].y),
-                            pack_bf16(v[2 * h + 1].z, v[2 * h + 1].w));
+    for (int h = 0; h < 2; ++h) {
+      const float4 a = v[2 * h], b = v[2 * h + 1];
+      const int left = p.core.N - col - 8 * h;
+      if (left >= 8) {
+        *reinterpret_cast<uint4*>(dst + 8 * h) = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+      } else {
+        const float f[7] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+          if (j < left) dst[8 * h + j] = __float2bfloat16_rn(f[j]);
+      }
+    }
   }
 };
 

@@ -120,9 +120,17 @@ __device__ __forceinline__ void add_partials(const Params& p, uint32_t base, int
       const int t = t0 + u * kStep;
 #pragma unroll
       for (int q = 1; q < S; ++q) { v[u][0].x += v[u][q].x; v[u][0].y += v[u][q].y; v[u][0].z += v[u][q].z; v[u][0].w += v[u][q].w; }
-      if (t < p.M)
-        *reinterpret_cast<uint2*>(p.out + (long long)t * p.ldo + n0 + lane * 4) =
-            make_uint2(pack_bf16(v[u][0].x, v[u][0].y), pack_bf16(v[u][0].z, v[u][0].w));
+      if (t >= p.M) continue;
+      __nv_bfloat16* dst = p.out + (long long)t * p.ldo + n0 + lane * 4;
+      const int left = p.N - n0 - lane * 4;           // columns from here on; what lies behind them is not ours
+      if (left >= 4) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v[u][0].x, v[u][0].y), pack_bf16(v[u][0].z, v[u][0].w));
+      } else {
+        const float f[3] = {v[u][0].x, v[u][0].y, v[u][0].z};
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (j < left) dst[j] = __float2bfloat16_rn(f[j]);
+      }
     }
   }
 }
