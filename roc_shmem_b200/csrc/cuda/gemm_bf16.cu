@@ -62,6 +62,15 @@ struct PlainBf16 : PolicyDefaults {
     *x = col;
     *y = row;
   }
+  static constexpr bool kRaggedCols = !kSplitK;
+  __device__ static __forceinline__ bool ragged_chunk(const Params& p, int col) { return (p.core.N & 7) && col < p.core.N && col + EPI_COLS > p.core.N; }
+  __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const float (&f)[64]) {
+    if (row >= p.core.M) return;
+    __nv_bfloat16* dst = p.out + row * p.ldc + col;
+#pragma unroll
+    for (int j = 0; j < 64; ++j)
+      if (col + j < p.core.N) dst[j] = __float2bfloat16_rn(f[j]);
+  }
   // 16 columns of a row: one 32-byte sector, as far as the matrix goes (N need not be a multiple of 8 when B is K-major)
   __device__ static __forceinline__ void store_row16(const Params& p, int row, int col, const float4 (&v)[4]) {
     if (row >= p.core.M) return;

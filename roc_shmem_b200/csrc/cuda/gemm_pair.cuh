@@ -212,6 +212,9 @@ struct PolicyDefaults {
   // kSwigluBwd: the accumulator is the gradient of the activations; each 32 columns of it become 64 columns of output, the
   // gradients of the matching gate and up pre-activations (swiglu_grad), and out_target gets the output column.
   static constexpr bool kStoreAct = false, kSwigluBwd = false;
+  // kRaggedCols: the output's width may end inside a 16-byte piece.  A TMA store fills the piece with zeros, over what lies
+  // behind the matrix; such a chunk (ragged_chunk) is written by store_ragged instead, element by element.
+  static constexpr bool kRaggedCols = false;
   // Operand layout.  Default: both operands K-major, one 128-row x 128-byte TMA box per operand, CTA and stage, and
   // shared-memory descriptors that step 32 bytes along K inside the swizzle atom.  A policy with MN-major operands
   // overrides the instruction descriptor, the stage-0 descriptors, the step per MMA and the loads.
@@ -516,6 +519,12 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           }
           P::adjust(prm, L, st, cc, f, ew, lane);
           if constexpr (P::kStoreAct) P::store_act(prm, cc.row0 + lane, cc.col0, f);
+          if constexpr (P::kRaggedCols) {
+            if (P::ragged_chunk(prm, cc.col0)) {
+              P::store_ragged(prm, cc.row0 + lane, cc.col0, f);
+              continue;
+            }
+          }
           stage_chunk(L.epi(ew), lane, f);
           if (lane == 0) {
             const CUtensorMap* map; int x, y;
