@@ -79,15 +79,15 @@ class LlamaMLP:
         if self.P == 1 and self._fills(2 * self.Fp):
             # one PE: nothing to gather, SwiGLU happens in the projection's epilogue
             if self.training:
-                if x_shard.data_ptr() != self.up.x_shard.data_ptr():
+                if x_shard is not None and x_shard.data_ptr() != self.up.x_shard.data_ptr():
                     self.up.x_shard.copy_(x_shard)               # the weight gradient reads it
                 grouped_gemm_act(self.up.gathered, self.w13, self.gu, self.h, 1)
             else:
-                grouped_gemm(self._operand(x_shard), self.w13, self.h, 1, fixed_rows=self.M, gated=True)
+                grouped_gemm(self._operand(x_shard, self.up.x_shard), self.w13, self.h, 1, fixed_rows=self.M, gated=True)
             self.launches += 1
         else:
             if self.P == 1 and not self.training:
-                gemm_bf16(self._operand(x_shard), self.w13, self.gu)
+                gemm_bf16(self._operand(x_shard, self.up.x_shard), self.w13, self.gu)
             else:
                 self.up(x_shard)
             self._chk(moe_fast.swiglu_fwd(self.gu.data_ptr(), self.rows.data_ptr(), 1, self.M, self.Fp, self.h.data_ptr(), s), "swiglu")
@@ -98,10 +98,16 @@ class LlamaMLP:
 
     __call__ = forward
 
-    @staticmethod
-    def _operand(x: torch.Tensor) -> torch.Tensor:
-        """`x` if the kernels can read it in place (rows contiguous and 16-byte aligned), else a copy."""
-        return x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
+    def _operand(self, x: Optional[torch.Tensor], buffer: torch.Tensor) -> torch.Tensor:
+        """`x` if the kernels, which get nothing but its address, can read it in place: bf16 [tokens, hidden] on this GPU, rows
+        contiguous, 16-byte aligned and apart.  Anything else goes through the layer's own `buffer`: copy_ converts type and
+        device and refuses a wrong shape; None means that the caller has written the rows there."""
+        if x is None:
+            return buffer
+        if (x.dtype is torch.bfloat16 and x.device == buffer.device and x.shape == buffer.shape and x.stride(1) == 1
+                and x.stride(0) >= x.shape[1] and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+            return x
+        return buffer.copy_(x)
 
     def backward(self, dy_shard: torch.Tensor) -> torch.Tensor:
         """Returns dx_shard [M/P, H]; weight gradients land in ``dw13`` / ``dw2``.  Must follow forward()."""
@@ -109,7 +115,7 @@ class LlamaMLP:
         s = current_stream()
         fused = self.P == 1 and self._fills(self.Fp)
         if self.P == 1:
-            dy = self._operand(dy_shard)                                           # nothing to gather
+            dy = self._operand(dy_shard, self.dgrad_h.x_shard)                     # nothing to gather
             if fused:
                 grouped_gemm_swiglu_bwd(dy, self.w2_t, self.gu, self.dgu, 1)       # dgu = SwiGLU' (dy @ W2)
             else:

@@ -115,3 +115,28 @@ def test_mixtral_block_autograd(rt):
     assert (mod.w2.grad.float() - w2r.grad).abs().max().item() <= 5e-2 * w2r.grad.abs().max().item() + 5e-2
     # the router's weights get their gradient through the softmax over the chosen experts
     assert (mod.wr.grad.float() - wrr.grad).abs().max().item() <= 8e-2 * wrr.grad.abs().max().item() + 5e-2
+
+
+@pytest.mark.parametrize("M", [512, 2560])
+def test_llama_mlp_single_pe_converts_its_inputs(rt, M):
+    """fp32, host and column-major inputs of both passes give what the same values give as bf16 on the GPU, on the fused route
+    and beside it; None reads the rows that the caller left in the layer's buffer."""
+    from roc_shmem_b200.models.llama import LlamaMLP
+    torch.manual_seed(4)
+    H, F = 512, 1024
+    w = [(torch.randn(s, device="cuda") * 0.05).to(torch.bfloat16) for s in ((F, H), (F, H), (H, F))]
+    x, dy = (torch.randn(M, H, device="cuda").to(torch.bfloat16) for _ in range(2))
+    serve, train = LlamaMLP(rt, H, F, M, training=False), LlamaMLP(rt, H, F, M, training=True)
+    assert train._fills(F) == (M == 2560)
+    serve.load(*w)
+    train.load(*w)
+    y, yt = serve.forward(x).clone(), train.forward(x).clone()
+    dx, dw13, dw2 = train.backward(dy).clone(), train.dw13.clone(), train.dw2.clone()
+    for f in (lambda v: v.float(), lambda v: v.cpu(), lambda v: v.t().contiguous().t(), lambda v: None):
+        serve.up.x_shard.copy_(x)
+        train.up.x_shard.copy_(x)
+        train.dgrad_h.x_shard.copy_(dy)
+        assert torch.equal(serve.forward(f(x)), y) and torch.equal(train.forward(f(x)), yt)
+        assert torch.equal(train.backward(f(dy)), dx) and torch.equal(train.dw13, dw13) and torch.equal(train.dw2, dw2)
+    serve.check()
+    train.check()
