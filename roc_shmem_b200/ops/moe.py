@@ -123,11 +123,20 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
         raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
+def _check_matrices(what: str, **matrices) -> None:
+    """Name = (tensor, rows, columns): bf16 matrices of that size with contiguous rows (the kernels get addresses only)."""
+    for name, (t, rows, cols) in matrices.items():
+        if t.dtype is not torch.bfloat16 or t.shape != (rows, cols) or t.stride(1) != 1:
+            raise ValueError(f"{what}: {name} must be a bf16 [{rows}, {cols}] matrix with contiguous rows, got {t.dtype} {tuple(t.shape)}")
+
+
 def grouped_gemm_act(a: torch.Tensor, b: torch.Tensor, gu: torch.Tensor, act: torch.Tensor, groups: int, *,
                      rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0, timeout_ms: int = 4000) -> None:
     """Training forward of the gated MLP in one kernel: gu_g = a_g @ b_g.T (interleaved gate / up pre-activations, kept for
     the backward pass) and act_g = silu(gate) * up.  a: [G*R, K], b: [G*N, K], gu: [G*R, N], act: [G*R, N/2]."""
     G = groups
+    R, K, N = a.shape[0], a.shape[1], b.shape[0] // G
+    _check_matrices("grouped_gemm_act", a=(a, R, K), b=(b, G * N, K), gu=(gu, R, N), act=(act, R, N // 2))
     st = _fast.grouped_gemm_act(a.data_ptr(), b.data_ptr(), gu.data_ptr(), act.data_ptr(), G, a.shape[0] // G, b.shape[0] // G, a.shape[1],
                                 a.stride(0), b.stride(0), gu.stride(0), act.stride(0), _p(rows), arrive, _p(expected), n_arrive, _stream(),
                                 timeout_ms)
@@ -141,6 +150,8 @@ def grouped_gemm_swiglu_bwd(dy: torch.Tensor, w2_t: torch.Tensor, gu: torch.Tens
     """d_gu_g = SwiGLU backward of (dy_g @ w2_t_g.T) at the pre-activations gu_g, in one kernel: the gradient of the
     activations never goes to memory.  dy: [G*R, K], w2_t: [G*N, K], gu and dgu: [G*R, 2N] (interleaved)."""
     G = groups
+    R, K, N = dy.shape[0], dy.shape[1], w2_t.shape[0] // G
+    _check_matrices("grouped_gemm_swiglu_bwd", dy=(dy, R, K), w2_t=(w2_t, G * N, K), gu=(gu, R, 2 * N), dgu=(dgu, R, 2 * N))
     st = _fast.grouped_gemm_swiglu_bwd(dy.data_ptr(), w2_t.data_ptr(), gu.data_ptr(), dgu.data_ptr(), G, dy.shape[0] // G,
                                        w2_t.shape[0] // G, dy.shape[1], dy.stride(0), w2_t.stride(0), gu.stride(0), dgu.stride(0), _p(rows),
                                        arrive, _p(expected), n_arrive, _stream(), timeout_ms)

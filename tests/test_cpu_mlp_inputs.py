@@ -81,3 +81,27 @@ def test_wrong_shapes_are_refused(make, fills, shape):
         with pytest.raises((RuntimeError, ValueError)):
             getattr(b, call)(torch.zeros(shape, dtype=torch.bfloat16))
         assert not seen
+
+
+@pytest.mark.parametrize("bad", ["type", "rows", "columns", "order"])
+@pytest.mark.parametrize("which", range(4))
+@pytest.mark.parametrize("backward", [False, True])
+def test_fused_products_check_their_matrices(monkeypatch, backward, which, bad):
+    from roc_shmem_b200.ops import moe
+    launched = []
+    monkeypatch.setattr(moe, "_fast", type("Native", (), {"__getattr__": lambda s, n: lambda *a: launched.append(n) or 0})())
+    monkeypatch.setattr(moe, "_stream", lambda: 0)
+    G, R, K, N = 2, 512, 64, 256
+    shapes = [(R, K), (G * N, K), (R, 2 * N), (R, 2 * N)] if backward else [(R, K), (G * N, K), (R, N), (R, N // 2)]
+    run = moe.grouped_gemm_swiglu_bwd if backward else moe.grouped_gemm_act
+    ts = [torch.zeros(s, dtype=torch.bfloat16) for s in shapes]
+    run(*ts, G)
+    assert len(launched) == 1
+    r, c = shapes[which]
+    ts[which] = {"type": torch.zeros(r, c), "rows": torch.zeros(r // 2, c, dtype=torch.bfloat16),
+                 "columns": torch.zeros(r, 2 * c, dtype=torch.bfloat16), "order": torch.zeros(c, r, dtype=torch.bfloat16).t()}[bad]
+    if (which, bad) == (1, "rows"):
+        ts[which] = ts[which][:r // 2 - 1]                   # (half the weights are the weights of a smaller problem)
+    with pytest.raises(ValueError):
+        run(*ts, G)
+    assert len(launched) == 1
