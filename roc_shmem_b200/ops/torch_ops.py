@@ -9,6 +9,7 @@ the fp8 kernel (forward only).  The reference has no PyTorch layer.
 from __future__ import annotations
 
 import torch
+from torch.utils._device import DeviceContext
 
 from .gemm import gemm_bf16
 from .gemm_fp8 import gemm_fp8, quantize_act, quantize_weight
@@ -100,6 +101,18 @@ class _LinearFn(torch.autograd.Function):
         return (gemm_bf16(dy, w, b_mn=True) if need_x else None, gemm_bf16(dy, x, a_mn=True, b_mn=True) if need_w else None)
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _unwatched() -> bool:
+    """Nobody watches or rewrites operators: no compilation or tracing, no dispatch or function mode (fake tensors, make_fx,
+    counters; the one of a default device only adds an argument to factories), no functorch transform (vmap, grad, jvp)."""
+    C = torch._C
+    modes = C._len_torch_function_stack()
+    return (C._len_torch_dispatch_stack() == 0 and C._functorch.peek_interpreter_stack() is None and C._get_tracing_state() is None
+            and (modes == 0 or modes == 1 and type(C._get_function_stack_at(0)) is DeviceContext) and not torch.compiler.is_compiling())
+
+
 class Linear(torch.nn.Module):
     """Drop-in bf16 ``nn.Linear`` (no bias) whose forward and both gradients run on the tcgen05 kernels."""
 
@@ -109,12 +122,14 @@ class Linear(torch.nn.Module):
         torch.nn.init.normal_(self.weight, std=0.02)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if torch.compiler.is_compiling():               # a traced program needs the registered operator
+        w = self.weight
+        # the registered operator for everything but plain tensors in GPU memory (meta, fake and other subclasses)
+        if not (x.is_cuda and w.is_cuda and type(x) in _PLAIN and type(w) in _PLAIN and _unwatched()):
             lead = x.shape[:-1]
-            return torch.ops.bshmem.linear(x.reshape(-1, x.shape[-1]), self.weight).reshape(*lead, -1)
+            return torch.ops.bshmem.linear(x.reshape(-1, x.shape[-1]), w).reshape(*lead, -1)
         if x.dim() == 2:
-            return _LinearFn.apply(x, self.weight)
-        return _LinearFn.apply(x.reshape(-1, x.shape[-1]), self.weight).reshape(*x.shape[:-1], -1)
+            return _LinearFn.apply(x, w)
+        return _LinearFn.apply(x.reshape(-1, x.shape[-1]), w).reshape(*x.shape[:-1], -1)
 
 
 # ---- collectives on the calling PE's runtime (roc_shmem_b200.current()) --------------------------------

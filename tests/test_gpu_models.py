@@ -140,3 +140,28 @@ def test_llama_mlp_single_pe_converts_its_inputs(rt, M):
         assert torch.equal(train.backward(f(dy)), dx) and torch.equal(train.dw13, dw13) and torch.equal(train.dw2, dw2)
     serve.check()
     train.check()
+
+
+def test_linear_under_transforms_and_modes():
+    """On the GPU: plain calls skip the dispatcher, watched ones do not, and both give the same numbers."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from roc_shmem_b200.ops.torch_ops import Linear
+    torch.manual_seed(5)
+    lin = Linear(128, 264, device="cuda")
+    x = torch.randn(3, 40, 128, device="cuda").to(torch.bfloat16)
+    y = lin(x)
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+    with Watch():
+        assert torch.equal(lin(x), y)
+    assert "bshmem.linear.default" in seen
+    assert torch.equal(torch.func.vmap(lin)(x), y)
+    with FakeTensorMode(allow_non_fake_inputs=True) as mode:
+        f = lin(mode.from_tensor(x))
+        assert f.shape == y.shape and f.device.type == "cuda"
