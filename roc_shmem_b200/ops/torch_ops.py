@@ -55,7 +55,7 @@ def _(dy, w):
     return dy.new_empty((dy.shape[0], w.shape[1]))
 
 
-def _linear_setup(ctx, inputs, output):
+def _save_inputs(ctx, inputs, output):
     ctx.save_for_backward(*inputs)
 
 
@@ -67,7 +67,15 @@ def _linear_backward(ctx, dy):
     return dx, dw
 
 
-linear.register_autograd(_linear_backward, setup_context=_linear_setup)
+def _dgrad_backward(ctx, g):
+    dy, w = ctx.saved_tensors
+    g = g.contiguous()
+    return (torch.ops.bshmem.linear(g, w) if ctx.needs_input_grad[0] else None,
+            torch.ops.bshmem.linear_wgrad(dy, g) if ctx.needs_input_grad[1] else None)
+
+
+linear.register_autograd(_linear_backward, setup_context=_save_inputs)
+linear_dgrad.register_autograd(_dgrad_backward, setup_context=_save_inputs)      # second order through dX; dW has none
 
 
 @torch.library.custom_op("bshmem::linear_fp8", mutates_args=())
@@ -89,14 +97,16 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
         _check_linear(x, w)
-        x, w = x.contiguous(), w.contiguous()
-        ctx.save_for_backward(x, w)
-        return gemm_bf16(x, w)
+        ctx.save_for_backward(x, w)          # the inputs themselves: second-order gradients go through them
+        return gemm_bf16(x.contiguous(), w.contiguous())
 
     @staticmethod
     def backward(ctx, dy):
+        # the registered operators where the gradients are differentiated or batched themselves, or watched
+        if torch.is_grad_enabled() or not _unwatched() or type(dy) is not torch.Tensor or torch._C._functorch.is_legacy_batchedtensor(dy):
+            return _linear_backward(ctx, dy)
         x, w = ctx.saved_tensors
-        dy = dy.contiguous()
+        x, w, dy = x.contiguous(), w.contiguous(), dy.contiguous()
         need_x, need_w = ctx.needs_input_grad
         return (gemm_bf16(dy, w, b_mn=True) if need_x else None, gemm_bf16(dy, x, a_mn=True, b_mn=True) if need_w else None)
 

@@ -63,3 +63,31 @@ def test_who_is_watching():
     inside = []
     torch.func.vmap(lambda v: (inside.append(_unwatched()), v)[1])(torch.zeros(2))
     assert inside == [False]
+
+
+@pytest.mark.parametrize("form", ["operator", "layer"])
+@pytest.mark.parametrize("noncontiguous", [False, True])
+def test_second_order_and_batched_gradients(lin, form, noncontiguous):
+    """Through dX as often as asked, against autograd's own product; dW has no formula and says so instead of dropping out."""
+    from roc_shmem_b200.ops.torch_ops import _LinearFn
+    run = torch.ops.bshmem.linear if form == "operator" else _LinearFn.apply
+    w = lin.weight.detach().requires_grad_(True)
+    v = _x(16, 8).t() if noncontiguous else _x(8, 16)
+    x = v.requires_grad_(True)
+    xr, wr = x.detach().float().requires_grad_(True), w.detach().float().requires_grad_(True)
+
+    def penalty(a, b, f):
+        dx, = torch.autograd.grad(f(a, b).float().pow(2).sum(), a, create_graph=True)
+        return dx.float().pow(2).sum() + f(a, b).float().sum()
+    got = torch.autograd.grad(penalty(x, w, run), (x, w))
+    ref = torch.autograd.grad(penalty(xr, wr, lambda a, b: a @ b.t()), (xr, wr))
+    for g, r in zip(got, ref):
+        assert (g.float() - r).norm() <= 2e-2 * r.norm()     # a chain of four bf16 products
+    dw, = torch.autograd.grad(run(x, w).float().pow(2).sum(), w, create_graph=True)
+    with pytest.raises(RuntimeError, match="autograd formula"):
+        torch.autograd.grad(dw.float().pow(2).sum(), x)
+    dy = _x(3, 8, 24)
+    dx, dw = torch.autograd.grad(run(x, w), (x, w), dy, is_grads_batched=True)
+    for i in range(3):
+        dxi, dwi = torch.autograd.grad(run(x, w), (x, w), dy[i])
+        assert torch.equal(dx[i], dxi) and torch.equal(dw[i], dwi)
