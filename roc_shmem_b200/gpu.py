@@ -399,6 +399,7 @@ class DeviceRuntime(Runtime):
 from .utils.trace import instrument as _instrument  # noqa: E402
 
 _instrument(DeviceRuntime, ("put", "get", "put_signal"))
+_instrument(DeviceContext, ("put", "get"))
 
 
 def init_device_runtime(boot: Bootstrap, cfg: Config, device: Optional[int] = None, proxy: bool = False) -> DeviceRuntime:

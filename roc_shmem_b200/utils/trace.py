@@ -9,6 +9,7 @@ from __future__ import annotations
 import contextlib
 import logging
 import os
+import threading
 
 logger = logging.getLogger("roc_shmem_b200")
 if not logger.handlers:
@@ -56,14 +57,23 @@ def log(pe: int, msg: str, *args, level: int = logging.DEBUG) -> None:
     logger.log(level, msg, *args, extra={"pe": pe})
 
 
+_inside = threading.local()      # .name: the range that the thread's innermost traced function has open
+
+
 def traced(name: str):
-    """Decorator: an NVTX range around a function (a flag test while tracing is off)."""
+    """Decorator: an NVTX range around a function (a flag test while tracing is off).  A method that hands over to the one it
+    overrides makes one range, not two."""
     def deco(fn):
         def wrapper(*a, **k):
-            if not _TRACE:
+            outer = getattr(_inside, "name", None)
+            if not _TRACE or outer == name:
                 return fn(*a, **k)
-            with nvtx_range(name):
-                return fn(*a, **k)
+            _inside.name = name
+            try:
+                with nvtx_range(name):
+                    return fn(*a, **k)
+            finally:
+                _inside.name = outer
         wrapper.__name__, wrapper.__doc__ = fn.__name__, fn.__doc__
         return wrapper
     return deco
