@@ -62,7 +62,7 @@ def _pycall():
     if _pycall_mod is None:
         with _lock:
             if _pycall_mod is None:
-                path = _LIB_DIR / "bshmem_pycall.so"
+                path = _LIB_DIR / _build.PYCALL
                 if not path.exists():
                     with _build_lock():
                         _build.build_pycall()

@@ -102,10 +102,14 @@ def build_host(force: bool = False) -> Path:
     return out
 
 
+# The one library that is bound to an interpreter carries its ABI tag: another Python version finds none and builds its own.
+PYCALL = "bshmem_pycall" + sysconfig.get_config_var("EXT_SUFFIX")
+
+
 def build_pycall(force: bool = False) -> Path:
     """The CPython callables over the native libraries (csrc/host/pycall.cc); needs the interpreter's own headers."""
     LIB.mkdir(exist_ok=True)
-    out = LIB / "bshmem_pycall.so"
+    out = LIB / PYCALL
     src = CSRC / "host/pycall.cc"
     if force or _stale(out, [src]):
         cmd = ["g++", "-std=c++17", "-O2", "-g", "-fPIC", "-shared", "-Wall", "-Wextra", "-Wno-missing-field-initializers",

@@ -135,3 +135,18 @@ def test_cmake_build_install_and_consumer(tmp_path):
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     r = subprocess.run([str(app / "b" / "app")], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and "CMAKE_CONSUMER_OK 5" in r.stdout, r.stdout + r.stderr
+
+
+def test_extension_module_is_bound_to_its_interpreter(tmp_path, monkeypatch):
+    """The CPython module over the native libraries carries the interpreter's ABI tag: a file that another version left in the
+    library folder is not taken for this one's."""
+    import sysconfig
+
+    from roc_shmem_b200 import build
+    assert sysconfig.get_config_var("EXT_SUFFIX") in build.build_pycall().name
+    for foreign in ("bshmem_pycall.so", "bshmem_pycall.cpython-39-x86_64-linux-gnu.so"):
+        (tmp_path / foreign).write_bytes(b"not for this interpreter")
+    monkeypatch.setattr(build, "LIB", tmp_path)
+    monkeypatch.setattr(_native, "_LIB_DIR", tmp_path)
+    monkeypatch.setattr(_native, "_pycall_mod", None)
+    assert _native._pycall().Native is not None              # built beside them, under its own name
