@@ -75,7 +75,7 @@ def _pycall():
 
 
 def fast(lib: C.CDLL, name: str):
-    """The declared entry point `name` of `lib` as a callable that takes plain integers (addresses included) and None.
+    """The declared entry point `name` of `lib` as a callable that takes integers, and int or None for an address.
 
     For entry points on a path that runs once per message or per layer: a ctypes call of the same function costs 1.5 to
     3 us, this one 0.15 us.  A result declared as a pointer comes back as an integer (0 = null)."""
@@ -83,7 +83,8 @@ def fast(lib: C.CDLL, name: str):
     if fn.argtypes is None:
         raise TypeError(f"{name}: declare argtypes first")
     kind = 0 if fn.restype is C.c_int else (2 if fn.restype is None else 1)
-    return _pycall().Native(C.cast(fn, C.c_void_p).value, len(fn.argtypes), kind)
+    pointers = sum(1 << i for i, t in enumerate(fn.argtypes) if t in (C.c_void_p, C.c_char_p) or issubclass(t, C._Pointer))
+    return _pycall().Native(C.cast(fn, C.c_void_p).value, len(fn.argtypes), kind, pointers)
 
 
 class _build_lock:

@@ -2,10 +2,11 @@
 //
 // ctypes builds an argument object, a conversion and a libffi call frame for every argument of every call: 1.5 to 3 us
 // for the 6 to 20 integers and addresses that the entry points here take, which is as long as a kernel launch and
-// shows wherever a program issues many small operations.  `Native(address, nargs, kind)` is a vectorcall object that
-// converts its Python integers (None = null) straight to machine words and calls the function: about 0.15 us.
+// shows wherever a program issues many small operations.  `Native(address, nargs, kind, pointers)` is a vectorcall object
+// that converts its arguments straight to machine words and calls the function: about 0.15 us.
 //
-// Only integer and pointer arguments are supported.  Every argument is passed as one 64-bit word: under the System V
+// Only integer and pointer arguments are supported, and they take what ctypes takes for them: an integer argument anything
+// with __index__ (a numpy integer, a one-element tensor) but not None; an address (bit i of `pointers`) an int or None.  Every argument is passed as one 64-bit word: under the System V
 // x86-64 and the AArch64 Linux calling conventions an int or pointer argument occupies one full register or stack
 // slot, of which the callee reads the width it declares (the same convention libffi relies on).
 // Like ctypes' CDLL, the interpreter lock is released around the call: blocking entry points wait for other threads.
@@ -29,6 +30,7 @@ struct Native {
   uintptr_t addr;
   int nargs;
   int kind;
+  uint32_t pointers;             // bit i: argument i is an address
 };
 
 template <size_t> using Word = uint64_t;
@@ -58,12 +60,21 @@ PyObject* native_call(PyObject* callable, PyObject* const* args, size_t nargsf, 
   uint64_t a[kMaxArgs];
   for (Py_ssize_t i = 0; i < n; ++i) {
     PyObject* o = args[i];
-    if (o == Py_None) { a[i] = 0; continue; }
-    if (!PyLong_Check(o)) {
-      PyErr_Format(PyExc_TypeError, "native function: argument %zd is a %s, not an integer or None", i, Py_TYPE(o)->tp_name);
-      return nullptr;
+    if (PyLong_Check(o)) {
+      a[i] = PyLong_AsUnsignedLongLongMask(o);       // negative integers keep their two's complement bits
+    } else if (self->pointers >> i & 1) {
+      if (o != Py_None) {
+        PyErr_Format(PyExc_TypeError, "native function: argument %zd is a %s, not an address or None", i, Py_TYPE(o)->tp_name);
+        return nullptr;
+      }
+      a[i] = 0;
+      continue;
+    } else {
+      PyObject* n_obj = PyNumber_Index(o);
+      if (!n_obj) return nullptr;
+      a[i] = PyLong_AsUnsignedLongLongMask(n_obj);
+      Py_DECREF(n_obj);
     }
-    a[i] = PyLong_AsUnsignedLongLongMask(o);     // negative integers keep their two's complement bits
     if (a[i] == (uint64_t)-1 && PyErr_Occurred()) return nullptr;
   }
   uint64_t r;
@@ -81,9 +92,10 @@ PyObject* native_call(PyObject* callable, PyObject* const* args, size_t nargsf, 
 PyObject* native_new(PyTypeObject* type, PyObject* args, PyObject*) {
   unsigned long long addr = 0;
   int nargs = 0, kind = 0;
-  if (!PyArg_ParseTuple(args, "Kii", &addr, &nargs, &kind)) return nullptr;
+  unsigned int pointers = 0;
+  if (!PyArg_ParseTuple(args, "KiiI", &addr, &nargs, &kind, &pointers)) return nullptr;
   if (addr == 0 || nargs < 0 || nargs > kMaxArgs || kind < RET_STATUS || kind > RET_VOID) {
-    PyErr_SetString(PyExc_ValueError, "Native(address, nargs, kind): bad address, argument count or result kind");
+    PyErr_SetString(PyExc_ValueError, "Native(address, nargs, kind, pointers): bad address, argument count or result kind");
     return nullptr;
   }
   Native* self = reinterpret_cast<Native*>(type->tp_alloc(type, 0));
@@ -92,6 +104,7 @@ PyObject* native_new(PyTypeObject* type, PyObject* args, PyObject*) {
   self->addr = (uintptr_t)addr;
   self->nargs = nargs;
   self->kind = kind;
+  self->pointers = pointers;
   return reinterpret_cast<PyObject*>(self);
 }
 
@@ -103,7 +116,7 @@ PyType_Slot native_slots[] = {
     {Py_tp_new, reinterpret_cast<void*>(native_new)},
     {Py_tp_call, reinterpret_cast<void*>(PyVectorcall_Call)},
     {Py_tp_members, native_members},
-    {Py_tp_doc, const_cast<char*>("Native(address, nargs, kind): an extern \"C\" function of integers and addresses")},
+    {Py_tp_doc, const_cast<char*>("Native(address, nargs, kind, pointers): an extern \"C\" function of integers and addresses")},
     {0, nullptr},
 };
 PyType_Spec native_spec = {"bshmem_pycall.Native", sizeof(Native), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL, native_slots};

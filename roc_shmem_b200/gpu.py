@@ -144,7 +144,8 @@ class DeviceContext(Context):
     def put(self, dest, src, pe, *, nbi=False, nbytes=None):
         rt = self.rt
         if isinstance(src, Tensor) and src.get_device() == rt._dev_index and isinstance(dest, Tensor):
-            st = rt._c_put_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), src.nbytes if nbytes is None else nbytes, pe, nbi)
+            st = rt._c_put_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), src.nbytes if nbytes is None else nbytes, pe,
+                               1 if nbi else 0)
             if st:
                 rt._check(st)
             return
@@ -153,7 +154,8 @@ class DeviceContext(Context):
     def get(self, dest, src, pe, *, nbi=False, nbytes=None):
         rt = self.rt
         if isinstance(dest, Tensor) and dest.get_device() == rt._dev_index and isinstance(src, Tensor):
-            st = rt._c_get_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), dest.nbytes if nbytes is None else nbytes, pe, nbi)
+            st = rt._c_get_dev(rt._hv, self.idx, dest.data_ptr(), src.data_ptr(), dest.nbytes if nbytes is None else nbytes, pe,
+                               1 if nbi else 0)
             if st:
                 rt._check(st)
             return
@@ -183,7 +185,7 @@ class DeviceRuntime(Runtime):
         """Copy `src` (any local buffer) into `dest`'s location on PE `pe`."""
         if isinstance(src, Tensor) and src.get_device() == self._dev_index and isinstance(dest, Tensor):
             st = self._c_put_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
-                                 src.nbytes if nbytes is None else nbytes, pe, nbi)
+                                 src.nbytes if nbytes is None else nbytes, pe, 1 if nbi else 0)
             if st:
                 self._check(st)
             return
@@ -193,7 +195,7 @@ class DeviceRuntime(Runtime):
         """Copy `src`'s location on PE `pe` into the local buffer `dest`."""
         if isinstance(dest, Tensor) and dest.get_device() == self._dev_index and isinstance(src, Tensor):
             st = self._c_get_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(),
-                                 dest.nbytes if nbytes is None else nbytes, pe, nbi)
+                                 dest.nbytes if nbytes is None else nbytes, pe, 1 if nbi else 0)
             if st:
                 self._check(st)
             return
@@ -204,7 +206,7 @@ class DeviceRuntime(Runtime):
         the payload is visible to a reader that observed the signal."""
         if isinstance(src, Tensor) and src.get_device() == self._dev_index and isinstance(dest, Tensor):
             st = self._c_put_signal_dev(self._hv, 0 if ctx is None else self._ctx(ctx), dest.data_ptr(), src.data_ptr(), src.nbytes,
-                                        _ptr_of(sig), value, op, pe, nbi)
+                                        _ptr_of(sig), value, op, pe, 1 if nbi else 0)
             if st:
                 self._check(st)
             return
@@ -267,7 +269,7 @@ class DeviceRuntime(Runtime):
                    ctas: int = 32, threads: int = 512, nbytes: Optional[int] = None) -> None:
         """Device-initiated put/get striped over `ctas` CTAs (enqueued, not synchronised).  Scope "bulk" moves the
         data with bulk async copies through shared memory (16-byte aligned addresses and size)."""
-        st = self._c_rma_kernel(self._hv, sym.data_ptr(), local.data_ptr(), local.nbytes if nbytes is None else nbytes, pe, put,
+        st = self._c_rma_kernel(self._hv, sym.data_ptr(), local.data_ptr(), local.nbytes if nbytes is None else nbytes, pe, 1 if put else 0,
                                 _SCOPES[scope], ctas, threads)
         if st:
             self._check(st)

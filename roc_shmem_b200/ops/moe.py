@@ -112,13 +112,14 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
     ra, rb = a.shape[0] // G, b.shape[0] // G
     if few is not None and rows is not None and G <= 64:
         st = _fast.grouped_gemm_few(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, a.shape[1], a.stride(0), b.stride(0),
-                                    out.stride(0), rows.data_ptr(), few[0], few[1], gated, arrive, _p(expected), n_arrive, _stream(),
-                                    timeout_ms)
+                                    out.stride(0), rows.data_ptr(), few[0], few[1], 1 if gated else 0, arrive, _p(expected), n_arrive,
+                                    _stream(), timeout_ms)
         if st != 0:
             raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
         return
     st = _fast.grouped_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, rb, a.shape[1], a.stride(0), b.stride(0), out.stride(0),
-                            _p(rows), fixed_rows, _p(klen), gated, arrive, _p(expected), n_arrive, _stream(), timeout_ms, max_ctas)
+                            _p(rows), fixed_rows, _p(klen), 1 if gated else 0, arrive, _p(expected), n_arrive, _stream(), timeout_ms,
+                            max_ctas)
     if st != 0:
         raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
