@@ -193,6 +193,18 @@ def few_bounds(P: int, G: int, cap: int, tokens: int, topk: int, max_tokens: int
     return min(cap, P * max_tokens), G
 
 
+class _Addresses:
+    """Addresses of a layer's buffers by name, as they are at the moment of the call: a caller may put others in their place."""
+
+    __slots__ = ("_of",)
+
+    def __init__(self, of):
+        self._of = of
+
+    def __getitem__(self, name: str) -> int:
+        return getattr(self._of, name).data_ptr()
+
+
 class MoELayer:
     """One MoE block: y[T, H] = combine(experts(dispatch(x)))  with forward and backward.
 
@@ -268,9 +280,7 @@ class MoELayer:
                             dropped=self.dropped.data_ptr(), arrive_sig=self.arrive.data_ptr())
         self.state = rt.device_state()
         self.ticket = torch.zeros((1,), dtype=torch.int32, device=dev)        # of the one-PE plan kernel
-        # addresses of the buffers above, which live as long as the layer
         self._plan_a, self._state_a = C.addressof(self.plan), C.addressof(self.state)
-        self._a = {k: v.data_ptr() for k, v in vars(self).items() if isinstance(v, torch.Tensor)}
         self.err_word = self.lib.bshmem_moe_gemm_error_word()
         self.calls = 0
         self.launches = 0
@@ -294,7 +304,7 @@ class MoELayer:
 
     def route(self, x: torch.Tensor) -> None:
         """Router, plan, count exchange and offsets for this call's tokens."""
-        T, s, a = x.shape[0], _stream(), self._a
+        T, s, a = x.shape[0], _stream(), _Addresses(self)
         n_entries = T * self.topk
         self.calls += 1
         self.parity = self.calls & 1
@@ -309,7 +319,7 @@ class MoELayer:
         self._chk(_fast.offsets(self._plan_a, a["counts_all"], self.parity, s), "offsets")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        T, s, a = x.shape[0], _stream(), self._a
+        T, s, a = x.shape[0], _stream(), _Addresses(self)
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
         local = P == 1                                             # no row leaves this GPU: no signals, no return buffer
@@ -364,7 +374,7 @@ class MoELayer:
         self.dw2), the routing weights (self.dtopk_w) and, through the softmax over the chosen experts, the router
         weights (self.dwr).  Must follow forward() of the same tokens; the forward's input must still be intact."""
         assert self.training
-        T, s, a = dout.shape[0], _stream(), self._a
+        T, s, a = dout.shape[0], _stream(), _Addresses(self)
         n_entries = T * self.topk
         G, cap, H, F, P = self.G, self.cap, self.H, self.F, self.P
         local = P == 1

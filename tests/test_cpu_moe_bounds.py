@@ -28,7 +28,6 @@ def test_bounds_hold_for_unequal_tokens(P, mine, other, topk, training, monkeypa
              "arrive", "counts", "counts_all", "ticket")
     for n in names:
         setattr(layer, n, torch.zeros(max_tokens, 1))
-    layer._a = {n: 0 for n in names}
     layer.w13, layer.w2 = torch.zeros(G, 2 * F, H), torch.zeros(G, H, F)
     layer.route = lambda x: None
     layer.forward(torch.zeros(mine, H))

@@ -155,3 +155,37 @@ def test_moe_forward_backward_single_pe(rt, training, tn_gemm):
     # reference's contribute differently; they are < 1 % of the rows, so compare with a matching tolerance)
     sr = wrr.grad.abs().max().item()
     assert (layer.dwr.float() - wrr.grad).abs().max().item() <= 8e-2 * sr + 5e-2
+
+
+def test_buffers_put_in_place_of_the_layers_own():
+    """The buffers are attributes: a caller that puts its own in their place (an output, a gradient) finds the results there."""
+    import roc_shmem_b200 as shmem
+    from roc_shmem_b200.ops.moe import MoELayer
+    rt = shmem.init("device", rank=0, world_size=1, heap_bytes=512 << 20, timeout_ms=5000)
+    try:
+        torch.manual_seed(3)
+        T, H, F, E = 300, 256, 512, 8
+        layer = MoELayer(rt, H, F, E, 2, T, capacity_factor=8.0)
+        for t in (layer.wr, layer.w13, layer.w2):
+            t.normal_(std=0.05)
+        layer.sync_transposes()
+        x, dy = torch.randn(T, H, device="cuda").to(torch.bfloat16), torch.randn(T, H, device="cuda").to(torch.bfloat16)
+        y = layer.forward(x).clone()
+        dx = layer.backward(dy).clone()
+        names = ("topk_idx", "topk_w", "pos", "gu", "hact", "yexp", "out", "dh", "dgu", "dxe", "dw13", "dw2", "dx", "dtopk_w", "dlogit",
+                 "dwr_f32", "dwr")
+        old = {n: getattr(layer, n) for n in names}
+        kept = {n: t.clone() for n, t in old.items()}
+        for n, t in old.items():
+            setattr(layer, n, torch.zeros_like(t))
+            t.fill_(3)
+        assert torch.equal(layer.forward(x), y) and torch.equal(layer.backward(dy), dx)
+        torch.cuda.synchronize()
+        for n in names:
+            assert bool((old[n] == 3).all()), n              # nothing written into a buffer that was taken away
+        for n in ("topk_idx", "topk_w", "pos", "dw13", "dw2", "dtopk_w", "dlogit"):
+            assert torch.equal(getattr(layer, n), kept[n]), n
+        assert torch.allclose(layer.dwr.float(), kept["dwr"].float(), rtol=2 ** -7, atol=1e-3)      # fp32 atomics in any order
+        layer.check()
+    finally:
+        shmem.finalize()
