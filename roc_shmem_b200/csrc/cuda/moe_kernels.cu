@@ -50,16 +50,18 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ---------------------------------------------------------------------------------------
 // The logits are a skinny product, T x H by H x E: a block takes 16 tokens, its eight warps share the reduction in steps of
 // 32 columns, and the tensor cores multiply (mma.sync: 64 columns at most are no work for a tcgen05 tile, whose launch and
-// epilogue cost more than these kernels take).  The products of bf16 numbers are exact in fp32; a warp's accumulator takes
-// at most H / 128 additions and the warps' sums are added in order, a shorter chain than the H / 32 of a warp that multiplies with
-// FMAs.  Fragments come straight from global memory, 16 bytes per lane: the reduction may run over the columns in any order
+// epilogue cost more than these kernels take).  The products of bf16 numbers are exact in fp32, but the unit truncates where it
+// adds, which shows in a chain over the whole reduction: rel. error of the probabilities against fp64 3.5e-7 (16384 x 4096, 8
+// experts) and 2.5e-7 (4096 x 2048, 64) where fp32 FMAs give 1.1e-7 and 1.6e-7.  So every product of 16 columns starts from
+// zero and the sums are fp32 additions, the warps' in a tree: 0.9e-7 and 1.1e-7, 31 and 14 us (29 and 14 with the chain).
+// Fragments come straight from global memory, 16 bytes per lane: the reduction may run over the columns in any order
 // as long as both operands agree, so a lane's eight consecutive columns stand for two k-steps' worth of its elements.
 // With a warp of FMAs per four tokens, Wr was read from L2 for every four and the FMAs took over for many experts: 16384 x
-// 4096, 8 experts 92 us; 12000 x 2048, 64 experts 245 us.
+// 4096, 8 experts 92 us; 12000 x 2048, 64 experts 245 us (44 now).
 constexpr int kRouterTok = 16;
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Softmax over the experts, top-k, weights renormalised over the chosen ones; one warp per token, `lg` in shared memory.
@@ -134,12 +136,28 @@ __global__ void __launch_bounds__(32 * kWarps) k_router_topk(const bf16* __restr
       for (int j = 0; j < kTiles; ++j)
         w[u][j] = in && j * 8 + g < E ? __ldg(reinterpret_cast<const uint4*>(wr + (size_t)(j * 8 + g) * H + col)) : zero;
     }
+    // Every product starts from zero.  Eight products per addition to the accumulator, four or two where registers are short
+    // (eight with 64 experts: 140 registers, 12000 x 2048 takes 59 us instead of 44).
+    constexpr int kStep = kTiles == 1 ? kUnroll : kTiles == 2 ? 2 : 1;
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
+    for (int u0 = 0; u0 < kUnroll; u0 += kStep)
 #pragma unroll
       for (int j = 0; j < kTiles; ++j) {
-        mma_bf16(acc[j], a[u].x, b[u].x, a[u].y, b[u].y, w[u][j].x, w[u][j].y);
-        mma_bf16(acc[j], a[u].z, b[u].z, a[u].w, b[u].w, w[u][j].z, w[u][j].w);
+        float c[2 * kStep][4];
+#pragma unroll
+        for (int v = 0; v < kStep; ++v) {
+          const int u = u0 + v;
+          mma_bf16(c[2 * v], a[u].x, b[u].x, a[u].y, b[u].y, w[u][j].x, w[u][j].y);
+          mma_bf16(c[2 * v + 1], a[u].z, b[u].z, a[u].w, b[u].w, w[u][j].z, w[u][j].w);
+        }
+#pragma unroll
+        for (int n = kStep; n > 0; n /= 2)
+#pragma unroll
+          for (int v = 0; v < n; ++v)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[v][i] += c[v + n][i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] += c[0][i];
       }
   }
   auto park = [&](bool add) {
@@ -166,10 +184,14 @@ __global__ void __launch_bounds__(32 * kWarps) k_router_topk(const bf16* __restr
     if (t >= T) break;
     __syncwarp();
     for (int e = lane; e < E; e += 32) {
-      float sum = part[0][r * kPitch + e];
+      float sum[8];
 #pragma unroll
-      for (int q = 1; q < 8; ++q) sum += part[q][r * kPitch + e];
-      lg[warp][e] = sum;
+      for (int q = 0; q < 8; ++q) sum[q] = part[q][r * kPitch + e];
+#pragma unroll
+      for (int step = 4; step > 0; step /= 2)
+#pragma unroll
+        for (int q = 0; q < step; ++q) sum[q] += sum[q + step];
+      lg[warp][e] = sum[0];
     }
     __syncwarp();
     router_select(lg[warp], E, topk, lane, topk_idx + (size_t)t * topk, topk_w + (size_t)t * topk, probs ? probs + (size_t)t * E : nullptr);

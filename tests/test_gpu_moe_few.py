@@ -176,3 +176,24 @@ def test_more_rows_and_groups_than_expected(rows, few, gated, N, K):
             ref, tol = ref.reshape(n, N // 2), tol.reshape(n, N // 2)
         err = (out[g * cap:g * cap + n].double() - ref).abs()
         assert bool((err <= ref.abs() * 2 ** -8 + tol + 1e-30).all()), (g, (err - tol).max().item())
+
+
+@pytest.mark.parametrize("T,H,E,topk", [(2048, 4096, 8, 2), (2048, 4096, 16, 2), (2048, 4096, 32, 2), (4096, 2048, 64, 8)])
+@pytest.mark.parametrize("scale", [0.02, 0.1])
+def test_router_keeps_fp32_sums(T, H, E, topk, scale):
+    """The probabilities against fp64: the logits' sums have to be fp32 additions, not a tensor-core chain over the reduction,
+    which truncates as it adds and was 2 to 4 times as far off.  In units of 2^-25, the mean size of an fp32 rounding: about three
+    for exponential, normalisation and result, and two of the logits' size for their 40 or so additions of partial sums."""
+    from roc_shmem_b200.ops.moe import moe_lib
+    torch.manual_seed(T + E)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    wr = (torch.randn(E, H, device="cuda") * scale).to(torch.bfloat16)
+    idx = torch.empty(T * topk, dtype=torch.int32, device="cuda")
+    w, probs = torch.empty(T * topk, device="cuda"), torch.empty(T, E, device="cuda")
+    assert moe_lib().bshmem_moe_router_topk(x.data_ptr(), wr.data_ptr(), T, H, E, topk, idx.data_ptr(), w.data_ptr(), probs.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    logits = x.double() @ wr.double().t()
+    ref = torch.softmax(logits, -1)
+    err = (probs.double() - ref).norm() / ref.norm()
+    assert err <= 2 ** -25 * (3 + logits.std().item() * 2), err.item()
