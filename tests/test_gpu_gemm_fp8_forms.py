@@ -42,3 +42,25 @@ def test_quantiser_edges(M, K, pad):
     assert torch.allclose(qa.scales.t(), scale, rtol=2 ** -22)
     step = x.float().abs().view(M, K // 128, 128) * 2 ** -4 + scale.view(M, K // 128, 1) * 2 ** -10   # normal, subnormal
     assert bool(((qa.dequantize() - x.float()).abs().view(M, K // 128, 128) <= step * 1.001).all())
+
+
+@pytest.mark.parametrize("M", [0, 65535 * 32, 65535 * 32 + 1])
+def test_quantiser_row_counts(M):
+    """No rows at all, and the last count of the tiled kernel's grid and the first beyond it."""
+    from roc_shmem_b200.ops.gemm_fp8 import quantize_act
+    x = torch.randint(-3, 4, (M, 128), device="cuda").to(torch.bfloat16)
+    qa = quantize_act(x)
+    torch.cuda.synchronize()
+    assert qa.q.shape == (M, 128) and qa.scales.shape == (1, M)
+    amax = x.abs().amax(1).float() if M else x.new_empty(0).float()
+    assert torch.allclose(qa.scales[0], torch.where(amax > 0, amax / 448, torch.ones_like(amax)), rtol=2 ** -22)
+    for at in (0, M // 2, M - 3):
+        if M:
+            part = (qa.q[at:at + 3].view(torch.float8_e4m3fn).float() * qa.scales[0, at:at + 3].unsqueeze(1))
+            assert torch.allclose(part, x[at:at + 3].float(), rtol=2 ** -4, atol=1e-6)       # e4m3: half a step is 2^-4
+
+
+def test_quantiser_without_columns():
+    from roc_shmem_b200.ops.gemm_fp8 import quantize_act
+    qa = quantize_act(torch.empty(5, 0, dtype=torch.bfloat16, device="cuda"))
+    assert qa.q.shape == (5, 0) and qa.scales.shape == (0, 5)
