@@ -848,7 +848,7 @@ int bshmem_gemm_fp8_blockscale(const void* A8, const float* scale_a, const void*
 // k-block kb goes to scales[kb * scale_ld + m] (scale_ld >= M: a shard can write its columns of a wider matrix).
 int bshmem_fp8_quant_act_ld(const void* x, int M, int K, int ldx, void* q, float* scales, int scale_ld, void* stream) {
   if (K % 128 || ldx % 4 || scale_ld < M) { host::last_error() = "fp8 quant: K % 128 != 0, ldx % 4 != 0 or scale_ld < M"; return 1; }
-  if (M <= 0 || K <= 0) return 0;        // nothing to quantise
+  if (M <= 0) return 0;                  // nothing to quantise
   // rows in blocks of 32 along the grid's y, which ends at 65535; beyond 2,097,120 rows the general kernel strides over them
   if (M <= 65535 * 32 && ldx % 8 == 0 && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q)) & 15)) {
     cudaLaunchConfig_t cfg = {};
