@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <utility>
 
 #include "../host/backend.h"
@@ -269,14 +270,39 @@ struct Pinned {
 };
 
 // What a host context owns on this backend: its ordering domain (a stream) and the pinned words its blocking calls
-// read results from.  Lane 0 is the default context; its stream is the settable PE stream.  Result words are handed
-// out round-robin per call, so threads that share a context do not read each other's answers.
+// read results from.  Lane 0 is the default context; its stream is the settable PE stream.
 struct Lane {
   cudaStream_t stream = nullptr;
   Pinned* pinned = nullptr;
   int* dstatus = nullptr;          // device status word of collectives launched on this lane
   std::atomic<unsigned> next{0};
+  std::atomic<bool> taken[kResultSlots] = {};      // slots whose call still waits for its answer
   bool open = false;
+};
+
+// A waiting call's own result slot of its lane, from before the launch until the answer has been read: threads that share the
+// lane do not meet on one, however many calls the others make meanwhile.  A call that nobody waits for has none (its kernel
+// signals nothing, also when it is replayed from a graph later on).
+class Ticket {
+ public:
+  explicit Ticket(Lane* lane) : lane_(lane) {
+    if (!lane) return;
+    for (;; std::this_thread::yield()) {             // beyond kResultSlots waiting calls: until one of them has returned
+      const unsigned k = lane->next.fetch_add(1, std::memory_order_relaxed);
+      slot = k % kResultSlots;
+      if (lane->taken[slot].exchange(true, std::memory_order_acquire)) continue;
+      done = {lane->pinned->done[slot], (uint64_t)k + 1};
+      return;
+    }
+  }
+  ~Ticket() { if (lane_) lane_->taken[slot].store(false, std::memory_order_release); }
+  Ticket(const Ticket&) = delete;
+  Ticket& operator=(const Ticket&) = delete;
+  unsigned slot = 0;
+  Done done{};
+
+ private:
+  Lane* lane_;
 };
 
 // Selection of the calling thread (see Backend::ctx_select) and an optional binding of the thread to one lane for
@@ -413,16 +439,6 @@ class GpuBackend final : public Backend {
     return check_device_error(what);
   }
 
-  // A call's result words: drawn per call, so threads that share a lane do not meet on one (see kResultSlots).
-  struct Ticket {
-    unsigned slot;
-    Done done;
-  };
-  Ticket draw(Lane& L) {
-    const unsigned k = L.next.fetch_add(1, std::memory_order_relaxed);
-    const unsigned i = k % kResultSlots;
-    return {i, {L.pinned->done[i], (uint64_t)k + 1}};
-  }
   // Waits until the kernel that got this ticket has signalled.  Polls for about 50 us; what takes longer (a wait_until,
   // a busy stream) or went wrong is left to a stream synchronisation.
   template <class Arrived>
@@ -451,7 +467,7 @@ class GpuBackend final : public Backend {
     };
     const int rc = poll(read, st);
     if (rc != BSHMEM_OK) return rc;
-    read();
+    if (!read()) { tl_err = "the call's kernel ended without an answer"; return BSHMEM_ERR_STATE; }
     *out = (uint32_t)lo | hi << 32;
     return BSHMEM_OK;
   }
@@ -494,9 +510,8 @@ class GpuBackend final : public Backend {
                  bool nbi) override {
     Lane& L = lane();
     const cudaStream_t st = stream_of(L);
-    Ticket t{};
     const bool wait = !nbi && blocking_now();
-    if (wait) t = draw(L);
+    const Ticket t(wait ? &L : nullptr);
     if (n == 0 || (tl_local_is_device && n <= kSmallSignalMax)) {
       RT_TRY(launch_small(k_put_signal, 1, n > 4096 ? 512 : 128, st, state_, heap_->base[pe] + dst_off, static_cast<const char*>(local), n,
                                                        reinterpret_cast<uint64_t*>(heap_->base[pe] + sig_off), sig_val, sig_op, t.done));
@@ -512,7 +527,7 @@ class GpuBackend final : public Backend {
   int read_word(int pe, uint64_t off, uint64_t size, uint64_t* out) override {
     Lane& L = lane();
     const cudaStream_t st = stream_of(L);
-    const Ticket t = draw(L);
+    const Ticket t(&L);
     RT_TRY(launch_small(k_read_word, 1, 1, st, heap_->base[pe] + off, (int)size, t.done));
     const int rc = wait_result(t, st, out);      // the value is the call's result: it is waited for in stream mode too
     if (rc != BSHMEM_OK) return rc;
@@ -525,10 +540,11 @@ class GpuBackend final : public Backend {
   int amo(int pe, uint64_t off, int dtype, int op, uint64_t value, uint64_t cond, uint64_t* fetched) override {
     Lane& L = lane();
     const cudaStream_t st = stream_of(L);
-    const Ticket t = draw(L);
+    const bool fetching = op <= BSHMEM_AMO_FETCH_CSWAP || op == BSHMEM_AMO_SWAP || (op >= BSHMEM_AMO_FETCH_AND && op <= BSHMEM_AMO_FETCH_XOR);
+    const bool wait = fetching || blocking_now();
+    const Ticket t(wait ? &L : nullptr);
     RT_TRY(launch_small(k_amo, 1, 1, st, state_, pe, off, dtype, op, value, cond, t.done));
-    bool fetching = op <= BSHMEM_AMO_FETCH_CSWAP || op == BSHMEM_AMO_SWAP || (op >= BSHMEM_AMO_FETCH_AND && op <= BSHMEM_AMO_FETCH_XOR);
-    if (fetching || blocking_now()) {
+    if (wait) {
       uint64_t old = 0;
       const int rc = wait_result(t, st, &old);
       if (rc != BSHMEM_OK) return rc;
@@ -550,9 +566,10 @@ class GpuBackend final : public Backend {
     s.timeout_ns = timeout_us * 1000ull;
     Lane& L = lane();
     const cudaStream_t st = stream_of(L);
-    const Ticket t = draw(L);
+    const bool wait = blocking_now();
+    const Ticket t(wait ? &L : nullptr);
     RT_TRY(launch_small(k_wait_until, 1, 1, st, s, off, dtype, cmp, value, t.done));
-    if (!blocking_now()) return BSHMEM_OK;
+    if (!wait) return BSHMEM_OK;
     uint64_t status = 0;
     int rc = wait_result(t, st, &status);
     if (rc != BSHMEM_OK) return rc;
@@ -567,7 +584,7 @@ class GpuBackend final : public Backend {
     s.stats = nullptr;
     Lane& L = lane();
     const cudaStream_t st = stream_of(L);
-    const Ticket t = draw(L);
+    const Ticket t(&L);
     RT_TRY(launch_small(k_wait_until, 1, 1, st, s, off, dtype, cmp, value, t.done));
     uint64_t status = 0;
     const int rc = wait_result(t, st, &status);
@@ -753,7 +770,7 @@ class GpuBackend final : public Backend {
       group_host_ = img;
     }
     GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
-    const Ticket t = draw(lanes_[0]);
+    const Ticket t(&lanes_[0]);
     int* status = &pinned_->status[t.slot];
     *status = 0;
     collk::GroupDone done;

@@ -98,3 +98,47 @@ def test_a_context_is_its_own_ordering_domain():
         b.destroy()
     finally:
         shmem.finalize()
+
+
+def test_a_waiting_call_keeps_its_answer():
+    """A fetching call waits for a busy stream while calls that nobody waits for run behind it, replayed from a graph that holds as
+    many as there are result slots: it returns its own answer.  So do more waiting calls at once than there are slots."""
+    import roc_shmem_b200 as shmem
+    rt = shmem.init("device", rank=0, world_size=1, heap_bytes=64 << 20, timeout_ms=5000)
+    try:
+        counter, other = rt.zeros((1,), torch.int64), rt.zeros((1,), torch.int64)
+        rt.set_blocking(False)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            rt.set_stream(torch.cuda.current_stream())
+            for _ in range(64):
+                rt.atomic_add(other, 1, 0)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            rt.set_stream(stream)
+            for i in range(20):
+                got, called = [], threading.Event()
+
+                def fetch():
+                    called.set()
+                    got.append(rt.atomic_fetch_add(counter, 5, 0))
+                torch.cuda._sleep(2_000_000)                 # about a millisecond: the answers come late
+                t = threading.Thread(target=fetch)
+                t.start()
+                called.wait()
+                graph.replay()
+                t.join()
+                assert got == [5 * i]
+                stream.synchronize()
+            answers = []
+            torch.cuda._sleep(20_000_000)
+            ths = [threading.Thread(target=lambda: answers.append(rt.atomic_fetch_add(counter, 1, 0))) for _ in range(150)]
+            for t in ths:
+                t.start()
+            for t in ths:
+                t.join()
+            assert sorted(answers) == list(range(100, 250))
+            assert rt.g(other, 0) == 20 * 64
+        del graph
+    finally:
+        shmem.finalize()
