@@ -29,6 +29,14 @@ struct CollArgs {
   int stage_oneshot;             // allreduce with stage_seq: 1 = every PE reduces the whole vector (one exchange), 0 = two-shot
 };
 
+// Whether a call's blocks move their shares through the bulk ring (of at least `min_bytes` each): the direct forms of fcollect
+// and alltoall on whole 16-byte pieces.  Nothing else of the unit uses it, and a block with a ring shares its multiprocessor
+// with few others.
+inline bool wants_move_ring(const CollArgs& a, int ctas, uint64_t min_bytes) {
+  const bool direct = (a.kind == 5 /* BSHMEM_COLL_FCOLLECT */ || a.kind == 6 /* BSHMEM_COLL_ALLTOALL */) && a.stage_seq == 0;
+  return direct && ((a.dst_off | a.src_off | a.n) & 15) == 0 && a.n / ctas >= min_bytes;
+}
+
 // Threads per block: 512 for the data-movement unit; 256 for the reduction units, whose unrolled multi-source loops
 // then have 255 registers per thread and compile without spills.
 constexpr int kMoveThreads = 512;

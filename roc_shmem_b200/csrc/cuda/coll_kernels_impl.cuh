@@ -28,7 +28,7 @@ uint32_t dyn_smem(const CollArgs&, int, int) { return kDynSmem; }
 constexpr uint32_t kDynSmem = coll::kMoveSmemBytes;
 uint32_t dyn_smem(const CollArgs& a, int ctas, int blocks) {
   int dev = 0, sms = 0;
-  if (a.n / ctas < coll::kMoveMinBytes || cudaGetDevice(&dev) != cudaSuccess ||
+  if (!wants_move_ring(a, ctas, coll::kMoveMinBytes) || cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || blocks > sms)
     return 0;
   return kDynSmem;
