@@ -757,8 +757,12 @@ class GpuBackend final : public Backend {
   int group_launch(const State* hs, const DTeam* ht, int n, const CollArgs& a, int ctas) {
     std::lock_guard<std::mutex> lock(group_mu_);
     if (!group_dev_) {
-      RT_TRY(cudaMalloc(&group_dev_, sizeof(GroupTable) + 16));
-      RT_TRY(cudaMemset(group_dev_, 0, sizeof(GroupTable) + 16));
+      // on the stream of the launch: it may be one that does not wait for the default stream
+      char* mem = nullptr;
+      RT_TRY(cudaMalloc(&mem, sizeof(GroupTable) + 16));
+      const cudaError_t e = cudaMemsetAsync(mem, 0, sizeof(GroupTable) + 16, stream_);
+      if (e != cudaSuccess) { cudaFree(mem); RT_TRY(e); }
+      group_dev_ = mem;
       memset(&group_host_, 0, sizeof(group_host_));
     }
     GroupTable img;

@@ -64,3 +64,31 @@ def test_group_moves(pes, ctas, nbytes):
                 assert torch.equal(d[:pes * nbytes], torch.cat([s[part] for s in src])) and bool((d[pes * nbytes:] == 7).all())
     finally:
         g.close()
+
+
+def test_first_collective_on_a_stream_of_its_own():
+    """A group made and used on a stream that does not wait for the default one, whose first call finds that stream busy: the
+    count of finished blocks starts at zero on the launch's stream (a call that returned early would find the old values)."""
+    import torch
+
+    from roc_shmem_b200 import gpu
+    from roc_shmem_b200.utils import dtypes as D
+    stream = torch.cuda.Stream()
+    for _ in range(3):
+        torch.cuda.synchronize()
+        junk = torch.full((1 << 20,), -1, dtype=torch.int32, device="cuda")          # what a fresh allocation may hold
+        del junk
+        torch.cuda.empty_cache()
+        with torch.cuda.stream(stream):
+            g = gpu.LocalGroup(4, heap_bytes=128 << 20)
+            src, dst = g.empty((4096,), torch.int32), g.empty((4096,), torch.int32)
+            for i, (s, d) in enumerate(zip(src, dst)):
+                s.fill_(i + 1)
+                d.zero_()
+            torch.cuda._sleep(20_000_000)
+            for _ in range(3):
+                g.collective(gpu.COLL_REDUCE, dst, src, 4096, dtype=torch.int32, op=D.SUM, ctas=4)
+                host = [d.cpu() for d in dst]
+                assert all(bool((h == 10).all()) for h in host)
+        for rt in g.pes:
+            rt.finalize()
