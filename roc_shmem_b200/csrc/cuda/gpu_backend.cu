@@ -782,9 +782,15 @@ class GpuBackend final : public Backend {
     done.word = t.done.word;
     done.token = t.done.token;
     cudaError_t e = collk::launch_group(dev->states, dev->teams, a, ctas, n, status, stream_, done);
-    if (e != cudaSuccess) { tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e); return BSHMEM_ERR_CUDA; }
+    if (e != cudaSuccess) {
+      cudaGetLastError();        // reported here, not at somebody's next launch
+      tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e);
+      return BSHMEM_ERR_CUDA;
+    }
     const int rc = wait_done(t, stream_);
-    return rc != BSHMEM_OK ? rc : *status;
+    if (rc != BSHMEM_OK || *status == BSHMEM_OK) return rc;
+    tl_err = std::string("device-side ") + bshmem_status_string(*status);
+    return *status;
   }
 
  private:
@@ -826,17 +832,18 @@ extern "C" {
 
 const char* bshmem_gpu_last_error(void) {
   if (!g_err.empty()) return g_err.c_str();
-  if (!tl_err.empty()) return tl_err.c_str();
   return gpu::heap_error().c_str();
 }
 
 int bshmem_gpu_heap_create(int my_pe, int n_pes, uint64_t heap_bytes, int device, int mode, void** heap) {
   gpu::Heap* h = nullptr;
+  g_err.clear();                 // what failed before on this thread is not this call's message
   int rc = gpu::heap_create(my_pe, n_pes, heap_bytes, device, mode, &h);
   if (rc == BSHMEM_OK) *heap = h;
   return rc;
 }
 int bshmem_gpu_heap_create_local_group(int n_pes, uint64_t heap_bytes, int device, void** heaps) {
+  g_err.clear();
   return gpu::heap_create_local_group(n_pes, heap_bytes, device, reinterpret_cast<gpu::Heap**>(heaps));
 }
 int bshmem_gpu_heap_export_fd(void* heap, int* fd) { return gpu::heap_export_fd(static_cast<gpu::Heap*>(heap), fd); }
@@ -1079,7 +1086,9 @@ int bshmem_gpu_group_collective(bshmem_handle_t* handles, int n, int team_slot, 
   CollArgs a{};
   a.kind = kind; a.dtype = dtype; a.op = op; a.root = root; a.dst_off = dst_off; a.src_off = src_off; a.n = count;
   if (ctas < 1) ctas = 1;
-  return g0->group_launch(hs, ht, n, a, ctas);
+  const int rc = g0->group_launch(hs, ht, n, a, ctas);
+  g_err = rc == BSHMEM_OK ? std::string() : g0->last_error();
+  return rc;
 }
 
 

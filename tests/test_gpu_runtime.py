@@ -340,3 +340,30 @@ def test_group_team_allreduce_low_latency_path(group):
         base = torch.arange(n, device="cuda", dtype=torch.float32) + rep
         assert torch.equal(dst[0], 2 * base + 20) and torch.equal(dst[2], 2 * base + 20)      # sum over PEs 0 and 2
         assert torch.equal(dst2[1], base + 30) and torch.equal(dst2[3], base + 30)            # max over PEs 1 and 3
+
+
+def test_error_messages_are_of_the_failing_call():
+    """A group that cannot be made does not report an earlier launch that did not fit, and the group works on after that one."""
+    import roc_shmem_b200 as shmem
+    from roc_shmem_b200 import gpu
+    from roc_shmem_b200.utils import dtypes as D
+    g = gpu.LocalGroup(8, heap_bytes=160 << 20)
+    try:
+        src, dst = g.empty((1 << 20,), torch.float32), g.empty((1 << 20,), torch.float32)
+        for t in src:
+            t.fill_(2)
+
+        def reduce(ctas):
+            g.collective(gpu.COLL_REDUCE, dst, src, 1 << 20, dtype=torch.float32, op=D.SUM, ctas=ctas)
+        with pytest.raises(shmem.ShmemError, match="cooperative"):                   # more blocks than the GPU holds at once
+            reduce(64)
+        with pytest.raises(shmem.ShmemError) as e:
+            gpu.LocalGroup(999)
+        assert "cooperative" not in str(e.value), str(e.value)
+        with pytest.raises(shmem.ShmemError, match="cooperative"):
+            reduce(64)
+        reduce(4)
+        assert all(bool((t == 16).all()) for t in dst)
+    finally:
+        for rt in g.pes:
+            rt.finalize()
