@@ -189,16 +189,18 @@ __device__ __forceinline__ bool check_target(const State& s, const void* sym, si
 
 // ---- ordering ---------------------------------------------------------------------------
 // fence: puts issued before it are delivered to each PE before puts issued after it.
-// quiet: every outstanding put/get/atomic of this thread is complete and visible.
-// With a load/store transport both are one fence, fence_peers.  It orders the thread's earlier accesses before its later ones as every PE sees them.  A system-scope fence takes 3 to 4 us on
-// a busy GPU, a GPU-scope one less than 1; the latter does when all PEs share the GPU.
+// quiet: every outstanding put/get/atomic of this thread is complete and visible, to the host as well: the local side of a get
+// may be pinned host memory, whose reader waits for what the thread writes after quiet.
+// With a load/store transport a fence is fence_peers: it orders the thread's earlier accesses before its later ones as every PE
+// sees them.  A system-scope fence takes 3 to 4 us on a busy GPU, a GPU-scope one less than 1; the latter does when all PEs
+// share the GPU.  quiet has system scope always.
 __device__ __forceinline__ void fence_peers(const State& s) {
   if (s.one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
   else asm volatile("fence.acq_rel.sys;" ::: "memory");
 }
 __device__ __forceinline__ void fence(const State& s) { fence_peers(s); stat(s, BSHMEM_DSTAT_FENCE); }
 __device__ __forceinline__ void fence_pe(const State& s, int) { fence(s); }
-__device__ __forceinline__ void quiet(const State& s) { fence_peers(s); stat(s, BSHMEM_DSTAT_QUIET); }
+__device__ __forceinline__ void quiet(const State& s) { asm volatile("fence.acq_rel.sys;" ::: "memory"); stat(s, BSHMEM_DSTAT_QUIET); }
 __device__ __forceinline__ void threadfence_system() { __threadfence_system(); }
 
 // ---- the copy engine: 16-byte vectors when both sides allow it ---------------------------
