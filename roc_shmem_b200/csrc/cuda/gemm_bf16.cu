@@ -1,6 +1,7 @@
-// gemm_bf16.cu — stand-alone tcgen05 bf16 GEMM:  C[M,N] = A[M,K] · B[N,K]^T
-// (both operands K-major, i.e. activations times a torch Linear weight), fp32
-// accumulation in TMEM, bf16 output through TMA stores; CTA pairs (cta_group::2) with
+// gemm_bf16.cu — stand-alone tcgen05 bf16 GEMM:  C[M,N] = op(A) · op(B)^T, each operand
+// K-major (activations, a torch Linear weight) or MN-major (as a gradient product finds it),
+// fp32 accumulation in TMEM, bf16 output through TMA stores (split tiles and a ragged last
+// column: direct stores); CTA pairs (cta_group::2) with
 // two accumulator stages, see gemm_pair.cuh.  This is the compute core
 // that the fused all-gather→GEMM and GEMM→reduce-scatter kernels build on; it has
 // no counterpart in the reference, which contains no GEMM.  Problems with few rows of A
@@ -169,8 +170,14 @@ struct SkinnyPlan {
 //    can split (4096x14336: 25.8 against 27.9)
 //  - above, only while the reduction can be split (3584x8192, 256 tokens: 19.8 against 24.7 for 256x256 tiles; 4096x14336
 //    unsplit: 38.0 against 31.6), and beyond 208 tokens only by four or more: split in two, a CTA loads all tokens for half of
-//    the reduction, a CTA pair on 256x256 tiles half of them (256 tokens: 8192x7168 34.6 against 31.6, 6168x4784 35.9 against
-//    27.5; 192 tokens: 29.1 against 31.1, 30.1 against 27.6; split in four, 14336x4096, 256 tokens: 33.6 against 42.9)
+//    the reduction, a CTA pair on 256x256 tiles half of them.  Where the lines cross depends on how the tiles fill the chip,
+//    few-token form against pairs at 176 / 208 / 224 / 240 / 256 tokens:
+//      8192x7168  30.2-31.8   32.1-33.3   33.3-34.4   37.1-34.8   38.7-35.7
+//      6168x4784  29.1-29.7   30.9-28.0   32.2-27.7   33.4-28.1   35.1-28.1
+//      3584x8192  16.4-18.8   17.4-19.0   17.3-18.9   18.7-18.9   20.0-19.0
+//      4096x6144  18.3-21.6   17.7-19.9   17.9-19.9   19.4-19.7   20.0-19.8
+//    208 gives up to 10 % away at 192 and 208 tokens for the second and about as much at 224 for the last two; split in four,
+//    14336x4096, 256 tokens: 33.6 against 42.9
 SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   if (M > skinny::MAX_TOKENS) return {0, false};
   const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS, kb = (K + skinny::BK - 1) / skinny::BK;

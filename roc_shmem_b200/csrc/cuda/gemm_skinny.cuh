@@ -18,7 +18,7 @@
 //   warps 2-5   epilogue
 // Every wait is bounded (see gemm_core.cuh).  The reference has no GEMM, hence no counterpart.
 #pragma once
-#include "gemm_core.cuh"
+#include "gemm_pair.cuh"
 
 namespace bshmem {
 namespace skinny {
@@ -26,6 +26,10 @@ namespace skinny {
 using gemm::Guard;
 using gemm::mbar_wait;
 using gemm::pack_bf16;
+using gemm2::cluster_ctarank;
+using gemm2::cluster_sync_all;
+using gemm2::ld_cluster_f4;
+using gemm2::mapa;
 
 constexpr int ROWS = 128;                          // weight rows of a tile
 constexpr int BK = 64;                             // bf16 elements per k-block: one 128-byte swizzle atom
@@ -56,29 +60,10 @@ struct Params {
 __host__ __device__ constexpr uint32_t stage_bytes(int nt) { return W_STAGE_BYTES + (uint32_t)nt * BK * 2; }
 __host__ __device__ constexpr uint32_t smem_bytes(int nt, int stages) { return stages * stage_bytes(nt) + CTRL_BYTES + 1024; }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-  float4 v;
-  // volatile keeps it behind the cluster barrier; without a memory clobber a run of them stays together
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
-}
 __device__ __forceinline__ float ld_cluster_f1(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
   return v;
-}
-__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-  return r;
 }
 
 struct Smem {
@@ -107,7 +92,7 @@ __device__ __forceinline__ void add_partials(const Params& p, uint32_t base, int
   constexpr int kTok = 8 / S < 1 ? 1 : 8 / S, kStep = S * (NUM_THREADS / 32);
   uint32_t src[S];
 #pragma unroll
-  for (int q = 0; q < S; ++q) src[q] = map_rank(base + lane * 16, q);
+  for (int q = 0; q < S; ++q) src[q] = mapa(base + lane * 16, q);
   for (int t0 = rank + warp * S; t0 < p.M; t0 += kTok * kStep) {
     float4 v[kTok][S];
 #pragma unroll
@@ -150,7 +135,7 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = p.split;
-  const int rank = split > 1 ? (int)cluster_rank() : 0;
+  const int rank = split > 1 ? (int)cluster_ctarank() : 0;
   const int n0 = (int)(blockIdx.x / split) * ROWS;
   const int kb_all = (p.K + BK - 1) / BK;
   const int kb0 = kb_all * rank / split, kb1 = kb_all * (rank + 1) / split;
@@ -245,14 +230,14 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
   ptx::tc_fence_before();
   __syncthreads();
   if (split > 1) {
-    cluster_sync();
+    cluster_sync_all();
     // every CTA adds the partials of the tokens rank, rank + split, ...
     if (!*L.abort_flag() && n0 + lane * 4 < p.N) {
       if (split == 2) add_partials<2>(p, L.base, rank, warp, lane, n0);
       else if (split == 4) add_partials<4>(p, L.base, rank, warp, lane, n0);
       else add_partials<8>(p, L.base, rank, warp, lane, n0);
     }
-    cluster_sync();                                  // nobody's shared memory goes away while it is being read
+    cluster_sync_all();                                  // nobody's shared memory goes away while it is being read
   }
   if (*L.abort_flag()) {
     // let copies and MMAs that are still in flight land before shared and tensor memory go away
@@ -271,7 +256,7 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
 
 // ---- grouped form: few tokens per group (the experts of a decode step) -----------------------------------------------
 //   C_g[rows_g, N] = X_g[rows_g, K] · W_g[N, K]^T  for every group g, the row counts read on the device.
-// Persistent CTAs over (group, chunk of up to 256 tokens, 128 weight rows); groups without rows cost nothing.  Two
+// Persistent CTAs over (group, chunk of up to 128 tokens, 128 weight rows); groups without rows cost nothing.  Two
 // accumulators, so that the epilogue of a tile overlaps the loads and MMAs of the next.  The stage size follows the
 // largest group of the call: 16 KiB of weights plus 128 bytes per token, as many stages as fit.
 // Gated: the weight rows are 32 gate rows followed by the matching 32 up rows, i.e. alternating quarters of the tensor
@@ -288,15 +273,15 @@ constexpr uint32_t GROUP_XCHG_BYTES = 2 * 2 * 16 * 32 * 4;             // two wa
 constexpr uint32_t GROUP_CTRL_BYTES = 8 * (2 * MAX_GROUP_STAGES + 6) + 16 + 4 * MAX_GROUPS;
 
 struct GroupedParams {
-  CUtensorMap map_w, map_x;      // weights [G * N, K] box {64, 128}; tokens [G * cap, K] box {64, 16}
+  CUtensorMap map_w, map_x;      // weights [G * N, K] box {64, 128}; tokens [G * cap, K] box {64, xbox}
   __nv_bfloat16* out;            // [G * cap, N] or gated [G * cap, N / 2]
   long long ldo;
   const int* rows;
   int G, cap, N, K;
-  int xbox;                      // token rows per TMA box: 16, 32, 64 or 128
+  int xbox;                      // token rows per TMA box: 16 or 32
   uint32_t ring_bytes;           // shared memory of the stages
   uint32_t tmem_cols;            // two accumulators
-  int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 256)
+  int nt_cap;                    // tokens per chunk that the tensor memory holds (multiple of 16, at most 128)
   int split;                     // > 1: clusters of that many CTAs share the reduction of a tile while each has one at most
   int P;                         // arrival words to wait for before the first token load (0: none)
   const unsigned long long* arrive;
@@ -385,7 +370,7 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   const uint32_t stage = W_STAGE_BYTES + (uint32_t)((nt_max + p.xbox - 1) / p.xbox * p.xbox) * BK * 2;
   const int stages = min((int)(p.ring_bytes / stage), MAX_GROUP_STAGES);
   const int kb_all = (p.K + BK - 1) / BK;
-  const int rank = split > 1 ? (int)cluster_rank() : 0;
+  const int rank = split > 1 ? (int)cluster_ctarank() : 0;
   const int kb0 = kb_all * rank / split, kb1 = kb_all * (rank + 1) / split;
   GroupedTiles it{L.rows(), p.G, p.N / ROWS, p.nt_cap, (int)blockIdx.x / split, (int)gridDim.x / split, 0, 0};
   struct { int grp, n_blk, tok0, ntok; } split_tile = {0, 0, 0, 0};
@@ -509,13 +494,13 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   ptx::tc_fence_before();
   __syncthreads();
   if (split > 1) {
-    cluster_sync();
+    cluster_sync_all();
     if (mine && !*L.abort_flag()) {
       // one warp per token; a lane's sum over the parts of weight row r of token t
       auto sum = [&](int t, int r) {
         float f = 0.f;
 #pragma unroll 4
-        for (int q = 0; q < split; ++q) f += ld_cluster_f1(map_rank(L.base + (t * ROWS + r) * 4, q));
+        for (int q = 0; q < split; ++q) f += ld_cluster_f1(mapa(L.base + (t * ROWS + r) * 4, q));
         return f;
       };
       for (int t = rank + warp * split; t < split_tile.ntok; t += split * (NUM_THREADS / 32)) {
@@ -532,7 +517,7 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
         }
       }
     }
-    cluster_sync();                                  // nobody's shared memory goes away while it is being read
+    cluster_sync_all();                                  // nobody's shared memory goes away while it is being read
   }
   if (*L.abort_flag()) {
     const unsigned long long t0 = ptx::globaltimer();

@@ -66,8 +66,8 @@ __device__ uint64_t amo_exec(W* p, int dtype, int op, uint64_t value, uint64_t c
   return (uint64_t)old;
 }
 
-// The kernels of messages are launched with programmatic serialization: such a launch costs the host 2.9 us instead of 3.7
-// and the kernel is on the device when its predecessor in the stream ends, for which it waits here before it touches anything.
+// The kernels of messages are launched with programmatic serialization: such a launch costs the host 2.9 us instead of 3.7 (2.4
+// on a faster host) and the kernel is on the device when its predecessor in the stream ends, for which it waits here before it touches anything.
 __device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 cudaError_t launch_overlapping(void (*kernel)(P...), unsigned grid, unsigned block, unsigned smem, cudaStream_t st, A&&... args) {
@@ -167,8 +167,8 @@ __global__ void k_write_word(char* dst, uint64_t v, int size) {
   for (int i = 0; i < size; ++i) reinterpret_cast<uint8_t*>(dst)[i] = (uint8_t)(v >> (8 * i));
 }
 
-// Small device-to-device messages.  A copy-engine request costs the host 3.4 us, a kernel launch 2.4 us (both measured
-// back to back), and that is the message rate; the copy itself is shorter than either.  A block moves kSmallPiece
+// Small device-to-device messages.  A copy-engine request costs the host 3.4 us, a kernel launch 2.4 us (measured
+// back to back on one host), and that is the message rate; the copy itself is shorter than either.  A block moves kSmallPiece
 // bytes: one 16-byte access per thread, so a message of up to kSmallCopyMax takes one round trip to memory.
 // The line: 64 puts of 256 KiB to 1 MiB take 157 to 162 us through the kernel and 245 to 259 us through the copy engine.
 // At 2 MiB (230 and 262 us) the kernel's own time shows, and that size stays with the copy engine, which takes no SM.

@@ -1,9 +1,10 @@
 // moe_gemm.cu — grouped (per-expert) tcgen05 GEMM for the MoE layer.  The K-major forms (gate/up, down and the two
-// data-gradient GEMMs) run on the CTA-pair main loop of gemm_pair.cuh (cta_group::2, the epilogue of one tile overlaps
-// the MMAs of the next); the weight-gradient form on token-major operands and the ragged-K form run on the
-// single-CTA main loop of gemm_core.cuh.
+// data-gradient GEMMs) and the weight-gradient form on token-major operands run on the CTA-pair main loop of gemm_pair.cuh
+// (cta_group::2, the epilogue of one tile overlaps the MMAs of the next), few rows per expert on the grouped form of
+// gemm_skinny.cuh; the ragged-K form runs on the single-CTA main loop of gemm_core.cuh, as does the weight-gradient form on a
+// device that holds no CTA pair of it.
 //
-//   C_g = A_g · B_g^T  for every local expert g, all operands K-major bf16:
+//   C_g = A_g · B_g^T  for every local expert g, bf16 operands, K-major but for the weight gradient's:
 //     rows mode   A: [G][cap rows][K]   B: [G][N][K]    C: [G][cap][N]
 //                 the row count of group g is read from device memory (tokens that arrived),
 //                 so no host synchronisation is needed between dispatch and the GEMM;

@@ -45,7 +45,7 @@ static __nv_bfloat16 __float2bfloat16_rn(float) { return 1; }
 struct Core { int M, N; };
 struct Params { Core core; __nv_bfloat16* out; long long ldc, ldo; int M, N; };
 constexpr int ROWS = 128, NUM_THREADS = 192;
-static uint32_t map_rank(uint32_t a, uint32_t) { return a; }
+static uint32_t mapa(uint32_t a, uint32_t) { return a; }
 static float4 ld_cluster_f4(uint32_t) { return {1, 1, 1, 1}; }
 """ + pair.replace("static __forceinline__", "static") + "\ntemplate <int S>\n" + few + r"""
 int main() {

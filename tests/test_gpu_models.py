@@ -29,7 +29,7 @@ def test_custom_op_linear_forward_backward():
     assert (y.float() - yr).abs().max().item() <= 2e-2 * yr.abs().max().item() + 1e-2
     assert (x.grad.float() - xr.grad).abs().max().item() <= 2e-2 * xr.grad.abs().max().item() + 1e-2
     assert (lin.weight.grad.float() - wr.grad).abs().max().item() <= 2e-2 * wr.grad.abs().max().item() + 1e-2
-    # odd shapes take the transposing fall-back of the weight gradient
+    # sizes that fill no tile, in all three products
     lin2 = Linear(136, 72, device="cuda")
     x2 = torch.randn(40, 136, device="cuda").to(torch.bfloat16).requires_grad_(True)
     lin2(x2).sum().backward()
