@@ -1,8 +1,8 @@
 // gemm_bf16.cu — stand-alone tcgen05 bf16 GEMM:  C[M,N] = op(A) · op(B)^T, each operand
 // K-major (activations, a torch Linear weight) or MN-major (as a gradient product finds it),
 // fp32 accumulation in TMEM, bf16 output through TMA stores (split tiles and a ragged last
-// column: direct stores); CTA pairs (cta_group::2) with
-// two accumulator stages, see gemm_pair.cuh.  This is the compute core
+// column: direct stores); CTA pairs (cta_group::2) on tiles of
+// 256 rows and 128 to 512 columns, see gemm_pair.cuh and plan_width.  This is the compute core
 // that the fused all-gather→GEMM and GEMM→reduce-scatter kernels build on; it has
 // no counterpart in the reference, which contains no GEMM.  Problems with few rows of A
 // take the weight-streaming kernel of gemm_skinny.cuh instead (plan_skinny says when).
@@ -20,6 +20,7 @@ namespace {
 struct PlainParams {
   CoreParams core;
   CUtensorMap map_a, map_b, map_c;
+  CUtensorMap map_b2, map_c2;  // B rows of a second accumulator (wide form), output boxes of 32 columns
   __nv_bfloat16* out;          // split form: the result, written directly
   long long ldc;
 };
@@ -28,10 +29,11 @@ struct PlainParams {
 // MN-major (true): A is stored [K][M], as a gradient GEMM finds it; a stage holds two 64-wide column blocks of 64 reduction
 // rows (8 KiB each, 128-byte swizzle), which the tensor core reads through MN-major descriptors — no transposed copy.
 // Rows and columns beyond the matrix, the reduction included, are zero-filled by TMA.
-template <bool kAmn, bool kBmn, bool kSplitK>
+enum Form { NARROW, WIDE, SPLIT };
+template <bool kAmn, bool kBmn, int kForm>
 struct PlainBf16 : PolicyDefaults {
   using Params = PlainParams;
-  static constexpr bool kSplit = kSplitK;
+  static constexpr bool kSplit = kForm == SPLIT, kWide = kForm == WIDE, kVarCols = !kSplit;
   static constexpr uint32_t kIdesc = kIdescBf16 | (kAmn ? 1u << 15 : 0u) | (kBmn ? 1u << 16 : 0u);
   static constexpr uint32_t kBlock = 64 * BK_BYTES;           // one 64 (MN) x 64 (K) block
   static constexpr uint32_t kKStepA = kAmn ? 2048 : UMMA_K_BYTES, kKStepB = kBmn ? 2048 : UMMA_K_BYTES;
@@ -52,6 +54,23 @@ struct PlainBf16 : PolicyDefaults {
       ptx::tma_load_2d(b_smem, mb, bar, kb * BK, b_row);
     }
   }
+  // MN-major column blocks are loaded whole, also where the CTA's half of an accumulator ends inside the second one
+  __device__ static __forceinline__ void load_b(const Params& p, const CUtensorMap* mb, uint32_t b_smem, uint32_t bar, int kb, int b_row, int, int, int) {
+    if constexpr (kBmn) {
+      ptx::tma_load_2d(b_smem, mb, bar, b_row, kb * BK);
+      ptx::tma_load_2d(b_smem + kBlock, mb, bar, b_row + 64, kb * BK);
+    } else {
+      ptx::tma_load_2d(b_smem, &p.map_b2, bar, kb * BK, b_row);
+    }
+  }
+  __device__ static __forceinline__ int acc_cols(const Params& p, int a) { return kVarCols ? p.core.acc_cols[a] : BN; }
+  __device__ static __forceinline__ uint32_t stage_tx(const Params& p) {
+    if constexpr (kBmn || !kVarCols) return kWide ? WIDE_STAGE_BYTES : STAGE_BYTES;
+    return A_STAGE_BYTES + (uint32_t)(p.core.acc_cols[0] + (kWide ? p.core.acc_cols[1] : 0)) / 2 * BK_BYTES;
+  }
+  __device__ static __forceinline__ int b_row(const Params& p, int, int n_blk) {
+    return n_blk * (acc_cols(p, 0) + (kWide ? acc_cols(p, 1) : 0));
+  }
   __device__ static __forceinline__ const CoreParams& core(const Params& p) { return p.core; }
   __device__ static __forceinline__ const CUtensorMap* map_a(const Params& p) { return &p.map_a; }
   __device__ static __forceinline__ const CUtensorMap* map_b(const Params& p) { return &p.map_b; }
@@ -63,14 +82,19 @@ struct PlainBf16 : PolicyDefaults {
     *x = col;
     *y = row;
   }
-  static constexpr bool kRaggedCols = !kSplitK;
+  __device__ static __forceinline__ void out_target_half(const Params& p, int row, int col, const CUtensorMap** map, int* x, int* y) {
+    *map = (row < p.core.M && col < p.core.N) ? &p.map_c2 : nullptr;
+    *x = col;
+    *y = row;
+  }
+  static constexpr bool kRaggedCols = kVarCols;
   __device__ static __forceinline__ bool ragged_chunk(const Params& p, int col) { return (p.core.N & 7) && col < p.core.N && col + EPI_COLS > p.core.N; }
-  __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const float (&f)[64]) {
+  __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const float (&f)[64], int cols) {
     if (row >= p.core.M) return;
     __nv_bfloat16* dst = p.out + row * p.ldc + col;
 #pragma unroll
     for (int j = 0; j < 64; ++j)
-      if (col + j < p.core.N) dst[j] = __float2bfloat16_rn(f[j]);
+      if (j < cols && col + j < p.core.N) dst[j] = __float2bfloat16_rn(f[j]);
   }
   // 16 columns of a row: one 32-byte sector, as far as the matrix goes (N need not be a multiple of 8 when B is K-major)
   __device__ static __forceinline__ void store_row16(const Params& p, int row, int col, const float4 (&v)[4]) {
@@ -95,16 +119,23 @@ struct PlainBf16 : PolicyDefaults {
 template <bool kAmn, bool kBmn>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) gemm_bf16_kernel(const __grid_constant__ PlainParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_mainloop<PlainBf16<kAmn, kBmn, false>>(prm, smem_raw);
+  gemm_mainloop<PlainBf16<kAmn, kBmn, NARROW>>(prm, smem_raw);
+}
+template <bool kAmn, bool kBmn>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) gemm_bf16_wide_kernel(const __grid_constant__ PlainParams prm) {
+  extern __shared__ uint8_t smem_raw[];
+  gemm_mainloop<PlainBf16<kAmn, kBmn, WIDE>>(prm, smem_raw);
 }
 template <bool kAmn, bool kBmn>                       // cluster size at launch: 2 * split
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_bf16_split_kernel(const __grid_constant__ PlainParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_mainloop<PlainBf16<kAmn, kBmn, true>>(prm, smem_raw);
+  gemm_mainloop<PlainBf16<kAmn, kBmn, SPLIT>>(prm, smem_raw);
 }
 using PlainKernel = void (*)(PlainParams);
 constexpr PlainKernel kPlainKernels[2][2] = {{gemm_bf16_kernel<false, false>, gemm_bf16_kernel<false, true>},
                                              {gemm_bf16_kernel<true, false>, gemm_bf16_kernel<true, true>}};
+constexpr PlainKernel kWideKernels[2][2] = {{gemm_bf16_wide_kernel<false, false>, gemm_bf16_wide_kernel<false, true>},
+                                            {gemm_bf16_wide_kernel<true, false>, gemm_bf16_wide_kernel<true, true>}};
 constexpr PlainKernel kSplitKernels[2][2] = {{gemm_bf16_split_kernel<false, false>, gemm_bf16_split_kernel<false, true>},
                                              {gemm_bf16_split_kernel<true, false>, gemm_bf16_split_kernel<true, true>}};
 
@@ -126,6 +157,8 @@ int ensure_device_state(int dev) {
   BSHMEM_CUDA_TRY(cudaMemset(g_err_dev[dev], 0, sizeof(int)));
   BSHMEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   for (auto& row : kPlainKernels)
+    for (PlainKernel k : row) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+  for (auto& row : kWideKernels)
     for (PlainKernel k : row) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
   for (auto& row : kSplitKernels)
     for (PlainKernel k : row) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
@@ -192,6 +225,39 @@ SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   if (full > 1) return {full, false};
   if (M <= 128) return {best(true), true};
   return {0, false};
+}
+
+// Columns of a tile's one accumulator, or of its two (wide form; see gemm_pair.cuh).  What a launch costs is the number of waves
+// times the width of a tile, as long as the tensor cores are the bound: 1000 x 7168 x 8192 takes 108 us as two waves of 256 columns
+// (112 tiles on 74 pairs), 98 as one of 448 and 95 as one of 416.  Beside that
+//  - a tile of one accumulator reads its A rows for half as many columns.  Per k-block it takes as long as (256 + width) / 2
+//    columns of a wide one (1000 x 7168 x 8192 by 224 columns: 107 us, also two waves), and under the power cap, where an SM's
+//    loads cost clock, 10 % more at the same number of columns (8192 x 8192 x 3584: 367 us, 350 by 512 columns; 8192 x 7168 x 8192:
+//    765, and 710 by 448).  With a few k-blocks this turns round, because a wide tile fills and drains the ring more often
+//    than it streams (7168 x 8192, 848 deep: 89.7 and 93.7 us; 384 deep: 55.6 and 57.6; 4096 x 4096, 744 deep: 26.5 and 25.4);
+//  - MN-major rows of B come in blocks of 64 columns per CTA, and what is loaded beyond the width counts half;
+//  - a wave has a beginning and an end, worth about 8 columns.
+// Over 30 problems of 264 to 8192 rows in the three layouts the choice was within 4 % of the best of ten widths.
+struct Width {
+  int cols[2];
+};
+Width plan_width(int M, int N, int K, int pairs, bool b_mn) {
+  const long long mb = (M + BM - 1) / BM;
+  const double deep = 0.91 + (K + BK - 1) / BK / 160.0, narrow = deep < 1.1 ? deep : 1.1;
+  Width best = {{BN, 0}};
+  double best_cost = 1e30;
+  for (int w = 2 * BN; w >= 128; w -= 32) {
+    if (w > BN && w < 352) continue;                  // two accumulators of less than 160 columns
+    const int c0 = w > BN ? (w + 63) / 64 * 32 : w, c1 = w - c0;
+    const int loaded = b_mn ? (c0 + 127) / 128 * 128 + (c1 + 127) / 128 * 128 : w;
+    const long long tiles = mb * ((N + w - 1) / w), waves = (tiles + pairs - 1) / pairs;
+    const double cost = waves * ((c1 ? 0.5 * (w + loaded) : narrow * 0.5 * (BN + loaded)) + 8);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = {{c0, c1}};
+    }
+  }
+  return best;
 }
 
 // Few tokens: weight-streaming kernel (gemm_skinny.cuh).
@@ -266,33 +332,44 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
     const SkinnyPlan plan = plan_skinny(M, N, K, dev);
     if (plan.split) return launch_skinny(A, B, C, M, N, K, lda, ldb, ldc, b_mn != 0, st, dev, timeout_ns, plan);
   }
+  int pairs = g_pairs[dev];
+  if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  // Few tiles: split each over the two or four pairs of a cluster while all clusters run at once.  Parking and adding the
+  // parts costs about 4 us, what a pair needs for 14 k-blocks.
+  const int kb = (K + BK - 1) / BK;
   PlainParams p;
+  p.core.split = 1;
+  if (max_ctas <= 1) {
+    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    if (tiles <= g_octs[dev] && kb >= 24) p.core.split = 4;
+    else if (tiles <= g_quads[dev] && kb >= 32) p.core.split = 2;
+  }
+  const Width w = p.core.split > 1 ? Width{{BN, 0}} : plan_width(M, N, K, pairs, b_mn != 0);
+  const int width = w.cols[0] + w.cols[1];
+  p.core.acc_cols[0] = w.cols[0];
+  p.core.acc_cols[1] = w.cols[1];
   p.core.M = M; p.core.N = N; p.core.K = K;
   p.core.num_m_blocks = (M + BM - 1) / BM;
-  p.core.num_n_blocks = (N + BN - 1) / BN;
-  p.core.group_m = 8;
+  p.core.num_n_blocks = (N + width - 1) / width;
+  // row blocks that are worked on side by side: wide tiles are fewer (8192 x 8192 x 3584 by 512 columns: 4, 8, 12, 16 row blocks
+  // 365, 355, 352, 350 us)
+  p.core.group_m = w.cols[1] ? 16 : 8;
   p.core.timeout_ns = timeout_ns;
   p.core.err = g_err_dev[dev];
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   rc = a_mn ? host::make_tmap_2d(&p.map_a, bf, 2, A, K, M, lda, 64, 64) : host::make_tmap_2d(&p.map_a, bf, 2, A, M, K, lda, CTA_M, 64);
   if (rc) return rc;
-  rc = b_mn ? host::make_tmap_2d(&p.map_b, bf, 2, B, K, N, ldb, 64, 64) : host::make_tmap_2d(&p.map_b, bf, 2, B, N, K, ldb, CTA_NLOAD, 64);
+  rc = b_mn ? host::make_tmap_2d(&p.map_b, bf, 2, B, K, N, ldb, 64, 64) : host::make_tmap_2d(&p.map_b, bf, 2, B, N, K, ldb, w.cols[0] / 2, 64);
+  if (rc) return rc;
+  if (w.cols[1] && !b_mn) rc = host::make_tmap_2d(&p.map_b2, bf, 2, B, N, K, ldb, w.cols[1] / 2, 64);
+  if (rc) return rc;
+  if ((w.cols[0] | w.cols[1]) & 63) rc = host::make_tmap_2d(&p.map_c2, bf, 2, C, M, N, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
   if (rc) return rc;
   rc = host::make_tmap_2d(&p.map_c, bf, 2, C, M, N, ldc, 32, EPI_COLS);
   if (rc) return rc;
   const int tiles = p.core.num_m_blocks * p.core.num_n_blocks;
-  int pairs = g_pairs[dev];
-  if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   p.out = static_cast<__nv_bfloat16*>(C);
   p.ldc = ldc;
-  // Few tiles: split each over the two or four pairs of a cluster while all clusters run at once.  Parking and adding the
-  // parts costs about 4 us, what a pair needs for 14 k-blocks.
-  const int kb = (K + BK - 1) / BK;
-  p.core.split = 1;
-  if (max_ctas <= 1) {
-    if (tiles <= g_octs[dev] && kb >= 24) p.core.split = 4;
-    else if (tiles <= g_quads[dev] && kb >= 32) p.core.split = 2;
-  }
   if (tiles < pairs) pairs = tiles;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs * p.core.split));
@@ -306,7 +383,7 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
   attr[1].val.clusterDim.x = (unsigned)(2 * p.core.split); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.core.split > 1 ? 2 : 1;
-  const auto& kernels = p.core.split > 1 ? kSplitKernels : kPlainKernels;
+  const auto& kernels = p.core.split > 1 ? kSplitKernels : w.cols[1] ? kWideKernels : kPlainKernels;
   BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernels[a_mn ? 1 : 0][b_mn ? 1 : 0], p));
   return 0;
 }

@@ -57,6 +57,7 @@ struct CoreParams {
   unsigned long long timeout_ns;
   int* err;                // device word: first error site, 0 = none
   int split;               // CTA-pair core, split form: pairs per tile
+  int acc_cols[2];         // CTA-pair core, policies with a width of their own: columns of the tile in accumulator 0 and 1
 };
 
 struct Guard {

@@ -1,7 +1,7 @@
 // gemm_pair.cuh — persistent tcgen05 GEMM main loop on CTA PAIRS (cta_group::2) for
 // sm_100a:  C[M,N] = A[M,K] · B[N,K]^T, bf16 operands, fp32 accumulation in TMEM.
 //
-// A thread-block cluster of two CTAs (two SMs of one TPC) owns a 256x256 output tile:
+// A thread-block cluster of two CTAs (two SMs of one TPC) owns an output tile of 256 rows and up to 256 columns:
 //   CTA r of the pair loads A rows [128r, 128r+128) and B rows [128r, 128r+128) of the
 //   tile — 32 KiB per stage and CTA, plain (non-multicast) TMA loads from this GPU's own
 //   memory — and holds the accumulator of its 128 output rows x 256 columns in its TMEM.
@@ -23,6 +23,11 @@
 //
 // tcgen05.commit (with its cluster-multicast form, a barrier arrival, not a load) hands
 // stages and accumulators back to BOTH CTAs.
+// Wide form (policy with kWide): a tile takes both accumulators, up to 512 columns.  Its A rows are loaded once for all of
+// them, a quarter less traffic from L2 per product, and read once from shared memory: the MMAs of a k-block go to the two
+// accumulators in turn, and the second of each two takes A from the collector buffer.  That is what bounds a long launch,
+// which runs at the clock that the power cap leaves: 8192 x 8192 x 3584 went from 367 to 350 us (1.31 -> 1.38 PFLOP/s).  The epilogue still overlaps the MMAs: at a tile's ends WIDE_BATCH k-blocks go into one
+// accumulator first, then into the other, so that each has the time of a batch to be drained.
 // Split form (policy with kSplit, for problems with fewer than about half as many tiles as the chip has pairs): the
 // cluster is S = 2 or 4 pairs that share one tile.  Each pair sums its share of K; then every CTA parks its fp32
 // accumulator (128 x 256, 128 KiB) over its drained ring, and after one cluster barrier CTA (pair j, half r) adds the S
@@ -66,6 +71,14 @@ constexpr uint32_t SMEM_BARS = 512;
 constexpr uint32_t SMEM_BYTES = SMEM_TILES + SMEM_BARS + 1024 /*alignment slack*/;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_COLS = 256;
+// Wide form: a stage holds B rows for both accumulators, and the same shared memory makes four of them.
+constexpr int WIDE_STAGES = 4;
+constexpr uint32_t WIDE_STAGE_BYTES = A_STAGE_BYTES + 2 * B_STAGE_BYTES;
+// k-blocks at a tile's ends that go into one accumulator before the other (at most WIDE_STAGES): one does not cover the drain
+// (8192 x 8192 x 3584: 354 us), with two or three (349, 348) the ring keeps a stage on its way, with four (350) none, which a
+// reduction of 16 k-blocks notices (7168 x 8192: 108 us; 108, 105, 104 with one, two, three).
+constexpr int WIDE_BATCH = 3;
+static_assert(WIDE_STAGES * WIDE_STAGE_BYTES == STAGES * STAGE_BYTES, "both forms share one carve-up");
 constexpr uint32_t kIdescBf16 = ptx::umma_idesc(1, 1, BM, BN);
 
 enum ErrSite : int {
@@ -118,6 +131,23 @@ __device__ __forceinline__ void umma2_f16(uint32_t d_tmem, uint64_t a_desc, uint
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Two MMAs of the same A, one after the other: the first keeps it in the collector buffer, the second reads it from there.
+__device__ __forceinline__ void umma2_f16_keep_a(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma2_f16_kept_a(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // One commit that arrives on the barrier at this offset in BOTH CTAs of the pair (two single-destination commits
 // per k-block cost the issuing thread 6 % of the GEMM's throughput).
 __device__ __forceinline__ void umma2_commit_both(uint32_t bar, uint32_t lead) {
@@ -159,8 +189,6 @@ __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, Guard& 
 struct Smem {
   uint32_t base;        // 1024-byte aligned
   uint8_t* gen;         // generic pointer to the same byte
-  __device__ __forceinline__ uint32_t a(int s) const { return base + s * STAGE_BYTES; }
-  __device__ __forceinline__ uint32_t b(int s) const { return base + s * STAGE_BYTES + A_STAGE_BYTES; }
   __device__ __forceinline__ uint32_t epi(int w) const { return base + STAGES * STAGE_BYTES + w * EPI_BUF_BYTES; }
   __device__ __forceinline__ uint8_t* epi_gen(int w) const { return gen + STAGES * STAGE_BYTES + w * EPI_BUF_BYTES; }
   __device__ __forceinline__ uint32_t bars() const { return base + SMEM_TILES; }
@@ -203,6 +231,15 @@ struct PolicyDefaults {
   struct EpiState {};
   // Split form: clusters of 2 * CoreParams::split CTAs, one tile each, output written by store_rows instead of TMA.
   static constexpr bool kSplit = false;
+  // Wide form: a tile takes both accumulators, columns [0, acc_cols(0)) and the acc_cols(1) behind them, and load_b loads the
+  // second one's rows of B.
+  static constexpr bool kWide = false;
+  // kVarCols: an accumulator may hold fewer than 256 columns (a multiple of 32), and out_target is asked for a 32-column box
+  // where a chunk of 64 does not fit.  The widths of the others are fixed.
+  static constexpr bool kVarCols = false;
+  template <class Params> __device__ static __forceinline__ int acc_cols(const Params&, int) { return BN; }
+  // bytes that the loads of a stage bring into one CTA
+  template <class Params> __device__ static __forceinline__ uint32_t stage_tx(const Params&) { return STAGE_BYTES; }
   // Gated epilogue: inside every 64-column chunk of the accumulator, columns 0-31 are gate pre-activations and 32-63
   // the matching up-projections; the epilogue writes silu(gate) * up, i.e. half as many output columns (the two
   // chunks of a warp make one 32 x 64 output box; out_target gets the OUTPUT column).
@@ -229,9 +266,14 @@ struct PolicyDefaults {
     ptx::tma_load_2d(a_smem, ma, bar, kb * BK, a_row);
     ptx::tma_load_2d(b_smem, mb, bar, kb * BK, b_row);
   }
+  // wide form: this CTA's rows of the second accumulator's columns
+  template <class Params>
+  __device__ static __forceinline__ void load_b(const Params&, const CUtensorMap* mb, uint32_t b_smem, uint32_t bar, int kb, int b_row, int, int, int) {
+    ptx::tma_load_2d(b_smem, mb, bar, kb * BK, b_row);
+  }
   // k-blocks of the tile's reduction (ragged per group in the grouped weight-gradient GEMM); at least 1
   template <class Params> __device__ static __forceinline__ int num_kb(const Params& p, int) { return (p.core.K + BK - 1) / BK; }
-  // first row of the 256-row block of A / of the 256-row block of B that tile (m_blk, n_blk) multiplies
+  // first row of the 256-row block of A / of the tile's block of B that tile (m_blk, n_blk) multiplies
   template <class Params> __device__ static __forceinline__ int a_row(const Params&, int m_blk) { return m_blk * BM; }
   template <class Params> __device__ static __forceinline__ int b_row(const Params&, int, int n_blk) { return n_blk * BN; }
   template <class Params> __device__ static __forceinline__ bool a_ready(const Params&, int, Guard&) { return true; }
@@ -264,6 +306,21 @@ __device__ __forceinline__ void stage_chunk(uint32_t buf, int lane, const float 
     const uint32_t w0 = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]), w1 = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
     const uint32_t w2 = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]), w3 = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
     const uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
+
+// The first 32 of them, for a store box of 32 columns: four pieces per row, piece j at (j ^ (row / 2 & 3)) under the
+// 64-byte swizzle.
+__device__ __forceinline__ void stage_half_chunk(uint32_t buf, int lane, const float (&f)[64]) {
+  const uint32_t rowbase = buf + lane * 64;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t w0 = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]), w1 = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
+    const uint32_t w2 = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]), w3 = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
+    const uint32_t dst = rowbase + ((j ^ ((lane >> 1) & 3)) << 4);
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
   }
   ptx::fence_proxy_async_smem();
@@ -319,6 +376,11 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
   const uint32_t crank = cluster_ctarank();
   const uint32_t rank = crank & 1, lead = crank & ~1u;   // the pair's first CTA issues the MMAs
   const int S = P::kSplit ? cp.split : 1;
+  constexpr int kStages = P::kWide ? WIDE_STAGES : STAGES, kAccs = P::kWide ? 2 : 1;      // accumulators per tile
+  constexpr uint32_t kStageBytes = P::kWide ? WIDE_STAGE_BYTES : STAGE_BYTES;
+  auto a_smem = [&](int s) { return L.base + s * kStageBytes; };
+  auto b_smem = [&](int s) { return L.base + s * kStageBytes + A_STAGE_BYTES; };
+  const int cols0 = P::acc_cols(prm, 0), cols1 = P::kWide ? P::acc_cols(prm, 1) : 0;      // of the tile's accumulators
   const int pair = blockIdx.x / (2 * S), num_pairs = gridDim.x / (2 * S);    // split form: index and number of tiles
   // k-blocks of a tile that this pair multiplies
   auto kb_range = [&](int m_blk, int* kb0, int* kb1) {
@@ -332,7 +394,7 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
     *L.abort_flag() = 0;
     for (int w = 0; w < NUM_THREADS / 32; ++w) *L.warp_state(w) = 0;
     for (int i = 0; i < 8; ++i) L.scratch()[i] = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       // first CTA: its own producer's expect_tx arrival plus the relay's arrival for the second CTA's stage
       ptx::mbar_init(L.full(s), rank == 0 ? 2 : 1);
       ptx::mbar_init(L.empty(s), 1);
@@ -369,18 +431,22 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
     if (lane == 0) {
       int s = 0; uint32_t ph = 0;
       bool ok = true;
+      const uint32_t tx = P::stage_tx(prm);
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         int m_blk, n_blk, kb0, kb1;
         P::tile_coords(prm, tile, &m_blk, &n_blk);
         if (!P::a_ready(prm, m_blk, g)) break;
         kb_range(m_blk, &kb0, &kb1);
         const int a_row = P::a_row(prm, m_blk) + (int)rank * CTA_M;
-        const int b_row = P::b_row(prm, m_blk, n_blk) + (int)rank * CTA_NLOAD;
+        const int b_row = P::b_row(prm, m_blk, n_blk) + (int)rank * (cols0 / 2);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!pair_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
-          ptx::mbar_arrive_expect_tx(L.full(s), STAGE_BYTES);
-          P::load_stage(prm, P::map_a(prm), P::map_b(prm), L.a(s), L.b(s), L.full(s), kb, a_row, b_row, m_blk, n_blk, (int)rank);
-          if (++s == STAGES) { s = 0; ph ^= 1; }
+          ptx::mbar_arrive_expect_tx(L.full(s), tx);
+          P::load_stage(prm, P::map_a(prm), P::map_b(prm), a_smem(s), b_smem(s), L.full(s), kb, a_row, b_row, m_blk, n_blk, (int)rank);
+          if constexpr (P::kWide)
+            P::load_b(prm, P::map_b(prm), b_smem(s) + B_STAGE_BYTES, L.full(s), kb,
+                      P::b_row(prm, m_blk, n_blk) + cols0 + (int)rank * (cols1 / 2), m_blk, n_blk, (int)rank);
+          if (++s == kStages) { s = 0; ph ^= 1; }
         }
       }
       ptx::grid_launch_dependents();       // all loads are on their way: the next kernel's blocks may take their places
@@ -391,33 +457,95 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       int s = 0; uint32_t ph = 0;
       uint32_t acc_ph = 0;          // bit a = phase of accumulator a
       bool ok = true;
-      const uint64_t desc_a0 = P::desc_a0(L.a(0)), desc_b0 = P::desc_b0(L.b(0));
+      const uint64_t desc_a0 = P::desc_a0(a_smem(0)), desc_b0 = P::desc_b0(b_smem(0));
+      // the instruction's N is the width of the accumulator
+      constexpr uint32_t kNoN = ~(0x3Fu << 17);
+      const uint32_t idesc0 = P::kVarCols ? (P::kIdesc & kNoN) | (uint32_t)(cols0 >> 3) << 17 : P::kIdesc;
+      const uint32_t idesc1 = P::kVarCols ? (P::kIdesc & kNoN) | (uint32_t)(cols1 >> 3) << 17 : P::kIdesc;
+      auto wait_acc = [&](int acc) {     // the epilogue warps of both CTAs must have drained it
+        if (!pair_wait(L.tmem_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_MMA_TMEM_EMPTY)) return false;
+        acc_ph ^= 1u << acc;
+        ptx::tc_fence_after();
+        return true;
+      };
+      auto wait_stage = [&](int st, uint32_t parity) {
+        if (!pair_wait(L.full(st), parity, g, ERR_MMA_FULL)) return false;
+        ptx::tc_fence_after();
+        return true;
+      };
+      // one k-block into one accumulator; which = 1: the second one's rows of B.  Descriptors differ only in the
+      // 16-byte-unit start address (low 14 bits; shared memory is < 256 KiB).
+      auto multiply = [&](int st, int acc, int which, bool first) {
+        const uint64_t da = desc_a0 + (uint64_t)((st * kStageBytes) >> 4);
+        const uint64_t db = desc_b0 + (uint64_t)((st * kStageBytes + which * B_STAGE_BYTES) >> 4);
+#pragma unroll
+        for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k)
+          umma2_f16(tmem_base + acc * ACC_COLS, da + (uint64_t)((k * P::kKStepA) >> 4), db + (uint64_t)((k * P::kKStepB) >> 4),
+                    which ? idesc1 : idesc0, (!first || k != 0) ? 1u : 0u);
+      };
       int ord = 0;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++ord) {
-        const int acc = ord & 1;
         int m_blk, n_blk, kb0, kb1;
         P::tile_coords(prm, tile, &m_blk, &n_blk);
         kb_range(m_blk, &kb0, &kb1);
-        // the epilogue warps of both CTAs must have drained this accumulator (two tiles ago)
-        if (!pair_wait(L.tmem_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_MMA_TMEM_EMPTY)) break;
-        acc_ph ^= 1u << acc;
-        ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!pair_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
-          ptx::tc_fence_after();
-          // descriptors differ only in the 16-byte-unit start address (low 14 bits; shared memory is < 256 KiB)
-          const uint64_t da = desc_a0 + (uint64_t)((s * STAGE_BYTES) >> 4);
-          const uint64_t db = desc_b0 + (uint64_t)((s * STAGE_BYTES) >> 4);
+        if constexpr (!P::kWide) {
+          const int acc = ord & 1;
+          if (!wait_acc(acc)) break;                   // drained two tiles ago
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!wait_stage(s, ph)) { ok = false; break; }
+            multiply(s, acc, 0, kb == kb0);
+            umma2_commit_both(L.empty(s), lead);       // stage reusable in both CTAs once these MMAs retire
+            if (++s == kStages) { s = 0; ph ^= 1; }
+          }
+          if (!ok) break;
+          umma2_commit_both(L.tmem_full(acc), lead);
+        } else {
+          // `count` stages into accumulator 0, then into accumulator 1, which hands them back.  The first and the last
+          // k-blocks of a tile go in batches: while accumulator 1 takes its last k-blocks, the epilogue
+          // drains accumulator 0, and while that takes the first ones of the next tile, accumulator 1 is drained.
+          auto batch = [&](int count, bool begin, bool end) {
+            if (begin && !wait_acc(0)) return false;
+            int t = s; uint32_t tph = ph;
+            for (int i = 0; i < count; ++i) {
+              if (!wait_stage(t, tph)) return false;
+              multiply(t, 0, 0, begin && i == 0);
+              if (++t == kStages) { t = 0; tph ^= 1; }
+            }
+            if (end) umma2_commit_both(L.tmem_full(0), lead);
+            if (begin && !wait_acc(1)) return false;
+            for (int i = 0; i < count; ++i) {
+              multiply(s, 1, 1, begin && i == 0);
+              umma2_commit_both(L.empty(s), lead);
+              if (++s == kStages) { s = 0; ph ^= 1; }
+            }
+            if (end) umma2_commit_both(L.tmem_full(1), lead);
+            return true;
+          };
+          // in between, both accumulators take a k-block together: A is read once for the two
+          auto multiply_both = [&](int st) {
+            const uint64_t da = desc_a0 + (uint64_t)((st * kStageBytes) >> 4), db = desc_b0 + (uint64_t)((st * kStageBytes) >> 4);
 #pragma unroll
-          for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k)
-            umma2_f16(d_tmem, da + (uint64_t)((k * P::kKStepA) >> 4), db + (uint64_t)((k * P::kKStepB) >> 4), P::kIdesc,
-                      (kb > kb0 || k != 0) ? 1u : 0u);
-          umma2_commit_both(L.empty(s), lead);       // stage reusable in both CTAs once these MMAs retire
-          if (++s == STAGES) { s = 0; ph ^= 1; }
+            for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k) {
+              const uint64_t a = da + (uint64_t)((k * P::kKStepA) >> 4), b = db + (uint64_t)((k * P::kKStepB) >> 4);
+              umma2_f16_keep_a(tmem_base, a, b, idesc0, 1u);
+              umma2_f16_kept_a(tmem_base + ACC_COLS, a, b + (B_STAGE_BYTES >> 4), idesc1, 1u);
+            }
+          };
+          const int n = kb1 - kb0;
+          if (n <= WIDE_BATCH) {
+            ok = batch(n, true, true);
+          } else {
+            const int last = min(n - WIDE_BATCH, WIDE_BATCH);
+            ok = batch(WIDE_BATCH, true, false);
+            for (int i = n - WIDE_BATCH - last; i > 0 && ok; --i) {
+              if (!wait_stage(s, ph)) { ok = false; break; }
+              multiply_both(s);
+              umma2_commit_both(L.empty(s), lead);
+              if (++s == kStages) { s = 0; ph ^= 1; }
+            }
+            ok = ok && batch(last, false, true);
+          }
         }
-        if (!ok) break;
-        umma2_commit_both(L.tmem_full(acc), lead);
       }
     }
     else if (lane == 0) {
@@ -431,7 +559,7 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!pair_wait(L.full(s), ph, g, ERR_RELAY_FULL)) { ok = false; break; }
           mbar_arrive_cluster(mapa(L.full(s), lead));
-          if (++s == STAGES) { s = 0; ph ^= 1; }
+          if (++s == kStages) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -443,15 +571,17 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
     uint32_t full_ph = 0;           // bit a = phase of accumulator a
     typename P::EpiState st{};
     bool ok = true;
-    int ord = 0;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++ord) {
+    int ord = 0;                    // accumulators before this one: a tile has kAccs of them
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs)
+    for (int part = 0; part < kAccs && ok; ++part, ++ord) {
       const int acc = ord & 1;
+      const int cols = part ? cols1 : cols0;
       Chunk ck;
       P::tile_coords(prm, tile, &ck.m_blk, &ck.n_blk);
       ck.ordinal = ord;
       ck.half = (int)rank;
       ck.row0 = P::a_row(prm, ck.m_blk) + (int)rank * CTA_M + quarter * 32;
-      ck.col0 = ck.n_blk * BN + colhalf * 128;
+      ck.col0 = ck.n_blk * (cols0 + cols1) + part * cols0 + colhalf * 128;
       // the tensor core is busy with this tile: do useful work until the accumulator is ready
       while (!mbar_try_wait_cluster(L.tmem_full(acc), ((full_ph >> acc) & 1))) {
         if (!P::idle_work(prm, ew, lane, g, tile, L.warp_state(warp))) {
@@ -486,11 +616,13 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       }
       if (!P::tile_begin(prm, L, st, ck, ew, lane, g)) { ok = false; break; }
       if constexpr (!P::kGated) {
+        const int left = P::kVarCols ? min(cols - colhalf * 128, 128) : 128;        // columns of this warp, a multiple of 32
+        if (left <= 0) acc_done();
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c * EPI_COLS < left; ++c) {
           float f[64];
           load_acc_chunk(tacc + c * EPI_COLS, f);
-          if (c == 1) acc_done();
+          if ((c + 1) * EPI_COLS >= left) acc_done();
           // the previous chunk's TMA store must have finished reading the staging buffer
           if (lane == 0) ptx::tma_wait_group_read<0>();
           __syncwarp();
@@ -521,7 +653,19 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           if constexpr (P::kStoreAct) P::store_act(prm, cc.row0 + lane, cc.col0, f);
           if constexpr (P::kRaggedCols) {
             if (P::ragged_chunk(prm, cc.col0)) {
-              P::store_ragged(prm, cc.row0 + lane, cc.col0, f);
+              P::store_ragged(prm, cc.row0 + lane, cc.col0, f, left - c * EPI_COLS);
+              continue;
+            }
+          }
+          if constexpr (P::kVarCols) {
+            if (left - c * EPI_COLS < EPI_COLS) {
+              stage_half_chunk(L.epi(ew), lane, f);
+              if (lane == 0) {
+                const CUtensorMap* map; int x, y;
+                P::out_target_half(prm, cc.row0, cc.col0, &map, &x, &y);
+                if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
+                ptx::tma_commit_group();
+              }
               continue;
             }
           }

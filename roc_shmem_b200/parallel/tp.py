@@ -37,8 +37,8 @@ class RowParallelLinear:
         self._launches = 0
         if self.P == 1:
             self.out = torch.empty((self.M, self.N), dtype=dtype, device=dev)
-            self.algorithm = ("tcgen05 GEMM on CTA pairs (cta_group::2, 256x256x64 tiles, 6-stage TMA ring, two TMEM "
-                              "accumulator stages); 1 PE: no collective")
+            self.algorithm = ("tcgen05 GEMM on CTA pairs (cta_group::2, tiles of 256 rows and up to 512 columns, TMA ring, two "
+                              "TMEM accumulators); 1 PE: no collective")
             self._fused = None
         else:
             from ..ops.fused_tp import GemmReduceScatter
