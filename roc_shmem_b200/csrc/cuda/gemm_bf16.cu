@@ -2,7 +2,7 @@
 // K-major (activations, a torch Linear weight) or MN-major (as a gradient product finds it),
 // fp32 accumulation in TMEM, bf16 output through TMA stores (split tiles and a ragged last
 // column: direct stores); CTA pairs (cta_group::2) on tiles of
-// 256 rows and 128 to 512 columns, see gemm_pair.cuh and plan_width.  This is the compute core
+// 256 rows and 128 to 512 columns, see gemm_pair.cuh and pair_plan.h.  This is the compute core
 // that the fused all-gather→GEMM and GEMM→reduce-scatter kernels build on; it has
 // no counterpart in the reference, which contains no GEMM.  Problems with few rows of A
 // take the weight-streaming kernel of gemm_skinny.cuh instead (plan_skinny says when).
@@ -10,6 +10,7 @@
 
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
+#include "pair_plan.h"
 #include "tma_host.h"
 
 using namespace bshmem;
@@ -33,7 +34,7 @@ enum Form { NARROW, WIDE, SPLIT };
 template <bool kAmn, bool kBmn, int kForm>
 struct PlainBf16 : PolicyDefaults {
   using Params = PlainParams;
-  static constexpr bool kSplit = kForm == SPLIT, kWide = kForm == WIDE, kVarCols = !kSplit;
+  static constexpr bool kSplit = kForm == SPLIT, kWide = kForm == WIDE, kVarCols = !kSplit, kHalfChunks = !kSplit;
   static constexpr uint32_t kIdesc = kIdescBf16 | (kAmn ? 1u << 15 : 0u) | (kBmn ? 1u << 16 : 0u);
   static constexpr uint32_t kBlock = 64 * BK_BYTES;           // one 64 (MN) x 64 (K) block
   static constexpr uint32_t kKStepA = kAmn ? 2048 : UMMA_K_BYTES, kKStepB = kBmn ? 2048 : UMMA_K_BYTES;
@@ -89,12 +90,12 @@ struct PlainBf16 : PolicyDefaults {
   }
   static constexpr bool kRaggedCols = kVarCols;
   __device__ static __forceinline__ bool ragged_chunk(const Params& p, int col) { return (p.core.N & 7) && col < p.core.N && col + EPI_COLS > p.core.N; }
-  __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const float (&f)[64], int cols) {
+  __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const uint32_t (&w)[32], int cols) {
     if (row >= p.core.M) return;
-    __nv_bfloat16* dst = p.out + row * p.ldc + col;
+    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out + row * p.ldc + col);
 #pragma unroll
     for (int j = 0; j < 64; ++j)
-      if (j < cols && col + j < p.core.N) dst[j] = __float2bfloat16_rn(f[j]);
+      if (j < cols && col + j < p.core.N) dst[j] = (uint16_t)(w[j / 2] >> 16 * (j & 1));
   }
   // 16 columns of a row: one 32-byte sector, as far as the matrix goes (N need not be a multiple of 8 when B is K-major)
   __device__ static __forceinline__ void store_row16(const Params& p, int row, int col, const float4 (&v)[4]) {
@@ -227,39 +228,6 @@ SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   return {0, false};
 }
 
-// Columns of a tile's one accumulator, or of its two (wide form; see gemm_pair.cuh).  What a launch costs is the number of waves
-// times the width of a tile, as long as the tensor cores are the bound: 1000 x 7168 x 8192 takes 108 us as two waves of 256 columns
-// (112 tiles on 74 pairs), 98 as one of 448 and 95 as one of 416.  Beside that
-//  - a tile of one accumulator reads its A rows for half as many columns.  Per k-block it takes as long as (256 + width) / 2
-//    columns of a wide one (1000 x 7168 x 8192 by 224 columns: 107 us, also two waves), and under the power cap, where an SM's
-//    loads cost clock, 10 % more at the same number of columns (8192 x 8192 x 3584: 367 us, 350 by 512 columns; 8192 x 7168 x 8192:
-//    765, and 710 by 448).  With a few k-blocks this turns round, because a wide tile fills and drains the ring more often
-//    than it streams (7168 x 8192, 848 deep: 89.7 and 93.7 us; 384 deep: 55.6 and 57.6; 4096 x 4096, 744 deep: 26.5 and 25.4);
-//  - MN-major rows of B come in blocks of 64 columns per CTA, and what is loaded beyond the width counts half;
-//  - a wave has a beginning and an end, worth about 8 columns.
-// Over 30 problems of 264 to 8192 rows in the three layouts the choice was within 4 % of the best of ten widths.
-struct Width {
-  int cols[2];
-};
-Width plan_width(int M, int N, int K, int pairs, bool b_mn) {
-  const long long mb = (M + BM - 1) / BM;
-  const double deep = 0.91 + (K + BK - 1) / BK / 160.0, narrow = deep < 1.1 ? deep : 1.1;
-  Width best = {{BN, 0}};
-  double best_cost = 1e30;
-  for (int w = 2 * BN; w >= 128; w -= 32) {
-    if (w > BN && w < 352) continue;                  // two accumulators of less than 160 columns
-    const int c0 = w > BN ? (w + 63) / 64 * 32 : w, c1 = w - c0;
-    const int loaded = b_mn ? (c0 + 127) / 128 * 128 + (c1 + 127) / 128 * 128 : w;
-    const long long tiles = mb * ((N + w - 1) / w), waves = (tiles + pairs - 1) / pairs;
-    const double cost = waves * ((c1 ? 0.5 * (w + loaded) : narrow * 0.5 * (BN + loaded)) + 8);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = {{c0, c1}};
-    }
-  }
-  return best;
-}
-
 // Few tokens: weight-streaming kernel (gemm_skinny.cuh).
 int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, bool w_mn, cudaStream_t st,
                   int dev, unsigned long long timeout_ns, const SkinnyPlan& plan) {
@@ -344,7 +312,7 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
     if (tiles <= g_octs[dev] && kb >= 24) p.core.split = 4;
     else if (tiles <= g_quads[dev] && kb >= 32) p.core.split = 2;
   }
-  const Width w = p.core.split > 1 ? Width{{BN, 0}} : plan_width(M, N, K, pairs, b_mn != 0);
+  const Width w = p.core.split > 1 ? Width{{BN, 0}} : plan_width((M + BM - 1) / BM, N, K, pairs, 32, b_mn != 0);
   const int width = w.cols[0] + w.cols[1];
   p.core.acc_cols[0] = w.cols[0];
   p.core.acc_cols[1] = w.cols[1];

@@ -234,9 +234,9 @@ struct PolicyDefaults {
   // Wide form: a tile takes both accumulators, columns [0, acc_cols(0)) and the acc_cols(1) behind them, and load_b loads the
   // second one's rows of B.
   static constexpr bool kWide = false;
-  // kVarCols: an accumulator may hold fewer than 256 columns (a multiple of 32), and out_target is asked for a 32-column box
-  // where a chunk of 64 does not fit.  The widths of the others are fixed.
-  static constexpr bool kVarCols = false;
+  // kVarCols: acc_cols may be less than 256 (a multiple of 64; with kHalfChunks of 32, and out_target_half is asked for a
+  // 32-column box where a chunk of 64 does not fit; gated of 128), and columns beyond N are not written.
+  static constexpr bool kVarCols = false, kHalfChunks = false;
   template <class Params> __device__ static __forceinline__ int acc_cols(const Params&, int) { return BN; }
   // bytes that the loads of a stage bring into one CTA
   template <class Params> __device__ static __forceinline__ uint32_t stage_tx(const Params&) { return STAGE_BYTES; }
@@ -244,7 +244,7 @@ struct PolicyDefaults {
   // the matching up-projections; the epilogue writes silu(gate) * up, i.e. half as many output columns (the two
   // chunks of a warp make one 32 x 64 output box; out_target gets the OUTPUT column).
   static constexpr bool kGated = false;
-  // Training forms of the gated MLP, on the plain epilogue (the accumulator's columns are stored as they are or replaced):
+  // Training forms of the gated MLP, with kVarCols (the accumulator's columns, rounded to bf16, are stored as they are or replaced):
   // kStoreAct: store_act() additionally gets every chunk (32 gate, 32 up) before it is stored, to write silu(gate) * up.
   // kSwigluBwd: the accumulator is the gradient of the activations; each 32 columns of it become 64 columns of output, the
   // gradients of the matching gate and up pre-activations (swiglu_grad), and out_target gets the output column.
@@ -312,16 +312,25 @@ __device__ __forceinline__ void stage_chunk(uint32_t buf, int lane, const float 
   __syncwarp();
 }
 
-// The first 32 of them, for a store box of 32 columns: four pieces per row, piece j at (j ^ (row / 2 & 3)) under the
-// 64-byte swizzle.
-__device__ __forceinline__ void stage_half_chunk(uint32_t buf, int lane, const float (&f)[64]) {
+// The same for values that are packed already, two to a word.
+__device__ __forceinline__ void stage_packed(uint32_t buf, int lane, const uint32_t (&w)[32]) {
+  const uint32_t rowbase = buf + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t dst = rowbase + ((j ^ (lane & 7)) << 4);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]), "r"(w[4 * j + 3]) : "memory");
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
+// The first 32 columns of them, for a store box of 32: four pieces per row, piece j at (j ^ (row / 2 & 3)) under the 64-byte
+// swizzle.
+__device__ __forceinline__ void stage_packed_half(uint32_t buf, int lane, const uint32_t (&w)[32]) {
   const uint32_t rowbase = buf + lane * 64;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uint32_t w0 = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]), w1 = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
-    const uint32_t w2 = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]), w3 = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
     const uint32_t dst = rowbase + ((j ^ ((lane >> 1) & 3)) << 4);
-    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]), "r"(w[4 * j + 3]) : "memory");
   }
   ptx::fence_proxy_async_smem();
   __syncwarp();
@@ -335,6 +344,18 @@ __device__ __forceinline__ void load_acc_chunk(uint32_t taddr, float (&f)[64]) {
   ptx::tmem_ld_wait();
 #pragma unroll
   for (int i = 0; i < 64; ++i) f[i] = __uint_as_float(v[i >> 5][i & 31]);
+}
+
+// The same, rounded to bf16 and packed.  Volatile: packed before the next columns are read, so that no more than 64 registers
+// hold unpacked ones.
+__device__ __forceinline__ void load_acc_packed(uint32_t taddr, uint32_t (&w)[32]) {
+  uint32_t v[2][32];
+  ptx::tmem_ld_32x32b_x32(taddr, v[0]);
+  ptx::tmem_ld_32x32b_x32(taddr + 32, v[1]);
+  ptx::tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    asm volatile("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(__uint_as_float(v[i >> 4][(2 * i + 1) & 31])), "f"(__uint_as_float(v[i >> 4][(2 * i) & 31])));
 }
 
 // Split form, behind the cluster barrier: this CTA's share of the sum, 16 columns of a row per thread and step.
@@ -615,60 +636,18 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
         break;                             // one tile per cluster; the rest happens behind the cluster barrier
       }
       if (!P::tile_begin(prm, L, st, ck, ew, lane, g)) { ok = false; break; }
-      if constexpr (!P::kGated) {
-        const int left = P::kVarCols ? min(cols - colhalf * 128, 128) : 128;        // columns of this warp, a multiple of 32
-        if (left <= 0) acc_done();
+      if constexpr (!P::kVarCols && !P::kGated) {
 #pragma unroll 1
-        for (int c = 0; c * EPI_COLS < left; ++c) {
+        for (int c = 0; c < 2; ++c) {
           float f[64];
           load_acc_chunk(tacc + c * EPI_COLS, f);
-          if ((c + 1) * EPI_COLS >= left) acc_done();
+          if (c == 1) acc_done();
           // the previous chunk's TMA store must have finished reading the staging buffer
           if (lane == 0) ptx::tma_wait_group_read<0>();
           __syncwarp();
           Chunk cc = ck;
           cc.col0 = ck.col0 + c * EPI_COLS;
-          if constexpr (P::kSwigluBwd) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-              float d[32], o[64];
-#pragma unroll
-              for (int i = 0; i < 32; ++i) d[i] = h == 0 ? f[i] : f[32 + i];
-              P::swiglu_grad(prm, cc.row0 + lane, cc.col0 + 32 * h, d, o);
-              if (h == 1) {                  // the first half's store has read the staging buffer
-                if (lane == 0) ptx::tma_wait_group_read<0>();
-                __syncwarp();
-              }
-              stage_chunk(L.epi(ew), lane, o);
-              if (lane == 0) {
-                const CUtensorMap* map; int x, y;
-                P::out_target(prm, cc.row0, 2 * (cc.col0 + 32 * h), &map, &x, &y);
-                if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
-                ptx::tma_commit_group();
-              }
-            }
-            continue;
-          }
           P::adjust(prm, L, st, cc, f, ew, lane);
-          if constexpr (P::kStoreAct) P::store_act(prm, cc.row0 + lane, cc.col0, f);
-          if constexpr (P::kRaggedCols) {
-            if (P::ragged_chunk(prm, cc.col0)) {
-              P::store_ragged(prm, cc.row0 + lane, cc.col0, f, left - c * EPI_COLS);
-              continue;
-            }
-          }
-          if constexpr (P::kVarCols) {
-            if (left - c * EPI_COLS < EPI_COLS) {
-              stage_half_chunk(L.epi(ew), lane, f);
-              if (lane == 0) {
-                const CUtensorMap* map; int x, y;
-                P::out_target_half(prm, cc.row0, cc.col0, &map, &x, &y);
-                if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
-                ptx::tma_commit_group();
-              }
-              continue;
-            }
-          }
           stage_chunk(L.epi(ew), lane, f);
           if (lane == 0) {
             const CUtensorMap* map; int x, y;
@@ -677,6 +656,91 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
             ptx::tma_commit_group();
           }
         }
+      } else if constexpr (P::kSwigluBwd || P::kStoreAct) {
+        const int left = min(cols - colhalf * 128, 128);        // of this warp, a multiple of 64; may be none
+        if (left <= 0) acc_done();
+#pragma unroll 1
+        for (int c = 0; c * EPI_COLS < left; ++c) {
+          float f[64];
+          load_acc_chunk(tacc + c * EPI_COLS, f);
+          if ((c + 1) * EPI_COLS >= left) acc_done();
+          const int col0 = ck.col0 + c * EPI_COLS;
+          if (col0 >= cp.N) continue;
+          auto store = [&](int col) {                        // the staged 64 columns
+            if (lane != 0) return;
+            const CUtensorMap* map; int x, y;
+            P::out_target(prm, ck.row0, col, &map, &x, &y);
+            if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
+            ptx::tma_commit_group();
+          };
+          if constexpr (P::kStoreAct) {
+            if (lane == 0) ptx::tma_wait_group_read<0>();    // the previous store has read the staging buffer
+            __syncwarp();
+            P::store_act(prm, ck.row0 + lane, col0, f);
+            stage_chunk(L.epi(ew), lane, f);
+            store(col0);
+          } else {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              float d[32], o[64];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) d[i] = h == 0 ? f[i] : f[32 + i];
+              P::swiglu_grad(prm, ck.row0 + lane, col0 + 32 * h, d, o);
+              if (lane == 0) ptx::tma_wait_group_read<0>();
+              __syncwarp();
+              stage_chunk(L.epi(ew), lane, o);
+              store(2 * (col0 + 32 * h));
+            }
+          }
+        }
+      } else if constexpr (!P::kGated) {
+        // In the wide form, where the tensor cores wait for the accumulator, all of the warp's columns are read, rounded and packed
+        // before the first are stored; else 64 at a time.
+        constexpr int kAtOnce = P::kWide ? 2 : 1;
+        const int left = min(cols - colhalf * 128, 128);        // of this warp, a multiple of 32; may be none
+        if (left <= 0) acc_done();
+#pragma unroll 1
+        for (int c0 = 0; c0 * EPI_COLS < left; c0 += kAtOnce) {
+          uint32_t w[kAtOnce][32];
+          if constexpr (P::kWide) {
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u)
+              if (u * EPI_COLS < left) load_acc_packed(tacc + u * EPI_COLS, w[u]);
+            acc_done();
+          } else {
+            float f[64];
+            load_acc_chunk(tacc + c0 * EPI_COLS, f);
+            if ((c0 + 1) * EPI_COLS >= left) acc_done();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) w[0][i] = pack_bf16(f[2 * i], f[2 * i + 1]);
+          }
+#pragma unroll
+          for (int u = 0; u < kAtOnce; ++u) {
+            const int mine = left - (c0 + u) * EPI_COLS, col0 = ck.col0 + (c0 + u) * EPI_COLS;
+            if (mine <= 0 || col0 >= cp.N) continue;
+            if constexpr (P::kRaggedCols) {
+              if (P::ragged_chunk(prm, col0)) {
+                P::store_ragged(prm, ck.row0 + lane, col0, w[u], mine);
+                continue;
+              }
+            }
+            if (lane == 0) ptx::tma_wait_group_read<0>();     // the previous store has read the staging buffer
+            __syncwarp();
+            const CUtensorMap* map; int x, y;
+            if (P::kHalfChunks && mine < EPI_COLS) stage_packed_half(L.epi(ew), lane, w[u]);
+            else stage_packed(L.epi(ew), lane, w[u]);
+            if (lane == 0) {
+              P::out_target(prm, ck.row0, col0, &map, &x, &y);
+              if constexpr (P::kHalfChunks) {
+                if (mine < EPI_COLS) P::out_target_half(prm, ck.row0, col0, &map, &x, &y);
+              }
+              if (map != nullptr) ptx::tma_store_2d(map, L.epi(ew), x, y);
+              ptx::tma_commit_group();
+            }
+          }
+        }
+      } else if (P::kVarCols && (colhalf * 128 >= cols || ck.col0 >= cp.N)) {
+        acc_done();
       } else {
         // the warp's two 64-column chunks (32 gate + 32 up each) make one 64-column output chunk
         if (lane == 0) ptx::tma_wait_group_read<0>();     // the previous tile's store has read the staging buffer

@@ -20,6 +20,7 @@
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
 #include "moe_common.h"
+#include "pair_plan.h"
 #include "tma_host.h"
 
 using namespace bshmem;
@@ -30,6 +31,7 @@ namespace {
 struct GroupedParams {
   CoreParams core;                 // N = output columns of the accumulator, K = full reduction length
   CUtensorMap map_a, map_b, map_c;
+  CUtensorMap map_b2;              // CTA pairs: B rows of a tile's second accumulator
   const int* rows;                 // [G] valid rows per group (rows mode) or null (all `fixed_rows`)
   const int* klen;                 // [G] reduction length per group (ragged-K mode) or null
   int G, fixed_rows;
@@ -159,16 +161,23 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) grouped_gemm_tn_kernel(const _
 
 // ---- the K-major rows mode on CTA pairs ---------------------------------------------------------------------------
 // Same tile schedule (a tile is 256 rows of one group x 256 accumulator columns) and the same parameters; each CTA of
-// the pair loads 128 rows of the A block and 128 rows of the B block, so the tensor maps have 128-row boxes.
+// the pair loads 128 rows of the A block and half of an accumulator's rows of B.  A tile has one accumulator or, in the
+// wide form, two (see gemm_pair.cuh); grouped_width chooses.
 namespace g2 = bshmem::gemm2;
 
 constexpr int kTableGroups = 64;
 
-template <bool kGatedEpi>
+template <bool kGatedEpi, bool kWideTile>
 struct GroupedPair : g2::PolicyDefaults {
   using Params = GroupedParams;
   using Base = Grouped<kGatedEpi>;
-  static constexpr bool kGated = kGatedEpi;
+  static constexpr bool kGated = kGatedEpi, kWide = kWideTile, kVarCols = true;
+  __device__ static __forceinline__ int acc_cols(const Params& p, int a) { return p.core.acc_cols[a]; }
+  __device__ static __forceinline__ int tile_cols(const Params& p) { return p.core.acc_cols[0] + (kWide ? p.core.acc_cols[1] : 0); }
+  __device__ static __forceinline__ uint32_t stage_tx(const Params& p) { return g2::A_STAGE_BYTES + (uint32_t)tile_cols(p) / 2 * g2::BK_BYTES; }
+  __device__ static __forceinline__ void load_b(const Params& p, const CUtensorMap*, uint32_t b_smem, uint32_t bar, int kb, int b_row, int, int, int) {
+    ptx::tma_load_2d(b_smem, &p.map_b2, bar, kb * g2::BK, b_row);
+  }
   __device__ static __forceinline__ const CoreParams& core(const Params& p) { return p.core; }
   __device__ static __forceinline__ const CUtensorMap* map_a(const Params& p) { return &p.map_a; }
   __device__ static __forceinline__ const CUtensorMap* map_b(const Params& p) { return &p.map_b; }
@@ -210,7 +219,7 @@ struct GroupedPair : g2::PolicyDefaults {
   }
   __device__ static __forceinline__ int a_row(const Params&, int m_blk) { return m_blk * g2::BM; }
   __device__ static __forceinline__ int b_row(const Params& p, int m_blk, int n_blk) {
-    return (m_blk / p.a_blocks_per_group) * p.b_rows_per_group + n_blk * g2::BN;
+    return (m_blk / p.a_blocks_per_group) * p.b_rows_per_group + n_blk * tile_cols(p);
   }
   // runs in the producer lane of BOTH CTAs: each loads its own half of the block
   __device__ static __forceinline__ bool a_ready(const Params& p, int, Guard& g) {
@@ -233,11 +242,14 @@ struct GroupedPair : g2::PolicyDefaults {
 
 // Training forward of the gated MLP: C keeps the interleaved gate / up pre-activations for the backward pass, and the
 // activations silu(gate) * up are written in the same epilogue, from the rounded values that C holds (a pass of its own
-// over C reads 2 and writes 1 of the 3 x 940 MB at 32768 rows x 14336: 440 us).  A lane owns a row: 64 consecutive bytes.
-struct GroupedPairAct : GroupedPair<false> {
+// over C reads 2 and writes 1 of the 3 x 940 MB at 32768 rows x 14336: 440 us).
+template <bool kWideTile>
+struct GroupedPairAct : GroupedPair<false, kWideTile> {
+  using Params = GroupedParams;
   static constexpr bool kStoreAct = true;
+  // a lane owns a row: 64 consecutive bytes
   __device__ static __forceinline__ void store_act(const Params& p, int row, int col, const float (&f)[64]) {
-    if (!live(p, row)) return;
+    if (!GroupedPairAct::live(p, row)) return;
     uint4* dst = reinterpret_cast<uint4*>(p.act + row * p.ld_act + col / 2);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -260,7 +272,7 @@ struct GroupedPairAct : GroupedPair<false> {
 // Backward through the activations: the accumulator is d_h = d_y · W2; the epilogue reads the saved pre-activations and
 // writes the gradients of the gate / up pre-activations, so that d_h never goes to memory (written and read again it was
 // 1.9 of the 4.7 GB that the separate pass moved in 700 us).
-struct GroupedPairSwigluBwd : GroupedPair<false> {
+struct GroupedPairSwigluBwd : GroupedPair<false, false> {
   static constexpr bool kSwigluBwd = true;
   __device__ static __forceinline__ void swiglu_grad(const Params& p, int row, int col, const float (&d)[32], float (&o)[64]) {
     const uint4* src = reinterpret_cast<const uint4*>(p.gu + row * p.ld_gu + 2 * col);
@@ -290,7 +302,9 @@ struct GroupedPairSwigluBwd : GroupedPair<false> {
 // Weight-gradient flavour on CTA pairs: both operands MN-major (token-major activations as they are), ragged
 // reduction over the group's tokens.  Per CTA and stage, each operand is two 64-wide MN blocks of 64 tokens (8 KiB per
 // block, 128-byte swizzle), i.e. the CTA's 128 of the tile's 256 rows / columns.
-struct GroupedPairTN : GroupedPair<false> {
+template <bool kWideTile>
+struct GroupedPairTN : GroupedPair<false, kWideTile> {
+  using Params = GroupedParams;
   static constexpr uint32_t kIdesc = ptx::umma_idesc_mn_major(1, 1, g2::BM, g2::BN);
   static constexpr uint32_t kBlock = 64 * g2::BK_BYTES;         // one 64 (MN) x 64 (tokens) block: 8 KiB
   static constexpr uint32_t kKStepA = 2048, kKStepB = 2048;     // one MMA consumes 16 tokens = two swizzle atoms
@@ -311,45 +325,56 @@ struct GroupedPairTN : GroupedPair<false> {
                                                     uint32_t b_smem, uint32_t bar, int kb, int, int, int m_blk, int n_blk, int rank) {
     const int g = m_blk / p.a_blocks_per_group;
     const int tok = g * p.k_rows_per_group + kb * 64;
-    const int m0 = (m_blk - g * p.a_blocks_per_group) * g2::BM + rank * g2::CTA_M, n0 = n_blk * g2::BN + rank * g2::CTA_NLOAD;
-    if (p.tn3d) {                  // one 16 KiB copy per operand: {64, 64 tokens, 2 column blocks}
-      ptx::tma_load_3d(a_smem, ma, bar, 0, tok, m0 / 64);
-      ptx::tma_load_3d(b_smem, mb, bar, 0, tok, n0 / 64);
-      return;
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      ptx::tma_load_2d(a_smem + i * kBlock, ma, bar, m0 + i * 64, tok);
-      ptx::tma_load_2d(b_smem + i * kBlock, mb, bar, n0 + i * 64, tok);
-    }
+    const int m0 = (m_blk - g * p.a_blocks_per_group) * g2::BM + rank * g2::CTA_M;
+    load_columns(p, ma, a_smem, bar, m0, tok);
+    load_columns(p, mb, b_smem, bar, n_blk * GroupedPairTN::tile_cols(p) + rank * (p.core.acc_cols[0] / 2), tok);
+  }
+  // the second accumulator has 256 columns, or 128: the CTA's 64 are then loaded together with the 64 next to them
+  __device__ static __forceinline__ void load_b(const Params& p, const CUtensorMap* mb, uint32_t b_smem, uint32_t bar, int kb, int, int m_blk,
+                                                int n_blk, int rank) {
+    const int tok = m_blk / p.a_blocks_per_group * p.k_rows_per_group + kb * 64;
+    load_columns(p, mb, b_smem, bar, n_blk * GroupedPairTN::tile_cols(p) + p.core.acc_cols[0] + rank * (p.core.acc_cols[1] / 2), tok);
+  }
+  __device__ static __forceinline__ uint32_t stage_tx(const Params&) { return kWideTile ? g2::WIDE_STAGE_BYTES : g2::STAGE_BYTES; }
+  __device__ static __forceinline__ void load_columns(const Params& p, const CUtensorMap* map, uint32_t smem, uint32_t bar, int col, int tok) {
+    if (p.tn3d) return ptx::tma_load_3d(smem, map, bar, 0, tok, col / 64);       // one 16 KiB copy: {64, 64 tokens, 2 column blocks}
+    ptx::tma_load_2d(smem, map, bar, col, tok);
+    ptx::tma_load_2d(smem + kBlock, map, bar, col + 64, tok);
   }
 };
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
-grouped_gemm_pair_kernel(const __grid_constant__ GroupedParams prm) {
+template <bool kWide>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1) grouped_gemm_pair_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  g2::gemm_mainloop<GroupedPair<false>>(prm, smem_raw);
+  g2::gemm_mainloop<GroupedPair<false, kWide>>(prm, smem_raw);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
-grouped_gemm_pair_gated_kernel(const __grid_constant__ GroupedParams prm) {
+template <bool kWide>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1) grouped_gemm_pair_gated_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  g2::gemm_mainloop<GroupedPair<true>>(prm, smem_raw);
+  g2::gemm_mainloop<GroupedPair<true, kWide>>(prm, smem_raw);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
-grouped_gemm_pair_act_kernel(const __grid_constant__ GroupedParams prm) {
+template <bool kWide>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1) grouped_gemm_pair_act_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  g2::gemm_mainloop<GroupedPairAct>(prm, smem_raw);
+  g2::gemm_mainloop<GroupedPairAct<kWide>>(prm, smem_raw);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
-grouped_gemm_pair_swiglu_bwd_kernel(const __grid_constant__ GroupedParams prm) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1) grouped_gemm_pair_swiglu_bwd_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
   g2::gemm_mainloop<GroupedPairSwigluBwd>(prm, smem_raw);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1)
-grouped_gemm_pair_tn_kernel(const __grid_constant__ GroupedParams prm) {
+template <bool kWide>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2::NUM_THREADS, 1) grouped_gemm_pair_tn_kernel(const __grid_constant__ GroupedParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  g2::gemm_mainloop<GroupedPairTN>(prm, smem_raw);
+  g2::gemm_mainloop<GroupedPairTN<kWide>>(prm, smem_raw);
 }
+using PairKernel = void (*)(GroupedParams);
+enum PairForm { ROWS_PLAIN, ROWS_GATED, ROWS_ACT, ROWS_SWIGLU_BWD, PAIR_TN };
+// [form][wide]
+constexpr PairKernel kPairKernels[][2] = {{grouped_gemm_pair_kernel<false>, grouped_gemm_pair_kernel<true>},
+                                          {grouped_gemm_pair_gated_kernel<false>, grouped_gemm_pair_gated_kernel<true>},
+                                          {grouped_gemm_pair_act_kernel<false>, grouped_gemm_pair_act_kernel<true>},
+                                          {grouped_gemm_pair_swiglu_bwd_kernel, nullptr},
+                                          {grouped_gemm_pair_tn_kernel<false>, grouped_gemm_pair_tn_kernel<true>}};
 
 // Few rows per group (decode): weight-streaming tiles, see gemm_skinny.cuh.
 template <bool kGated>
@@ -390,21 +415,30 @@ int ensure(int dev) {
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_swiglu_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
-  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_pair_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
+  for (auto& form : kPairKernels)
+    for (PairKernel k : form)
+      if (k) BSHMEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2::SMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skinny::SMEM_FULL));
-  g_pairs[dev] = g2::max_resident_pairs(grouped_gemm_pair_kernel, g_sms[dev]);
+  g_pairs[dev] = g2::max_resident_pairs(kPairKernels[ROWS_PLAIN][0], g_sms[dev]);
   return 0;
 }
 
-enum RowsForm { ROWS_PLAIN, ROWS_GATED, ROWS_ACT, ROWS_SWIGLU_BWD };
+// Widths for a launch on CTA pairs (plan_width).  The host knows the row blocks exactly where all groups have `fixed` rows;
+// with counts on the device it takes four fifths of a group's capacity for its rows, the share that a layer with the usual
+// capacity factor of 1.25 fills.  In the wide form the epilogue of one accumulator delays that of the other, and the tensor
+// cores wait for both: with the activations in it, some 8000 cycles per tile (32768 x 28672 by 512 columns, 4096 deep: 6.48 ms, by
+// 256: 6.07; 8192 x 7168, 8192 deep, where 448 columns save half a wave: 0.74 against 0.77), with their derivative more
+// (32768 x 14336, 4096 deep: 3.86 against 3.34 ms; 8192 x 3584, 8192 deep: 477 against 444 us).  Groups of one row block stream
+// weights and gain nothing (training step of 1240 tokens, 64 experts of 1024, hidden 2048: 779 us, 791 with wide tiles).
+g2::Width grouped_width(PairForm form, int G, int capacity, bool counted, int N, int K, int pairs) {
+  const long long rows = counted ? (capacity * 4LL + 4) / 5 : capacity;
+  return g2::plan_width(G * ((rows + BM - 1) / BM), N, K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
+                        form == ROWS_SWIGLU_BWD || (counted && rows <= BM) ? BN : 2 * BN, form == ROWS_ACT ? 8000 : 0);
+}
 
 // A launch of the CTA-pair kernels that may overlap the tail of the stream's previous kernel.
-int launch_pairs(void (*kernel)(GroupedParams), const GroupedParams& p, int pairs, cudaStream_t st) {
+int launch_pairs(PairKernel kernel, const GroupedParams& p, int pairs, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs));
   cfg.blockDim = dim3(g2::NUM_THREADS);
@@ -430,7 +464,7 @@ const char* bshmem_moe_gemm_last_error() { return host::last_error().c_str(); }
 //   klen_dev   per-group reduction lengths on the device, or null → K
 //   gated      1: accumulator columns are interleaved gate/up, C gets N/2 columns of silu(gate)*up
 //   arrive/expected/P  optional arrival words to wait for before the first load (P = 0: none)
-static int grouped_gemm_rows(RowsForm form, const void* A, const void* B, void* C, int G, int a_rows_per_group, int b_rows_per_group, int N,
+static int grouped_gemm_rows(PairForm form, const void* A, const void* B, void* C, int G, int a_rows_per_group, int b_rows_per_group, int N,
                              int K, int lda, int ldb, int ldc, const int* rows_dev, int fixed_rows, const int* klen_dev, const void* arrive,
                              const int* expected, int P, void* stream, int timeout_ms, int max_ctas, void* act, int ld_act, const void* gu,
                              int ld_gu) {
@@ -460,21 +494,26 @@ static int grouped_gemm_rows(RowsForm form, const void* A, const void* B, void* 
   if (!pair && (form == ROWS_ACT || form == ROWS_SWIGLU_BWD)) { host::last_error() = "grouped gemm: this form needs CTA pairs"; return 1; }
   p.act = static_cast<__nv_bfloat16*>(act); p.ld_act = ld_act;
   p.gu = static_cast<const __nv_bfloat16*>(gu); p.ld_gu = ld_gu;
-  const int box_rows_a = pair ? g2::CTA_M : BM, box_rows_b = pair ? g2::CTA_NLOAD : BN;
+  int pairs = g_pairs[dev];
+  if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  const g2::Width w = pair ? grouped_width(form, G, rows_dev ? a_rows_per_group : p.fixed_rows, rows_dev != nullptr, N, K, pairs) : g2::Width{{BN, 0}};
+  if (pair) {
+    p.core.acc_cols[0] = w.cols[0]; p.core.acc_cols[1] = w.cols[1];
+    p.core.num_n_blocks = (N + w.cols[0] + w.cols[1] - 1) / (w.cols[0] + w.cols[1]);
+  }
+  const int box_rows_a = pair ? g2::CTA_M : BM, box_rows_b = pair ? w.cols[0] / 2 : BN;
   rc = host::make_tmap_2d(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)G * a_rows_per_group, K, lda, box_rows_a, 64);
   if (rc) return rc;
   rc = host::make_tmap_2d(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, (uint64_t)G * b_rows_per_group, K, ldb, box_rows_b, 64);
+  if (rc) return rc;
+  if (w.cols[1]) rc = host::make_tmap_2d(&p.map_b2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, (uint64_t)G * b_rows_per_group, K, ldb, w.cols[1] / 2, 64);
   if (rc) return rc;
   rc = host::make_tmap_2d(&p.map_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, C, (uint64_t)G * a_rows_per_group,
                           form == ROWS_GATED ? N / 2 : form == ROWS_SWIGLU_BWD ? 2 * N : N, ldc, 32, EPI_COLS);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (pair) {
-    int pairs = g_pairs[dev];
-    if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-    constexpr void (*kernels[])(GroupedParams) = {grouped_gemm_pair_kernel, grouped_gemm_pair_gated_kernel, grouped_gemm_pair_act_kernel,
-                                                  grouped_gemm_pair_swiglu_bwd_kernel};
-    return launch_pairs(kernels[form], p, pairs, st);
+    return launch_pairs(kPairKernels[form][w.cols[1] ? 1 : 0], p, pairs, st);
   } else {
     int ctas = g_sms[dev];
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
@@ -602,6 +641,14 @@ int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int
   // only if the device cannot hold a pair of this kernel
   const bool pair = g_pairs[dev] > 0;
   const uint32_t blocks = pair ? 2 : 4;
+  int pairs = g_pairs[dev];
+  if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  // the reduction is a group's tokens
+  const g2::Width w = pair ? grouped_width(PAIR_TN, G, M, false, N, (int)(cap * 4LL / 5), pairs) : g2::Width{{BN, 0}};
+  if (pair) {
+    p.core.acc_cols[0] = w.cols[0]; p.core.acc_cols[1] = w.cols[1];
+    p.core.num_n_blocks = (N + w.cols[0] + w.cols[1] - 1) / (w.cols[0] + w.cols[1]);
+  }
   // preferred: one 3-D copy per operand and stage; if the driver refuses that view, boxes of 64 MN-elements
   // (128 bytes, the swizzle span) by 64 tokens, one per column block
   static const bool no3d = getenv("B200SHMEM_TN_2D") != nullptr;
@@ -619,9 +666,7 @@ int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (pair) {
-    int pairs = g_pairs[dev];
-    if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-    return launch_pairs(grouped_gemm_pair_tn_kernel, p, pairs, st);
+    return launch_pairs(kPairKernels[PAIR_TN][w.cols[1] ? 1 : 0], p, pairs, st);
   } else {
     int ctas = g_sms[dev];
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;

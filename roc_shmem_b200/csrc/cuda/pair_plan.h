@@ -1,0 +1,48 @@
+// pair_plan.h — how wide the tiles of a CTA-pair GEMM (gemm_pair.cuh) are.  Plain C++.
+#pragma once
+
+namespace bshmem {
+namespace gemm2 {
+
+// Columns of a tile's one accumulator, or of its two (wide form; see gemm_pair.cuh).  What a launch costs is the number of waves
+// times the width of a tile, as long as the tensor cores are the bound: 1000 x 7168 x 8192 takes 108 us as two waves of 256 columns
+// (112 tiles on 74 pairs), 98 as one of 448 and 95 as one of 416.  Beside that
+//  - a tile of one accumulator reads its A rows for half as many columns.  Per k-block it takes as long as (256 + width) / 2
+//    columns of a wide one (1000 x 7168 x 8192 by 224 columns: 107 us, also two waves), and under the power cap, where an SM's
+//    loads cost clock, 10 % more at the same number of columns (8192 x 8192 x 3584: 367 us, 350 by 512 columns; 8192 x 7168 x 8192:
+//    765, and 710 by 448).  With a few k-blocks this turns round, because a wide tile fills and drains the ring more often
+//    than it streams (7168 x 8192, 848 deep: 89.7 and 93.7 us; 384 deep: 55.6 and 57.6; 4096 x 4096, 744 deep: 26.5 and 25.4);
+//  - of an MN-major B two blocks of 64 columns per CTA and accumulator are loaded whatever the width; what lies beyond it counts half;
+//  - the rows of A are a share of a wide tile's loads too, about 26 columns' worth;
+//  - a wave has a beginning and an end, worth about 8 columns.
+// Without `exact`, row_blocks is an estimate, and a launch is taken to lose half a wave (16 groups of about 770 rows, 1024 columns, 2048 and
+// 4096 deep: 155 us for both by 256 columns, 171 by 512).
+// `wide_delay`: cycles that a tile's epilogue keeps the tensor cores waiting in the wide form (two per column and k-block).
+// `step`: what an accumulator's columns are a multiple of, 32 or, where the epilogue wants more, 64 or 128.
+// Over 30 problems of 264 to 8192 rows in the three layouts the choice was within 4 % of the best of ten widths.
+struct Width {
+  int cols[2];
+};
+inline Width plan_width(long long row_blocks, int N, int K, int pairs, int step, bool b_mn, bool exact = true, int widest = 512,
+                        int wide_delay = 0) {
+  constexpr int BN = 256;
+  const double blocks = (K + 63) / 64, narrow = 0.91 + blocks / 160 < 1.1 ? 0.91 + blocks / 160 : 1.1;
+  Width best = {{BN, 0}};
+  double best_cost = 1e30;
+  for (int w = widest; w >= 128; w -= step) {
+    if (w > BN && w < 352) continue;                  // two accumulators of less than 160 columns
+    const int c0 = w > BN ? (w + 2 * step - 1) / (2 * step) * step : w, c1 = w - c0;
+    const int loaded = !b_mn ? w : c1 ? 2 * BN : BN;
+    const long long tiles = row_blocks * ((N + w - 1) / w);
+    const double waves = exact ? (double)((tiles + pairs - 1) / pairs) : tiles > pairs / 2 ? 0.5 + (double)tiles / pairs : 1.0;
+    const double cost = waves * ((c1 ? 26 + 0.95 * 0.5 * (w + loaded) + wide_delay / (2 * blocks) : narrow * 0.5 * (BN + loaded)) + 8);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = {{c0, c1}};
+    }
+  }
+  return best;
+}
+
+}  // namespace gemm2
+}  // namespace bshmem
