@@ -58,3 +58,29 @@ def test_quantiser_row_counts(M):
         if M:
             part = (qa.q[at:at + 3].view(torch.float8_e4m3fn).float() * qa.scales[0, at:at + 3].unsqueeze(1))
             assert torch.allclose(part, x[at:at + 3].float(), rtol=2 ** -4, atol=1e-6)       # e4m3: half a step is 2^-4
+
+
+# 152 and 200 tiles on 148 SMs: four tiles of the last wave on clusters of four and eight, 52 on clusters of two; too few k-blocks
+@pytest.mark.parametrize("M,N,K", [(128 * 38, 1024, 128 * 16), (128 * 38, 1024, 128 * 33), (128 * 25, 2048, 128 * 25), (128 * 25, 2048, 128 * 9)])
+def test_gemm_fp8_last_wave_split(M, N, K):
+    test_gemm_fp8_split_and_plain(M, N, K)
+
+
+def test_gemm_fp8_last_wave_in_a_chain():
+    """What follows a product in the stream waits for all of it: each product's result becomes the next one's activations."""
+    from roc_shmem_b200.ops.gemm_fp8 import fp8_error_site, gemm_fp8, quantize_act, quantize_weight
+    M, N, K = 128 * 38, 1024, 4096
+    torch.manual_seed(1)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w, back = (quantize_weight((torch.randn(*s, device="cuda") * 0.03).to(torch.bfloat16)) for s in ((N, K), (K, N)))
+    first = None
+    for _ in range(5):
+        y = x
+        for _ in range(4):
+            y = gemm_fp8(quantize_act(gemm_fp8(quantize_act(y), w, torch.zeros(M, N, dtype=torch.bfloat16, device="cuda"))), back,
+                         torch.zeros(M, K, dtype=torch.bfloat16, device="cuda"))
+        if first is None:
+            torch.cuda.synchronize()
+            first = y.clone()
+        assert torch.equal(y, first) and bool(torch.isfinite(y.float()).all())
+    assert fp8_error_site() == 0
