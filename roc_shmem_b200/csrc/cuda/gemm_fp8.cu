@@ -840,7 +840,7 @@ int bshmem_gemm_fp8_blockscale(const void* A8, const float* scale_a, const void*
       if (tiles <= g_clusters[dev][i] && K / FBK >= 4 * (2 << i)) { p.split = 2 << i; break; }
   // Whole waves of tiles, then a last wave that is partly empty: its tiles go to a launch of the split form behind this one, if
   // that saves 12 of a CTA's k-blocks (some 6 us; parking and adding the parts takes about 4).  4096 x 7168 x 8192 has 896 tiles for
-  // 148 SMs, 6.05 waves: 262 us became 249 (with the quantiser 292 and 280; the clock under the power cap takes back the rest).
+  // 148 SMs, 6.05 waves: with the quantiser 292 us became 280.
   const int rest = tiles % ctas, kb = K / FBK;
   int rest_split = 1;
   if (max_ctas <= 0 && p.split == 1 && tiles > ctas && rest)
