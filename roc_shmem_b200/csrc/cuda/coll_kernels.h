@@ -69,6 +69,12 @@ struct GroupDone {
 // All PEs of a local group at once: states / teams are device arrays of n entries (a team with my_idx < 0 sits out).
 cudaError_t launch_group(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status,
                          cudaStream_t stream, const GroupDone& done = GroupDone());
+// The same as one thread-block cluster, for at most kClusterBlocks blocks of all PEs together, every one of them a member: the
+// blocks of a cluster run at the same time without a cooperative launch, and synchronise by its barrier.  states / teams are
+// HOST arrays of n entries and travel as kernel parameters.
+constexpr int kClusterBlocks = 8;
+cudaError_t launch_cluster(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status, cudaStream_t stream,
+                           const GroupDone& done);
 // Loads every kernel module now (a lazy first load from another thread could need a device-wide quiet point).
 void preload();
 
@@ -77,6 +83,7 @@ void preload();
   cudaError_t launch_##name(const State&, const DTeam&, const CollArgs&, int, int*, cudaStream_t);                       \
   cudaError_t launch_group_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t,             \
                                   const GroupDone&);                                                                     \
+  cudaError_t launch_cluster_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t, const GroupDone&); \
   void preload_##name();
 BSHMEM_COLL_UNIT(move)
 BSHMEM_COLL_UNIT(f32)

@@ -756,6 +756,16 @@ class GpuBackend final : public Backend {
   // copied and freed per call and a synchronous read of the status, the call cost 40 us around a 16 us kernel.)
   int group_launch(const State* hs, const DTeam* ht, int n, const CollArgs& a, int ctas) {
     std::lock_guard<std::mutex> lock(group_mu_);
+    bool all = true;
+    for (int i = 0; i < n; ++i) all = all && ht[i].my_idx >= 0 && ht[i].size == n;
+    if (all && ctas * n <= collk::kClusterBlocks) {
+      const Ticket t(&lanes_[0]);
+      pinned_->status[t.slot] = 0;
+      collk::GroupDone done;
+      done.word = t.done.word;
+      done.token = t.done.token;
+      return group_wait(t, collk::launch_cluster(hs, ht, a, ctas, n, &pinned_->status[t.slot], stream_, done), "cluster launch: ");
+    }
     if (!group_dev_) {
       // on the stream of the launch: it may be one that does not wait for the default stream
       char* mem = nullptr;
@@ -775,22 +785,23 @@ class GpuBackend final : public Backend {
     }
     GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
     const Ticket t(&lanes_[0]);
-    int* status = &pinned_->status[t.slot];
-    *status = 0;
+    pinned_->status[t.slot] = 0;
     collk::GroupDone done;
     done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
     done.word = t.done.word;
     done.token = t.done.token;
-    cudaError_t e = collk::launch_group(dev->states, dev->teams, a, ctas, n, status, stream_, done);
-    if (e != cudaSuccess) {
+    return group_wait(t, collk::launch_group(dev->states, dev->teams, a, ctas, n, &pinned_->status[t.slot], stream_, done), "cooperative launch: ");
+  }
+  int group_wait(const Ticket& t, cudaError_t launched, const char* what) {
+    if (launched != cudaSuccess) {
       cudaGetLastError();        // reported here, not at somebody's next launch
-      tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e);
+      tl_err = std::string(what) + cudaGetErrorString(launched);
       return BSHMEM_ERR_CUDA;
     }
-    const int rc = wait_done(t, stream_);
-    if (rc != BSHMEM_OK || *status == BSHMEM_OK) return rc;
-    tl_err = std::string("device-side ") + bshmem_status_string(*status);
-    return *status;
+    const int rc = wait_done(t, stream_), status = pinned_->status[t.slot];
+    if (rc != BSHMEM_OK || status == BSHMEM_OK) return rc;
+    tl_err = std::string("device-side ") + bshmem_status_string(status);
+    return status;
   }
 
  private:

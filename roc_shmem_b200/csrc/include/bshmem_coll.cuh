@@ -110,8 +110,22 @@ __device__ __forceinline__ int team_sync_mc(const State& s, const Team& t, int c
   return rc;
 }
 
+// All members' blocks in one cluster (BSHMEM_ONE_CLUSTER): the hardware's barrier, which every block reaches because none of them
+// waits for anything else.  A flag exchange through memory takes 2 us, this 0.3.
+__device__ __forceinline__ int team_sync_cluster(const State& s) {
+  const unsigned long long t0 = s.stats ? dev::timer() : 0;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x == 0 && s.stats) {
+    dev::stat(s, BSHMEM_DSTAT_BARRIER);
+    dev::stat(s, BSHMEM_DSTAT_BARRIER_NS, dev::timer() - t0);
+    dev::trace(s, BSHMEM_TRACE_BARRIER, s.my_pe, dev::timer() - t0);
+  }
+  return BSHMEM_OK;
+}
+
 __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta = 0) {
   if (t.slot < 0) return active_set_sync(s, t);
+  if (s.one_gpu == BSHMEM_ONE_CLUSTER) return team_sync_cluster(s);
   if (t.slot == 0 && t.size == s.n_pes && s.mc_base != nullptr && s.n_pes > 1) return team_sync_mc(s, t, cta);
   __shared__ int sync_status;
   const int tid = threadIdx.x;
@@ -260,6 +274,7 @@ __device__ __forceinline__ void reduce_vec_body(int nsrc, const T* const* srcs, 
 // A stage is 32 KiB whatever the number of sources, so that a source's share is a whole number of 16-byte vectors per
 // thread for up to eight sources and 256 threads (with 48 KiB, 1.5 vectors), and four of them leave three on their way
 // while one is reduced.
+constexpr size_t kBulkMinBytes = 64 * 1024;       // of a block's range
 constexpr int kBulkStages = 4;
 constexpr uint32_t kBulkStageBytes = 32 * 1024;
 // Results leave the same way: parked in one of two buffers of a source's share of a stage, copied to all destinations
@@ -410,7 +425,7 @@ __device__ __forceinline__ void reduce_range_op(const State& s, int nsrc, const 
   }
   size_t v0 = vbeg / VE, v1 = vend / VE;
   // big aligned ranges go through shared memory with bulk async copies when the kernel provides the buffer
-  if (bulk != nullptr && aligned && (v1 - v0) * 16 >= (size_t)64 * 1024 && nsrc <= 16 &&
+  if (bulk != nullptr && aligned && (v1 - v0) * 16 >= kBulkMinBytes && nsrc <= 16 &&
       (OP == BSHMEM_SUM || OP == BSHMEM_MAX || OP == BSHMEM_MIN)) {
     if (reduce_bulk<T, OP>(s, nsrc, srcs, ndst, dsts, vbeg, vend, bulk)) v0 = v1;     // nothing left for the register path
     else return;
@@ -583,8 +598,9 @@ __device__ __forceinline__ int team_reduce_ll(const State& s, const Team& t, int
 template <typename T>
 __device__ __forceinline__ int team_reduce(const State& s, const Team& t, int op, T* dest, const T* source, size_t n,
                                            int cta = 0, int ncta = 1, unsigned long long ll_epoch = 0, char* bulk = nullptr) {
-  // small vectors on the world team: one exchange (the condition is the same on every PE: symmetric addresses)
-  if ((n * sizeof(T)) % (sizeof(T) > 4 ? sizeof(T) : 4) == 0 && n > 0 &&
+  // small vectors on the world team: one exchange (the condition is the same on every PE: symmetric addresses); blocks of one
+  // cluster read each other's vectors at once
+  if (s.one_gpu != BSHMEM_ONE_CLUSTER && (n * sizeof(T)) % (sizeof(T) > 4 ? sizeof(T) : 4) == 0 && n > 0 &&
       ((reinterpret_cast<uintptr_t>(dest) | reinterpret_cast<uintptr_t>(source)) & (sizeof(T) > 4 ? 7 : 3)) == 0) {
     if (t.slot == 0 && t.size == s.n_pes) {
       if (ncta == 1 && n * sizeof(T) <= BSHMEM_LL_PAYLOAD_BYTES) return team_reduce_ll<T>(s, t, op, dest, source, n);
