@@ -1,0 +1,117 @@
+"""Non-blocking messages of a context through its ring (csrc/cuda/gpu_backend.cu, k_ring): sizes around its limit and its 16-byte
+pieces, windows beyond its slots, pauses in which the serving block ends, messages that depend on earlier ones, other operations of the
+same context in between, and several threads."""
+import threading
+import time
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def rt():
+    import roc_shmem_b200 as shmem
+    r = shmem.init("device", rank=0, world_size=1, heap_bytes=256 << 20)
+    yield r
+    shmem.finalize()
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 64, 100, 4096, 16383, 16384, 16385])
+@pytest.mark.parametrize("window", [1, 17, 600])
+def test_windows(rt, n, window):
+    import roc_shmem_b200 as shmem
+    ctx = rt.ctx_create(shmem.CTX_SERIALIZED)
+    sym, src, back = rt.empty((window, n), torch.uint8), torch.randint(0, 256, (window, n), dtype=torch.uint8, device="cuda"), torch.zeros(window, n, dtype=torch.uint8, device="cuda")
+    sym.zero_()
+    torch.cuda.synchronize()
+    for pause in (0, 3e-5):                          # longer than the block waits for a message
+        for i in range(window):
+            ctx.put(sym[i], src[i], 0, nbi=True)
+            if pause and i % 37 == 0:
+                time.sleep(pause)
+        ctx.quiet()
+        assert torch.equal(sym, src)
+        for i in range(window):
+            ctx.get(back[i], sym[i], 0, nbi=True)
+        ctx.quiet()
+        assert torch.equal(back, src)
+        src.add_(1)
+        torch.cuda.synchronize()
+    ctx.destroy()
+
+
+def test_dependent_messages_keep_their_order(rt):
+    """Each message reads what the one before wrote, or overwrites it; a fence orders messages that share nothing."""
+    import roc_shmem_b200 as shmem
+    ctx = rt.ctx_create(shmem.CTX_SERIALIZED)
+    n, steps = 4096, 300
+    sym, a, b = rt.empty((n,), torch.uint8), torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.zeros(n, dtype=torch.uint8, device="cuda")
+    rows = torch.arange(steps, device="cuda").to(torch.uint8).view(-1, 1).repeat(1, n).contiguous()
+    got = torch.zeros_like(rows)
+    torch.cuda.synchronize()
+    for i in range(steps):
+        ctx.put(sym, rows[i], 0, nbi=True)
+        ctx.get(got[i], sym, 0, nbi=True)
+        if i % 50 == 0:
+            ctx.fence()
+    ctx.put(sym, a, 0, nbi=True)
+    ctx.put(sym[8:72], rows[9][8:72], 0, nbi=True)      # into the middle of the one before
+    ctx.get(b, sym, 0, nbi=True)
+    ctx.quiet()
+    assert torch.equal(got, rows)
+    assert bool((b[8:72] == 9).all()) and int(b.sum()) == 9 * 64
+    ctx.destroy()
+
+
+def test_other_operations_follow_the_messages(rt):
+    import roc_shmem_b200 as shmem
+    ctx = rt.ctx_create(shmem.CTX_SERIALIZED)
+    word, big, flag = rt.zeros((4,), torch.int64), rt.zeros((1 << 20,), torch.uint8), rt.zeros((1,), torch.int64)
+    vals = torch.arange(1, 65, dtype=torch.int64, device="cuda")
+    src = torch.full((1 << 20,), 5, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(64):
+        ctx.put(word[:1], vals[i:i + 1], 0, nbi=True)
+        assert rt.atomic_fetch_add(word[:1], 1000, 0, ctx=ctx) == i + 1      # sees the message, and the next message overwrites it
+        ctx.put(word[1:2], vals[i:i + 1], 0, nbi=True)
+        if i % 4 == 0:
+            ctx.put(big, src, 0, nbi=True)                                  # too large for the ring
+        if i % 5 == 0:
+            ctx.put(word[2:3], vals[i:i + 1], 0)                            # blocking
+            assert int(word[2]) == i + 1 and int(word[1]) == i + 1
+        rt.put_signal(word[3:4], vals[i:i + 1], flag, i + 1, 0, ctx=ctx)
+        assert int(flag) == i + 1 and int(word[3]) == i + 1 and int(word[1]) == i + 1
+    ctx.quiet()
+    assert torch.equal(big, src)
+    ctx.destroy()
+
+
+def test_threads(rt):
+    """Three threads, two of them on one context, each with rows of its own."""
+    import roc_shmem_b200 as shmem
+    shared, own = rt.ctx_create(0), rt.ctx_create(0)
+    rows, n, rounds = 40, 256, 25
+    sym = rt.zeros((3, rows, n), torch.uint8)
+    src = torch.randint(0, 256, (3, rounds, rows, n), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(t, ctx):
+        torch.cuda.set_device(0)
+        for r in range(rounds):
+            for i in range(rows):
+                ctx.put(sym[t, i], src[t, r, i], 0, nbi=True)
+            ctx.quiet()
+            if not torch.equal(sym[t], src[t, r]):
+                bad.append((t, r))
+
+    threads = [threading.Thread(target=work, args=(t, c)) for t, c in enumerate((shared, shared, own))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    assert not bad and not any(t.is_alive() for t in threads)
+    shared.destroy()
+    own.destroy()
