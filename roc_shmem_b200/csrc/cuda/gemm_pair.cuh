@@ -25,9 +25,10 @@
 // stages and accumulators back to BOTH CTAs.
 // Wide form (policy with kWide): a tile takes both accumulators, up to 512 columns.  Its A rows are loaded once for all of
 // them, a quarter less traffic from L2 per product, and read once from shared memory: the MMAs of a k-block go to the two
-// accumulators in turn, and the second of each two takes A from the collector buffer.  That is what bounds a long launch,
-// which runs at the clock that the power cap leaves: 8192 x 8192 x 3584 went from 367 to 350 us (1.31 -> 1.38 PFLOP/s).  The epilogue still overlaps the MMAs: at a tile's ends WIDE_BATCH k-blocks go into one
-// accumulator first, then into the other, so that each has the time of a batch to be drained.
+// accumulators in turn, and the second of each two takes A from the collector buffer.  What is moved counts because a long
+// launch runs at the clock that the power cap leaves: 8192 x 8192 x 3584 went from 367 to 350 us (1.31 -> 1.38 PFLOP/s).  The
+// epilogue still overlaps the MMAs: at a tile's ends WIDE_BATCH k-blocks go into one accumulator first, then into the
+// other, so that each has the time of a batch to be drained.
 // Split form (policy with kSplit, for problems with fewer than about half as many tiles as the chip has pairs): the
 // cluster is S = 2 or 4 pairs that share one tile.  Each pair sums its share of K; then every CTA parks its fp32
 // accumulator (128 x 256, 128 KiB) over its drained ring, and after one cluster barrier CTA (pair j, half r) adds the S

@@ -4,7 +4,7 @@
  *   heap_create → export descriptor → (exchange through the bootstrap) → import every
  *   peer → [multicast create/import → add_device → barrier → bind] → gpu_init.
  * For single-GPU tests a "local group" puts all PEs of a job into one process on
- * one device; their collectives run as ONE cooperative launch (group_collective).
+ * one device; their collectives run as ONE launch (group_collective).
  */
 #ifndef BSHMEM_GPU_H_
 #define BSHMEM_GPU_H_
