@@ -210,7 +210,7 @@ __host__ __device__ constexpr uint64_t ring_tag16(uint32_t index) { return (uint
 __host__ __device__ constexpr uint64_t ring_tag32(uint32_t index) { return (uint64_t)(index + 1) << 32; }
 __device__ __forceinline__ void st_host(uint64_t* p, uint64_t v) { asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
 
-__global__ void __launch_bounds__(kRingThreads) k_ring(State s, Ring* ring, uint32_t next, uint32_t generation) {
+__global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next, uint32_t generation) {
   after_predecessor();
   __shared__ struct { char* dst; const char* src; uint32_t n; } msg[kRingBatch];
   __shared__ int found, over;          // messages of the batch; whether the block is to end (1) or has nothing left (2)
@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(State s, Ring* ring, uint
       __syncthreads();
       next += count;
       if (threadIdx.x == 0) {
-        dev::fence_peers(s);
+        // system scope, also on one GPU: a quiet that sees the count ends like a stream synchronisation, for readers on the host too
+        asm volatile("fence.acq_rel.sys;" ::: "memory");
         st_host(&ring->consumed, next);
       }
     }
@@ -540,7 +541,7 @@ class GpuBackend final : public Backend {
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) >> 48) == 0;
   }
   int ring_start(Lane& L, uint32_t from) {
-    RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, state_, L.ring, from, L.generation + 1));
+    RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring, from, L.generation + 1));
     ++L.generation;
     L.serving.store(true, std::memory_order_release);
     return BSHMEM_OK;
