@@ -28,6 +28,7 @@
 #include "../include/bshmem_gpu.h"
 #include "coll_kernels.h"
 #include "gpu_heap.h"
+#include "message_ring.h"
 
 using namespace bshmem;
 using dev::State;
@@ -186,28 +187,9 @@ __global__ void __launch_bounds__(256) k_copy_small(char* dst, const char* src, 
 // block's place.  The host path bounds a window of messages: 64 puts of 64 bytes and a quiet took 177 us by one launch each
 // (2.4 us apart and more), 44 so.  A block with sixteen warps moves a message per warp, 16 KiB in four round trips to memory, as fast as
 // the host writes them.
-//  - A message is three words, two addresses of 48 bits and a size, each beside a part of its number, so that each word says by
-//    itself whether it has arrived (no order of the words is relied upon), and an acquire fence behind them.
-//  - Messages between two fences of the context are unordered, as the API has it, except that one which touches what an
-//    earlier one touches waits for it, as does the first behind a fence (kRingOrdered).
-//  - A block that ends says so first (closed), then looks for messages once more; the host looks at `closed` behind each message
-//    that it has written.  One of the two sees the other, and `final` says how far the block got.  Other operations of the
-//    context tell the block to end (stop) and follow it in the stream.
-struct alignas(32) RingSlot { uint64_t w[4]; };
-constexpr unsigned kRingSlots = 256, kRingThreads = 512, kRingBatch = kRingThreads / 32, kRingMessageMax = 16u << 10;
-constexpr uint32_t kRingOrdered = 1u << 31;
+// message_ring.h has the protocol.
+constexpr unsigned kRingThreads = 512, kRingBatch = kRingThreads / 32;
 constexpr unsigned long long kRingIdleNs = 5000, kRingLifeNs = 100000;
-struct Ring {                          // pinned host memory
-  RingSlot slot[kRingSlots];
-  alignas(64) uint64_t closed;         // by the block: its generation
-  alignas(64) uint64_t final;          // by the block at its end: generation << 32 | messages taken since the ring exists
-  alignas(64) uint64_t consumed;       // by the block: messages done since the ring exists (32 bits)
-  alignas(64) uint64_t stop;           // by the host: generation that is to end
-};
-// What stands beside the words of message `index`: 16 bits for an address (they differ from those of the message that the
-// slot held before), 32 for the size.
-__host__ __device__ constexpr uint64_t ring_tag16(uint32_t index) { return (uint64_t)((index / kRingSlots + 1) & 0xFFFF) << 48; }
-__host__ __device__ constexpr uint64_t ring_tag32(uint32_t index) { return (uint64_t)(index + 1) << 32; }
 __device__ __forceinline__ void st_host(uint64_t* p, uint64_t v) { asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
 
 __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next, uint32_t generation) {
@@ -230,8 +212,7 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next
       if (lane == 31) asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(stop) : "l"(&ring->stop) : "memory");
       stop = __shfl_sync(0xffffffffu, stop, 31);
       const uint64_t low48 = (1ull << 48) - 1;
-      const bool here = lane < kRingBatch && (v0 & ~low48) == ring_tag16(index) && (v1 & ~low48) == ring_tag16(index) &&
-                        (v2 & ~0xFFFFFFFFull) == ring_tag32(index);
+      const bool here = lane < kRingBatch && ring_arrived(v0, v1, v2, index, generation);
       const uint32_t size = (uint32_t)v2;
       const unsigned got = __ballot_sync(0xffffffffu, here), starts = __ballot_sync(0xffffffffu, here && (size & kRingOrdered)) & ~1u;
       int count = __ffs(~got) - 1;
@@ -239,14 +220,14 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next
       if (lane < count) {
         msg[lane].dst = reinterpret_cast<char*>(v0 & low48);
         msg[lane].src = reinterpret_cast<const char*>(v1 & low48);
-        msg[lane].n = size & ~kRingOrdered;
+        msg[lane].n = size & kRingSizeMask;
       }
       if (count) asm volatile("fence.acq_rel.sys;" ::: "memory");   // what the host had seen done before it wrote the message
       if (lane == 0) {
         const unsigned long long now = dev::timer();
         if (count) last = now;
         found = count;
-        over = closing ? (count ? 0 : 2) : stop == generation || now - begun > kRingLifeNs || now - last > kRingIdleNs ? 1 : 0;
+        over = closing ? (count ? 0 : 2) : ring_stopped(stop, generation) || now - begun > kRingLifeNs || now - last > kRingIdleNs ? 1 : 0;
       }
     }
     __syncthreads();
@@ -372,14 +353,7 @@ struct Lane {
   std::atomic<unsigned> next{0};
   std::atomic<bool> taken[kResultSlots] = {};      // slots whose call still waits for its answer
   bool open = false;
-  // the message ring of a context other than the default one, whose stream the caller owns (see k_ring)
-  Ring* ring = nullptr;
-  std::mutex ring_mu;
-  uint32_t head = 0, generation = 0;               // messages written, blocks launched
-  std::atomic<bool> serving{false};                // a block may be taking messages
-  bool order_next = false;
-  struct Span { uintptr_t dst, src; uint32_t n; } recent[16];      // messages since the last ordered one
-  int n_recent = 0;
+  RingWriter ring;                                 // of a context other than the default one, whose stream the caller owns (see k_ring)
 };
 
 // A waiting call's own result slot of its lane, from before the launch until the answer has been read: threads that share the
@@ -485,11 +459,10 @@ class GpuBackend final : public Backend {
     memset(L.pinned, 0, sizeof(Pinned));
     RT_TRY(cudaMalloc(&L.dstatus, sizeof(int)));
     RT_TRY(cudaMemset(L.dstatus, 0, sizeof(int)));
-    RT_TRY(cudaHostAlloc(&L.ring, sizeof(Ring), cudaHostAllocMapped));
-    memset(L.ring, 0, sizeof(Ring));
-    L.head = L.generation = 0;
-    L.order_next = false;
-    L.n_recent = 0;
+    Ring* ring = nullptr;
+    RT_TRY(cudaHostAlloc(&ring, sizeof(Ring), cudaHostAllocMapped));
+    memset(ring, 0, sizeof(Ring));
+    L.ring.open(ring);
     L.open = true;
     return BSHMEM_OK;
   }
@@ -501,7 +474,7 @@ class GpuBackend final : public Backend {
     if (L.stream) { cudaStreamSynchronize(L.stream); cudaStreamDestroy(L.stream); L.stream = nullptr; }
     if (L.pinned) { cudaFreeHost(L.pinned); L.pinned = nullptr; }
     if (L.dstatus) { cudaFree(L.dstatus); L.dstatus = nullptr; }
-    if (L.ring) { cudaFreeHost(L.ring); L.ring = nullptr; }
+    if (L.ring.ring) { cudaFreeHost(L.ring.ring); L.ring.ring = nullptr; }
   }
   void ctx_select(int idx) override { tl_selected_ctx = idx; }
   // Everything the calling thread issues from now on (collectives too) runs on context idx's lane; -1 unbinds.
@@ -522,67 +495,23 @@ class GpuBackend final : public Backend {
   cudaStream_t stream_of(const Lane& L) const { return &L == &lanes_[0] ? stream_ : L.stream; }
 
   // ---- the message ring of a context (see k_ring) ----------------------------------------
-  static uint64_t ring_word(const uint64_t& w) { return reinterpret_cast<const std::atomic<uint64_t>&>(w).load(std::memory_order_acquire); }
-  static uint32_t ring_consumed(const Lane& L) { return (uint32_t)ring_word(L.ring->consumed); }
-  // The lane's stream for anything but a ring message: the block that serves the ring is told to end, and what is enqueued now
-  // follows it.  Every message written so far precedes the word that tells it, so the block takes them all.
+  // The lane's stream for anything but a ring message: it follows the messages written so far.
   cudaStream_t enter(Lane& L) {
-    if (L.serving.load(std::memory_order_acquire)) {
-      std::lock_guard<std::mutex> lock(L.ring_mu);
-      if (L.serving.load(std::memory_order_relaxed)) {
-        reinterpret_cast<std::atomic<uint64_t>&>(L.ring->stop).store(L.generation, std::memory_order_release);
-        L.serving.store(false, std::memory_order_release);
-      }
-    }
+    if (L.ring.ring) L.ring.stop();
     return stream_of(L);
   }
   bool ring_takes(const Lane& L, const void* a, const void* b, uint64_t n, bool nbi) const {
-    return nbi && tl_local_is_device && n > 0 && n <= kRingMessageMax && L.ring && !thread_is_bound() &&
+    return nbi && tl_local_is_device && n > 0 && n <= kRingMessageMax && L.ring.ring && !thread_is_bound() &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) >> 48) == 0;
   }
-  int ring_start(Lane& L, uint32_t from) {
-    RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring, from, L.generation + 1));
-    ++L.generation;
-    L.serving.store(true, std::memory_order_release);
-    return BSHMEM_OK;
-  }
-  // Whether the message has to wait for the ones before it; keeps the list of those that it may run beside.
-  static bool ring_ordered(Lane& L, uintptr_t dst, uintptr_t src, uint32_t n) {
-    auto meet = [](uintptr_t a, uint32_t na, uintptr_t b, uint32_t nb) { return a < b + nb && b < a + na; };
-    bool ordered = L.order_next || L.n_recent == (int)(sizeof(L.recent) / sizeof(L.recent[0]));
-    for (int i = 0; i < L.n_recent && !ordered; ++i) {
-      const Lane::Span& r = L.recent[i];
-      ordered = meet(dst, n, r.dst, r.n) || meet(dst, n, r.src, r.n) || meet(src, n, r.dst, r.n);
-    }
-    if (ordered) L.n_recent = 0;
-    L.order_next = false;
-    L.recent[L.n_recent++] = {dst, src, n};
-    return ordered;
-  }
   int ring_message(Lane& L, char* dst, const char* src, uint32_t n) {
-    std::lock_guard<std::mutex> lock(L.ring_mu);
-    if (L.head - ring_consumed(L) >= kRingSlots) {
-      const int rc = poll([&] { return L.head - ring_consumed(L) < kRingSlots; }, L.stream);      // the block takes all, then ends
-      if (rc != BSHMEM_OK) return rc;
-    }
-    const uint32_t index = L.head++;
-    const uint64_t d = reinterpret_cast<uintptr_t>(dst), s = reinterpret_cast<uintptr_t>(src);
-    auto* w = reinterpret_cast<std::atomic<uint64_t>*>(L.ring->slot[index % kRingSlots].w);
-    w[0].store(ring_tag16(index) | d, std::memory_order_relaxed);
-    w[1].store(ring_tag16(index) | s, std::memory_order_relaxed);
-    w[2].store(ring_tag32(index) | n | (ring_ordered(L, d, s, n) ? kRingOrdered : 0), std::memory_order_release);
-    uint32_t from = index;
-    if (L.serving.load(std::memory_order_relaxed)) {
-      std::atomic_thread_fence(std::memory_order_seq_cst);
-      if (ring_word(L.ring->closed) != L.generation) return BSHMEM_OK;
-      // the block has decided to end: it says how far it got in a moment
-      const int rc = poll([&] { return (uint32_t)(ring_word(L.ring->final) >> 32) == L.generation; }, L.stream);
-      if (rc != BSHMEM_OK) return rc;
-      L.serving.store(false, std::memory_order_release);
-      from = (uint32_t)ring_word(L.ring->final);
-      if (from == L.head) return BSHMEM_OK;
-    }
-    return ring_start(L, from);
+    return L.ring.message(
+        reinterpret_cast<uintptr_t>(dst), reinterpret_cast<uintptr_t>(src), n,
+        [&](uint32_t from, uint32_t generation) -> int {
+          RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
+          return BSHMEM_OK;
+        },
+        [&](auto arrived) { return poll(arrived, L.stream); });
   }
 
   bshmem_error_record_t last_record(bool clear) override {
@@ -732,10 +661,7 @@ class GpuBackend final : public Backend {
   // operations of one stream reach each PE in order; so do ring messages across this
   int fence() override {
     Lane& L = lane();
-    if (L.ring) {
-      std::lock_guard<std::mutex> lock(L.ring_mu);
-      L.order_next = true;
-    }
+    if (L.ring.ring) L.ring.fence();
     return BSHMEM_OK;
   }
   int quiet() override {
@@ -744,12 +670,10 @@ class GpuBackend final : public Backend {
     // host; bshmem_gpu_synchronize() is the explicit host-side wait.
     if (!blocking_now()) return BSHMEM_OK;
     Lane& L = lane();                                     // this context's operations only
-    if (L.serving.load(std::memory_order_acquire)) {
-      // everything enqueued before the block that serves the ring was done when it began
-      uint32_t head;
-      { std::lock_guard<std::mutex> lock(L.ring_mu); head = L.head; }
+    uint32_t head;
+    if (L.ring.ring && L.ring.serving(&head)) {
       for (int i = 0; i < 2000; ++i) {
-        if ((int32_t)(ring_consumed(L) - head) >= 0) return check_device_error("quiet");
+        if (L.ring.done(head)) return check_device_error("quiet");
 #if defined(__x86_64__)
         __builtin_ia32_pause();
 #endif

@@ -88,6 +88,46 @@ def test_other_operations_follow_the_messages(rt):
     ctx.destroy()
 
 
+@pytest.mark.parametrize("kind", ["large", "copy engine", "host buffer", "put_signal", "p"])
+@pytest.mark.parametrize("before,behind", [(1, 1), (1, 40), (64, 300), (0, 700)])
+def test_messages_behind_an_operation_that_nobody_waits_for(rt, kind, before, behind):
+    """Messages, an operation of the stream, a fence, a message into the operation's range and more behind it: after quiet all of it
+    is done, in that order, and nothing is done again once the sources hold something else."""
+    import roc_shmem_b200 as shmem
+    ctx = rt.ctx_create(shmem.CTX_SERIALIZED)
+    n = {"large": 1 << 20, "copy engine": 8 << 20, "host buffer": 1 << 18, "put_signal": 1 << 17, "p": 8}[kind]
+    sym, small, flag = rt.zeros((n,), torch.uint8), rt.zeros((before + behind, 64), torch.uint8), rt.zeros((1,), torch.int64)
+    src = torch.zeros(n, dtype=torch.uint8, device="cpu" if kind == "host buffer" else "cuda")
+    if kind == "host buffer":
+        src = src.pin_memory()
+    msgs, patch = torch.zeros(before + behind, 64, dtype=torch.uint8, device="cuda"), torch.zeros(2, dtype=torch.uint8, device="cuda")
+    for r in range(12):
+        src.fill_(r + 1)
+        msgs.fill_(r + 1)
+        patch.fill_(r + 101)
+        torch.cuda.synchronize()
+        for i in range(before):
+            ctx.put(small[i], msgs[i], 0, nbi=True)
+        if kind == "put_signal":
+            ctx.put_signal(sym, src, flag, r + 1, 0, nbi=True)
+        elif kind == "p":
+            rt.p(sym.view(torch.int64), (r + 1) * 0x0101010101010101, 0, ctx=ctx)
+        else:
+            ctx.put(sym, src, 0, nbi=True)
+        ctx.fence()
+        ctx.put(sym[3:5], patch, 0, nbi=True)
+        for i in range(before, before + behind):
+            ctx.put(small[i], msgs[i], 0, nbi=True)
+        ctx.quiet()
+        for t in (src, msgs, patch):
+            t.fill_(200)
+        torch.cuda.synchronize()
+        if kind == "put_signal":
+            assert int(flag) == r + 1
+        assert int((sym == r + 1).sum()) == n - 2 and bool((sym[3:5] == r + 101).all()) and bool((small == r + 1).all()), r
+    ctx.destroy()
+
+
 def test_threads(rt):
     """Three threads, two of them on one context, each with rows of its own."""
     import roc_shmem_b200 as shmem
