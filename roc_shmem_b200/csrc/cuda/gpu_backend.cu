@@ -495,10 +495,16 @@ class GpuBackend final : public Backend {
   cudaStream_t stream_of(const Lane& L) const { return &L == &lanes_[0] ? stream_ : L.stream; }
 
   // ---- the message ring of a context (see k_ring) ----------------------------------------
-  // The lane's stream for anything but a ring message: it follows the messages written so far.
-  cudaStream_t enter(Lane& L) {
-    if (L.ring.ring) L.ring.stop();
-    return stream_of(L);
+  // The lane's stream for anything but a ring message: it follows the messages written so far.  Messages of other threads wait until
+  // the operation is enqueued: to be called then, before the operation is waited for.
+  struct Entry {
+    cudaStream_t st;
+    std::unique_lock<std::mutex> held;               // of a lane with a ring
+    void enqueued() { if (held) held.unlock(); }
+  };
+  Entry enter(Lane& L) {
+    if (L.ring.ring) return {stream_of(L), L.ring.stop()};
+    return {stream_of(L), {}};
   }
   bool ring_takes(const Lane& L, const void* a, const void* b, uint64_t n, bool nbi) const {
     return nbi && tl_local_is_device && n > 0 && n <= kRingMessageMax && L.ring.ring && !thread_is_bound() &&
@@ -599,25 +605,28 @@ class GpuBackend final : public Backend {
   int put(int pe, uint64_t dst_off, const void* local, uint64_t n, bool nbi) override {
     Lane& L = lane();
     if (ring_takes(L, heap_->base[pe] + dst_off, local, n, nbi)) return ring_message(L, heap_->base[pe] + dst_off, static_cast<const char*>(local), (uint32_t)n);
-    const cudaStream_t st = enter(L);
-    const int rc = move(heap_->base[pe] + dst_off, static_cast<const char*>(local), n, st);
+    Entry e = enter(L);
+    const int rc = move(heap_->base[pe] + dst_off, static_cast<const char*>(local), n, e.st);
+    e.enqueued();
     if (rc != BSHMEM_OK || nbi) return rc;
-    return finish("put", st);
+    return finish("put", e.st);
   }
   int get(int pe, void* local, uint64_t src_off, uint64_t n, bool nbi) override {
     Lane& L = lane();
     if (ring_takes(L, heap_->base[pe] + src_off, local, n, nbi)) return ring_message(L, static_cast<char*>(local), heap_->base[pe] + src_off, (uint32_t)n);
-    const cudaStream_t st = enter(L);
-    const int rc = move(static_cast<char*>(local), heap_->base[pe] + src_off, n, st);
+    Entry e = enter(L);
+    const int rc = move(static_cast<char*>(local), heap_->base[pe] + src_off, n, e.st);
+    e.enqueued();
     if (rc != BSHMEM_OK || nbi) return rc;
-    return finish("get", st);
+    return finish("get", e.st);
   }
   int put_signal(int pe, uint64_t dst_off, const void* local, uint64_t n, uint64_t sig_off, uint64_t sig_val, int sig_op,
                  bool nbi) override {
     Lane& L = lane();
-    const cudaStream_t st = enter(L);
     const bool wait = !nbi && blocking_now();
     const Ticket t(wait ? &L : nullptr);
+    Entry e = enter(L);
+    const cudaStream_t st = e.st;
     if (n == 0 || (tl_local_is_device && n <= kSmallSignalMax)) {
       RT_TRY(launch_small(k_put_signal, 1, n > 4096 ? 512 : 128, st, state_, heap_->base[pe] + dst_off, static_cast<const char*>(local), n,
                                                        reinterpret_cast<uint64_t*>(heap_->base[pe] + sig_off), sig_val, sig_op, t.done));
@@ -626,33 +635,37 @@ class GpuBackend final : public Backend {
       if (rc != BSHMEM_OK) return rc;
       RT_TRY(launch_small(k_signal, 1, 1, st, state_, pe, sig_off, sig_val, sig_op, t.done));
     }
+    e.enqueued();
     if (!wait) return BSHMEM_OK;
     const int rc = wait_done(t, st);
     return rc != BSHMEM_OK ? rc : check_device_error("put_signal");
   }
   int read_word(int pe, uint64_t off, uint64_t size, uint64_t* out) override {
     Lane& L = lane();
-    const cudaStream_t st = enter(L);
     const Ticket t(&L);
-    RT_TRY(launch_small(k_read_word, 1, 1, st, heap_->base[pe] + off, (int)size, t.done));
-    const int rc = wait_result(t, st, out);      // the value is the call's result: it is waited for in stream mode too
+    Entry e = enter(L);
+    RT_TRY(launch_small(k_read_word, 1, 1, e.st, heap_->base[pe] + off, (int)size, t.done));
+    e.enqueued();
+    const int rc = wait_result(t, e.st, out);      // the value is the call's result: it is waited for in stream mode too
     if (rc != BSHMEM_OK) return rc;
     return blocking_now() ? check_device_error("get") : BSHMEM_OK;
   }
   int write_word(int pe, uint64_t off, uint64_t bits, uint64_t size) override {
-    RT_TRY(launch_small(k_write_word, 1, 1, enter(lane()), heap_->base[pe] + off, bits, (int)size));
+    const Entry e = enter(lane());
+    RT_TRY(launch_small(k_write_word, 1, 1, e.st, heap_->base[pe] + off, bits, (int)size));
     return BSHMEM_OK;
   }
   int amo(int pe, uint64_t off, int dtype, int op, uint64_t value, uint64_t cond, uint64_t* fetched) override {
     Lane& L = lane();
-    const cudaStream_t st = enter(L);
     const bool fetching = op <= BSHMEM_AMO_FETCH_CSWAP || op == BSHMEM_AMO_SWAP || (op >= BSHMEM_AMO_FETCH_AND && op <= BSHMEM_AMO_FETCH_XOR);
     const bool wait = fetching || blocking_now();
     const Ticket t(wait ? &L : nullptr);
-    RT_TRY(launch_small(k_amo, 1, 1, st, state_, pe, off, dtype, op, value, cond, t.done));
+    Entry e = enter(L);
+    RT_TRY(launch_small(k_amo, 1, 1, e.st, state_, pe, off, dtype, op, value, cond, t.done));
+    e.enqueued();
     if (wait) {
       uint64_t old = 0;
-      const int rc = wait_result(t, st, &old);
+      const int rc = wait_result(t, e.st, &old);
       if (rc != BSHMEM_OK) return rc;
       if (fetched) *fetched = old;
     }
@@ -679,20 +692,22 @@ class GpuBackend final : public Backend {
 #endif
       }
     }
-    RT_TRY(cudaStreamSynchronize(enter(L)));
+    const cudaStream_t st = enter(L).st;
+    RT_TRY(cudaStreamSynchronize(st));
     return check_device_error("quiet");
   }
   int wait_until(uint64_t off, int dtype, int cmp, uint64_t value, uint64_t timeout_us) override {
     State s = state_;
     s.timeout_ns = timeout_us * 1000ull;
     Lane& L = lane();
-    const cudaStream_t st = enter(L);
     const bool wait = blocking_now();
     const Ticket t(wait ? &L : nullptr);
-    RT_TRY(launch_small(k_wait_until, 1, 1, st, s, off, dtype, cmp, value, t.done));
+    Entry e = enter(L);
+    RT_TRY(launch_small(k_wait_until, 1, 1, e.st, s, off, dtype, cmp, value, t.done));
+    e.enqueued();
     if (!wait) return BSHMEM_OK;
     uint64_t status = 0;
-    int rc = wait_result(t, st, &status);
+    int rc = wait_result(t, e.st, &status);
     if (rc != BSHMEM_OK) return rc;
     rc = (int)(uint32_t)status;
     if (rc != BSHMEM_OK) tl_err = "wait_until: device-side timeout";
@@ -704,11 +719,12 @@ class GpuBackend final : public Backend {
     s.err = nullptr;
     s.stats = nullptr;
     Lane& L = lane();
-    const cudaStream_t st = enter(L);
     const Ticket t(&L);
-    RT_TRY(launch_small(k_wait_until, 1, 1, st, s, off, dtype, cmp, value, t.done));
+    Entry e = enter(L);
+    RT_TRY(launch_small(k_wait_until, 1, 1, e.st, s, off, dtype, cmp, value, t.done));
+    e.enqueued();
     uint64_t status = 0;
-    const int rc = wait_result(t, st, &status);
+    const int rc = wait_result(t, e.st, &status);
     if (rc != BSHMEM_OK) return rc;
     *result = (uint32_t)status == BSHMEM_OK ? 1 : 0;
     return BSHMEM_OK;
@@ -740,7 +756,6 @@ class GpuBackend final : public Backend {
       if (ctas > coll_ctas_) ctas = coll_ctas_;
     }
     Lane& L = coll_lane();
-    const cudaStream_t st = enter(L);
     const bool main_lane = &L == &lanes_[0];   // the slot / staging fast paths count calls per PE, so only the PE stream takes them
     a.ll_epoch = 0;
     const uint64_t unit = bshmem_dtype_size(a.dtype) > 4 ? bshmem_dtype_size(a.dtype) : 4;
@@ -790,7 +805,10 @@ class GpuBackend final : public Backend {
         if (ctas < 1) ctas = 1;
       }
     }
+    Entry e = enter(L);
+    const cudaStream_t st = e.st;
     RT_TRY(collk::launch(state_, team_of(g), a, ctas, L.dstatus, st));
+    e.enqueued();
     if (!blocking_now()) return BSHMEM_OK;
     int rc = 0;
     RT_TRY(cudaMemcpyAsync(&rc, L.dstatus, sizeof(int), cudaMemcpyDeviceToHost, st));

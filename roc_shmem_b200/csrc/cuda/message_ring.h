@@ -62,13 +62,16 @@ class RingWriter {
     serving_ = order_next_ = false;
     n_recent_ = 0;
   }
-  // Before anything but a message is enqueued in the context's stream.  Every message written so far precedes the word that tells
-  // the block to end, so the block takes them all.
-  void stop() {
-    std::lock_guard<std::mutex> lock(mu_);
-    if (!serving_) return;
-    reinterpret_cast<std::atomic<uint64_t>&>(ring->stop).store(generation_, std::memory_order_release);
-    serving_ = false;
+  // Before anything but a message is enqueued in the context's stream, and held until it is there: a block that another thread's
+  // message launched in between would stand before the operation, and what follows would take it to stand behind (serving()).
+  // Every message written so far precedes the word that tells the block to end, so the block takes them all.
+  std::unique_lock<std::mutex> stop() {
+    std::unique_lock<std::mutex> lock(mu_);
+    if (serving_) {
+      reinterpret_cast<std::atomic<uint64_t>&>(ring->stop).store(generation_, std::memory_order_release);
+      serving_ = false;
+    }
+    return lock;
   }
   void fence() {
     std::lock_guard<std::mutex> lock(mu_);

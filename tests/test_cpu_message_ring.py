@@ -110,15 +110,16 @@ struct Context {
                             return 0;
                           });
   }
-  void operation(double t) {
-    writer.stop();
-    stream.enqueue([t] { spin(t); ++operations; });
+  void operation(double t, std::atomic<int>* over = nullptr) {
+    const auto held = writer.stop();
+    spin(3);
+    stream.enqueue([t, over] { spin(t); ++operations; if (over) *over = 1; });
   }
   void quiet() {
     uint32_t head;
     if (writer.serving(&head))
       for (int i = 0; i < 2000; ++i) { if (writer.done(head)) return; std::this_thread::yield(); }
-    writer.stop();
+    (void)writer.stop();
     stream.sync();
   }
 };
@@ -148,7 +149,29 @@ static int windows(int before, int behind, double length, int rounds) {
   return 0;
 }
 
-int main(int, char** a) { return windows(atoi(a[1]), atoi(a[2]), atof(a[3]), atoi(a[4])); }
+// One thread's operations and quiets beside another thread's messages in the same context.
+static int shared(int rounds) {
+  Context c;
+  std::atomic<bool> end{false};
+  std::thread other([&] { for (uint32_t id = 0; !end && id < kMessages; ++id) { c.message(id); spin(3); } });
+  int left = 0;
+  for (int r = 0; r < rounds; ++r) {
+    std::atomic<int> over{0};
+    c.operation(30, &over);
+    c.quiet();
+    if (!over) { ++left; c.stream.sync(); }
+  }
+  end = true;
+  other.join();
+  c.stream.sync();
+  printf("left %d\n", left);
+  return 0;
+}
+
+int main(int n, char** a) {
+  if (n == 2) return shared(atoi(a[1]));
+  return windows(atoi(a[1]), atoi(a[2]), atof(a[3]), atoi(a[4]));
+}
 """
 
 
@@ -168,3 +191,9 @@ def model(tmp_path_factory):
 def test_messages_around_an_operation(model, before, behind, length, rounds):
     r = model(before, behind, length, rounds)
     assert r.returncode == 0 and r.stdout == "early 0 left 0 unordered 0 repeated 0\n", r.stdout + r.stderr
+
+
+def test_two_threads_on_a_context(model):
+    """A quiet covers its own thread's operation, also where another thread's message launched a block meanwhile."""
+    r = model(2000)
+    assert r.returncode == 0 and r.stdout == "left 0\n", r.stdout + r.stderr

@@ -155,3 +155,47 @@ def test_threads(rt):
     assert not bad and not any(t.is_alive() for t in threads)
     shared.destroy()
     own.destroy()
+
+
+def test_quiet_of_one_thread_beside_messages_of_another(rt):
+    """One context: a thread's large puts are done when its quiet returns, whatever blocks another thread's messages launch meanwhile."""
+    ctx = rt.ctx_create(0)
+    n, rounds = 1 << 20, 150
+    big, small = rt.zeros((n,), torch.uint8), rt.zeros((32, 64), torch.uint8)
+    src, msgs = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.randint(0, 256, (32, 64), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    bad, end = [], threading.Event()
+
+    def puts():
+        try:
+            torch.cuda.set_device(0)
+            for r in range(rounds):
+                src.fill_(r % 250 + 1)
+                torch.cuda.current_stream().synchronize()
+                ctx.put(big, src, 0, nbi=True)
+                ctx.quiet()
+                if not bool((big == r % 250 + 1).all()):
+                    bad.append(r)
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+        finally:
+            end.set()
+
+    def messages():
+        try:
+            torch.cuda.set_device(0)
+            while not end.is_set():
+                for i in range(32):
+                    ctx.put(small[i], msgs[i], 0, nbi=True)
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+
+    threads = [threading.Thread(target=f) for f in (puts, messages)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    assert not bad and not any(t.is_alive() for t in threads), bad
+    ctx.quiet()
+    assert torch.equal(small, msgs)
+    ctx.destroy()
