@@ -511,13 +511,15 @@ class GpuBackend final : public Backend {
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) >> 48) == 0;
   }
   int ring_message(Lane& L, char* dst, const char* src, uint32_t n) {
-    return L.ring.message(
+    const int rc = L.ring.message(
         reinterpret_cast<uintptr_t>(dst), reinterpret_cast<uintptr_t>(src), n,
         [&](uint32_t from, uint32_t generation) -> int {
           RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
           return BSHMEM_OK;
         },
         [&](auto arrived) { return poll(arrived, L.stream); });
+    if (rc == BSHMEM_ERR_STATE) tl_err = "the context's messages were not taken";
+    return rc;
   }
 
   bshmem_error_record_t last_record(bool clear) override {

@@ -86,13 +86,14 @@ class RingWriter {
   bool done(uint32_t head) const { return (int32_t)(consumed() - head) >= 0; }
 
   // One message.  start(from, generation) launches a block that serves the ring from message `from` on; wait(arrived) returns when
-  // arrived() or at the end of all blocks launched so far.  Both return a status.
+  // arrived() or at the end of all blocks launched so far.  Both return a status; BSHMEM_ERR_STATE: the blocks have ended without it.
   template <class Start, class Wait>
   int message(uint64_t dst, uint64_t src, uint32_t n, Start start, Wait wait) {
     std::lock_guard<std::mutex> lock(mu_);
     if (head_ - consumed() >= kRingSlots) {
       const int rc = wait([&] { return head_ - consumed() < kRingSlots; });      // the block takes all, then ends
       if (rc != BSHMEM_OK) return rc;
+      if (head_ - consumed() >= kRingSlots) return BSHMEM_ERR_STATE;             // nothing undelivered is written over
     }
     const uint32_t index = head_;
     const uint32_t size = n | (ordered(dst, src, n) ? kRingOrdered : 0);
@@ -109,15 +110,13 @@ class RingWriter {
       const int rc = wait([&] { return (uint32_t)(word(ring->final) >> 32) == generation_; });
       if (rc != BSHMEM_OK) return rc;
       serving_ = false;
-      if ((uint32_t)word(ring->final) == head_) return BSHMEM_OK;
+      const uint64_t final = word(ring->final);
+      if ((uint32_t)(final >> 32) != generation_) return unserved(index, BSHMEM_ERR_STATE);
+      if ((uint32_t)final == head_) return BSHMEM_OK;
       w[2].store(ring_tag32(index) | ring_for(generation_ + 1) | size, std::memory_order_release);
     }
     const int rc = start(index, generation_ + 1);
-    if (rc != BSHMEM_OK) {                           // nobody takes it
-      head_ = index;
-      order_next_ = true;
-      return rc;
-    }
+    if (rc != BSHMEM_OK) return unserved(index, rc);
     ++generation_;
     serving_ = true;
     return BSHMEM_OK;
@@ -126,6 +125,11 @@ class RingWriter {
  private:
   static uint64_t word(const uint64_t& w) { return reinterpret_cast<const std::atomic<uint64_t>&>(w).load(std::memory_order_acquire); }
   uint32_t consumed() const { return (uint32_t)word(ring->consumed); }
+  int unserved(uint32_t index, int rc) {             // nobody takes message `index`
+    head_ = index;
+    order_next_ = true;
+    return rc;
+  }
   // Whether the message has to wait for the ones before it; keeps the list of those that it may run beside.
   bool ordered(uint64_t dst, uint64_t src, uint32_t n) {
     auto meet = [](uint64_t a, uint32_t na, uint64_t b, uint32_t nb) { return a < b + nb && b < a + na; };

@@ -168,7 +168,29 @@ static int shared(int rounds) {
   return 0;
 }
 
+// Nobody takes the messages: an error once the slots are full, and none of them is written over.
+static int full() {
+  Ring ring;
+  memset(&ring, 0, sizeof(ring));
+  RingWriter w;
+  w.open(&ring);
+  int launched = 0, rc = 0;
+  uint32_t sent = 0;
+  auto message = [&] { return w.message(sent, 1ull << 40, 1, [&](uint32_t, uint32_t) { return ++launched, 0; }, [](auto) { return 0; }); };
+  while (sent < 2 * kRingSlots && !(rc = message())) ++sent;
+  Ring before = ring;
+  const int again = message();
+  printf("%u %d %d %d %d\n", sent, launched, rc == BSHMEM_ERR_STATE, again == rc, memcmp(&before, &ring, sizeof(ring)));
+  // the block ended without a word of how far it got
+  ring.closed = 1;
+  ring.consumed = sent;
+  const int lost = message();
+  printf("%d\n", lost == BSHMEM_ERR_STATE);
+  return 0;
+}
+
 int main(int n, char** a) {
+  if (n == 1) return full();
   if (n == 2) return shared(atoi(a[1]));
   return windows(atoi(a[1]), atoi(a[2]), atof(a[3]), atoi(a[4]));
 }
@@ -197,3 +219,8 @@ def test_two_threads_on_a_context(model):
     """A quiet covers its own thread's operation, also where another thread's message launched a block meanwhile."""
     r = model(2000)
     assert r.returncode == 0 and r.stdout == "left 0\n", r.stdout + r.stderr
+
+
+def test_a_ring_that_nobody_empties(model):
+    r = model()
+    assert r.returncode == 0 and r.stdout == "256 1 1 1 0\n1\n", r.stdout + r.stderr
