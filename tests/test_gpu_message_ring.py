@@ -136,23 +136,27 @@ def test_threads(rt):
     sym = rt.zeros((3, rows, n), torch.uint8)
     src = torch.randint(0, 256, (3, rounds, rows, n), dtype=torch.uint8, device="cuda")
     torch.cuda.synchronize()
-    bad = []
+    bad, done = [], []
 
     def work(t, ctx):
-        torch.cuda.set_device(0)
-        for r in range(rounds):
-            for i in range(rows):
-                ctx.put(sym[t, i], src[t, r, i], 0, nbi=True)
-            ctx.quiet()
-            if not torch.equal(sym[t], src[t, r]):
-                bad.append((t, r))
+        try:
+            torch.cuda.set_device(0)
+            for r in range(rounds):
+                for i in range(rows):
+                    ctx.put(sym[t, i], src[t, r, i], 0, nbi=True)
+                ctx.quiet()
+                if not torch.equal(sym[t], src[t, r]):
+                    bad.append((t, r))
+                done.append((t, r))
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
 
     threads = [threading.Thread(target=work, args=(t, c)) for t, c in enumerate((shared, shared, own))]
     for t in threads:
         t.start()
     for t in threads:
         t.join(60)
-    assert not bad and not any(t.is_alive() for t in threads)
+    assert not bad and not any(t.is_alive() for t in threads) and len(done) == 3 * rounds, bad
     shared.destroy()
     own.destroy()
 
