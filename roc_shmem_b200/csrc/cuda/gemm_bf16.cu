@@ -11,6 +11,7 @@
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
 #include "pair_plan.h"
+#include "prefetch_plan.h"
 #include "tma_host.h"
 
 using namespace bshmem;
@@ -245,6 +246,8 @@ int launch_skinny(const void* A, const void* B, void* C, int M, int N, int K, in
   p.tmem_cols = 32;
   while (p.tmem_cols < (uint32_t)p.nt) p.tmem_cols *= 2;
   p.split = plan.split;
+  p.prefetch = skinny::prefetch_blocks(M, 2ll * ldb, (K + skinny::BK - 1) / skinny::BK / plan.split);
+  if (p.prefetch > p.stages) p.prefetch = p.stages;
   const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS;
   int rc = w_mn ? host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, K, N, ldb, skinny::BK, 64)
                 : host::make_tmap_2d(&p.map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, N, K, ldb, skinny::ROWS, skinny::BK);

@@ -52,6 +52,7 @@ struct Params {
   int nt;                        // tokens of the MMA: M rounded up to 16
   int stages;
   int split;                     // CTAs of a cluster that share a tile's reduction (1, 2, 4 or 8)
+  int prefetch;                  // weight blocks a CTA prefetches into L2 (see prefetch_plan.h), at most `stages`
   uint32_t tmem_cols;
   unsigned long long timeout_ns;
   int* err;
@@ -154,10 +155,9 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
     ptx::tmem_relinquish();
   }
   // This CTA's weights start on their way to L2 while the previous kernel of the stream still runs.  They may not be read yet, it could
-  // be writing them, but a prefetch reads nothing.  A ring's worth of blocks: us without / 2 / 4 / a ring / all of them, 16 tokens, 3584 -> 8192: 13.8 13.4 13.1
-  // 13.0 13.1; 4096 -> 4096: 9.9 9.3 8.9 9.0 9.3; 6 tokens, 8192 -> 7168: 22.3 22.1 22.1 21.8 25.7; 193 tokens, 8192 -> 8192: 36.0 35.8 35.9 35.7 42.5.
+  // be writing them, but a prefetch reads nothing.
   if (warp == 2 && lane == 0)
-    for (int kb = kb0; kb < min(kb1, kb0 + p.stages); ++kb) {
+    for (int kb = kb0; kb < min(kb1, kb0 + p.prefetch); ++kb) {
       if constexpr (kWmn) {
         ptx::tma_prefetch_2d(&p.map_w, n0, kb * BK);
         ptx::tma_prefetch_2d(&p.map_w, n0 + 64, kb * BK);
