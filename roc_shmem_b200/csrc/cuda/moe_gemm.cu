@@ -424,16 +424,14 @@ int ensure(int dev) {
   return 0;
 }
 
-// Widths for a launch on CTA pairs (plan_width).  The host knows the row blocks exactly where all groups have `fixed` rows;
-// with counts on the device it takes four fifths of a group's capacity for its rows, the share that a layer with the usual
-// capacity factor of 1.25 fills.  In the wide form the epilogue of one accumulator delays that of the other, and the tensor
+// Widths for a launch on CTA pairs (plan_width).  The host knows the row blocks exactly where all groups have `rows` rows; with
+// counts on the device (`counted`) they are an estimate (group_rows).  In the wide form the epilogue of one accumulator delays that of the other, and the tensor
 // cores wait for both: with the activations in it, some 8000 cycles per tile (32768 x 28672 by 512 columns, 4096 deep: 6.48 ms, by
 // 256: 6.07; 8192 x 7168, 8192 deep, where 448 columns save half a wave: 0.74 against 0.77), with their derivative more
 // (32768 x 14336, 4096 deep: 3.86 against 3.34 ms; 8192 x 3584, 8192 deep: 477 against 444 us).  Groups of one row block stream
 // weights and gain nothing (training step of 1240 tokens, 64 experts of 1024, hidden 2048: 779 us, 791 with wide tiles).
-g2::Width grouped_width(PairForm form, int G, int capacity, bool counted, int N, int K, int pairs) {
-  const long long rows = counted ? (capacity * 4LL + 4) / 5 : capacity;
-  return g2::plan_width(G * ((rows + BM - 1) / BM), N, K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
+g2::Width grouped_width(PairForm form, int G, int rows, bool counted, int N, int K, int pairs) {
+  return g2::plan_width(G * ((rows + BM - 1LL) / BM), N, K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
                         form == ROWS_SWIGLU_BWD || (counted && rows <= BM) ? BN : 2 * BN, form == ROWS_ACT ? 8000 : 0);
 }
 
@@ -460,7 +458,8 @@ extern "C" {
 const char* bshmem_moe_gemm_last_error() { return host::last_error().c_str(); }
 
 // Grouped GEMM.  A: [G * a_rows_per_group, K] (lda), B: [G * b_rows_per_group, K] (ldb), C: [G * a_rows_per_group, N_out] (ldc).
-//   rows_dev   per-group valid row counts on the device, or null → every group has `fixed_rows` rows
+//   rows_dev   per-group valid row counts on the device (`fixed_rows`: about how many they are, 0 → not known; any counts are right), or
+//              null → every group has `fixed_rows` rows
 //   klen_dev   per-group reduction lengths on the device, or null → K
 //   gated      1: accumulator columns are interleaved gate/up, C gets N/2 columns of silu(gate)*up
 //   arrive/expected/P  optional arrival words to wait for before the first load (P = 0: none)
@@ -496,7 +495,7 @@ static int grouped_gemm_rows(PairForm form, const void* A, const void* B, void* 
   p.gu = static_cast<const __nv_bfloat16*>(gu); p.ld_gu = ld_gu;
   int pairs = g_pairs[dev];
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-  const g2::Width w = pair ? grouped_width(form, G, rows_dev ? a_rows_per_group : p.fixed_rows, rows_dev != nullptr, N, K, pairs) : g2::Width{{BN, 0}};
+  const g2::Width w = pair ? grouped_width(form, G, rows_dev ? g2::group_rows(a_rows_per_group, fixed_rows) : p.fixed_rows, rows_dev != nullptr, N, K, pairs) : g2::Width{{BN, 0}};
   if (pair) {
     p.core.acc_cols[0] = w.cols[0]; p.core.acc_cols[1] = w.cols[1];
     p.core.num_n_blocks = (N + w.cols[0] + w.cols[1] - 1) / (w.cols[0] + w.cols[1]);
@@ -535,9 +534,9 @@ int bshmem_moe_grouped_gemm(const void* A, const void* B, void* C, int G, int a_
 // [.., N / 2] (ld_act % 8 == 0) gets silu(gate) * up.
 int bshmem_moe_grouped_gemm_act(const void* A, const void* B, void* C, void* act, int G, int a_rows_per_group, int N, int K, int lda, int ldb,
                                 int ldc, int ld_act, const int* rows_dev, const void* arrive, const int* expected, int P, void* stream,
-                                int timeout_ms) {
+                                int timeout_ms, int about_rows) {
   if (!act || ld_act % 8) { host::last_error() = "grouped gemm (act): needs an activation buffer, leading dimension % 8 == 0"; return 1; }
-  return grouped_gemm_rows(ROWS_ACT, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, 0, nullptr, arrive, expected, P, stream,
+  return grouped_gemm_rows(ROWS_ACT, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, rows_dev ? about_rows : 0, nullptr, arrive, expected, P, stream,
                            timeout_ms, 0, act, ld_act, nullptr, 0);
 }
 
@@ -545,9 +544,9 @@ int bshmem_moe_grouped_gemm_act(const void* A, const void* B, void* C, void* act
 // [.., 2 N] (ld_gu % 8 == 0); C [.., 2 N] gets their gradients.
 int bshmem_moe_grouped_gemm_swiglu_bwd(const void* A, const void* B, const void* gu, void* C, int G, int a_rows_per_group, int N, int K,
                                        int lda, int ldb, int ld_gu, int ldc, const int* rows_dev, const void* arrive, const int* expected,
-                                       int P, void* stream, int timeout_ms) {
+                                       int P, void* stream, int timeout_ms, int about_rows) {
   if (!gu || ld_gu % 8) { host::last_error() = "grouped gemm (swiglu): needs the pre-activations, leading dimension % 8 == 0"; return 1; }
-  return grouped_gemm_rows(ROWS_SWIGLU_BWD, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, 0, nullptr, arrive, expected, P,
+  return grouped_gemm_rows(ROWS_SWIGLU_BWD, A, B, C, G, a_rows_per_group, N, N, K, lda, ldb, ldc, rows_dev, rows_dev ? about_rows : 0, nullptr, arrive, expected, P,
                            stream, timeout_ms, 0, nullptr, 0, gu, ld_gu);
 }
 
@@ -615,9 +614,9 @@ int bshmem_moe_grouped_gemm_few(const void* A, const void* B, void* C, int G, in
 
 // Weight-gradient GEMM on token-major operands: C_g[M, N] = A_g^T · B_g for every group.
 //   A: [G * cap, M] (lda), B: [G * cap, N] (ldb), C: [G * M, N] (ldc); the number of tokens of group g is
-//   klen_dev[g] (<= cap).  Token rows [klen, next multiple of 64) must be zero in A and B.
+//   klen_dev[g] (<= cap; about_len: about how many they are, 0: not known).  Token rows [klen, next multiple of 64) must be zero in A and B.
 int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int cap, int M, int N, int lda, int ldb, int ldc,
-                               const int* klen_dev, void* stream, int timeout_ms, int max_ctas) {
+                               const int* klen_dev, void* stream, int timeout_ms, int max_ctas, int about_len) {
   if (G < 1 || M % BM || N % BN || cap % 64 || lda % 8 || ldb % 8 || ldc % 8 || !klen_dev) {
     host::last_error() = "grouped gemm (transposed operands): needs M % 256 == 0, N % 256 == 0, capacity % 64 == 0, leading dimensions % 8 == 0";
     return 1;
@@ -644,7 +643,7 @@ int bshmem_moe_grouped_gemm_tn(const void* A, const void* B, void* C, int G, int
   int pairs = g_pairs[dev];
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   // the reduction is a group's tokens
-  const g2::Width w = pair ? grouped_width(PAIR_TN, G, M, false, N, (int)(cap * 4LL / 5), pairs) : g2::Width{{BN, 0}};
+  const g2::Width w = pair ? grouped_width(PAIR_TN, G, M, false, N, g2::group_rows(cap, about_len), pairs) : g2::Width{{BN, 0}};
   if (pair) {
     p.core.acc_cols[0] = w.cols[0]; p.core.acc_cols[1] = w.cols[1];
     p.core.num_n_blocks = (N + w.cols[0] + w.cols[1] - 1) / (w.cols[0] + w.cols[1]);

@@ -44,5 +44,13 @@ inline Width plan_width(long long row_blocks, int N, int K, int pairs, int step,
   return best;
 }
 
+// Rows of a group whose count is on the device, as far as the host knows: about `about`, as the caller says, else four fifths of its
+// capacity, the share that a layer with the usual capacity factor of 1.25 fills.  A layer built for 16384 tokens that gets 1717 (16
+// experts of 2048, hidden 1024, two per token: 215 rows for a capacity of 2560) was planned as eight full row blocks per expert
+// and took 85.3 us, 78.4 by the widths for one.
+inline int group_rows(int capacity, int about) {
+  return about > 0 ? (about < capacity ? about : capacity) : (int)((capacity * 4LL + 4) / 5);
+}
+
 }  // namespace gemm2
 }  // namespace bshmem

@@ -65,10 +65,10 @@ def moe_lib() -> C.CDLL:
         f("bshmem_moe_swiglu_bwd", VP, VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_transpose_pad", VP, VP, I, I, I, VP, VP)
         f("bshmem_moe_grouped_gemm", VP, VP, VP, I, I, I, I, I, I, I, I, VP, I, VP, I, VP, VP, I, VP, I, I)
-        f("bshmem_moe_grouped_gemm_act", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I)
-        f("bshmem_moe_grouped_gemm_swiglu_bwd", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I)
+        f("bshmem_moe_grouped_gemm_act", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I, I)
+        f("bshmem_moe_grouped_gemm_swiglu_bwd", VP, VP, VP, VP, I, I, I, I, I, I, I, I, VP, VP, VP, I, VP, I, I)
         f("bshmem_moe_grouped_gemm_few", VP, VP, VP, I, I, I, I, I, I, I, VP, I, I, I, VP, VP, I, VP, I)
-        f("bshmem_moe_grouped_gemm_tn", VP, VP, VP, I, I, I, I, I, I, I, VP, VP, I, I)
+        f("bshmem_moe_grouped_gemm_tn", VP, VP, VP, I, I, I, I, I, I, I, VP, VP, I, I, I)
         f("bshmem_moe_zero_pad_rows", VP, I, VP, I, VP, I, VP, I, VP, I, I, VP)
         f("bshmem_moe_gemm_error_site", I)
         f("bshmem_moe_gemm_error_word", res=VP)
@@ -103,11 +103,12 @@ def interleave_gate_up(w1: torch.Tensor, w3: torch.Tensor) -> torch.Tensor:
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: int, *, rows: Optional[torch.Tensor] = None,
                  fixed_rows: int = 0, klen: Optional[torch.Tensor] = None, gated: bool = False, arrive=None, expected=None,
-                 n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0, few: Optional[tuple] = None) -> None:
+                 n_arrive: int = 0, timeout_ms: int = 4000, max_ctas: int = 0, few: Optional[tuple] = None, about_rows: int = 0) -> None:
     """out_g = a_g @ b_g.T per group on the tcgen05 grouped kernel.  a: [G*Ra, K], b: [G*Rb, K], out: [G*Ra, N or N/2].
     `few` = (most rows of a group, most groups with rows): the caller expects about 100 rows per group or less; the
     weight-streaming form takes such problems.  The two numbers set its launch shape; a call whose counts exceed them is
-    slower and as right."""
+    slower and as right.  `about_rows`: about how many rows a group has, where `rows` says it on the device only (0: not
+    known); it sets the width of the tiles, and any counts are right."""
     G = groups
     ra, rb = a.shape[0] // G, b.shape[0] // G
     if few is not None and rows is not None and G <= 64:
@@ -118,7 +119,7 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: in
             raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
         return
     st = _fast.grouped_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, ra, rb, rb, a.shape[1], a.stride(0), b.stride(0), out.stride(0),
-                            _p(rows), fixed_rows, _p(klen), 1 if gated else 0, arrive, _p(expected), n_arrive, _stream(), timeout_ms,
+                            _p(rows), about_rows if rows is not None else fixed_rows, _p(klen), 1 if gated else 0, arrive, _p(expected), n_arrive, _stream(), timeout_ms,
                             max_ctas)
     if st != 0:
         raise RuntimeError(f"grouped gemm failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
@@ -132,7 +133,8 @@ def _check_matrices(what: str, **matrices) -> None:
 
 
 def grouped_gemm_act(a: torch.Tensor, b: torch.Tensor, gu: torch.Tensor, act: torch.Tensor, groups: int, *,
-                     rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0, timeout_ms: int = 4000) -> None:
+                     rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0, timeout_ms: int = 4000,
+                     about_rows: int = 0) -> None:
     """Training forward of the gated MLP in one kernel: gu_g = a_g @ b_g.T (interleaved gate / up pre-activations, kept for
     the backward pass) and act_g = silu(gate) * up.  a: [G*R, K], b: [G*N, K], gu: [G*R, N], act: [G*R, N/2]."""
     G = groups
@@ -140,14 +142,14 @@ def grouped_gemm_act(a: torch.Tensor, b: torch.Tensor, gu: torch.Tensor, act: to
     _check_matrices("grouped_gemm_act", a=(a, R, K), b=(b, G * N, K), gu=(gu, R, N), act=(act, R, N // 2))
     st = _fast.grouped_gemm_act(a.data_ptr(), b.data_ptr(), gu.data_ptr(), act.data_ptr(), G, a.shape[0] // G, b.shape[0] // G, a.shape[1],
                                 a.stride(0), b.stride(0), gu.stride(0), act.stride(0), _p(rows), arrive, _p(expected), n_arrive, _stream(),
-                                timeout_ms)
+                                timeout_ms, about_rows)
     if st != 0:
         raise RuntimeError(f"grouped gemm (act) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 def grouped_gemm_swiglu_bwd(dy: torch.Tensor, w2_t: torch.Tensor, gu: torch.Tensor, dgu: torch.Tensor, groups: int, *,
                             rows: Optional[torch.Tensor] = None, arrive=None, expected=None, n_arrive: int = 0,
-                            timeout_ms: int = 4000) -> None:
+                            timeout_ms: int = 4000, about_rows: int = 0) -> None:
     """d_gu_g = SwiGLU backward of (dy_g @ w2_t_g.T) at the pre-activations gu_g, in one kernel: the gradient of the
     activations never goes to memory.  dy: [G*R, K], w2_t: [G*N, K], gu and dgu: [G*R, 2N] (interleaved)."""
     G = groups
@@ -155,20 +157,20 @@ def grouped_gemm_swiglu_bwd(dy: torch.Tensor, w2_t: torch.Tensor, gu: torch.Tens
     _check_matrices("grouped_gemm_swiglu_bwd", dy=(dy, R, K), w2_t=(w2_t, G * N, K), gu=(gu, R, 2 * N), dgu=(dgu, R, 2 * N))
     st = _fast.grouped_gemm_swiglu_bwd(dy.data_ptr(), w2_t.data_ptr(), gu.data_ptr(), dgu.data_ptr(), G, dy.shape[0] // G,
                                        w2_t.shape[0] // G, dy.shape[1], dy.stride(0), w2_t.stride(0), gu.stride(0), dgu.stride(0), _p(rows),
-                                       arrive, _p(expected), n_arrive, _stream(), timeout_ms)
+                                       arrive, _p(expected), n_arrive, _stream(), timeout_ms, about_rows)
     if st != 0:
         raise RuntimeError(f"grouped gemm (swiglu) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
 
 def grouped_gemm_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, groups: int, counts: torch.Tensor, *,
-                    timeout_ms: int = 4000, max_ctas: int = 0) -> None:
+                    timeout_ms: int = 4000, max_ctas: int = 0, about_rows: int = 0) -> None:
     """out_g[M, N] = a_g.T @ b_g per group with token-major operands a: [G*cap, M], b: [G*cap, N] and
     `counts[g]` tokens per group; both operands go to the tensor core MN-major, no transpose is materialised.
-    Token rows [counts[g], next multiple of 64) of a and b must be zero (see zero_pad_rows)."""
+    Token rows [counts[g], next multiple of 64) of a and b must be zero (see zero_pad_rows).  `about_rows` as in grouped_gemm."""
     G = groups
     cap = a.shape[0] // G
     st = _fast.grouped_gemm_tn(a.data_ptr(), b.data_ptr(), out.data_ptr(), G, cap, a.shape[1], b.shape[1], a.stride(0), b.stride(0),
-                               out.stride(0), counts.data_ptr(), _stream(), timeout_ms, max_ctas)
+                               out.stride(0), counts.data_ptr(), _stream(), timeout_ms, max_ctas, about_rows)
     if st != 0:
         raise RuntimeError(f"grouped gemm (tn) failed ({st}): {moe_lib().bshmem_moe_gemm_last_error().decode()}")
 
@@ -332,6 +334,7 @@ class MoELayer:
             return bounds if P * n_entries <= limit * self.E else None
 
         few_up, few_down = few(2 * F), few(H)
+        about = max(1, P * n_entries // self.E)                    # rows of an expert
         self.route(x)
         par = self.parity
         if local:
@@ -345,18 +348,19 @@ class MoELayer:
         if self.training:
             if few_up is None:
                 grouped_gemm_act(self.recv, self.w13.view(G * 2 * F, H), self.gu, self.hact, G, rows=self.recv_count,
-                                 timeout_ms=self.timeout_ms, **wait)
+                                 timeout_ms=self.timeout_ms, about_rows=about, **wait)
             else:
                 grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.gu, G, rows=self.recv_count, timeout_ms=self.timeout_ms,
-                             few=few_up, **wait)
+                             few=few_up, about_rows=about, **wait)
                 self._chk(_fast.swiglu_fwd(a["gu"], a["recv_count"], G, cap, F, a["hact"], s), "swiglu")
             self._x_in = x                                         # the router's backward needs the layer input
             self._few_h, self._few_x = few(F), few_down
         else:
             grouped_gemm(self.recv, self.w13.view(G * 2 * F, H), self.hact, G, rows=self.recv_count, gated=True,
-                         timeout_ms=self.timeout_ms, few=few_up, **wait)
+                         timeout_ms=self.timeout_ms, few=few_up, about_rows=about, **wait)
         self.launches += 1
-        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms, few=few_down)
+        grouped_gemm(self.hact, self.w2.view(G * H, F), self.yexp, G, rows=self.recv_count, timeout_ms=self.timeout_ms, few=few_down,
+                     about_rows=about)
         self.launches += 1
         if local:
             self._chk(_fast.combine_local(self._plan_a, a["yexp"], a["topk_w"], a["topk_idx"], a["pos"], T, self.topk, H, a["out"], 0, s),
@@ -381,6 +385,7 @@ class MoELayer:
         par = self.parity
         rc = self.recv_count
         dy = self.recv_bwd
+        about = max(1, P * n_entries // self.E)                    # rows of an expert
         if local:
             # w * d_out into the experts' gradient buffers, and in the same pass the gradients of the routing weights and of
             # the chosen experts' logits
@@ -403,14 +408,16 @@ class MoELayer:
             wait = dict(arrive=self._sig_ptr(par, SIG_BWD_DISPATCH), expected=self.expect_from, n_arrive=P)
         # d_hact = d_y · W2 (B operand = W2^T [F, H], K = H) and through SwiGLU to d_gu
         if self._few_h is None:
-            grouped_gemm_swiglu_bwd(dy, self.w2_t.view(G * F, H), self.gu, self.dgu, G, rows=rc, timeout_ms=self.timeout_ms, **wait)
+            grouped_gemm_swiglu_bwd(dy, self.w2_t.view(G * F, H), self.gu, self.dgu, G, rows=rc, timeout_ms=self.timeout_ms,
+                                    about_rows=about, **wait)
         else:
-            grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_h, **wait)
+            grouped_gemm(dy, self.w2_t.view(G * F, H), self.dh, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_h,
+                         about_rows=about, **wait)
             self._chk(_fast.swiglu_bwd(a["gu"], a["dh"], rc.data_ptr(), G, cap, F, a["dgu"], s), "swiglu bwd")
         # dW2 = d_y^T · hact: token-major operands straight into the MN-major tensor-core path
         if self.tn_gemm:
             zero_pad_rows((dy, self.hact, self.dgu, self.xsave), G, rc)
-            grouped_gemm_tn(dy, self.hact, self.dw2.view(G * H, F), G, rc, timeout_ms=self.timeout_ms)
+            grouped_gemm_tn(dy, self.hact, self.dw2.view(G * H, F), G, rc, timeout_ms=self.timeout_ms, about_rows=about)
         else:                          # explicit transposes + ragged-K K-major GEMM
             ta = self.t_a[: G * H * cap].view(G * H, cap)
             tb = self.t_b[: G * F * cap].view(G * F, cap)
@@ -419,14 +426,15 @@ class MoELayer:
             grouped_gemm(ta, tb, self.dw2.view(G * H, F), G, fixed_rows=H, klen=rc, timeout_ms=self.timeout_ms)
         # dW13 = d_gu^T · x and d_x = d_gu · W13
         if self.tn_gemm:
-            grouped_gemm_tn(self.dgu, self.xsave, self.dw13.view(G * 2 * F, H), G, rc, timeout_ms=self.timeout_ms)
+            grouped_gemm_tn(self.dgu, self.xsave, self.dw13.view(G * 2 * F, H), G, rc, timeout_ms=self.timeout_ms, about_rows=about)
         else:
             ta2 = self.t_a[: G * 2 * F * cap].view(G * 2 * F, cap)
             tb2 = self.t_b[: G * H * cap].view(G * H, cap)
             self._chk(_fast.transpose_pad(a["dgu"], rc.data_ptr(), G, cap, 2 * F, ta2.data_ptr(), s), "transpose")
             self._chk(_fast.transpose_pad(self.xsave.data_ptr(), rc.data_ptr(), G, cap, H, tb2.data_ptr(), s), "transpose")
             grouped_gemm(ta2, tb2, self.dw13.view(G * 2 * F, H), G, fixed_rows=2 * F, klen=rc, timeout_ms=self.timeout_ms)
-        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_x)
+        grouped_gemm(self.dgu, self.w13_t.view(G * H, 2 * F), self.dxe, G, rows=rc, timeout_ms=self.timeout_ms, few=self._few_x,
+                     about_rows=about)
         self.launches += 4
         if local:
             # d_x = sum over k of the experts' rows + the router path (d_logits · Wr), written once
