@@ -430,9 +430,12 @@ int ensure(int dev) {
 // 256: 6.07; 8192 x 7168, 8192 deep, where 448 columns save half a wave: 0.74 against 0.77), with their derivative more
 // (32768 x 14336, 4096 deep: 3.86 against 3.34 ms; 8192 x 3584, 8192 deep: 477 against 444 us).  Groups of one row block stream
 // weights and gain nothing (training step of 1240 tokens, 64 experts of 1024, hidden 2048: 779 us, 791 with wide tiles).
+// The gated form delays by less, which shows with counted groups: sustained, by 256 and by 512 columns, 8 groups of 750 rows, 8192 columns,
+// 2048 deep 180 and 190 us, of 1366 rows 323 and 333, of 2250 rows 485 and 477; 28672 columns, 4096 deep, 750 rows 1263 and 1225, 1931 rows
+// 2894 and 2850.  4000 cycles put the line near 2500 deep.
 g2::Width grouped_width(PairForm form, int G, int rows, bool counted, int N, int K, int pairs) {
   return g2::plan_width(G * ((rows + BM - 1LL) / BM), N, K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
-                        form == ROWS_SWIGLU_BWD || (counted && rows <= BM) ? BN : 2 * BN, form == ROWS_ACT ? 8000 : 0);
+                        form == ROWS_SWIGLU_BWD || (counted && rows <= BM) ? BN : 2 * BN, form == ROWS_ACT ? 8000 : form == ROWS_GATED && counted ? 4000 : 0);
 }
 
 // A launch of the CTA-pair kernels that may overlap the tail of the stream's previous kernel.

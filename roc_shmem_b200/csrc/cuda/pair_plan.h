@@ -15,11 +15,12 @@ namespace gemm2 {
 //  - of an MN-major B two blocks of 64 columns per CTA and accumulator are loaded whatever the width; what lies beyond it counts half;
 //  - the rows of A are a share of a wide tile's loads too, about 26 columns' worth;
 //  - a wave has a beginning and an end, worth about 8 columns.
-// Without `exact`, row_blocks is an estimate, and a launch is taken to lose half a wave (16 groups of about 770 rows, 1024 columns, 2048 and
-// 4096 deep: 155 us for both by 256 columns, 171 by 512).
+// Without `exact`, row_blocks is an estimate: two accumulators have to be the better choice both where a launch loses half a wave, as
+// with unequal groups, and by whole waves, as with equal ones.  Sustained, by 256 and by 512 columns: 16 groups of 1125 rows, 1024
+// columns, 2048 deep (better by the first, 2.16 waves paid as three) 83.3 and 88.7 us, 1629 rows 113.5 and 118.0; 8 groups of 1931 rows,
+// 2048 columns, 4096 deep 220 and 230; of 750 rows (worse by both) 97 and 109; of 2250 rows (better by both) 248 and 241, 8192 deep 494 and 468.
 // `wide_delay`: cycles that a tile's epilogue keeps the tensor cores waiting in the wide form (two per column and k-block).
 // `step`: what an accumulator's columns are a multiple of, 32 or, where the epilogue wants more, 64 or 128.
-// Over 30 problems of 264 to 8192 rows in the three layouts the choice was within 4 % of the best of ten widths.
 struct Width {
   int cols[2];
 };
@@ -27,21 +28,19 @@ inline Width plan_width(long long row_blocks, int N, int K, int pairs, int step,
                         int wide_delay = 0) {
   constexpr int BN = 256;
   const double blocks = (K + 63) / 64, narrow = 0.91 + blocks / 160 < 1.1 ? 0.91 + blocks / 160 : 1.1;
-  Width best = {{BN, 0}};
-  double best_cost = 1e30;
+  struct { double cost, whole; Width w; } best[2] = {{1e30, 1e30, {{BN, 0}}}, {1e30, 1e30, {{BN, 0}}}};      // of one accumulator, of two
   for (int w = widest; w >= 128; w -= step) {
     if (w > BN && w < 352) continue;                  // two accumulators of less than 160 columns
     const int c0 = w > BN ? (w + 2 * step - 1) / (2 * step) * step : w, c1 = w - c0;
     const int loaded = !b_mn ? w : c1 ? 2 * BN : BN;
     const long long tiles = row_blocks * ((N + w - 1) / w);
-    const double waves = exact ? (double)((tiles + pairs - 1) / pairs) : tiles > pairs / 2 ? 0.5 + (double)tiles / pairs : 1.0;
-    const double cost = waves * ((c1 ? 26 + 0.95 * 0.5 * (w + loaded) + wide_delay / (2 * blocks) : narrow * 0.5 * (BN + loaded)) + 8);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = {{c0, c1}};
-    }
+    const double per_wave = (c1 ? 26 + 0.95 * 0.5 * (w + loaded) + wide_delay / (2 * blocks) : narrow * 0.5 * (BN + loaded)) + 8;
+    const double whole = (double)((tiles + pairs - 1) / pairs) * per_wave;
+    const double cost = exact ? whole : (tiles > pairs / 2 ? 0.5 + (double)tiles / pairs : 1.0) * per_wave;
+    auto& b = best[c1 ? 1 : 0];
+    if (cost < b.cost) b = {cost, whole, {{c0, c1}}};
   }
-  return best;
+  return best[1].cost <= best[0].cost && best[1].whole <= best[0].whole ? best[1].w : best[0].w;
 }
 
 // Rows of a group whose count is on the device, as far as the host knows: about `about`, as the caller says, else four fifths of its
