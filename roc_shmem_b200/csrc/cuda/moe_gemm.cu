@@ -438,8 +438,11 @@ int ensure(int dev) {
 // The gated form delays by less, which shows with counted groups: sustained, by 256 and by 512 columns, 8 groups of 750 rows, 8192 columns,
 // 2048 deep 180 and 190 us, of 1366 rows 323 and 333, of 2250 rows 485 and 477; 28672 columns, 4096 deep, 750 rows 1263 and 1225, 1931 rows
 // 2894 and 2850.  4000 cycles put the line near 2500 deep.
+// In the weight gradients wide tiles pay at shorter reductions than in the plain product: 750 tokens, 8 groups of 2048 x 4096 102.6 and 94.3
+// us, 64 of 2048 x 2048 437 and 373, one of 4096 x 3584 25.2 and 24.2; 375 tokens 62.4 and 62.4, 251 and 234, 16.6 and 16.4.  They are
+// planned as if they were 256 deeper, which puts the line near 600.
 g2::Width grouped_width(PairForm form, int G, int rows, bool counted, int N, int K, int pairs) {
-  return g2::plan_width(G * ((rows + BM - 1LL) / BM), N, K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
+  return g2::plan_width(G * ((rows + BM - 1LL) / BM), N, form == PAIR_TN ? K + 256 : K, pairs, form == ROWS_GATED || form == PAIR_TN ? 128 : 64, form == PAIR_TN, !counted,
                         form == ROWS_SWIGLU_BWD || (counted && rows <= BM) ? BN : 2 * BN, form == ROWS_ACT ? 8000 : form == ROWS_GATED && counted ? 4000 : 0);
 }
 
