@@ -28,6 +28,7 @@
 #include "../include/bshmem_gpu.h"
 #include "coll_kernels.h"
 #include "gpu_heap.h"
+#include "launch_choice.h"
 #include "message_ring.h"
 
 using namespace bshmem;
@@ -899,50 +900,48 @@ class GpuBackend final : public Backend {
     std::lock_guard<std::mutex> lock(group_mu_);
     bool all = true;
     for (int i = 0; i < n; ++i) all = all && ht[i].my_idx >= 0 && ht[i].size == n;
-    if (all && ctas * n <= collk::kClusterBlocks) {
-      const Ticket t(&lanes_[0]);
-      pinned_->status[t.slot] = 0;
-      collk::GroupDone done;
-      done.word = t.done.word;
-      done.token = t.done.token;
-      return group_wait(t, collk::launch_cluster(hs, ht, a, ctas, n, &pinned_->status[t.slot], stream_, done), "cluster launch: ");
-    }
-    if (!group_dev_) {
-      // on the stream of the launch: it may be one that does not wait for the default stream
-      char* mem = nullptr;
-      RT_TRY(cudaMalloc(&mem, sizeof(GroupTable) + 16));
-      const cudaError_t e = cudaMemsetAsync(mem, 0, sizeof(GroupTable) + 16, stream_);
-      if (e != cudaSuccess) { cudaFree(mem); RT_TRY(e); }
-      group_dev_ = mem;
-      memset(&group_host_, 0, sizeof(group_host_));
-    }
-    GroupTable img;
-    memset(&img, 0, sizeof(img));
-    memcpy(img.states, hs, sizeof(State) * n);
-    memcpy(img.teams, ht, sizeof(DTeam) * n);
-    if (memcmp(&img, &group_host_, sizeof(img)) != 0) {
-      RT_TRY(cudaMemcpyAsync(group_dev_, &img, sizeof(img), cudaMemcpyHostToDevice, stream_));
-      group_host_ = img;
-    }
-    GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
     const Ticket t(&lanes_[0]);
-    pinned_->status[t.slot] = 0;
+    int* status = &pinned_->status[t.slot];
+    *status = 0;
     collk::GroupDone done;
-    done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
     done.word = t.done.word;
     done.token = t.done.token;
-    return group_wait(t, collk::launch_group(dev->states, dev->teams, a, ctas, n, &pinned_->status[t.slot], stream_, done), "cooperative launch: ");
-  }
-  int group_wait(const Ticket& t, cudaError_t launched, const char* what) {
-    if (launched != cudaSuccess) {
+    auto cluster = [&] {
+      const cudaError_t e = collk::launch_cluster(hs, ht, a, ctas, n, status, stream_, done);
+      if (e != cudaSuccess) cudaGetLastError();      // not for somebody's next launch
+      return e == cudaSuccess ? (int)BSHMEM_OK : (int)BSHMEM_ERR_CUDA;
+    };
+    auto cooperative = [&]() -> int {
+      if (!group_dev_) {
+        // on the stream of the launch: it may be one that does not wait for the default stream
+        char* mem = nullptr;
+        RT_TRY(cudaMalloc(&mem, sizeof(GroupTable) + 16));
+        const cudaError_t e = cudaMemsetAsync(mem, 0, sizeof(GroupTable) + 16, stream_);
+        if (e != cudaSuccess) { cudaFree(mem); RT_TRY(e); }
+        group_dev_ = mem;
+        memset(&group_host_, 0, sizeof(group_host_));
+      }
+      GroupTable img;
+      memset(&img, 0, sizeof(img));
+      memcpy(img.states, hs, sizeof(State) * n);
+      memcpy(img.teams, ht, sizeof(DTeam) * n);
+      if (memcmp(&img, &group_host_, sizeof(img)) != 0) {
+        RT_TRY(cudaMemcpyAsync(group_dev_, &img, sizeof(img), cudaMemcpyHostToDevice, stream_));
+        group_host_ = img;
+      }
+      GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
+      done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
+      const cudaError_t e = collk::launch_group(dev->states, dev->teams, a, ctas, n, status, stream_, done);
+      if (e == cudaSuccess) return BSHMEM_OK;
       cudaGetLastError();        // reported here, not at somebody's next launch
-      tl_err = std::string(what) + cudaGetErrorString(launched);
+      tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e);
       return BSHMEM_ERR_CUDA;
-    }
-    const int rc = wait_done(t, stream_), status = pinned_->status[t.slot];
-    if (rc != BSHMEM_OK || status == BSHMEM_OK) return rc;
-    tl_err = std::string("device-side ") + bshmem_status_string(status);
-    return status;
+    };
+    int rc = launch_preferred(all && ctas * n <= collk::kClusterBlocks, (int)BSHMEM_OK, cluster, cooperative);
+    if (rc == BSHMEM_OK) rc = wait_done(t, stream_);
+    if (rc != BSHMEM_OK || *status == BSHMEM_OK) return rc;
+    tl_err = std::string("device-side ") + bshmem_status_string(*status);
+    return *status;
   }
 
  private:
