@@ -305,6 +305,7 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
   }
   int pairs = g_pairs[dev];
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  if (pairs < 1) { host::last_error() = "gemm: the device holds no CTA pair of this kernel"; return 1; }
   // Few tiles: split each over the two or four pairs of a cluster while all clusters run at once.  Parking and adding the
   // parts costs about 4 us, what a pair needs for 14 k-blocks.
   const int kb = (K + BK - 1) / BK;

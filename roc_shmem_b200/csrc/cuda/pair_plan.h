@@ -20,6 +20,7 @@ namespace gemm2 {
 // columns, 2048 deep (better by the first, 2.16 waves paid as three) 83.3 and 88.7 us, 1629 rows 113.5 and 118.0; 8 groups of 1931 rows,
 // 2048 columns, 4096 deep 220 and 230; of 750 rows (worse by both) 97 and 109; of 2250 rows (better by both) 248 and 241, 8192 deep 494 and 468.
 // `wide_delay`: cycles that a tile's epilogue keeps the tensor cores waiting in the wide form (two per column and k-block).
+// `pairs`: that work at the same time; with none (nothing can be launched) as with one.
 // `step`: what an accumulator's columns are a multiple of, 32 or, where the epilogue wants more, 64 or 128.
 struct Width {
   int cols[2];
@@ -27,6 +28,7 @@ struct Width {
 inline Width plan_width(long long row_blocks, int N, int K, int pairs, int step, bool b_mn, bool exact = true, int widest = 512,
                         int wide_delay = 0) {
   constexpr int BN = 256;
+  if (pairs < 1) pairs = 1;
   const double blocks = (K + 63) / 64, narrow = 0.91 + blocks / 160 < 1.1 ? 0.91 + blocks / 160 : 1.1;
   struct { double cost, whole; Width w; } best[2] = {{1e30, 1e30, {{BN, 0}}}, {1e30, 1e30, {{BN, 0}}}};      // of one accumulator, of two
   for (int w = widest; w >= 128; w -= step) {
