@@ -55,10 +55,7 @@ constexpr int BM = 256, BN = 256;                 // tile of the CTA pair
 constexpr int CTA_M = 128, CTA_NLOAD = 128;       // rows of A / of B one CTA loads
 constexpr int BK_BYTES = 128;
 constexpr int BK = 64;                            // bf16 elements per k-block
-#ifndef BSHMEM_PAIR_STAGES
-#define BSHMEM_PAIR_STAGES 6
-#endif
-constexpr int STAGES = BSHMEM_PAIR_STAGES;
+constexpr int STAGES = 6;
 constexpr int UMMA_K_BYTES = 32;
 constexpr int NUM_EPI_WARPS = 8;
 constexpr int NUM_THREADS = 32 * (2 + NUM_EPI_WARPS);
