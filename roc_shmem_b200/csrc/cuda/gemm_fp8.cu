@@ -340,7 +340,10 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
   }
 
   // Behind the plain form of the same product nothing has to be waited for: its blocks have waited for everything before it, and its
-  // tiles are others.  What follows in the stream waits for this kernel only, so this one ends after that (below).
+  // tiles are others.  This relies on every block of that form launching its dependents only behind its own wait, and on what that
+  // wait found done (the quantiser's output in L2) being seen by blocks that start afterwards; the programming model as such promises
+  // it to the kernel that waits.  What follows in the stream waits for this kernel only, so this one ends after that (below).
+  // Its tiles are added up in shares of K, an order of its own: fp32 as before, the last bits differ from the plain form's.
   if constexpr (kMode == F8_PLAIN) ptx::grid_dependency_wait();
   if constexpr (kSplit) {
     if (!prm.behind) ptx::grid_dependency_wait();

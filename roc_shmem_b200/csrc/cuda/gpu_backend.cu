@@ -182,12 +182,14 @@ __global__ void __launch_bounds__(256) k_copy_small(char* dst, const char* src, 
   const uint64_t b = blockIdx.x * kSmallPiece, e = b + kSmallPiece < n ? b + kSmallPiece : n;
   dev::copy_bytes<dev::BLOCK>(dst + b, src + b, e - b);
 }
-// Non-blocking messages of a context, up to kRingMessageMax bytes between device buffers, need no launch each: the host writes them into a
-// ring in pinned memory and one block on the context's stream takes them from there.  The block is launched by the first
-// message, stays while messages follow one another closely (kRingIdleNs) and at most kRingLifeNs, and takes no more than this one
-// block's place.  The host path bounds a window of messages: 64 puts of 64 bytes and a quiet took 177 us by one launch each
-// (2.4 us apart and more), 44 so.  A block with sixteen warps moves a message per warp, 16 KiB in four round trips to memory, as fast as
-// the host writes them.
+// Non-blocking messages of a context, up to kRingMessageMax bytes between device buffers, need no launch each: the host writes
+// them into a ring in pinned memory and one block on the context's stream takes them from there.  The block is launched by the
+// first message, stays while messages follow one another closely (kRingIdleNs) and at most kRingLifeNs.  While it stays it has
+// its multiprocessor's place, beside kernels that take a whole one per block too: 8192 x 8192 x 3584 products with 64 messages
+// before each take 358 to 360 us (356 to 361 with one launch per message); 1024 rows 50 (173 to 181), with four messages 49
+// (43).  Ending after 2 us without a message instead of 5 gains nothing there and costs a window 8 of 48 us.  The host path
+// bounds a window of messages: 64 puts of 64 bytes and a quiet took 177 us by one launch each (2.4 us apart and more), 44 so.  A
+// block with sixteen warps moves a message per warp, 16 KiB in four round trips to memory, as fast as the host writes them.
 // message_ring.h has the protocol.
 constexpr unsigned kRingThreads = 512, kRingBatch = kRingThreads / 32;
 constexpr unsigned long long kRingIdleNs = 5000, kRingLifeNs = 100000;
