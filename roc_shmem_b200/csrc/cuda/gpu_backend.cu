@@ -392,6 +392,18 @@ thread_local int tl_bound_ctx = -1;
 thread_local bool tl_local_is_device = false;   // the caller vouches that the local buffer is memory of this PE's GPU
 thread_local std::string tl_err;
 
+// While it exists, the calling thread may synchronise streams that are not captured although another one is.
+class RelaxedCapture {
+ public:
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  RelaxedCapture(const RelaxedCapture&) = delete;
+  RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 class GpuBackend final : public Backend {
  public:
   GpuBackend(gpu::Heap* heap, bool own_heap) : heap_(heap), own_heap_(own_heap) {}
@@ -520,7 +532,11 @@ class GpuBackend final : public Backend {
           RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
           return BSHMEM_OK;
         },
-        [&](auto arrived) { return poll(arrived, L.stream); });
+        [&](auto arrived) {
+          // a message that nobody waits for may be sent while another stream is captured: its wait for room is no part of that
+          const RelaxedCapture relaxed;
+          return poll(arrived, L.stream);
+        });
     if (rc == BSHMEM_ERR_STATE) tl_err = "the context's messages were not taken";
     return rc;
   }

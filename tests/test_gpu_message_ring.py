@@ -203,3 +203,26 @@ def test_quiet_of_one_thread_beside_messages_of_another(rt):
     ctx.quiet()
     assert torch.equal(small, msgs)
     ctx.destroy()
+
+
+def test_more_messages_than_slots_while_a_stream_is_captured(rt):
+    """Non-blocking puts behind long copies, more of them than the ring has slots, while another stream is captured."""
+    ctx = rt.ctx_create(0)
+    big, small = rt.zeros((64 << 20,), torch.uint8), rt.zeros((600, 64), torch.uint8)
+    src, msgs = torch.full((64 << 20,), 3, dtype=torch.uint8, device="cuda"), torch.randint(0, 256, (600, 64), dtype=torch.uint8, device="cuda")
+    x, g = torch.zeros(16, device="cuda"), torch.cuda.CUDAGraph()
+    rows = list(zip(small.unbind(0), msgs.unbind(0)))
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        for _ in range(64):
+            ctx.put(big, src, 0, nbi=True)
+        for d, s in rows:
+            ctx.put(d, s, 0, nbi=True)
+        x.add_(1)
+    ctx.quiet()
+    assert torch.equal(small, msgs) and bool((big == 3).all())
+    g.replay()
+    torch.cuda.synchronize()
+    assert bool((x == 2).all())
+    ctx.destroy()
