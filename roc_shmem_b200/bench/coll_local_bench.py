@@ -1,4 +1,4 @@
-"""Device collectives of a local group (all PEs of the job on ONE GPU, one cooperative launch per collective):
+"""Device collectives of a local group (all PEs of the job on ONE GPU, one launch per collective):
 timing and a correctness check of allreduce / reduce-scatter / fcollect / alltoall without any NVLink hop.
 
     python -m roc_shmem_b200.bench.coll_local_bench [--pes 4] [--bytes 67108864] [--op allreduce] [--dtype float32] [--iters 5]

@@ -41,14 +41,13 @@ cudaError_t launch_group(const State* states, const DTeam* teams, const CollArgs
   }
 }
 
-cudaError_t launch_cluster(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status, cudaStream_t stream,
-                           const GroupDone& done) {
-  switch (unit_of(a)) {
-    case U_MOVE: return launch_cluster_move(states, teams, a, ctas, n, status, stream, done);
-    case U_F32: return launch_cluster_f32(states, teams, a, ctas, n, status, stream, done);
-    case U_F16: return launch_cluster_f16(states, teams, a, ctas, n, status, stream, done);
-    case U_I32: return launch_cluster_i32(states, teams, a, ctas, n, status, stream, done);
-    case U_I8: return launch_cluster_i8(states, teams, a, ctas, n, status, stream, done);
+cudaError_t launch_pass(const GroupPass& g, int ctas, cudaStream_t stream) {
+  switch (unit_of(g.a)) {
+    case U_MOVE: return launch_pass_move(g, ctas, stream);
+    case U_F32: return launch_pass_f32(g, ctas, stream);
+    case U_F16: return launch_pass_f16(g, ctas, stream);
+    case U_I32: return launch_pass_i32(g, ctas, stream);
+    case U_I8: return launch_pass_i8(g, ctas, stream);
     default: return cudaErrorInvalidValue;
   }
 }

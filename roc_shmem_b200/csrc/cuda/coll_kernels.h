@@ -3,8 +3,9 @@
 // The device collectives of bshmem_coll.cuh are templates over the element type and the operator; instantiating all
 // of them in one translation unit takes many minutes.  The kernels are therefore split by element class into
 // translation units of their own (built in parallel): data movement and synchronisation, 4/8-byte floats, 2-byte
-// floats, 4/8-byte integers, 1/2-byte integers.  Each unit has one kernel for a PE per launch and one for all PEs
-// of a local group in a single cooperative launch (blockIdx.y = PE), and the host picks the unit by (kind, dtype).
+// floats, 4/8-byte integers, 1/2-byte integers.  Each unit has one kernel for a PE per launch, one for all PEs of a local
+// group in a single cooperative launch (blockIdx.y = PE) and one for a local group as one pass over all members' memory, and the
+// host picks the unit by (kind, dtype).
 // Parity: these are the bodies behind library/src/roc_shmem.cpp's host collectives (:1033-1128), which the
 // reference forwards to MPI.
 #pragma once
@@ -69,12 +70,21 @@ struct GroupDone {
 // All PEs of a local group at once: states / teams are device arrays of n entries (a team with my_idx < 0 sits out).
 cudaError_t launch_group(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status,
                          cudaStream_t stream, const GroupDone& done = GroupDone());
-// The same as one thread-block cluster, for at most kClusterBlocks blocks of all PEs together, every one of them a member: the
-// blocks of a cluster run at the same time without a cooperative launch, and synchronise by its barrier.  states / teams are
-// HOST arrays of n entries and travel as kernel parameters.
-constexpr int kClusterBlocks = 8;
-cudaError_t launch_cluster(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status, cudaStream_t stream,
-                           const GroupDone& done);
+// The same without any exchange, for a collective that moves data (not sync, barrier or the host's exchange) and whose members are all
+// here: what they bring is in place when the launch begins, and its end is the end of the call, so each block reads from every member
+// and writes to every member.  Blocks do not wait for one another, and the launch needs no co-operation.
+struct GroupPass {
+  char* base[BSHMEM_MAX_PES];                   // heap of team member k, 16-byte aligned
+  unsigned long long* stats[BSHMEM_MAX_PES];    // its counters and trace, or null
+  int pe[BSHMEM_MAX_PES];
+  int size;
+  CollArgs a;
+  GroupDone done;
+};
+inline bool pass_kind(int kind) {
+  return kind >= 2 /* BSHMEM_COLL_BROADCAST */ && kind <= 6 /* BSHMEM_COLL_ALLTOALL */ || kind == 8 /* BSHMEM_COLL_REDUCE_ROOT */;
+}
+cudaError_t launch_pass(const GroupPass& g, int ctas, cudaStream_t stream);
 // Loads every kernel module now (a lazy first load from another thread could need a device-wide quiet point).
 void preload();
 
@@ -83,7 +93,7 @@ void preload();
   cudaError_t launch_##name(const State&, const DTeam&, const CollArgs&, int, int*, cudaStream_t);                       \
   cudaError_t launch_group_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t,             \
                                   const GroupDone&);                                                                     \
-  cudaError_t launch_cluster_##name(const State*, const DTeam*, const CollArgs&, int, int, int*, cudaStream_t, const GroupDone&); \
+  cudaError_t launch_pass_##name(const GroupPass&, int, cudaStream_t);                                                   \
   void preload_##name();
 BSHMEM_COLL_UNIT(move)
 BSHMEM_COLL_UNIT(f32)

@@ -1,9 +1,7 @@
 // coll_kernels_impl.cuh — body of one collective-kernel translation unit.  The including .cu defines
 //   COLL_UNIT        name of the unit (move, f32, ...)
 //   COLL_TYPES(X)    X(dtype code, C type) for every element type the unit reduces (empty for `move`)
-// and gets a per-PE kernel, a local-group kernel and their launchers (see coll_kernels.h).
-#include <cstring>
-
+// and gets a per-PE kernel, the kernels of a local group and their launchers (see coll_kernels.h).
 #include "../include/bshmem_coll.cuh"
 #include "../include/bshmem_gpu.h"
 #include "coll_kernels.h"
@@ -121,8 +119,9 @@ __device__ __forceinline__ void group_failed(int* status, int rc) {
   __threadfence_system();
 }
 
-// All PEs of a local group in ONE cooperative launch: blockIdx.y is the PE.  Used to exercise the multi-PE
-// algorithms on a single GPU (kernels that wait on one another must not be separate launches on one device).
+// All PEs of a local group in ONE cooperative launch: blockIdx.y is the PE.  Runs the multi-PE algorithms, flag exchanges
+// included, on a single GPU (kernels that wait on one another must not be separate launches on one device): syncs, and what is
+// no pass (below).
 // The block works on a copy of its PE's state in shared memory (a private copy is 220 bytes of local memory per thread).
 __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(const State* states, const DTeam* teams,
                                                                                 CollArgs a, int* status, GroupDone done) {
@@ -149,29 +148,195 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(c
   }
 }
 
-// The group as one cluster.  Bound by the launch and two round trips to memory: allreduce of 16 KiB of fp32 over 4 PEs, whole call,
-// 14.9 us, cooperatively launched with flags in memory 19.5.
-struct ClusterGroup {
-  State states[kClusterBlocks];
-  DTeam teams[kClusterBlocks];
-};
-__global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_cluster_, COLL_UNIT)(const __grid_constant__ ClusterGroup g, CollArgs a, int* status,
-                                                                                  GroupDone done) {
-  __shared__ State s;
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(&g.states[blockIdx.y]);
-  for (unsigned i = threadIdx.x; i < sizeof(State) / 4; i += kThreads) reinterpret_cast<uint32_t*>(&s)[i] = src[i];
-  const DTeam t = g.teams[blockIdx.y];
-  __syncthreads();
-  if (threadIdx.x == 0) s.one_gpu = BSHMEM_ONE_CLUSTER;
-  __syncthreads();
-  asm volatile("griddepcontrol.wait;" ::: "memory");         // launched before its predecessor's end
-  const int rc = run_coll(s, t, a, blockIdx.x, gridDim.x);
-  if (rc != BSHMEM_OK && threadIdx.x == 0) group_failed(status, rc);
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
-    __threadfence();
-    asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(done.word), "l"(done.token) : "memory");
+// ---- the group as one pass (GroupPass) ----
+// Bound by the launch and one round trip to memory where little is moved, by HBM beyond.  Before: up to eight blocks as a cluster with
+// two barriers, more of them cooperatively with two flag exchanges, large reductions staged through shared memory.  Whole calls, before
+// and now, us: allreduce 16 KiB fp32, 4 PEs 14.9 -> 10.5; 1 MiB bf16, 8 PEs 23.4 -> 12.6; 32 MiB fp32, 8 PEs 117 -> 103; reduce-scatter
+// 32 MiB bf16, 8 PEs 83.7 -> 59.8 (302 MB, 46 at the copy rate), 32 MiB fp32, 4 PEs 50.0 -> 39.8; fcollect 16 MiB, 8 PEs 44.4 -> 38.4;
+// alltoall 32 MiB, 8 PEs 107 -> 101, 2 MiB, 4 PEs 20.0 -> 13.5.
+// 512 threads with 16 loads of 16 bytes each on their way keep 128 KB in flight per block; a block to a multiprocessor, as many as
+// the caller asked for.
+constexpr int kPassThreads = 512;
+
+__device__ __forceinline__ State pass_state(const GroupPass& g) {      // what the counters and the trace take of a state
+  State s;
+  s.stats = g.stats[blockIdx.y];
+  s.my_pe = g.pe[blockIdx.y];
+  return s;
+}
+// The launch's blocks are counted, and the last one tells the host.  A system fence per block took 4 us; the group shares the GPU.
+__device__ __forceinline__ void pass_end(const GroupPass& g, unsigned long long cap, unsigned long long traced_bytes) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const State s = pass_state(g);
+    dev::stat(s, BSHMEM_DSTAT_COLL);
+    dev::trace_with(s, cap, BSHMEM_TRACE_COLL, s.my_pe, traced_bytes);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned n = gridDim.x * gridDim.y;
+    if (atomicInc(g.done.count, n - 1) == n - 1) {
+      __threadfence();
+      asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(g.done.word), "l"(g.done.token) : "memory");
+    }
+  }
+}
+__device__ __forceinline__ unsigned long long pass_trace_capacity(const GroupPass& g) {
+  return blockIdx.x == 0 && threadIdx.x == 0 ? dev::trace_capacity(pass_state(g)) : 0ull;
+}
+
+#ifndef COLL_UNIT_MOVE
+// nv vectors of every member from byte src_at of its heap on, reduced in team order, to byte dst_at of the heaps of members
+// [d0, d0 + nd).  NS sources (more than `size`: those beyond it are left out), U vectors of each on their way per thread.
+template <typename T, int OP, int NS, int U>
+__device__ __forceinline__ void pass_vectors(const GroupPass& g, uint64_t src_at, uint64_t dst_at, int d0, int nd, size_t nv) {
+  using A = typename coll::Acc<T>::type;
+  constexpr int VE = 16 / sizeof(T);
+  for (size_t v0 = threadIdx.x; v0 < nv; v0 += (size_t)U * blockDim.x) {
+    coll::Vec16<T> in[U][NS];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t v = v0 + (size_t)u * blockDim.x;
+      if (v < nv) {
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+          if (k < g.size) in[u][k].raw = *reinterpret_cast<const uint4*>(g.base[k] + src_at + v * 16);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t v = v0 + (size_t)u * blockDim.x;
+      if (v < nv) {
+        A acc[VE];
+#pragma unroll
+        for (int e = 0; e < VE; ++e) acc[e] = coll::to_acc<T>(in[u][0].e[e]);
+#pragma unroll
+        for (int k = 1; k < NS; ++k) {
+          if (k < g.size) {
+#pragma unroll
+            for (int e = 0; e < VE; ++e) acc[e] = coll::apply<A>(OP, acc[e], coll::to_acc<T>(in[u][k].e[e]));
+          }
+        }
+        coll::Vec16<T> out;
+#pragma unroll
+        for (int e = 0; e < VE; ++e) out.e[e] = coll::from_acc<T>(acc[e]);
+        for (int d = d0; d < d0 + nd; ++d) *reinterpret_cast<uint4*>(g.base[d] + dst_at + v * 16) = out.raw;
+      }
+    }
+  }
+}
+template <typename T, int OP>
+__device__ __forceinline__ void pass_reduce_op(const GroupPass& g, uint64_t src_at, uint64_t dst_at, int d0, int nd, size_t n) {
+  using A = typename coll::Acc<T>::type;
+  constexpr int VE = 16 / sizeof(T);
+  const size_t nv = ((src_at | dst_at) & 15) == 0 ? n / VE : 0;
+  // the types and operators of bulk reductions in unrolled form, the rest in a general one
+  constexpr bool kHot = (OP == BSHMEM_SUM || OP == BSHMEM_MAX || OP == BSHMEM_MIN) &&
+                        (std::is_same<T, float>::value || std::is_same<T, double>::value || std::is_same<T, __half>::value ||
+                         std::is_same<T, __nv_bfloat16>::value || std::is_same<T, int32_t>::value || std::is_same<T, long long>::value);
+  if constexpr (kHot) {
+    switch (g.size) {
+      case 2: pass_vectors<T, OP, 2, 8>(g, src_at, dst_at, d0, nd, nv); break;
+      case 4: pass_vectors<T, OP, 4, 4>(g, src_at, dst_at, d0, nd, nv); break;
+      case 8: pass_vectors<T, OP, 8, 2>(g, src_at, dst_at, d0, nd, nv); break;
+      default: pass_vectors<T, OP, BSHMEM_MAX_PES, 1>(g, src_at, dst_at, d0, nd, nv);
+    }
+  } else {
+    pass_vectors<T, OP, BSHMEM_MAX_PES, 1>(g, src_at, dst_at, d0, nd, nv);
+  }
+  // what is left behind the last whole vector, or all of it where the two sides are not on 16-byte boundaries
+  for (size_t i = nv * VE + threadIdx.x; i < n; i += blockDim.x) {
+    A acc = coll::to_acc<T>(reinterpret_cast<const T*>(g.base[0] + src_at)[i]);
+    for (int k = 1; k < g.size; ++k) acc = coll::apply<A>(OP, acc, coll::to_acc<T>(reinterpret_cast<const T*>(g.base[k] + src_at)[i]));
+    for (int d = d0; d < d0 + nd; ++d) reinterpret_cast<T*>(g.base[d] + dst_at)[i] = coll::from_acc<T>(acc);
+  }
+}
+
+// A block's share: of an allreduce and a rooted reduction a part of the vector, of a reduce-scatter a part of member blockIdx.y's
+// block.  An element is read and written by one thread, so the results may take the place of the sources.
+template <typename T>
+__global__ void __launch_bounds__(kPassThreads) COLL_CAT(k_coll_pass_, COLL_UNIT)(const __grid_constant__ GroupPass g) {
+  const CollArgs& a = g.a;
+  const unsigned long long cap = pass_trace_capacity(g);
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // launched before its predecessor's end
+  const int me = blockIdx.y;
+  const bool scatter = a.kind == BSHMEM_COLL_REDUCE_SCATTER;
+  size_t b, e;
+  if (scatter) coll::split_range(a.n, gridDim.x, blockIdx.x, 16 / sizeof(T), &b, &e);
+  else coll::split_range(a.n, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x, 16 / sizeof(T), &b, &e);
+  const uint64_t dst_at = a.dst_off + b * sizeof(T), src_at = a.src_off + (b + (scatter ? (size_t)me * a.n : 0)) * sizeof(T);
+  const int d0 = a.kind == BSHMEM_COLL_REDUCE ? 0 : scatter ? me : a.root, nd = a.kind == BSHMEM_COLL_REDUCE ? g.size : 1;
+  switch (a.op) {
+    case BSHMEM_SUM: pass_reduce_op<T, BSHMEM_SUM>(g, src_at, dst_at, d0, nd, e - b); break;
+    case BSHMEM_MIN: pass_reduce_op<T, BSHMEM_MIN>(g, src_at, dst_at, d0, nd, e - b); break;
+    case BSHMEM_MAX: pass_reduce_op<T, BSHMEM_MAX>(g, src_at, dst_at, d0, nd, e - b); break;
+    case BSHMEM_PROD: pass_reduce_op<T, BSHMEM_PROD>(g, src_at, dst_at, d0, nd, e - b); break;
+    default:
+      if constexpr (!std::is_floating_point<typename coll::Acc<T>::type>::value) {
+        if (a.op == BSHMEM_AND) pass_reduce_op<T, BSHMEM_AND>(g, src_at, dst_at, d0, nd, e - b);
+        else if (a.op == BSHMEM_OR) pass_reduce_op<T, BSHMEM_OR>(g, src_at, dst_at, d0, nd, e - b);
+        else pass_reduce_op<T, BSHMEM_XOR>(g, src_at, dst_at, d0, nd, e - b);
+      }
+  }
+  pass_end(g, cap, a.kind == BSHMEM_COLL_REDUCE_ROOT ? a.n * sizeof(T) : 0);
+}
+#else
+// fcollect: member blockIdx.y's block to everybody, read once.  alltoall: member blockIdx.y's blocks to their owners.  broadcast: the
+// root's vector to member blockIdx.y, the root's own dest left as it is.
+__global__ void __launch_bounds__(kPassThreads) k_coll_pass_move(const __grid_constant__ GroupPass g) {
+  const CollArgs& a = g.a;
+  const unsigned long long cap = pass_trace_capacity(g);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int me = blockIdx.y;
+  size_t b, e;
+  coll::split_range(a.n, gridDim.x, blockIdx.x, 16, &b, &e);
+  const size_t n = e - b;
+  if (a.kind == BSHMEM_COLL_BROADCAST) {
+    if (me != a.root) dev::copy_bytes<dev::BLOCK>(g.base[me] + a.dst_off + b, g.base[a.root] + a.src_off + b, n);
+  } else if (a.kind == BSHMEM_COLL_ALLTOALL) {
+    for (int k = 0; k < g.size; ++k) {
+      const int j = (me + k) % g.size;
+      dev::copy_bytes<dev::BLOCK>(g.base[j] + a.dst_off + (uint64_t)me * a.n + b, g.base[me] + a.src_off + (uint64_t)j * a.n + b, n);
+    }
+  } else {
+    const uint64_t src_at = a.src_off + b, dst_at = a.dst_off + (uint64_t)me * a.n + b;
+    size_t done = 0;
+    if (((src_at | dst_at) & 15) == 0) {
+      constexpr int U = 8;
+      const size_t nv = n >> 4;
+      const uint4* src = reinterpret_cast<const uint4*>(g.base[me] + src_at);
+      for (size_t v0 = threadIdx.x; v0 < nv; v0 += (size_t)U * blockDim.x) {
+        uint4 x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (v0 + (size_t)u * blockDim.x < nv) x[u] = src[v0 + (size_t)u * blockDim.x];
+        for (int d = 0; d < g.size; ++d) {
+          uint4* dst = reinterpret_cast<uint4*>(g.base[d] + dst_at);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (v0 + (size_t)u * blockDim.x < nv) dst[v0 + (size_t)u * blockDim.x] = x[u];
+        }
+      }
+      done = nv << 4;
+    }
+    for (int d = 0; d < g.size; ++d) dev::copy_bytes<dev::BLOCK>(g.base[d] + dst_at + done, g.base[me] + src_at + done, n - done);
+  }
+  pass_end(g, cap, 0);
+}
+#endif
+
+template <class Kernel>
+cudaError_t launch_pass_kernel(Kernel* kernel, const GroupPass& g, int ctas, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas, (unsigned)g.size);
+  cfg.blockDim = dim3(kPassThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, g);
 }
 
 }  // namespace
@@ -190,36 +355,33 @@ cudaError_t COLL_CAT(launch_group_, COLL_UNIT)(const State* states, const DTeam*
                                      dyn_smem(a, ctas, ctas * n), stream);
 }
 
-cudaError_t COLL_CAT(launch_cluster_, COLL_UNIT)(const State* states, const DTeam* teams, const CollArgs& a, int ctas, int n, int* status,
-                                                 cudaStream_t stream, const GroupDone& done) {
-  ClusterGroup g;
-  memset(&g, 0, sizeof(g));
-  memcpy(g.states, states, sizeof(State) * n);
-  memcpy(g.teams, teams, sizeof(DTeam) * n);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas, (unsigned)n);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = dyn_smem(a, ctas, ctas * n);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)ctas; attr[1].val.clusterDim.y = (unsigned)n; attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, COLL_CAT(k_coll_cluster_, COLL_UNIT), g, a, status, done);
+cudaError_t COLL_CAT(launch_pass_, COLL_UNIT)(const GroupPass& g, int ctas, cudaStream_t stream) {
+#ifdef COLL_UNIT_MOVE
+  return launch_pass_kernel(k_coll_pass_move, g, ctas, stream);
+#else
+  switch (g.a.dtype) {
+#define COLL_CASE(code, T) case code: return launch_pass_kernel(COLL_CAT(k_coll_pass_, COLL_UNIT)<T>, g, ctas, stream);
+    COLL_TYPES(COLL_CASE)
+#undef COLL_CASE
+  }
+  return cudaErrorInvalidValue;
+#endif
 }
 
 void COLL_CAT(preload_, COLL_UNIT)() {
   cudaFuncAttributes fa;
-  cudaFuncGetAttributes(&fa, COLL_CAT(k_coll_cluster_, COLL_UNIT));
+#ifdef COLL_UNIT_MOVE
+  cudaFuncGetAttributes(&fa, k_coll_pass_move);
+#else
+#define COLL_CASE(code, T) cudaFuncGetAttributes(&fa, COLL_CAT(k_coll_pass_, COLL_UNIT)<T>);
+  COLL_TYPES(COLL_CASE)
+#undef COLL_CASE
+#endif
   cudaFuncGetAttributes(&fa, COLL_CAT(k_coll_, COLL_UNIT));
   cudaFuncGetAttributes(&fa, COLL_CAT(k_coll_group_, COLL_UNIT));
   if (kDynSmem) {      // per device: the caller has made the PE's device current
     cudaFuncSetAttribute(COLL_CAT(k_coll_, COLL_UNIT), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
     cudaFuncSetAttribute(COLL_CAT(k_coll_group_, COLL_UNIT), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
-    cudaFuncSetAttribute(COLL_CAT(k_coll_cluster_, COLL_UNIT), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
   }
 }
 

@@ -437,6 +437,7 @@ class GpuBackend final : public Backend {
     int sms = 0;
     RT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, heap_->device));
     if (coll_ctas_ > sms) coll_ctas_ = sms;
+    sms_ = sms;
     return BSHMEM_OK;
   }
 
@@ -763,7 +764,7 @@ class GpuBackend final : public Backend {
     if (heap_->mode == gpu::HEAP_LOCAL_GROUP) {
       // PEs of a local group share one GPU: a per-PE launch that waits for the others must not
       // exist.  Host syncs are no-ops (the caller owns ordering); data collectives go through
-      // bshmem_gpu_group_collective, which runs all PEs in one cooperative launch.
+      // bshmem_gpu_group_collective, which runs all PEs in one launch.
       if (a.kind == BSHMEM_COLL_SYNC || a.kind == BSHMEM_COLL_BARRIER) return BSHMEM_OK;
       tl_err = std::string(what) + ": use the group collective entry for a local group";
       return BSHMEM_ERR_UNSUPPORTED;
@@ -911,34 +912,38 @@ class GpuBackend final : public Backend {
 
   int* dstatus() const { return dstatus_; }
 
-  // A collective of the local group whose first PE this is.  The PE table stays on the device and is rewritten only when
-  // it differs from the last call's; completion and status come back through pinned words.  (With a table allocated,
+  // A collective of the local group whose first PE this is: one pass over all members' memory where every member of the team is
+  // here and the call's blocks fit the device one to a multiprocessor, else the multi-PE algorithms in a cooperative launch (which
+  // turns away what does not fit).  The PE table of that one stays on the device and is rewritten only when it differs
+  // from the last call's; completion and status come back through pinned words.  (With a table allocated,
   // copied and freed per call and a synchronous read of the status, the call cost 40 us around a 16 us kernel.)
   int group_launch(const State* hs, const DTeam* ht, int n, const CollArgs& a, int ctas) {
     std::lock_guard<std::mutex> lock(group_mu_);
-    bool all = true;
-    for (int i = 0; i < n; ++i) all = all && ht[i].my_idx >= 0 && ht[i].size == n;
     const Ticket t(&lanes_[0]);
     int* status = &pinned_->status[t.slot];
     *status = 0;
     collk::GroupDone done;
     done.word = t.done.word;
     done.token = t.done.token;
-    auto cluster = [&] {
-      const cudaError_t e = collk::launch_cluster(hs, ht, a, ctas, n, status, stream_, done);
+    if (!group_dev_) {
+      // on the stream of the launch: it may be one that does not wait for the default stream
+      char* mem = nullptr;
+      RT_TRY(cudaMalloc(&mem, sizeof(GroupTable) + 16));
+      const cudaError_t e = cudaMemsetAsync(mem, 0, sizeof(GroupTable) + 16, stream_);
+      if (e != cudaSuccess) { cudaFree(mem); RT_TRY(e); }
+      group_dev_ = mem;
+      memset(&group_host_, 0, sizeof(group_host_));
+    }
+    done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
+    collk::GroupPass pass;
+    auto one_pass = [&] {
+      pass.a = a;
+      pass.done = done;
+      const cudaError_t e = collk::launch_pass(pass, ctas, stream_);
       if (e != cudaSuccess) cudaGetLastError();      // not for somebody's next launch
       return e == cudaSuccess ? (int)BSHMEM_OK : (int)BSHMEM_ERR_CUDA;
     };
     auto cooperative = [&]() -> int {
-      if (!group_dev_) {
-        // on the stream of the launch: it may be one that does not wait for the default stream
-        char* mem = nullptr;
-        RT_TRY(cudaMalloc(&mem, sizeof(GroupTable) + 16));
-        const cudaError_t e = cudaMemsetAsync(mem, 0, sizeof(GroupTable) + 16, stream_);
-        if (e != cudaSuccess) { cudaFree(mem); RT_TRY(e); }
-        group_dev_ = mem;
-        memset(&group_host_, 0, sizeof(group_host_));
-      }
       GroupTable img;
       memset(&img, 0, sizeof(img));
       memcpy(img.states, hs, sizeof(State) * n);
@@ -948,14 +953,13 @@ class GpuBackend final : public Backend {
         group_host_ = img;
       }
       GroupTable* dev = reinterpret_cast<GroupTable*>(group_dev_);
-      done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
       const cudaError_t e = collk::launch_group(dev->states, dev->teams, a, ctas, n, status, stream_, done);
       if (e == cudaSuccess) return BSHMEM_OK;
       cudaGetLastError();        // reported here, not at somebody's next launch
       tl_err = std::string("cooperative launch: ") + cudaGetErrorString(e);
       return BSHMEM_ERR_CUDA;
     };
-    int rc = launch_preferred(all && ctas * n <= collk::kClusterBlocks, (int)BSHMEM_OK, cluster, cooperative);
+    int rc = launch_preferred(ctas * n <= sms_ && passes(hs, ht, n, a, &pass), (int)BSHMEM_OK, one_pass, cooperative);
     if (rc == BSHMEM_OK) rc = wait_done(t, stream_);
     if (rc != BSHMEM_OK || *status == BSHMEM_OK) return rc;
     tl_err = std::string("device-side ") + bshmem_status_string(*status);
@@ -963,6 +967,35 @@ class GpuBackend final : public Backend {
   }
 
  private:
+  // Whether a group's collective can run as one pass (and over which members): every member of the team is here, they agree on where each
+  // of them lives, and the call is one that the pass knows.  What does not fit keeps its own answer from the general form, errors included.
+  static bool passes(const State* hs, const DTeam* ht, int n, const CollArgs& a, collk::GroupPass* pass) {
+    if (!collk::pass_kind(a.kind)) return false;
+    int size = 0, found = 0, slot = -1;
+    bool seen[BSHMEM_MAX_PES] = {};
+    for (int i = 0; i < n; ++i) {
+      const int k = ht[i].my_idx;
+      if (k < 0) continue;
+      if (found++ == 0) { size = ht[i].size; slot = ht[i].slot; }
+      if (size < 1 || size > BSHMEM_MAX_PES || k >= size || seen[k] || ht[i].size != size || ht[i].slot != slot || slot < 0) return false;
+      seen[k] = true;
+      pass->base[k] = hs[i].heap_base[hs[i].my_pe];
+      pass->stats[k] = hs[i].stats;
+      pass->pe[k] = hs[i].my_pe;
+      if (!hs[i].one_gpu || reinterpret_cast<uintptr_t>(pass->base[k]) & 15) return false;
+    }
+    if (found == 0 || found != size) return false;
+    const bool rooted = a.kind == BSHMEM_COLL_BROADCAST || a.kind == BSHMEM_COLL_REDUCE_ROOT;
+    if (rooted && (a.root < 0 || a.root >= size)) return false;
+    for (int i = 0; i < n; ++i)
+      for (int k = 0; k < size && ht[i].my_idx >= 0; ++k) {
+        const int pe = ht[i].pe_start + k * ht[i].stride;
+        if (pe < 0 || pe >= hs[i].n_pes || hs[i].heap_base[pe] != pass->base[k]) return false;
+      }
+    pass->size = size;
+    return true;
+  }
+
   struct GroupTable {
     State states[BSHMEM_MAX_PES];
     DTeam teams[BSHMEM_MAX_PES];
@@ -979,7 +1012,7 @@ class GpuBackend final : public Backend {
   int* dstatus_ = nullptr;
   bool blocking_ = true;
   bool use_nvls_ = false;
-  int coll_ctas_ = 32;
+  int coll_ctas_ = 32, sms_ = 0;
   Lane lanes_[BSHMEM_MAX_CTXS];
   unsigned long long ll_epoch_ = 0;     // epochs of host-launched low-latency allreduces
   unsigned long long stage_seq_ = 0;    // call numbers of staged one-exchange collectives
@@ -1227,7 +1260,7 @@ int bshmem_gpu_ctx_put_signal_dev(bshmem_handle_t h, bshmem_ctx_t c, void* dest,
              : bshmem_ctx_putmem_signal(h, c, dest, src, n, sig, value, sig_op, pe);
 }
 
-// One collective for a whole local group in a single cooperative launch (single-GPU emulation).
+// One collective for a whole local group in a single launch.
 // handles[n]: the group's runtimes; team_slot: the team to run on (every member passes the same
 // offsets, as with any symmetric call).
 int bshmem_gpu_group_collective(bshmem_handle_t* handles, int n, int team_slot, int kind, int dtype, int op, int root,

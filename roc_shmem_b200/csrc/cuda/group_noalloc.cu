@@ -1,8 +1,8 @@
 // group_noalloc.cu — bshmem_gpu_group_collective_noalloc(): the group collective for
 // callers that must not allocate device memory.  See bshmem_gpu_noalloc.h for who those
 // callers are and for the limits; this file holds the fixed scratch array, its one-time
-// address look-up and the launch (of the same cooperative kernels the allocating entry runs,
-// coll_kernels.h, handed pointers into the array).
+// address look-up and the launch (of the cooperative kernels, in which the PEs
+// exchange flags as PEs on several GPUs do; coll_kernels.h, handed pointers into the array).
 #include <cuda_runtime.h>
 
 #include <cstring>

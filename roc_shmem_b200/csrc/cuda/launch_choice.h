@@ -4,8 +4,7 @@
 namespace bshmem {
 
 // The preferred form where it fits and the device accepts it, the general one otherwise: a form that is only the faster one does not
-// turn a call away that the other can serve (a cluster of eight blocks with their shared memory needs eight free
-// multiprocessors of one GPC, which a partition of the device may not have).
+// turn a call away that the other can serve.
 template <class Status, class Preferred, class General>
 Status launch_preferred(bool fits, Status success, Preferred preferred, General general) {
   if (fits && preferred() == success) return success;

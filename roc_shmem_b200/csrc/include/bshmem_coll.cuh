@@ -110,22 +110,8 @@ __device__ __forceinline__ int team_sync_mc(const State& s, const Team& t, int c
   return rc;
 }
 
-// All members' blocks in one cluster (BSHMEM_ONE_CLUSTER): the hardware's barrier, which every block reaches because none of them
-// waits for anything else.  A flag exchange through memory takes 2 us, this 0.3.
-__device__ __forceinline__ int team_sync_cluster(const State& s) {
-  const unsigned long long t0 = s.stats ? dev::timer() : 0;
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (threadIdx.x == 0 && s.stats) {
-    dev::stat(s, BSHMEM_DSTAT_BARRIER);
-    dev::stat(s, BSHMEM_DSTAT_BARRIER_NS, dev::timer() - t0);
-    dev::trace(s, BSHMEM_TRACE_BARRIER, s.my_pe, dev::timer() - t0);
-  }
-  return BSHMEM_OK;
-}
-
 __device__ __forceinline__ int team_sync(const State& s, const Team& t, int cta = 0) {
   if (t.slot < 0) return active_set_sync(s, t);
-  if (s.one_gpu == BSHMEM_ONE_CLUSTER) return team_sync_cluster(s);
   if (t.slot == 0 && t.size == s.n_pes && s.mc_base != nullptr && s.n_pes > 1) return team_sync_mc(s, t, cta);
   __shared__ int sync_status;
   const int tid = threadIdx.x;
@@ -598,9 +584,8 @@ __device__ __forceinline__ int team_reduce_ll(const State& s, const Team& t, int
 template <typename T>
 __device__ __forceinline__ int team_reduce(const State& s, const Team& t, int op, T* dest, const T* source, size_t n,
                                            int cta = 0, int ncta = 1, unsigned long long ll_epoch = 0, char* bulk = nullptr) {
-  // small vectors on the world team: one exchange (the condition is the same on every PE: symmetric addresses); blocks of one
-  // cluster read each other's vectors at once
-  if (s.one_gpu != BSHMEM_ONE_CLUSTER && (n * sizeof(T)) % (sizeof(T) > 4 ? sizeof(T) : 4) == 0 && n > 0 &&
+  // small vectors on the world team: one exchange (the condition is the same on every PE: symmetric addresses)
+  if ((n * sizeof(T)) % (sizeof(T) > 4 ? sizeof(T) : 4) == 0 && n > 0 &&
       ((reinterpret_cast<uintptr_t>(dest) | reinterpret_cast<uintptr_t>(source)) & (sizeof(T) > 4 ? 7 : 3)) == 0) {
     if (t.slot == 0 && t.size == s.n_pes) {
       if (ncta == 1 && n * sizeof(T) <= BSHMEM_LL_PAYLOAD_BYTES) return team_reduce_ll<T>(s, t, op, dest, source, n);

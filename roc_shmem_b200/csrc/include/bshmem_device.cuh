@@ -84,9 +84,6 @@ typedef struct {
   uint32_t debug;
   uint32_t one_gpu;                    /* every PE lives on this GPU: GPU scope orders accesses for all of them */
 } bshmem_dev_state_t;
-/* Value of one_gpu that only a kernel's own copy of the state has: the blocks of all PEs are one thread-block cluster, its
- * barrier synchronises them. */
-#define BSHMEM_ONE_CLUSTER 2u
 
 enum {
   BSHMEM_DSTAT_PUT = 0, BSHMEM_DSTAT_GET, BSHMEM_DSTAT_PUT_SIGNAL, BSHMEM_DSTAT_P, BSHMEM_DSTAT_G, BSHMEM_DSTAT_AMO,

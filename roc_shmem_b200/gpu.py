@@ -489,8 +489,11 @@ def init_device_runtime(boot: Bootstrap, cfg: Config, device: Optional[int] = No
 class LocalGroup:
     """All PEs of a job inside ONE process on ONE GPU — for tests on a single
     device.  Host RMA/atomics work per PE as usual; collectives and team splits
-    run for the whole group at once (one cooperative launch), because kernels
-    that wait on one another must never be separate launches on one GPU."""
+    run for the whole group at once (one launch), because kernels
+    that wait on one another must never be separate launches on one GPU.
+    Collectives that move data are one pass over all members' memory, without
+    the barriers of PEs on several GPUs (their device counters count none);
+    `bshmem_gpu_group_collective_noalloc` runs those algorithms as they are."""
 
     def __init__(self, n_pes: int, heap_bytes: int = 64 << 20, device: int = 0, config: Optional[Config] = None):
         self.lib = cuda_lib()

@@ -1,5 +1,4 @@
-"""Group collectives whose blocks are one cluster (at most eight blocks of all PEs together) against the cooperative launch of the same
-call (more blocks) at odd sizes, for every kind, with results in place of the sources, and in a team that leaves PEs out."""
+"""Group collectives of at most eight blocks of all PEs together against the same call with more blocks, at odd sizes, for every kind, with results in place of the sources, and in a team that leaves PEs out."""
 import pytest
 import torch
 
