@@ -20,6 +20,9 @@
 //               expects two arrivals (a load without the cta_group qualifier can only
 //               signal a barrier of the CTA it writes to)
 //   warps 2-9   epilogue: warp w drains TMEM lanes 32*(w%4).., columns 128*(w>=6)..
+// Producer, issuer and relay are loops of their whole warp; one elected lane issues (see ptx::elect_one): a k-block then takes the 512
+// cycles of its MMAs, where from a lane in a branch of its own the issue and the wait took 565.  Long launches gain less, since the power cap
+// takes the clock down: 8192 x 8192 x 3584 341 -> 339 us, training of 1000 x 8192 -> 7168 296 -> 290, the 8192-token MLP step 3387 -> 3333.
 //
 // tcgen05.commit (with its cluster-multicast form, a barrier arrival, not a load) hands
 // stages and accumulators back to BOTH CTAs.
@@ -181,6 +184,11 @@ __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, Guard& 
     }
   }
   return true;
+}
+
+// The same by a whole warp: one answer for all lanes, so that the warp stays together.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, Guard& g, int site) {
+  return __all_sync(0xffffffffu, pair_wait(bar, parity, g, site));
 }
 
 // Shared-memory carve-up (shared-window byte addresses).
@@ -447,31 +455,33 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      bool ok = true;
-      const uint32_t tx = P::stage_tx(prm);
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int m_blk, n_blk, kb0, kb1;
-        P::tile_coords(prm, tile, &m_blk, &n_blk);
-        if (!P::a_ready(prm, m_blk, g)) break;
-        kb_range(m_blk, &kb0, &kb1);
-        const int a_row = P::a_row(prm, m_blk) + (int)rank * CTA_M;
-        const int b_row = P::b_row(prm, m_blk, n_blk) + (int)rank * (cols0 / 2);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!pair_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    bool ok = true;
+    const uint32_t tx = P::stage_tx(prm);
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      int m_blk, n_blk, kb0, kb1;
+      P::tile_coords(prm, tile, &m_blk, &n_blk);
+      if (!__all_sync(0xffffffffu, !leader || P::a_ready(prm, m_blk, g))) break;
+      kb_range(m_blk, &kb0, &kb1);
+      const int a_row = P::a_row(prm, m_blk) + (int)rank * CTA_M;
+      const int b_row = P::b_row(prm, m_blk, n_blk) + (int)rank * (cols0 / 2);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!warp_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
+        if (leader) {
           ptx::mbar_arrive_expect_tx(L.full(s), tx);
           P::load_stage(prm, P::map_a(prm), P::map_b(prm), a_smem(s), b_smem(s), L.full(s), kb, a_row, b_row, m_blk, n_blk, (int)rank);
           if constexpr (P::kWide)
             P::load_b(prm, P::map_b(prm), b_smem(s) + B_STAGE_BYTES, L.full(s), kb,
                       P::b_row(prm, m_blk, n_blk) + cols0 + (int)rank * (cols1 / 2), m_blk, n_blk, (int)rank);
-          if (++s == kStages) { s = 0; ph ^= 1; }
         }
+        if (++s == kStages) { s = 0; ph ^= 1; }
       }
-      ptx::grid_launch_dependents();       // all loads are on their way: the next kernel's blocks may take their places
     }
+    if (leader) ptx::grid_launch_dependents();       // all loads are on their way: the next kernel's blocks may take their places
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    const bool leader = ptx::elect_one();
+    if (rank == 0) {
       // ------------------------------ MMA issuer (first CTA) ---------------------------------
       int s = 0; uint32_t ph = 0;
       uint32_t acc_ph = 0;          // bit a = phase of accumulator a
@@ -482,18 +492,18 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
       const uint32_t idesc0 = P::kVarCols ? (P::kIdesc & kNoN) | (uint32_t)(cols0 >> 3) << 17 : P::kIdesc;
       const uint32_t idesc1 = P::kVarCols ? (P::kIdesc & kNoN) | (uint32_t)(cols1 >> 3) << 17 : P::kIdesc;
       auto wait_acc = [&](int acc) {     // the epilogue warps of both CTAs must have drained it
-        if (!pair_wait(L.tmem_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_MMA_TMEM_EMPTY)) return false;
+        if (!warp_wait(L.tmem_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_MMA_TMEM_EMPTY)) return false;
         acc_ph ^= 1u << acc;
         ptx::tc_fence_after();
         return true;
       };
       auto wait_stage = [&](int st, uint32_t parity) {
-        if (!pair_wait(L.full(st), parity, g, ERR_MMA_FULL)) return false;
+        if (!warp_wait(L.full(st), parity, g, ERR_MMA_FULL)) return false;
         ptx::tc_fence_after();
         return true;
       };
-      // one k-block into one accumulator; which = 1: the second one's rows of B.  Descriptors differ only in the
-      // 16-byte-unit start address (low 14 bits; shared memory is < 256 KiB).
+      // What the leader does.  One k-block into one accumulator; which = 1: the second one's rows of B.  Descriptors differ only in
+      // the 16-byte-unit start address (low 14 bits; shared memory is < 256 KiB).
       auto multiply = [&](int st, int acc, int which, bool first) {
         const uint64_t da = desc_a0 + (uint64_t)((st * kStageBytes) >> 4);
         const uint64_t db = desc_b0 + (uint64_t)((st * kStageBytes + which * B_STAGE_BYTES) >> 4);
@@ -512,12 +522,14 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           if (!wait_acc(acc)) break;                   // drained two tiles ago
           for (int kb = kb0; kb < kb1; ++kb) {
             if (!wait_stage(s, ph)) { ok = false; break; }
-            multiply(s, acc, 0, kb == kb0);
-            umma2_commit_both(L.empty(s), lead);       // stage reusable in both CTAs once these MMAs retire
+            if (leader) {
+              multiply(s, acc, 0, kb == kb0);
+              umma2_commit_both(L.empty(s), lead);     // stage reusable in both CTAs once these MMAs retire
+            }
             if (++s == kStages) { s = 0; ph ^= 1; }
           }
           if (!ok) break;
-          umma2_commit_both(L.tmem_full(acc), lead);
+          if (leader) umma2_commit_both(L.tmem_full(acc), lead);
         } else {
           // `count` stages into accumulator 0, then into accumulator 1, which hands them back.  The first and the last
           // k-blocks of a tile go in batches: while accumulator 1 takes its last k-blocks, the epilogue
@@ -527,17 +539,19 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
             int t = s; uint32_t tph = ph;
             for (int i = 0; i < count; ++i) {
               if (!wait_stage(t, tph)) return false;
-              multiply(t, 0, 0, begin && i == 0);
+              if (leader) multiply(t, 0, 0, begin && i == 0);
               if (++t == kStages) { t = 0; tph ^= 1; }
             }
-            if (end) umma2_commit_both(L.tmem_full(0), lead);
+            if (end && leader) umma2_commit_both(L.tmem_full(0), lead);
             if (begin && !wait_acc(1)) return false;
             for (int i = 0; i < count; ++i) {
-              multiply(s, 1, 1, begin && i == 0);
-              umma2_commit_both(L.empty(s), lead);
+              if (leader) {
+                multiply(s, 1, 1, begin && i == 0);
+                umma2_commit_both(L.empty(s), lead);
+              }
               if (++s == kStages) { s = 0; ph ^= 1; }
             }
-            if (end) umma2_commit_both(L.tmem_full(1), lead);
+            if (end && leader) umma2_commit_both(L.tmem_full(1), lead);
             return true;
           };
           // in between, both accumulators take a k-block together: A is read once for the two
@@ -558,8 +572,10 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
             ok = batch(WIDE_BATCH, true, false);
             for (int i = n - WIDE_BATCH - last; i > 0 && ok; --i) {
               if (!wait_stage(s, ph)) { ok = false; break; }
-              multiply_both(s);
-              umma2_commit_both(L.empty(s), lead);
+              if (leader) {
+                multiply_both(s);
+                umma2_commit_both(L.empty(s), lead);
+              }
               if (++s == kStages) { s = 0; ph ^= 1; }
             }
             ok = ok && batch(last, false, true);
@@ -567,7 +583,7 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
         }
       }
     }
-    else if (lane == 0) {
+    else {
       // ------------------------------ relay (second CTA) --------------------------------------
       int s = 0; uint32_t ph = 0;
       bool ok = true;
@@ -576,8 +592,8 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
         P::tile_coords(prm, tile, &m_blk, &n_blk);
         kb_range(m_blk, &kb0, &kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!pair_wait(L.full(s), ph, g, ERR_RELAY_FULL)) { ok = false; break; }
-          mbar_arrive_cluster(mapa(L.full(s), lead));
+          if (!warp_wait(L.full(s), ph, g, ERR_RELAY_FULL)) { ok = false; break; }
+          if (leader) mbar_arrive_cluster(mapa(L.full(s), lead));
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
       }

@@ -55,6 +55,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 // Per-thread asynchronous copies, global -> shared; each thread waits for its own groups.
+// Whether the phase is complete now.  An answer takes some 100 cycles, so it can be asked for ahead of what needs it.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// One lane of a warp that is here as a whole.  A role that issues tensor-core and TMA instructions is a loop of the whole warp, the waits
+// included, with only the instructions themselves under this: what they take stays in uniform registers.  In a branch of one lane
+// each tcgen05.mma costs that lane 63 cycles (four and a commit 289, so 102), and the loop around it more than the MMAs' own time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
