@@ -100,6 +100,7 @@ struct Fp8Params {
   int split;
   int first_tile, end_tile;    // the launch's share of the tiles (plain and split form)
   int behind;                  // split form, launched behind the plain one for the last tiles of the same product
+  int halves;                  // split form: blocks and tiles are those of CTA pairs, `tile` counts their halves of 128 rows
   Fp8Ag ag;                    // used by the all-gather variant only
 };
 struct Fp8RsParams {
@@ -114,7 +115,10 @@ enum : int { ERR_F8_A_READY = 123, ERR_F8_PEER_READY = 124, ERR_F8_PEER_DONE = 1
 // rank me+1, me+2, ... which is also the order in which the pull warps fetch them.
 template <int kMode>
 __device__ __forceinline__ void f8_tile_coords(const Fp8Params& p, const Fp8Rs* rs, int tile, int* m_blk, int* n_blk) {
-  if constexpr (kMode == F8_PLAIN || kMode == F8_SPLIT) {
+  if constexpr (kMode == F8_SPLIT) {
+    raster_coords(p.core, tile >> p.halves, m_blk, n_blk);
+    if (p.halves) *m_blk = 2 * *m_blk + (tile & 1);
+  } else if constexpr (kMode == F8_PLAIN) {
     raster_coords(p.core, tile, m_blk, n_blk);
   } else if constexpr (kMode == F8_RS) {
     // owner-major, owners visited in the order me+1, me+2, ..., me: the P ranks always write to P different owners
@@ -620,6 +624,10 @@ __global__ void __launch_bounds__(FNUM_THREADS, 1) gemm_rs_fp8_kernel(const __gr
   gemm_fp8_body<F8_RS>(prm.base, &prm.rs, smem_raw);
 }
 
+}  // namespace
+#include "gemm_fp8_pair.cuh"
+namespace {
+
 // ---- quantisers ------------------------------------------------------------------------------
 __device__ __forceinline__ uint8_t to_e4m3(float x) {
   return (uint8_t)__nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3);
@@ -759,6 +767,7 @@ __global__ void quant_w_128x128_kernel(const __nv_bfloat16* __restrict__ w, int 
 int* g_err_dev[64] = {};
 int g_sms[64] = {};
 int g_clusters[64][3] = {};    // clusters of 2 / 4 / 8 CTAs of the split form that the device holds at once
+int g_pairs[64] = {};          // CTA pairs, 0: none (the kernel's registers do not make up what its warps hand each other)
 
 struct AgPlan {
   bshmem_dev_state_t st;
@@ -800,6 +809,11 @@ int ensure(int dev) {
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_fp8_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
   for (int i = 0; i < 3; ++i)
     g_clusters[dev][i] = gemm2::max_resident_clusters(gemm_fp8_split_kernel, g_sms[dev], 2 << i, FPLAIN_THREADS, FSMEM_BYTES);
+  BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PSMEM_BYTES));
+  cudaFuncAttributes fa;
+  BSHMEM_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm_fp8_pair_kernel));
+  if (fa.numRegs == PREGS_LAUNCH)
+    g_pairs[dev] = gemm2::max_resident_clusters(gemm_fp8_pair_kernel, g_sms[dev], 2, PTHREADS, PSMEM_BYTES);
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(ag_gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
   BSHMEM_CUDA_TRY(cudaFuncSetAttribute(gemm_rs_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM_BYTES));
   return 0;
@@ -851,40 +865,72 @@ int bshmem_gemm_fp8_blockscale(const void* A8, const float* scale_a, const void*
   if (max_ctas <= 0)
     for (int i = 2; i >= 0; --i)
       if (tiles <= g_clusters[dev][i] && K / FBK >= 4 * (2 << i)) { p.split = 2 << i; break; }
-  // Whole waves of tiles, then a last wave that is partly empty: its tiles go to a launch of the split form behind this one, if
-  // that saves 12 of a CTA's k-blocks (some 6 us; parking and adding the parts takes about 4).  4096 x 7168 x 8192 has 896 tiles for
-  // 148 SMs, 6.05 waves: with the quantiser 292 us became 280.
-  const int rest = tiles % ctas, kb = K / FBK;
-  int rest_split = 1;
-  if (max_ctas <= 0 && p.split == 1 && tiles > ctas && rest)
-    for (int i = 2; i >= 0 && rest_split == 1; --i) {
-      const int n = 2 << i;
-      if (rest <= g_clusters[dev][i] && kb >= 4 * n && kb * (n - 1) / n >= 12) rest_split = n;
-    }
-  p.end_tile = rest_split > 1 ? tiles - rest : tiles;
-  auto launch = [&](int clusters, int split) -> int {
+  // What a wave holds of the tiles is units: CTAs, or pairs and their tiles of 256 rows.  Whole waves, then a last one that is partly
+  // empty: its tiles go to a launch of the split form behind this one, if that saves 12 of a CTA's k-blocks (some 6 us; parking and
+  // adding the parts takes about 4).  4096 x 7168 x 8192 has 896 tiles for 148 SMs, 6.05 waves: with the quantiser 292 us became 280.
+  const int kb = K / FBK;
+  struct Form { int units, tiles, rest, rest_split; float waves; };
+  auto form = [&](bool pair) {
+    Form f;
+    f.tiles = pair ? (M + 2 * FBM - 1) / (2 * FBM) * p.core.num_n_blocks : tiles;
+    f.units = pair ? (ctas / 2 < g_pairs[dev] ? ctas / 2 : g_pairs[dev]) : ctas;
+    if (f.units > f.tiles) f.units = f.tiles;
+    f.rest = f.tiles % f.units << (pair ? 1 : 0);               // in tiles of 128 rows
+    f.rest_split = 1;
+    if (max_ctas <= 0 && f.tiles > f.units && f.rest && (!pair || M % (2 * FBM) == 0))
+      for (int i = 2; i >= 0 && f.rest_split == 1; --i) {
+        const int n = 2 << i;
+        if (f.rest <= g_clusters[dev][i] && kb >= 4 * n && kb * (n - 1) / n >= 12) f.rest_split = n;
+      }
+    f.waves = (float)(f.tiles / f.units) + (f.rest == 0 ? 0.f : f.rest_split > 1 ? 1.f / f.rest_split + 24.f / kb : 1.f);
+    return f;
+  };
+  // Pairs where they can work (reductions in whole groups, scales that can be copied in bulk) and their wave, which takes 0.85 of the
+  // time of the other's (four shapes of two waves and more, 0.81 to 0.88), makes up for tiles that halve less evenly: 640 x 14336 x 4096, three waves
+  // of pairs and two of CTAs, would take 56 us for 47; 1024 x 7168 x 8192, two and two, takes 70 for 77.
+  bool pairs = false;
+  Form f = form(false);
+  if (p.split == 1 && g_pairs[dev] > 0 && ctas >= 2 && K % (FBK * PGROUP) == 0 && !(reinterpret_cast<uintptr_t>(scale_a) & 15)) {
+    const Form fp = form(true);
+    if (fp.waves * 0.85f <= f.waves) { f = fp; pairs = true; }
+  }
+  if (p.split == 1 && pairs) {
+    p.core.num_m_blocks = (M + 2 * FBM - 1) / (2 * FBM);
+    p.core.group_m = 16;
+    rc = host::make_tmap_2d(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B8, N, K, K, 64, FBK);
+    if (rc) return rc;
+  }
+  const int rest_split = p.split == 1 ? f.rest_split : 1;
+  p.end_tile = p.split > 1 ? tiles : rest_split > 1 ? f.tiles - f.tiles % f.units : f.tiles;
+  auto launch = [&](int clusters, int split, bool pair) -> int {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(clusters * split));
-    cfg.blockDim = dim3(FPLAIN_THREADS);
-    cfg.dynamicSmemBytes = FSMEM_BYTES;
+    const int size = pair ? 2 : split;
+    cfg.gridDim = dim3((unsigned)(clusters * size));
+    cfg.blockDim = dim3(pair ? PTHREADS : FPLAIN_THREADS);
+    cfg.dynamicSmemBytes = pair ? PSMEM_BYTES : FSMEM_BYTES;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.x = (unsigned)size; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = split > 1 ? 2 : 1;
-    BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, split > 1 ? gemm_fp8_split_kernel : gemm_fp8_blockscale_kernel, p));
+    cfg.numAttrs = size > 1 ? 2 : 1;
+    BSHMEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair ? gemm_fp8_pair_kernel : split > 1 ? gemm_fp8_split_kernel : gemm_fp8_blockscale_kernel, p));
     return 0;
   };
-  rc = launch(ctas, p.split);
+  rc = launch(p.split == 1 ? f.units : ctas, p.split, pairs);
   if (rc || rest_split == 1) return rc;
-  p.first_tile = tiles - rest;
-  p.end_tile = tiles;
+  if (pairs) {
+    rc = host::make_tmap_2d(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B8, N, K, K, FBN, FBK);
+    if (rc) return rc;
+    p.halves = 1;
+  }
+  p.first_tile = p.end_tile << p.halves;
+  p.end_tile = f.tiles << p.halves;
   p.split = rest_split;
   p.behind = 1;
-  return launch(rest, rest_split);
+  return launch(f.rest, rest_split, false);
 }
 
 // x: [M, K] bf16 (ldx elements, % 4 == 0, 8-byte aligned rows) -> q [M, K] e4m3 + scales; the scale of row m and
