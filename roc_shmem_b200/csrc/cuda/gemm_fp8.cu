@@ -20,7 +20,8 @@
 // What bounds it is the life of a product (MMAs, commit, barrier, tensor-memory load, release):
 // about 0.5 us per k-block with two of them on their way.  4096 x 7168 x 8192 takes 235 us; with
 // the scales fetched into registers, where every use of the queue waited for an L2 round trip, it
-// took 272.  CTA pairs on 256x256 or 256x128 tiles (half the loads of B) were slower, 245 and 398 us.
+// took 272.  CTA pairs whose promotion never waits for what it could have asked for take 207
+// (gemm_fp8_pair.cuh), and most products go to them.
 // Every wait is bounded (see gemm_core.cuh); there is no counterpart in the reference.
 #include <cuda_fp8.h>
 
@@ -361,41 +362,49 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
     }
   } else if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      bool ok = true;
-      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-        int m_blk, n_blk;
-        f8_tile_coords<kMode>(prm, rs, tile, &m_blk, &n_blk);
-        if constexpr (kAG) {
-          if (m_blk / prm.ag.blocks_per_rank != prm.ag.my_rank) {
-            if (!wait_ge<false>(prm.ag.arrived + m_blk, (unsigned long long)prm.ag.pieces_per_block * prm.ag.call, g, ERR_F8_A_READY)) break;
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+      int m_blk, n_blk;
+      f8_tile_coords<kMode>(prm, rs, tile, &m_blk, &n_blk);
+      if constexpr (kAG) {
+        if (m_blk / prm.ag.blocks_per_rank != prm.ag.my_rank) {
+          bool arrived = true;
+          if (leader) {
+            arrived = wait_ge<false>(prm.ag.arrived + m_blk, (unsigned long long)prm.ag.pieces_per_block * prm.ag.call, g, ERR_F8_A_READY);
             ptx::fence_proxy_async_all();
           }
+          if (!__all_sync(0xffffffffu, arrived)) break;
         }
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
+      }
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!gemm2::warp_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) { ok = false; break; }
+        if (leader) {
           ptx::mbar_arrive_expect_tx(L.full(s), FSTAGE_BYTES);
           ptx::tma_load_2d(L.a(s), &prm.map_a, L.full(s), (kb0 + kb) * FBK, m_blk * FBM);
           ptx::tma_load_2d(L.b(s), &prm.map_b, L.full(s), (kb0 + kb) * FBK, n_blk * FBN);
-          if (++s == FSTAGES) { s = 0; ph ^= 1; }
         }
+        if (++s == FSTAGES) { s = 0; ph ^= 1; }
       }
-      if constexpr (kMode == F8_PLAIN || kSplit) ptx::grid_launch_dependents();
+    }
+    if constexpr (kMode == F8_PLAIN || kSplit) {
+      if (leader) ptx::grid_launch_dependents();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      uint32_t it = 0;                       // k-blocks issued so far: buffer = it & 1, use count = it >> 1
-      bool ok = true;
-      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int buf = it & 1;
-          // the epilogue must have drained this buffer's previous product
-          if (!mbar_wait(L.part_empty(buf), ((it >> 1) & 1) ^ 1, g, ERR_F8_PART_EMPTY)) { ok = false; break; }
-          if (!mbar_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
-          ptx::tc_fence_after();
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    uint32_t it = 0;                       // k-blocks issued so far: buffer = it & 1, use count = it >> 1
+    bool ok = true;
+    for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        const int buf = it & 1;
+        // the epilogue must have drained this buffer's previous product
+        if (!gemm2::warp_wait(L.part_empty(buf), ((it >> 1) & 1) ^ 1, g, ERR_F8_PART_EMPTY)) { ok = false; break; }
+        if (!gemm2::warp_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
+        ptx::tc_fence_after();
+        if (leader) {
           const uint32_t a0 = L.a(s), b0 = L.b(s);
 #pragma unroll
           for (int k = 0; k < FBK / UMMA_K_BYTES; ++k)
@@ -403,8 +412,8 @@ __device__ __forceinline__ void gemm_fp8_body(const Fp8Params& prm, const Fp8Rs*
                              ptx::umma_desc_sw128(b0 + k * UMMA_K_BYTES), kIdescFp8, k != 0 ? 1u : 0u);
           ptx::umma_commit(L.empty(s));            // smem stage reusable once these MMAs retire
           ptx::umma_commit(L.part_full(buf));      // product of this k-block complete
-          if (++s == FSTAGES) { s = 0; ph ^= 1; }
         }
+        if (++s == FSTAGES) { s = 0; ph ^= 1; }
       }
     }
   } else {

@@ -16,6 +16,9 @@
 //   warp 0      TMA producer: {128 weight rows, nt token rows} x 64 of K per stage, plain loads of local memory
 //   warp 1      MMA issuer: tcgen05.mma.cta_group::1 M128 x N=nt x K16
 //   warps 2-5   epilogue
+// Producer and issuer are loops of their whole warp, one elected lane issues (see ptx::elect_one); from a lane in a branch of its own,
+// us: 16 x 3584 x 8192 13.05 (now 12.81), 64 x 4096 x 4096 10.8 (10.5), 100 x 2048 x 2048 7.4 (7.0), 128 x 8192 x 8192 28.5 (27.8); the grouped
+// form, 32 tokens on 8 experts of 14336: 452.5 (448.7).
 // Every wait is bounded (see gemm_core.cuh).  The reference has no GEMM, hence no counterpart.
 #pragma once
 #include "gemm_pair.cuh"
@@ -30,6 +33,7 @@ using gemm2::cluster_ctarank;
 using gemm2::cluster_sync_all;
 using gemm2::ld_cluster_f4;
 using gemm2::mapa;
+using gemm2::warp_wait;
 
 constexpr int ROWS = 128;                          // weight rows of a tile
 constexpr int BK = 64;                             // bf16 elements per k-block: one 128-byte swizzle atom
@@ -176,10 +180,11 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
 
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) break;
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!warp_wait(L.empty(s), ph ^ 1, g, ERR_PRODUCER_EMPTY)) break;
+      if (leader) {
         ptx::mbar_arrive_expect_tx(L.full(s), L.stage);
         if constexpr (kWmn) {
           ptx::tma_load_2d(L.w(s), &p.map_w, L.full(s), n0, kb * BK);
@@ -188,25 +193,26 @@ __device__ __forceinline__ void body(const Params& p, uint8_t* smem_raw) {
           ptx::tma_load_2d(L.w(s), &p.map_w, L.full(s), kb * BK, n0);
         }
         ptx::tma_load_2d(L.x(s), &p.map_x, L.full(s), kb * BK, 0);
-        if (++s == p.stages) { s = 0; ph ^= 1; }
       }
+      if (++s == p.stages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)p.nt) | (kWmn ? 1u << 15 : 0u);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
-        ptx::tc_fence_after();
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)p.nt) | (kWmn ? 1u << 15 : 0u);
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!warp_wait(L.full(s), ph, g, ERR_MMA_FULL)) { ok = false; break; }
+      ptx::tc_fence_after();
+      if (leader) {
         const uint64_t dw = kWmn ? ptx::umma_desc_sw128_ex(L.w(s), W_STAGE_BYTES / 2, 1024) : ptx::umma_desc_sw128(L.w(s));
         const uint64_t dx = ptx::umma_desc_sw128(L.x(s));
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(tmem, dw + (kWmn ? 128 : 2) * k, dx + 2 * k, idesc, (kb > kb0 || k) ? 1u : 0u);
         ptx::umma_commit(L.empty(s));
-        if (++s == p.stages) { s = 0; ph ^= 1; }
       }
-      if (ok) ptx::umma_commit(L.acc_full());
+      if (++s == p.stages) { s = 0; ph ^= 1; }
     }
+    if (ok && leader) ptx::umma_commit(L.acc_full());
   } else {
     ok = mbar_wait(L.acc_full(), 0, g, ERR_EPI_FULL);
     ptx::tc_fence_after();
@@ -394,48 +400,53 @@ __device__ __forceinline__ void grouped_body(const GroupedParams& p, uint8_t* sm
   int grp, n_blk, tok0, ntok;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      bool ok = true;
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0;
+    bool ok = true;
+    if (leader) {
       for (int q = 0; q < p.P && ok; ++q) ok = gemm::wait_ge<true>(p.arrive + q, (unsigned long long)p.expected[q], g, ERR_G_ARRIVE);
       if (p.P) ptx::fence_proxy_async_all();         // peer stores (generic proxy) before the TMA reads
-      while (ok && it.next(&grp, &n_blk, &tok0, &ntok)) {
-        const int boxes = (ntok + p.xbox - 1) / p.xbox;
-        const uint32_t box_bytes = (uint32_t)p.xbox * BK * 2;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(L.empty(s), ph ^ 1, g, ERR_G_PRODUCER_EMPTY)) { ok = false; break; }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    while (ok && it.next(&grp, &n_blk, &tok0, &ntok)) {
+      const int boxes = (ntok + p.xbox - 1) / p.xbox;
+      const uint32_t box_bytes = (uint32_t)p.xbox * BK * 2;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!warp_wait(L.empty(s), ph ^ 1, g, ERR_G_PRODUCER_EMPTY)) { ok = false; break; }
+        if (leader) {
           const uint32_t w = L.base + s * stage, x = w + W_STAGE_BYTES;
           ptx::mbar_arrive_expect_tx(L.full(s), W_STAGE_BYTES + boxes * box_bytes);
           ptx::tma_load_2d(w, &p.map_w, L.full(s), kb * BK, grp * p.N + n_blk * ROWS);
           for (int b = 0; b < boxes; ++b)
             ptx::tma_load_2d(x + b * box_bytes, &p.map_x, L.full(s), kb * BK, grp * p.cap + tok0 + b * p.xbox);
-          if (++s == stages) { s = 0; ph ^= 1; }
         }
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      ptx::grid_launch_dependents();
     }
+    if (leader) ptx::grid_launch_dependents();
   } else if (warp == 1) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0, acc_ph = 0;
-      bool ok = true;
-      for (int ord = 0; ok && it.next(&grp, &n_blk, &tok0, &ntok); ++ord) {
-        const int acc = ord & 1;
-        if (!mbar_wait(L.acc_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_G_MMA_ACC)) break;
-        acc_ph ^= 1u << acc;
+    const bool leader = ptx::elect_one();
+    int s = 0; uint32_t ph = 0, acc_ph = 0;
+    bool ok = true;
+    for (int ord = 0; ok && it.next(&grp, &n_blk, &tok0, &ntok); ++ord) {
+      const int acc = ord & 1;
+      if (!warp_wait(L.acc_empty(acc), ((acc_ph >> acc) & 1) ^ 1, g, ERR_G_MMA_ACC)) break;
+      acc_ph ^= 1u << acc;
+      ptx::tc_fence_after();
+      const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)((ntok + 15) / 16 * 16));
+      const uint32_t d = tmem + acc * p.nt_cap;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!warp_wait(L.full(s), ph, g, ERR_G_MMA_FULL)) { ok = false; break; }
         ptx::tc_fence_after();
-        const uint32_t idesc = ptx::umma_idesc(1, 1, ROWS, (uint32_t)((ntok + 15) / 16 * 16));
-        const uint32_t d = tmem + acc * p.nt_cap;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(L.full(s), ph, g, ERR_G_MMA_FULL)) { ok = false; break; }
-          ptx::tc_fence_after();
+        if (leader) {
           const uint64_t dw = ptx::umma_desc_sw128(L.base + s * stage), dx = ptx::umma_desc_sw128(L.base + s * stage + W_STAGE_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) ptx::umma_f16(d, dw + 2 * k, dx + 2 * k, idesc, (kb > kb0 || k) ? 1u : 0u);
           ptx::umma_commit(L.empty(s));
-          if (++s == stages) { s = 0; ph ^= 1; }
         }
-        if (ok) ptx::umma_commit(L.acc_full(acc));
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
+      if (ok && leader) ptx::umma_commit(L.acc_full(acc));
     }
   } else {
     const int quarter = warp & 3;
