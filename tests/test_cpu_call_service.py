@@ -1,0 +1,92 @@
+"""The protocol of served calls (csrc/cuda/call_service.h): the host's side as it is, the serving block (k_calls) as host threads that end
+when they please.  Every request is carried out once and answered, or refused and not carried out."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CUDA = Path(__file__).resolve().parents[1] / "roc_shmem_b200" / "csrc" / "cuda"
+
+MODEL = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+#include <thread>
+#include <vector>
+#include "call_service.h"
+using namespace bshmem;
+
+static CallSlot slot;
+static std::atomic<uint64_t> answer{0};
+static std::vector<std::atomic<int>> times(1 << 20);
+static auto& word(uint64_t& w) { return reinterpret_cast<std::atomic<uint64_t>&>(w); }
+
+static void block(uint32_t seq, uint32_t generation, int looks) {      // k_calls: ends after `looks` looks without a request
+  while (true) {
+    uint32_t req[kCallWords];
+    bool here = false;
+    for (int i = 0; i < looks && !here; ++i) {
+      here = true;
+      for (unsigned k = 0; k < kCallWords; ++k) {
+        const uint64_t v = word(slot.w[k]).load(std::memory_order_relaxed);
+        req[k] = (uint32_t)v;
+        here = here && (uint32_t)(v >> 32) == seq;
+      }
+      if (!here) std::this_thread::yield();
+    }
+    if (!here) break;
+    ++times[req[CALL_VALUE]];
+    answer.store((uint64_t)req[CALL_TOKEN] << 32 | (req[CALL_VALUE] ^ req[CALL_HEAD]), std::memory_order_release);
+    ++seq;
+  }
+  word(slot.final).store((uint64_t)generation << 32 | (seq - 1), std::memory_order_release);
+}
+
+int main(int, char** a) {
+  const int n = atoi(a[1]), looks = atoi(a[2]), refuse = atoi(a[3]);
+  std::vector<std::thread> blocks;
+  CallWriter w;
+  w.slot = &slot;
+  std::mt19937 rng(looks);
+  int wrong = 0, refused = 0;
+  for (int i = 0; i < n; ++i) {
+    Call call(CALL_AMO, 1, 2, 8);
+    call.set(CALL_VALUE, (uint64_t)i).set(CALL_TOKEN, (uint64_t)i + 1);
+    const bool done = w.run(call,
+        [&](uint32_t first, uint32_t generation) {
+          if (refuse && (int)(rng() % refuse) == 0) return (int)BSHMEM_ERR_CUDA;
+          blocks.emplace_back(block, first, generation, 1 + (int)(rng() % looks));
+          return (int)BSHMEM_OK;
+        },
+        [&] { return (answer.load(std::memory_order_acquire) >> 32) == (uint64_t)i + 1; },
+        [&] { for (auto& t : blocks) if (t.joinable()) t.join(); return (int)BSHMEM_OK; });
+    if (done) wrong += times[i] != 1 || (uint32_t)answer.load() != ((uint32_t)i ^ call.w[CALL_HEAD]);
+    else { ++refused; wrong += times[i] != 0; }
+    if (rng() % 8 == 0) for (unsigned k = rng() % 400; k; --k) std::this_thread::yield();
+  }
+  for (auto& t : blocks) if (t.joinable()) t.join();
+  for (int i = 0; i < n; ++i) wrong += times[i] > 1;
+  printf("wrong %d refused %s\n", wrong, refused ? "some" : "none");
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def model(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("needs a C++ compiler")
+    d = tmp_path_factory.mktemp("calls")
+    (d / "model.cc").write_text(MODEL)
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(CUDA), "-o", str(d / "model"), str(d / "model.cc"), "-lpthread"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    return lambda *a: subprocess.run([str(d / "model")] + [str(x) for x in a], capture_output=True, text=True, timeout=120)
+
+
+@pytest.mark.parametrize("calls,looks,refuse,expect", [(3000, 300, 0, "none"), (3000, 20000, 0, "none"), (2000, 200, 3, "some")])
+def test_every_call_once(model, calls, looks, refuse, expect):
+    r = model(calls, looks, refuse)
+    assert r.returncode == 0 and r.stdout == f"wrong 0 refused {expect}\n", r.stdout + r.stderr
