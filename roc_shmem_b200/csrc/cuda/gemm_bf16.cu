@@ -307,16 +307,22 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   if (pairs < 1) { host::last_error() = "gemm: the device holds no CTA pair of this kernel"; return 1; }
   // Few tiles: split each over the two or four pairs of a cluster while all clusters run at once.  Parking and adding the
-  // parts costs about 4 us, what a pair needs for 14 k-blocks.
+  // parts costs about 4 us, what a pair needs for 14 k-blocks.  Where tiles of 128 columns make one wave they are the better answer up
+  // to deeper reductions, in every layout (us, 32 / 40 / 48 / 56 / 64 k-blocks): 512 x 2048 10.9 / 12.9 / 14.6 / 16.3 / 18.0, split in
+  // two 12.9 / 14.2 / 15.5 / 16.6 / 17.8; 768 x 1024 9.6 / 11.9 / 13.7 / 15.6 / 17.2, split in four 11.1 / 12.0 / 12.9 / 13.7 / 14.4.
+  // No wider tile is better than these then: 512 x 2048 x 1536, both operands MN-major, by 128 / 160 / 192 / 224 / 256 columns
+  // 9.3 / 10.1 / 10.4 / 11.4 / 13.0.
   const int kb = (K + BK - 1) / BK;
   PlainParams p;
   p.core.split = 1;
+  const long long row_blocks = (M + BM - 1) / BM;
+  const bool one_wave = row_blocks * ((N + 127) / 128) <= pairs;
   if (max_ctas <= 1) {
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    if (tiles <= g_octs[dev] && kb >= 24) p.core.split = 4;
-    else if (tiles <= g_quads[dev] && kb >= 32) p.core.split = 2;
+    const long long tiles = row_blocks * ((N + BN - 1) / BN);
+    if (tiles <= g_octs[dev] && kb >= (one_wave ? 41 : 24)) p.core.split = 4;
+    else if (tiles <= g_quads[dev] && kb >= (one_wave ? 60 : 32)) p.core.split = 2;
   }
-  const Width w = p.core.split > 1 ? Width{{BN, 0}} : plan_width((M + BM - 1) / BM, N, K, pairs, 32, b_mn != 0);
+  const Width w = p.core.split > 1 ? Width{{BN, 0}} : one_wave ? Width{{128, 0}} : plan_width(row_blocks, N, K, pairs, 32, b_mn != 0);
   const int width = w.cols[0] + w.cols[1];
   p.core.acc_cols[0] = w.cols[0];
   p.core.acc_cols[1] = w.cols[1];
