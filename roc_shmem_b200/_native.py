@@ -87,6 +87,16 @@ def fast(lib: C.CDLL, name: str):
     return _pycall().Native(C.cast(fn, C.c_void_p).value, len(fn.argtypes), kind, pointers)
 
 
+def mover(lib: C.CDLL, name: str, handle: int, context: int, device: int, local: int, general, check):
+    """put or get of a context as a callable that reads the tensors' addresses and sizes itself (csrc/host/pycall.cc), for calls
+    (dest, src, pe, nbi=True or False) of plain tensors whose `local`-th is on `device`; anything else goes to `general`."""
+    import torch
+    table = getattr(torch.Tensor, "__dlpack_c_exchange_api__", None)
+    if table is None:                             # a torch without it
+        return general
+    return _pycall().Mover(C.cast(getattr(lib, name), C.c_void_p).value, handle, context, device, local, torch.Tensor, table, general, check)
+
+
 class _build_lock:
     """Inter-process lock around an import-time build (ranks of one job share the source tree)."""
 

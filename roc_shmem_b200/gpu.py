@@ -141,6 +141,19 @@ def _gpu_error(lib, what: str, status: int) -> None:
 class DeviceContext(Context):
     """Context of a DeviceRuntime: messages between device buffers go straight to the native call."""
 
+    def __init__(self, rt, idx, options, team):
+        super().__init__(rt, idx, options, team)
+        if type(self).put is DeviceContext.put and type(self).get is DeviceContext.get:
+            # the methods below without an interpreter's frame around them; calls of another form still come here
+            self.put = _native.mover(rt.lib, "bshmem_gpu_ctx_put_dev", rt._hv, idx, rt._dev_index, 1, self.put, rt._check)
+            self.get = _native.mover(rt.lib, "bshmem_gpu_ctx_get_dev", rt._hv, idx, rt._dev_index, 0, self.get, rt._check)
+
+    def destroy(self):
+        super().destroy()
+        for move in (self.put, self.get):             # also those that the caller keeps
+            if hasattr(move, "context"):
+                move.context = self.idx
+
     def put(self, dest, src, pe, *, nbi=False, nbytes=None):
         rt = self.rt
         if isinstance(src, Tensor) and src.get_device() == rt._dev_index and isinstance(dest, Tensor):
