@@ -61,7 +61,9 @@ inline void extent(int kind, int dtype, uint64_t count, int team_size, uint64_t*
 // One PE: `ctas` blocks on `stream`; a non-zero device status lands in *status (first one wins).
 cudaError_t launch(const State& s, const DTeam& t, const CollArgs& a, int ctas, int* status, cudaStream_t stream);
 // How a group launch tells the host that all of its blocks are done: a pinned word that receives `token`, and a device
-// counter (zero, and zero again afterwards).  word == null: the caller synchronises the stream instead.
+// counter (zero, and zero again afterwards); a pass of at most kPassWords blocks has a word for each of them instead and no counter.
+// word == null: the caller synchronises the stream instead.
+constexpr int kPassWords = 8;
 struct GroupDone {
   unsigned int* count = nullptr;
   uint64_t* word = nullptr;

@@ -440,6 +440,7 @@ struct Pinned {
   int status[kResultSlots];
   uint64_t done[kResultSlots][2];  // completion tokens and results (see Done)
   CallSlot calls;                  // lane 0's
+  uint64_t pass[collk::kPassWords];    // lane 0's: a group's pass of a few blocks, one word per block
 };
 
 // What a host context owns on this backend: its ordering domain (a stream) and the pinned words its blocking calls
@@ -1092,12 +1093,20 @@ class GpuBackend final : public Backend {
     }
     done.count = reinterpret_cast<unsigned int*>(group_dev_ + sizeof(GroupTable));
     collk::GroupPass pass;
+    int words = 0;
     auto one_pass = [&] {
       pass.a = a;
       pass.done = done;
+      words = ctas * pass.size <= collk::kPassWords ? ctas * pass.size : 0;
+      if (words) {
+        pass.done.word = pinned_->pass;
+        pass.done.count = nullptr;
+      }
       const cudaError_t e = collk::launch_pass(pass, ctas, stream_);
-      if (e != cudaSuccess) cudaGetLastError();      // not for somebody's next launch
-      return e == cudaSuccess ? (int)BSHMEM_OK : (int)BSHMEM_ERR_CUDA;
+      if (e == cudaSuccess) return (int)BSHMEM_OK;
+      cudaGetLastError();                              // not for somebody's next launch
+      words = 0;
+      return (int)BSHMEM_ERR_CUDA;
     };
     auto cooperative = [&]() -> int {
       GroupTable img;
@@ -1116,7 +1125,12 @@ class GpuBackend final : public Backend {
       return BSHMEM_ERR_CUDA;
     };
     int rc = launch_preferred(ctas * n <= sms_ && passes(hs, ht, n, a, &pass), (int)BSHMEM_OK, one_pass, cooperative);
-    if (rc == BSHMEM_OK) rc = wait_done(t, stream_);
+    if (rc == BSHMEM_OK)
+      rc = words ? poll([&] {
+             while (words && reinterpret_cast<const std::atomic<uint64_t>&>(pinned_->pass[words - 1]).load(std::memory_order_acquire) == t.done.token) --words;
+             return words == 0;
+           }, stream_)
+                 : wait_done(t, stream_);
     if (rc != BSHMEM_OK || *status == BSHMEM_OK) return rc;
     tl_err = std::string("device-side ") + bshmem_status_string(*status);
     return *status;
