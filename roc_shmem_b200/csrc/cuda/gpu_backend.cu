@@ -205,68 +205,82 @@ __global__ void __launch_bounds__(256) k_copy_small(char* dst, const char* src, 
   const uint64_t b = blockIdx.x * kSmallPiece, e = b + kSmallPiece < n ? b + kSmallPiece : n;
   dev::copy_bytes<dev::BLOCK>(dst + b, src + b, e - b);
 }
-// Non-blocking messages of a context, up to kRingMessageMax bytes between device buffers, need no launch each: the host writes
-// them into a ring in pinned memory and one block on the context's stream takes them from there.  The block is launched by the
+// Non-blocking messages of a context between device buffers need no launch each: the host writes them into a ring in pinned memory
+// and one block on the context's stream takes them from there (16 KiB and less; longer ones: k_ring_wide).  The block is launched by the
 // first message, stays while messages follow one another closely (kRingIdleNs) and at most kRingLifeNs.  While it stays it has
 // its multiprocessor's place, beside kernels that take a whole one per block too: 8192 x 8192 x 3584 products with 64 messages
 // before each take 358 to 360 us (356 to 361 with one launch per message); 1024 rows 50 (173 to 181), with four messages 49
 // (43).  Ending after 2 us without a message instead of 5 gains nothing there and costs a window 8 of 48 us.  The host path
-// bounds a window of messages: 64 puts of 64 bytes and a quiet took 177 us by one launch each (2.4 us apart and more), 44 so.  A
-// block with sixteen warps moves a message per warp, 16 KiB in four round trips to memory, as fast as the host writes them.
+// bounds a window of messages: 64 puts of 64 bytes and a quiet took 177 us by one launch each (2.4 us apart and more), 25 so.  A
+// block with sixteen warps moves a message per warp, 16 KiB in four round trips to memory.
 // message_ring.h has the protocol.
 constexpr unsigned kRingThreads = 512, kRingBatch = kRingThreads / 32;
 constexpr unsigned long long kRingIdleNs = 5000, kRingLifeNs = 100000;
 __device__ __forceinline__ void st_host(uint64_t* p, uint64_t v) { asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
 
+struct RingMessages {
+  struct { char* dst; const char* src; uint32_t n; } msg[kRingBatch];
+  int found, over;                     // messages of the batch; whether the block is to end (1) or has nothing left (2)
+};
+// One look at the ring, by one warp.  The last load acquires: what the host had seen done before it wrote a message is behind it (a
+// window of 64 puts of 64 bytes takes 25 us so, 29 with relaxed loads and a fence of system scope, 59 if all three acquire).
+__device__ __forceinline__ void ring_look(Ring* ring, uint32_t next, uint32_t generation, int lane, bool closing, unsigned long long begun,
+                                          unsigned long long& last, RingMessages& b) {
+  const uint32_t index = next + lane;
+  const uint64_t* w = ring->slot[index % kRingSlots].w;
+  uint64_t v0 = 0, v1 = 0, v2 = 0, stop = 0;
+  if (lane == 31) asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(stop) : "l"(&ring->stop) : "memory");
+  if (lane < kRingBatch) {
+    asm volatile("ld.relaxed.sys.global.v2.u64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "l"(w) : "memory");
+    asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v2) : "l"(w + 2) : "memory");       // last: what follows it waits for it
+  }
+  stop = __shfl_sync(0xffffffffu, stop, 31);
+  const uint64_t low48 = (1ull << 48) - 1;
+  const bool here = lane < kRingBatch && ring_arrived(v0, v1, v2, index, generation);
+  const uint32_t size = (uint32_t)v2;
+  const unsigned got = __ballot_sync(0xffffffffu, here), starts = __ballot_sync(0xffffffffu, here && (size & kRingOrdered)) & ~1u;
+  int count = __ffs(~got) - 1;
+  if (starts && __ffs(starts) - 1 < count) count = __ffs(starts) - 1;      // an ordered message begins a batch
+  if (lane < count) {
+    b.msg[lane].dst = reinterpret_cast<char*>(v0 & low48);
+    b.msg[lane].src = reinterpret_cast<const char*>(v1 & low48);
+    b.msg[lane].n = size & kRingSizeMask;
+  }
+  if (lane == 0) {
+    const unsigned long long now = dev::timer();
+    if (count) last = now;
+    b.found = count;
+    b.over = closing ? (count ? 0 : 2) : ring_stopped(stop, generation) || now - begun > kRingLifeNs || now - last > kRingIdleNs ? 1 : 0;
+  }
+  __syncwarp();
+}
+
+// The last warp says how far the messages are done, while the first one looks for more.  System scope, also on one GPU: a quiet that
+// sees the count ends like a stream synchronisation, for readers on the host too.
+constexpr unsigned kRingPublisher = kRingThreads - 32;
+__device__ __forceinline__ void ring_publish(Ring* ring, uint32_t next) {
+  if (threadIdx.x == kRingPublisher) {
+    asm volatile("fence.acq_rel.sys;" ::: "memory");
+    st_host(&ring->consumed, next);
+  }
+}
+
 __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next, uint32_t generation) {
   after_predecessor();
-  __shared__ struct { char* dst; const char* src; uint32_t n; } msg[kRingBatch];
-  __shared__ int found, over;          // messages of the batch; whether the block is to end (1) or has nothing left (2)
+  __shared__ RingMessages b;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long begun = dev::timer();
   unsigned long long last = begun;
   bool closing = false;
   while (true) {
-    if (warp == 0) {
-      const uint32_t index = next + lane;
-      const uint64_t* w = ring->slot[index % kRingSlots].w;
-      uint64_t v0 = 0, v1 = 0, v2 = 0, stop = 0;
-      if (lane < kRingBatch) {
-        asm volatile("ld.relaxed.sys.global.v2.u64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "l"(w) : "memory");
-        asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(v2) : "l"(w + 2) : "memory");
-      }
-      if (lane == 31) asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(stop) : "l"(&ring->stop) : "memory");
-      stop = __shfl_sync(0xffffffffu, stop, 31);
-      const uint64_t low48 = (1ull << 48) - 1;
-      const bool here = lane < kRingBatch && ring_arrived(v0, v1, v2, index, generation);
-      const uint32_t size = (uint32_t)v2;
-      const unsigned got = __ballot_sync(0xffffffffu, here), starts = __ballot_sync(0xffffffffu, here && (size & kRingOrdered)) & ~1u;
-      int count = __ffs(~got) - 1;
-      if (starts && __ffs(starts) - 1 < count) count = __ffs(starts) - 1;      // an ordered message begins a batch
-      if (lane < count) {
-        msg[lane].dst = reinterpret_cast<char*>(v0 & low48);
-        msg[lane].src = reinterpret_cast<const char*>(v1 & low48);
-        msg[lane].n = size & kRingSizeMask;
-      }
-      if (count) asm volatile("fence.acq_rel.sys;" ::: "memory");   // what the host had seen done before it wrote the message
-      if (lane == 0) {
-        const unsigned long long now = dev::timer();
-        if (count) last = now;
-        found = count;
-        over = closing ? (count ? 0 : 2) : ring_stopped(stop, generation) || now - begun > kRingLifeNs || now - last > kRingIdleNs ? 1 : 0;
-      }
-    }
+    if (warp == 0) ring_look(ring, next, generation, lane, closing, begun, last, b);
     __syncthreads();
-    const int count = found, end = over;
+    const int count = b.found, end = b.over;
     if (count) {
-      if (warp < count) dev::copy_bytes<dev::WARP>(msg[warp].dst, msg[warp].src, msg[warp].n);
+      if (warp < count) dev::copy_bytes<dev::WARP>(b.msg[warp].dst, b.msg[warp].src, b.msg[warp].n);
       __syncthreads();
       next += count;
-      if (threadIdx.x == 0) {
-        // system scope, also on one GPU: a quiet that sees the count ends like a stream synchronisation, for readers on the host too
-        asm volatile("fence.acq_rel.sys;" ::: "memory");
-        st_host(&ring->consumed, next);
-      }
+      ring_publish(ring, next);
     }
     if (end == 2) break;
     if (end == 1) {
@@ -278,7 +292,79 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
+  if (threadIdx.x == kRingPublisher) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
+}
+
+// The same by a cluster of eight blocks, for messages that one block is too slow for.  The first block looks at the ring and tells
+// the others what it found; the batch is copied in pieces of 4 KiB, one round trip to memory of a warp, by the warps of all blocks
+// in turn.  Windows of 64 puts, us, by a launch each (2.1 to 2.5 us apart, the host's) and so: 17 KB 159 -> 55, 64 KiB 159 -> 70, 256 KiB
+// 160 -> 95, 512 KiB 152 to 160 -> 140, 1 MiB 147 -> 232; hence the limit.  Up to 16 KiB one block is as fast (8 KiB 46, the cluster 54) and holds
+// one multiprocessor, not eight: products of 1024 rows with 64 messages of 64 KiB before each take 67 us (164 by launches, 47 alone),
+// with four 52 (47).  Ending after 2 us without a message instead of 5 changes neither.
+constexpr unsigned kRingBlocks = 8, kRingPiece = 4096;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __launch_bounds__(kRingThreads) k_ring_wide(Ring* ring, uint32_t next, uint32_t generation) {
+  after_predecessor();
+  __shared__ RingMessages b;
+  static_assert(sizeof(RingMessages) % 4 == 0, "passed on in words");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, block = blockIdx.x;
+  const unsigned long long begun = dev::timer();
+  unsigned long long last = begun;
+  bool closing = false;
+  cluster_barrier();                                           // every block's memory is there to be written to
+  while (true) {
+    if (block == 0 && warp == 0) {
+      do ring_look(ring, next, generation, lane, closing, begun, last, b);
+      while (b.found == 0 && b.over == 0);
+      const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&b);
+      for (unsigned i = lane; i < sizeof(RingMessages) / 4; i += 32) {
+        const uint32_t word = reinterpret_cast<const uint32_t*>(&b)[i];
+        for (unsigned r = 1; r < kRingBlocks; ++r) {
+          uint32_t there;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine + i * 4), "r"(r));
+          asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"(word) : "memory");
+        }
+      }
+    }
+    cluster_barrier();
+    const int count = b.found, end = b.over;
+    unsigned piece = block * kRingBatch + warp, first = 0;
+    for (int m = 0; m < count; ++m) {
+      const uint32_t n = b.msg[m].n, pieces = (n + kRingPiece - 1) / kRingPiece;
+      for (; piece - first < pieces; piece += kRingBlocks * kRingBatch) {
+        const uint32_t at = (piece - first) * kRingPiece;
+        dev::copy_bytes<dev::WARP>(b.msg[m].dst + at, b.msg[m].src + at, min(kRingPiece, n - at));
+      }
+      first += pieces;
+    }
+    cluster_barrier();                                         // all of it is copied, and the batch has been read
+    next += count;
+    if (block == 0 && count) ring_publish(ring, next);
+    if (block == 0 && threadIdx.x == 0 && end == 1) {
+      st_host(&ring->closed, generation);
+      asm volatile("fence.sc.sys;" ::: "memory");
+    }
+    if (end == 2) break;
+    if (end == 1) closing = true;
+    __syncwarp();
+  }
+  if (block == 0 && threadIdx.x == kRingPublisher)
+    asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
+}
+cudaLaunchConfig_t ring_wide_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kRingBlocks);
+  cfg.blockDim = dim3(kRingThreads);
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kRingBlocks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cfg;
 }
 
 // Payload and signal of a small message in one block: the block barrier orders every thread's stores before the
@@ -536,6 +622,11 @@ class GpuBackend final : public Backend {
     RT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, heap_->device));
     if (coll_ctas_ > sms) coll_ctas_ = sms;
     sms_ = sms;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t wide = ring_wide_config(attr, nullptr);
+    int clusters = 0;
+    ring_wide_ = cudaOccupancyMaxActiveClusters(&clusters, k_ring_wide, &wide) == cudaSuccess && clusters > 0;
+    if (!ring_wide_) cudaGetLastError();
     return BSHMEM_OK;
   }
 
@@ -622,14 +713,22 @@ class GpuBackend final : public Backend {
     return {stream_of(L), {}};
   }
   bool ring_takes(const Lane& L, const void* a, const void* b, uint64_t n, bool nbi) const {
-    return nbi && tl_local_is_device && n > 0 && n <= kRingMessageMax && L.ring.ring && !thread_is_bound() &&
+    const bool skewed = ((reinterpret_cast<uintptr_t>(a) ^ reinterpret_cast<uintptr_t>(b)) & 15) != 0;
+    return nbi && tl_local_is_device && n > 0 && n <= (!ring_wide_ ? kRingNarrowMax : skewed ? kSmallCopyMaxSkewed : kRingMessageMax) && L.ring.ring &&
+           !thread_is_bound() &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) >> 48) == 0;
   }
   int ring_message(Lane& L, char* dst, const char* src, uint32_t n) {
     const int rc = L.ring.message(
         reinterpret_cast<uintptr_t>(dst), reinterpret_cast<uintptr_t>(src), n,
         [&](uint32_t from, uint32_t generation) -> int {
-          RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
+          if (n > kRingNarrowMax) {
+            cudaLaunchAttribute attr[2];
+            const cudaLaunchConfig_t cfg = ring_wide_config(attr, L.stream);
+            RT_TRY(cudaLaunchKernelEx(&cfg, k_ring_wide, L.ring.ring, from, generation));
+          } else {
+            RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
+          }
           return BSHMEM_OK;
         },
         [&](auto arrived) {
@@ -1183,6 +1282,7 @@ class GpuBackend final : public Backend {
   bool blocking_ = true;
   bool use_nvls_ = false;
   int coll_ctas_ = 32, sms_ = 0;
+  bool ring_wide_ = false;              // the device takes the cluster of k_ring_wide
   std::mutex calls_mu_;                 // one request at a time
   CallWriter calls_;
   cudaStream_t calls_stream_ = nullptr;
