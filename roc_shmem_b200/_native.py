@@ -87,14 +87,17 @@ def fast(lib: C.CDLL, name: str):
     return _pycall().Native(C.cast(fn, C.c_void_p).value, len(fn.argtypes), kind, pointers)
 
 
-def mover(lib: C.CDLL, name: str, handle: int, context: int, device: int, local: int, general, check):
+def mover(lib: C.CDLL, name: str, context, method: str, plain, local: int):
     """put or get of a context as a callable that reads the tensors' addresses and sizes itself (csrc/host/pycall.cc), for calls
-    (dest, src, pe, nbi=True or False) of plain tensors whose `local`-th is on `device`; anything else goes to `general`."""
+    (dest, src, pe, nbi=True or False) of plain tensors whose `local`-th is on the runtime's device, while `method` of the context's
+    type is `plain`; anything else goes to that method."""
     import torch
     table = getattr(torch.Tensor, "__dlpack_c_exchange_api__", None)
     if table is None:                             # a torch without it
-        return general
-    return _pycall().Mover(C.cast(getattr(lib, name), C.c_void_p).value, handle, context, device, local, torch.Tensor, table, general, check)
+        return getattr(context, method)
+    rt = context.rt
+    return _pycall().Mover(C.cast(getattr(lib, name), C.c_void_p).value, rt._hv, context.idx, rt._dev_index, local, torch.Tensor, table,
+                           context, method, plain, rt._check)
 
 
 class _build_lock:

@@ -8,7 +8,7 @@
 // `Mover` is the same for the messages of a context, put(dest, src, pe, nbi=...): it takes the tensors themselves and reads their addresses
 // and sizes through DLPack's C exchange table.  What the attribute look-ups of a Python method and its frame add to that was three
 // quarters of a small message's 0.6 us: a window of 64 non-blocking puts of 64 bytes took 41 us, so 25.  Calls of any other form go to the
-// general method that the object was made with.
+// method of the context's type; so do all while that is another one than it was (tracing puts a method with ranges there).
 //
 // Only integer and pointer arguments are supported, and they take what ctypes takes for them: an integer argument anything
 // with __index__ (a numpy integer, a one-element tensor) but not None; an address (bit i of `pointers`) an int or None.  Every argument is passed as one 64-bit word: under the System V
@@ -156,7 +156,8 @@ struct Mover {
   int context, device, local;    // local: which argument is this PE's own buffer and says how much is moved, 0 = dest, 1 = src
   int (*describe)(void*, DlTensor*);
   PyObject* tensor;              // the type whose instances `describe` takes
-  PyObject* general;             // the method for every other call
+  PyObject *owner, *name;        // the context, and the method of its type for every other call
+  PyObject* plain;               // that method as this one stands for it
   PyObject* check;               // raises for a status
 };
 PyObject* g_nbi = nullptr;       // the interned keyword
@@ -196,7 +197,19 @@ bool move_at_once(const Mover* m, PyObject* const* args, Py_ssize_t n, PyObject*
 PyObject* mover_call(PyObject* callable, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   const Mover* m = reinterpret_cast<Mover*>(callable);
   uint64_t a[7];
-  if (!move_at_once(m, args, PyVectorcall_NARGS(nargsf), kwnames, a)) return PyObject_Vectorcall(m->general, args, nargsf, kwnames);
+  PyTypeObject* type = Py_TYPE(m->owner);
+  PyObject* method = _PyType_Lookup(type, m->name);            // borrowed
+  if (!method) return PyErr_Format(PyExc_AttributeError, "%U", m->name);
+  if (method != m->plain || !move_at_once(m, args, PyVectorcall_NARGS(nargsf), kwnames, a)) {
+    const descrgetfunc bind = Py_TYPE(method)->tp_descr_get;
+    Py_INCREF(method);
+    PyObject* bound = bind ? bind(method, m->owner, reinterpret_cast<PyObject*>(type)) : Py_NewRef(method);
+    Py_DECREF(method);
+    if (!bound) return nullptr;
+    PyObject* result = PyObject_Vectorcall(bound, args, nargsf, kwnames);
+    Py_DECREF(bound);
+    return result;
+  }
   int status;
   Py_BEGIN_ALLOW_THREADS
   status = (int32_t)(uint32_t)thunk<7>(m->addr, a);
@@ -207,8 +220,8 @@ PyObject* mover_call(PyObject* callable, PyObject* const* args, size_t nargsf, P
 PyObject* mover_new(PyTypeObject* type, PyObject* args, PyObject*) {
   unsigned long long addr = 0, handle = 0;
   int context = 0, device = 0, local = 0;
-  PyObject *tensor, *capsule, *general, *check;
-  if (!PyArg_ParseTuple(args, "KKiiiOOOO", &addr, &handle, &context, &device, &local, &tensor, &capsule, &general, &check)) return nullptr;
+  PyObject *tensor, *capsule, *owner, *name, *plain, *check;
+  if (!PyArg_ParseTuple(args, "KKiiiOOOUOO", &addr, &handle, &context, &device, &local, &tensor, &capsule, &owner, &name, &plain, &check)) return nullptr;
   const auto* x = static_cast<const DlExchange*>(PyCapsule_GetPointer(capsule, "dlpack_exchange_api"));
   if (!x) return nullptr;
   if (!addr || !PyType_Check(tensor) || (local != 0 && local != 1) || x->version.major != 1 || !x->describe) {
@@ -225,7 +238,10 @@ PyObject* mover_new(PyTypeObject* type, PyObject* args, PyObject*) {
   m->local = local;
   m->describe = x->describe;
   m->tensor = Py_NewRef(tensor);
-  m->general = Py_NewRef(general);
+  m->owner = Py_NewRef(owner);
+  m->name = Py_NewRef(name);
+  PyUnicode_InternInPlace(&m->name);
+  m->plain = Py_NewRef(plain);
   m->check = Py_NewRef(check);
   return reinterpret_cast<PyObject*>(m);
 }
@@ -233,14 +249,17 @@ int mover_traverse(PyObject* o, visitproc visit, void* arg) {
   Mover* m = reinterpret_cast<Mover*>(o);
   Py_VISIT(Py_TYPE(o));
   Py_VISIT(m->tensor);
-  Py_VISIT(m->general);
+  Py_VISIT(m->owner);
+  Py_VISIT(m->plain);
   Py_VISIT(m->check);
   return 0;
 }
 int mover_clear(PyObject* o) {
   Mover* m = reinterpret_cast<Mover*>(o);
   Py_CLEAR(m->tensor);
-  Py_CLEAR(m->general);
+  Py_CLEAR(m->owner);
+  Py_CLEAR(m->name);
+  Py_CLEAR(m->plain);
   Py_CLEAR(m->check);
   return 0;
 }
@@ -263,8 +282,8 @@ PyType_Slot mover_slots[] = {
     {Py_tp_clear, reinterpret_cast<void*>(mover_clear)},
     {Py_tp_dealloc, reinterpret_cast<void*>(mover_dealloc)},
     {Py_tp_members, mover_members},
-    {Py_tp_doc, const_cast<char*>("Mover(address, handle, context, device, local, tensor type, exchange table, general method, status check): "
-                                  "put or get of a context, called as its general method is")},
+    {Py_tp_doc, const_cast<char*>("Mover(address, handle, context, device, local, tensor type, exchange table, owner, name, plain method, "
+                                  "status check): put or get of a context, called as its method of that name is")},
     {0, nullptr},
 };
 PyType_Spec mover_spec = {"bshmem_pycall.Mover", sizeof(Mover), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL | Py_TPFLAGS_HAVE_GC, mover_slots};

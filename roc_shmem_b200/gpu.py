@@ -141,12 +141,13 @@ def _gpu_error(lib, what: str, status: int) -> None:
 class DeviceContext(Context):
     """Context of a DeviceRuntime: messages between device buffers go straight to the native call."""
 
-    def __init__(self, rt, idx, options, team):
-        super().__init__(rt, idx, options, team)
-        if type(self).put is DeviceContext.put and type(self).get is DeviceContext.get:
-            # the methods below without an interpreter's frame around them; calls of another form still come here
-            self.put = _native.mover(rt.lib, "bshmem_gpu_ctx_put_dev", rt._hv, idx, rt._dev_index, 1, self.put, rt._check)
-            self.get = _native.mover(rt.lib, "bshmem_gpu_ctx_get_dev", rt._hv, idx, rt._dev_index, 0, self.get, rt._check)
+    @classmethod
+    def _created(cls, rt, idx, options, team):
+        self = cls(rt, idx, options, team)
+        # put and get without an interpreter's frame around them, while they are the methods below and not, say, their traced forms
+        self.put = _native.mover(rt.lib, "bshmem_gpu_ctx_put_dev", self, "put", _CONTEXT_PUT, 1)
+        self.get = _native.mover(rt.lib, "bshmem_gpu_ctx_get_dev", self, "get", _CONTEXT_GET, 0)
+        return self
 
     def destroy(self):
         super().destroy()
@@ -175,11 +176,14 @@ class DeviceContext(Context):
         rt.get(dest, src, pe, ctx=self, nbi=nbi, nbytes=nbytes)
 
 
+_CONTEXT_PUT, _CONTEXT_GET = DeviceContext.put, DeviceContext.get
+
+
 class DeviceRuntime(Runtime):
     """Runtime over the NVLink backend, plus the GPU-only knobs."""
 
     backend = "device"
-    _context_type = DeviceContext
+    _context_type = DeviceContext._created
 
     def __init__(self, lib, handle, device: torch.device, heap, own_heap: bool = True):
         super().__init__(lib, handle,
