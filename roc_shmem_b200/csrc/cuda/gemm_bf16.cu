@@ -7,6 +7,7 @@
 // no counterpart in the reference, which contains no GEMM.  Problems with few rows of A
 // take the weight-streaming kernel of gemm_skinny.cuh instead (plan_skinny says when).
 #include <atomic>
+#include <utility>
 
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
@@ -25,6 +26,7 @@ struct PlainParams {
   CUtensorMap map_b2, map_c2;  // B rows of a second accumulator (wide form), output boxes of 32 columns
   __nv_bfloat16* out;          // split form: the result, written directly
   long long ldc;
+  int turned;                  // A and B have changed places, the maps of C are for its transpose
 };
 
 // One policy per operand layout.  K-major (kAmn / kBmn false): A is stored [M][K], one 128-row x 64 box per CTA and stage.
@@ -81,14 +83,16 @@ struct PlainBf16 : PolicyDefaults {
   }
   __device__ static __forceinline__ void out_target(const Params& p, int row, int col, const CUtensorMap** map, int* x, int* y) {
     *map = (row < p.core.M && col < p.core.N) ? &p.map_c : nullptr;
-    *x = col;
-    *y = row;
+    *x = p.turned ? row : col;
+    *y = p.turned ? col : row;
   }
   __device__ static __forceinline__ void out_target_half(const Params& p, int row, int col, const CUtensorMap** map, int* x, int* y) {
     *map = (row < p.core.M && col < p.core.N) ? &p.map_c2 : nullptr;
-    *x = col;
-    *y = row;
+    *x = p.turned ? row : col;
+    *y = p.turned ? col : row;
   }
+  static constexpr bool kTurns = kVarCols;
+  __device__ static __forceinline__ bool turned(const Params& p) { return p.turned; }
   static constexpr bool kRaggedCols = kVarCols;
   __device__ static __forceinline__ bool ragged_chunk(const Params& p, int col) { return (p.core.N & 7) && col < p.core.N && col + EPI_COLS > p.core.N; }
   __device__ static __forceinline__ void store_ragged(const Params& p, int row, int col, const uint32_t (&w)[32], int cols) {
@@ -322,7 +326,26 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
     if (tiles <= g_octs[dev] && kb >= (one_wave ? 41 : 24)) p.core.split = 4;
     else if (tiles <= g_quads[dev] && kb >= (one_wave ? 60 : 32)) p.core.split = 2;
   }
-  const Width w = p.core.split > 1 ? Width{{BN, 0}} : one_wave ? Width{{128, 0}} : plan_width(row_blocks, N, K, pairs, 32, b_mn != 0);
+  // Tiles have 256 rows, but their columns come in steps of 32: where that leaves less of them empty, A and B change places and C is
+  // stored transposed (its TMA boxes are cut off on 16 bytes, so N is a multiple of 8); the bits are the same.  us before, with tiles of
+  // two accumulators from 352 columns on, and now, with those from 288: 264 x 8192 x 3584 22.9 and 18.9, 320 x 7168 x 8192 52.5 and 40.5,
+  // 640 x 4096 x 14336 86 and 62, 1152 x 8192 x 3584 69 and 58.  Not for an MN-major A, which would be loaded like an MN-major B
+  // (see plan_width), nor narrow tiles of two accumulators for such a B: 264 x 14336 x 4096 so took 63, as it is 50.  A threshold of 3 %,
+  // about what the estimates are good for.
+  auto plan = [&](int rows, int cols, bool mn) { return plan_width((rows + BM - 1) / BM, cols, K, pairs, 32, mn, true, 512, 0, mn ? 352 : 288); };
+  Width w = p.core.split > 1 ? Width{{BN, 0}} : one_wave ? Width{{128, 0}} : plan(M, N, b_mn != 0);
+  p.turned = 0;
+  if (p.core.split == 1 && !one_wave && !a_mn && N % 8 == 0) {
+    const Width t = plan(N, M, false);
+    if (t.cost < 0.97 * w.cost) {
+      w = t;
+      p.turned = 1;
+      std::swap(A, B);
+      std::swap(M, N);
+      std::swap(lda, ldb);
+      std::swap(a_mn, b_mn);
+    }
+  }
   const int width = w.cols[0] + w.cols[1];
   p.core.acc_cols[0] = w.cols[0];
   p.core.acc_cols[1] = w.cols[1];
@@ -341,9 +364,12 @@ int bshmem_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int
   if (rc) return rc;
   if (w.cols[1] && !b_mn) rc = host::make_tmap_2d(&p.map_b2, bf, 2, B, N, K, ldb, w.cols[1] / 2, 64);
   if (rc) return rc;
-  if ((w.cols[0] | w.cols[1]) & 63) rc = host::make_tmap_2d(&p.map_c2, bf, 2, C, M, N, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+  if ((w.cols[0] | w.cols[1]) & 63)
+    rc = p.turned ? host::make_tmap_2d(&p.map_c2, bf, 2, C, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_NONE)
+                  : host::make_tmap_2d(&p.map_c2, bf, 2, C, M, N, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
   if (rc) return rc;
-  rc = host::make_tmap_2d(&p.map_c, bf, 2, C, M, N, ldc, 32, EPI_COLS);
+  rc = p.turned ? host::make_tmap_2d(&p.map_c, bf, 2, C, N, M, ldc, EPI_COLS, 32, CU_TENSOR_MAP_SWIZZLE_NONE)
+                : host::make_tmap_2d(&p.map_c, bf, 2, C, M, N, ldc, 32, EPI_COLS);
   if (rc) return rc;
   const int tiles = p.core.num_m_blocks * p.core.num_n_blocks;
   p.out = static_cast<__nv_bfloat16*>(C);

@@ -258,6 +258,11 @@ struct PolicyDefaults {
   // kRaggedCols: the output's width may end inside a 16-byte piece.  A TMA store fills the piece with zeros, over what lies
   // behind the matrix; such a chunk (ragged_chunk) is written by store_ragged instead, element by element.
   static constexpr bool kRaggedCols = false;
+  // kTurns, with kVarCols and kHalfChunks: turned(prm) says that the output is stored transposed, element (row, column) of the tile at
+  // (column, row) of the matrix.  The maps of out_target and out_target_half then have boxes of 64 and of 32 columns of the tile by
+  // 32 rows, without a swizzle.
+  static constexpr bool kTurns = false;
+  template <class Params> __device__ static __forceinline__ bool turned(const Params&) { return false; }
   // Operand layout.  Default: both operands K-major, one 128-row x 128-byte TMA box per operand, CTA and stage, and
   // shared-memory descriptors that step 32 bytes along K inside the swizzle atom.  A policy with MN-major operands
   // overrides the instruction descriptor, the stage-0 descriptors, the step per MMA and the loads.
@@ -337,6 +342,20 @@ __device__ __forceinline__ void stage_packed_half(uint32_t buf, int lane, const 
   for (int j = 0; j < 4; ++j) {
     const uint32_t dst = rowbase + ((j ^ ((lane >> 1) & 3)) << 4);
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]), "r"(w[4 * j + 3]) : "memory");
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
+
+// 64 columns of the warp's 32 rows for a transposed store: column j's 32 values in a row of 64 bytes, two lanes' values to a word.
+__device__ __forceinline__ void stage_turned(uint32_t buf, int lane, const uint32_t (&w)[32]) {
+  const bool odd = lane & 1;
+  const uint32_t at = buf + (odd ? 64 : 0) + (lane >> 1) * 4;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, w[j], 1);
+    const uint32_t v = odd ? __byte_perm(other, w[j], 0x7632) : __byte_perm(w[j], other, 0x5410);
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + j * 128), "r"(v) : "memory");
   }
   ptx::fence_proxy_async_smem();
   __syncwarp();
@@ -732,8 +751,10 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
           for (int u = 0; u < kAtOnce; ++u) {
             const int mine = left - (c0 + u) * EPI_COLS, col0 = ck.col0 + (c0 + u) * EPI_COLS;
             if (mine <= 0 || col0 >= cp.N) continue;
+            bool turned = false;
+            if constexpr (P::kTurns) turned = P::turned(prm);
             if constexpr (P::kRaggedCols) {
-              if (P::ragged_chunk(prm, col0)) {
+              if (!turned && P::ragged_chunk(prm, col0)) {
                 P::store_ragged(prm, ck.row0 + lane, col0, w[u], mine);
                 continue;
               }
@@ -741,7 +762,8 @@ __device__ __forceinline__ void gemm_mainloop(const typename P::Params& prm, uin
             if (lane == 0) ptx::tma_wait_group_read<0>();     // the previous store has read the staging buffer
             __syncwarp();
             const CUtensorMap* map; int x, y;
-            if (P::kHalfChunks && mine < EPI_COLS) stage_packed_half(L.epi(ew), lane, w[u]);
+            if (turned) stage_turned(L.epi(ew), lane, w[u]);
+            else if (P::kHalfChunks && mine < EPI_COLS) stage_packed_half(L.epi(ew), lane, w[u]);
             else stage_packed(L.epi(ew), lane, w[u]);
             if (lane == 0) {
               P::out_target(prm, ck.row0, col0, &map, &x, &y);

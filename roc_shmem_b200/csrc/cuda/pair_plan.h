@@ -22,25 +22,28 @@ namespace gemm2 {
 // `wide_delay`: cycles that a tile's epilogue keeps the tensor cores waiting in the wide form (two per column and k-block).
 // `pairs`: that work at the same time; with none (nothing can be launched) as with one.
 // `step`: what an accumulator's columns are a multiple of, 32 or, where the epilogue wants more, 64 or 128.
+// `narrowest_wide`: the least columns of a tile of two accumulators.
 struct Width {
   int cols[2];
+  double cost = 0;      // of the launch by whole waves, what an MN-major B adds left out
 };
 inline Width plan_width(long long row_blocks, int N, int K, int pairs, int step, bool b_mn, bool exact = true, int widest = 512,
-                        int wide_delay = 0) {
+                        int wide_delay = 0, int narrowest_wide = 352) {
   constexpr int BN = 256;
   if (pairs < 1) pairs = 1;
   const double blocks = (K + 63) / 64, narrow = 0.91 + blocks / 160 < 1.1 ? 0.91 + blocks / 160 : 1.1;
   struct { double cost, whole; Width w; } best[2] = {{1e30, 1e30, {{BN, 0}}}, {1e30, 1e30, {{BN, 0}}}};      // of one accumulator, of two
   for (int w = widest; w >= 128; w -= step) {
-    if (w > BN && w < 352) continue;                  // two accumulators of less than 160 columns
+    if (w > BN && w < narrowest_wide) continue;
     const int c0 = w > BN ? (w + 2 * step - 1) / (2 * step) * step : w, c1 = w - c0;
     const int loaded = !b_mn ? w : c1 ? 2 * BN : BN;
     const long long tiles = row_blocks * ((N + w - 1) / w);
     const double per_wave = (c1 ? 26 + 0.95 * 0.5 * (w + loaded) + wide_delay / (2 * blocks) : narrow * 0.5 * (BN + loaded)) + 8;
-    const double whole = (double)((tiles + pairs - 1) / pairs) * per_wave;
+    const long long waves = (tiles + pairs - 1) / pairs;
+    const double whole = (double)waves * per_wave;
     const double cost = exact ? whole : (tiles > pairs / 2 ? 0.5 + (double)tiles / pairs : 1.0) * per_wave;
     auto& b = best[c1 ? 1 : 0];
-    if (cost < b.cost) b = {cost, whole, {{c0, c1}}};
+    if (cost < b.cost) b = {cost, whole, {{c0, c1}, (double)waves * ((c1 ? 26 + 0.95 * w : narrow * 0.5 * (BN + w)) + 8)}};
   }
   return best[1].cost <= best[0].cost && best[1].whole <= best[0].whole ? best[1].w : best[0].w;
 }
