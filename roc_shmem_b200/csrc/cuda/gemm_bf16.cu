@@ -217,9 +217,15 @@ struct SkinnyPlan {
 //      4096x6144  18.3-21.6   17.7-19.9   17.9-19.9   19.4-19.7   20.0-19.8
 //    208 gives up to 10 % away at 192 and 208 tokens for the second and about as much at 224 for the last two; split in four,
 //    14336x4096, 256 tokens: 33.6 against 42.9
+//  - above 64 tokens a short reduction leaves a CTA few k-blocks to hide the exchange of its parts behind, and a CTA pair on one wave of
+//    tiles of 128 columns needs about 0.16 us per k-block whatever the tokens.  The lines cross at 88 + 4.5 tokens per k-block, for every
+//    N that makes one wave (1024 to 8192), few-token form against pairs:  8 k-blocks 112 / 128 / 256 tokens 6.1-5.7 / 6.2-5.8 / 8.1-5.8;
+//    16: 144 / 160 / 256  7.3-7.1 / 7.8-7.1 / 9.7-7.1;  24: 192 / 224 / 256  8.8-8.4 / 9.6-8.4 / 10.4-8.5;  32: 224 / 256  9.5-9.6 /
+//    10.2-9.6;  40: 256  10.3-10.8
 SkinnyPlan plan_skinny(int M, int N, int K, int dev) {
   if (M > skinny::MAX_TOKENS) return {0, false};
   const int tiles = (N + skinny::ROWS - 1) / skinny::ROWS, kb = (K + skinny::BK - 1) / skinny::BK;
+  if (M > 64 && kb <= 32 && 2 * M >= 176 + 9 * kb && (N + 127) / 128 <= g_pairs[dev]) return {0, false};
   auto best = [&](bool half) {
     int s = 1;
     while (s < 8 && kb >= 8 * s && (half ? tiles * s <= g_sms[dev] : tiles <= skinny_clusters(dev, 2 * s))) s *= 2;

@@ -23,3 +23,26 @@ def test_one_wave(M, N, K, a_mn, b_mn):
     # bf16 rounding of the result, plus fp32 sums of K products in any order
     tol = ref.abs() * 2 ** -8 + K * 2 ** -24 * (a.abs() @ b.abs().t())
     assert bool(((buf[:M, :N].double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("kb,tokens", [(4, 106), (8, 124), (12, 142), (20, 178), (32, 232), (32, 256), (33, 256)])
+@pytest.mark.parametrize("N", [128, 1032, 9472, 9473])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_few_tokens_on_pairs(kb, tokens, N, b_mn):
+    """Both sides of the line between the few-token form and pairs on one wave of tiles of 128 columns."""
+    from roc_shmem_b200.ops.gemm import gemm_bf16, gemm_error_site
+    if b_mn and N % 8:
+        pytest.skip("refused: TMA needs rows of a multiple of 16 bytes")
+    K = 64 * kb - 8
+    for M in (tokens - 1, tokens):
+        torch.manual_seed(M + N + K)
+        a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
+        buf = torch.full((M + 1, (N + 15) // 8 * 8), 7.0, dtype=torch.bfloat16, device="cuda")
+        gemm_bf16(a, b.t().contiguous() if b_mn else b, buf[:M, :N], b_mn=b_mn)
+        torch.cuda.synchronize()
+        assert gemm_error_site() == 0
+        assert bool((buf[:, N:] == 7).all()) and bool((buf[M:] == 7).all())
+        a, b = a.double(), b.double()
+        ref = a @ b.t()
+        tol = ref.abs() * 2 ** -8 + K * 2 ** -24 * (a.abs() @ b.abs().t())
+        assert bool(((buf[:M, :N].double() - ref).abs() <= tol).all())
