@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(c
 // ---- the group as one pass (GroupPass) ----
 // Bound by the launch and one round trip to memory where little is moved, by HBM beyond.  Before: up to eight blocks as a cluster with
 // two barriers, more of them cooperatively with two flag exchanges, large reductions staged through shared memory.  Whole calls, before
-// and now, us: allreduce 16 KiB fp32, 4 PEs 14.9 -> 10.5; 1 MiB bf16, 8 PEs 23.4 -> 12.6; 32 MiB fp32, 8 PEs 117 -> 103; reduce-scatter
+// and now, us: allreduce 16 KiB fp32, 4 PEs 14.9 -> 9.6; 1 MiB bf16, 8 PEs 23.4 -> 12.6; 32 MiB fp32, 8 PEs 117 -> 103; reduce-scatter
 // 32 MiB bf16, 8 PEs 83.7 -> 59.8 (302 MB, 46 at the copy rate), 32 MiB fp32, 4 PEs 50.0 -> 39.8; fcollect 16 MiB, 8 PEs 44.4 -> 38.4;
 // alltoall 32 MiB, 8 PEs 107 -> 101, 2 MiB, 4 PEs 20.0 -> 13.5.
 // 512 threads with 16 loads of 16 bytes each on their way keep 128 KB in flight per block; a block to a multiprocessor, as many as
