@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(c
 // two barriers, more of them cooperatively with two flag exchanges, large reductions staged through shared memory.  Whole calls, before
 // and now, us: allreduce 16 KiB fp32, 4 PEs 14.9 -> 9.6; 1 MiB bf16, 8 PEs 23.4 -> 12.6; 32 MiB fp32, 8 PEs 117 -> 103; reduce-scatter
 // 32 MiB bf16, 8 PEs 83.7 -> 59.8 (302 MB, 46 at the copy rate), 32 MiB fp32, 4 PEs 50.0 -> 39.8; fcollect 16 MiB, 8 PEs 44.4 -> 38.4;
-// alltoall 32 MiB, 8 PEs 107 -> 101, 2 MiB, 4 PEs 20.0 -> 13.5.
+// alltoall 32 MiB, 8 PEs 110 -> 98, 2 MiB, 4 PEs 20.1 -> 12.3.
 // 512 threads with 16 loads of 16 bytes each on their way keep 128 KB in flight per block; a block to a multiprocessor, as many as
 // the caller asked for.
 constexpr int kPassThreads = 512;
@@ -286,6 +286,38 @@ __global__ void __launch_bounds__(kPassThreads) COLL_CAT(k_coll_pass_, COLL_UNIT
   pass_end(g, cap, a.kind == BSHMEM_COLL_REDUCE_ROOT ? a.n * sizeof(T) : 0);
 }
 #else
+// Member me's part of an alltoall from byte b of its blocks on, nv vectors of each, as one range: eight vectors on their way per thread
+// whatever block they belong to.  Block by block, each with an end of its own, 8 PEs: 256 KiB per block 12.3 us in the kernel, 8.2 so;
+// 2.8 MB 65.6 and 61.4 (359 MB: 55 at the copy rate); four on their way 71.6, sixteen 67.4.
+__device__ __forceinline__ void pass_exchange(const GroupPass& g, int me, size_t b, size_t nv) {
+  const CollArgs& a = g.a;
+  constexpr int U = 8;
+  if (nv == 0) return;
+  int k = 0;                                     // the block of the next vector, counted from the own one on
+  size_t v = threadIdx.x;
+  auto wrap = [&] {
+    while (k < g.size && v >= nv) { v -= nv; ++k; }
+  };
+  wrap();
+  while (k < g.size) {
+    uint4 x[U];
+    uint4* d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      d[u] = nullptr;
+      if (k < g.size) {
+        const int j = me + k < g.size ? me + k : me + k - g.size;
+        x[u] = reinterpret_cast<const uint4*>(g.base[me] + a.src_off + (uint64_t)j * a.n + b)[v];
+        d[u] = reinterpret_cast<uint4*>(g.base[j] + a.dst_off + (uint64_t)me * a.n + b) + v;
+        v += kPassThreads;
+        wrap();
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (d[u]) *d[u] = x[u];
+  }
+}
 // fcollect: member blockIdx.y's block to everybody, read once.  alltoall: member blockIdx.y's blocks to their owners.  broadcast: the
 // root's vector to member blockIdx.y, the root's own dest left as it is.
 __global__ void __launch_bounds__(kPassThreads) k_coll_pass_move(const __grid_constant__ GroupPass g) {
@@ -299,9 +331,13 @@ __global__ void __launch_bounds__(kPassThreads) k_coll_pass_move(const __grid_co
   if (a.kind == BSHMEM_COLL_BROADCAST) {
     if (me != a.root) dev::copy_bytes<dev::BLOCK>(g.base[me] + a.dst_off + b, g.base[a.root] + a.src_off + b, n);
   } else if (a.kind == BSHMEM_COLL_ALLTOALL) {
-    for (int k = 0; k < g.size; ++k) {
-      const int j = (me + k) % g.size;
-      dev::copy_bytes<dev::BLOCK>(g.base[j] + a.dst_off + (uint64_t)me * a.n + b, g.base[me] + a.src_off + (uint64_t)j * a.n + b, n);
+    if (((a.src_off | a.dst_off | a.n) & 15) == 0) {
+      pass_exchange(g, me, b, n >> 4);
+    } else {
+      for (int k = 0; k < g.size; ++k) {
+        const int j = (me + k) % g.size;
+        dev::copy_bytes<dev::BLOCK>(g.base[j] + a.dst_off + (uint64_t)me * a.n + b, g.base[me] + a.src_off + (uint64_t)j * a.n + b, n);
+      }
     }
   } else {
     const uint64_t src_at = a.src_off + b, dst_at = a.dst_off + (uint64_t)me * a.n + b;

@@ -115,3 +115,11 @@ def test_a_team_that_leaves_pes_out(both):
     slots = both.g.team_split(0, 1, 2, both.pes // 2)      # the odd PEs
     for kind in (gpu.COLL_REDUCE, gpu.COLL_REDUCE_SCATTER, gpu.COLL_FCOLLECT, gpu.COLL_ALLTOALL, gpu.COLL_BROADCAST, gpu.COLL_REDUCE_ROOT):
         both.check(kind, torch.float32, D.SUM, 3001, 2, root=both.pes // 2 - 1, slot=slots[1], members=list(range(1, both.pes, 2)))
+
+
+@pytest.mark.parametrize("n", [16, 16 * 7, 16 * 512, 16 * 4095, 16 * 4097, 16 * 100_003])
+def test_alltoall_of_whole_vectors(both, n):
+    """Blocks of whole vectors are moved as one range per block of the launch: from fewer vectors than threads to several rounds of it."""
+    for start in (0, 4, 16):
+        for ctas in (1, 3, 148 // both.pes):
+            both.check(both.gpu.COLL_ALLTOALL, torch.uint8, 0, n, ctas, start)
