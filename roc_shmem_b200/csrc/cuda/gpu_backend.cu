@@ -397,6 +397,9 @@ constexpr unsigned long long kCallIdleNs = 8000, kCallLifeNs = 500000;
 // so before the block is launched: single calls, a few of them and those with a synchronisation between them stay launches.
 constexpr long long kCallSeriesNs = 15000;
 constexpr int kCallSeries = 4;
+// Puts with signal: what the block copies as fast as two launches begin.  The four calls above with 32 / 64 / 128 / 256 / 400 / 512 KiB by launches
+// 33.9 / 34.4 / 34.4 / 34.4 / 34.3 / 34.6 us, so 25.8 / 26.2 / 26.9 / 30.0 / 33.0 / 40.0.  (Off each other's alignment kSmallSignalMax.)
+constexpr uint64_t kServedSignalMax = 256u << 10;
 __global__ void __launch_bounds__(kCallThreads) k_calls(State s, const CallSlot* slot, uint64_t* final, uint32_t seq, uint32_t generation) {
   __shared__ uint32_t req[kCallWords];
   __shared__ int over;
@@ -876,7 +879,8 @@ class GpuBackend final : public Backend {
     Lane& L = lane();
     const bool wait = !nbi && blocking_now();
     const Ticket t(wait ? &L : nullptr);
-    if (wait && (n == 0 || (tl_local_is_device && n <= kSmallSignalMax))) {
+    const bool skewed = (((reinterpret_cast<uintptr_t>(heap_->base[pe]) + dst_off) ^ reinterpret_cast<uintptr_t>(local)) & 15) != 0;
+    if (wait && (n == 0 || (tl_local_is_device && n <= (skewed ? kSmallSignalMax : kServedSignalMax)))) {
       Call call(CALL_PUT_SIGNAL, 0, sig_op, 0);
       call.set(CALL_ADDR, reinterpret_cast<uintptr_t>(heap_->base[pe] + dst_off)).set(CALL_VALUE, sig_val);
       call.set(CALL_OTHER, reinterpret_cast<uintptr_t>(local)).set(CALL_SIG, reinterpret_cast<uintptr_t>(heap_->base[pe] + sig_off));

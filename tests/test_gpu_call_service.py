@@ -132,3 +132,23 @@ def test_while_another_stream_is_captured(rt):
         assert bool((out == 1).all())
     finally:
         rt.set_stream(torch.cuda.current_stream())
+
+
+@pytest.mark.parametrize("n", [32768, 32769, 65536, 100_001, 262143, 262144, 262145])
+@pytest.mark.parametrize("skew", [0, 1, 4])
+def test_payloads_of_a_series(rt, n, skew):
+    """Both sides of what the block takes as a put with signal, on and off the two sides' common alignment."""
+    box, flag = rt.empty((n + 64,), torch.uint8), rt.zeros((1,), torch.int64)
+    src = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    for i in range(1, 13):
+        src.copy_(torch.randint(0, 256, (n + 64,), dtype=torch.uint8, device="cuda"))
+        box.fill_(7)
+        torch.cuda.synchronize()
+        for _ in range(6):
+            rt.g(flag, 0)                                  # a series is running
+        rt.put_signal(box[16 + skew:16 + skew + n], src[16:16 + n], flag, i, 0)
+        rt.wait_until(flag, "ge", i)
+        assert torch.equal(box[16 + skew:16 + skew + n], src[16:16 + n])
+        assert bool((box[:16 + skew] == 7).all()) and bool((box[16 + skew + n:] == 7).all())
+    rt.free(box, collective=False)
+    rt.free(flag, collective=False)
