@@ -385,7 +385,9 @@ __global__ void __launch_bounds__(512) k_put_signal(State s, char* dst, const ch
 // Blocking calls of the default context that follow one another closely need no launch each.  While one block on a stream of the
 // runtime's own looks at a slot in pinned memory, a call is a store by the host, the operation, and the answer in the call's own words:
 // 2.3 us where a launch and its answer take 6.6.  The calls belong behind what the caller's stream holds, so the host asks first
-// whether that stream is idle (1.4 us); if it is not, the call is a launch in that stream as ever.  No order is lost the other way: a
+// whether that stream is idle (1.4 us); if it is not, the call is a launch in that stream as ever.  Of a blocking stream that is not asked:
+// its launches wait for the legacy default stream, and its answer leaves out what is there; the legacy stream's own counts all that
+// its launches wait for.  No order is lost the other way: a
 // call has been answered before the caller enqueues anything else.  The first calls of a series are launches too, and a block that has
 // waited kCallIdleNs for a request, or lived for kCallLifeNs, ends: a device-wide synchronisation behind a series waits that long for it.
 // Fetch-add, put with signal of 4 KiB, wait and read, over and over: 32.8 us by launches, 22.5 so.  The
@@ -751,7 +753,10 @@ class GpuBackend final : public Backend {
 
   // ---- knobs used by the C entry points below ---------------------------------
   // (cudaStream_t)-1 selects the runtime's own stream; any other handle (0 = the legacy default stream) is used as given.
-  void set_stream(cudaStream_t s) { stream_ = (s == reinterpret_cast<cudaStream_t>(-1)) ? own_stream_ : s; }
+  void set_stream(cudaStream_t s) {
+    stream_ = (s == reinterpret_cast<cudaStream_t>(-1)) ? own_stream_ : s;
+    stream_tells_ = -1;
+  }
   cudaStream_t stream() const { return stream_; }
   void set_blocking(bool b) { blocking_ = b; }
   void set_coll_ctas(int n) { if (n >= 1 && n <= BSHMEM_MAX_COLL_CTAS) coll_ctas_ = n; }
@@ -806,14 +811,23 @@ class GpuBackend final : public Backend {
   // Whether the call has been carried out and answered() is true.  Where it is not, nothing has happened: the caller launches.
   template <class Answered>
   bool served(const Lane& L, const Ticket& t, Call& call, Answered answered) {
-    if (&L != &lanes_[0] || thread_is_bound()) return false;
+    if (&L != &lanes_[0] || thread_is_bound() || stream_tells_ == 0) return false;
     const std::unique_lock<std::mutex> lock(calls_mu_, std::try_to_lock);
     if (!lock) return false;
     const long long now = std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()).count();
     calls_close_ = now - calls_last_ < kCallSeriesNs ? calls_close_ + 1 : 0;
     calls_last_ = now;
     if (calls_close_ < kCallSeries) return false;
-    const RelaxedCapture relaxed;                    // the question is no part of another stream's capture
+    const RelaxedCapture relaxed;                    // the questions are no part of another stream's capture
+    if (stream_tells_ < 0) {                         // not where the stream is set: it may be capturing
+      unsigned flags = cudaStreamNonBlocking;
+      if (stream_ && stream_ != cudaStreamLegacy && cudaStreamGetFlags(stream_, &flags) != cudaSuccess) {
+        cudaGetLastError();
+        flags = 0;
+      }
+      stream_tells_ = (flags & cudaStreamNonBlocking) ? 1 : 0;
+      if (!stream_tells_) return false;
+    }
     if (cudaStreamQuery(stream_) != cudaSuccess) {
       cudaGetLastError();                            // "not ready" is not for somebody's next launch
       return false;
@@ -1286,6 +1300,7 @@ class GpuBackend final : public Backend {
   bool blocking_ = true;
   bool use_nvls_ = false;
   int coll_ctas_ = 32, sms_ = 0;
+  std::atomic<int> stream_tells_{1};    // whether its being idle says that its launches would run at once (see k_calls); -1: not known yet
   bool ring_wide_ = false;              // the device takes the cluster of k_ring_wide
   std::mutex calls_mu_;                 // one request at a time
   CallWriter calls_;

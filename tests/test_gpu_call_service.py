@@ -152,3 +152,40 @@ def test_payloads_of_a_series(rt, n, skew):
         assert bool((box[:16 + skew] == 7).all()) and bool((box[16 + skew + n:] == 7).all())
     rt.free(box, collective=False)
     rt.free(flag, collective=False)
+
+
+@pytest.fixture()
+def blocking_stream():
+    """A stream that the legacy default stream and it wait for one another (torch's own streams do not)."""
+    import ctypes as C
+    handle = C.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(C.addressof(handle))) == 0
+    yield torch.cuda.ExternalStream(handle.value)
+    torch.cuda.synchronize()
+    assert int(torch.cuda.cudart().cudaStreamDestroy(handle.value)) == 0
+
+
+@pytest.mark.parametrize("runtime_on", ["legacy", "blocking"])
+def test_work_that_the_stream_waits_for(rt, blocking_stream, runtime_on):
+    """The runtime on one of the legacy default stream and a blocking stream, work on the other one: a call follows it, as a launch would."""
+    word = rt.zeros((1,), torch.int64)
+    legacy = torch.cuda.default_stream()
+    mine, other = (legacy, blocking_stream) if runtime_on == "legacy" else (blocking_stream, legacy)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        torch.cuda._sleep(400_000)
+        word.add_(100)
+    torch.cuda.synchronize()
+    try:
+        rt.set_stream(mine)
+        with torch.cuda.stream(other):
+            for i in range(50):
+                rt.atomic_set(word, 0, 0)
+                torch.cuda.synchronize()
+                for _ in range(10):
+                    rt.g(word, 0)                          # a series is running
+                graph.replay()                             # some 200 us, launched in less time than ends a series
+                assert rt.atomic_fetch_add(word, 1, 0) == 100
+                assert rt.g(word, 0) == 101
+    finally:
+        rt.set_stream(torch.cuda.current_stream())
