@@ -391,8 +391,9 @@ __global__ void __launch_bounds__(512) k_put_signal(State s, char* dst, const ch
 // call has been answered before the caller enqueues anything else.  The first calls of a series are launches too, and a block that has
 // waited kCallIdleNs for a request, or lived for kCallLifeNs, ends: a device-wide synchronisation behind a series waits that long for it.
 // Fetch-add, put with signal of 4 KiB, wait and read, over and over: 32.8 us by launches, 22.5 so.  The
-// look at the slot is an acquire, so that the block sees what kernels wrote before the host asked; what it wrote itself is
-// visible before its answer.  call_service.h has the protocol.
+// look at the slot is an acquire, so that the block sees what kernels wrote before the host asked.  The block's stream is ordered against the
+// caller's by answers alone, so an answer comes when what the call did has been done at its place: an atomic's carries what was there, and a
+// fence stands between a signal and its answer.  call_service.h has the protocol.
 constexpr unsigned kCallThreads = 512;
 constexpr unsigned long long kCallIdleNs = 8000, kCallLifeNs = 500000;
 // From one call to the next of a series, on the host (a launch and its answer take 8 of that, a new block for the next call 12), and how many have to follow one another
@@ -448,6 +449,7 @@ __global__ void __launch_bounds__(kCallThreads) k_calls(State s, const CallSlot*
         if (threadIdx.x == 0) {
           dev::fence_peers(s);
           dev::signal_update(reinterpret_cast<uint64_t*>(pair(CALL_SIG)), value, op);
+          dev::fence_peers(s);         // no stream orders what follows the answer behind the signal
           signal_done(done);
         }
         break;

@@ -3,7 +3,8 @@ quiet publishes to the host too, whatever the PEs share; a fence orders for the 
 import re
 from pathlib import Path
 
-HEADER = Path(__file__).resolve().parents[1] / "roc_shmem_b200" / "csrc" / "include" / "bshmem_device.cuh"
+CSRC = Path(__file__).resolve().parents[1] / "roc_shmem_b200" / "csrc"
+HEADER = CSRC / "include" / "bshmem_device.cuh"
 
 
 def _body(name: str) -> str:
@@ -25,3 +26,12 @@ def test_fence_has_the_scope_of_its_peers():
     assert "fence_peers" in _body("fence")
     peers = _body("fence_peers")
     assert peers.index("one_gpu") < peers.index("fence.acq_rel.gpu") < peers.index("else") < peers.index("fence.acq_rel.sys")
+
+
+def test_a_served_signal_is_there_before_its_answer():
+    """k_calls answers from a stream of its own: payload, fence, signal, fence, answer."""
+    text = (CSRC / "cuda" / "gpu_backend.cu").read_text()
+    case = text[text.index("case CALL_PUT_SIGNAL:\n"):]
+    case = case[:case.index("break;")]
+    steps = re.findall(r"copy_bytes<|__syncthreads|fence_peers|signal_update|signal_done", case)
+    assert steps == ["copy_bytes<", "__syncthreads", "fence_peers", "signal_update", "fence_peers", "signal_done"]
