@@ -151,10 +151,12 @@ __global__ void __launch_bounds__(PTHREADS, 1) gemm_fp8_pair_kernel(const __grid
             const uint32_t buf = i & 1, drained = ((i >> 1) & 1) ^ 1;      // products alternate between two buffers, tiles are whole groups
             const uint64_t da = da0 + (uint64_t)((s * PSTAGE_BYTES) >> 4), db = db0 + (uint64_t)((s * PSTAGE_BYTES) >> 4);
             const uint32_t d = tmem_base + buf * 256;
+            // Asked ahead by every lane, and agreed on where it is needed: lanes need not see the same, and the waits are the whole warp's.
+            // One vote for the first two: 222 us for 4096 x 7168 x 8192, as without votes; a vote each 224.5, a reduction of all three 235.
             const bool there = ptx::mbar_test(L.full(s), ph);
             const bool free0 = ptx::mbar_test(L.part_empty(buf, 0), drained), free1 = ptx::mbar_test(L.part_empty(buf, 1), drained);
-            if (!there && !gemm2::warp_wait(L.full(s), ph, g, ERR_F8P_FULL)) { ok = false; break; }
-            if (!free0 && !gemm2::warp_wait(L.part_empty(buf, 0), drained, g, ERR_F8P_PART_EMPTY)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, there && free0) &&
+                !(gemm2::warp_wait(L.full(s), ph, g, ERR_F8P_FULL) && gemm2::warp_wait(L.part_empty(buf, 0), drained, g, ERR_F8P_PART_EMPTY))) { ok = false; break; }
             ptx::tc_fence_after();
             auto multiply = [&](int h) {
 #pragma unroll
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) gemm_fp8_pair_kernel(const __grid
               gemm2::umma2_commit_both(L.part_full(buf, h), 0);
             };
             if (leader) multiply(0);
-            if (!free1 && !gemm2::warp_wait(L.part_empty(buf, 1), drained, g, ERR_F8P_PART_EMPTY)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, free1) && !gemm2::warp_wait(L.part_empty(buf, 1), drained, g, ERR_F8P_PART_EMPTY)) { ok = false; break; }
             ptx::tc_fence_after();
             if (leader) {
               multiply(1);
