@@ -1364,8 +1364,8 @@ int bshmem_gpu_init(void* heap, const bshmem_config_t* cfg, int coll_ctas, int o
   auto* be = new GpuBackend(static_cast<gpu::Heap*>(heap), own_heap != 0);
   int rc = be->setup(c, coll_ctas);
   // Load every kernel of this library now.  With lazy module loading the first launch of a kernel
-  // can need a device-wide quiet point; if that first launch came from the proxy thread while a user
-  // kernel is spinning on the proxy's answer, neither would ever finish.
+  // can need a device-wide quiet point; if that first launch came from the proxy thread, or a host thread that
+  // answers, while a user kernel is spinning on the answer, neither would ever finish.
   {
     cudaFuncAttributes fa;
     cudaFuncGetAttributes(&fa, k_amo);
@@ -1376,6 +1376,8 @@ int bshmem_gpu_init(void* heap, const bshmem_config_t* cfg, int coll_ctas, int o
     cudaFuncGetAttributes(&fa, k_write_word);
     cudaFuncGetAttributes(&fa, k_copy_small);
     cudaFuncGetAttributes(&fa, k_ring);
+    cudaFuncGetAttributes(&fa, k_ring_wide);
+    cudaFuncGetAttributes(&fa, k_calls);
     cudaFuncGetAttributes(&fa, k_rma);
     cudaFuncGetAttributes(&fa, k_rma_bulk);
     collk::preload();
