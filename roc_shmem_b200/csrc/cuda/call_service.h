@@ -6,6 +6,9 @@
 //  - A block serves request after request, from the one it was launched for on, and ends after a while without one or at the end of its
 //    life.  Its last word, `final`, says up to which request it got: all of them have been answered, none behind them will be.
 //  - The host waits for the answer or for that word.  A request that the block left is given to the next block.
+//  - A block may be launched ahead of its first request (prepare) and is asked once it says that it is there (ready), so that no
+//    request waits for a place on the device: beside a kernel that leaves none, and that may itself wait for the call, the host launches
+//    what needs less of one.
 #pragma once
 #include <atomic>
 #include <cstdint>
@@ -31,12 +34,30 @@ struct Call {
 };
 struct CallSlot {                      // pinned host memory
   alignas(128) uint64_t w[16];
+  alignas(128) uint64_t begun;         // by the block at its start: its generation
   alignas(128) uint64_t final;         // by the block at its end: generation << 32 | the last request it answered
 };
 
 class CallWriter {
  public:
   CallSlot* slot = nullptr;
+
+  // All of it under the lock that makes the caller the only one.
+  // Launches a block for the requests to come, unless one may be taking them.
+  template <class Start>
+  bool prepare(Start start) {
+    if (serving_) return true;
+    if (start(seq_ + 1, generation_ + 1) != BSHMEM_OK) return false;
+    launched();
+    return true;
+  }
+  bool serving() const { return serving_; }
+  // Whether the block is there and has not ended yet, as far as the host can see.
+  bool ready() {
+    if (serving_ && ended()) serving_ = false;
+    return serving_ && word(slot->begun) == generation_;
+  }
+  unsigned taken() const { return taken_; }          // requests that the last block has answered
 
   // One request; the caller holds the lock that makes it the only one.  start(first, generation) launches a block that serves from request
   // `first` on, answered() looks at the caller's words, wait() returns when all blocks launched so far have ended; both return a
@@ -46,20 +67,21 @@ class CallWriter {
     const uint32_t seq = ++seq_;
     for (unsigned i = 0; i < kCallWords; ++i)
       reinterpret_cast<std::atomic<uint64_t>&>(slot->w[i]).store((uint64_t)seq << 32 | call.w[i], std::memory_order_release);
-    const auto& final = reinterpret_cast<const std::atomic<uint64_t>&>(slot->final);
     for (int attempt = 0; attempt < 2; ++attempt) {
       if (!serving_) {
         if (start(seq, generation_ + 1) != BSHMEM_OK) return false;
-        ++generation_;
-        serving_ = true;
+        launched();
       }
       for (unsigned it = 0;; ++it) {
-        if (answered()) return true;
-        const uint64_t f = final.load(std::memory_order_acquire);
-        if ((uint32_t)(f >> 32) == generation_) {
+        if (answered()) {
+          ++taken_;
+          return true;
+        }
+        if (ended()) {
           serving_ = false;
-          if ((int32_t)((uint32_t)f - seq) >= 0) return answered();       // the answer precedes this word
-          break;
+          if ((int32_t)((uint32_t)word(slot->final) - seq) < 0) break;
+          ++taken_;
+          return answered();                         // the answer precedes the last word
         }
         if (it == 4000) {
           if (wait() != BSHMEM_OK) return false;
@@ -74,7 +96,15 @@ class CallWriter {
   }
 
  private:
+  static uint64_t word(const uint64_t& w) { return reinterpret_cast<const std::atomic<uint64_t>&>(w).load(std::memory_order_acquire); }
+  bool ended() const { return (uint32_t)(word(slot->final) >> 32) == generation_; }
+  void launched() {
+    ++generation_;
+    serving_ = true;
+    taken_ = 0;
+  }
   uint32_t seq_ = 0, generation_ = 0;                // requests written, blocks launched
+  unsigned taken_ = 0;
   bool serving_ = false;                             // the last block may be taking requests
 };
 

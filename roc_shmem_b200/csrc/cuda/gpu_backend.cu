@@ -396,16 +396,17 @@ __global__ void __launch_bounds__(512) k_put_signal(State s, char* dst, const ch
 // fence stands between a signal and its answer.  call_service.h has the protocol.
 constexpr unsigned kCallThreads = 512;
 constexpr unsigned long long kCallIdleNs = 8000, kCallLifeNs = 500000;
-// From one call to the next of a series, on the host (a launch and its answer take 8 of that, a new block for the next call 12), and how many have to follow one another
-// so before the block is launched: single calls, a few of them and those with a synchronisation between them stay launches.
+// From one call to the next of a series, on the host (a launch and its answer take 8 of that), and how many have to follow one another
+// so before the block is launched, in the shadow of a call's own launch; it is asked when it says that it is there: single calls, a few of them and those with a synchronisation between them stay launches.
 constexpr long long kCallSeriesNs = 15000;
 constexpr int kCallSeries = 4;
 // Puts with signal: what the block copies as fast as two launches begin.  The four calls above with 32 / 64 / 128 / 256 / 400 / 512 KiB by launches
 // 33.9 / 34.4 / 34.4 / 34.4 / 34.3 / 34.6 us, so 25.8 / 26.2 / 26.9 / 30.0 / 33.0 / 40.0.  (Off each other's alignment kSmallSignalMax.)
 constexpr uint64_t kServedSignalMax = 256u << 10;
-__global__ void __launch_bounds__(kCallThreads) k_calls(State s, const CallSlot* slot, uint64_t* final, uint32_t seq, uint32_t generation) {
+__global__ void __launch_bounds__(kCallThreads) k_calls(State s, CallSlot* slot, uint32_t seq, uint32_t generation) {
   __shared__ uint32_t req[kCallWords];
   __shared__ int over;
+  if (threadIdx.x == 0) st_host(&slot->begun, generation);
   const int lane = threadIdx.x & 31;
   const unsigned long long begun = dev::timer();
   while (true) {
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(kCallThreads) k_calls(State s, const CallSlot*
     __syncthreads();
     ++seq;
   }
-  if (threadIdx.x == 0) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(final), "l"((uint64_t)generation << 32 | (seq - 1)) : "memory");
+  if (threadIdx.x == 0) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&slot->final), "l"((uint64_t)generation << 32 | (seq - 1)) : "memory");
 }
 
 // Runs after the payload copy on the same stream: publish, then update the signal word.
@@ -834,17 +835,25 @@ class GpuBackend final : public Backend {
       cudaGetLastError();                            // "not ready" is not for somebody's next launch
       return false;
     }
+    if (!calls_.ready()) {
+      calls_wanted_ = !calls_.serving();
+      return false;
+    }
     call.set(CALL_DONE, reinterpret_cast<uintptr_t>(t.done.word)).set(CALL_TOKEN, t.done.token);
-    return calls_.run(
-        call,
-        [&](uint32_t first, uint32_t generation) -> int {
-          RT_TRY(launch_small(k_calls, 1, kCallThreads, calls_stream_, state_, calls_.slot, &calls_.slot->final, first, generation));
-          return BSHMEM_OK;
-        },
-        answered, [&]() -> int {
-          RT_TRY(cudaStreamSynchronize(calls_stream_));
-          return BSHMEM_OK;
-        });
+    return calls_.run(call, [](uint32_t, uint32_t) -> int { return BSHMEM_ERR_STATE; }, answered, [&]() -> int {
+      RT_TRY(cudaStreamSynchronize(calls_stream_));  // the block is there: to its end
+      return BSHMEM_OK;
+    });
+  }
+  // Between a call's launch and its wait: the block for the calls to come, if the call would have liked one.
+  void prepare_calls() {
+    if (!calls_wanted_.load(std::memory_order_relaxed)) return;
+    const std::unique_lock<std::mutex> lock(calls_mu_, std::try_to_lock);
+    if (!lock || !calls_wanted_.exchange(false)) return;
+    calls_.prepare([&](uint32_t first, uint32_t generation) -> int {
+      RT_TRY(launch_small(k_calls, 1, kCallThreads, calls_stream_, state_, calls_.slot, first, generation));
+      return BSHMEM_OK;
+    });
   }
   bool served(const Lane& L, const Ticket& t, Call& call, uint64_t* result) {
     return served(L, t, call, [&] { return read_result(t, result); });
@@ -916,6 +925,7 @@ class GpuBackend final : public Backend {
     }
     e.enqueued();
     if (!wait) return BSHMEM_OK;
+    prepare_calls();
     const int rc = wait_done(t, st);
     return rc != BSHMEM_OK ? rc : check_device_error("put_signal");
   }
@@ -928,6 +938,7 @@ class GpuBackend final : public Backend {
     Entry e = enter(L);
     RT_TRY(launch_small(k_read_word, 1, 1, e.st, heap_->base[pe] + off, (int)size, t.done));
     e.enqueued();
+    prepare_calls();
     const int rc = wait_result(t, e.st, out);      // the value is the call's result: it is waited for in stream mode too
     if (rc != BSHMEM_OK) return rc;
     return blocking_now() ? check_device_error("get") : BSHMEM_OK;
@@ -955,6 +966,7 @@ class GpuBackend final : public Backend {
     RT_TRY(launch_small(k_amo, 1, 1, e.st, state_, pe, off, dtype, op, value, cond, t.done));
     e.enqueued();
     if (wait) {
+      prepare_calls();
       uint64_t old = 0;
       const int rc = wait_result(t, e.st, &old);
       if (rc != BSHMEM_OK) return rc;
@@ -1004,6 +1016,7 @@ class GpuBackend final : public Backend {
     RT_TRY(launch_small(k_wait_until, 1, 1, e.st, s, off, dtype, cmp, value, t.done));
     e.enqueued();
     if (!wait) return BSHMEM_OK;
+    prepare_calls();
     uint64_t status = 0;
     int rc = wait_result(t, e.st, &status);
     if (rc != BSHMEM_OK) return rc;
@@ -1305,6 +1318,7 @@ class GpuBackend final : public Backend {
   std::atomic<int> stream_tells_{1};    // whether its being idle says that its launches would run at once (see k_calls); -1: not known yet
   bool ring_wide_ = false;              // the device takes the cluster of k_ring_wide
   std::mutex calls_mu_;                 // one request at a time
+  std::atomic<bool> calls_wanted_{false};
   CallWriter calls_;
   cudaStream_t calls_stream_ = nullptr;
   long long calls_last_ = 0;            // when the last blocking call of the default context was made

@@ -90,3 +90,64 @@ def model(tmp_path_factory):
 def test_every_call_once(model, calls, looks, refuse, expect):
     r = model(calls, looks, refuse)
     assert r.returncode == 0 and r.stdout == f"wrong 0 refused {expect}\n", r.stdout + r.stderr
+
+
+# ---- a block that is launched ahead, on a device that may have no place for it ----
+AHEAD = MODEL[:MODEL.index("int main(")].replace("static void block(uint32_t seq", """static std::atomic<bool> place{true};
+static std::atomic<int> blocks_there{0};
+static void block_body(uint32_t, uint32_t, int);
+static void block(uint32_t seq, uint32_t generation, int looks) {
+  while (!place.load()) std::this_thread::yield();
+  ++blocks_there;
+  word(slot.begun).store(generation, std::memory_order_relaxed);
+  block_body(seq, generation, looks);
+}
+static void block_body(uint32_t seq""") + r"""
+int main(int, char** a) {
+  const int n = atoi(a[1]), looks = atoi(a[2]), full = atoi(a[3]);     // full: calls in a row without a place for a block
+  std::vector<std::thread> blocks;
+  CallWriter w;
+  w.slot = &slot;
+  std::mt19937 rng(looks);
+  int wrong = 0, served = 0, waited = 0;
+  for (int i = 0; i < n; ++i) {
+    if (full) place = i / full % 2 == 0;
+    Call call(CALL_AMO, 1, 2, 8);
+    call.set(CALL_VALUE, (uint64_t)i).set(CALL_TOKEN, (uint64_t)i + 1);
+    bool done = false;
+    if (w.ready()) {
+      done = w.run(call, [](uint32_t, uint32_t) { return (int)BSHMEM_ERR_STATE; },
+                   [&] { return (answer.load(std::memory_order_acquire) >> 32) == (uint64_t)i + 1; },
+                   [&] { waited += blocks_there.load() < (int)blocks.size(); std::this_thread::yield(); return (int)BSHMEM_OK; });
+      if (done) wrong += times[i] != 1 || (uint32_t)answer.load() != ((uint32_t)i ^ call.w[CALL_HEAD]);
+    }
+    if (done) ++served;
+    else {
+      wrong += times[i]++ != 0;                                          // by a launch
+      w.prepare([&](uint32_t first, uint32_t generation) {
+        blocks.emplace_back(block, first, generation, 1 + (int)(rng() % looks));
+        return (int)BSHMEM_OK;
+      });
+      for (unsigned k = rng() % 50; k; --k) std::this_thread::yield();
+    }
+  }
+  place = true;
+  for (auto& t : blocks) if (t.joinable()) t.join();
+  for (int i = 0; i < n; ++i) wrong += times[i] != 1;
+  printf("wrong %d waited %d served %s\n", wrong, waited, served ? "some" : "none");
+  return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("calls,looks,full", [(3000, 3000, 0), (3000, 3000, 100), (500, 20000, 500)])
+def test_no_call_waits_for_a_block_to_begin(tmp_path, calls, looks, full):
+    """Each call once, by the block or by a launch, also while a block that was launched has no place to run."""
+    if shutil.which("g++") is None:
+        pytest.skip("needs a C++ compiler")
+    (tmp_path / "ahead.cc").write_text(AHEAD)
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(CUDA), "-o", str(tmp_path / "ahead"), str(tmp_path / "ahead.cc"), "-lpthread"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([str(tmp_path / "ahead")] + [str(x) for x in (calls, looks, full)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "wrong 0 waited 0 served some\n", r.stdout + r.stderr
