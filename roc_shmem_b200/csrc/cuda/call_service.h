@@ -38,6 +38,50 @@ struct CallSlot {                      // pinned host memory
   alignas(128) uint64_t final;         // by the block at its end: generation << 32 | the last request it answered
 };
 
+// Which calls are worth the question whether their stream is idle, and a block: those that follow some others closely.  How many others is
+// what the program's calls have been like: a refusal (the stream holds something) and a block that ended after a few requests make it
+// more, a block that was worth its launch brings it back.  So a program that mostly enqueues work between its calls, or synchronises
+// behind a few of them, asks once in a while and otherwise calls as if there were no blocks.
+class CallSeries {
+ public:
+  static constexpr long long kCloseNs = 15000;       // from one call to the next (a launch and its answer take 8 of that)
+  static constexpr unsigned kFew = 4, kMany = 64, kWorth = 16;
+  bool long_enough(long long now_ns) {               // a call; whether it is to be asked for
+    close_ = now_ns - last_ < kCloseNs ? close_ + 1 : 0;
+    last_ = now_ns;
+    return long_enough();
+  }
+  bool long_enough() const { return close_ >= needed_; }
+  void refused() {
+    needed_ = 2 * needed_ < kMany ? 2 * needed_ : kMany;
+    close_ = 0;
+  }
+  void ended(unsigned taken) {                       // a block, after so many requests
+    if (taken >= kWorth) needed_ = kFew;
+    else refused();
+  }
+
+ private:
+  long long last_ = -kCloseNs;
+  unsigned close_ = 0, needed_ = kFew;
+};
+// The same for what a call asks ahead of its own launch: not again for a while after an answer that it had no use for.
+class AskAhead {
+ public:
+  bool now() {
+    if (skip_ == 0) return true;
+    --skip_;
+    return false;
+  }
+  void told(bool useful) {
+    missed_ = useful ? 0 : 2 * missed_ + 1 < 63 ? 2 * missed_ + 1 : 63;
+    skip_ = missed_;
+  }
+
+ private:
+  unsigned skip_ = 0, missed_ = 0;
+};
+
 class CallWriter {
  public:
   CallSlot* slot = nullptr;

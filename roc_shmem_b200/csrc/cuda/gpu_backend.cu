@@ -388,18 +388,17 @@ __global__ void __launch_bounds__(512) k_put_signal(State s, char* dst, const ch
 // whether that stream is idle (1.4 us); if it is not, the call is a launch in that stream as ever.  Of a blocking stream that is not asked:
 // its launches wait for the legacy default stream, and its answer leaves out what is there; the legacy stream's own counts all that
 // its launches wait for.  No order is lost the other way: a
-// call has been answered before the caller enqueues anything else.  The first calls of a series are launches too, and a block that has
-// waited kCallIdleNs for a request, or lived for kCallLifeNs, ends: a device-wide synchronisation behind a series waits that long for it.
-// Fetch-add, put with signal of 4 KiB, wait and read, over and over: 32.8 us by launches, 22.5 so.  The
+// call has been answered before the caller enqueues anything else.  A block that has waited kCallIdleNs for a request, or lived for kCallLifeNs,
+// ends: until then a device-wide synchronisation waits for it, and a kernel that wants every multiprocessor for one of them (with 5 us the gaps of
+// a loop of calls end it).  So blocks are launched, in the shadow of a call's own launch, where the program has had a use for them
+// (CallSeries), and asked when they say that they are there.  us, by launches / so: fetch-add, put with signal of 4 KiB, wait and read, over and
+// over 33.9 / 25.5; with a device-wide synchronisation behind each of these passes 40.0 / 40.7 (45.3 while every series had its block); a
+// kernel, then a call 13.9 / 14.0 (14.5 while every series asked); a kernel, then two 21.8 / 22.1 (23.0); single passes the same.  The
 // look at the slot is an acquire, so that the block sees what kernels wrote before the host asked.  The block's stream is ordered against the
 // caller's by answers alone, so an answer comes when what the call did has been done at its place: an atomic's carries what was there, and a
 // fence stands between a signal and its answer.  call_service.h has the protocol.
 constexpr unsigned kCallThreads = 512;
 constexpr unsigned long long kCallIdleNs = 8000, kCallLifeNs = 500000;
-// From one call to the next of a series, on the host (a launch and its answer take 8 of that), and how many have to follow one another
-// so before the block is launched, in the shadow of a call's own launch; it is asked when it says that it is there: single calls, a few of them and those with a synchronisation between them stay launches.
-constexpr long long kCallSeriesNs = 15000;
-constexpr int kCallSeries = 4;
 // Puts with signal: what the block copies as fast as two launches begin.  The four calls above with 32 / 64 / 128 / 256 / 400 / 512 KiB by launches
 // 33.9 / 34.4 / 34.4 / 34.4 / 34.3 / 34.6 us, so 25.8 / 26.2 / 26.9 / 30.0 / 33.0 / 40.0.  (Off each other's alignment kSmallSignalMax.)
 constexpr uint64_t kServedSignalMax = 256u << 10;
@@ -813,14 +812,12 @@ class GpuBackend final : public Backend {
   // ---- blocking calls through a block that is there already (see k_calls) ----------------
   // Whether the call has been carried out and answered() is true.  Where it is not, nothing has happened: the caller launches.
   template <class Answered>
-  bool served(const Lane& L, const Ticket& t, Call& call, Answered answered) {
+  bool served(const Lane& L, const Ticket& t, Call& call, Answered answered, AskAhead* ahead = nullptr) {
     if (&L != &lanes_[0] || thread_is_bound() || stream_tells_ == 0) return false;
     const std::unique_lock<std::mutex> lock(calls_mu_, std::try_to_lock);
     if (!lock) return false;
     const long long now = std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()).count();
-    calls_close_ = now - calls_last_ < kCallSeriesNs ? calls_close_ + 1 : 0;
-    calls_last_ = now;
-    if (calls_close_ < kCallSeries) return false;
+    if (!series_.long_enough(now) || (ahead && !ahead->now())) return false;
     const RelaxedCapture relaxed;                    // the questions are no part of another stream's capture
     if (stream_tells_ < 0) {                         // not where the stream is set: it may be capturing
       unsigned flags = cudaStreamNonBlocking;
@@ -831,32 +828,43 @@ class GpuBackend final : public Backend {
       stream_tells_ = (flags & cudaStreamNonBlocking) ? 1 : 0;
       if (!stream_tells_) return false;
     }
-    if (cudaStreamQuery(stream_) != cudaSuccess) {
+    // a launch of this lane's last call has answered, and may be about to end
+    int asks = calls_served_ ? 1 : 4;
+    calls_served_ = false;
+    while (cudaStreamQuery(stream_) != cudaSuccess) {
       cudaGetLastError();                            // "not ready" is not for somebody's next launch
+      if (--asks) continue;
+      series_.refused();
       return false;
     }
-    if (!calls_.ready()) {
-      calls_wanted_ = !calls_.serving();
-      return false;
+    bool done = false;
+    if (calls_.ready()) {
+      call.set(CALL_DONE, reinterpret_cast<uintptr_t>(t.done.word)).set(CALL_TOKEN, t.done.token);
+      done = calls_.run(call, [](uint32_t, uint32_t) -> int { return BSHMEM_ERR_STATE; }, answered, [&]() -> int {
+        RT_TRY(cudaStreamSynchronize(calls_stream_));  // the block is there: to its end
+        return BSHMEM_OK;
+      });
     }
-    call.set(CALL_DONE, reinterpret_cast<uintptr_t>(t.done.word)).set(CALL_TOKEN, t.done.token);
-    return calls_.run(call, [](uint32_t, uint32_t) -> int { return BSHMEM_ERR_STATE; }, answered, [&]() -> int {
-      RT_TRY(cudaStreamSynchronize(calls_stream_));  // the block is there: to its end
-      return BSHMEM_OK;
-    });
+    if (calls_block_ && !calls_.serving()) {
+      calls_block_ = false;
+      series_.ended(calls_.taken());
+    }
+    calls_wanted_ = !done && !calls_block_ && series_.long_enough();
+    calls_served_ = done;
+    return done;
   }
   // Between a call's launch and its wait: the block for the calls to come, if the call would have liked one.
   void prepare_calls() {
     if (!calls_wanted_.load(std::memory_order_relaxed)) return;
     const std::unique_lock<std::mutex> lock(calls_mu_, std::try_to_lock);
     if (!lock || !calls_wanted_.exchange(false)) return;
-    calls_.prepare([&](uint32_t first, uint32_t generation) -> int {
+    calls_block_ = calls_.prepare([&](uint32_t first, uint32_t generation) -> int {
       RT_TRY(launch_small(k_calls, 1, kCallThreads, calls_stream_, state_, calls_.slot, first, generation));
       return BSHMEM_OK;
     });
   }
-  bool served(const Lane& L, const Ticket& t, Call& call, uint64_t* result) {
-    return served(L, t, call, [&] { return read_result(t, result); });
+  bool served(const Lane& L, const Ticket& t, Call& call, uint64_t* result, AskAhead* ahead = nullptr) {
+    return served(L, t, call, [&] { return read_result(t, result); }, ahead);
   }
 
   int check_device_error(const char* what) {
@@ -1009,7 +1017,12 @@ class GpuBackend final : public Backend {
       Call call(CALL_TEST, dtype, cmp, 0);
       call.set(CALL_ADDR, reinterpret_cast<uintptr_t>(local_base() + off)).set(CALL_VALUE, value);
       uint64_t answer = 0;
-      if (served(L, asked, call, &answer) && (uint32_t)answer == BSHMEM_OK) return BSHMEM_OK;
+      if (served(L, asked, call, &answer, &waits_)) {
+        const bool holds = (uint32_t)answer == BSHMEM_OK;
+        const std::lock_guard<std::mutex> lock(calls_mu_);
+        waits_.told(holds);
+        if (holds) return BSHMEM_OK;
+      }
     }
     const Ticket t(wait ? &L : nullptr);
     Entry e = enter(L);
@@ -1319,10 +1332,12 @@ class GpuBackend final : public Backend {
   bool ring_wide_ = false;              // the device takes the cluster of k_ring_wide
   std::mutex calls_mu_;                 // one request at a time
   std::atomic<bool> calls_wanted_{false};
+  bool calls_block_ = false;            // launched, and not seen to have ended
+  bool calls_served_ = false;           // the last call was carried out by a block
+  CallSeries series_;
+  AskAhead waits_;
   CallWriter calls_;
   cudaStream_t calls_stream_ = nullptr;
-  long long calls_last_ = 0;            // when the last blocking call of the default context was made
-  int calls_close_ = 0;                 // how many have followed their predecessor closely
   Lane lanes_[BSHMEM_MAX_CTXS];
   unsigned long long ll_epoch_ = 0;     // epochs of host-launched low-latency allreduces
   unsigned long long stage_seq_ = 0;    // call numbers of staged one-exchange collectives

@@ -151,3 +151,52 @@ def test_no_call_waits_for_a_block_to_begin(tmp_path, calls, looks, full):
     assert r.returncode == 0, r.stderr[-3000:]
     r = subprocess.run([str(tmp_path / "ahead")] + [str(x) for x in (calls, looks, full)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "wrong 0 waited 0 served some\n", r.stdout + r.stderr
+
+
+# ---- when a call asks ----
+POLICY = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "call_service.h"
+using namespace bshmem;
+int main(int, char** a) {
+  // `calls` calls `gap` ns apart, a kernel before every `every`-th of them (0: none), a block for every series that ends after `taken` requests
+  const int calls = atoi(a[1]), gap = atoi(a[2]), every = atoi(a[3]), taken = atoi(a[4]);
+  CallSeries s;
+  int asked = 0, refused = 0, blocks = 0, left = 0;
+  for (int i = 0; i < calls; ++i) {
+    if (!s.long_enough((long long)i * gap + 1000000)) continue;
+    ++asked;
+    if (every && i % every == 0) { s.refused(); ++refused; continue; }
+    if (left == 0) { ++blocks; left = taken; }
+    else if (--left == 0) s.ended((unsigned)taken);
+  }
+  AskAhead w;
+  int useless = 0;
+  for (int i = 0; i < calls; ++i)
+    if (w.now()) { ++useless; w.told(false); }
+  w.told(true);
+  printf("%d %d %d %d %d\n", asked, refused, blocks, useless, (int)w.now());
+  return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("calls,gap,every,taken,most_asked,most_refused,most_blocks", [
+    (10000, 20000, 0, 90, 0, 0, 0),             # no series
+    (10000, 8000, 0, 90, 10000, 0, 120),        # a loop of calls: a block for every 90 of them
+    (10000, 8000, 1, 90, 180, 180, 0),          # a kernel before each: asked every 65th time
+    (10000, 8000, 0, 3, 700, 0, 170),           # blocks that end after 3: one for some 65 calls
+])
+def test_a_program_that_has_no_use_for_blocks_does_not_pay_for_them(tmp_path, calls, gap, every, taken, most_asked, most_refused, most_blocks):
+    if shutil.which("g++") is None:
+        pytest.skip("needs a C++ compiler")
+    (tmp_path / "policy.cc").write_text(POLICY)
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(CUDA), "-o", str(tmp_path / "policy"), str(tmp_path / "policy.cc")],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = subprocess.run([str(tmp_path / "policy")] + [str(x) for x in (calls, gap, every, taken)], capture_output=True, text=True, timeout=60).stdout
+    asked, refused, blocks, useless, again = map(int, out.split())
+    assert asked <= most_asked and refused <= most_refused and blocks <= most_blocks, out
+    assert most_blocks != 120 or (asked > 9900 and blocks > 100), out
+    assert useless <= calls // 60 and again == 1, out
