@@ -295,76 +295,143 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next
   if (threadIdx.x == kRingPublisher) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
 }
 
-// The same by a cluster of eight blocks, for messages that one block is too slow for.  The first block looks at the ring and tells
-// the others what it found; the batch is copied in pieces of 4 KiB, one round trip to memory of a warp, by the warps of all blocks
-// in turn.  Windows of 64 puts, us, by a launch each (2.1 to 2.5 us apart, the host's) and so: 17 KB 159 -> 55, 64 KiB 159 -> 70, 256 KiB
-// 160 -> 95, 512 KiB 152 to 160 -> 140, 1 MiB 147 -> 232; hence the limit.  Up to 16 KiB one block is as fast (8 KiB 46, the cluster 54) and holds
-// one multiprocessor, not eight: products of 1024 rows with 64 messages of 64 KiB before each take 67 us (164 by launches, 47 alone),
-// with four 52 (47).  Ending after 2 us without a message instead of 5 changes neither.
-constexpr unsigned kRingBlocks = 8, kRingPiece = 4096;
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// The same by several blocks, for messages that one block is too slow for.  The first block to run looks at the ring; those that have
+// come by the time it finds messages take their part of them, pieces of 4 KiB, one round trip to memory of a warp, in turn.  None of them is
+// needed: beside a kernel that leaves a single place, of what a launch per message took, the first block does all, and the rest pass
+// through behind it.  (As a cluster of eight blocks of 512 threads, all of which had to find their places at once, this had no progress there.)
+// Windows of 64 puts, us, by a launch each (2.3 to 2.7 us apart, the host's) / as a cluster / so: 17 KB 175 / 60 / 44, 64 KiB 175 / 68 / 47, 256 KiB
+// 175 / 94 / 66, 512 KiB 175 / 140 / 95.  Up to 16 KiB one block is as fast (8 KiB 45) and holds one multiprocessor.  Products of 1024 rows with 64
+// messages of 64 KiB before each 180 / 71 / 57, with four 47.8 / 52 / 48.2 (without any 41.5).  All of it in this GPU's own memory; a
+// peer's is behind a link, where a block moves less.
+constexpr unsigned kWideThreads = 256, kWideBlocks = 16, kWideWarps = kWideThreads / 32, kWidePublisher = kWideThreads - 32, kRingPiece = 4096;
+constexpr unsigned long long kWideLimitNs = 2000000000;        // of the waits for one another, each of which ends by itself
+struct RingShare {                     // device memory, zero between launches
+  unsigned long long batch;            // by the first block: the batch's number | how many blocks it is for; number ~0: no more
+  unsigned int came, done, left;       // blocks: begun, finished with their parts (of all batches), ended
+  RingMessages b;
+};
+__device__ __forceinline__ void copy_pieces(const RingMessages& b, int count, unsigned piece, unsigned step) {
+  unsigned first = 0;
+  for (int m = 0; m < count; ++m) {
+    const uint32_t n = b.msg[m].n, pieces = (n + kRingPiece - 1) / kRingPiece;
+    for (; piece - first < pieces; piece += step) {
+      const uint32_t at = (piece - first) * kRingPiece;
+      dev::copy_bytes<dev::WARP>(b.msg[m].dst + at, b.msg[m].src + at, min(kRingPiece, n - at));
+    }
+    first += pieces;
+  }
 }
-__global__ void __launch_bounds__(kRingThreads) k_ring_wide(Ring* ring, uint32_t next, uint32_t generation) {
-  after_predecessor();
-  __shared__ RingMessages b;
-  static_assert(sizeof(RingMessages) % 4 == 0, "passed on in words");
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, block = blockIdx.x;
+__device__ __forceinline__ void ring_share_out(Ring* ring, RingShare* share, RingMessages& b, uint32_t next, uint32_t generation) {
+  __shared__ unsigned blocks;          // that the batch is for
+  __shared__ int failed;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long begun = dev::timer();
   unsigned long long last = begun;
+  unsigned batch = 0, parts = 0;       // of the publisher: the others' parts handed out so far
   bool closing = false;
-  cluster_barrier();                                           // every block's memory is there to be written to
+  if (threadIdx.x == 0) failed = 0;
   while (true) {
-    if (block == 0 && warp == 0) {
+    if (warp == 0) {
       do ring_look(ring, next, generation, lane, closing, begun, last, b);
       while (b.found == 0 && b.over == 0);
-      const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&b);
-      for (unsigned i = lane; i < sizeof(RingMessages) / 4; i += 32) {
-        const uint32_t word = reinterpret_cast<const uint32_t*>(&b)[i];
-        for (unsigned r = 1; r < kRingBlocks; ++r) {
-          uint32_t there;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine + i * 4), "r"(r));
-          asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"(word) : "memory");
+    }
+    __syncthreads();                   // the others' parts of the last batch are done, too
+    const int count = b.found, end = b.over;
+    if (failed) break;
+    if (count) {
+      if (warp == 0) {
+        unsigned pieces = lane < count ? (b.msg[lane].n + kRingPiece - 1) / kRingPiece : 0;
+        pieces = __reduce_add_sync(0xffffffffu, pieces);
+        unsigned here = 1;
+        if (pieces > kWideWarps) {
+          for (unsigned i = lane; i < sizeof(RingMessages) / 4; i += 32) reinterpret_cast<uint32_t*>(&share->b)[i] = reinterpret_cast<const uint32_t*>(&b)[i];
+          asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(&share->came) : "memory");
+          here = __shfl_sync(0xffffffffu, here, 0);
+          __syncwarp();
+        }
+        if (lane == 0) {
+          blocks = here;
+          if (here > 1) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(&share->batch), "l"((unsigned long long)(batch + 1) << 32 | here) : "memory");
+        }
+      }
+      __syncthreads();
+      const unsigned here = blocks;
+      batch += here > 1;
+      copy_pieces(b, count, warp, here * kWideWarps);
+      __syncthreads();
+      next += count;
+      // one thread waits for the others' parts and says how far the messages are done, while the first warp looks for more
+      if (threadIdx.x == kWidePublisher) {
+        parts += here - 1;
+        bool ok = here == 1;
+        for (const unsigned long long t0 = dev::timer(); !ok && dev::timer() - t0 < kWideLimitNs;) {
+          unsigned done;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(&share->done) : "memory");
+          ok = done == parts;
+        }
+        if (ok) {
+          asm volatile("fence.acq_rel.sys;" ::: "memory");
+          st_host(&ring->consumed, next);
+        } else {
+          failed = 1;
+          st_host(&ring->failed, generation);
         }
       }
     }
-    cluster_barrier();
-    const int count = b.found, end = b.over;
-    unsigned piece = block * kRingBatch + warp, first = 0;
-    for (int m = 0; m < count; ++m) {
-      const uint32_t n = b.msg[m].n, pieces = (n + kRingPiece - 1) / kRingPiece;
-      for (; piece - first < pieces; piece += kRingBlocks * kRingBatch) {
-        const uint32_t at = (piece - first) * kRingPiece;
-        dev::copy_bytes<dev::WARP>(b.msg[m].dst + at, b.msg[m].src + at, min(kRingPiece, n - at));
-      }
-      first += pieces;
-    }
-    cluster_barrier();                                         // all of it is copied, and the batch has been read
-    next += count;
-    if (block == 0 && count) ring_publish(ring, next);
-    if (block == 0 && threadIdx.x == 0 && end == 1) {
-      st_host(&ring->closed, generation);
-      asm volatile("fence.sc.sys;" ::: "memory");
-    }
     if (end == 2) break;
-    if (end == 1) closing = true;
+    if (end == 1) {
+      if (threadIdx.x == 0) {
+        st_host(&ring->closed, generation);
+        asm volatile("fence.sc.sys;" ::: "memory");
+      }
+      closing = true;
+    }
     __syncwarp();
   }
-  if (block == 0 && threadIdx.x == kRingPublisher)
-    asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(&share->batch), "l"(~0ull) : "memory");
+  if (threadIdx.x == kWidePublisher) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&ring->final), "l"((uint64_t)generation << 32 | next) : "memory");
 }
-cudaLaunchConfig_t ring_wide_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kRingBlocks);
-  cfg.blockDim = dim3(kRingThreads);
-  cfg.stream = st;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kRingBlocks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return cfg;
+__device__ __forceinline__ void ring_take_part(RingShare* share, RingMessages& b, unsigned me) {
+  __shared__ unsigned blocks;          // that the batch is for; 0: no more
+  unsigned seen = 0;                   // thread 0's
+  while (true) {
+    if (threadIdx.x == 0) {
+      unsigned long long v = 0;
+      const unsigned long long t0 = dev::timer();
+      do {
+        if (dev::timer() - t0 > 2 * kWideLimitNs) v = ~0ull;   // beyond what the first block lives and waits
+        else asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&share->batch) : "memory");
+        if (v != ~0ull && me >= (unsigned)v) seen = (unsigned)(v >> 32);    // not for this block
+      } while ((unsigned)(v >> 32) == seen);
+      seen = (unsigned)(v >> 32);
+      blocks = v == ~0ull ? 0 : (unsigned)v;
+    }
+    __syncthreads();
+    const unsigned here = blocks;
+    if (!here) return;
+    for (unsigned i = threadIdx.x; i < sizeof(RingMessages) / 4; i += kWideThreads)
+      reinterpret_cast<uint32_t*>(&b)[i] = __ldcg(reinterpret_cast<const uint32_t*>(&share->b) + i);
+    __syncthreads();
+    copy_pieces(b, b.found, me * kWideWarps + (threadIdx.x >> 5), here * kWideWarps);
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&share->done) : "memory");
+  }
+}
+__global__ void __launch_bounds__(kWideThreads) k_ring_wide(Ring* ring, RingShare* share, uint32_t next, uint32_t generation) {
+  after_predecessor();
+  __shared__ RingMessages b;
+  __shared__ unsigned order;
+  static_assert(sizeof(RingMessages) % 4 == 0, "passed on in words");
+  if (threadIdx.x == 0) order = atomicAdd(&share->came, 1u);
+  __syncthreads();
+  if (order == 0) ring_share_out(ring, share, b, next, generation);
+  else ring_take_part(share, b, order);
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&share->left, 1u) == gridDim.x - 1) {      // nobody looks at it any more
+    share->batch = 0;
+    share->came = share->done = share->left = 0;
+  }
 }
 
 // Payload and signal of a small message in one block: the block barrier orders every thread's stores before the
@@ -546,6 +613,7 @@ struct Lane {
   std::atomic<bool> taken[kResultSlots] = {};      // slots whose call still waits for its answer
   bool open = false;
   RingWriter ring;                                 // of a context other than the default one, whose stream the caller owns (see k_ring)
+  RingShare* share = nullptr;                      // of the ring's blocks
 };
 
 // A waiting call's own result slot of its lane, from before the launch until the answer has been read: threads that share the
@@ -629,11 +697,6 @@ class GpuBackend final : public Backend {
     RT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, heap_->device));
     if (coll_ctas_ > sms) coll_ctas_ = sms;
     sms_ = sms;
-    cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t wide = ring_wide_config(attr, nullptr);
-    int clusters = 0;
-    ring_wide_ = cudaOccupancyMaxActiveClusters(&clusters, k_ring_wide, &wide) == cudaSuccess && clusters > 0;
-    if (!ring_wide_) cudaGetLastError();
     return BSHMEM_OK;
   }
 
@@ -675,6 +738,8 @@ class GpuBackend final : public Backend {
     Ring* ring = nullptr;
     RT_TRY(cudaHostAlloc(&ring, sizeof(Ring), cudaHostAllocMapped));
     memset(ring, 0, sizeof(Ring));
+    RT_TRY(cudaMalloc(&L.share, sizeof(RingShare)));
+    RT_TRY(cudaMemset(L.share, 0, sizeof(RingShare)));
     L.ring.open(ring);
     L.open = true;
     return BSHMEM_OK;
@@ -688,6 +753,7 @@ class GpuBackend final : public Backend {
     if (L.pinned) { cudaFreeHost(L.pinned); L.pinned = nullptr; }
     if (L.dstatus) { cudaFree(L.dstatus); L.dstatus = nullptr; }
     if (L.ring.ring) { cudaFreeHost(L.ring.ring); L.ring.ring = nullptr; }
+    if (L.share) { cudaFree(L.share); L.share = nullptr; }
   }
   void ctx_select(int idx) override { tl_selected_ctx = idx; }
   // Everything the calling thread issues from now on (collectives too) runs on context idx's lane; -1 unbinds.
@@ -721,7 +787,7 @@ class GpuBackend final : public Backend {
   }
   bool ring_takes(const Lane& L, const void* a, const void* b, uint64_t n, bool nbi) const {
     const bool skewed = ((reinterpret_cast<uintptr_t>(a) ^ reinterpret_cast<uintptr_t>(b)) & 15) != 0;
-    return nbi && tl_local_is_device && n > 0 && n <= (!ring_wide_ ? kRingNarrowMax : skewed ? kSmallCopyMaxSkewed : kRingMessageMax) && L.ring.ring &&
+    return nbi && tl_local_is_device && n > 0 && n <= (skewed ? kSmallCopyMaxSkewed : kRingMessageMax) && L.ring.ring &&
            !thread_is_bound() &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) >> 48) == 0;
   }
@@ -729,13 +795,8 @@ class GpuBackend final : public Backend {
     const int rc = L.ring.message(
         reinterpret_cast<uintptr_t>(dst), reinterpret_cast<uintptr_t>(src), n,
         [&](uint32_t from, uint32_t generation) -> int {
-          if (n > kRingNarrowMax) {
-            cudaLaunchAttribute attr[2];
-            const cudaLaunchConfig_t cfg = ring_wide_config(attr, L.stream);
-            RT_TRY(cudaLaunchKernelEx(&cfg, k_ring_wide, L.ring.ring, from, generation));
-          } else {
-            RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
-          }
+          if (n > kRingNarrowMax) RT_TRY(launch_small(k_ring_wide, kWideBlocks, kWideThreads, L.stream, L.ring.ring, L.share, from, generation));
+          else RT_TRY(launch_small(k_ring, 1, kRingThreads, L.stream, L.ring.ring, from, generation));
           return BSHMEM_OK;
         },
         [&](auto arrived) {
@@ -1005,6 +1066,10 @@ class GpuBackend final : public Backend {
     }
     const cudaStream_t st = enter(L).st;
     RT_TRY(cudaStreamSynchronize(st));
+    if (L.ring.ring && L.ring.failed()) {
+      tl_err = "the context's messages were not taken";
+      return BSHMEM_ERR_STATE;
+    }
     return check_device_error("quiet");
   }
   int wait_until(uint64_t off, int dtype, int cmp, uint64_t value, uint64_t timeout_us) override {
@@ -1329,7 +1394,6 @@ class GpuBackend final : public Backend {
   bool use_nvls_ = false;
   int coll_ctas_ = 32, sms_ = 0;
   std::atomic<int> stream_tells_{1};    // whether its being idle says that its launches would run at once (see k_calls); -1: not known yet
-  bool ring_wide_ = false;              // the device takes the cluster of k_ring_wide
   std::mutex calls_mu_;                 // one request at a time
   std::atomic<bool> calls_wanted_{false};
   bool calls_block_ = false;            // launched, and not seen to have ended

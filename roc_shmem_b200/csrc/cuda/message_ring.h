@@ -1,4 +1,4 @@
-// message_ring.h — the ring through which a context's non-blocking messages reach the block, or the cluster of blocks, that serves it
+// message_ring.h — the ring through which a context's non-blocking messages reach the block, or the blocks, that serve it
 // (k_ring and k_ring_wide in gpu_backend.cu): its words, and the host's side.  Plain C++ but for the annotations, so that the two
 // sides' protocol also runs as host threads (tests/test_cpu_message_ring.py, tests/test_cpu_message_ring_sizes.py).
 //
@@ -10,8 +10,8 @@
 //    at the ring then, and must leave that message alone.
 //  - Messages between two fences of the context are unordered, as the API has it, except that one which touches what an
 //    earlier one touches waits for it, as does the first behind a fence (kRingOrdered).
-//  - One block takes messages of up to kRingNarrowMax bytes, a cluster of blocks all.  A longer message that finds the one block
-//    tells it to end, as an operation would, and is for the cluster behind it, which takes the short ones that follow as well.
+//  - One block takes messages of up to kRingNarrowMax bytes, several all.  A longer message that finds the one block
+//    tells it to end, as an operation would, and is for the blocks behind it, which take the short ones that follow as well.
 //  - A block that ends says so first (closed), then looks for messages once more; the host looks at `closed` behind each message
 //    that it has written.  One of the two sees the other, and `final` says how far the block got.  A message that it left is
 //    given to the next block.
@@ -39,6 +39,7 @@ struct Ring {                          // pinned host memory
   alignas(64) uint64_t final;          // by the block at its end: generation << 32 | messages taken since the ring exists
   alignas(64) uint64_t consumed;       // by the block: messages done since the ring exists (32 bits)
   alignas(64) uint64_t stop;           // by the host: this generation, and those before it, are to end
+  alignas(64) uint64_t failed;         // by the block, should blocks wait for one another in vain: its generation.  (In front of `stop`: a window 1.5 us longer.)
 };
 // What stands beside the words of message `index`: 16 bits that differ from those of the message that the slot held before; and
 // the generation beside the size (a block's successor starts at its end, so 15 bits do).
@@ -82,8 +83,9 @@ class RingWriter {
     return serving_;
   }
   bool done(uint32_t head) const { return (int32_t)(consumed() - head) >= 0; }
+  bool failed() const { return word(ring->failed) != 0; }
 
-  // One message.  start(from, generation) launches what serves the ring from message `from` on, a cluster for a message of more than
+  // One message.  start(from, generation) launches what serves the ring from message `from` on, several blocks for a message of more than
   // kRingNarrowMax bytes; wait(arrived) returns when arrived() or at the end of all blocks launched so far.  Both return a status;
   // BSHMEM_ERR_STATE: the blocks have ended without it.
   template <class Start, class Wait>
@@ -152,7 +154,7 @@ class RingWriter {
 
   std::mutex mu_;
   uint32_t head_ = 0, generation_ = 0;               // messages written, blocks launched
-  bool serving_ = false, wide_ = false;              // the last block, a cluster of them if wide_, may be taking messages
+  bool serving_ = false, wide_ = false;              // the last block, several of them if wide_, may be taking messages
   bool order_next_ = false;
   struct Span { uint64_t dst, src; uint32_t n; } recent_[16];      // messages since the last ordered one
   int n_recent_ = 0;

@@ -1,4 +1,4 @@
-"""Long non-blocking messages of a context (the ring's cluster of blocks): sizes around its pieces and its limits, mixed with short ones, off
+"""Long non-blocking messages of a context (the ring's form of several blocks): sizes around its pieces and its limits, mixed with short ones, off
 16-byte boundaries, in both directions, behind one another where they touch, and around operations of the context."""
 import pytest
 import torch
@@ -97,7 +97,7 @@ def test_more_than_the_ring_holds(rt, ctx):
 
 
 def test_what_the_stream_wrote_before(rt, ctx):
-    """The messages of a window behind a synchronised kernel move what it wrote, window after window through the same blocks."""
+    """The messages of a window behind a synchronised kernel move what it wrote."""
     n = 50_000
     sym, local = rt.zeros((8, n), torch.int32), torch.zeros((8, n), dtype=torch.int32, device="cuda")
     for i in range(1, 60):
@@ -107,4 +107,41 @@ def test_what_the_stream_wrote_before(rt, ctx):
             ctx.put(sym[k], local[k], 0, nbi=True)
         ctx.quiet()
         assert bool((sym == i).all())
+    rt.free(sym, collective=False)
+
+
+def test_what_the_messages_wrote_before(rt, ctx):
+    """Within one window, through the same blocks: a buffer is read by messages, written by another one, and read again, over and over."""
+    n, rounds = 300_000, 30
+    sym, values = rt.zeros((2 * rounds + 1, n), torch.uint8), _random(rounds * n).view(rounds, n)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        sym.zero_()
+        torch.cuda.synchronize()
+        for i in range(rounds):
+            ctx.put(sym[0], values[i], 0, nbi=True)
+            ctx.put(sym[2 * i + 1], sym[0], 0, nbi=True)
+            ctx.get(sym[2 * i + 2], sym[0], 0, nbi=True)
+        ctx.quiet()
+        assert torch.equal(sym[1::2], values) and torch.equal(sym[2::2], values)
+    rt.free(sym, collective=False)
+
+
+def test_beside_products(rt, ctx):
+    """Blocks that find a place late, or not before the messages are done."""
+    a = torch.randn(4096, 4096, device="cuda", dtype=torch.bfloat16)
+    side, n = torch.cuda.Stream(), 200_000
+    sym, local = rt.zeros((16, n), torch.uint8), _random(16 * n).view(16, n)
+    torch.cuda.synchronize()
+    for count in (1, 2, 5, 16) * 10:
+        sym.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                a @ a
+        for k in range(count):
+            ctx.put(sym[k], local[k], 0, nbi=True)
+        ctx.quiet()
+        assert torch.equal(sym[:count], local[:count])
+    torch.cuda.synchronize()
     rt.free(sym, collective=False)
