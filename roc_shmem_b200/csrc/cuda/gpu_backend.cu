@@ -299,11 +299,13 @@ __global__ void __launch_bounds__(kRingThreads) k_ring(Ring* ring, uint32_t next
 // come by the time it finds messages take their part of them, pieces of 4 KiB, one round trip to memory of a warp, in turn.  None of them is
 // needed: beside a kernel that leaves a single place, of what a launch per message took, the first block does all, and the rest pass
 // through behind it.  (As a cluster of eight blocks of 512 threads, all of which had to find their places at once, this had no progress there.)
-// Windows of 64 puts, us, by a launch each (2.3 to 2.7 us apart, the host's) / as a cluster / so: 17 KB 175 / 60 / 44, 64 KiB 175 / 68 / 47, 256 KiB
-// 175 / 94 / 66, 512 KiB 175 / 140 / 95.  Up to 16 KiB one block is as fast (8 KiB 45) and holds one multiprocessor.  Products of 1024 rows with 64
-// messages of 64 KiB before each 180 / 71 / 57, with four 47.8 / 52 / 48.2 (without any 41.5).  All of it in this GPU's own memory; a
-// peer's is behind a link, where a block moves less.
+// us by a launch each (2.3 to 2.7 apart, the host's) / as a cluster / so.  Windows of 64 puts of 17 KB 175 / 56 / 35, 64 KiB 175 / 69 / 38, 256 KiB
+// 175 / 95 / 63, 512 KiB 175 / 140 / 93; eight puts of 64 KiB and a quiet 26 / 20 / 15, two 13 / 22 / 12.  A product of 1024 rows behind one message of
+// 64 KiB 42.7 / 46.3 / 42.6, behind four 49 / 52 / 49, behind 64 160 / 70 / 56 (41.5 without any).  Up to 16 KiB one block is as fast and holds
+// one multiprocessor.  All of it in this GPU's own memory; a peer's is behind a link, where a block moves less.
+// A batch of up to four rounds of the first block's warps is not handed out: that takes 2 us.
 constexpr unsigned kWideThreads = 256, kWideBlocks = 16, kWideWarps = kWideThreads / 32, kWidePublisher = kWideThreads - 32, kRingPiece = 4096;
+constexpr unsigned long long kWideComeNs = 3000;               // from the first block's begin on
 constexpr unsigned long long kWideLimitNs = 2000000000;        // of the waits for one another, each of which ends by itself
 struct RingShare {                     // device memory, zero between launches
   unsigned long long batch;            // by the first block: the batch's number | how many blocks it is for; number ~0: no more
@@ -343,9 +345,12 @@ __device__ __forceinline__ void ring_share_out(Ring* ring, RingShare* share, Rin
         unsigned pieces = lane < count ? (b.msg[lane].n + kRingPiece - 1) / kRingPiece : 0;
         pieces = __reduce_add_sync(0xffffffffu, pieces);
         unsigned here = 1;
-        if (pieces > kWideWarps) {
+        if (pieces > 4 * kWideWarps) {
           for (unsigned i = lane; i < sizeof(RingMessages) / 4; i += 32) reinterpret_cast<uint32_t*>(&share->b)[i] = reinterpret_cast<const uint32_t*>(&b)[i];
-          asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(&share->came) : "memory");
+          // launched together, they come together; a moment for those that are behind, once
+          if (lane == 0)
+            do asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(&share->came) : "memory");
+            while (here != gridDim.x && dev::timer() - begun < kWideComeNs);
           here = __shfl_sync(0xffffffffu, here, 0);
           __syncwarp();
         }
@@ -358,6 +363,7 @@ __device__ __forceinline__ void ring_share_out(Ring* ring, RingShare* share, Rin
       const unsigned here = blocks;
       batch += here > 1;
       copy_pieces(b, count, warp, here * kWideWarps);
+      last = dev::timer();             // idle from here on
       __syncthreads();
       next += count;
       // one thread waits for the others' parts and says how far the messages are done, while the first warp looks for more
