@@ -96,8 +96,11 @@ def mover(lib: C.CDLL, name: str, context, method: str, plain, local: int):
     if table is None:                             # a torch without it
         return getattr(context, method)
     rt = context.rt
-    return _pycall().Mover(C.cast(getattr(lib, name), C.c_void_p).value, rt._hv, context.idx, rt._dev_index, local, torch.Tensor, table,
-                           context, method, plain, rt._check)
+    try:
+        return _pycall().Mover(C.cast(getattr(lib, name), C.c_void_p).value, rt._hv, context.idx, rt._dev_index, local, torch.Tensor, table,
+                               context, method, plain, rt._check)
+    except ValueError:                            # a table of another version, or without what is used of it
+        return getattr(context, method)
 
 
 class _build_lock:

@@ -1,6 +1,7 @@
 """put and get of a device context as the runtime makes it (csrc/host/pycall.cc, Mover), with recorders in place of the native calls."""
 import ctypes as C
 
+import pytest
 import torch
 
 from tests.test_cpu_tracing import _runtime, ranges  # noqa: F401  (ranges: a fixture)
@@ -24,3 +25,28 @@ def test_a_native_message_has_its_range(ranges):  # noqa: F811
             assert ranges == [f"bshmem.{name}"] * (2 if on else 0)
     if hasattr(torch.Tensor, "__dlpack_c_exchange_api__"):
         assert type(ctx.put) is _native._pycall().Mover
+
+
+class _Table(C.Structure):
+    _fields_ = [("major", C.c_uint32), ("minor", C.c_uint32), ("older", C.c_void_p), ("allocate", C.c_void_p), ("owned_from", C.c_void_p),
+                ("to", C.c_void_p), ("describe", C.c_void_p), ("work_stream", C.c_void_p)]
+
+
+@pytest.mark.parametrize("fault", ["another version", "nothing to describe a tensor with", "another capsule"])
+def test_a_context_without_a_table_for_it(ranges, monkeypatch, fault):  # noqa: F811
+    """Where torch's table is not the one that is known, a context is created all the same, with the general methods."""
+    from roc_shmem_b200 import gpu
+    table = _Table(2 if fault == "another version" else 1, 0, describe=None if fault.startswith("nothing") else 1)
+    new = C.pythonapi.PyCapsule_New
+    new.restype, new.argtypes = C.py_object, [C.c_void_p, C.c_char_p, C.c_void_p]
+    name = C.create_string_buffer(b"another" if fault == "another capsule" else b"dlpack_exchange_api")
+    monkeypatch.setattr(torch.Tensor, "__dlpack_c_exchange_api__", new(C.addressof(table), name, None), raising=False)
+    rt, _ = _runtime(-1)
+    lib, calls = C.CDLL(None), []
+    rt.lib, rt._check = type("Lib", (), {"bshmem_gpu_ctx_put_dev": lib.labs, "bshmem_gpu_ctx_get_dev": lib.labs}), None
+    rt._c_put_dev, rt._c_get_dev = (lambda *a: calls.append("put")), (lambda *a: calls.append("get"))
+    ctx = gpu.DeviceRuntime._context_type(rt, 1, 0, None)
+    t = torch.zeros(4)
+    ctx.put(t, t, 0)
+    ctx.get(t, t, 0, nbi=True)
+    assert calls == ["put", "get"] and not hasattr(ctx.put, "context")
