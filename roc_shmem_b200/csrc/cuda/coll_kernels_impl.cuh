@@ -154,8 +154,11 @@ __global__ void __launch_bounds__(kThreads) COLL_CAT(k_coll_group_, COLL_UNIT)(c
 // and now, us: allreduce 16 KiB fp32, 4 PEs 14.9 -> 9.6; 1 MiB bf16, 8 PEs 23.4 -> 12.6; 32 MiB fp32, 8 PEs 117 -> 103; reduce-scatter
 // 32 MiB bf16, 8 PEs 83.7 -> 59.8 (302 MB, 46 at the copy rate), 32 MiB fp32, 4 PEs 50.0 -> 39.8; fcollect 16 MiB, 8 PEs 44.4 -> 38.4;
 // alltoall 32 MiB, 8 PEs 110 -> 98, 2 MiB, 4 PEs 20.1 -> 12.3.
-// 512 threads with 16 loads of 16 bytes each on their way keep 128 KB in flight per block; a block to a multiprocessor, as many as
-// the caller asked for.
+// 512 threads; a reduction has up to 16 loads of 16 bytes on their way per thread, and so 128 KB per block, a move eight; a block to a
+// multiprocessor, as many as the caller asked for.  24 MB per PE in 128 blocks, us, staged as before / one vector at a time for numbers of members
+// other than 2, 4 and 8 and for the rarer types and operators / so:  fp32 sum, 3 / 6 / 7 PEs 48.5 / 49.5 / 37.9, 76 / 88 / 68, 90 / 95 / 78; int16
+// maximum, 2 PEs 36.4 / 53 / 23.5; fp32 product, 8 PEs 135 / 102 / 83; reduce-scatter of int8 sums, 5 PEs 67 / 63 / 40.  One vector
+// at a time is still the better way for the rarer operators on eight bytes: AND of 7 PEs 141 / 73, two at a time 78.
 constexpr int kPassThreads = 512;
 
 __device__ __forceinline__ State pass_state(const GroupPass& g) {      // what the counters and the trace take of a state
@@ -194,7 +197,7 @@ __device__ __forceinline__ unsigned long long pass_trace_capacity(const GroupPas
 // nv vectors of every member from byte src_at of its heap on, reduced in team order, to byte dst_at of the heaps of members
 // [d0, d0 + nd).  NS sources (more than `size`: those beyond it are left out), U vectors of each on their way per thread.
 template <typename T, int OP, int NS, int U>
-__device__ __forceinline__ void pass_vectors(const GroupPass& g, uint64_t src_at, uint64_t dst_at, int d0, int nd, size_t nv) {
+__device__ __forceinline__ void pass_vectors(const GroupPass& g, int size, uint64_t src_at, uint64_t dst_at, int d0, int nd, size_t nv) {
   using A = typename coll::Acc<T>::type;
   constexpr int VE = 16 / sizeof(T);
   for (size_t v0 = threadIdx.x; v0 < nv; v0 += (size_t)U * blockDim.x) {
@@ -205,7 +208,7 @@ __device__ __forceinline__ void pass_vectors(const GroupPass& g, uint64_t src_at
       if (v < nv) {
 #pragma unroll
         for (int k = 0; k < NS; ++k)
-          if (k < g.size) in[u][k].raw = *reinterpret_cast<const uint4*>(g.base[k] + src_at + v * 16);
+          if (k < size) in[u][k].raw = *reinterpret_cast<const uint4*>(g.base[k] + src_at + v * 16);
       }
     }
 #pragma unroll
@@ -217,7 +220,7 @@ __device__ __forceinline__ void pass_vectors(const GroupPass& g, uint64_t src_at
         for (int e = 0; e < VE; ++e) acc[e] = coll::to_acc<T>(in[u][0].e[e]);
 #pragma unroll
         for (int k = 1; k < NS; ++k) {
-          if (k < g.size) {
+          if (k < size) {
 #pragma unroll
             for (int e = 0; e < VE; ++e) acc[e] = coll::apply<A>(OP, acc[e], coll::to_acc<T>(in[u][k].e[e]));
           }
@@ -235,20 +238,18 @@ __device__ __forceinline__ void pass_reduce_op(const GroupPass& g, uint64_t src_
   using A = typename coll::Acc<T>::type;
   constexpr int VE = 16 / sizeof(T);
   const size_t nv = ((src_at | dst_at) & 15) == 0 ? n / VE : 0;
-  // the types and operators of bulk reductions in unrolled form, the rest in a general one
+  // sixteen loads on their way per thread, or what the number of members leaves of the next form's; for the types and operators of bulk
+  // reductions also without a question per load whether there is such a member (1 % of 32 MiB)
   constexpr bool kHot = (OP == BSHMEM_SUM || OP == BSHMEM_MAX || OP == BSHMEM_MIN) &&
                         (std::is_same<T, float>::value || std::is_same<T, double>::value || std::is_same<T, __half>::value ||
                          std::is_same<T, __nv_bfloat16>::value || std::is_same<T, int32_t>::value || std::is_same<T, long long>::value);
-  if constexpr (kHot) {
-    switch (g.size) {
-      case 2: pass_vectors<T, OP, 2, 8>(g, src_at, dst_at, d0, nd, nv); break;
-      case 4: pass_vectors<T, OP, 4, 4>(g, src_at, dst_at, d0, nd, nv); break;
-      case 8: pass_vectors<T, OP, 8, 2>(g, src_at, dst_at, d0, nd, nv); break;
-      default: pass_vectors<T, OP, BSHMEM_MAX_PES, 1>(g, src_at, dst_at, d0, nd, nv);
-    }
-  } else {
-    pass_vectors<T, OP, BSHMEM_MAX_PES, 1>(g, src_at, dst_at, d0, nd, nv);
-  }
+  if (kHot && g.size == 8) pass_vectors<T, OP, 8, 2>(g, 8, src_at, dst_at, d0, nd, nv);
+  else if (kHot && g.size == 4) pass_vectors<T, OP, 4, 4>(g, 4, src_at, dst_at, d0, nd, nv);
+  else if (kHot && g.size == 2) pass_vectors<T, OP, 2, 8>(g, 2, src_at, dst_at, d0, nd, nv);
+  else if (g.size <= 2) pass_vectors<T, OP, 2, 8>(g, g.size, src_at, dst_at, d0, nd, nv);
+  else if (g.size <= 4) pass_vectors<T, OP, 4, 4>(g, g.size, src_at, dst_at, d0, nd, nv);
+  else if (g.size <= 8 && (kHot || sizeof(T) < 8)) pass_vectors<T, OP, 8, 2>(g, g.size, src_at, dst_at, d0, nd, nv);
+  else pass_vectors<T, OP, BSHMEM_MAX_PES, 1>(g, g.size, src_at, dst_at, d0, nd, nv);
   // what is left behind the last whole vector, or all of it where the two sides are not on 16-byte boundaries
   for (size_t i = nv * VE + threadIdx.x; i < n; i += blockDim.x) {
     A acc = coll::to_acc<T>(reinterpret_cast<const T*>(g.base[0] + src_at)[i]);

@@ -63,7 +63,7 @@ class Both:
         self.g.close()
 
 
-@pytest.fixture(scope="module", params=[1, 2, 3, 4, 8])
+@pytest.fixture(scope="module", params=[1, 2, 3, 4, 5, 7, 8, 9])
 def both(request):
     b = Both(request.param)
     yield b
