@@ -740,12 +740,12 @@ class GpuBackend final : public Backend {
     RT_TRY(cudaHostAlloc(&L.pinned, sizeof(Pinned), cudaHostAllocMapped));
     memset(L.pinned, 0, sizeof(Pinned));
     RT_TRY(cudaMalloc(&L.dstatus, sizeof(int)));
-    RT_TRY(cudaMemset(L.dstatus, 0, sizeof(int)));
+    RT_TRY(cudaMemsetAsync(L.dstatus, 0, sizeof(int), L.stream));       // where they are used: that stream does not wait for the default one
     Ring* ring = nullptr;
     RT_TRY(cudaHostAlloc(&ring, sizeof(Ring), cudaHostAllocMapped));
     memset(ring, 0, sizeof(Ring));
     RT_TRY(cudaMalloc(&L.share, sizeof(RingShare)));
-    RT_TRY(cudaMemset(L.share, 0, sizeof(RingShare)));
+    RT_TRY(cudaMemsetAsync(L.share, 0, sizeof(RingShare), L.stream));
     L.ring.open(ring);
     L.open = true;
     return BSHMEM_OK;

@@ -35,3 +35,11 @@ def test_a_served_signal_is_there_before_its_answer():
     case = case[:case.index("break;")]
     steps = re.findall(r"copy_bytes<|__syncthreads|fence_peers|signal_update|signal_done", case)
     assert steps == ["copy_bytes<", "__syncthreads", "fence_peers", "signal_update", "fence_peers", "signal_done"]
+
+
+def test_a_contexts_words_are_cleared_where_they_are_used():
+    """A context's stream does not wait for the default stream: what its kernels find zeroed is zeroed in that stream."""
+    text = (CSRC / "cuda" / "gpu_backend.cu").read_text()
+    body = text[text.index("int ctx_open("):text.index("void ctx_close(")]
+    assert re.findall(r"cudaMalloc\(&L\.(\w+)", body) == re.findall(r"cudaMemsetAsync\(L\.(\w+), 0, sizeof\(\w+\), L\.stream\)", body)
+    assert "cudaMemset(" not in body

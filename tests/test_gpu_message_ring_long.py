@@ -145,3 +145,19 @@ def test_beside_products(rt, ctx):
         assert torch.equal(sym[:count], local[:count])
     torch.cuda.synchronize()
     rt.free(sym, collective=False)
+
+
+def test_a_context_made_while_the_default_stream_is_busy(rt):
+    n = 200_000
+    sym, local = rt.zeros((8, n), torch.uint8), _random(8 * n).view(8, n)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        sym.zero_()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)
+        with rt.ctx_create() as c:
+            for k in range(8):
+                c.put(sym[k], local[k], 0, nbi=True)
+            c.quiet()
+        assert torch.equal(sym, local)
+    rt.free(sym, collective=False)
