@@ -177,6 +177,7 @@ bool move_at_once(const Mover* m, PyObject* const* args, Py_ssize_t n, PyObject*
       return false;
     }
   const DlTensor& l = t[m->local];
+  if (!t[0].data || !t[1].data) return false;        // tensors that a transformation made up have none
   if (l.device.type != kDlCuda || l.device.id != m->device || (l.dtype.bits & 7)) return false;
   uint64_t bytes = (uint64_t)(l.dtype.bits >> 3) * l.dtype.lanes;
   for (int i = 0; i < l.ndim; ++i) bytes *= (uint64_t)l.shape[i];
