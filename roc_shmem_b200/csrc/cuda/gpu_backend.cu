@@ -474,6 +474,7 @@ constexpr unsigned kCallThreads = 512;
 constexpr unsigned long long kCallIdleNs = 8000, kCallLifeNs = 500000;
 // Puts with signal: what the block copies as fast as two launches begin.  The four calls above with 32 / 64 / 128 / 256 / 400 / 512 KiB by launches
 // 33.9 / 34.4 / 34.4 / 34.4 / 34.3 / 34.6 us, so 25.8 / 26.2 / 26.9 / 30.0 / 33.0 / 40.0.  (Off each other's alignment kSmallSignalMax.)
+// All of it in this GPU's own memory: over a link one block moves some 50 GB/s.
 constexpr uint64_t kServedSignalMax = 256u << 10;
 __global__ void __launch_bounds__(kCallThreads) k_calls(State s, CallSlot* slot, uint32_t seq, uint32_t generation) {
   __shared__ uint32_t req[kCallWords];

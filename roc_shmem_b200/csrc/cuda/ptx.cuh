@@ -54,8 +54,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Per-thread asynchronous copies, global -> shared; each thread waits for its own groups.
-// Whether the phase is complete now.  An answer takes some 100 cycles, so it can be asked for ahead of what needs it.
+// Whether the phase is complete now, as this lane sees it.  An answer takes some 100 cycles, so it can be asked for ahead of what needs it.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -70,6 +69,7 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
   return p != 0;
 }
+// Per-thread asynchronous copies, global -> shared; each thread waits for its own groups.
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
