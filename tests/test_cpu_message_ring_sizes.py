@@ -1,4 +1,4 @@
-"""Messages of both kinds in a context's ring (csrc/cuda/message_ring.h): short ones that one block takes and long ones that are for a cluster,
+"""Messages of both kinds in a context's ring (csrc/cuda/message_ring.h): short ones that one block takes and long ones that are for several,
 mixed, around operations of the stream.  The model of tests/test_cpu_message_ring.py with sizes, and blocks that know which they are."""
 import shutil
 import subprocess
