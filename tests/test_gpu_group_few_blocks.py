@@ -71,7 +71,8 @@ def test_few_blocks_and_many(pes, ctas, n):
 
 
 def test_more_blocks_than_multiprocessors():
-    """The exchanging form's launch, which wants them all at once, turns such calls away; the passes in between share its device table and counter."""
+    """The exchanging form's launch, which wants them all at once, turns such calls away, and takes barriers; the passes in between share its device
+    table and counter."""
     import roc_shmem_b200 as shmem
     from roc_shmem_b200 import gpu
     pes, n = 8, 4099
@@ -93,6 +94,7 @@ def test_more_blocks_than_multiprocessors():
                 want = [None] * pes
             else:
                 g.collective(kind, dst, src, n * 4, root=3, ctas=ctas)
+            g.collective(gpu.COLL_BARRIER, None, None, 0, ctas=1 + i % 3)
             for d, w in zip(dst, want):
                 m = 0 if w is None else w.numel()
                 assert (w is None or torch.equal(d[:m], w)) and bool((d[m:] == 7).all()), (i, ctas, kind)
